@@ -5,7 +5,9 @@ plus the reference-named C++ launchers (``include/helios_b200_shim.hpp``).  This
 Python host side used by the tests and the benchmark: it loads the library with ctypes and exposes
 one function per reference launcher, under the reference's names and argument order
 (``helios::attn::*`` in src/cuda/attn/attn.cuh, ``helios::aux::*`` in src/cuda/aux/gdn.cuh and
-dsa_topk.cuh of the reference tree), taking torch CUDA tensors as device buffers.
+dsa_topk.cuh of the reference tree), taking torch CUDA tensors as device buffers.  The calls of a
+decode or prefill step go through a small CPython binding (``csrc/binding.cpp``) bound to the same library;
+set-up and multi-GPU calls go through ctypes.
 
 There is no CPU path: calling a compute entry point without the library or without a CUDA device
 raises.  PyTorch is used for device memory and streams only.
@@ -114,6 +116,26 @@ def load_library():
     return _lib
 
 
+class _LazyBinding:
+    """Stands in for the CPython binding until the first call through it."""
+
+    def __getattr__(self, name):
+        global _native
+        _require_cuda()                       # the binding's torch libraries are the loaded ones
+        try:
+            from . import _binding
+        except ImportError as exc:
+            raise RuntimeError("helios_glm53flash_b200/_binding.so is not built (run `python -m helios_glm53flash_b200.build` or "
+                               "__graft_entry__.build()); this package has no fallback path") from exc
+        lib = load_library()
+        _binding.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in SIGNATURES})
+        _native = _binding
+        return getattr(_binding, name)
+
+
+_native = _LazyBinding()
+
+
 def status_string(status):
     return load_library().hk_status_string(int(status)).decode()
 
@@ -141,6 +163,13 @@ def _call(name, *args):
         raise HeliosB200Error(name, st)
 
 
+def _run(name, *args):
+    """one entry point through the binding: tensors and None as they are, the stream (None = torch's current one) last"""
+    st = getattr(_native, name)(*args)
+    if st:
+        raise HeliosB200Error(name, st)
+
+
 def _scratch(nbytes, device, stream=None):
     """A torch-owned scratch buffer (256-byte aligned by the caching allocator).  The kernels that use it run on
     `stream`; when that is not torch's current stream the block is recorded on it, so that the caching allocator
@@ -158,9 +187,8 @@ def _scratch(nbytes, device, stream=None):
 def cuda_causal_conv1d_update(x, conv_state, slots, weight, bias, out, bsz, dim, seqlen, state_size,
                               K, activation, history, stream=None):
     """helios::aux::cuda_causal_conv1d_update (src/cuda/aux/gdn.cuh:67-83)."""
-    _call("hk_conv1d_update", _ptr(x), _ptr(conv_state), _ptr(slots), _ptr(weight), _ptr(bias),
-          _ptr(out), bsz, dim, seqlen, state_size, K, int(bool(activation)), int(bool(history)),
-          _stream(stream))
+    _run("hk_conv1d_update", x, conv_state, slots, weight, bias, out, bsz, dim, seqlen, state_size, K, 1 if activation else 0, 1
+         if history else 0, stream)
 
 
 def cuda_recurrent_gated_delta_rule(mixed_qkv, g, beta, recurrent_state, core_attn_out, bsz, seqlen,
@@ -172,24 +200,21 @@ def cuda_recurrent_gated_delta_rule(mixed_qkv, g, beta, recurrent_state, core_at
     As the C++ launcher of this library does, long channelwise calls go to the chunked tensor-core
     kernel; ``force_recurrent`` keeps the per-token kernel.  ``out_f32`` optionally receives the
     output before bf16 rounding."""
-    chunked = not force_recurrent and load_library().hk_kda_dispatch_is_chunked(
-        seqlen, num_k_heads, num_v_heads, k_head_dim, v_head_dim, history_stride, int(bool(channelwise)),
-        int(bool(history))) != 0
+    chunked = not force_recurrent and _native.hk_kda_dispatch_is_chunked(
+        seqlen, num_k_heads, num_v_heads, k_head_dim, v_head_dim, history_stride, 1 if channelwise else 0,
+        1 if history else 0)
     if chunked:
-        nbytes = load_library().hk_kda_chunked_workspace_bytes(bsz, seqlen, num_v_heads)
-        ws = workspace if workspace is not None else _scratch(nbytes, mixed_qkv.device, stream)
-        st = load_library().hk_kda_chunked_prefill(
-            _ptr(mixed_qkv), _ptr(g), _ptr(beta), _ptr(recurrent_state), _ptr(core_attn_out),
-            _ptr(out_f32), bsz, seqlen, num_v_heads, _ptr(slots), _ptr(ws), ws.numel(),
-            _stream(stream))
+        ws = workspace
+        if ws is None:
+            ws = _scratch(_native.hk_kda_chunked_workspace_bytes(bsz, seqlen, num_v_heads), mixed_qkv.device, stream)
+        st = _native.hk_kda_chunked_prefill(mixed_qkv, g, beta, recurrent_state, core_attn_out, out_f32, bsz, seqlen, num_v_heads,
+                                            slots, ws, ws, stream)
         if st == HK_OK:
             return "chunked"
         if st != HK_ERR_UNSUPPORTED:
             raise HeliosB200Error("hk_kda_chunked_prefill", st)
-    _call("hk_kda_recurrent", _ptr(mixed_qkv), _ptr(g), _ptr(beta), _ptr(recurrent_state),
-          _ptr(core_attn_out), _ptr(out_f32), bsz, seqlen, num_k_heads, num_v_heads, k_head_dim,
-          v_head_dim, history_stride, _ptr(slots), int(bool(channelwise)), int(bool(history)),
-          _stream(stream))
+    _run("hk_kda_recurrent", mixed_qkv, g, beta, recurrent_state, core_attn_out, out_f32, bsz, seqlen, num_k_heads, num_v_heads,
+         k_head_dim, v_head_dim, history_stride, slots, 1 if channelwise else 0, 1 if history else 0, stream)
     return "recurrent"
 
 
@@ -207,9 +232,8 @@ def kda_decode_step(x, conv_state, conv_weight, conv_bias, g, beta, rec_state, o
         tickets = _decode_tickets.get(key)
         if tickets is None:
             tickets = _decode_tickets[key] = torch.zeros(bsz * num_heads, dtype=torch.int32, device=x.device)
-    _call("hk_kda_decode_step", _ptr(x), _ptr(conv_state), _ptr(conv_weight), _ptr(conv_bias), _ptr(g), _ptr(beta),
-          _ptr(rec_state), _ptr(out), _ptr(out_f32), _ptr(conv_out), bsz, num_heads, _ptr(slots), _ptr(tickets),
-          _stream(stream))
+    _run("hk_kda_decode_step", x, conv_state, conv_weight, conv_bias, g, beta, rec_state, out, out_f32, conv_out, bsz,
+         num_heads, slots, tickets, stream)
 
 
 def kda_decode_layer(x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_log, lower_bound, rec_state, out, norm_w,
@@ -225,10 +249,9 @@ def kda_decode_layer(x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_l
         tickets = _decode_tickets.get(key)
         if tickets is None:
             tickets = _decode_tickets[key] = torch.zeros(2 * bsz * num_heads, dtype=torch.int32, device=x32.device)
-    _call("hk_kda_decode_layer", _ptr(x32), _ptr(conv_state), _ptr(conv_weight), _ptr(conv_bias), _ptr(f), _ptr(b), _ptr(dt_bias),
-          _ptr(a_log), float(lower_bound), _ptr(rec_state), _ptr(out), _ptr(out_f32), _ptr(norm_w), _dtype_code(norm_w),
-          _ptr(gate_out), _dtype_code(gate_out), _ptr(y), _dtype_code(y), float(epsilon), float(constant_bias), int(gate_act),
-          bsz, num_heads, _ptr(slots), _ptr(tickets), _stream(stream))
+    _run("hk_kda_decode_layer", x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_log, lower_bound, rec_state, out,
+         out_f32, norm_w, norm_w, gate_out, gate_out, y, y, epsilon, constant_bias, int(gate_act), bsz, num_heads, slots,
+         tickets, stream)
 
 
 def kda_chunked_set_form(form):
@@ -245,11 +268,11 @@ def kda_chunked_prefill_gated(mixed_qkv, f, b, dt_bias, a_log, lower_bound, recu
     """Chunked KDA prefill that forms g and beta itself from the raw gate projection ``f``, the raw beta
     logit ``b`` and the layer's ``dt_bias`` / ``a_log`` (the arithmetic of helios::glue::kda_gate,
     src/engine/glue2.cu:347-360), head dim 128."""
-    nbytes = load_library().hk_kda_chunked_workspace_bytes(bsz, seqlen, num_heads)
-    ws = workspace if workspace is not None else _scratch(nbytes, mixed_qkv.device, stream)
-    _call("hk_kda_chunked_prefill_gated", _ptr(mixed_qkv), _ptr(f), _ptr(b), _ptr(dt_bias), _ptr(a_log),
-          float(lower_bound), _ptr(recurrent_state), _ptr(core_attn_out), _ptr(out_f32), bsz, seqlen,
-          num_heads, _ptr(slots), _ptr(ws), ws.numel(), _stream(stream))
+    ws = workspace
+    if ws is None:
+        ws = _scratch(_native.hk_kda_chunked_workspace_bytes(bsz, seqlen, num_heads), mixed_qkv.device, stream)
+    _run("hk_kda_chunked_prefill_gated", mixed_qkv, f, b, dt_bias, a_log, lower_bound, recurrent_state, core_attn_out, out_f32,
+         bsz, seqlen, num_heads, slots, ws, ws, stream)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -257,82 +280,67 @@ def kda_chunked_prefill_gated(mixed_qkv, f, b, dt_bias, a_log, lower_bound, recu
 # ---------------------------------------------------------------------------------------------
 def kda_transpose_cast(dst_bf16, src, S, F, stream=None):
     """helios::glue::kda_transpose_cast (src/engine/glue2.cuh:61): [S][F] f32 -> [F][S] bf16."""
-    _call("hk_kda_transpose_cast", _ptr(dst_bf16), _ptr(src), S, F, _stream(stream))
+    _run("hk_kda_transpose_cast", dst_bf16, src, S, F, stream)
 
 
 def kda_gate(b, f, dt_bias, a_log, lower_bound, beta_bf16, g, S, H, Dk, stream=None):
     """helios::glue::kda_gate (src/engine/glue2.cuh:62-63)."""
-    _call("hk_kda_gate", _ptr(b), _ptr(f), _ptr(dt_bias), _ptr(a_log), float(lower_bound), _ptr(beta_bf16),
-          _ptr(g), S, H, Dk, _stream(stream))
+    _run("hk_kda_gate", b, f, dt_bias, a_log, lower_bound, beta_bf16, g, S, H, Dk, stream)
 
 
 def kda_prepare(qkv, b, f, dt_bias, a_log, lower_bound, mixed_qkv_bf16, beta_bf16, g, S, F, H, Dk,
                 stream=None):
     """helios::glue::kda_prepare (src/engine/glue2.cuh:64-67)."""
-    _call("hk_kda_prepare", _ptr(qkv), _ptr(b), _ptr(f), _ptr(dt_bias), _ptr(a_log), float(lower_bound),
-          _ptr(mixed_qkv_bf16), _ptr(beta_bf16), _ptr(g), S, F, H, Dk, _stream(stream))
+    _run("hk_kda_prepare", qkv, b, f, dt_bias, a_log, lower_bound, mixed_qkv_bf16, beta_bf16, g, S, F, H, Dk, stream)
 
 
 def kda_cast_conv(x_f32, conv_state, slots, weight, bias, out, bsz, dim, seqlen, activation, stream=None):
     """kda_transpose_cast + cuda_causal_conv1d_update(K = 4) in one pass over token-major fp32 input."""
-    _call("hk_kda_cast_conv", _ptr(x_f32), _ptr(conv_state), _ptr(slots), _ptr(weight), _ptr(bias), _ptr(out),
-          bsz, dim, seqlen, int(bool(activation)), _stream(stream))
-
-
-def _dtype_code(t):
-    torch = _require_cuda()
-    return {torch.float16: HK_F16, torch.bfloat16: HK_BF16, torch.float32: HK_F32}[t.dtype]
+    _run("hk_kda_cast_conv", x_f32, conv_state, slots, weight, bias, out, bsz, dim, seqlen, 1 if activation else 0, stream)
 
 
 def gated_rms_norm(x, w, y, g, rows, dim, epsilon, constant_bias=0.0, w_groups=1, gate_first=False,
                    gate_act=0, stream=None):
     """helios::aux::gated_rms_norm (src/cuda/aux/norm.cuh:71-87); dtypes taken from the tensors."""
-    _call("hk_gated_rms_norm", _ptr(x), _ptr(w), _dtype_code(w), _ptr(y), _dtype_code(y), _ptr(g),
-          _dtype_code(g), rows, dim, float(epsilon), float(constant_bias), w_groups, int(bool(gate_first)),
-          int(gate_act), _stream(stream))
+    _run("hk_gated_rms_norm", x, w, w, y, y, g, g, rows, dim, epsilon, constant_bias, w_groups, 1 if gate_first else 0,
+         int(gate_act), stream)
 
 
 def layernorm_f16(x, w, b, y, rows, dim, eps, stream=None):
     """helios::glue::layernorm_f16 (src/engine/glue2.cuh:73-75)."""
-    _call("hk_layernorm_f16", _ptr(x), _ptr(w), _ptr(b), _ptr(y), rows, dim, float(eps), _stream(stream))
+    _run("hk_layernorm_f16", x, w, b, y, rows, dim, eps, stream)
 
 
 def mla_decode_prologue(kv_pre, ln_w, ckv, eps_rms, idx_k, knorm_w, knorm_b, idx_kn, eps_ln, idx_g, raw_ring, raw_rows,
                         pool_k_nt, ape, pos, q_pos_out=None, stream=None):
     """cache append + indexer key layer norm + pooled-key write of ONE new token (src/engine/runner.cpp:569-584) in one
     launch; q_pos_out (device int32[1], optional) receives pos"""
-    _call("hk_mla_decode_prologue", _ptr(kv_pre), _ptr(ln_w), _ptr(ckv), float(eps_rms), _ptr(idx_k), _ptr(knorm_w),
-          _ptr(knorm_b), _ptr(idx_kn), float(eps_ln), _ptr(idx_g), _ptr(raw_ring), raw_rows, _ptr(pool_k_nt), _ptr(ape),
-          int(pos), _ptr(q_pos_out), _stream(stream))
+    _run("hk_mla_decode_prologue", kv_pre, ln_w, ckv, eps_rms, idx_k, knorm_w, knorm_b, idx_kn, eps_ln, idx_g, raw_ring,
+         raw_rows, pool_k_nt, ape, int(pos), q_pos_out, stream)
 
 
 def mla_cache_append(kv_pre, ln_w, ckv, pos, n, eps, ckv_new=None, stream=None):
     """aux::rms_norm (fp32 in, fp16 weight, fp16 out, dim 512) + the copy into the latent cache
     (src/engine/runner.cpp:569-572) as one kernel."""
-    _call("hk_mla_cache_append", _ptr(kv_pre), _ptr(ln_w), _ptr(ckv), _ptr(ckv_new), pos, n, float(eps),
-          _stream(stream))
+    _run("hk_mla_cache_append", kv_pre, ln_w, ckv, ckv_new, pos, n, eps, stream)
 
 
 def dsa_topk(scores, s_stride, indices, R, T, k, k_pad, t_ptr=None, t_seq=0, stream=None):
     """helios::aux::dsa_topk (src/cuda/aux/dsa_topk.cuh:15-27)."""
-    _call("hk_dsa_topk", _ptr(scores), s_stride, _ptr(indices), R, T, k, k_pad, _ptr(t_ptr), t_seq,
-          _stream(stream))
+    _run("hk_dsa_topk", scores, s_stride, indices, R, T, k, k_pad, t_ptr, t_seq, stream)
 
 
 def dsa_topk_expand(scores, s_stride, indices, raw_idx, q_pos, R, T, k, after_scorer=False, stream=None):
     """dsa_topk (k_pad = 512) with pool_expand_row folded in: indices [R, 512] and raw_idx [R, 2052] in one kernel"""
-    _call("hk_dsa_topk_expand", _ptr(scores), s_stride, _ptr(indices), _ptr(raw_idx), _ptr(q_pos), R, T, k,
-          int(bool(after_scorer)), _stream(stream))
+    _run("hk_dsa_topk_expand", scores, s_stride, indices, raw_idx, q_pos, R, T, k, 1 if after_scorer else 0, stream)
 
 
 def indexer_select(q_idx, pool_k_nt, w, q_pos, scores, indices, raw_idx, m, npools, k=512, stream=None, score_stride=None,
                    n_heads=32):
     """decode-step selection: indexer_score -> top-k with the expansion folded in, two launches (the second a
     programmatic dependent of the first); scores = fp16 workspace [m, score_stride]"""
-    torch = _require_cuda()
-    dtype = HK_BF16 if q_idx.dtype == torch.bfloat16 else HK_F16
-    _call("hk_indexer_select", _ptr(q_idx), _ptr(pool_k_nt), _ptr(w), _ptr(q_pos), _ptr(scores), _ptr(indices),
-          _ptr(raw_idx), m, npools, npools if score_stride is None else score_stride, n_heads, dtype, k, _stream(stream))
+    _run("hk_indexer_select", q_idx, pool_k_nt, w, q_pos, scores, indices, raw_idx, m, npools, npools if score_stride is None
+         else score_stride, n_heads, q_idx, k, stream)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -340,17 +348,14 @@ def indexer_select(q_idx, pool_k_nt, w, q_pos, scores, indices, raw_idx, m, npoo
 # ---------------------------------------------------------------------------------------------
 def kpool_write(idx_k, idx_g, raw_ring, raw_rows, pool_k_nt, ape, pos_start, n_new, stream=None):
     """helios::attn::kpool_write (src/cuda/attn/attn.cuh:80-87)."""
-    _call("hk_kpool_write", _ptr(idx_k), _ptr(idx_g), _ptr(raw_ring), raw_rows, _ptr(pool_k_nt),
-          _ptr(ape), pos_start, n_new, _stream(stream))
+    _run("hk_kpool_write", idx_k, idx_g, raw_ring, raw_rows, pool_k_nt, ape, pos_start, n_new, stream)
 
 
 def indexer_score(q_idx, pool_k_nt, w, q_pos, scores, m, npools, stream=None, score_stride=None,
                   n_heads=32):
     """helios::attn::indexer_score (src/cuda/attn/attn.cuh:49-55); fp16 or bf16 keys by tensor dtype."""
-    torch = _require_cuda()
-    dtype = HK_BF16 if q_idx.dtype == torch.bfloat16 else HK_F16
-    _call("hk_indexer_score", _ptr(q_idx), _ptr(pool_k_nt), _ptr(w), _ptr(q_pos), _ptr(scores), m,
-          npools, npools if score_stride is None else score_stride, n_heads, dtype, _stream(stream))
+    _run("hk_indexer_score", q_idx, pool_k_nt, w, q_pos, scores, m, npools, npools if score_stride is None else score_stride,
+         n_heads, q_idx, stream)
 
 
 indexer_score_mma = indexer_score
@@ -358,18 +363,17 @@ indexer_score_mma = indexer_score
 
 def indexer_score_legacy(q_idx, pool_k, w, q_pos, scores, m, npools, pk_stride, stream=None):
     """helios::attn::indexer_score_legacy (src/cuda/attn/attn.cuh:46-48)."""
-    _call("hk_indexer_score_legacy", _ptr(q_idx), _ptr(pool_k), _ptr(w), _ptr(q_pos), _ptr(scores),
-          m, npools, pk_stride, _stream(stream))
+    _run("hk_indexer_score_legacy", q_idx, pool_k, w, q_pos, scores, m, npools, pk_stride, stream)
 
 
 def pool_expand(pool_idx, q_pos, raw_idx, m, cur_pos, stream=None, n_sel=512):
     """helios::attn::pool_expand (src/cuda/attn/attn.cuh:60-65): one cur_pos for every row."""
-    _call("hk_pool_expand", _ptr(pool_idx), None, _ptr(raw_idx), m, cur_pos, n_sel, _stream(stream))
+    _run("hk_pool_expand", pool_idx, None, raw_idx, m, cur_pos, n_sel, stream)
 
 
 def pool_expand_row(pool_idx, q_pos, raw_idx, m, stream=None, n_sel=512):
     """helios::attn::pool_expand_row (src/cuda/attn/attn.cuh:67-72)."""
-    _call("hk_pool_expand", _ptr(pool_idx), _ptr(q_pos), _ptr(raw_idx), m, 0, n_sel, _stream(stream))
+    _run("hk_pool_expand", pool_idx, q_pos, raw_idx, m, 0, n_sel, stream)
 
 
 def mla_auto_splits(m, n_keys):
@@ -380,24 +384,17 @@ def mla_partial_bytes(n_split, rows):
     return load_library().hk_mla_partial_bytes(n_split, rows)
 
 
-def _cache_rows(ckv, ckv_rows):
-    """rows of a [rows][512] cache tensor (0 = unknown, for buffers that are not laid out that way)"""
-    if ckv_rows is not None:
-        return int(ckv_rows)
-    return int(ckv.numel() // 512) if ckv.dim() >= 1 and ckv.numel() % 512 == 0 else 0
-
-
 def mla_sparse_decode(q_lat, ckv, raw_idx, kidx, lat_out, m, stream=None, scale=0.0625, n_heads=64,
                       n_split=0, workspace=None, ckv_rows=None):
     """helios::attn::mla_sparse_decode (src/cuda/attn/attn.cuh:93-99) with explicit scale / heads; the cache's row
     count is taken from the tensor, so row numbers beyond it are skipped instead of read."""
     if n_split <= 0:
-        n_split = mla_auto_splits(m, kidx)
+        n_split = _native.hk_mla_auto_splits(m, kidx)
     ws = workspace
     if n_split > 1 and ws is None:
         ws = _scratch(mla_partial_bytes(n_split, m * n_heads), q_lat.device, stream)
-    _call("hk_mla_sparse", _ptr(q_lat), _ptr(ckv), _cache_rows(ckv, ckv_rows), _ptr(raw_idx), kidx, _ptr(lat_out), m, n_heads,
-          float(scale), n_split, _ptr(ws), 0 if ws is None else ws.numel(), _stream(stream))
+    _run("hk_mla_sparse", q_lat, ckv, ckv if ckv_rows is None else ckv_rows, raw_idx, kidx, lat_out, m, n_heads, scale, n_split,
+         ws, ws, stream)
 
 
 def mla_sparse_decode_static(q_lat, ckv, raw_idx, kidx, lat_out, m, stream=None, scale=0.0625, n_split=0):
@@ -405,8 +402,7 @@ def mla_sparse_decode_static(q_lat, ckv, raw_idx, kidx, lat_out, m, stream=None,
     split partials use the library's built-in ~8 MiB device array (n_split * m <= 64), so neither
     this wrapper nor the library allocates anything.  Calls on one device share that array: do not
     let two of them overlap on the GPU."""
-    _call("hk_mla_sparse_static", _ptr(q_lat), _ptr(ckv), _ptr(raw_idx), kidx, _ptr(lat_out), m, float(scale),
-          n_split, _stream(stream))
+    _run("hk_mla_sparse_static", q_lat, ckv, raw_idx, kidx, lat_out, m, scale, n_split, stream)
 
 
 def mla_dense_prefill(q_lat, ckv, lat_out, qlen, pos_start, stream=None, scale=0.0625, n_heads=64,
@@ -414,39 +410,35 @@ def mla_dense_prefill(q_lat, ckv, lat_out, qlen, pos_start, stream=None, scale=0
     """helios::attn::mla_dense_prefill (src/cuda/attn/attn.cuh:104-108); qlen = 1 is dense decode.
     kv_base / kv_len (device int64 / int32 per row) select per-row cache ranges (batched decode)."""
     if n_split <= 0:
-        n_split = mla_auto_splits(qlen, n_keys_hint if n_keys_hint else pos_start + qlen)
+        n_split = _native.hk_mla_auto_splits(qlen, n_keys_hint if n_keys_hint else pos_start + qlen)
     ws = workspace
     if n_split > 1 and ws is None:
         ws = _scratch(mla_partial_bytes(n_split, qlen * n_heads), q_lat.device, stream)
-    _call("hk_mla_dense", _ptr(q_lat), _ptr(ckv), _cache_rows(ckv, ckv_rows), _ptr(kv_base), _ptr(kv_len), pos_start,
-          _ptr(lat_out), qlen, n_heads, float(scale), n_split, _ptr(ws),
-          0 if ws is None else ws.numel(), _stream(stream))
+    _run("hk_mla_dense", q_lat, ckv, ckv if ckv_rows is None else ckv_rows, kv_base, kv_len, pos_start, lat_out, qlen, n_heads,
+         scale, n_split, ws, ws, stream)
 
 
 def mla_dense_partial(q_lat, ckv, kv_base, kv_len, pos_start, part_m, part_l, part_acc, m,
                       n_heads=64, scale=0.0625, stream=None):
     """One split's un-normalised (m, l, acc) partial - the unit of split-KV across GPUs."""
-    _call("hk_mla_dense_partial", _ptr(q_lat), _ptr(ckv), _ptr(kv_base), _ptr(kv_len), pos_start,
-          _ptr(part_m), _ptr(part_l), _ptr(part_acc), m, n_heads, float(scale), _stream(stream))
+    _run("hk_mla_dense_partial", q_lat, ckv, kv_base, kv_len, pos_start, part_m, part_l, part_acc, m, n_heads, scale, stream)
 
 
 def mla_dense_partial_ws(q_lat, ckv, kv_base, kv_len, pos_start, part_m, part_l, part_acc, m, n_keys_hint,
                          n_heads=64, scale=0.0625, n_split=0, workspace=None, stream=None):
     """One partial set computed with every SM of this GPU (local splits merged on the GPU)."""
     if n_split <= 0:
-        n_split = mla_auto_splits(m, n_keys_hint)
+        n_split = _native.hk_mla_auto_splits(m, n_keys_hint)
     ws = workspace
     if n_split > 1 and ws is None:
         ws = _scratch(mla_partial_bytes(n_split, m * n_heads), q_lat.device, stream)
-    _call("hk_mla_dense_partial_ws", _ptr(q_lat), _ptr(ckv), _ptr(kv_base), _ptr(kv_len), pos_start, _ptr(part_m),
-          _ptr(part_l), _ptr(part_acc), m, n_heads, float(scale), n_split, n_keys_hint, _ptr(ws),
-          0 if ws is None else ws.numel(), _stream(stream))
+    _run("hk_mla_dense_partial_ws", q_lat, ckv, kv_base, kv_len, pos_start, part_m, part_l, part_acc, m, n_heads, scale,
+         n_split, n_keys_hint, ws, ws, stream)
 
 
 def lse_combine(part_m, part_l, part_acc, n_split, rows, out, stream=None):
     """Standalone split-KV log-sum-exp combine (the reference merges in-kernel, attn.cu:462-481)."""
-    _call("hk_lse_combine", _ptr(part_m), _ptr(part_l), _ptr(part_acc), n_split, rows, _ptr(out),
-          _stream(stream))
+    _run("hk_lse_combine", part_m, part_l, part_acc, n_split, rows, out, stream)
 
 
 def lse_combine_ptrs(ptrs_m, ptrs_l, ptrs_acc, n_split, rows, out, stream=None):
@@ -552,22 +544,22 @@ def lse_combine_peers(ptrs_m, ptrs_l, ptrs_acc, n_split, rows, out, local_flags,
 
 
 def q_latent(q_nope, kv_b, q_lat, m, stream=None):
-    _call("hk_q_latent", _ptr(q_nope), _ptr(kv_b), _ptr(q_lat), m, _stream(stream))
+    _run("hk_q_latent", q_nope, kv_b, q_lat, m, stream)
 
 
 q_latent_t = q_latent
 
 
 def o_absorb(lat_out, kv_b, o, m, stream=None):
-    _call("hk_o_absorb", _ptr(lat_out), _ptr(kv_b), _ptr(o), m, _stream(stream))
+    _run("hk_o_absorb", lat_out, kv_b, o, m, stream)
 
 
 def wuv_transpose(kv_b, wuv_t, stream=None):
-    _call("hk_wuv_transpose", _ptr(kv_b), _ptr(wuv_t), _stream(stream))
+    _run("hk_wuv_transpose", kv_b, wuv_t, stream)
 
 
 def o_absorb_t(lat_out, wuv_t, o, nrows, stream=None):
-    _call("hk_o_absorb_t", _ptr(lat_out), _ptr(wuv_t), _ptr(o), nrows, _stream(stream))
+    _run("hk_o_absorb_t", lat_out, wuv_t, o, nrows, stream)
 
 
 def read_device_status(reset=True):

@@ -117,22 +117,27 @@ class TrunkAttention:
         self._events = []
         return tot
 
+    # The library takes addresses and explicit row counts, so where a call works on the FIRST n rows of a buffer it is
+    # given the whole buffer: a torch slice costs the host about as much as a launch, and a decode step of 45 layers
+    # made some 300 of them (2.4 ms of host time around 1.1 ms of kernels).
     def kda_layer(self, L, n, timed=False):
         hk, ki, B, H, D, dim = self.hk, self.kda_in, self.B, self.H, self.D, self.dim
-        x32, f, b = ki["x32"][:, :n], ki["f"][:, :n], ki["b"][:, :n]
-        if n != self.max_chunk:
-            x32, f, b = x32.contiguous(), f.contiguous(), b.contiguous()
-        qkv, rec = self.qkv.view(-1)[:B * n * dim].view(B, n, dim), self.rec_out.view(-1)[:B * n * H * D].view(B, n, H, D)
+        x32, f, b = ki["x32"], ki["f"], ki["b"]
+        if B > 1 and n != self.max_chunk:
+            x32, f, b = x32[:, :n].contiguous(), f[:, :n].contiguous(), b[:, :n].contiguous()
         if n == 1 and self.fused:
             # a decoded token: the whole layer (cast, gates, conv, recurrence, gated norm) is one launch
-            y = self.kda_y[:B * H]
-            hk.kda_decode_layer(x32.reshape(B, dim), self.conv_state[L], ki["conv_w"], None, f.reshape(B, H, D), b.reshape(B, H),
-                                ki["dt_bias"], ki["a_log"], ki["lower_bound"], self.rec_state[L], rec, ki["norm_w"],
-                                ki["gate_out"][:B * H], y, B, H, epsilon=1e-6, gate_act=1)
+            hk.kda_decode_layer(x32, self.conv_state[L], ki["conv_w"], None, f, b, ki["dt_bias"], ki["a_log"], ki["lower_bound"],
+                                self.rec_state[L], self.rec_out, ki["norm_w"], ki["gate_out"], self.kda_y, B, H, epsilon=1e-6,
+                                gate_act=1)
             if self.keep:
-                self.kept.setdefault(("kda", L), []).append((rec.clone(), y.clone()))
+                self.kept.setdefault(("kda", L), []).append((self.rec_out.view(-1)[:B * H * D].view(B, 1, H, D).clone(),
+                                                             self.kda_y[:B * H].clone()))
             return
-        elif self.fused:
+        if B == 1 and n != self.max_chunk:
+            x32, f, b = x32[:, :n], f[:, :n], b[:, :n]
+        qkv, rec = self.qkv.view(-1)[:B * n * dim].view(B, n, dim), self.rec_out.view(-1)[:B * n * H * D].view(B, n, H, D)
+        if self.fused:
             hk.kda_cast_conv(x32, self.conv_state[L], None, ki["conv_w"], None, qkv, B, dim, n, True)
             if timed:
                 self._mark("kda_cast_conv")
@@ -198,25 +203,24 @@ class TrunkAttention:
         wb = self if bufs is None else bufs                    # work buffers: the chunk's shared ones, or this sequence's own
         if n == 1 and self.fused:
             # a decoded token: append, key layer norm, pooled-key write and the position in one launch
-            hk.mla_decode_prologue(mi["kv_pre"][:1], mi["ln_w"], ckv, 1e-6, mi["idx_k"][:1], mi["knorm_w"], mi["knorm_b"],
-                                   wb.idx_kn[:1], 1e-5, mi["idx_g"][:1], ring, self.ring_rows, pool, mi["ape"], pos,
-                                   q_pos_out=wb.qpos[:1])
+            hk.mla_decode_prologue(mi["kv_pre"], mi["ln_w"], ckv, 1e-6, mi["idx_k"], mi["knorm_w"], mi["knorm_b"],
+                                   wb.idx_kn, 1e-5, mi["idx_g"], ring, self.ring_rows, pool, mi["ape"], pos,
+                                   q_pos_out=wb.qpos)
         else:
-            hk.mla_cache_append(mi["kv_pre"][:n], mi["ln_w"], ckv, pos, n, 1e-6)
-            hk.layernorm_f16(mi["idx_k"][:n], mi["knorm_w"], mi["knorm_b"], wb.idx_kn[:n], n, 128, 1e-5)
-            hk.kpool_write(wb.idx_kn[:n], mi["idx_g"][:n], ring, self.ring_rows, pool, mi["ape"], pos, n)
+            hk.mla_cache_append(mi["kv_pre"], mi["ln_w"], ckv, pos, n, 1e-6)
+            hk.layernorm_f16(mi["idx_k"], mi["knorm_w"], mi["knorm_b"], wb.idx_kn, n, 128, 1e-5)
+            hk.kpool_write(wb.idx_kn, mi["idx_g"], ring, self.ring_rows, pool, mi["ape"], pos, n)
             t.arange(pos, pos + n, dtype=t.int32, device="cuda", out=wb.qpos[:n])
         if timed:
             self._mark("mla_append_kpool")
-        hk.q_latent(mi["q_nope"][:n], mi["kv_b"], wb.q_lat[:n], n)
+        hk.q_latent(mi["q_nope"], mi["kv_b"], wb.q_lat, n)
         if timed:
             self._mark("mla_q_latent")
         npools = (pos + n) // 4
         ktop = min(512, npools)
         if n <= 8 and self.fused and npools > 0:
             # decode rows: scores, top-k and expansion as two launches
-            sc = wb.scores.view(-1)[:n * npools].view(n, npools)
-            hk.indexer_select(mi["q_idx"][:n], pool, mi["w"][:n], wb.qpos[:n], sc, wb.topk[:n], wb.raw_idx[:n], n, npools, k=ktop)
+            hk.indexer_select(mi["q_idx"], pool, mi["w"], wb.qpos, wb.scores, wb.topk, wb.raw_idx, n, npools, k=ktop)
             blocks = ()
         else:
             blocks = range(0, n, IDX_BLOCK)
@@ -239,10 +243,10 @@ class TrunkAttention:
         need = hk.mla_partial_bytes(ns, n * 64) if ns > 1 else 0
         if need > wb.sparse_ws.numel():
             wb.sparse_ws = t.empty(need, dtype=t.uint8, device="cuda")
-        hk.mla_sparse_decode(wb.q_lat[:n], ckv, wb.raw_idx[:n], KIDX, wb.lat_out[:n], n, n_split=ns, workspace=wb.sparse_ws)
+        hk.mla_sparse_decode(wb.q_lat, ckv, wb.raw_idx, KIDX, wb.lat_out, n, n_split=ns, workspace=wb.sparse_ws)
         if timed:
             self._mark("mla_sparse_attention")
-        hk.o_absorb(wb.lat_out[:n], mi["kv_b"], wb.o_abs[:n], n)
+        hk.o_absorb(wb.lat_out, mi["kv_b"], wb.o_abs, n)
         if timed:
             self._mark("mla_o_absorb")
         if self.keep:
@@ -253,6 +257,8 @@ class TrunkAttention:
         """all layers over rows pos .. pos + n - 1 (prefill chunk, or a decode step with n = 1).  The model interleaves
         the two kinds (three KDA layers, then one MLA layer); with synthetic inputs the order inside a chunk does not
         change any result, so the layers run kind by kind."""
+        if n > self.max_chunk or pos + n > self.cap:
+            raise ValueError("rows %d .. %d: the trunk holds %d rows per chunk and %d positions" % (pos, pos + n - 1, self.max_chunk, self.cap))
         if timed:
             self._mark("begin")
         for L in range(self.n_kda):
