@@ -183,6 +183,102 @@ __global__ __launch_bounds__(AB_THREADS, 1) void absorb_gemm_tc_kernel(
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
 }
 
+// ------------------------------------------------------------------------------------------------
+// A few rows (decode, at most 32): the 16.8 MB of weights are all there is to move.  The kernel above gives such a call 128
+// (q) or 64 (o) CTAs of 128-row tiles whose two-stage ring has at most 96 KB in flight, on 64 SMs for o: 7.8 and 10.5 us.
+// Here the WEIGHTS are the M operand, 64 output columns per CTA (512 and 256 CTAs, all resident), the rows are N (8 to 32),
+// and a CTA requests its whole K at once (32 / 64 KB, a barrier per 64-channel chunk): no ring, no empty barriers.
+// As a programmatic dependent it pulls its weights into L2 while the kernel before it still runs.
+// ------------------------------------------------------------------------------------------------
+constexpr int AF_BM = 64, AF_BK = 64, AF_MAX_ROWS = 32, AF_THREADS = 128;
+constexpr uint32_t AF_A_CHUNK = AF_BM * AF_BK * 2;            // 8 KB
+
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* tmap, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(tmap)),
+               "r"(x), "r"(y)
+               : "memory");
+}
+
+// W_MN: weights [k][n] with n contiguous, else [n][k].  nb = rows rounded up to 8 (box rows of tmap_x).
+template <bool W_MN, int K>
+__global__ __launch_bounds__(AF_THREADS) void absorb_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_w,
+                                                                     const __grid_constant__ CUtensorMap tmap_x,
+                                                                     __half* __restrict__ out, int n_rows, int nb, int n_out,
+                                                                     int w_rows_per_head, int w_row_off, int* __restrict__ status) {
+  constexpr int NK = K / AF_BK;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* sW = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* sX = sW + NK * AF_A_CHUNK;
+  __shared__ uint64_t full_bar[NK], done_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = tc::warp_index_uniform();
+  const int n0 = blockIdx.x * AF_BM, h = blockIdx.y;
+  const uint32_t x_chunk = (uint32_t)nb * AF_BK * 2;
+  pdl_trigger();
+  const int wy = h * w_rows_per_head + w_row_off + (W_MN ? 0 : n0);
+  if (tid == 0) {
+    for (int kc = 0; kc < NK; kc++) {
+      tma_prefetch_2d(&tmap_w, W_MN ? n0 : kc * AF_BK, wy + (W_MN ? kc * AF_BK : 0));
+      tc::mbar_init(&full_bar[kc], 1);
+    }
+    tc::mbar_init(&done_bar, 1);
+    tc::mbar_fence_init();
+    abort_flag = 0;
+    pdl_wait();
+    for (int kc = 0; kc < NK; kc++) {
+      tc::mbar_arrive_expect_tx(&full_bar[kc], AF_A_CHUNK + x_chunk);
+      tma_load_2d(sW + kc * AF_A_CHUNK, &tmap_w, W_MN ? n0 : kc * AF_BK, wy + (W_MN ? kc * AF_BK : 0), &full_bar[kc]);
+      tma_load_2d(sX + kc * x_chunk, &tmap_x, h * K + kc * AF_BK, 0, &full_bar[kc]);
+    }
+  }
+  if (warp == 1) tc::tmem_alloc(&tmem_slot, 32);
+  pdl_wait();
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_slot;
+  if (warp == 1) {
+    // whole warp, one elected lane issues (tc05.cuh): M64 products leave every ~24 cycles
+    const uint32_t leader = tc::elect_one();
+    const uint32_t idesc = tc::make_idesc(AF_BM, nb, tc::FMT_F16, tc::FMT_F16, W_MN, false);
+#pragma unroll 1
+    for (int kc = 0; kc < NK; kc++) {
+      const bool landed = tc::mbar_wait(&full_bar[kc], 0, &abort_flag, 1);
+      if (!__all_sync(0xffffffffu, landed)) break;
+      tc::fence_after_sync();
+      const uint32_t w_addr = tc::smem_u32(sW + kc * AF_A_CHUNK), x_addr = tc::smem_u32(sX + kc * x_chunk);
+#pragma unroll
+      for (int k16 = 0; k16 < AF_BK / 16; k16++)
+        tc::mma_f16_if(leader, tmem, tc::make_sdesc_sw128(w_addr + k16 * (W_MN ? 2048 : 32), W_MN ? 8192 : 16, 1024),
+                       tc::make_sdesc_sw128(x_addr + k16 * 32, 16, 1024), idesc, kc > 0 || k16 > 0);
+    }
+    tc::mma_commit_if(leader, &done_bar);
+  }
+  const bool ok = tc::mbar_wait(&done_bar, 0, &abort_flag, 2);
+  tc::fence_after_sync();
+  // output column 16 w + i sits in TMEM lane 32 w + i, i < 16
+  if (__all_sync(0xffffffffu, ok)) {
+#pragma unroll 1
+    for (int c0 = 0; c0 < nb; c0 += 16) {
+      uint32_t v[16];
+      tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0, v);
+      tc::tmem_ld_wait();
+      if (lane < 16) {
+        __half* o = out + ((size_t)c0 * 64 + h) * n_out + n0 + warp * 16 + lane;
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+          if (c0 + j < n_rows) o[(size_t)j * 64 * n_out] = __float2half_rn(__uint_as_float(v[j]));
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) tc::tmem_dealloc(tmem, 32);
+  if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -214,11 +310,41 @@ static bool make_map_2d(CUtensorMap* m, const void* base, uint64_t rows, uint64_
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <bool W_MN, int K>
+static int absorb_few_rows(const void* x, const void* w, void* out, int n_rows, int n_out, uint64_t w_rows, uint64_t w_cols,
+                           int w_rows_per_head, int w_row_off, cudaStream_t s) {
+  const int nb = (n_rows + 7) & ~7;
+  alignas(64) CUtensorMap mw, mx;
+  memset(&mw, 0, sizeof(mw));
+  memset(&mx, 0, sizeof(mx));
+  if (!make_map_2d(&mw, w, w_rows, w_cols, AF_BM, AF_BK) || !make_map_2d(&mx, x, (uint64_t)n_rows, (uint64_t)64 * K, nb, AF_BK))
+    return HK_ERR_UNSUPPORTED;
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    const int most = K / AF_BK * (AF_A_CHUNK + AF_MAX_ROWS * AF_BK * 2) + 1024;
+    if (cudaFuncSetAttribute(absorb_few_rows_kernel<W_MN, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
+      return HK_ERR_CUDA;
+    attr_set[dev] = true;
+  }
+  const size_t smem = (size_t)(K / AF_BK) * (AF_A_CHUNK + nb * AF_BK * 2) + 1024;
+  return pdl_launch(absorb_few_rows_kernel<W_MN, K>, dim3(n_out / AF_BM, 64), dim3(AF_THREADS), smem, s, mw, mx, (__half*)out, n_rows,
+                    nb, n_out, w_rows_per_head, w_row_off, device_status_ptr()) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
+}
+
 // a [n_rows][64*K], weights as described above, out [n_rows][64*n_out]; returns HK_ERR_UNSUPPORTED when the
 // tensor maps cannot be built (the caller then uses the CUDA-core kernels)
 int absorb_gemm_tc(const void* a, const void* b, void* out, int n_rows, int K, int n_out, bool b_mn,
                    uint64_t b_rows, uint64_t b_cols, int b_rows_per_head, int b_row_off, cudaStream_t s) {
   if (!aligned(a, 16) || !aligned(b, 16) || !aligned(out, 16)) return HK_ERR_UNSUPPORTED;
+  if (n_rows <= AF_MAX_ROWS) {   // q_latent (K 256, n contiguous), o_absorb (K 512, k contiguous), o_absorb_t (K 512, n contiguous)
+    if (K == 256 && b_mn) return absorb_few_rows<true, 256>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
+    if (K == 512 && !b_mn) return absorb_few_rows<false, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
+    if (K == 512 && b_mn) return absorb_few_rows<true, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
+  }
   alignas(64) CUtensorMap ma, mb;
   memset(&ma, 0, sizeof(ma));
   memset(&mb, 0, sizeof(mb));

@@ -52,21 +52,28 @@ __device__ __forceinline__ int block_exscan(int v, int* scratch, int* total) {
   return scratch[warp] + incl - v;
 }
 
-// load 8 consecutive keys starting at element i8*8 (VEC: one 16-byte load), invalid ones as 0
-template <bool VEC>
-__device__ __forceinline__ void load8(const uint16_t* row, int i8, int T, uint32_t (&key)[8]) {
-  const int base = i8 * 8;
-  if (VEC && base + 8 <= T) {
-    uint4 v = *reinterpret_cast<const uint4*>(row + base);
-    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+// Rows are read as aligned 16-byte pieces whatever the row's start: piece i8 of a row that starts `lead` elements behind a
+// 16-byte boundary holds elements 8 i8 - lead .. 8 i8 - lead + 7.  (Score rows follow one another with the caller's stride, the
+// pool count, so seven of eight contexts have rows off the boundary; one 2-byte load per score made those sweeps 2-4 times
+// longer.)  Pieces that reach over an end of the row are read element by element; what lies outside is key 0, never selected.
+__device__ __forceinline__ int row_lead(const uint16_t* row) { return (int)((reinterpret_cast<uintptr_t>(row) & 15) >> 1); }
+__device__ __forceinline__ uint4 load8_raw(const uint16_t* row, int lead, int i8, int T) {
+  const int base = i8 * 8 - lead;
+  if (base >= 0 && base + 8 <= T) return *reinterpret_cast<const uint4*>(row + base);
+  uint32_t w[4] = {0, 0, 0, 0};   // 0xffff = key 0
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      key[2 * j] = topk_key(w[j] & 0xffffu);
-      key[2 * j + 1] = topk_key(w[j] >> 16);
-    }
-  } else {
+  for (int j = 0; j < 8; j++) {
+    const uint32_t u = base + j >= 0 && base + j < T ? row[base + j] : 0xffffu;
+    w[j >> 1] |= u << (16 * (j & 1));
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void keys8(uint4 v, uint32_t (&key)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int j = 0; j < 8; j++) key[j] = (base + j < T) ? topk_key(row[base + j]) : 0u;
+  for (int j = 0; j < 4; j++) {
+    key[2 * j] = topk_key(w[j] & 0xffffu);
+    key[2 * j + 1] = topk_key(w[j] >> 16);
   }
 }
 
@@ -94,10 +101,9 @@ struct TopkSink {
 };
 
 // One row by one CTA of TK_THREADS threads; `row` and the sink's index row may point to global or shared memory.
-template <bool VEC>
 __device__ __forceinline__ void topk_row(const uint16_t* row, const TopkSink row_o, int T, int k, int k_pad) {
   const int t = threadIdx.x;
-  const int n_slots = (T + 7) >> 3;
+  const int lead = row_lead(row), n_slots = (T + lead + 7) >> 3;
 
   __shared__ int hist[2048];
   __shared__ int scan_ws[TK_WARPS + 1];
@@ -108,7 +114,7 @@ __device__ __forceinline__ void topk_row(const uint16_t* row, const TopkSink row
   __syncthreads();
   for (int i8 = t; i8 < n_slots; i8 += TK_THREADS) {
     uint32_t key[8];
-    load8<VEC>(row, i8, T, key);
+    keys8(load8_raw(row, lead, i8, T), key);
 #pragma unroll
     for (int j = 0; j < 8; j++)
       if (key[j] > KEY_NEG_INF) atomicAdd(&hist[key[j] >> 5], 1);
@@ -141,7 +147,7 @@ __device__ __forceinline__ void topk_row(const uint16_t* row, const TopkSink row
     __syncthreads();
     for (int i8 = t; i8 < n_slots; i8 += TK_THREADS) {
       uint32_t key[8];
-      load8<VEC>(row, i8, T, key);
+      keys8(load8_raw(row, lead, i8, T), key);
 #pragma unroll
       for (int j = 0; j < 8; j++)
         if ((int)(key[j] >> 5) == b1) atomicAdd(&hist[key[j] & 31u], 1);
@@ -174,7 +180,7 @@ __device__ __forceinline__ void topk_row(const uint16_t* row, const TopkSink row
     uint32_t m_gt = 0, m_eq = 0;
     if (i8 < n_slots) {
       uint32_t key[8];
-      load8<VEC>(row, i8, T, key);
+      keys8(load8_raw(row, lead, i8, T), key);
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         if (key[j] > thresh && key[j] > KEY_NEG_INF) m_gt |= 1u << j;
@@ -186,7 +192,7 @@ __device__ __forceinline__ void topk_row(const uint16_t* row, const TopkSink row
     const int ex = block_exscan(packed, scan_ws, &tot);
     int o_gt = base_gt + (ex & 0xffff);
     int o_eq = base_eq + (ex >> 16);
-    const int ibase = i8 * 8;
+    const int ibase = i8 * 8 - lead;
     while (m_gt) {
       const int j = __ffs((int)m_gt) - 1;
       m_gt &= m_gt - 1;
@@ -207,28 +213,28 @@ __device__ __forceinline__ void topk_row(const uint16_t* row, const TopkSink row
 }
 
 // raw != nullptr: the expanded token rows [R][4 k_pad + 4] are written as well, row r clipped at q_pos[r]
-template <bool VEC>
 __global__ __launch_bounds__(TK_THREADS) void dsa_topk_kernel(
     const uint16_t* scores, int* __restrict__ out, int T, int s_stride, int k,
     int k_pad, const int* __restrict__ t_ptr, int t_seq, int* __restrict__ raw, const int* __restrict__ q_pos) {
-  // behind a kernel that allowed its dependents to start early (the scorer): wait for its scores
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
   if (t_ptr) T = t_seq > 0 ? t_ptr[blockIdx.x / t_seq] : *t_ptr;
   TopkSink sink{out + (size_t)blockIdx.x * k_pad,
                 raw ? reinterpret_cast<int4*>(raw + (size_t)blockIdx.x * (4 * k_pad + 4)) : nullptr,
                 raw ? q_pos[blockIdx.x] : 0};
-  topk_row<VEC>(scores + (size_t)blockIdx.x * s_stride, sink, T, k, k_pad);
+  topk_row(scores + (size_t)blockIdx.x * s_stride, sink, T, k, k_pad);
 }
 
 
 // ------------------------------------------------------------------------------------------------
-// Rows of at most 65,536 scores (the decode case is ONE such row): a thread-block cluster of 8 CTAs
-// works on a row, CTA c on elements [8192 c, 8192 (c+1)), every thread on 8 consecutive elements that
-// stay in registers, so the row is read from global memory once and no sweep is longer than 8 keys
-// per thread.  The CTAs meet through distributed shared memory: the bucket histograms are summed
-// slice-wise and the sums stored into every CTA, each CTA then finds the crossing bucket itself; the
-// low-bit count sets are read by every CTA, which finds the threshold and, from the per-CTA counts, the
+// A few long rows (the decode case is ONE row): a thread-block cluster of 8 CTAs works on a row, CTA c on pieces
+// [1024 NP c, 1024 NP (c + 1)), every thread on NP consecutive pieces of 8 elements that stay in registers, so the row is
+// read from global memory once and no sweep is longer than 8 NP keys per thread.  The CTAs meet through distributed shared
+// memory: the bucket histograms are summed slice-wise and the sums stored into every CTA, each CTA then finds the crossing
+// bucket itself; the low-bit count sets are read by every CTA, which finds the threshold and, from the per-CTA counts, the
 // offset of its own ordered output - four cluster barriers in all, no hand-back round trips.
+// NP = 1, 2, 4 cover rows of 65,535, 131,071 and 262,143 scores at any alignment (1M tokens of context).  One row of 65,540
+// scores (262,160 tokens) took 33.9 us in the one-CTA kernel and takes 9.3 us here.
 // ------------------------------------------------------------------------------------------------
 #ifdef HK_TOPK_TRACE
 __device__ long long hk_topk_trace[16];
@@ -237,14 +243,28 @@ __device__ long long hk_topk_trace[16];
 #define TK_TRACE(slot) do { } while (0)
 #endif
 constexpr int TKC_CTAS = 8;
-constexpr int TKC_MAX_T = TKC_CTAS * TK_THREADS * 8;      // 65536
+constexpr int TKC_PIECES = TKC_CTAS * TK_THREADS;         // pieces of 8 elements that NP = 1 holds
+constexpr int TKC_MAX_NP = 4;
 
-template <bool VEC>
+// f(j, key) over the 8 NP keys of a thread's pieces, j ascending with the element index
+template <int NP, class F>
+__device__ __forceinline__ void for_keys(const uint4 (&pc)[NP], F f) {
+#pragma unroll
+  for (int u = 0; u < NP; u++) {
+    uint32_t key[8];
+    keys8(pc[u], key);
+#pragma unroll
+    for (int j = 0; j < 8; j++) f(8 * u + j, key[j]);
+  }
+}
+
+template <int NP>
 __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void dsa_topk_cluster_kernel(
     const uint16_t* scores, int* __restrict__ out, int T, int s_stride, int k, int k_pad,
     int* __restrict__ raw, const int* __restrict__ q_pos) {
   namespace cg = cooperative_groups;
-  asm volatile("griddepcontrol.wait;" ::: "memory");   // see dsa_topk_kernel
+  pdl_trigger();
+  pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int c = (int)cluster.block_rank();
   const int row_id = blockIdx.x / TKC_CTAS;
@@ -261,15 +281,16 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
   __shared__ int sh_off[6];        // threshold low bits, count above threshold, this CTA's bases, total ties
 
   TK_TRACE(0);
-  uint32_t key[8];
-  const int i8 = c * TK_THREADS + t;
-  load8<VEC>(row, i8, T, key);     // beyond T: key 0, never selectable
+  const int lead = row_lead(row), i8 = (c * TK_THREADS + t) * NP;
+  uint4 pc[NP];
+#pragma unroll
+  for (int u = 0; u < NP; u++) pc[u] = load8_raw(row, lead, i8 + u, T);
   for (int i = t; i < 2048; i += TK_THREADS) hist[i] = 0;
   if (t < 33) low[t] = 0;
   __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 8; j++)
-    if (key[j] > KEY_NEG_INF) atomicAdd(&hist[key[j] >> 5], 1);
+  for_keys<NP>(pc, [&](int, uint32_t key) {
+    if (key > KEY_NEG_INF) atomicAdd(&hist[key >> 5], 1);
+  });
   cluster.sync();                  // (1) all local histograms complete
   TK_TRACE(1);
   // slice c of the buckets is summed over the eight CTAs by CTA c and stored into EVERY CTA's copy of
@@ -300,12 +321,11 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
   // (fewer than k selectable entries, or k == 0) every selectable key counts as "above".
   const int b_eff = b1 < 0 ? 31 : b1;
   int n_above = 0;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const int bk = (int)(key[j] >> 5);
-    if (bk == b1) atomicAdd(&low[key[j] & 31u], 1);
+  for_keys<NP>(pc, [&](int, uint32_t key) {
+    const int bk = (int)(key >> 5);
+    if (bk == b1) atomicAdd(&low[key & 31u], 1);
     n_above += bk > b_eff;
-  }
+  });
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) n_above += __shfl_xor_sync(0xffffffffu, n_above, o);
   if (lane == 0 && n_above) atomicAdd(&low[32], n_above);
@@ -364,17 +384,16 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
   TK_TRACE(4);
   // ---- ordered compaction inside the CTA, offset by the counts of the CTAs before it ----
   uint32_t m_gt = 0, m_eq = 0;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    if (key[j] > thresh && key[j] > KEY_NEG_INF) m_gt |= 1u << j;
-    if (key[j] == thresh && n_eq_take > 0) m_eq |= 1u << j;
-  }
+  for_keys<NP>(pc, [&](int j, uint32_t key) {
+    if (key > thresh && key > KEY_NEG_INF) m_gt |= 1u << j;
+    if (key == thresh && n_eq_take > 0) m_eq |= 1u << j;
+  });
   int tot;
   const int ex = block_exscan(__popc(m_gt) | (__popc(m_eq) << 16), scan_ws, &tot);
   TK_TRACE(5);
   int o_gt = sh_off[2] + (ex & 0xffff);
   int o_eq = sh_off[3] + (ex >> 16);
-  const int ibase = i8 * 8;
+  const int ibase = i8 * 8 - lead;
   while (m_gt) {
     const int j = __ffs((int)m_gt) - 1;
     m_gt &= m_gt - 1;
@@ -404,33 +423,23 @@ extern "C" __attribute__((visibility("default"))) int hk_debug_topk_trace(long l
 #endif
 
 namespace hk {
-// common launcher; raw != nullptr adds the expansion, pdl launches the kernel as a programmatic dependent of the
-// kernel before it in the stream (which must have released its dependents: the decode scorer does)
+// common launcher; raw != nullptr adds the expansion
 static int topk_launch(const void* scores, int s_stride, int* indices, int R, int T, int k, int k_pad, const int* t_ptr,
-                       int t_seq, int* raw, const int* q_pos, bool pdl, cudaStream_t s) {
-  const bool vec = (s_stride % 8 == 0) && aligned(scores, 16);
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(TK_THREADS);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+                       int t_seq, int* raw, const int* q_pos, cudaStream_t s) {
   const uint16_t* sc = (const uint16_t*)scores;
   cudaError_t e;
-  if (T > 16384 && T <= TKC_MAX_T && R <= 16 && !t_ptr) {
+  // pieces of the longest-reaching row: rows of a stride that is no multiple of 8 start at any offset
+  const int lead = R == 1 || s_stride % 8 == 0 ? (int)(((uintptr_t)scores & 15) >> 1) : 7;
+  const int64_t pieces = ((int64_t)T + lead + 7) / 8;
+  if (T > 16384 && pieces <= (int64_t)TKC_PIECES * TKC_MAX_NP && R <= 16 && !t_ptr) {
     // a few long rows (decode): one 8-CTA cluster per row.  With many rows (prefill) the clusters queue for
     // eight free SMs of one GPC each and the one-CTA kernel below is 3 to 20 times faster (measured at
     // 64 to 4,096 rows); up to 16,384 scores one CTA is as fast as the cluster even for a single row.
-    cfg.gridDim = dim3(R * TKC_CTAS);
-    e = vec ? cudaLaunchKernelEx(&cfg, dsa_topk_cluster_kernel<true>, sc, indices, T, s_stride, k, k_pad, raw, q_pos)
-            : cudaLaunchKernelEx(&cfg, dsa_topk_cluster_kernel<false>, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
+    auto kern = pieces <= TKC_PIECES ? dsa_topk_cluster_kernel<1>
+                                     : (pieces <= 2 * TKC_PIECES ? dsa_topk_cluster_kernel<2> : dsa_topk_cluster_kernel<4>);
+    e = pdl_launch(kern, dim3(R * TKC_CTAS), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
   } else {
-    cfg.gridDim = dim3(R);
-    e = vec ? cudaLaunchKernelEx(&cfg, dsa_topk_kernel<true>, sc, indices, T, s_stride, k, k_pad, t_ptr, t_seq, raw, q_pos)
-            : cudaLaunchKernelEx(&cfg, dsa_topk_kernel<false>, sc, indices, T, s_stride, k, k_pad, t_ptr, t_seq, raw, q_pos);
+    e = pdl_launch(dsa_topk_kernel, dim3(R), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, t_ptr, t_seq, raw, q_pos);
   }
   return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
@@ -442,7 +451,7 @@ HK_API int hk_dsa_topk(const void* scores, int s_stride, int* indices, int R, in
   HK_REQUIRE(scores && indices && R >= 0 && T >= 0 && k >= 0 && k <= k_pad && s_stride >= 0);
   HK_REQUIRE(k <= 32767);  // packed 16-bit counters in the compaction scan
   if (R == 0) return HK_OK;
-  return topk_launch(scores, s_stride, indices, R, T, k, k_pad, t_ptr, t_seq, nullptr, nullptr, false, as_stream(stream));
+  return topk_launch(scores, s_stride, indices, R, T, k, k_pad, t_ptr, t_seq, nullptr, nullptr, as_stream(stream));
 }
 
 HK_API int hk_dsa_topk_expand(const void* scores, int s_stride, int* indices, int* raw_idx, const int* q_pos, int R, int T,
@@ -450,8 +459,9 @@ HK_API int hk_dsa_topk_expand(const void* scores, int s_stride, int* indices, in
   using namespace hk;
   HK_REQUIRE(scores && indices && raw_idx && q_pos && R >= 0 && T >= 0 && k >= 0 && k <= 512 && s_stride >= 0);
   HK_REQUIRE(aligned(raw_idx, 16));
+  (void)after_scorer;   // every selection kernel is launched as a programmatic dependent now
   if (R == 0) return HK_OK;
-  return topk_launch(scores, s_stride, indices, R, T, k, 512, nullptr, 0, raw_idx, q_pos, after_scorer != 0, as_stream(stream));
+  return topk_launch(scores, s_stride, indices, R, T, k, 512, nullptr, 0, raw_idx, q_pos, as_stream(stream));
 }
 
 #include "dsa_select_splitkv.cuh"

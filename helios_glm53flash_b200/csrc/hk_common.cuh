@@ -6,6 +6,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 
 #include "../../include/helios_b200.h"
 
@@ -46,6 +47,32 @@ inline int sm_count() {
     cached[dev] = n > 0 ? n : 148;
   }
   return cached[dev];
+}
+
+// ---- programmatic dependent launch ----
+// The small kernels of a decode step take 2-10 us each, of which 1-2 us are the drain of one grid and the start of the
+// next.  They are launched with programmatic stream serialisation: a kernel calls pdl_trigger() at entry, so that the next
+// one's CTAs are placed while it runs, and pdl_wait() before its first access to memory that an earlier kernel may have
+// written (or may still read).  EVERY kernel launched this way executes pdl_wait() in every CTA: the wait covers the grid
+// before it only, and the chain of waits is what orders a kernel behind all earlier ones.  Ahead of the wait a kernel may set
+// up barriers and tensor memory and prefetch into L2, which stays coherent; it may not load or store anything.
+// Behind a kernel that never triggers the attribute changes nothing.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 // device word (per device) where kernels record that a bounded wait gave up; see hk_read_device_status

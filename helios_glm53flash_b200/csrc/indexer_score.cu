@@ -165,9 +165,7 @@ __global__ __launch_bounds__(128) void indexer_tc_decode_kernel(
   __shared__ int abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = lane >> 4, chunk = lane & 15;    // a warp instruction covers 2 rows x 16 chunks
-  // a selection kernel launched as this grid's programmatic dependent may be placed now; it waits for this grid's
-  // completion itself before it reads a score
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_trigger();
 
   if (tid == 0) {
     tc::mbar_init(&bar, 1);
@@ -175,6 +173,12 @@ __global__ __launch_bounds__(128) void indexer_tc_decode_kernel(
     abort_flag = 0;
   }
   if (warp == 0) tc::tmem_alloc(&tmem_slot, tmem_cols);
+  // this CTA's first key tile on its way into L2 while the kernel before this one finishes
+  if (tid == 0) {
+    const int p0 = blockIdx.x * IX_TILE_P;
+    tc::prefetch_l2(pk + (size_t)p0 * IDX_DIM, (uint32_t)min(IX_TILE_P, npools - p0) * IDX_DIM * 2);
+  }
+  pdl_wait();
   // query rows -> B operand
   for (int r2 = warp; r2 < nb / 2; r2 += 4) {
     const int row = r2 * 2 + sub;
@@ -333,10 +337,10 @@ HK_API int hk_indexer_score(const void* q_idx, const void* pool_k_nt, const void
     if (grid_x > tiles) grid_x = tiles;
     cudaStream_t sd = as_stream(stream);
     int* std_ = device_status_ptr();
-    if (dtype == HK_F16)
-      indexer_tc_decode_kernel<0><<<grid_x, 128, smem, sd>>>((const uint16_t*)q_idx, (const uint16_t*)pool_k_nt, (const uint16_t*)w, q_pos, (__half*)scores, m, npools, score_stride, tiles, cols, std_);
-    else
-      indexer_tc_decode_kernel<1><<<grid_x, 128, smem, sd>>>((const uint16_t*)q_idx, (const uint16_t*)pool_k_nt, (const uint16_t*)w, q_pos, (__half*)scores, m, npools, score_stride, tiles, cols, std_);
+    auto kern = dtype == HK_F16 ? indexer_tc_decode_kernel<0> : indexer_tc_decode_kernel<1>;
+    if (pdl_launch(kern, dim3(grid_x), dim3(128), smem, sd, (const uint16_t*)q_idx, (const uint16_t*)pool_k_nt, (const uint16_t*)w,
+                   q_pos, (__half*)scores, m, npools, score_stride, tiles, cols, std_) != cudaSuccess)
+      return HK_ERR_CUDA;
     HK_LAUNCH_CHECK();
     return HK_OK;
   }

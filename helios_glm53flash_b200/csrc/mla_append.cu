@@ -120,6 +120,8 @@ __global__ void __launch_bounds__(128) mla_decode_prologue_kernel(
     __half* __restrict__ pk_nt, const float* __restrict__ ape, int pos, int* __restrict__ q_pos_out) {
   __shared__ __half s_kn[128];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_trigger();
+  pdl_wait();
   if (warp == 0) append_row(kv_pre, ln_w, ckv + (size_t)pos * LATENT, nullptr, eps_rms, lane);
   if (warp == 1) layernorm_row(idx_k, knorm_w, knorm_b, idx_kn, s_kn, 128, eps_ln, lane);
   if (threadIdx.x == 64 && q_pos_out) *q_pos_out = pos;
@@ -161,11 +163,12 @@ HK_API int hk_mla_decode_prologue(const float* kv_pre, const void* ln_w_f16, voi
   HK_REQUIRE(kv_pre && ln_w_f16 && ckv && idx_k && knorm_w && knorm_b && idx_g && raw_ring && pool_k_nt && ape);
   HK_REQUIRE(pos >= 0 && raw_rows > 0 && (raw_rows >= hk::POOL || raw_rows >= pos + 1));
   HK_REQUIRE(hk::aligned(kv_pre, 16) && hk::aligned(ln_w_f16, 8) && hk::aligned(ckv, 8));
-  hk::mla_decode_prologue_kernel<<<1, 128, 0, hk::as_stream(stream)>>>(
-      kv_pre, static_cast<const __half*>(ln_w_f16), static_cast<__half*>(ckv), eps_rms, static_cast<const __half*>(idx_k),
-      static_cast<const __half*>(knorm_w), static_cast<const __half*>(knorm_b), static_cast<__half*>(idx_kn), eps_ln,
-      static_cast<const __half*>(idx_g), static_cast<__half*>(raw_ring), raw_rows, static_cast<__half*>(pool_k_nt), ape, pos,
-      q_pos_out);
+  if (hk::pdl_launch(hk::mla_decode_prologue_kernel, dim3(1), dim3(128), 0, hk::as_stream(stream), kv_pre,
+                     static_cast<const __half*>(ln_w_f16), static_cast<__half*>(ckv), eps_rms, static_cast<const __half*>(idx_k),
+                     static_cast<const __half*>(knorm_w), static_cast<const __half*>(knorm_b), static_cast<__half*>(idx_kn), eps_ln,
+                     static_cast<const __half*>(idx_g), static_cast<__half*>(raw_ring), raw_rows, static_cast<__half*>(pool_k_nt),
+                     ape, pos, q_pos_out) != cudaSuccess)
+    return HK_ERR_CUDA;
   HK_LAUNCH_CHECK();
   return HK_OK;
 }

@@ -63,27 +63,12 @@ static int launch_simt(const MlaArgs& a, cudaStream_t s) {
   return cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 
-// Launched with programmatic stream serialisation: the flash kernel releases its dependents at entry, so the
-// combine's CTAs are placed while the partial kernel still runs and block in griddepcontrol.wait (first statement
-// of lse_combine_kernel) until that grid has completed and its writes are visible; the launch latency of the
-// second kernel disappears from every decode step.  Behind any other kernel the attribute only delays the start
-// until that kernel has finished, as a plain launch would.
 template <int GROUPS>
 static int combine_launch(const float* pm, const float* pl, const float* pa, int n_split, int64_t rows, __half* out,
                           cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)rows);
-  cfg.blockDim = dim3(128 * GROUPS);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const float* const* none = nullptr;
-  return cudaLaunchKernelEx(&cfg, lse_combine_kernel<false, GROUPS>, pm, pl, pa, none, none, none, n_split, rows, out) ==
-                 cudaSuccess
+  return pdl_launch(lse_combine_kernel<false, GROUPS>, dim3((unsigned)rows), dim3(128 * GROUPS), 0, s, pm, pl, pa, none, none, none,
+                    n_split, rows, out) == cudaSuccess
              ? HK_OK
              : HK_ERR_CUDA;
 }
@@ -91,18 +76,10 @@ static int combine_launch(const float* pm, const float* pl, const float* pa, int
 template <int GROUPS>
 static int combine_cs_launch(const float* pm, const float* pl, const float* pa, int n_split, int64_t rows, __half* out,
                              cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)rows, LSE_CSPLIT);
-  cfg.blockDim = dim3(32 * GROUPS);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, lse_combine_cs_kernel<GROUPS>, pm, pl, pa, n_split, rows, out) == cudaSuccess ? HK_OK
-                                                                                                                 : HK_ERR_CUDA;
+  return pdl_launch(lse_combine_cs_kernel<GROUPS>, dim3((unsigned)rows, LSE_CSPLIT), dim3(32 * GROUPS), 0, s, pm, pl, pa, n_split,
+                    rows, out) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 static int combine(const float* pm, const float* pl, const float* pa, int n_split, int64_t rows,

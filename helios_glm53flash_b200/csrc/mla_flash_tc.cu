@@ -143,9 +143,8 @@ __global__ __launch_bounds__(G4 ? FT_G4_THREADS : FT_THREADS, 1) void mla_flash_
   const int warp_u = tc::warp_index_uniform();
   const bool mma_warp = warp_u == 4 || warp_u == 12;   // 4 issues S = Q K^T, 12 issues O^T += V^T P^T
   const int sp = blockIdx.x, r = blockIdx.y;
-  // a kernel launched as this grid's programmatic dependent (the LSE combine) may be placed from now on; it waits
-  // for this grid's completion itself before it reads anything
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
   FT_CTA_STAMP(0);
   if (tid == 0) FT_TRACE(13, 0);                      // kernel entry
   const bool sparse = a.raw_idx != nullptr;
@@ -193,6 +192,7 @@ __global__ __launch_bounds__(G4 ? FT_G4_THREADS : FT_THREADS, 1) void mla_flash_
       }
     }
   }
+  // (not ahead of the barrier set-up and the first copies: there it cost a many-wave launch 4 %)
   if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
   if (n_tiles > 0) {
     // Q [64 heads][512] -> K-major operand tile, staged by ALL warps with every load of a thread in flight at
@@ -703,11 +703,10 @@ int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s) {
     }
   }
   dim3 grid(a.n_split, a.m);
-  if (use_tma == 2)
-    mla_flash_tc_kernel<true><<<grid, FT_G4_THREADS, FS_SMEM, s>>>(a, device_status_ptr(), tmap, use_tma);
-  else
-    mla_flash_tc_kernel<false><<<grid, FT_THREADS, FS_SMEM, s>>>(a, device_status_ptr(), tmap, use_tma);
-  return cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+  auto kern = use_tma == 2 ? mla_flash_tc_kernel<true> : mla_flash_tc_kernel<false>;
+  const cudaError_t e = pdl_launch(kern, grid, dim3(use_tma == 2 ? FT_G4_THREADS : FT_THREADS), FS_SMEM, s, a, device_status_ptr(),
+                                   tmap, use_tma);
+  return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 
 }  // namespace hk

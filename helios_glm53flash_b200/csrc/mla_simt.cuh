@@ -241,9 +241,8 @@ __global__ __launch_bounds__(128 * GROUPS) void lse_combine_kernel(
     const float* __restrict__ part_acc, const float* const* __restrict__ ptrs_m,
     const float* const* __restrict__ ptrs_l, const float* const* __restrict__ ptrs_acc,
     int n_split, int64_t rows, __half* __restrict__ out) {
-  // when launched as a programmatic dependent of the kernel that writes the partials: wait until that grid has
-  // completed and its writes are visible (a no-op after a plain launch)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
   const int64_t r = blockIdx.x;
   float gm, gl;
   float4 o;
@@ -267,7 +266,8 @@ template <int GROUPS>
 __global__ __launch_bounds__(32 * GROUPS) void lse_combine_cs_kernel(
     const float* __restrict__ part_m, const float* __restrict__ part_l, const float* __restrict__ part_acc,
     int n_split, int64_t rows, __half* __restrict__ out) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");   // see lse_combine_kernel
+  pdl_trigger();
+  pdl_wait();
   constexpr int LANES = 128 / LSE_CSPLIT;
   const int64_t r = blockIdx.x;
   const int cpart = blockIdx.y;

@@ -143,6 +143,18 @@ def test_topk_bit_exact_vs_oracle_and_reference(R, T, k, k_pad, stride_pad, offs
         assert np.array_equal(refi, want), "oracle pinned to the reference's top-k (set, order, padding)"
 
 
+@pytest.mark.parametrize("R,T,stride_pad,offset", [(1, 65529, 0, 7), (1, 65537, 0, 0), (3, 65552, 1, 5), (1, 131065, 0, 7), (2, 131080, 3, 0),
+                                                    (1, 262137, 0, 7), (1, 262145, 0, 0), (18, 16390, 1, 1), (20, 9, 0, 3)])
+def test_topk_at_the_edges_of_its_row_forms(R, T, stride_pad, offset):
+    """rows off the 16-byte boundary, and the longest row of every pieces-per-thread count of the cluster form"""
+    r = synth.rng(R + T)
+    sc = np.round(r.standard_normal((R, T + stride_pad), dtype=np.float32) * 16) / 16
+    sc[:, T - 40:T] += 3.0                                     # selected entries at the very end of a row
+    scb = synth.f32_to_f16_bits(sc)
+    got = _topk_gpu(scb, T + stride_pad, R, T, 512, 512, offset=offset)
+    assert np.array_equal(got, orc.dsa_topk(scb, T + stride_pad, R, T, 512, 512))
+
+
 def test_topk_selects_the_true_top_k():
     """independent of the oracle: the selection is a true top-k, above-threshold entries come out in
     ascending index order followed by the threshold ties in ascending index order"""

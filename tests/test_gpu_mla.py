@@ -176,6 +176,28 @@ def test_absorbed_projections_vs_oracle(m):
     assert sum_rel(f(bits(o1)), want_o) < 2e-3 and sum_rel(f(bits(o2)), want_o) < 2e-3
 
 
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 17, 32, 33])
+def test_absorbed_projections_of_few_rows(m):
+    """weights-as-M form (up to 32 rows, N = rows rounded up to 8) and the first size beyond it; rows past m stay untouched"""
+    r = synth.rng(10 + m)
+    qn = synth.f32_to_f16_bits(r.uniform(-1, 1, (m, 64, 256)).astype(np.float32))
+    kb = synth.f32_to_f16_bits((0.3 * r.uniform(-1, 1, (32768, 512))).astype(np.float32))
+    lo = synth.f32_to_f16_bits(r.uniform(-1, 1, (m, 64, 512)).astype(np.float32))
+    dq, dkb, dlo = dev_f16(qn), dev_f16(kb), dev_f16(lo)
+    ql = torch.full((m + 1, 64, 512), 7.0, dtype=torch.float16, device="cuda")
+    o1, o2 = (torch.full((m + 1, 64, 256), 7.0, dtype=torch.float16, device="cuda") for _ in range(2))
+    wt = torch.empty(64, 512, 256, dtype=torch.float16, device="cuda")
+    hk.q_latent(dq, dkb, ql, m)
+    hk.o_absorb(dlo, dkb, o1, m)
+    hk.wuv_transpose(dkb, wt)
+    hk.o_absorb_t(dlo, wt, o2, m)
+    torch.cuda.synchronize()
+    assert hk.read_device_status() == 0
+    f = synth.f16_bits_to_f32
+    for got, want in ((ql, f(orc.q_latent(qn, kb, m))), (o1, f(orc.o_absorb(lo, kb, m))), (o2, f(orc.o_absorb(lo, kb, m)))):
+        assert max_rel(f(bits(got[:m])), want) < 2e-3 and (got[m:] == 7).all()
+
+
 def test_peer_combine_on_one_gpu_and_bounded_wait_times_out_cleanly():
     """the cross-GPU combine path with every 'peer' on this GPU: flags set by hk_peer_signal release the
     wait; a slot that nothing sets makes the bounded wait expire - the kernel returns, the status word
