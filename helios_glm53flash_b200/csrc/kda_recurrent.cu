@@ -11,6 +11,7 @@
 // D = 128, NV = 32 is exactly the reference's 4 x 32 order (gdn.cu:683-705).
 #include "hk_common.cuh"
 #include "kda_norm_common.cuh"
+#include "tc05.cuh"
 
 namespace hk {
 
@@ -139,15 +140,23 @@ __global__ __launch_bounds__(128) void kda_recurrent_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------
-// Decode step with the short convolution inside: x -> conv(K = 4) + SiLU -> bf16 q|k|v -> recurrence, one launch.
-// The reference runs cuda_causal_conv1d_update and cuda_recurrent_gated_delta_rule back to back for every decoded
-// token (src/engine/runner.cpp:443-471); at 2-3 us per launch the pair is bound by launch latency, not by the 4 MB
-// of state.  Same grid as the recurrence, (batch, head, value slice): every CTA convolves the head's 128 q and 128 k
-// channels itself (from the window state as it was before the call) and the value channels of its slice; the rolling
-// window of the q / k channels is written back once, by whichever slice of the head is the LAST to have read it (a
-// ticket counter per (batch, head) in caller memory; nobody waits for anybody).  Arithmetic and rounding are those of
-// the two separate kernels, so results are bit-identical to calling them in turn.
+// Arithmetic shared by the decode kernels and the per-token kernel below (channelwise decay, D = 128): a token run through
+// either gives the same bits.  The 128 state rows of a column form 16 groups, group rg = the 4-row chunks rg and rg + 16; a group
+// sum runs over its even and its odd rows separately (the two halves of a packed fp32 pair), ascending; groups rg and rg + 8 are
+// added first, then the 8 sums as a balanced tree.  S_c = S_c d_c;
+// kv = sum k_c S_c;  u = (v - kv) * beta;  S_c = fma(k_c, u, S_c);  o = sum q_c S_c.
 // ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ float tree8(float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
+  return __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), __fadd_rn(a2, a3)), __fadd_rn(__fadd_rn(a4, a5), __fadd_rn(a6, a7)));
+}
+// 128 channels of one token in one warp, channel lane + 32 u in x[u]: 1 / |x|
+__device__ __forceinline__ float inv_norm(const float (&x)[4]) {
+  float s = 0.f;
+#pragma unroll
+  for (int u = 0; u < 4; u++) s = fmaf(x[u], x[u], s);
+  return rsqrtf(warp_sum(s) + 1e-6f);
+}
+
 // window and taps of one channel arrive as one 8-byte load each
 __device__ __forceinline__ float conv4_silu_bf16(uint2 st, uint2 w, float bias, float cur) {
   // fp32 fma chain over the window [st1, st2, st3, x], taps ascending; SiLU as a / (1 + exp(-a)); rounded to bf16
@@ -167,265 +176,597 @@ __device__ __forceinline__ uint2 conv4_rolled(uint2 st, __nv_bfloat16 cur) {
   return r;
 }
 
-template <int NV>
-__global__ __launch_bounds__(128) void kda_decode_conv_kernel(
-    const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ conv_state, const __nv_bfloat16* __restrict__ conv_w,
-    const __nv_bfloat16* __restrict__ conv_bias, const float* __restrict__ g, const __nv_bfloat16* __restrict__ beta,
-    float* __restrict__ state, __nv_bfloat16* __restrict__ out, float* __restrict__ out_f32,
-    __nv_bfloat16* __restrict__ conv_out, int H, float scale, const int* __restrict__ slots, int* __restrict__ tickets) {
-  constexpr int D = 128;
-  constexpr int KG = 128 / NV, RPT = D / KG;
-  const int b = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * NV;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j = tid % NV, kg = tid / NV;
-  const int dim = 3 * H * D;
-  const int slot = slots ? slots[b] : b;
-  float* my_state = state + ((size_t)slot * H + head) * D * D + (size_t)(kg * RPT) * D + v0 + j;
-  __shared__ float sh_q[D], sh_k[D], sh_d[D];
-  __shared__ float sh_red[2][4];
-  __shared__ float sh_part[2][KG][NV];
-  __shared__ int sh_last;
+// ---------------------------------------------------------------------------------------------
+// Decode: the short convolution and the recurrence of ONE token per sequence in one launch, and (LAYER) everything else the
+// KDA layer does with it - cast of the projected row, gate preparation in front, gated RMS norm behind.  The reference runs
+// two launches here for the step and five for the layer (src/engine/runner.cpp:433-489); every value is formed by the same
+// operations as in the separate kernels of this library, so results are bit-identical to calling them in turn.
+//
+// A CTA owns a whole head (64 KB of state): 8 warps hold the state (warp = row group, lane = 4 columns), three more prepare
+// the token (q with its norm; k with its norm and the decay; v) and one of them finishes the output.  With the head in one
+// CTA nothing crosses CTAs: the earlier form, 4 or 8 value slices per head, handed the q / k window and the head's outputs
+// over through two ticket counters, an atomic and an L2 round trip each (5.4 us per layer of 32 heads).
+//
+//   few heads: one head per CTA, state straight between global memory and registers (latency: one memory round trip,
+//     three barriers);
+//   many heads (more than 2 per SM): persistent, one CTA per SM, heads stream through shared memory as 64 KB bulk copies: two
+//     stages inwards, each asked for again as soon as its head sits in registers, and one outwards (stores straight from
+//     registers held the SM to 26 B per cycle: 49 us for 1,536 heads); the token of the next head is prepared meanwhile.
+// ---------------------------------------------------------------------------------------------
+struct DecodeArgs {
+  const void* x;                        // LAYER: fp32 projection row [dim], else bf16 [dim]
+  __nv_bfloat16* conv_state;
+  const __nv_bfloat16 *conv_w, *conv_bias;
+  const float* g;                       // LAYER: raw gate projection f, else log decay
+  const void* beta;                     // LAYER: fp32 logit, else bf16 beta
+  const float *dt_bias, *a_log;
+  float lower_bound;
+  float* state;
+  __nv_bfloat16* out;
+  float* out_f32;
+  __nv_bfloat16* conv_out;
+  const void *norm_w, *gate_out;
+  void* y;
+  int w_bf16, g_bf16, y_f16, gate_act;
+  float eps, cbias, scale;
+  int H, n_heads;                       // heads of a sequence; batch * H
+  const int* slots;
+};
 
-  float S[RPT];
-#pragma unroll
-  for (int i = 0; i < RPT; i++) S[i] = my_state[(size_t)i * D];
+struct alignas(16) DecodeToken {                    // one head's token, prepared
+  float q[128], k[128], d[128], v[128];
+  float beta;
+};
 
-  // ---- short convolution of this head's q and k channels (thread = channel) and of this slice's value channel j ----
-  const __nv_bfloat16* xb = x + (size_t)b * dim;                       // [dim][1]
-  __nv_bfloat16* cs = conv_state + (size_t)slot * dim * 4;
-  const int cq = head * D + tid, ck = (H + head) * D + tid, cv = (2 * H + head) * D + v0 + j;
-  const __nv_bfloat16 xq = xb[cq], xk = xb[ck], xv = xb[cv];
-  const uint2 sq4 = *reinterpret_cast<const uint2*>(cs + (size_t)cq * 4), wq4 = __ldg(reinterpret_cast<const uint2*>(conv_w + (size_t)cq * 4));
-  const uint2 sk4 = *reinterpret_cast<const uint2*>(cs + (size_t)ck * 4), wk4 = __ldg(reinterpret_cast<const uint2*>(conv_w + (size_t)ck * 4));
-  const uint2 sv4 = *reinterpret_cast<const uint2*>(cs + (size_t)cv * 4), wv4 = __ldg(reinterpret_cast<const uint2*>(conv_w + (size_t)cv * 4));
-  const float q = conv4_silu_bf16(sq4, wq4, conv_bias ? __bfloat162float(conv_bias[cq]) : 0.f, __bfloat162float(xq));
-  const float k = conv4_silu_bf16(sk4, wk4, conv_bias ? __bfloat162float(conv_bias[ck]) : 0.f, __bfloat162float(xk));
-  const float v = conv4_silu_bf16(sv4, wv4, conv_bias ? __bfloat162float(conv_bias[cv]) : 0.f, __bfloat162float(xv));
-  const float gv = g[((size_t)b * H + head) * D + tid];
-  const float beta_h = __bfloat162float(beta[(size_t)b * H + head]);
+constexpr int KD_STATE_WARPS = 8, KD_WARPS = 11, KD_THREADS = KD_WARPS * 32;
 
-  // ---- L2 normalisation of q and k over the D channels ----
-  float sq = warp_sum(q * q), sk = warp_sum(k * k);
-  if (lane == 0) {
-    sh_red[0][warp] = sq;
-    sh_red[1][warp] = sk;
-  }
-  __syncthreads();
-  {
-    float tq = 0.f, tk = 0.f;
+// role 0: q, 1: k and decay, 2: v; one warp each
+template <bool LAYER>
+__device__ __forceinline__ void decode_prepare(const DecodeArgs& a, DecodeToken& t, int bh, int role, int lane) {
+  const int b = bh / a.H, head = bh - b * a.H, dim = 3 * a.H * 128;
+  const int slot = a.slots ? a.slots[b] : b;
+  const int c0 = (role * a.H + head) * 128 + lane;
+  __nv_bfloat16* cs = a.conv_state + ((size_t)slot * dim + c0) * 4;
+  __nv_bfloat16 x[4];
+  uint2 st[4], w[4];
+  float bias[4], gv[4];
 #pragma unroll
-    for (int w = 0; w < 4; w++) {
-      tq += sh_red[0][w];
-      tk += sh_red[1][w];
-    }
-    sh_q[tid] = q * rsqrtf(tq + 1e-6f);
-    sh_k[tid] = k * rsqrtf(tk + 1e-6f);
-    sh_d[tid] = __expf(gv);
+  for (int u = 0; u < 4; u++) {
+    const size_t xi = (size_t)b * dim + c0 + 32 * u;
+    if (LAYER) x[u] = __float2bfloat16(reinterpret_cast<const float*>(a.x)[xi]);
+    else x[u] = reinterpret_cast<const __nv_bfloat16*>(a.x)[xi];
+    st[u] = *reinterpret_cast<const uint2*>(cs + 128 * u);
+    w[u] = *reinterpret_cast<const uint2*>(a.conv_w + (size_t)(c0 + 32 * u) * 4);
+    bias[u] = a.conv_bias ? __bfloat162float(a.conv_bias[c0 + 32 * u]) : 0.f;
+    if (role == 1) gv[u] = a.g[(size_t)bh * 128 + lane + 32 * u];
   }
-  // every thread of this CTA has read the old q / k window (first barrier): thread 0 takes a ticket now and looks at it
-  // at the end of the kernel, so the round trip of the atomic runs under the recurrence
-  int ticket = 0;
-  if (tid == 0) ticket = atomicAdd(tickets + (size_t)b * H + head, 1);
-  __syncthreads();
-  // the value window of this slice is private to the CTA: every thread has read it (barrier above)
-  if (kg == 0) {
-    *reinterpret_cast<uint2*>(cs + (size_t)cv * 4) = conv4_rolled(sv4, xv);
-    if (conv_out) conv_out[(size_t)b * dim + cv] = __float2bfloat16_rn(v);
-  }
-  float sum = 0.f;
+  float z[4];
 #pragma unroll
-  for (int i = 0; i < RPT; i++) {
-    const int c = kg * RPT + i;
-    sum = sum + sh_k[c] * sh_d[c] * S[i];
+  for (int u = 0; u < 4; u++) {
+    z[u] = conv4_silu_bf16(st[u], w[u], bias[u], __bfloat162float(x[u]));
+    *reinterpret_cast<uint2*>(cs + 128 * u) = conv4_rolled(st[u], x[u]);
+    if (!LAYER && a.conv_out) a.conv_out[(size_t)b * dim + c0 + 32 * u] = __float2bfloat16_rn(z[u]);
   }
-  sh_part[0][kg][j] = sum;
-  __syncthreads();
-  float kv = 0.f;
+  if (role == 2) {
 #pragma unroll
-  for (int p = 0; p < KG; p++) kv = __fadd_rn(kv, sh_part[0][p][j]);
-  const float vp = v - kv;
-  float o = 0.f;
-#pragma unroll
-  for (int i = 0; i < RPT; i++) {
-    const int c = kg * RPT + i;
-    const float st = S[i] * sh_d[c] + sh_k[c] * vp * beta_h;
-    S[i] = st;
-    o = o + sh_q[c] * st;
+    for (int u = 0; u < 4; u++) t.v[lane + 32 * u] = z[u];
+    if (lane == 0)
+      t.beta = LAYER ? __bfloat162float(__float2bfloat16(1.0f / (1.0f + __expf(-reinterpret_cast<const float*>(a.beta)[bh]))))
+                     : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.beta)[bh]);
+    return;
   }
-  sh_part[1][kg][j] = o;
-  __syncthreads();
-  if (kg == 0) {
-    float tot = 0.f;
+  const float r = inv_norm(z);
+  float decay = 0.f;
+  if (LAYER && role == 1) decay = __expf(a.a_log[head]);
 #pragma unroll
-    for (int p = 0; p < KG; p++) tot = __fadd_rn(tot, sh_part[1][p][j]);
-    tot *= scale;
-    const size_t oi = ((size_t)b * H + head) * D + v0 + j;
-    out[oi] = __float2bfloat16_rz(tot);
-    if (out_f32) out_f32[oi] = tot;
-  }
-#pragma unroll
-  for (int i = 0; i < RPT; i++) my_state[(size_t)i * D] = S[i];
-  // The slice that drew the last ticket knows that every slice of the head has read the q / k window: it rolls the
-  // window and leaves the counter at zero for the next call.
-  if (tid == 0) {
-    const int last = ticket == (int)gridDim.z - 1;
-    if (last) tickets[(size_t)b * H + head] = 0;
-    sh_last = last;
-  }
-  __syncthreads();
-  if (sh_last) {
-    *reinterpret_cast<uint2*>(cs + (size_t)cq * 4) = conv4_rolled(sq4, xq);
-    *reinterpret_cast<uint2*>(cs + (size_t)ck * 4) = conv4_rolled(sk4, xk);
-    if (conv_out) {
-      conv_out[(size_t)b * dim + cq] = __float2bfloat16_rn(q);
-      conv_out[(size_t)b * dim + ck] = __float2bfloat16_rn(k);
+  for (int u = 0; u < 4; u++) {
+    const int c = lane + 32 * u;
+    const float n = __fmul_rn(z[u], r);
+    if (role == 0) {
+      t.q[c] = n;
+    } else {
+      const float gl = LAYER ? gate_value(gv[u], a.dt_bias[head * 128 + c], decay, a.lower_bound) : gv[u];
+      t.k[c] = n;
+      t.d[c] = __expf(gl);
     }
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// The whole KDA layer of a decoded token in ONE launch: cast of the projected q|k|v row, gate preparation, short
-// convolution, recurrence, gated RMS norm.  The reference's decode runs kda_transpose_cast, kda_gate,
-// cuda_causal_conv1d_update, cuda_recurrent_gated_delta_rule and gated_rms_norm here (src/engine/runner.cpp:433-489);
-// at 2-3 us per launch, over 34 layers, the launches are most of a decode step.  Same grid and arithmetic as
-// kda_decode_conv_kernel with, in front, x = bf16(x32) and g = gate_value(f), beta = bf16(sigmoid(b)) computed in
-// place, and behind it the norm of the head's 128 outputs, done by whichever value slice of the head is the LAST to
-// have written its outputs (second ticket counter; it reads the other slices' bf16 outputs from L2).  Every value is
-// formed by the same operations as in the separate kernels: results are bit-identical to the five-call sequence.
-// ---------------------------------------------------------------------------------------------
-template <int NV>
-__global__ __launch_bounds__(128) void kda_decode_layer_kernel(
-    const float* __restrict__ x32, __nv_bfloat16* __restrict__ conv_state, const __nv_bfloat16* __restrict__ conv_w,
-    const __nv_bfloat16* __restrict__ conv_bias, const float* __restrict__ f, const float* __restrict__ bgate,
-    const float* __restrict__ dt_bias, const float* __restrict__ a_log, float lower_bound, float* __restrict__ state,
-    __nv_bfloat16* out, float* __restrict__ out_f32, const void* __restrict__ norm_w, int w_bf16,
-    const void* __restrict__ gate_out, int g_bf16, void* __restrict__ y, int y_f16, float eps, float cbias, int gate_act, int H,
-    float scale, const int* __restrict__ slots, int* __restrict__ tickets) {
-  constexpr int D = 128;
-  constexpr int KG = 128 / NV, RPT = D / KG;
-  const int b = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * NV;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j = tid % NV, kg = tid / NV;
-  const int dim = 3 * H * D;
-  const int slot = slots ? slots[b] : b;
-  const size_t bh = (size_t)b * H + head;
-  float* my_state = state + ((size_t)slot * H + head) * D * D + (size_t)(kg * RPT) * D + v0 + j;
-  __shared__ float sh_q[D], sh_k[D], sh_d[D];
-  __shared__ float sh_red[2][4];
-  __shared__ float sh_part[2][KG][NV];
-  __shared__ int sh_last, sh_last2;
+// state rows of warp w: groups w (i < 8) and w + 8; columns 4 lane .. 4 lane + 3
+__device__ __forceinline__ int state_row(int w, int i) { return 4 * (w + 8 * (i >> 3) + 16 * ((i >> 2) & 1)) + (i & 3); }
+struct GroupSums {                      // even and odd rows of the two groups
+  float4 s[4];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int u = 0; u < 4; u++) s[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __device__ __forceinline__ void add(int i, float c, float4 v) {
+    float4& a = s[2 * (i >> 3) + (i & 1)];
+    a.x = fmaf(c, v.x, a.x); a.y = fmaf(c, v.y, a.y); a.z = fmaf(c, v.z, a.z); a.w = fmaf(c, v.w, a.w);
+  }
+  __device__ __forceinline__ float4 total() const {
+    return make_float4(__fadd_rn(__fadd_rn(s[0].x, s[1].x), __fadd_rn(s[2].x, s[3].x)), __fadd_rn(__fadd_rn(s[0].y, s[1].y), __fadd_rn(s[2].y, s[3].y)),
+                       __fadd_rn(__fadd_rn(s[0].z, s[1].z), __fadd_rn(s[2].z, s[3].z)), __fadd_rn(__fadd_rn(s[0].w, s[1].w), __fadd_rn(s[2].w, s[3].w)));
+  }
+};
 
-  float S[RPT];
+__device__ __forceinline__ void state_kv(float4 (&S)[16], const DecodeToken& t, int rg, int lane, float (*part)[128]) {
+  GroupSums a;
+  a.clear();
 #pragma unroll
-  for (int i = 0; i < RPT; i++) S[i] = my_state[(size_t)i * D];
+  for (int i = 0; i < 16; i++) {
+    const int c = state_row(rg, i);
+    const float d = t.d[c];
+    S[i] = make_float4(__fmul_rn(S[i].x, d), __fmul_rn(S[i].y, d), __fmul_rn(S[i].z, d), __fmul_rn(S[i].w, d));
+    a.add(i, t.k[c], S[i]);
+  }
+  *reinterpret_cast<float4*>(&part[rg][4 * lane]) = a.total();
+}
+__device__ __forceinline__ float4 part_tree(const float (*part)[128], int lane) {
+  float4 p[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) p[i] = *reinterpret_cast<const float4*>(&part[i][4 * lane]);
+  return make_float4(tree8(p[0].x, p[1].x, p[2].x, p[3].x, p[4].x, p[5].x, p[6].x, p[7].x),
+                     tree8(p[0].y, p[1].y, p[2].y, p[3].y, p[4].y, p[5].y, p[6].y, p[7].y),
+                     tree8(p[0].z, p[1].z, p[2].z, p[3].z, p[4].z, p[5].z, p[6].z, p[7].z),
+                     tree8(p[0].w, p[1].w, p[2].w, p[3].w, p[4].w, p[5].w, p[6].w, p[7].w));
+}
+__device__ __forceinline__ void state_update(float4 (&S)[16], const DecodeToken& t, int rg, int lane, const float (*part)[128],
+                                             float (*opart)[128]) {
+  const float4 kv = part_tree(part, lane);
+  const float4 v = *reinterpret_cast<const float4*>(&t.v[4 * lane]);
+  const float be = t.beta;
+  const float4 un = make_float4(__fmul_rn(__fsub_rn(v.x, kv.x), be), __fmul_rn(__fsub_rn(v.y, kv.y), be),
+                                __fmul_rn(__fsub_rn(v.z, kv.z), be), __fmul_rn(__fsub_rn(v.w, kv.w), be));
+  GroupSums a;
+  a.clear();
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    const int c = state_row(rg, i);
+    const float k = t.k[c];
+    S[i].x = fmaf(k, un.x, S[i].x);
+    S[i].y = fmaf(k, un.y, S[i].y);
+    S[i].z = fmaf(k, un.z, S[i].z);
+    S[i].w = fmaf(k, un.w, S[i].w);
+    a.add(i, t.q[c], S[i]);
+  }
+  *reinterpret_cast<float4*>(&opart[rg][4 * lane]) = a.total();
+}
 
-  const float* xb = x32 + (size_t)b * dim;
-  __nv_bfloat16* cs = conv_state + (size_t)slot * dim * 4;
-  const int cq = head * D + tid, ck = (H + head) * D + tid, cv = (2 * H + head) * D + v0 + j;
-  const __nv_bfloat16 xq = __float2bfloat16(xb[cq]), xk = __float2bfloat16(xb[ck]), xv = __float2bfloat16(xb[cv]);
-  const uint2 sq4 = *reinterpret_cast<const uint2*>(cs + (size_t)cq * 4), wq4 = __ldg(reinterpret_cast<const uint2*>(conv_w + (size_t)cq * 4));
-  const uint2 sk4 = *reinterpret_cast<const uint2*>(cs + (size_t)ck * 4), wk4 = __ldg(reinterpret_cast<const uint2*>(conv_w + (size_t)ck * 4));
-  const uint2 sv4 = *reinterpret_cast<const uint2*>(cs + (size_t)cv * 4), wv4 = __ldg(reinterpret_cast<const uint2*>(conv_w + (size_t)cv * 4));
-  const float q = conv4_silu_bf16(sq4, wq4, conv_bias ? __bfloat162float(conv_bias[cq]) : 0.f, __bfloat162float(xq));
-  const float k = conv4_silu_bf16(sk4, wk4, conv_bias ? __bfloat162float(conv_bias[ck]) : 0.f, __bfloat162float(xk));
-  const float v = conv4_silu_bf16(sv4, wv4, conv_bias ? __bfloat162float(conv_bias[cv]) : 0.f, __bfloat162float(xv));
-  const float gv = gate_value(f[bh * D + tid], __ldg(dt_bias + head * D + tid), __expf(__ldg(a_log + head)), lower_bound);
-  const float beta_h = __bfloat162float(__float2bfloat16(1.0f / (1.0f + __expf(-bgate[bh]))));
-
-  float sq = warp_sum(q * q), sk = warp_sum(k * k);
-  if (lane == 0) {
-    sh_red[0][warp] = sq;
-    sh_red[1][warp] = sk;
+// one warp: the head's 128 outputs (lane = 4 columns), and LAYER: their gated RMS norm, as the one-warp-per-row norm kernel
+template <bool LAYER>
+__device__ __forceinline__ void decode_finish(const DecodeArgs& a, const float (*opart)[128], int bh, int lane) {
+  const size_t o = (size_t)bh * 128 + 4 * lane;
+  float4 ga, w4;
+  if (LAYER) {
+    ga = a.g_bf16 ? load4(reinterpret_cast<const __nv_bfloat16*>(a.gate_out) + o) : load4(reinterpret_cast<const float*>(a.gate_out) + o);
+    w4 = a.w_bf16 ? load4(reinterpret_cast<const __nv_bfloat16*>(a.norm_w) + 4 * lane) : load4(reinterpret_cast<const float*>(a.norm_w) + 4 * lane);
   }
-  __syncthreads();
-  {
-    float tq = 0.f, tk = 0.f;
+  float4 tot = part_tree(opart, lane);
+  tot.x *= a.scale; tot.y *= a.scale; tot.z *= a.scale; tot.w *= a.scale;
+  __nv_bfloat16 h[4] = {__float2bfloat16_rz(tot.x), __float2bfloat16_rz(tot.y), __float2bfloat16_rz(tot.z), __float2bfloat16_rz(tot.w)};
+  if (LAYER) {
+    uint2 r;
+    r.x = __bfloat16_as_ushort(h[0]) | ((uint32_t)__bfloat16_as_ushort(h[1]) << 16);
+    r.y = __bfloat16_as_ushort(h[2]) | ((uint32_t)__bfloat16_as_ushort(h[3]) << 16);
+    *reinterpret_cast<uint2*>(a.out + o) = r;
+  } else {
 #pragma unroll
-    for (int w = 0; w < 4; w++) {
-      tq += sh_red[0][w];
-      tk += sh_red[1][w];
-    }
-    sh_q[tid] = q * rsqrtf(tq + 1e-6f);
-    sh_k[tid] = k * rsqrtf(tk + 1e-6f);
-    sh_d[tid] = __expf(gv);
+    for (int u = 0; u < 4; u++) a.out[o + u] = h[u];
   }
-  int ticket = 0;
-  if (tid == 0) ticket = atomicAdd(tickets + bh, 1);
-  __syncthreads();
-  if (kg == 0) *reinterpret_cast<uint2*>(cs + (size_t)cv * 4) = conv4_rolled(sv4, xv);
-  float sum = 0.f;
-#pragma unroll
-  for (int i = 0; i < RPT; i++) {
-    const int c = kg * RPT + i;
-    sum = sum + sh_k[c] * sh_d[c] * S[i];
+  if (a.out_f32) {
+    a.out_f32[o] = tot.x; a.out_f32[o + 1] = tot.y; a.out_f32[o + 2] = tot.z; a.out_f32[o + 3] = tot.w;
   }
-  sh_part[0][kg][j] = sum;
-  __syncthreads();
-  float kv = 0.f;
-#pragma unroll
-  for (int p = 0; p < KG; p++) kv = __fadd_rn(kv, sh_part[0][p][j]);
-  const float vp = v - kv;
-  float o = 0.f;
-#pragma unroll
-  for (int i = 0; i < RPT; i++) {
-    const int c = kg * RPT + i;
-    const float st = S[i] * sh_d[c] + sh_k[c] * vp * beta_h;
-    S[i] = st;
-    o = o + sh_q[c] * st;
-  }
-  sh_part[1][kg][j] = o;
-  __syncthreads();
-  if (kg == 0) {
-    float tot = 0.f;
-#pragma unroll
-    for (int p = 0; p < KG; p++) tot = __fadd_rn(tot, sh_part[1][p][j]);
-    tot *= scale;
-    const size_t oi = bh * D + v0 + j;
-    out[oi] = __float2bfloat16_rz(tot);
-    if (out_f32) out_f32[oi] = tot;
-    __threadfence();                       // the outputs of this slice are visible before its second ticket is drawn
-  }
-#pragma unroll
-  for (int i = 0; i < RPT; i++) my_state[(size_t)i * D] = S[i];
-  __syncthreads();
-  if (tid == 0) {
-    const int last = ticket == (int)gridDim.z - 1;
-    if (last) tickets[bh] = 0;
-    sh_last = last;
-    int* t2 = tickets + (size_t)gridDim.x * H + bh;
-    const int last2 = atomicAdd(t2, 1) == (int)gridDim.z - 1;
-    if (last2) *t2 = 0;
-    sh_last2 = last2;
-  }
-  __syncthreads();
-  if (sh_last) {
-    *reinterpret_cast<uint2*>(cs + (size_t)cq * 4) = conv4_rolled(sq4, xq);
-    *reinterpret_cast<uint2*>(cs + (size_t)ck * 4) = conv4_rolled(sk4, xk);
-  }
-  if (sh_last2 && warp == 0) {
-    // gated RMS norm of the head's 128 outputs: lane = four channels, as the one-warp-per-row norm kernel
-    __threadfence();
-    const uint2 xr = __ldcg(reinterpret_cast<const uint2*>(out + bh * D) + lane);
-    const float4 xa = make_float4(bf16lo(xr.x), bf16hi(xr.x), bf16lo(xr.y), bf16hi(xr.y));
-    const float4 ga = g_bf16 ? load4(reinterpret_cast<const __nv_bfloat16*>(gate_out) + bh * D + 4 * lane)
-                             : load4(reinterpret_cast<const float*>(gate_out) + bh * D + 4 * lane);
-    const float4 w4 = w_bf16 ? load4(reinterpret_cast<const __nv_bfloat16*>(norm_w) + 4 * lane)
-                             : load4(reinterpret_cast<const float*>(norm_w) + 4 * lane);
-    float s = warp_sum(sum_squares(0.f, xa));
-    const float rmf = rsqrtf(s / (float)D + eps);
-    const float4 r = finish4(xa, w4, ga, rmf, cbias, false, gate_act);
-    if (y_f16) store4(reinterpret_cast<__half*>(y) + bh * D + 4 * lane, r);
-    else store4(reinterpret_cast<float*>(y) + bh * D + 4 * lane, r);
+  if (LAYER) {
+    const float4 xa = make_float4(__bfloat162float(h[0]), __bfloat162float(h[1]), __bfloat162float(h[2]), __bfloat162float(h[3]));
+    const float s = warp_sum(sum_squares(0.f, xa));
+    const float4 r = finish4(xa, w4, ga, rsqrtf(s / 128.0f + a.eps), a.cbias, false, a.gate_act);
+    if (a.y_f16) store4(reinterpret_cast<__half*>(a.y) + o, r);
+    else store4(reinterpret_cast<float*>(a.y) + o, r);
   }
 }
 
-template <int NV>
-static int launch_decode_conv(const __nv_bfloat16* x, __nv_bfloat16* conv_state, const __nv_bfloat16* w, const __nv_bfloat16* bias,
-                              const float* g, const __nv_bfloat16* beta, float* state, __nv_bfloat16* out, float* out_f32,
-                              __nv_bfloat16* conv_out, int bsz, int H, const int* slots, int* tickets, cudaStream_t s) {
-  kda_decode_conv_kernel<NV><<<dim3(bsz, H, 128 / NV), 128, 0, s>>>(x, conv_state, w, bias, g, beta, state, out, out_f32, conv_out,
-                                                                    H, 1.0f / sqrtf(128.0f), slots, tickets);
-  return cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+__device__ __forceinline__ float* head_state(const DecodeArgs& a, int bh) {
+  const int b = bh / a.H, head = bh - b * a.H;
+  const int slot = a.slots ? a.slots[b] : b;
+  return a.state + ((size_t)slot * a.H + head) * 128 * 128;
+}
+
+// VEC: the state is 16-byte aligned
+template <bool LAYER, bool VEC>
+__global__ __launch_bounds__(KD_THREADS) void kda_decode_kernel(const DecodeArgs a) {
+  const int bh = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ __align__(16) DecodeToken tok;
+  __shared__ __align__(16) float part[8][128], opart[8][128];
+  pdl_wait();
+  float4 S[16];
+  float* sp = nullptr;
+  if (warp < KD_STATE_WARPS) {
+    sp = head_state(a, bh) + 4 * lane;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const float* p = sp + state_row(warp, i) * 128;
+      S[i] = VEC ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+    }
+  } else {
+    decode_prepare<LAYER>(a, tok, bh, warp - KD_STATE_WARPS, lane);
+  }
+  __syncthreads();
+  if (warp < KD_STATE_WARPS) state_kv(S, tok, warp, lane, part);
+  __syncthreads();
+  if (warp < KD_STATE_WARPS) {
+    state_update(S, tok, warp, lane, part, opart);
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      float* p = sp + state_row(warp, i) * 128;
+      if (VEC) *reinterpret_cast<float4*>(p) = S[i];
+      else { p[0] = S[i].x; p[1] = S[i].y; p[2] = S[i].z; p[3] = S[i].w; }
+    }
+  }
+  __syncthreads();
+  if (warp == KD_STATE_WARPS) decode_finish<LAYER>(a, opart, bh, lane);
+}
+
+// persistent form: CTA c takes heads c, c + gridDim.x, ...
+constexpr int KD_STAGES = 2;
+constexpr size_t KD_STREAM_SMEM = (size_t)(KD_STAGES + 1) * 65536;
+template <bool LAYER>
+__global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const DecodeArgs a, int* __restrict__ status) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ __align__(16) DecodeToken tok[2];
+  __shared__ __align__(16) float part[8][128], opart[2][8][128];
+  __shared__ uint64_t full[KD_STAGES];
+  __shared__ int abort_flag;
+  const int step = gridDim.x, first = blockIdx.x;
+  const int n = (a.n_heads - first + step - 1) / step;          // >= 1: the grid is no larger than the head count
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < KD_STAGES; s++) tc::mbar_init(&full[s], 1);
+    tc::mbar_fence_init();
+    abort_flag = 0;
+  }
+  pdl_wait();
+  auto fetch = [&](int i) {                                     // thread 0: head i of this CTA into its stage
+    tc::mbar_arrive_expect_tx(&full[i % KD_STAGES], 65536);
+    tc::bulk_g2s(smem + (i % KD_STAGES) * 65536, head_state(a, first + i * step), 65536, &full[i % KD_STAGES]);
+  };
+  if (threadIdx.x == 0)
+    for (int i = 0; i < KD_STAGES && i < n; i++) fetch(i);
+  if (warp >= KD_STATE_WARPS) decode_prepare<LAYER>(a, tok[0], first, warp - KD_STATE_WARPS, lane);
+  __syncthreads();
+  bool ok = true;
+  for (int i = 0; i < n; i++) {
+    const int bh = first + i * step;
+    const float4* st = reinterpret_cast<const float4*>(smem + (i % KD_STAGES) * 65536) + lane;
+    if (warp < KD_STATE_WARPS) {
+      ok = tc::mbar_wait(&full[i % KD_STAGES], (i / KD_STAGES) & 1, &abort_flag, 1);
+      float4 S[16];
+#pragma unroll
+      for (int r = 0; r < 16; r++) S[r] = st[state_row(warp, r) * 32];
+      state_kv(S, tok[i & 1], warp, lane, part);
+      if (threadIdx.x == 0) tc::bulk_wait_read<0>();
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (threadIdx.x == 0 && i + KD_STAGES < n) fetch(i + KD_STAGES);
+      state_update(S, tok[i & 1], warp, lane, part, opart[i & 1]);
+      // the outward stage is free: thread 0 has waited for its last reader, and passed the barrier above, since
+      float4* so = reinterpret_cast<float4*>(smem + KD_STAGES * 65536) + lane;
+#pragma unroll
+      for (int r = 0; r < 16; r++) so[state_row(warp, r) * 32] = S[r];
+      tc::fence_async_smem();
+    } else {
+      if (i > 0 && warp == KD_WARPS - 1) decode_finish<LAYER>(a, opart[(i - 1) & 1], bh - step, lane);
+      if (i + 1 < n) decode_prepare<LAYER>(a, tok[(i + 1) & 1], bh + step, warp - KD_STATE_WARPS, lane);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && ok && !abort_flag) {
+      tc::bulk_s2g(head_state(a, bh), smem + KD_STAGES * 65536, 65536);
+      tc::bulk_commit();
+    }
+  }
+  if (warp == KD_WARPS - 1) decode_finish<LAYER>(a, opart[(n - 1) & 1], first + (n - 1) * step, lane);
+  if (threadIdx.x == 0) {
+    tc::bulk_wait_all<0>();
+    if (abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
+  }
+}
+
+template <bool LAYER>
+static int launch_decode(const DecodeArgs& a, cudaStream_t s) {
+  const bool vec = aligned(a.state, 16);
+  if (vec && a.n_heads > 2 * sm_count()) {
+    static bool attr_set[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+      if (cudaFuncSetAttribute(kda_decode_stream_kernel<LAYER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KD_STREAM_SMEM) != cudaSuccess)
+        return HK_ERR_CUDA;
+      attr_set[dev] = true;
+    }
+    const int grid = sm_count();
+    return pdl_launch(kda_decode_stream_kernel<LAYER>, dim3(grid), dim3(KD_THREADS), KD_STREAM_SMEM, s, a, device_status_ptr()) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+  }
+  auto kern = vec ? kda_decode_kernel<LAYER, true> : kda_decode_kernel<LAYER, false>;
+  return pdl_launch(kern, dim3(a.n_heads), dim3(KD_THREADS), 0, s, a) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Token by token with channelwise decay, D = 128, no history: short prompts, and decode through the launchers.
+//
+// What bounds it is the chain from token to token.  The kernel above takes 1.07 us per token: every token is normalised inside
+// the chain and crosses four block barriers.  Here a warp owns 2 CPL columns, lane (rg, c) the 8 rows of group rg of CPL
+// columns, and the sums over the 16 groups are shuffles: no barrier inside the chain.  Everything that does not depend on the
+// state (norms, decay) is prepared for 8 tokens at a time in the other half of a double buffer, a warp per token: one
+// block barrier per 8 tokens.  The products run as packed fp32 pairs (two rows per instruction).
+// Shared memory is the other limit: a warp reads a token's three prepared vectors (1.5 KB) whatever it does with them, as
+// 6 reads of 4 wavefronts.  With 8 groups over 8 lanes (and k * d as a fourth vector) it was 16 reads (64 heads: 0.84 us per token with one column per lane,
+// 0.57 with four).  The output sums of four tokens are taken together and exchange HALF of their values at each step (15
+// shuffles for 16 values instead of 64).
+// CPL is the one that yields 256 CTAs or more from 64, 32 and 16 chains.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+
+// Sums of N values per lane over the 16 lanes of a half warp, lanes 8 apart first, then 1, 2, 4.  While a lane has more than
+// one value it keeps one half and hands the other to its partner; a lane ends with the sum of value sum_index (the same in
+// all lanes that agree in the bits used; sum_owner picks one of them).
+template <int N>
+__device__ __forceinline__ int sum_index(int lane) {
+  const int b3 = (lane >> 3) & 1, b0 = lane & 1, b1 = (lane >> 1) & 1, b2 = (lane >> 2) & 1;
+  if (N == 16) return 8 * b3 + 4 * b0 + 2 * b1 + b2;
+  if (N == 8) return 4 * b3 + 2 * b0 + b1;
+  if (N == 4) return 2 * b3 + b0;
+  if (N == 2) return b3;
+  return 0;
+}
+template <int N>
+__device__ __forceinline__ bool sum_owner(int lane) {
+  return N == 16 || (lane & (N == 8 ? 4 : (N == 4 ? 6 : (N == 2 ? 7 : 15)))) == 0;
+}
+template <int N>
+__device__ __forceinline__ float lane_sums(const float* v, int lane) {
+  float x[N];
+#pragma unroll
+  for (int i = 0; i < N; i++) x[i] = v[i];
+  int n = N;
+#pragma unroll
+  for (int st = 0; st < 4; st++) {
+    const int m = st == 0 ? 8 : 1 << (st - 1);
+    if (n > 1) {
+      n >>= 1;
+#pragma unroll
+      for (int i = 0; i < N / 2; i++) {
+        if (i < n) {
+          const bool up = lane & m;
+          const float keep = up ? x[i + n] : x[i], give = up ? x[i] : x[i + n];
+          x[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, m));
+        }
+      }
+    } else {
+      x[0] = __fadd_rn(x[0], __shfl_xor_sync(0xffffffffu, x[0], m));
+    }
+  }
+  return x[0];
+}
+constexpr int RC_TB = 8, RC_WARPS = 4;
+template <int COLS>
+struct alignas(16) RecBatch {           // 8 prepared tokens
+  float q[RC_TB][128], k[RC_TB][128], d[RC_TB][128], v[RC_TB][COLS], beta[RC_TB];
+};
+
+template <int CPL>
+__global__ __launch_bounds__(RC_WARPS * 32) void kda_recurrent_cols_kernel(
+    const __nv_bfloat16* __restrict__ mixed_qkv, const float* __restrict__ g, const __nv_bfloat16* __restrict__ beta,
+    float* __restrict__ state, __nv_bfloat16* __restrict__ out, float* __restrict__ out_f32, int seqlen, int Hk, int Hv, float scale,
+    const int* __restrict__ slots) {
+  constexpr int COLS = RC_WARPS * 2 * CPL, TPW = RC_TB / RC_WARPS;      // columns of the CTA, tokens a warp prepares
+  __shared__ RecBatch<COLS> rb[2];
+  __shared__ __align__(16) float s_o[2][RC_TB][COLS];
+  const int b = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * COLS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = lane & 15, col = (warp * 2 + (lane >> 4)) * CPL;       // first column of this lane
+  const int k_head = head / (Hv / Hk);
+  const size_t row = (size_t)2 * Hk * 128 + (size_t)Hv * 128;
+  pdl_wait();
+  const int slot = slots ? slots[b] : b;
+  const __nv_bfloat16* tok = mixed_qkv + (size_t)b * seqlen * row;
+  const float* gp = g + ((size_t)b * seqlen * Hv + head) * 128;
+  const __nv_bfloat16* bp = beta + (size_t)b * seqlen * Hv + head;
+  float* sp = state + ((size_t)slot * Hv + head) * 128 * 128 + v0 + col;
+
+  // tokens warp, warp + 4 of a batch: channel lane + 32 u of q, k, g, columns lane, lane + 32 of v
+  constexpr int NVL = (COLS + 31) / 32;
+  // (kept as loaded: a conversion here would wait for the load before the tokens in hand)
+  __nv_bfloat16 rq[TPW][4], rk[TPW][4], rv[TPW][NVL], rbeta[TPW];
+  float rgt[TPW][4];
+  auto fetch = [&](int s0) {
+#pragma unroll
+    for (int p = 0; p < TPW; p++) {
+      const int s = s0 + warp + p * RC_WARPS;
+      if (s >= seqlen) break;
+      const __nv_bfloat16* t = tok + (size_t)s * row;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        rq[p][u] = t[(size_t)k_head * 128 + lane + 32 * u];
+        rk[p][u] = t[(size_t)(Hk + k_head) * 128 + lane + 32 * u];
+        rgt[p][u] = gp[(size_t)s * Hv * 128 + lane + 32 * u];
+      }
+#pragma unroll
+      for (int u = 0; u < NVL; u++)
+        if (lane + 32 * u < COLS) rv[p][u] = t[(size_t)2 * Hk * 128 + (size_t)head * 128 + v0 + lane + 32 * u];
+      rbeta[p] = bp[(size_t)s * Hv];
+    }
+  };
+  auto prepare = [&](RecBatch<COLS>& r, int s0) {
+#pragma unroll
+    for (int p = 0; p < TPW; p++) {
+      const int t = warp + p * RC_WARPS;
+      if (s0 + t >= seqlen) break;
+      float fq[4], fk[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        fq[u] = __bfloat162float(rq[p][u]);
+        fk[u] = __bfloat162float(rk[p][u]);
+      }
+      const float iq = inv_norm(fq), ik = inv_norm(fk);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int c = lane + 32 * u;
+        r.q[t][c] = __fmul_rn(fq[u], iq);
+        r.k[t][c] = __fmul_rn(fk[u], ik);
+        r.d[t][c] = __expf(rgt[p][u]);
+      }
+#pragma unroll
+      for (int u = 0; u < NVL; u++)
+        if (lane + 32 * u < COLS) r.v[t][lane + 32 * u] = __bfloat162float(rv[p][u]);
+      if (lane == 0) r.beta[t] = __bfloat162float(rbeta[p]);
+    }
+  };
+  fetch(0);
+  // rows 4 (rg + 16 j) + e of the lane's columns, packed by row pairs
+  auto ld_cols = [&](int r, float (&x)[CPL]) {
+    const float* p = sp + (size_t)r * 128;
+    if constexpr (CPL == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(p);
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    } else if constexpr (CPL == 2) {
+      const float2 v = *reinterpret_cast<const float2*>(p);
+      x[0] = v.x; x[1] = v.y;
+    } else {
+      x[0] = p[0];
+    }
+  };
+  auto st_cols = [&](int r, const float (&x)[CPL]) {
+    float* p = sp + (size_t)r * 128;
+    if constexpr (CPL == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+    else if constexpr (CPL == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+    else p[0] = x[0];
+  };
+  uint64_t S[CPL][4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int r0 = 4 * (rg + 16 * (i >> 1)) + 2 * (i & 1);
+    float x0[CPL], x1[CPL];
+    ld_cols(r0, x0);
+    ld_cols(r0 + 1, x1);
+#pragma unroll
+    for (int c = 0; c < CPL; c++) S[c][i] = pack2(x0[c], x1[c]);
+  }
+  prepare(rb[0], 0);
+  __syncthreads();
+  int buf = 0;
+  for (int s0 = 0; s0 < seqlen; s0 += RC_TB, buf ^= 1) {
+    const int n = min(RC_TB, seqlen - s0);
+    fetch(s0 + RC_TB);
+    const RecBatch<COLS>& r = rb[buf];
+    // A token's operands are read while the token before it is in its shuffles: read where they are used, they were a
+    // third of the chain.
+    struct Operands {
+      uint64_t k[4], d[4], q[4];
+      float v[CPL], be;
+    };
+    auto operands = [&](int t, Operands& o) {
+      auto pieces = [&](const float (*p)[128], uint64_t (&x)[4]) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&p[t][4 * (rg + 16 * j)]);
+          x[2 * j] = w.x;
+          x[2 * j + 1] = w.y;
+        }
+      };
+      pieces(r.d, o.d);
+      pieces(r.k, o.k);
+      pieces(r.q, o.q);
+      o.be = r.beta[t];
+#pragma unroll
+      for (int c = 0; c < CPL; c++) o.v[c] = r.v[t][col + c];
+    };
+    auto token = [&](int t, Operands& o, float* ov) {
+      auto group_sum = [&](const uint64_t (&x)[4], float* y) {
+#pragma unroll
+        for (int c = 0; c < CPL; c++) {
+          uint64_t acc = 0;
+#pragma unroll
+          for (int i = 0; i < 4; i++) acc = fma2(x[i], S[c][i], acc);
+          float lo, hi;
+          unpack2(acc, lo, hi);
+          y[c] = __fadd_rn(lo, hi);
+        }
+      };
+      float y[CPL];
+#pragma unroll
+      for (int c = 0; c < CPL; c++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) S[c][i] = mul2(S[c][i], o.d[i]);
+      group_sum(o.k, y);
+      Operands next;
+      operands(min(t + 1, RC_TB - 1), next);
+      // every lane needs the sums of all its columns: plain butterfly (halving the values and spreading them again takes
+      // as many instructions and two more exchanges on the chain)
+#pragma unroll
+      for (int st = 0; st < 4; st++)
+#pragma unroll
+        for (int c = 0; c < CPL; c++) y[c] = __fadd_rn(y[c], __shfl_xor_sync(0xffffffffu, y[c], st == 0 ? 8 : 1 << (st - 1)));
+#pragma unroll
+      for (int c = 0; c < CPL; c++) {
+        const float un = __fmul_rn(__fsub_rn(o.v[c], y[c]), o.be);
+        const uint64_t u2 = pack2(un, un);
+#pragma unroll
+        for (int i = 0; i < 4; i++) S[c][i] = fma2(o.k[i], u2, S[c][i]);
+      }
+      group_sum(o.q, ov);
+      o = next;
+    };
+    Operands ops;
+    operands(0, ops);
+    int t = 0;
+#pragma unroll 1
+    for (; t + 4 <= n; t += 4) {
+      float ov[4 * CPL];                                 // group sums of the outputs of four tokens
+#pragma unroll
+      for (int tt = 0; tt < 4; tt++) token(t + tt, ops, ov + tt * CPL);
+      const float o = lane_sums<4 * CPL>(ov, lane);
+      const int idx = sum_index<4 * CPL>(lane);          // value (token t + idx / CPL, column col + idx % CPL)
+      if (sum_owner<4 * CPL>(lane)) s_o[buf][t + idx / CPL][col + idx % CPL] = o;
+    }
+#pragma unroll 1
+    for (; t < n; t++) {
+      float ov[CPL];
+      token(t, ops, ov);
+      const float o = lane_sums<CPL>(ov, lane);
+      if (sum_owner<CPL>(lane)) s_o[buf][t][col + sum_index<CPL>(lane)] = o;
+    }
+    prepare(rb[buf ^ 1], s0 + RC_TB);
+    __syncthreads();
+    for (int i = tid; i < n * COLS; i += RC_WARPS * 32) {
+      const float tot = s_o[buf][i / COLS][i % COLS] * scale;
+      const size_t oi = (((size_t)b * seqlen + s0 + i / COLS) * Hv + head) * 128 + v0 + i % COLS;
+      out[oi] = __float2bfloat16_rz(tot);
+      if (out_f32) out_f32[oi] = tot;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int r0 = 4 * (rg + 16 * (i >> 1)) + 2 * (i & 1);
+    float x0[CPL], x1[CPL];
+#pragma unroll
+    for (int c = 0; c < CPL; c++) unpack2(S[c][i], x0[c], x1[c]);
+    st_cols(r0, x0);
+    st_cols(r0 + 1, x1);
+  }
 }
 
 template <int D, int NV>
@@ -462,6 +803,15 @@ HK_API int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* b
   auto bt = (const __nv_bfloat16*)beta;
   auto o = (__nv_bfloat16*)out;
   cudaStream_t s = as_stream(stream);
+  if (k_head_dim == 128 && channelwise && !history && history_stride == 1) {
+    const int64_t chains = (int64_t)bsz * num_v_heads;
+    const int cpl = !aligned(state, 16) || chains < 32 ? 1 : (chains < 64 ? 2 : 4);
+    auto kern = cpl == 4 ? kda_recurrent_cols_kernel<4> : (cpl == 2 ? kda_recurrent_cols_kernel<2> : kda_recurrent_cols_kernel<1>);
+    return pdl_launch(kern, dim3(bsz, num_v_heads, 16 / cpl), dim3(RC_WARPS * 32), 0, s, q, g, bt, state, o, out_f32, seqlen, num_k_heads,
+                      num_v_heads, 1.0f / sqrtf(128.0f), slots) == cudaSuccess
+               ? HK_OK
+               : HK_ERR_CUDA;
+  }
   // narrower column slices when the (batch x head) count alone cannot cover the SMs
   const bool narrow = (long)bsz * num_v_heads * 4 < sm_count();
   if (k_head_dim == 128) {
@@ -484,17 +834,22 @@ HK_API int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_
   using namespace hk;
   HK_REQUIRE(x && conv_state && conv_weight && g && beta && rec_state && out && tickets);
   HK_REQUIRE(bsz > 0 && bsz <= 65535 && num_heads > 0 && num_heads <= 65535);
-  auto xb = (const __nv_bfloat16*)x;
-  auto cs = (__nv_bfloat16*)conv_state;
-  auto cw = (const __nv_bfloat16*)conv_weight;
-  auto cb = (const __nv_bfloat16*)conv_bias;
-  auto bt = (const __nv_bfloat16*)beta;
-  auto o = (__nv_bfloat16*)out;
-  auto co = (__nv_bfloat16*)conv_out;
-  cudaStream_t s = as_stream(stream);
-  const bool narrow = (long)bsz * num_heads * 4 < sm_count();
-  return narrow ? launch_decode_conv<16>(xb, cs, cw, cb, g, bt, rec_state, o, out_f32, co, bsz, num_heads, slots, tickets, s)
-                : launch_decode_conv<32>(xb, cs, cw, cb, g, bt, rec_state, o, out_f32, co, bsz, num_heads, slots, tickets, s);
+  DecodeArgs a{};
+  a.x = x;
+  a.conv_state = (__nv_bfloat16*)conv_state;
+  a.conv_w = (const __nv_bfloat16*)conv_weight;
+  a.conv_bias = (const __nv_bfloat16*)conv_bias;
+  a.g = g;
+  a.beta = beta;
+  a.state = rec_state;
+  a.out = (__nv_bfloat16*)out;
+  a.out_f32 = out_f32;
+  a.conv_out = (__nv_bfloat16*)conv_out;
+  a.scale = 1.0f / sqrtf(128.0f);
+  a.H = num_heads;
+  a.n_heads = bsz * num_heads;
+  a.slots = slots;
+  return launch_decode<false>(a, as_stream(stream));
 }
 
 HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f,
@@ -511,16 +866,31 @@ HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* c
   HK_REQUIRE(gate_act == 0 || gate_act == 1);
   HK_REQUIRE(aligned(out, 8) && aligned(norm_w, w_type == HK_F32 ? 16 : 8) && aligned(y, y_type == HK_F32 ? 16 : 8) &&
              aligned(gate_out, g_type == HK_F32 ? 16 : 8));
-  cudaStream_t s = as_stream(stream);
-  const float scale = 1.0f / sqrtf(128.0f);
-  const bool narrow = (long)bsz * num_heads * 4 < sm_count();
-#define HK_DL(NV)                                                                                                          \
-  kda_decode_layer_kernel<NV><<<dim3(bsz, num_heads, 128 / NV), 128, 0, s>>>(                                              \
-      x32, (__nv_bfloat16*)conv_state, (const __nv_bfloat16*)conv_weight, (const __nv_bfloat16*)conv_bias, f, b, dt_bias, a_log,  \
-      lower_bound, rec_state, (__nv_bfloat16*)out, out_f32, norm_w, w_type == HK_BF16, gate_out, g_type == HK_BF16, y,        \
-      y_type == HK_F16, epsilon, constant_bias, gate_act, num_heads, scale, slots, tickets)
-  if (narrow) HK_DL(16); else HK_DL(32);
-#undef HK_DL
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  DecodeArgs a{};
+  a.x = x32;
+  a.conv_state = (__nv_bfloat16*)conv_state;
+  a.conv_w = (const __nv_bfloat16*)conv_weight;
+  a.conv_bias = (const __nv_bfloat16*)conv_bias;
+  a.g = f;
+  a.beta = b;
+  a.dt_bias = dt_bias;
+  a.a_log = a_log;
+  a.lower_bound = lower_bound;
+  a.state = rec_state;
+  a.out = (__nv_bfloat16*)out;
+  a.out_f32 = out_f32;
+  a.norm_w = norm_w;
+  a.gate_out = gate_out;
+  a.y = y;
+  a.w_bf16 = w_type == HK_BF16;
+  a.g_bf16 = g_type == HK_BF16;
+  a.y_f16 = y_type == HK_F16;
+  a.gate_act = gate_act;
+  a.eps = epsilon;
+  a.cbias = constant_bias;
+  a.scale = 1.0f / sqrtf(128.0f);
+  a.H = num_heads;
+  a.n_heads = bsz * num_heads;
+  a.slots = slots;
+  return launch_decode<true>(a, as_stream(stream));
 }

@@ -75,9 +75,7 @@ int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* beta, fl
  *   conv_weight [3*H*128][4] bf16   conv_bias [3*H*128] bf16 or NULL   g [bsz][H][128] f32   beta [bsz][H] bf16
  *   rec_state [slots][H][128][128] f32 (in place)   out [bsz][H][128] bf16 (rz)   out_f32 optional
  *   conv_out optional [bsz][3*H*128] bf16: the convolved q|k|v (what the two-kernel sequence leaves in between).
- *   tickets: bsz*H device ints, zero before the first call; every call leaves them zero (the slices of a head count
- *   themselves there to find out which one rolls the head's q / k window).  Calls that share `tickets` must not
- *   overlap on the GPU.                                                                                          */
+ *   tickets: bsz*H device ints, zero before the first call; left zero (earlier forms counted a head's slices there).   */
 int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_weight, const void* conv_bias, const float* g,
                        const void* beta, float* rec_state, void* out, float* out_f32, void* conv_out, int bsz,
                        int num_heads, const int* slots, int* tickets, void* stream);
@@ -89,7 +87,7 @@ int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_weight,
  * norm_w [128] of w_type (HK_F32 / HK_BF16), gate_out [bsz*H][128] of g_type (HK_F32 / HK_BF16).  `out` (bf16) and
  * out_f32 (optional) receive the recurrence output.  The reference's decode runs five launches here
  * (src/engine/runner.cpp:433-489); results are bit-identical to calling the five in turn.
- * tickets: 2 * bsz * H zeroed ints of caller memory, left zeroed; calls sharing them must not overlap on the GPU.   */
+ * tickets: 2 * bsz * H zeroed ints of caller memory, left zeroed (not used any more).                               */
 int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f,
                         const float* b, const float* dt_bias, const float* a_log, float lower_bound, float* rec_state,
                         void* out, float* out_f32, const void* norm_w, int w_type, const void* gate_out, int g_type, void* y,
@@ -106,7 +104,8 @@ int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_wei
  * more chains when a number of chain CTAs in [16, 48] divides their count, e.g. 64 heads or 8 x 32: a chain CTA then
  * walks several chains one after the other); the other SMs prepare the chunks and hand them over through a ring of 16
  * chunk slots per chain CTA (workspace = chain CTAs * 16 * 74,240 B + flags, independent of seqlen; it stays in L2).
- * Other calls run as two kernels with one 74,240-byte workspace unit per (batch, head, chunk).
+ * Other calls run as two kernels with one 74,240-byte workspace unit per (batch, head, chunk); short calls (all units fit the
+ * ring's memory, up to 16 chunks per chain) run as two kernels in it.
  * hk_kda_chunked_set_form(1) selects the two-kernel form for every later call and workspace query of this
  * process, hk_kda_chunked_set_form(0) the automatic choice (default).                              */
 int hk_kda_chunked_set_form(int form);
@@ -199,9 +198,8 @@ int hk_dsa_topk(const void* scores, int s_stride, int* indices, int R, int T, in
                 const int* t_ptr, int t_seq, void* stream);
 
 /* hk_dsa_topk with hk_pool_expand folded into the output writes: indices [R][512] as hk_dsa_topk (k_pad = 512) AND
- * raw_idx [R][2052] as hk_pool_expand(indices, q_pos) would give, in one kernel.  after_scorer != 0: the kernel is
- * launched as a programmatic dependent of the kernel before it in the stream (use only directly behind
- * hk_indexer_score of at most 8 rows, which releases its dependents early).                                       */
+ * raw_idx [R][2052] as hk_pool_expand(indices, q_pos) would give, in one kernel.  after_scorer is accepted for
+ * earlier callers and has no effect: every selection kernel is launched as a programmatic dependent.              */
 int hk_dsa_topk_expand(const void* scores, int s_stride, int* indices, int* raw_idx, const int* q_pos, int R, int T,
                        int k, int after_scorer, void* stream);
 

@@ -349,3 +349,55 @@ def test_decode_layer_in_one_launch_equals_the_five_call_sequence(H, bsz, w_bf16
     assert np.array_equal(bits(out_a.reshape(steps, bsz, H, D)), bits(out_b)), "recurrence outputs"
     assert torch.equal(y_a, y_b), "normalised outputs"
     assert torch.isfinite(y_b.float()).all()
+
+
+@pytest.mark.parametrize("H,bsz,slots", [(64, 5, False), (8, 41, True), (33, 9, True)])
+def test_decode_of_many_heads_streams_the_same_bits(H, bsz, slots):
+    """more heads than two per SM: the persistent form (heads stream through shared memory, ragged last round) against the
+    per-sequence calls, which take the one-head-per-CTA form; carried window and state, slots out of order"""
+    D, dim = 128, 3 * H * 128
+    gen = torch.Generator(device="cuda").manual_seed(H)
+
+    def rnd(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+    raw = synth.kda_raw_gates(1, H, D, seed=9)
+    dtb, alog, lb = dev(raw["dt_bias"]), dev(raw["a_log"]), raw["lower_bound"]
+    w, nw = (0.1 * rnd(dim, 4)).to(torch.bfloat16), 1.0 + 0.1 * rnd(D)
+    cs, st = rnd(bsz, dim, 4).to(torch.bfloat16), 0.1 * rnd(bsz, 1, H, D, D)
+    order = torch.randperm(bsz, generator=torch.Generator().manual_seed(1)).to(torch.int32).cuda() if slots else None
+    res = []
+    for whole in (True, False):
+        c, s = cs.clone(), st.clone()
+        out, y = torch.empty(2, bsz, H, D, dtype=torch.bfloat16, device="cuda"), torch.empty(2, bsz, H * D, dtype=torch.float16, device="cuda")
+        gen.manual_seed(7)
+        for t in range(2):
+            x, f, b, go = rnd(bsz, dim), rnd(bsz, H, D), rnd(bsz, H), rnd(bsz, H * D)
+            if whole:
+                hk.kda_decode_layer(x, c, w, None, f, b, dtb, alog, lb, s, out[t], nw, go, y[t], bsz, H, slots=order)
+            else:
+                for i in range(bsz):
+                    j = int(order[i]) if slots else i
+                    hk.kda_decode_layer(x[i], c[j], w, None, f[i], b[i], dtb, alog, lb, s[j], out[t, i], nw, go[i], y[t, i], 1, H)
+        torch.cuda.synchronize()
+        res.append((out, y, c, s))
+    assert hk.read_device_status() == 0
+    for whole, single in zip(*res):
+        assert torch.equal(whole, single)
+
+
+@pytest.mark.parametrize("T,Hk,Hv,bsz", [(1, 2, 4, 1), (7, 3, 3, 2), (8, 1, 2, 1), (9, 4, 4, 3), (63, 2, 2, 1)])
+def test_per_token_kernel_around_its_batches_of_eight(T, Hk, Hv, bsz):
+    """token counts either side of the 8 prepared at a time, grouped key heads, against the oracle"""
+    D = 128
+    inp = synth.kda_inputs(T, Hv, D, bsz=bsz, seed=T)
+    qkv = inp["mixed_qkv"].reshape(bsz, T, 3, Hv, D)
+    qkv = np.concatenate([qkv[:, :, 0, :Hk].reshape(bsz, T, -1), qkv[:, :, 1, :Hk].reshape(bsz, T, -1), qkv[:, :, 2].reshape(bsz, T, -1)], axis=2)
+    s0 = (0.1 * synth.rng(3).standard_normal((bsz, 1, Hv, D, D), dtype=np.float32)).astype(np.float32)
+    _, o_32, o_st = orc.kda_recurrent(np.ascontiguousarray(qkv), inp["g"], inp["beta"], s0, bsz, T, Hk, Hv, D, D)
+    q, g, b, st = dev_bf16(qkv), dev(inp["g"]), dev_bf16(inp["beta"]), dev(s0)
+    out = torch.empty(bsz, T, Hv, D, dtype=torch.bfloat16, device="cuda")
+    f32 = torch.empty(bsz, T, Hv, D, dtype=torch.float32, device="cuda")
+    hk.cuda_recurrent_gated_delta_rule(q, g, b, st, out, bsz, T, Hk, Hv, D, D, 1, None, True, False, out_f32=f32)
+    torch.cuda.synchronize()
+    assert max_rel(f32.cpu().numpy(), o_32) < 1e-4 and frob_rel(st.cpu().numpy(), o_st) < 1e-5
+    assert np.array_equal(bits(out), (f32.cpu().numpy().view(np.uint32) >> 16).astype(np.uint16)), "rounded toward zero"
