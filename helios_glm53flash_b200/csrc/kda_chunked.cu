@@ -704,6 +704,7 @@ __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
     abort_flag = 0;
   }
   if (tid < 32) tc::tmem_alloc(&tmem_slot, 256);
+  pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -747,9 +748,6 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
   const int vs = blockIdx.x, head = blockIdx.y, b = blockIdx.z;
   const int v0 = vs * KNV;
   const uint8_t* unit0 = ws + ((size_t)b * n_chunks * H + head) * U_BYTES;   // unit of chunk c: + c * H * U_BYTES
-  const int slot = slots ? slots[b] : b;
-  float* st = state + ((size_t)slot * H + head) * KD * KD + (size_t)tid * KD + v0;  // row k = tid
-
   if (tid == 0) {
     for (int i = 0; i < S_NSTAGE; i++) tc::mbar_init(&full_bar[i], 1);
     tc::mbar_init(&mma_bar, 1);
@@ -762,7 +760,10 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
   for (int i = tid; i < 8192 / 16; i += 128) {
     for (int st_i = 0; st_i < S_NSTAGE; st_i++) reinterpret_cast<uint4*>(smem + st_i * S_STAGE + S_BB)[i] = make_uint4(0, 0, 0, 0);
   }
+  pdl_wait();
   // state slice: thread = k row, 32 fp32 values in registers; fp16 copy as the B operand
+  const int slot = slots ? slots[b] : b;
+  float* st = state + ((size_t)slot * H + head) * KD * KD + (size_t)tid * KD + v0;  // row k = tid
   float S[KNV];
 #pragma unroll
   for (int u = 0; u < KNV / 4; u++) {
@@ -1440,6 +1441,15 @@ int fused_slots(long long n_jobs) {
   }
   return 0;
 }
+// Short calls run as two kernels although a fused form exists, in the ring's memory: the fused launch costs about 33 us before
+// its first chunk is through (flags cleared, cooperative launch, ring start-up) and 2.6 us per chunk of a chain, the two
+// kernels 15 us and 1.4 us per chunk and wave of scan CTAs (four per chain).  Measured at 32 heads: 64 tokens 33 -> 25 us,
+// 512 53 -> 40, 1,024 77 -> 68, equal at 1,536; 8 heads x 1,024 tokens 71 -> 43; 8 sequences x 64 heads x 64 tokens 176 -> 118.
+// The line: all units fit the ring's memory (16 chunks per slot), and either one wave of scan CTAs or at most 12 chunks
+// (48 heads x 1,024 tokens, two waves: 106 fused, 119 as two kernels).
+bool short_call(long long n_jobs, int n_chunks, int n_slots) {
+  return n_jobs * n_chunks <= (long long)KR * n_slots && (KVS * n_jobs <= sm_count() || n_chunks <= 12);
+}
 size_t fused_flag_bytes(int n_slots) {
   return (((size_t)F_FLAG_INTS + (size_t)n_slots * (KR + 1)) * sizeof(int) + 255) / 256 * 256;
 }
@@ -1497,7 +1507,8 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
   }
   cudaStream_t s = as_stream(stream);
   int* st = device_status_ptr();
-  if (const int n_slots = fused_slots((long long)bsz * num_heads)) {
+  const int n_slots = fused_slots((long long)bsz * num_heads);
+  if (n_slots && !short_call((long long)bsz * num_heads, n_chunks, n_slots)) {
     // one cooperative launch: chain slots on the first n_slots CTAs, preparation workers on all others
     const int n_jobs = bsz * num_heads;
     const size_t flag_bytes = fused_flag_bytes(n_slots);
@@ -1557,20 +1568,15 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
     return e == cudaSuccess ? HK_OK : HK_ERR_CUDA;
   }
   const dim3 grid(num_heads, n_chunks, bsz);
-  if (gated)
-    kda_chunk_prep_kernel<true><<<grid, 256, P1_SMEM, s>>>((const __nv_bfloat16*)mixed_qkv, g_or_f, beta_or_b,
-                                                         (uint8_t*)workspace, seqlen, num_heads, n_chunks,
-                                                         2 * sm_count(), st, dt_bias, a_log, lower_bound);
-  else
-    kda_chunk_prep_kernel<false><<<grid, 256, P1_SMEM, s>>>((const __nv_bfloat16*)mixed_qkv, g_or_f, beta_or_b,
-                                                          (uint8_t*)workspace, seqlen, num_heads, n_chunks,
-                                                          2 * sm_count(), st, nullptr, nullptr, 0.f);
-  HK_LAUNCH_CHECK();
-  kda_chunk_scan_kernel<<<dim3(KVS, num_heads, bsz), 128, P2_SMEM, s>>>(
-      (const uint8_t*)workspace, state, (__nv_bfloat16*)out, out_f32, seqlen, num_heads, n_chunks,
-      slots, 1.0f / sqrtf((float)KD), st);
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  auto prep = gated ? kda_chunk_prep_kernel<true> : kda_chunk_prep_kernel<false>;
+  if (pdl_launch(prep, grid, dim3(256), P1_SMEM, s, (const __nv_bfloat16*)mixed_qkv, g_or_f, beta_or_b, (uint8_t*)workspace, seqlen,
+                 num_heads, n_chunks, 2 * sm_count(), st, gated ? dt_bias : nullptr, gated ? a_log : nullptr,
+                 gated ? lower_bound : 0.f) != cudaSuccess)
+    return HK_ERR_CUDA;
+  return pdl_launch(kda_chunk_scan_kernel, dim3(KVS, num_heads, bsz), dim3(128), P2_SMEM, s, (const uint8_t*)workspace, state,
+                    (__nv_bfloat16*)out, out_f32, seqlen, num_heads, n_chunks, slots, 1.0f / sqrtf((float)KD), st) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 }  // namespace
 }  // namespace hk
