@@ -8,9 +8,11 @@
 //                      shared memory: a lane keeps 2 channels x 16 (or 32) tokens in registers (32-byte reads
 //                      per channel row, 128-byte warp stores per output row).
 //   conv4_tile_kernel  other prefill lengths: a CTA transposes a [64 channel][128 token] tile
-//                      through shared memory: 16-byte coalesced reads along tokens (the input is
-//                      channel-major), 128-byte coalesced writes along channels (the output is
-//                      token-major).  HBM-bound: 2 B read + 2 B written per channel-token.
+//                      through shared memory: 16-byte reads along tokens (the input is channel-major),
+//                      128-byte coalesced writes along channels (the output is token-major).  The rows of a
+//                      length that is no multiple of 8 start anywhere: they are read as the aligned 16-byte
+//                      pieces that cover them (2-byte loads, 32 per thread, before: 6.5 us for 37 tokens x 24,576
+//                      channels).  HBM-bound: 2 B read + 2 B written per channel-token.
 //   conv_generic_kernel decode and every other case (any K <= 16, history, ragged shapes): one
 //                      thread per channel; with seqlen = 1 its accesses are contiguous in channels.
 #include "hk_common.cuh"
@@ -20,12 +22,12 @@ namespace hk {
 constexpr int CONV_MAX_K = 16;
 constexpr int CT_CH = 64;       // channels per tile
 constexpr int CT_TOK = 128;     // tokens per tile
-constexpr int CT_STRIDE = 138;  // bf16 elements per shared row: 8 halo slots + 128 tokens + 2 pad
-                                // (69 words, odd, so channel-strided reads spread over the banks)
+constexpr int CT_STRIDE = 146;  // bf16 elements per shared row: 8 halo slots + 17 pieces of 8 + 2 pad
+                                // (73 words, odd, so channel-strided reads spread over the banks)
 
 __device__ __forceinline__ float silu_fast(float a) { return a * (1.0f / (1.0f + __expf(-a))); }
 
-template <bool ACT, bool VEC>
+template <bool ACT>
 __global__ __launch_bounds__(256) void conv4_tile_kernel(
     const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ state,
     const int* __restrict__ slots, const __nv_bfloat16* __restrict__ weight,
@@ -38,28 +40,31 @@ __global__ __launch_bounds__(256) void conv4_tile_kernel(
   const int tid = threadIdx.x;
   const __nv_bfloat16* xb = x + ((size_t)b * dim + d0) * seqlen;
 
-  // ---- stage the tile: rows = channels, 8 tokens per 16-byte load ----
-  if (VEC) {
-    for (int idx = tid; idx < CT_CH * (CT_TOK / 8); idx += 256) {
-      int r = idx >> 4, c = idx & 15;
-      int s = s0 + c * 8;
-      if (s < seqlen) {
-        uint4 v = ld_stream16(xb + (size_t)r * seqlen + s);
-        uint32_t* dst = reinterpret_cast<uint32_t*>(xs + r * CT_STRIDE + 8 + c * 8);
-        dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
-      }
-    }
-  } else {
-    for (int idx = tid; idx < CT_CH * CT_TOK; idx += 256) {
-      int r = idx >> 7, c = idx & 127;
-      int s = s0 + c;
-      if (s < seqlen) xs[r * CT_STRIDE + 8 + c] = xb[(size_t)r * seqlen + s];
+  pdl_wait();
+  // ---- stage the tile: rows = channels.  Piece c of row r covers tokens s0 - lead + 8 c ..., lead = elements between the
+  //      16-byte boundary and token s0 of that row; token s sits in column 8 + lead + (s - s0).  Pieces that reach over an
+  //      end of the row or of the tile are copied element by element. ----
+  const int s_end = min(seqlen, s0 + CT_TOK);
+  auto row_lead = [&](int r) { return (int)((reinterpret_cast<uintptr_t>(xb + (size_t)r * seqlen + s0) & 15) >> 1); };
+  for (int idx = tid; idx < CT_CH * 17; idx += 256) {
+    const int r = idx / 17, c = idx - r * 17;
+    const __nv_bfloat16* src = xb + (size_t)r * seqlen;
+    const int s = s0 - row_lead(r) + 8 * c;
+    __nv_bfloat16* dst = xs + r * CT_STRIDE + 8 + c * 8;
+    if (s >= s0 && s + 8 <= s_end) {
+      const uint4 v = ld_stream16(src + s);
+      uint32_t* d4 = reinterpret_cast<uint32_t*>(dst);
+      d4[0] = v.x; d4[1] = v.y; d4[2] = v.z; d4[3] = v.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        if (s + e >= s0 && s + e < s_end) dst[e] = src[s + e];
     }
   }
   // ---- halo (3 tokens before the tile) and, in the first tile, the state update ----
   if (tid < CT_CH) {
     const int r = tid;
-    __nv_bfloat16* hrow = xs + r * CT_STRIDE + 5;
+    __nv_bfloat16* hrow = xs + r * CT_STRIDE + 5 + row_lead(r);
     if (s0 == 0) {
       const int slot = slots ? slots[b] : b;
       __nv_bfloat16* st = state + ((size_t)slot * dim + d0 + r) * state_size;
@@ -78,7 +83,7 @@ __global__ __launch_bounds__(256) void conv4_tile_kernel(
   }
   __syncthreads();
 
-  // ---- compute: lane owns 2 adjacent channels, warp owns 16 consecutive tokens ----
+  // ---- compute: lane owns 2 adjacent channels; the warps share the tile's tokens evenly (16 each in a whole tile) ----
   const int lane = tid & 31, wid = tid >> 5;
   const int c0 = lane * 2;
   const uint4 wv = *reinterpret_cast<const uint4*>(weight + (size_t)(d0 + c0) * 4);
@@ -89,15 +94,14 @@ __global__ __launch_bounds__(256) void conv4_tile_kernel(
     b0 = __bfloat162float(bias[d0 + c0]);
     b1 = __bfloat162float(bias[d0 + c0 + 1]);
   }
-  const __nv_bfloat16* r0 = xs + c0 * CT_STRIDE + 8;
-  const __nv_bfloat16* r1 = r0 + CT_STRIDE;
-  const int t0 = wid * 16;
+  const __nv_bfloat16* r0 = xs + c0 * CT_STRIDE + 8 + row_lead(c0);
+  const __nv_bfloat16* r1 = xs + (c0 + 1) * CT_STRIDE + 8 + row_lead(c0 + 1);
+  const int n_tok = s_end - s0, per = (n_tok + 7) >> 3, t0 = wid * per;
   float a0 = __bfloat162float(r0[t0 - 3]), a1 = __bfloat162float(r0[t0 - 2]), a2 = __bfloat162float(r0[t0 - 1]);
   float e0 = __bfloat162float(r1[t0 - 3]), e1 = __bfloat162float(r1[t0 - 2]), e2 = __bfloat162float(r1[t0 - 1]);
   __nv_bfloat16* ob = out + ((size_t)b * seqlen) * dim + d0 + c0;
 #pragma unroll 4
-  for (int t = t0; t < t0 + 16; t++) {
-    if (s0 + t >= seqlen) break;
+  for (int t = t0; t < min(t0 + per, n_tok); t++) {
     float a3 = __bfloat162float(r0[t]), e3 = __bfloat162float(r1[t]);
     float y0 = fmaf(w03, a3, fmaf(w02, a2, fmaf(w01, a1, fmaf(w00, a0, b0))));
     float y1 = fmaf(w13, e3, fmaf(w12, e2, fmaf(w11, e1, fmaf(w10, e0, b1))));
@@ -129,6 +133,7 @@ __global__ __launch_bounds__(256) void conv4_row_kernel(
   const int c0 = blockIdx.x * CT_CH + lane * 2;
   const int t0 = (blockIdx.y * 8 + wid) * NT;
   const int b = blockIdx.z;
+  pdl_wait();
   if (t0 >= seqlen) return;                                  // warp-uniform
   const __nv_bfloat16* r0 = x + ((size_t)b * dim + c0) * seqlen;
   const __nv_bfloat16* r1 = r0 + seqlen;
@@ -200,6 +205,7 @@ __global__ __launch_bounds__(256) void conv_generic_kernel(
     const int* __restrict__ slots, const __nv_bfloat16* __restrict__ weight,
     const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, int dim, int seqlen,
     int state_size, int K) {
+  pdl_wait();
   const int d = blockIdx.x * 256 + threadIdx.x;
   if (d >= dim) return;
   const int b = blockIdx.y;
@@ -256,19 +262,22 @@ __global__ __launch_bounds__(256) void conv_generic_kernel(
 // and walks CR_TOK consecutive tokens with the three previous inputs in registers.  Inputs are rounded
 // to bf16 first, so the result equals transpose-cast followed by the channel-major convolution, bit for
 // bit.  x [bsz][seqlen][dim] f32, out [bsz][seqlen][dim] bf16, state [slots][dim][4] bf16.
-constexpr int CR_TOK = 64;
+// 64 tokens per thread, 16 in short calls: 1,003 tokens x 12,288 channels gave 384 CTAs of 64, eight round trips to memory in a
+// row each (22 us); while 64-token CTAs do not fill every slot of the GPU, more and shorter ones hide more of it.
+constexpr int CR_TOK = 64, CR_TOK_SHORT = 16;
 
 __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-template <bool ACT>
+template <bool ACT, int TOK>
 __global__ __launch_bounds__(128) void conv4_cast_rows_kernel(
     const float* __restrict__ x, __nv_bfloat16* __restrict__ state, const int* __restrict__ slots,
     const __nv_bfloat16* __restrict__ weight, const __nv_bfloat16* __restrict__ bias,
     __nv_bfloat16* __restrict__ out, int dim, int seqlen) {
+  pdl_wait();
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (c >= dim) return;
-  const int s0 = blockIdx.y * CR_TOK, b = blockIdx.z;
-  const int s1 = min(s0 + CR_TOK, seqlen);
+  const int s0 = blockIdx.y * TOK, b = blockIdx.z;
+  const int s1 = min(s0 + TOK, seqlen);
   const float* xb = x + (size_t)b * seqlen * dim + c;
   float w[4][4], bs[4] = {0.f, 0.f, 0.f, 0.f};
   {
@@ -354,15 +363,15 @@ HK_API int hk_kda_cast_conv(const float* x, void* conv_state, const int* slots, 
   HK_REQUIRE(bsz > 0 && bsz <= 65535 && dim > 0 && dim % 4 == 0 && seqlen > 0);
   HK_REQUIRE((seqlen + CR_TOK - 1) / CR_TOK <= 65535);
   HK_REQUIRE(aligned(x, 16) && aligned(conv_state, 16) && aligned(weight, 16) && aligned(out, 8));
-  dim3 grid((dim / 4 + 127) / 128, (seqlen + CR_TOK - 1) / CR_TOK, bsz);
-  auto st = (__nv_bfloat16*)conv_state;
-  auto w = (const __nv_bfloat16*)weight;
-  auto bs = (const __nv_bfloat16*)bias;
-  auto o = (__nv_bfloat16*)out;
-  if (activation) conv4_cast_rows_kernel<true><<<grid, 128, 0, as_stream(stream)>>>(x, st, slots, w, bs, o, dim, seqlen);
-  else            conv4_cast_rows_kernel<false><<<grid, 128, 0, as_stream(stream)>>>(x, st, slots, w, bs, o, dim, seqlen);
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  const int groups = (dim / 4 + 127) / 128;
+  const bool brief = (int64_t)groups * ((seqlen + CR_TOK - 1) / CR_TOK) * bsz < (int64_t)sm_count() * 12;
+  const int tok = brief ? CR_TOK_SHORT : CR_TOK;
+  auto kern = activation ? (brief ? conv4_cast_rows_kernel<true, CR_TOK_SHORT> : conv4_cast_rows_kernel<true, CR_TOK>)
+                         : (brief ? conv4_cast_rows_kernel<false, CR_TOK_SHORT> : conv4_cast_rows_kernel<false, CR_TOK>);
+  return pdl_launch(kern, dim3(groups, (seqlen + tok - 1) / tok, bsz), dim3(128), 0, as_stream(stream), x, (__nv_bfloat16*)conv_state,
+                    slots, (const __nv_bfloat16*)weight, (const __nv_bfloat16*)bias, (__nv_bfloat16*)out, dim, seqlen) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 HK_API int hk_conv1d_update(const void* x, void* conv_state, const int* slots, const void* weight,
@@ -381,32 +390,20 @@ HK_API int hk_conv1d_update(const void* x, void* conv_state, const int* slots, c
 
   const bool tile_ok = (K == 4) && !history && (dim % CT_CH == 0) && seqlen >= 16 &&
                        aligned(weight, 16) && aligned(out, 4);
+  cudaError_t e;
   if (tile_ok && seqlen % 16 == 0 && aligned(x, 16)) {
     // one 16-token group per lane: two groups (NG = 2) measured slower (419 vs 367 us at 32K tokens), fewer warps per SM
-
-    dim3 grid(dim / CT_CH, (seqlen + CT_TOK - 1) / CT_TOK, bsz);
-    if (activation) conv4_row_kernel<true, 1><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size);
-    else            conv4_row_kernel<false, 1><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size);
+    const dim3 grid(dim / CT_CH, (seqlen + CT_TOK - 1) / CT_TOK, bsz);
+    e = pdl_launch(activation ? conv4_row_kernel<true, 1> : conv4_row_kernel<false, 1>, grid, dim3(256), 0, s, xs, st, slots, w, bs, o, dim,
+                   seqlen, state_size);
   } else if (tile_ok) {
-    dim3 grid(dim / CT_CH, (seqlen + CT_TOK - 1) / CT_TOK, bsz);
-    const bool vec = (seqlen % 8 == 0) && aligned(x, 16);
-    if (activation) {
-      if (vec) conv4_tile_kernel<true, true><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size);
-      else     conv4_tile_kernel<true, false><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size);
-    } else {
-      if (vec) conv4_tile_kernel<false, true><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size);
-      else     conv4_tile_kernel<false, false><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size);
-    }
+    const dim3 grid(dim / CT_CH, (seqlen + CT_TOK - 1) / CT_TOK, bsz);
+    e = pdl_launch(activation ? conv4_tile_kernel<true> : conv4_tile_kernel<false>, grid, dim3(256), 0, s, xs, st, slots, w, bs, o, dim,
+                   seqlen, state_size);
   } else {
-    dim3 grid((dim + 255) / 256, bsz);
-    if (activation) {
-      if (history) conv_generic_kernel<true, true><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size, K);
-      else         conv_generic_kernel<true, false><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size, K);
-    } else {
-      if (history) conv_generic_kernel<false, true><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size, K);
-      else         conv_generic_kernel<false, false><<<grid, 256, 0, s>>>(xs, st, slots, w, bs, o, dim, seqlen, state_size, K);
-    }
+    auto kern = activation ? (history ? conv_generic_kernel<true, true> : conv_generic_kernel<true, false>)
+                           : (history ? conv_generic_kernel<false, true> : conv_generic_kernel<false, false>);
+    e = pdl_launch(kern, dim3((dim + 255) / 256, bsz), dim3(256), 0, s, xs, st, slots, w, bs, o, dim, seqlen, state_size, K);
   }
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  return e == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }

@@ -21,6 +21,7 @@ constexpr int TT = 64;
 __global__ void __launch_bounds__(256) transpose_cast_kernel(const float* __restrict__ src,
                                                              __nv_bfloat16* __restrict__ dst, int S, int F) {
   __shared__ float tile[TT][TT + 1];
+  pdl_wait();
   const int s0 = blockIdx.y * TT, f0 = blockIdx.x * TT;
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
   float v[16];
@@ -58,6 +59,7 @@ __global__ void __launch_bounds__(256) gate_kernel(const float* __restrict__ b, 
                                                    const float* __restrict__ a_log, float lb,
                                                    __nv_bfloat16* __restrict__ beta, float* __restrict__ g,
                                                    size_t n_quads, int HD4, int Dk4, size_t n_beta) {
+  pdl_wait();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (size_t i0 = first; i0 < n_quads; i0 += 4 * stride) {
@@ -92,6 +94,7 @@ __global__ void __launch_bounds__(256) gate_scalar_kernel(const float* __restric
                                                           const float* __restrict__ a_log, float lb,
                                                           __nv_bfloat16* __restrict__ beta, float* __restrict__ g,
                                                           size_t n, int HD, int Dk, size_t n_beta) {
+  pdl_wait();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (size_t i = first; i < n; i += stride) {
@@ -138,6 +141,7 @@ template <typename W, typename Y, typename G, int ROWS, bool TWO>
 __global__ void __launch_bounds__(256, 3) gated_rms_norm_warp_kernel(
     const __nv_bfloat16* __restrict__ x, const W* __restrict__ w, Y* __restrict__ y, const G* __restrict__ g,
     float eps, long long rows, int dim, float cbias, int w_groups, int gate_first, int gate_act) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long step = (((long long)gridDim.x * blockDim.x) >> 5) * ROWS;
@@ -205,6 +209,7 @@ __global__ void __launch_bounds__(1024) gated_rms_norm_block_kernel(
     const __nv_bfloat16* __restrict__ x, const W* __restrict__ w, Y* __restrict__ y, const G* __restrict__ g,
     float eps, int dim, float cbias, int w_groups, int gate_first, int gate_act) {
   __shared__ float sums[32];
+  pdl_wait();
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const size_t row = blockIdx.x;
   const int columns = dim >> 2;
@@ -247,18 +252,15 @@ int launch_gated_rms_norm(const void* x, const void* w, void* y, const void* g, 
     const long long ctas_needed = (warps_needed + 7) / 8;
     const long long cap = (long long)sm_count() * 3;       // resident CTAs only: every warp streams many row sets
     const int grid = (int)(ctas_needed < cap ? ctas_needed : cap);
-    if (dim <= 128)
-      gated_rms_norm_warp_kernel<W, Y, G, 4, false><<<grid, 256, 0, st>>>(xp, wp, yp, gp, eps, rows, dim, cbias,
-                                                                         w_groups, gate_first, gate_act);
-    else
-      gated_rms_norm_warp_kernel<W, Y, G, 2, true><<<grid, 256, 0, st>>>(xp, wp, yp, gp, eps, rows, dim, cbias,
-                                                                        w_groups, gate_first, gate_act);
-  } else {
-    gated_rms_norm_block_kernel<W, Y, G><<<(unsigned)rows, 1024, 0, st>>>(xp, wp, yp, gp, eps, dim, cbias, w_groups,
-                                                                          gate_first, gate_act);
+    auto kern = dim <= 128 ? gated_rms_norm_warp_kernel<W, Y, G, 4, false> : gated_rms_norm_warp_kernel<W, Y, G, 2, true>;
+    return pdl_launch(kern, dim3(grid), dim3(256), 0, st, xp, wp, yp, gp, eps, rows, dim, cbias, w_groups, gate_first, gate_act) == cudaSuccess
+               ? HK_OK
+               : HK_ERR_CUDA;
   }
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  return pdl_launch(gated_rms_norm_block_kernel<W, Y, G>, dim3((unsigned)rows), dim3(1024), 0, st, xp, wp, yp, gp, eps, dim, cbias,
+                    w_groups, gate_first, gate_act) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 }  // namespace
@@ -270,9 +272,10 @@ HK_API int hk_kda_transpose_cast(void* dst_bf16, const float* src, int S, int F,
   HK_REQUIRE((F + hk::TT - 1) / hk::TT <= 2147483647 && (S + hk::TT - 1) / hk::TT <= 65535);
   HK_REQUIRE(hk::aligned(dst_bf16, 4));
   dim3 grid((F + hk::TT - 1) / hk::TT, (S + hk::TT - 1) / hk::TT);
-  hk::transpose_cast_kernel<<<grid, 256, 0, hk::as_stream(stream)>>>(src, static_cast<__nv_bfloat16*>(dst_bf16), S, F);
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  return hk::pdl_launch(hk::transpose_cast_kernel, grid, dim3(256), 0, hk::as_stream(stream), src, static_cast<__nv_bfloat16*>(dst_bf16),
+                        S, F) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 HK_API int hk_kda_gate(const float* b, const float* f, const float* dt_bias, const float* a_log,
@@ -285,14 +288,13 @@ HK_API int hk_kda_gate(const float* b, const float* f, const float* dt_bias, con
   const size_t items = vec ? n / 4 : n;
   const size_t want = (items + 255) / 256, cap = (size_t)hk::sm_count() * 32;
   const int grid = (int)(want < cap ? want : cap);
-  if (vec)
-    hk::gate_kernel<<<grid, 256, 0, hk::as_stream(stream)>>>(b, f, dt_bias, a_log, lower_bound, beta, g, n / 4,
-                                                             H * Dk / 4, Dk / 4, n_beta);
-  else
-    hk::gate_scalar_kernel<<<grid, 256, 0, hk::as_stream(stream)>>>(b, f, dt_bias, a_log, lower_bound, beta, g, n,
-                                                                    H * Dk, Dk, n_beta);
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  cudaStream_t st = hk::as_stream(stream);
+  const cudaError_t e =
+      vec ? hk::pdl_launch(hk::gate_kernel, dim3(grid), dim3(256), 0, st, b, f, dt_bias, a_log, lower_bound, beta, g, n / 4, H * Dk / 4,
+                           Dk / 4, n_beta)
+          : hk::pdl_launch(hk::gate_scalar_kernel, dim3(grid), dim3(256), 0, st, b, f, dt_bias, a_log, lower_bound, beta, g, n, H * Dk,
+                           Dk, n_beta);
+  return e == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 
 HK_API int hk_kda_prepare(const float* qkv, const float* b, const float* f, const float* dt_bias,
