@@ -188,16 +188,9 @@ __global__ __launch_bounds__(AB_THREADS, 1) void absorb_gemm_tc_kernel(
 // (q) or 64 (o) CTAs of 128-row tiles whose two-stage ring has at most 96 KB in flight, on 64 SMs for o: 7.8 and 10.5 us.
 // Here the WEIGHTS are the M operand, 64 output columns per CTA (512 and 256 CTAs, all resident), the rows are N (8 to 32),
 // and a CTA requests its whole K at once (32 / 64 KB, a barrier per 64-channel chunk): no ring, no empty barriers.
-// As a programmatic dependent it pulls its weights into L2 while the kernel before it still runs.
 // ------------------------------------------------------------------------------------------------
 constexpr int AF_BM = 64, AF_BK = 64, AF_MAX_ROWS = 32, AF_THREADS = 128;
 constexpr uint32_t AF_A_CHUNK = AF_BM * AF_BK * 2;            // 8 KB
-
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* tmap, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(tmap)),
-               "r"(x), "r"(y)
-               : "memory");
-}
 
 // W_MN: weights [k][n] with n contiguous, else [n][k].  nb = rows rounded up to 8 (box rows of tmap_x).
 template <bool W_MN, int K>
@@ -216,13 +209,9 @@ __global__ __launch_bounds__(AF_THREADS) void absorb_few_rows_kernel(const __gri
   const int warp = tc::warp_index_uniform();
   const int n0 = blockIdx.x * AF_BM, h = blockIdx.y;
   const uint32_t x_chunk = (uint32_t)nb * AF_BK * 2;
-  pdl_trigger();
   const int wy = h * w_rows_per_head + w_row_off + (W_MN ? 0 : n0);
   if (tid == 0) {
-    for (int kc = 0; kc < NK; kc++) {
-      tma_prefetch_2d(&tmap_w, W_MN ? n0 : kc * AF_BK, wy + (W_MN ? kc * AF_BK : 0));
-      tc::mbar_init(&full_bar[kc], 1);
-    }
+    for (int kc = 0; kc < NK; kc++) tc::mbar_init(&full_bar[kc], 1);
     tc::mbar_init(&done_bar, 1);
     tc::mbar_fence_init();
     abort_flag = 0;

@@ -216,7 +216,6 @@ __device__ __forceinline__ void topk_row(const uint16_t* row, const TopkSink row
 __global__ __launch_bounds__(TK_THREADS) void dsa_topk_kernel(
     const uint16_t* scores, int* __restrict__ out, int T, int s_stride, int k,
     int k_pad, const int* __restrict__ t_ptr, int t_seq, int* __restrict__ raw, const int* __restrict__ q_pos) {
-  pdl_trigger();
   pdl_wait();
   if (t_ptr) T = t_seq > 0 ? t_ptr[blockIdx.x / t_seq] : *t_ptr;
   TopkSink sink{out + (size_t)blockIdx.x * k_pad,
@@ -263,7 +262,6 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
     const uint16_t* scores, int* __restrict__ out, int T, int s_stride, int k, int k_pad,
     int* __restrict__ raw, const int* __restrict__ q_pos) {
   namespace cg = cooperative_groups;
-  pdl_trigger();
   pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int c = (int)cluster.block_rank();

@@ -50,15 +50,16 @@ inline int sm_count() {
 }
 
 // ---- programmatic dependent launch ----
-// The small kernels of a decode step take 2-10 us each, of which 1-2 us are the drain of one grid and the start of the
-// next.  They are launched with programmatic stream serialisation: a kernel calls pdl_trigger() at entry, so that the next
-// one's CTAs are placed while it runs, and pdl_wait() before its first access to memory that an earlier kernel may have
-// written (or may still read).  EVERY kernel launched this way executes pdl_wait() in every CTA: the wait covers the grid
-// before it only, and the chain of waits is what orders a kernel behind all earlier ones.  Ahead of the wait a kernel may set
-// up barriers and tensor memory and prefetch into L2, which stays coherent; it may not load or store anything.
-// Behind a kernel that never triggers the attribute changes nothing.
+// The small kernels of a decode step take 2-10 us each, and a plain launch behind a running kernel adds 1-2 us to each.  They
+// are launched with programmatic stream serialisation and wait (pdl_wait) before their first access to memory that an earlier
+// kernel may have written or may still read: the launch itself is over when the kernel before them ends.  EVERY kernel
+// launched this way executes pdl_wait() in every CTA: the wait covers the grid before it only, and the chain of waits is what
+// orders a kernel behind all earlier ones.
+// No kernel releases its dependents early (griddepcontrol.launch_dependents): CTAs placed beside a running grid land where
+// that grid left room, not evenly - the per-token KDA kernel behind the convolution took twice as long - and the decode
+// chains gained nothing (MLA layer of one token 39.7 us with, 39.2 without; selection + attention 26.8 / 25.9).
+// Launches of many waves are plain: as programmatic dependents the convolution of 32K tokens took 495 us instead of 362.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>
 inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
@@ -71,7 +72,7 @@ inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = (int64_t)grid.x * grid.y * grid.z <= 8 * sm_count() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 

@@ -165,7 +165,6 @@ __global__ __launch_bounds__(128) void indexer_tc_decode_kernel(
   __shared__ int abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = lane >> 4, chunk = lane & 15;    // a warp instruction covers 2 rows x 16 chunks
-  pdl_trigger();
 
   if (tid == 0) {
     tc::mbar_init(&bar, 1);
@@ -173,11 +172,6 @@ __global__ __launch_bounds__(128) void indexer_tc_decode_kernel(
     abort_flag = 0;
   }
   if (warp == 0) tc::tmem_alloc(&tmem_slot, tmem_cols);
-  // this CTA's first key tile on its way into L2 while the kernel before this one finishes
-  if (tid == 0) {
-    const int p0 = blockIdx.x * IX_TILE_P;
-    tc::prefetch_l2(pk + (size_t)p0 * IDX_DIM, (uint32_t)min(IX_TILE_P, npools - p0) * IDX_DIM * 2);
-  }
   pdl_wait();
   // query rows -> B operand
   for (int r2 = warp; r2 < nb / 2; r2 += 4) {

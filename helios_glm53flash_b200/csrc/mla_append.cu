@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(128) mla_decode_prologue_kernel(
     __half* __restrict__ pk_nt, const float* __restrict__ ape, int pos, int* __restrict__ q_pos_out) {
   __shared__ __half s_kn[128];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  pdl_trigger();
   pdl_wait();
   if (warp == 0) append_row(kv_pre, ln_w, ckv + (size_t)pos * LATENT, nullptr, eps_rms, lane);
   if (warp == 1) layernorm_row(idx_k, knorm_w, knorm_b, idx_kn, s_kn, 128, eps_ln, lane);

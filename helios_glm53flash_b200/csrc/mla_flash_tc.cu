@@ -143,7 +143,6 @@ __global__ __launch_bounds__(G4 ? FT_G4_THREADS : FT_THREADS, 1) void mla_flash_
   const int warp_u = tc::warp_index_uniform();
   const bool mma_warp = warp_u == 4 || warp_u == 12;   // 4 issues S = Q K^T, 12 issues O^T += V^T P^T
   const int sp = blockIdx.x, r = blockIdx.y;
-  pdl_trigger();
   pdl_wait();
   FT_CTA_STAMP(0);
   if (tid == 0) FT_TRACE(13, 0);                      // kernel entry
