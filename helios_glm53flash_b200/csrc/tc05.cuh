@@ -333,6 +333,32 @@ __device__ __forceinline__ void mma_f16_if(uint32_t leader, uint32_t d_tmem, uin
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
       : "memory");
 }
+// ---- weight-stationary form (M = 64 over all 128 lanes) ----
+// A plain M = 64 product uses 64 of the 128 lanes and takes N / 2 cycles.  The .ws form puts columns 0 .. N/2 - 1 of rows 0-63
+// into lanes 0-63 and columns N/2 .. N - 1 into lanes 64-127 and takes N / 4 plus about 12 cycles, or the time shared memory
+// needs for its operands at 128 B per cycle.  Measured per K16 step: operands in shared memory N 64 32, N 128 48, N 256 80
+// cycles; A in tensor memory 28, 44, 76.  A in tensor memory (64 rows, two fp16 per column) must sit in lanes 0-63 AND in
+// lanes 64-127: the two halves of the array read their own copy.  N is 64, 128 or 256.
+__device__ __forceinline__ void mma_ws_f16_if(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.ws.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ws_f16_tmem_a_if(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                                     bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.ws.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
+      : "memory");
+}
 __device__ __forceinline__ void mma_commit_if(uint32_t leader, uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"

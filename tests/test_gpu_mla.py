@@ -94,6 +94,46 @@ def test_dense_batched_decode_over_concatenated_caches():
     assert max_rel(synth.f16_bits_to_f32(bits(out)), o32) < TOL
 
 
+@pytest.mark.parametrize("n_split", [1, 4])
+def test_attention_at_the_edges_of_the_key_tiles(n_split):
+    """key counts either side of 64-key tiles and of the three tiles in flight: dense rows whose range is followed by NaN rows
+    that must not be touched, and gathered rows with holes, a whole tile of them first; maxima that move late (rescale)"""
+    lens = np.array([1, 15, 63, 64, 65, 127, 128, 129, 191, 192, 193, 257, 0], dtype=np.int32)
+    B, L = len(lens), 300
+    inp = synth.mla_inputs(B * L, B, seed=91, cache_std=0.5)
+    ckv = synth.f16_bits_to_f32(inp["ckv"]).reshape(B, L, 512)
+    ckv[:, 100:] *= 8.0                                             # scores of later keys beat the first tiles' by far
+    for i, n in enumerate(lens):
+        ckv[i, n:] = np.nan
+    bad = synth.f32_to_f16_bits(ckv.reshape(B * L, 512))
+    clean = synth.f32_to_f16_bits(np.nan_to_num(ckv).reshape(B * L, 512))
+    base = (np.arange(B) * L).astype(np.int64)
+    _, o32 = orc.mla_attend(inp["q_lat"], clean, B, 64, 0.0625, kv_base=base, kv_len=lens)
+    out = torch.empty(B, 64, 512, dtype=torch.float16, device="cuda")
+    hk.mla_dense_prefill(dev_f16(inp["q_lat"]), dev_f16(bad), out, B, 0, kv_base=dev(base), kv_len=dev(lens), n_keys_hint=L, n_split=n_split)
+    torch.cuda.synchronize()
+    assert hk.read_device_status() == 0
+    g = synth.f16_bits_to_f32(bits(out))
+    for i in range(B):
+        assert max_rel(g[i], o32[i]) < TOL if lens[i] else (g[i] == 0).all(), lens[i]
+    for kidx in (1, 63, 64, 65, 130, 192, 200):
+        r = np.random.RandomState(kidx)
+        ridx = r.randint(0, B * L, (B, kidx)).astype(np.int32)
+        ridx[:, ::5] = -1
+        ridx[3, :64] = -1
+        ridx[4] = -1
+        ridx[5, -1] = B * L                                         # behind the cache: a hole
+        want = ridx.copy()
+        want[5, -1] = -1
+        _, o32 = orc.mla_attend(inp["q_lat"], clean, B, 64, 0.0625, raw_idx=want, kidx=kidx)
+        hk.mla_sparse_decode(dev_f16(inp["q_lat"]), dev_f16(clean), dev(ridx), kidx, out, B, n_split=n_split)
+        torch.cuda.synchronize()
+        assert hk.read_device_status() == 0
+        g = synth.f16_bits_to_f32(bits(out))
+        for i in range(B):
+            assert max_rel(g[i], o32[i]) < TOL if (want[i] >= 0).any() else (g[i] == 0).all(), (kidx, i)
+
+
 def test_partials_and_combine_vs_oracle():
     m, L, S = 2, 900, 3
     inp = synth.mla_inputs(L, m, seed=21, cache_std=0.5)
