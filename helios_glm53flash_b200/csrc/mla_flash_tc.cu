@@ -26,6 +26,11 @@
 // with ONE TMA tensor copy each (3-D box {64 channels, 64 keys, 8 blocks}); gathered rows, and the last tile of a ragged
 // dense range, as gather4 copies (four cache rows x one 64-channel block each, 128 per tile; a negative row number reads as
 // zeros, so nothing behind the range is read).
+//
+// Many gathered rows (prefill) run on a persistent grid, one CTA per SM that walks rows: a row's own costs - its first loads,
+// Q into tensor memory, O out - were 14 K cycles of the 75 K of 2,052 keys.  Here the next row's Q and keys come through the
+// ring while the current row is in its last tiles, Q is a pseudo-tile of the ring that the softmax warps move while
+// the row's last P V runs, and O leaves through the P buffers.
 // All hand-offs are mbarriers with bounded waits, executed by every lane of the waiting warp.
 #include <cuda.h>   // CUtensorMap (types only; the encoder is fetched through the runtime at first use)
 
@@ -50,29 +55,57 @@ constexpr uint32_t FP_BYTES = FT_HEADS * FT_KEYS * 2;
 constexpr uint32_t FS_MISC = FS_P + 2 * FP_BYTES;
 constexpr uint32_t FS_SMEM = FS_MISC + 2048 + 1024;        // + slack to align the base to 1 KB (swizzle atoms)
 constexpr uint32_t FT_O = 0, FT_S = 256, FT_Q = 320;       // tensor-memory columns: O 2 x 128, S 2 x 32, Q 192
-constexpr uint32_t FT_QPITCH = (LATENT - FT_QS) * 2 + 16;  // row pitch of the staged queries: conflict-free 16-byte rows
 constexpr int FT_POLL_NS = 40;                    // poll back-off of the waiting warps
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_THRESHOLD = 8.0f;         // log2 units: P stays below 2^8, fine for fp16
-// warps 0-3 softmax and epilogue (one TMEM lane quarter each), 4 issues S = Q K^T, 5 issues O += P V, the rest load tiles.
-// A warp gets one gather4 copy out per about 90 cycles whichever lanes issue them: eight warps for gathered rows; dense
-// ranges need them for the ragged last tile only.
+// warps 0-3 softmax, Q into tensor memory and epilogue (a TMEM lane quarter each), 4 issues S = Q K^T, 5 issues O += P V, the
+// others load tiles (dense ranges need more than one only for the ragged last tile).
 template <bool G4>
 struct FtRoles {
-  static constexpr int LOAD_WARPS = G4 ? 8 : 4, THREADS = (6 + LOAD_WARPS) * 32, COPIES = 128 / LOAD_WARPS;
+  static constexpr int LOAD_WARPS = 4, THREADS = (6 + LOAD_WARPS) * 32, SLOTS = FT_KEYS / LOAD_WARPS;   // key slots per loader warp
 };
 
 struct FtMisc {
-  uint64_t k_full[FT_NBUF], t_done[FT_NBUF];      // per tile buffer: tile landed, its P V finished
-  uint64_t s_full[2], s_free[2], p_full[2];       // per S / P buffer
-  uint64_t q_ready;
-  unsigned long long mask[FT_NBUF];               // valid key slots of the tile in the buffer
+  uint64_t full[FT_NBUF], free[FT_NBUF];          // ring slot (a key tile or a row's Q): landed, may be overwritten
+  uint64_t s_full[2], s_free[2], p_full[2], pv_done[2];   // per tile parity
+  uint64_t q_ready, o_free;                       // per row
+  uint8_t mask[FT_NBUF][FT_KEYS / 8];             // valid key slots of the tile in the ring slot
   float mx[2][128];                               // tile maxima, by softmax thread and tile parity
   float l[128];
   uint32_t tmem;
   int abort_flag;
 };
 static_assert(sizeof(FtMisc) <= 2048, "misc area");
+
+// One work item: a row and a key split.
+struct FtItem {
+  int r, sp, k0, k1, n_tiles;
+  int64_t base;
+  __device__ __forceinline__ int keys(int t) const { return min(FT_KEYS, k1 - k0 - t * FT_KEYS); }
+};
+template <bool G4>
+__device__ __forceinline__ FtItem ft_item(const MlaArgs& a, int idx) {
+  FtItem it;
+  it.sp = idx % a.n_split;
+  it.r = idx / a.n_split;
+  // rows of a causal chunk grow with their number: the longest first, so that the CTAs end together
+  if (!G4 && !a.kv_len) it.r = a.m - 1 - it.r;
+  int n;
+  it.base = 0;
+  if (G4) {
+    n = a.kidx;
+  } else {
+    n = a.kv_len ? a.kv_len[it.r] : a.pos_start + it.r + 1;
+    it.base = a.kv_base ? a.kv_base[it.r] : 0;
+    if (a.ckv_rows > 0) n = (int)max((int64_t)0, min((int64_t)n, a.ckv_rows - it.base));   // never past the end of the cache
+  }
+  // split boundaries on tile granularity
+  const int tiles = (n + FT_KEYS - 1) / FT_KEYS, per = (tiles + a.n_split - 1) / a.n_split;
+  it.k0 = min(n, it.sp * per * FT_KEYS);
+  it.k1 = min(n, (it.sp + 1) * per * FT_KEYS);
+  it.n_tiles = (it.k1 - it.k0 + FT_KEYS - 1) / FT_KEYS;
+  return it;
+}
 
 __device__ __forceinline__ void tma_load_tile(void* smem_dst, const CUtensorMap* tmap, int row, uint64_t* bar) {
   asm volatile(
@@ -86,20 +119,26 @@ __device__ __forceinline__ void tma_load_tile(void* smem_dst, const CUtensorMap*
 // [row][512 channels] with a box of {64 channels, 1 row}; the instruction names four row coordinates, the copy engine
 // lays the four 128-byte pieces down one after the other and applies the 128-byte swizzle by destination address, i.e.
 // exactly key slots k .. k+3 of a block of the tile layout.  A negative row is outside the tensor: zero fill.
-__device__ __forceinline__ void tma_gather4_rows(void* smem_dst, const CUtensorMap* tmap, int channel, int r0, int r1, int r2,
-                                                 int r3, uint64_t* bar) {
+// Executed by the whole warp with warp-uniform operands, issued by the lane with leader != 0: the eight copies of a key quad
+// differ in two numbers.  Issued lane by lane (each lane its own copy) a copy cost about 90 cycles of operand moves, 1,440 per
+// warp and tile, and the three-slot ring stood still for them: 2,110 cycles per tile of gathered rows against 1,760 dense.
+__device__ __forceinline__ void tma_gather4_rows(uint32_t leader, uint32_t smem_dst, const CUtensorMap* tmap, int channel, int r0, int r1,
+                                                 int r2, int r3, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(
-          tc::smem_u32(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(channel), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(tc::smem_u32(bar))
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %8, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];\n\t}" ::"r"(
+          smem_dst),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(channel), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(bar), "r"(leader)
       : "memory");
 }
 
-// G4: gathered rows (raw_idx); otherwise dense ranges.  tmap_box: 3-D map of the cache, tmap_rows: 2-D map for gather4.
+// G4: gathered rows (raw_idx); otherwise dense ranges.  tmap_box: 3-D map of the cache, tmap_rows: 2-D map of the cache for
+// gather4, tmap_q: the queries as tmap_box, tmap_o: 2-D map of the final output.
 template <bool G4>
-__global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(MlaArgs a, int* __restrict__ status,
-                                                                               const __grid_constant__ CUtensorMap tmap_box,
-                                                                               const __grid_constant__ CUtensorMap tmap_rows) {
+__global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(
+    MlaArgs a, int* __restrict__ status, const __grid_constant__ CUtensorMap tmap_box, const __grid_constant__ CUtensorMap tmap_rows,
+    const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_o) {
   using R = FtRoles<G4>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -109,155 +148,125 @@ __global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(M
   const int tid = threadIdx.x, lane = tid & 31;
   // provably warp-uniform role index: the issuing warps' branches stay converged for the compiler
   const int warp = tc::warp_index_uniform();
-  pdl_wait();
-  // rows of a causal chunk grow with their number: the longest first, so that the last wave ends together
-  const int sp = blockIdx.x, r = (!G4 && !a.kv_len) ? a.m - 1 - (int)blockIdx.y : (int)blockIdx.y;
-  int n;
-  int64_t base = 0;
-  if (G4) {
-    n = a.kidx;
-  } else {
-    n = a.kv_len ? a.kv_len[r] : a.pos_start + r + 1;
-    base = a.kv_base ? a.kv_base[r] : 0;
-    if (a.ckv_rows > 0) n = (int)max((int64_t)0, min((int64_t)n, a.ckv_rows - base));   // never past the end of the cache
-  }
-  // split boundaries on tile granularity
-  const int tiles_total = (n + FT_KEYS - 1) / FT_KEYS;
-  const int tiles_per = (tiles_total + a.n_split - 1) / a.n_split;
-  const int k0 = min(n, sp * tiles_per * FT_KEYS), k1 = min(n, (sp + 1) * tiles_per * FT_KEYS);
-  const int n_tiles = (k1 - k0 + FT_KEYS - 1) / FT_KEYS;
-  auto tile_keys = [&](int t) { return min(FT_KEYS, k1 - k0 - t * FT_KEYS); };
-  auto whole = [&](int t) { return !G4 && tile_keys(t) == FT_KEYS; };       // arrives as one box
-
+  const int n_items = a.n_split * a.m, step = gridDim.x;
+  // A CTA with one item of at most two tiles (a decode split) never needs Q's ring slot back: S reads Q from there, and the
+  // 0.6 us of moving it are saved.
+  bool direct_q = false;
   if (tid == 0) {
 #pragma unroll
     for (int b = 0; b < FT_NBUF; b++) {
-      tc::mbar_init(&ms.k_full[b], R::LOAD_WARPS);
-      tc::mbar_init(&ms.t_done[b], 1);
+      tc::mbar_init(&ms.full[b], R::LOAD_WARPS);
+      tc::mbar_init(&ms.free[b], 1);
     }
 #pragma unroll
     for (int b = 0; b < 2; b++) {
       tc::mbar_init(&ms.s_full[b], 1);
       tc::mbar_init(&ms.s_free[b], 128);
       tc::mbar_init(&ms.p_full[b], 128);
+      tc::mbar_init(&ms.pv_done[b], 1);
     }
     tc::mbar_init(&ms.q_ready, 128);
+    tc::mbar_init(&ms.o_free, 128);
     tc::mbar_fence_init();
     ms.abort_flag = 0;
-    // The boxes of the first two tiles leave at once and fly while the queries are staged (in the third buffer).  The
-    // byte count is raised without an arrival; the loader warps arrive later like for every tile.
-    for (int t = 0; t < FT_NBUF - 1 && t < n_tiles; t++)
-      if (whole(t)) {
-        tc::mbar_expect_tx(&ms.k_full[t], FT_TILE);
-        tma_load_tile(smem + FS_K + t * FT_TILE, &tmap_box, (int)(base + k0 + t * FT_KEYS), &ms.k_full[t]);
-      }
   }
-  // (not ahead of the barrier set-up and the first copies: there it cost a many-wave launch 4 %)
   if (warp == 0) tc::tmem_alloc(&ms.tmem, 512);
-  if (n_tiles > 0) {
-    // Q: channels 0-127 -> the swizzled A operand, the rest -> rows in the third tile buffer, from where the softmax
-    // threads carry them into tensor memory.  All warps, every load of a thread in flight at once.
-    constexpr int NI = (FT_HEADS * 64 + R::THREADS - 1) / R::THREADS;      // 16-byte pieces per thread
-    const uint4* q = reinterpret_cast<const uint4*>(a.q_lat + (size_t)r * FT_HEADS * LATENT);
-    uint4 qs[NI];
-#pragma unroll
-    for (int u = 0; u < NI; u++) {
-      const int i = tid + u * R::THREADS;
-      if (i < FT_HEADS * 64) qs[u] = q[i];
-    }
-#pragma unroll
-    for (int u = 0; u < NI; u++) {
-      const int i = tid + u * R::THREADS, h = i >> 6, c = i & 63;
-      if (i < FT_HEADS * 64) {
-        uint8_t* dst = c < FT_QS / 8 ? smem + FS_Q + tc::sw128_off(h, c, FT_HEADS * 128)
-                                     : smem + FS_K + (FT_NBUF - 1) * FT_TILE + h * FT_QPITCH + (c - FT_QS / 8) * 16;
-        *reinterpret_cast<uint4*>(dst) = qs[u];
-      }
-    }
-    tc::fence_async_smem();
-  }
+  pdl_wait();
+  if (step >= n_items) direct_q = ft_item<G4>(a, blockIdx.x).n_tiles < FT_NBUF;
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = ms.tmem;
   bool ok = true;
 
+  // Every role walks the same items and counts the same way: u = ring slots used so far, g = key tiles, q = rows with keys.
   if (warp >= 6) {
-    // =========================== loaders: the key tiles ===========================
+    // =========================== loaders: per row its Q, then its key tiles ===========================
     const int lw = warp - 6;
-    // copy u of a tile: key quad u / 8, channel block u % 8
-    const int u0 = lw * R::COPIES + lane;
-    const bool issuer = lane < R::COPIES;
-    auto row_of = [&](int tile, int slot) -> int {         // cache row of a key slot, -1 = hole
-      const int p = k0 + tile * FT_KEYS + slot;
-      if (tile >= n_tiles || p >= k1) return -1;
-      if (!G4) return (int)(base + p);
+    const uint32_t leader = tc::elect_one();
+    // cache row of key slot lw * SLOTS + lane of a tile, -1 = hole; volatile, so that a look-ahead load is issued where it stands
+    auto row_of = [&](const FtItem& it, int tile) -> int {
+      const int p = it.k0 + tile * FT_KEYS + lw * R::SLOTS + lane;
+      if (lane >= R::SLOTS || p >= it.k1) return -1;
+      if (!G4) return (int)(it.base + p);
       int v;
-      asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(a.raw_idx + (size_t)r * a.kidx + p));
+      asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(a.raw_idx + (size_t)it.r * a.kidx + p));
       return v;
     };
     // gathered row numbers beyond the cache are holes
     auto in_cache = [&](int v) -> int { return (v < 0 || (a.ckv_rows > 0 && (int64_t)v >= a.ckv_rows)) ? -1 : v; };
-    // Row numbers are fetched TWO tiles ahead with volatile loads, so that they are issued where they stand and not moved
-    // down to their first use (the row list of a query is read once, from HBM).
-    int qa[4], qb[4], ma[2] = {-1, -1}, mb[2] = {-1, -1};
+    // Gathered row numbers are fetched two tiles ahead (the row list of a query is read once, from HBM), across rows.
+    int cur = -1, nxt = -1, ahead_item = blockIdx.x, ahead_tile = 0;
+    FtItem ahead = ft_item<G4>(a, ahead_item);
+    auto fetch = [&]() -> int {
+      if (!G4 || ahead_item >= n_items || ahead.n_tiles == 0) return -1;   // (gathered rows: every item has the same keys)
+      const int v = row_of(ahead, ahead_tile);
+      if (++ahead_tile == ahead.n_tiles) {
+        ahead_tile = 0;
+        ahead_item += step;
+        if (ahead_item < n_items) ahead = ft_item<G4>(a, ahead_item);
+      }
+      return v;
+    };
     if (G4) {
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        qa[e] = issuer ? row_of(0, (u0 >> 3) * 4 + e) : -1;
-        qb[e] = issuer ? row_of(1, (u0 >> 3) * 4 + e) : -1;
-      }
-      if (lw == 0) {
-#pragma unroll
-        for (int e = 0; e < 2; e++) { ma[e] = row_of(0, 32 * e + lane); mb[e] = row_of(1, 32 * e + lane); }
-      }
+      cur = fetch();
+      nxt = fetch();
     }
-    for (int tile = 0; tile < n_tiles; tile++) {
-      const int buf = tile % FT_NBUF;
-      uint8_t* dst = smem + FS_K + buf * FT_TILE;
-      int rows[4];
-      unsigned long long mask = 0;
-      if (G4) {
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          rows[e] = in_cache(qa[e]);
-          qa[e] = qb[e];
-          qb[e] = issuer ? row_of(tile + 2, (u0 >> 3) * 4 + e) : -1;
-        }
-        if (lw == 0) {
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            mask |= (unsigned long long)__ballot_sync(0xffffffffu, in_cache(ma[e]) >= 0) << (32 * e);
-            ma[e] = mb[e];
-            mb[e] = row_of(tile + 2, 32 * e + lane);
-          }
-        }
-      } else {
-        mask = ~0ull >> (FT_KEYS - tile_keys(tile));
-      }
-      // the buffer is free: its last P V is done; the third buffer held the queries first
-      if (tile >= FT_NBUF) ok = tc::mbar_wait<FT_POLL_NS>(&ms.t_done[buf], (tile / FT_NBUF - 1) & 1, abort_flag, 5) && ok;
-      else if (tile == FT_NBUF - 1) ok = tc::mbar_wait<FT_POLL_NS>(&ms.q_ready, 0, abort_flag, 4) && ok;
-      if (lw == 0 && lane == 0) ms.mask[buf] = mask;
-      if (whole(tile)) {
+    uint32_t u = 0;
+    auto next_slot = [&]() -> int {                        // waits until the slot may be overwritten
+      const int b = u % FT_NBUF;
+      if (u >= FT_NBUF) ok = tc::mbar_wait<FT_POLL_NS>(&ms.free[b], (u / FT_NBUF - 1) & 1, abort_flag, 5) && ok;
+      u++;
+      return b;
+    };
+    for (int idx = blockIdx.x; idx < n_items; idx += step) {
+      const FtItem it = ft_item<G4>(a, idx);
+      if (it.n_tiles == 0) continue;
+      {
+        const int b = next_slot();
         if (lane == 0) {
-          if (lw == 0 && tile >= FT_NBUF - 1) {
-            tc::mbar_arrive_expect_tx(&ms.k_full[buf], FT_TILE);
-            tma_load_tile(dst, &tmap_box, (int)(base + k0 + tile * FT_KEYS), &ms.k_full[buf]);
+          if (lw == 0) {
+            tc::mbar_arrive_expect_tx(&ms.full[b], FT_TILE);
+            tma_load_tile(smem + FS_K + b * FT_TILE, &tmap_q, it.r * FT_HEADS, &ms.full[b]);
           } else {
-            tc::mbar_arrive(&ms.k_full[buf]);            // nothing to add, or the box left at kernel entry
+            tc::mbar_arrive(&ms.full[b]);
           }
         }
-      } else {
-        if (lane == 0) tc::mbar_arrive_expect_tx(&ms.k_full[buf], R::COPIES * 512);
+      }
+      for (int tile = 0; tile < it.n_tiles; tile++) {
+        int row;
+        if (G4) {
+          row = in_cache(cur);
+          cur = nxt;
+          nxt = fetch();
+        } else {
+          row = row_of(it, tile);
+        }
+        const uint32_t valid = __ballot_sync(0xffffffffu, row >= 0);
+        const int b = next_slot();
+        if (lane < R::SLOTS / 8) ms.mask[b][lw * (R::SLOTS / 8) + lane] = (uint8_t)(valid >> (8 * lane));
         __syncwarp();
-        if (issuer) {
-          const int kq = u0 >> 3, blk = u0 & 7;
-          if (!G4) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) rows[e] = row_of(tile, kq * 4 + e);
+        if (!G4 && it.keys(tile) == FT_KEYS) {             // a whole tile of a dense range: one box
+          if (lane == 0) {
+            if (lw == 0) {
+              tc::mbar_arrive_expect_tx(&ms.full[b], FT_TILE);
+              tma_load_tile(smem + FS_K + b * FT_TILE, &tmap_box, (int)(it.base + it.k0 + tile * FT_KEYS), &ms.full[b]);
+            } else {
+              tc::mbar_arrive(&ms.full[b]);
+            }
           }
-          tma_gather4_rows(dst + blk * FT_BLK + kq * 512, &tmap_rows, blk * 64, rows[0], rows[1], rows[2], rows[3], &ms.k_full[buf]);
+        } else {
+          if (lane == 0) tc::mbar_arrive_expect_tx(&ms.full[b], R::SLOTS * LATENT * 2);
+          __syncwarp();
+          const uint32_t dst = tc::smem_u32(smem + FS_K) + b * FT_TILE + lw * R::SLOTS * 128, bar = tc::smem_u32(&ms.full[b]);
+#pragma unroll
+          for (int j = 0; j < R::SLOTS / 4; j++) {
+            const int r0 = __shfl_sync(0xffffffffu, row, 4 * j), r1 = __shfl_sync(0xffffffffu, row, 4 * j + 1);
+            const int r2 = __shfl_sync(0xffffffffu, row, 4 * j + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * j + 3);
+#pragma unroll
+            for (int blk = 0; blk < 8; blk++)
+              tma_gather4_rows(leader, dst + blk * FT_BLK + j * 512, &tmap_rows, blk * 64, r0, r1, r2, r3, bar);
+          }
         }
       }
     }
@@ -273,45 +282,74 @@ __global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(M
       const bool done = tc::mbar_wait<FT_POLL_NS>(bar, parity, abort_flag, code);
       ok = __all_sync(0xffffffffu, done) != 0 && ok;
     };
+    uint32_t u = 0, g = 0, q = 0;
     if (warp == 4) {
       const uint32_t idesc = tc::make_idesc(64, FT_KEYS, tc::FMT_F16, tc::FMT_F16, false, false);
-      const uint64_t qd = tc::make_sdesc_sw128(tc::smem_u32(smem + FS_Q), 16, 1024);
-      if (n_tiles > 0) wait_u(&ms.q_ready, 0, 11);
-      for (int tile = 0; tile < n_tiles; tile++) {
-        const int b = tile & 1, kb = tile % FT_NBUF;
-        wait_u(&ms.k_full[kb], (tile / FT_NBUF) & 1, 1);
-        if (tile >= 2) wait_u(&ms.s_free[b], ((tile - 2) >> 1) & 1, 2);
-        tc::fence_after_sync();
-        // keys as N in 1 KB atoms; 16 channels = 32 B inside the 128-byte row, 64 channels per block
-        const uint64_t kd = tc::make_sdesc_sw128(tc::smem_u32(smem + FS_K + kb * FT_TILE), 16, 1024);
+      // Addresses pass through an empty asm where their descriptors are built: the compiler would otherwise keep 32
+      // loop-invariant descriptors per operand in registers and spill in the softmax loop.
+      auto desc = [](const uint8_t* p) {
+        uint32_t addr = tc::smem_u32(p);
+        asm volatile("" : "+r"(addr));
+        return tc::make_sdesc_sw128(addr, 16, 1024);
+      };
+      for (int idx = blockIdx.x; idx < n_items; idx += step) {
+        const int n_tiles = ft_item<G4>(a, idx).n_tiles;
+        if (n_tiles == 0) continue;
+        if (direct_q) wait_u(&ms.full[0], 0, 15);
+        else wait_u(&ms.q_ready, q & 1, 13);
+        u++;                                               // the row's Q
+        q++;
+        for (int tile = 0; tile < n_tiles; tile++, u++, g++) {
+          const int b = g & 1, kb = u % FT_NBUF;
+          wait_u(&ms.full[kb], (u / FT_NBUF) & 1, 1);
+          if (g >= 2) wait_u(&ms.s_free[b], ((g - 2) >> 1) & 1, 2);
+          tc::fence_after_sync();
+          // keys as N in 1 KB atoms; 16 channels = 32 B inside the 128-byte row, 64 channels per block
+          const uint64_t kd = desc(smem + FS_K + kb * FT_TILE), qd = desc(smem + (direct_q ? FS_K : FS_Q));
+          if (direct_q) {
 #pragma unroll
-        for (int kk = 0; kk < LATENT / 16; kk++) {
-          const uint64_t bd = tc::sdesc_advance(kd, (kk >> 2) * FT_BLK + (kk & 3) * 32);
-          if (kk < FT_QS / 16)
-            tc::mma_ws_f16_if(leader, tmem + FT_S + b * 32, tc::sdesc_advance(qd, (kk >> 2) * (FT_HEADS * 128) + (kk & 3) * 32), bd, idesc, kk > 0);
-          else
-            tc::mma_ws_f16_tmem_a_if(leader, tmem + FT_S + b * 32, tmem + FT_Q + (kk - FT_QS / 16) * 8, bd, idesc, true);
+            for (int kk = 0; kk < LATENT / 16; kk++) {
+              const uint32_t off = (kk >> 2) * FT_BLK + (kk & 3) * 32;
+              tc::mma_ws_f16_if(leader, tmem + FT_S + b * 32, tc::sdesc_advance(qd, off), tc::sdesc_advance(kd, off), idesc, kk > 0);
+            }
+          } else
+#pragma unroll
+          for (int kk = 0; kk < LATENT / 16; kk++) {
+            const uint64_t bd = tc::sdesc_advance(kd, (kk >> 2) * FT_BLK + (kk & 3) * 32);
+            if (kk < FT_QS / 16)
+              tc::mma_ws_f16_if(leader, tmem + FT_S + b * 32, tc::sdesc_advance(qd, (kk >> 2) * (FT_HEADS * 128) + (kk & 3) * 32), bd, idesc, kk > 0);
+            else
+              tc::mma_ws_f16_tmem_a_if(leader, tmem + FT_S + b * 32, tmem + FT_Q + (kk - FT_QS / 16) * 8, bd, idesc, true);
+          }
+          tc::mma_commit_if(leader, &ms.s_full[b]);
         }
-        tc::mma_commit_if(leader, &ms.s_full[b]);
       }
     } else {
       const uint32_t idesc = tc::make_idesc(64, 256, tc::FMT_F16, tc::FMT_F16, false, true);
-      for (int tile = 0; tile < n_tiles; tile++) {
-        const int b = tile & 1, kb = tile % FT_NBUF;
-        wait_u(&ms.p_full[b], (tile >> 1) & 1, 3);
-        tc::fence_after_sync();
-        const uint64_t pd = tc::make_sdesc_sw128(tc::smem_u32(smem + FS_P + b * FP_BYTES), 16, 1024);
-        // V: N = 256 channels = four 64-channel blocks (leading offset), K = keys in 8-row atoms of 1 KB
-        const uint64_t vd = tc::make_sdesc_sw128(tc::smem_u32(smem + FS_K + kb * FT_TILE), FT_BLK, 1024);
-        const int steps = (tile_keys(tile) + 15) >> 4;    // a ragged tile ends early
+      for (int idx = blockIdx.x; idx < n_items; idx += step) {
+        const FtItem it = ft_item<G4>(a, idx);
+        if (it.n_tiles == 0) continue;
+        u++;
+        for (int tile = 0; tile < it.n_tiles; tile++, u++, g++) {
+          const int b = g & 1, kb = u % FT_NBUF;
+          wait_u(&ms.p_full[b], (g >> 1) & 1, 3);
+          if (tile == 0 && q > 0) wait_u(&ms.o_free, (q - 1) & 1, 14);   // the row before has left the accumulator
+          tc::fence_after_sync();
+          const uint64_t pd = tc::make_sdesc_sw128(tc::smem_u32(smem + FS_P + b * FP_BYTES), 16, 1024);
+          // V: N = 256 channels = four 64-channel blocks (leading offset), K = keys in 8-row atoms of 1 KB
+          const uint64_t vd = tc::make_sdesc_sw128(tc::smem_u32(smem + FS_K + kb * FT_TILE), FT_BLK, 1024);
+          const int steps = (it.keys(tile) + 15) >> 4;     // a ragged tile ends early
 #pragma unroll
-        for (int nh = 0; nh < 2; nh++)
+          for (int nh = 0; nh < 2; nh++)
 #pragma unroll
-          for (int kk = 0; kk < FT_KEYS / 16; kk++)
-            if (kk < steps)
-              tc::mma_ws_f16_if(leader, tmem + FT_O + nh * 128, tc::sdesc_advance(pd, kk * 32),
-                                tc::sdesc_advance(vd, nh * 4 * FT_BLK + kk * 2048), idesc, tile > 0 || kk > 0);
-        tc::mma_commit_if(leader, &ms.t_done[kb]);
+            for (int kk = 0; kk < FT_KEYS / 16; kk++)
+              if (kk < steps)
+                tc::mma_ws_f16_if(leader, tmem + FT_O + nh * 128, tc::sdesc_advance(pd, kk * 32),
+                                  tc::sdesc_advance(vd, nh * 4 * FT_BLK + kk * 2048), idesc, tile > 0 || kk > 0);
+          tc::mma_commit_if(leader, &ms.pv_done[b]);
+          tc::mma_commit_if(leader, &ms.free[kb]);
+        }
+        q++;
       }
     }
   } else {
@@ -320,144 +358,198 @@ __global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(M
     const int head = tid & 63, half = tid >> 6;
     const uint32_t lanes = (uint32_t)(warp * 32) << 16;
     const float sc2 = a.scale * LOG2E;
-    if (n_tiles > 0) {
-      const uint8_t* row = smem + FS_K + (FT_NBUF - 1) * FT_TILE + head * FT_QPITCH;
+    const bool final_out = a.out != nullptr;
+    uint32_t u = 0, g = 0;
+    auto wait_pv = [&](uint32_t tile_g, int code) { ok = tc::mbar_wait<FT_POLL_NS>(&ms.pv_done[tile_g & 1], (tile_g >> 1) & 1, abort_flag, code) && ok; };
+    // The row's Q: ring slot -> shared-memory operand (channels 0-127, the same layout) and tensor memory.  The products that
+    // read the row before have completed: these warps have seen its last S.
+    auto move_q = [&]() {
+      const int b = u % FT_NBUF;
+      ok = tc::mbar_wait<FT_POLL_NS>(&ms.full[b], (u / FT_NBUF) & 1, abort_flag, 11) && ok;
+      tc::fence_after_sync();
+      const uint8_t* src = smem + FS_K + b * FT_TILE;
+#pragma unroll
+      for (int i = 0; i < (int)(FT_QS * FT_HEADS * 2 / 16 / 128); i++)
+        reinterpret_cast<uint4*>(smem + FS_Q)[tid + 128 * i] = reinterpret_cast<const uint4*>(src)[tid + 128 * i];
 #pragma unroll 1
-      for (int c0 = 0; c0 < (LATENT - FT_QS) / 2; c0 += 32) {
+      for (int j = FT_QS / 64; j < 8; j++) {
         uint32_t v[32];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const uint4 w = *reinterpret_cast<const uint4*>(row + c0 * 4 + u * 16);
-          v[4 * u] = w.x; v[4 * u + 1] = w.y; v[4 * u + 2] = w.z; v[4 * u + 3] = w.w;
+        for (int c = 0; c < 8; c++) {
+          const uint4 w = *reinterpret_cast<const uint4*>(src + j * FT_BLK + head * 128 + ((c ^ (head & 7)) << 4));
+          v[4 * c] = w.x; v[4 * c + 1] = w.y; v[4 * c + 2] = w.z; v[4 * c + 3] = w.w;
         }
-        tc::tmem_st32(tmem + FT_Q + c0 + lanes, v);
+        tc::tmem_st32(tmem + FT_Q + (j - FT_QS / 64) * 32 + lanes, v);
       }
       tc::tmem_st_wait();
-      tc::fence_before_sync();
-      tc::mbar_arrive(&ms.q_ready);
-    }
-    float m = -INFINITY, l = 0.f;
-    for (int tile = 0; tile < n_tiles; tile++) {
-      const int b = tile & 1, kb = tile % FT_NBUF;
-      ok = tc::mbar_wait<FT_POLL_NS>(&ms.k_full[kb], (tile / FT_NBUF) & 1, abort_flag, 6) && ok;   // makes the tile's mask visible
-      ok = tc::mbar_wait<FT_POLL_NS>(&ms.s_full[b], (tile >> 1) & 1, abort_flag, 7) && ok;
-      tc::fence_after_sync();
-      uint32_t sv[32];
-      tc::tmem_ld32(tmem + FT_S + b * 32 + lanes, sv);
-      tc::tmem_ld_wait();
-      tc::fence_before_sync();
-      tc::mbar_arrive(&ms.s_free[b]);
-      const uint32_t mask = (uint32_t)(ms.mask[kb] >> (32 * half));
-      float tmax = -INFINITY;
-#pragma unroll
-      for (int j = 0; j < 32; j++) {
-        const float v = (mask >> j) & 1u ? __uint_as_float(sv[j]) * sc2 : -INFINITY;
-        sv[j] = __float_as_uint(v);
-        tmax = fmaxf(tmax, v);
-      }
-      ms.mx[b][tid] = tmax;
-      // the two warps of these heads: named barriers 1 (warps 0, 2) and 2 (warps 1, 3)
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 1)) : "memory");
-      tmax = fmaxf(tmax, ms.mx[b][tid ^ 64]);
-      const bool move = tmax > m + RESCALE_THRESHOLD || (m == -INFINITY && tmax > -INFINITY);
-      float alpha = 1.f;
-      if (move) {
-        alpha = m == -INFINITY ? 0.f : exp2f(m - tmax);
-        m = tmax;
-        l *= alpha;
-      }
-      if (tile > 0 && __any_sync(0xffffffffu, move)) {
-        // rare: a head's reference max moved.  O is rescaled after the previous tile's P V has completed and before this
-        // tile's is issued (it waits for p_full below); both warps of these heads take the same decision.
-        ok = tc::mbar_wait<FT_POLL_NS>(&ms.t_done[(tile - 1) % FT_NBUF], ((tile - 1) / FT_NBUF) & 1, abort_flag, 8) && ok;
-        tc::fence_after_sync();
-#pragma unroll 1
-        for (int c0 = 0; c0 < 256; c0 += 32) {
-          uint32_t o[32];
-          tc::tmem_ld32(tmem + FT_O + c0 + lanes, o);
-          tc::tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 32; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-          tc::tmem_st32(tmem + FT_O + c0 + lanes, o);
-        }
-        tc::tmem_st_wait();
-      }
-      // the P buffer of this parity was last read by the P V of tile - 2
-      if (tile >= 2) ok = tc::mbar_wait<FT_POLL_NS>(&ms.t_done[(tile - 2) % FT_NBUF], ((tile - 2) / FT_NBUF) & 1, abort_flag, 9) && ok;
-      uint8_t* prow = smem + FS_P + b * FP_BYTES;
-      const float mref = m == -INFINITY ? 0.f : m;         // every key so far is a hole: exp2(-inf) = 0 below
-      float sum = 0.f;
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        uint4 w;
-        uint32_t* wp = &w.x;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float p0 = exp2f(__uint_as_float(sv[8 * u + 2 * e]) - mref), p1 = exp2f(__uint_as_float(sv[8 * u + 2 * e + 1]) - mref);
-          sum += p0 + p1;
-          const __half2 hp = __floats2half2_rn(p0, p1);
-          wp[e] = *reinterpret_cast<const uint32_t*>(&hp);
-        }
-        *reinterpret_cast<uint4*>(prow + tc::sw128_off(head, half * 4 + u, FT_BLK)) = w;
-      }
-      l += sum;
       tc::fence_async_smem();
       tc::fence_before_sync();
-      tc::mbar_arrive(&ms.p_full[b]);
-    }
-    // ---- epilogue: wait for the last P V, lay the rows out in the (now idle) tile buffers, hand them to the copy engine ----
-    ms.l[tid] = l;
-    if (n_tiles > 0) ok = tc::mbar_wait<FT_POLL_NS>(&ms.t_done[(n_tiles - 1) % FT_NBUF], ((n_tiles - 1) / FT_NBUF) & 1, abort_flag, 10) && ok;
-    tc::fence_after_sync();
-    asm volatile("bar.sync 3, 128;" ::: "memory");
-    l += ms.l[tid ^ 64];
-    const bool final_out = a.out != nullptr;
-    const float f = l > 0.f ? (final_out ? 1.f / l : 1.f) : 0.f;
-    const uint32_t row_bytes = LATENT * (final_out ? 2 : 4), pitch = row_bytes + 16;
-    uint8_t* orow = smem + FS_K + head * pitch;
-#pragma unroll 1
-    for (int c0 = 0; c0 < 256; c0 += 32) {
-      uint32_t o[32];
-      if (n_tiles > 0) {
-        tc::tmem_ld32(tmem + FT_O + c0 + lanes, o);
+      tc::mbar_arrive(&ms.q_ready);
+      asm volatile("bar.sync 3, 128;" ::: "memory");
+      if (tid == 0) tc::mbar_arrive(&ms.free[b]);
+      u++;
+    };
+    auto next_row = [&](int idx) {                         // the first item from idx on that has keys
+      while (idx < n_items && ft_item<G4>(a, idx).n_tiles == 0) idx += step;
+      return idx;
+    };
+    int q_item = next_row(blockIdx.x);                     // the row whose Q is moved next
+    if (direct_q) u = 1;
+    else if (q_item < n_items) move_q();
+    for (int idx = blockIdx.x; idx < n_items; idx += step) {
+      const FtItem it = ft_item<G4>(a, idx);
+      float m = -INFINITY, l = 0.f;
+      for (int tile = 0; tile < it.n_tiles; tile++, u++, g++) {
+        const int b = g & 1, kb = u % FT_NBUF;
+        ok = tc::mbar_wait<FT_POLL_NS>(&ms.full[kb], (u / FT_NBUF) & 1, abort_flag, 6) && ok;   // makes the tile's mask visible
+        ok = tc::mbar_wait<FT_POLL_NS>(&ms.s_full[b], (g >> 1) & 1, abort_flag, 7) && ok;
+        tc::fence_after_sync();
+        uint32_t sv[32];
+        tc::tmem_ld32(tmem + FT_S + b * 32 + lanes, sv);
         tc::tmem_ld_wait();
-      } else {
+        tc::fence_before_sync();
+        tc::mbar_arrive(&ms.s_free[b]);
+        const uint32_t mask = *reinterpret_cast<const uint32_t*>(&ms.mask[kb][4 * half]);
+        float tmax = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < 32; j++) o[j] = 0u;
-      }
+        for (int j = 0; j < 32; j++) {
+          const float v = (mask >> j) & 1u ? __uint_as_float(sv[j]) * sc2 : -INFINITY;
+          sv[j] = __float_as_uint(v);
+          tmax = fmaxf(tmax, v);
+        }
+        ms.mx[b][tid] = tmax;
+        // the two warps of these heads: named barriers 1 (warps 0, 2) and 2 (warps 1, 3)
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 1)) : "memory");
+        tmax = fmaxf(tmax, ms.mx[b][tid ^ 64]);
+        const bool move = tmax > m + RESCALE_THRESHOLD || (m == -INFINITY && tmax > -INFINITY);
+        float alpha = 1.f;
+        if (move) {
+          alpha = m == -INFINITY ? 0.f : exp2f(m - tmax);
+          m = tmax;
+          l *= alpha;
+        }
+        if (tile > 0 && __any_sync(0xffffffffu, move)) {
+          // rare: a head's reference max moved.  O is rescaled after the previous tile's P V has completed and before this
+          // tile's is issued (it waits for p_full below); both warps of these heads take the same decision.
+          wait_pv(g - 1, 8);
+          tc::fence_after_sync();
+#pragma unroll 1
+          for (int c0 = 0; c0 < 256; c0 += 32) {
+            uint32_t o[32];
+            tc::tmem_ld32(tmem + FT_O + c0 + lanes, o);
+            tc::tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; j++) o[j] = l > 0.f ? __float_as_uint(__uint_as_float(o[j]) * f) : 0u;
-      const int ch = (c0 >> 7) * 256 + half * 128 + (c0 & 127);
-      if (final_out) {
+            for (int j = 0; j < 32; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+            tc::tmem_st32(tmem + FT_O + c0 + lanes, o);
+          }
+          tc::tmem_st_wait();
+        }
+        // the P buffer of this parity was last read by the P V two tiles ago (a row's first two tiles: its predecessor's
+        // epilogue has waited for all of them)
+        if (tile >= 2) wait_pv(g - 2, 9);
+        uint8_t* prow = smem + FS_P + b * FP_BYTES;
+        const float mref = m == -INFINITY ? 0.f : m;       // every key so far is a hole: exp2(-inf) = 0 below
+        float sum = 0.f;
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int v = 0; v < 4; v++) {
           uint4 w;
           uint32_t* wp = &w.x;
 #pragma unroll
           for (int e = 0; e < 4; e++) {
-            const __half2 h2 = __floats2half2_rn(__uint_as_float(o[8 * u + 2 * e]), __uint_as_float(o[8 * u + 2 * e + 1]));
-            wp[e] = *reinterpret_cast<const uint32_t*>(&h2);
+            const float p0 = exp2f(__uint_as_float(sv[8 * v + 2 * e]) - mref), p1 = exp2f(__uint_as_float(sv[8 * v + 2 * e + 1]) - mref);
+            sum += p0 + p1;
+            const __half2 hp = __floats2half2_rn(p0, p1);
+            wp[e] = *reinterpret_cast<const uint32_t*>(&hp);
           }
-          *reinterpret_cast<uint4*>(orow + ch * 2 + u * 16) = w;
+          *reinterpret_cast<uint4*>(prow + tc::sw128_off(head, half * 4 + v, FT_BLK)) = w;
         }
-      } else {
+        l += sum;
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        tc::mbar_arrive(&ms.p_full[b]);
+      }
+      // ---- epilogue of the row ----
+      ms.l[tid] = l;
+      if (it.n_tiles > 0) {
+        q_item = next_row(q_item + step);
+        if (q_item < n_items) move_q();
+        wait_pv(g - 1, 10);
+      }
+      tc::fence_after_sync();
+      asm volatile("bar.sync 3, 128;" ::: "memory");
+      l += ms.l[tid ^ 64];
+      const float f = l > 0.f ? (final_out ? 1.f / l : 1.f) : 0.f;
+      auto load_o = [&](int c0, uint32_t (&o)[32]) {       // 32 of this thread's 256 channels, weighed
+        if (it.n_tiles > 0) {
+          tc::tmem_ld32(tmem + FT_O + c0 + lanes, o);
+          tc::tmem_ld_wait();
+        }
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-          *reinterpret_cast<uint4*>(orow + ch * 4 + u * 16) = make_uint4(o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
+        for (int j = 0; j < 32; j++) o[j] = l > 0.f ? __float_as_uint(__uint_as_float(o[j]) * f) : 0u;
+      };
+      if (final_out) {
+        // Four rounds of 2 x 64 channels through the P buffers: channels 256 (c0 / 128) + 128 half + c0 % 128 ... of all heads
+        // as a swizzled box each.
+#pragma unroll 1
+        for (int c0 = 0; c0 < 256; c0 += 64) {
+          uint8_t* box = smem + FS_P + half * FP_BYTES;
+          if (tid == 0) tc::bulk_wait_read<0>();           // the boxes of the round before have left
+          asm volatile("bar.sync 3, 128;" ::: "memory");
+#pragma unroll
+          for (int hc = 0; hc < 2; hc++) {
+            uint32_t o[32];
+            load_o(c0 + 32 * hc, o);
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+              uint4 w;
+              uint32_t* wp = &w.x;
+#pragma unroll
+              for (int e = 0; e < 4; e++) {
+                const __half2 h2 = __floats2half2_rn(__uint_as_float(o[8 * v + 2 * e]), __uint_as_float(o[8 * v + 2 * e + 1]));
+                wp[e] = *reinterpret_cast<const uint32_t*>(&h2);
+              }
+              *reinterpret_cast<uint4*>(box + tc::sw128_off(head, hc * 4 + v, FT_BLK)) = w;
+            }
+          }
+          tc::fence_async_smem();
+          asm volatile("bar.sync 3, 128;" ::: "memory");
+          if (tid == 0 && ok && !*abort_flag) {
+#pragma unroll
+            for (int hf = 0; hf < 2; hf++)
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&tmap_o),
+                           "r"((c0 >> 7) * 256 + hf * 128 + (c0 & 127)), "r"(it.r * FT_HEADS), "r"(tc::smem_u32(smem + FS_P + hf * FP_BYTES))
+                           : "memory");
+            tc::bulk_commit();
+          }
+        }
+        tc::fence_before_sync();
+        if (it.n_tiles > 0) tc::mbar_arrive(&ms.o_free);
+        if (tid == 0) tc::bulk_wait_read<0>();
+        asm volatile("bar.sync 3, 128;" ::: "memory");     // P may be written again
+      } else {
+        // a partial (the CTA's only item): fp32 rows in the idle ring, one bulk copy per head
+        const uint32_t pitch = LATENT * 4 + 16;
+        uint8_t* orow = smem + FS_K + head * pitch;
+#pragma unroll 1
+        for (int c0 = 0; c0 < 256; c0 += 32) {
+          uint32_t o[32];
+          load_o(c0, o);
+          const int ch = (c0 >> 7) * 256 + half * 128 + (c0 & 127);
+#pragma unroll
+          for (int v = 0; v < 8; v++)
+            *reinterpret_cast<uint4*>(orow + ch * 4 + v * 16) = make_uint4(o[4 * v], o[4 * v + 1], o[4 * v + 2], o[4 * v + 3]);
+        }
+        tc::fence_async_smem();
+        asm volatile("bar.sync 3, 128;" ::: "memory");
+        const size_t rows = (size_t)a.m * FT_HEADS, rh = (size_t)it.r * FT_HEADS + head;
+        if (half == 0 && ok && !*abort_flag) {
+          tc::bulk_s2g(a.part_acc + ((size_t)it.sp * rows + rh) * LATENT, orow, LATENT * 4);
+          tc::bulk_commit();
+          a.part_m[(size_t)it.sp * rows + rh] = (m == -INFINITY || !(l > 0.f)) ? -INFINITY : m / LOG2E;
+          a.part_l[(size_t)it.sp * rows + rh] = l;
+          tc::bulk_wait_read<0>();
+        }
       }
-    }
-    tc::fence_async_smem();
-    asm volatile("bar.sync 3, 128;" ::: "memory");
-    const size_t rows = (size_t)a.m * FT_HEADS, rh = (size_t)r * FT_HEADS + head;
-    if (half == 0 && ok && !*abort_flag) {
-      char* dst = final_out ? reinterpret_cast<char*>(a.out + rh * LATENT) : reinterpret_cast<char*>(a.part_acc + ((size_t)sp * rows + rh) * LATENT);
-      tc::bulk_s2g(dst, orow, row_bytes);
-      tc::bulk_commit();
-      if (!final_out) {
-        a.part_m[(size_t)sp * rows + rh] = (m == -INFINITY || !(l > 0.f)) ? -INFINITY : m / LOG2E;
-        a.part_l[(size_t)sp * rows + rh] = l;
-      }
-      tc::bulk_wait_read<0>();
     }
   }
   tc::fence_before_sync();
@@ -509,9 +601,11 @@ int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s) {
   }
   // Tensor maps over the latent cache.  The row extent is the cache's row count when the caller gave it (the copy engine
   // zero-fills anything past the end), else an upper bound.
-  alignas(64) CUtensorMap box, rows;
+  alignas(64) CUtensorMap box, rows, qmap, omap;
   memset(&box, 0, sizeof(box));
   memset(&rows, 0, sizeof(rows));
+  memset(&qmap, 0, sizeof(qmap));
+  memset(&omap, 0, sizeof(omap));
   const cuuint64_t extent = a.ckv_rows > 0 ? (cuuint64_t)a.ckv_rows : (cuuint64_t)1 << 31;
   const cuuint32_t ones[3] = {1, 1, 1};
   {
@@ -522,18 +616,32 @@ int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s) {
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return HK_ERR_UNSUPPORTED;
   }
-  if (!a.raw_idx) {
-    const cuuint64_t dims[3] = {64, extent, 8};
+  // 64 rows x 512 channels as one box: whole key tiles of a dense range, and a row's 64 heads of Q
+  auto box_map = [&](CUtensorMap* m, const void* p, cuuint64_t n) {
+    const cuuint64_t dims[3] = {64, n, 8};
     const cuuint64_t strides[2] = {LATENT * 2, 128};
-    const cuuint32_t b[3] = {64, FT_KEYS, 8};
-    if (encode(&box, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)a.ckv, dims, strides, b, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    const cuuint32_t b[3] = {64, 64, 8};
+    return encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(p), dims, strides, b, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  static_assert(FT_KEYS == 64 && FT_HEADS == 64, "one box shape for keys and queries");
+  const cuuint64_t q_rows = (cuuint64_t)a.m * FT_HEADS;
+  if (!box_map(&qmap, a.q_lat, q_rows) || (!a.raw_idx && !box_map(&box, a.ckv, extent))) return HK_ERR_UNSUPPORTED;
+  if (a.out) {
+    const cuuint64_t dims[2] = {LATENT, q_rows};
+    const cuuint64_t strides[1] = {LATENT * 2};
+    const cuuint32_t b[2] = {64, 64};
+    if (encode(&omap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.out, dims, strides, b, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return HK_ERR_UNSUPPORTED;
   }
-  const dim3 grid(a.n_split, a.m);
+  // Gathered rows: at most a CTA per SM (592 rows of 2,048 keys 180 -> 166 us).  Dense rows, whose loads start faster: a CTA
+  // each (600 rows at 32,768 keys 2.72 ms, persistent 2.85).  Partials always: their rows leave through the idle ring.
+  const int64_t items = (int64_t)a.n_split * a.m;
+  const dim3 grid((unsigned)(a.raw_idx && a.out && items > sm_count() ? sm_count() : items));
   const cudaError_t e =
-      a.raw_idx ? pdl_launch(mla_flash_tc_kernel<true>, grid, dim3(FtRoles<true>::THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows)
-                : pdl_launch(mla_flash_tc_kernel<false>, grid, dim3(FtRoles<false>::THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows);
+      a.raw_idx ? pdl_launch(mla_flash_tc_kernel<true>, grid, dim3(FtRoles<true>::THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap)
+                : pdl_launch(mla_flash_tc_kernel<false>, grid, dim3(FtRoles<false>::THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap);
   return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 
