@@ -4,13 +4,10 @@
 // with kv_b the raw [64*512][512] fp16 tensor (rows h*512 .. +255 = W_uk[h], +256 .. +511 = W_uv[h]);
 // reference: src/cuda/attn/attn.cu:12-130 (one block per (row, head), the head's weights re-read per row).
 //
-// One kernel, a batched GEMM D[128 rows x 256] = A[128 x K] B[K x 256] per CTA (grid = N tiles x row tiles
-// x heads): K runs in chunks of 64 through a 3-stage ring of TMA tensor copies (128-byte-swizzle boxes:
-// A [128 rows][64 k]; B either [64 k][256 n] with n contiguous - W_uk, transposed W_uv - or [256 n][64 k]
-// with k contiguous - raw W_uv, so o_absorb needs no transposed copy of the weights), one thread issues
-// the copies, one the tcgen05.mma (M128 N256 K16, fp32 accumulators in 256 TMEM columns), four warps
-// write the tile out as fp16.  Rows past the end of the batch are zero-filled by the copy engine and not
-// stored.  All waits are bounded.
+// Two kernels: up to 32 rows with the weights as the M operand (below), more rows in 256 x 256 tiles.  Operands arrive as TMA
+// tensor copies in 128-byte-swizzle boxes (A [rows][64 k]; W either [64 k][64 n] with n contiguous - W_uk, transposed W_uv - or
+// [n][64 k] with k contiguous - raw W_uv, so o_absorb needs no transposed copy of the weights).  Rows past the end of the batch
+// are zero-filled by the copy engine and not stored.  All waits are bounded.
 #include <cuda.h>   // CUtensorMap (types only; the encoder is fetched through the runtime at first use)
 
 #include <cstdlib>
@@ -21,15 +18,23 @@
 
 namespace hk {
 
-// Two stages, not three: 97 KB of shared memory and 256 TMEM columns per CTA let TWO CTAs share an SM, so one CTA's
-// epilogue (64 KB of fp16 out of TMEM) runs under the other's copies and products: 202 -> 170 us (q) and 135 -> 122 us
-// (o) at 4,096 rows.  K is only 256 or 512 (4 or 8 chunks), so a deeper ring inside one CTA has little to overlap.
-constexpr int AB_BM = 128, AB_BN = 256, AB_BK = 64, AB_STAGES = 2;
-constexpr uint32_t AB_A_BYTES = AB_BM * AB_BK * 2;            // 16 KB
-constexpr uint32_t AB_B_BYTES = AB_BN * AB_BK * 2;            // 32 KB
-constexpr uint32_t AB_STAGE = AB_A_BYTES + AB_B_BYTES;        // 48 KB
-constexpr uint32_t AB_SMEM = AB_STAGES * AB_STAGE + 1024;     // + slack to align the base to 1 KB
-constexpr int AB_THREADS = 192;
+// Persistent CTAs over tiles of 256 rows x 256 columns x one head, K in chunks of 64 channels through a three-stage ring of
+// 64 KB.  What bounds it is the traffic between L2 and the SMs, which needs some 190 KB in flight per SM to pass 34 B per cycle:
+// 128-row tiles, two CTAs per SM and 96 KB each, moved 805 / 786 MB for the 403 MB that 4,096 rows cannot do without (113 us
+// q_latent, 89 us o_absorb); a weight tile of 128 KB kept in shared memory left a ring of 64 KB and 20-24 B per cycle (87, 103).
+// Here it is 524 MB: 86 and 80 us.  Tiles run over columns, heads, rows: the CTAs at work write one stretch of whole output rows
+// and read all 16.8 MB of weights, which stay in L2.  At 512 rows 20.9 -> 14.8 and 16.6 -> 14.3 us, at 33 rows 8.7 -> 6.1 and
+// 10.6 -> 6.6 (all copies of a tile fly at once).
+// Warp 0 copies in, warp 1 issues the products (converged, elected lane) into 2 x 256 tensor-memory columns, warps 2-9 write
+// out: a lane takes its whole row of the accumulator as fp16 into registers (the products of the next tile can start), then the
+// warp sends it off in boxes of 32 rows x 64 columns through 4 KB of its own, with no barrier between warps.
+constexpr int AB_BM = 128, AB_BN = 256, AB_BK = 64, AB_STAGES = 3;
+constexpr uint32_t AB_A_BYTES = AB_BM * AB_BK * 2;            // 16 KB, two per stage
+constexpr uint32_t AB_W_BYTES = AB_BN * AB_BK * 2;            // 32 KB
+constexpr uint32_t AB_STAGE = 2 * AB_A_BYTES + AB_W_BYTES;
+constexpr uint32_t AB_BOX = 32 * 128;                         // one output box
+constexpr int AB_THREADS = 320;
+constexpr uint32_t AB_SMEM = AB_STAGES * AB_STAGE + 8 * AB_BOX + 1024;   // + slack to align the base to 1 KB
 
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* tmap, int x, int y, uint64_t* bar) {
   asm volatile(
@@ -39,155 +44,176 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
       : "memory");
 }
 
-// B_MN: the weight tile has n contiguous ([k][n] in memory), else k contiguous ([n][k]).
-// a_col0 / b_*0: element coordinates of this head's operands inside the two tensor maps.
-template <bool B_MN>
+// W_MN: the weight tile has n contiguous ([k][n] in memory), else k contiguous ([n][k]).
+template <bool W_MN, int K>
 __global__ __launch_bounds__(AB_THREADS, 1) void absorb_gemm_tc_kernel(
-    const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-    const __grid_constant__ CUtensorMap tmap_o, int use_tma_out,
-    __half* __restrict__ out, int n_rows, int K, int n_out, int b_rows_per_head, int b_row_off,
-    int* __restrict__ status) {
+    const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_o,
+    int n_rows, int n_tiles, int w_rows_per_head, int w_row_off, int* __restrict__ status) {
+  constexpr int NK = K / AB_BK;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
-  __shared__ uint64_t full_bar[AB_STAGES], empty_bar[AB_STAGES], done_bar;
+  __shared__ uint64_t full_bar[AB_STAGES], empty_bar[AB_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nt = blockIdx.x, row0 = blockIdx.y * AB_BM, h = blockIdx.z;
-  const int nk = K / AB_BK;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = tc::warp_index_uniform();
+  const int total = 64 * n_tiles * ((n_rows + 2 * AB_BM - 1) / (2 * AB_BM));
 
   if (tid == 0) {
     for (int i = 0; i < AB_STAGES; i++) {
       tc::mbar_init(&full_bar[i], 1);
       tc::mbar_init(&empty_bar[i], 1);
     }
-    tc::mbar_init(&done_bar, 1);
+    for (int i = 0; i < 2; i++) {
+      tc::mbar_init(&acc_full[i], 1);
+      tc::mbar_init(&acc_empty[i], 4);
+    }
     tc::mbar_fence_init();
     abort_flag = 0;
   }
-  if (warp == 2) tc::tmem_alloc(&tmem_slot, AB_BN);
+  if (warp == 2) tc::tmem_alloc(&tmem_slot, 512);
+  pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_slot;
+  auto place = [&](int t, int& n0, int& h, int& row0) {
+    n0 = (t % n_tiles) * AB_BN;
+    h = (t / n_tiles) & 63;
+    row0 = t / n_tiles / 64 * 2 * AB_BM;
+  };
 
   if (warp == 0) {
     if (lane == 0) {
-      // ---- producer: one A box and the B boxes of every K chunk ----
-      for (int kc = 0; kc < nk; kc++) {
-        const int s = kc % AB_STAGES;
-        if (kc >= AB_STAGES && !tc::mbar_wait<32>(&empty_bar[s], ((kc / AB_STAGES) - 1) & 1, &abort_flag, 1)) break;
-        uint8_t* sa = smem + s * AB_STAGE;
-        uint8_t* sb = sa + AB_A_BYTES;
-        tc::mbar_arrive_expect_tx(&full_bar[s], AB_STAGE);
-        tma_load_2d(sa, &tmap_a, h * K + kc * AB_BK, row0, &full_bar[s]);
-        if (B_MN) {
-          // [k][n]: four boxes of 64 n x 64 k, each a stack of 8-row swizzle atoms
+      uint32_t n = 0;                                        // chunks so far
+      bool ok = true;
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        int n0, h, row0;
+        place(t, n0, h, row0);
+        const bool two = row0 + AB_BM < n_rows;              // the second half has rows
+        const int wy = h * w_rows_per_head + w_row_off;
+        for (int kc = 0; kc < NK; kc++, n++) {
+          const int s = n % AB_STAGES;
+          if (n >= AB_STAGES && !tc::mbar_wait<32>(&empty_bar[s], (n / AB_STAGES - 1) & 1, &abort_flag, 1)) {
+            ok = false;
+            break;
+          }
+          uint8_t* sa = smem + s * AB_STAGE;
+          uint8_t* sw = sa + 2 * AB_A_BYTES;
+          tc::mbar_arrive_expect_tx(&full_bar[s], AB_W_BYTES + (two ? 2 : 1) * AB_A_BYTES);
+          tma_load_2d(sa, &tmap_a, h * K + kc * AB_BK, row0, &full_bar[s]);
+          if (two) tma_load_2d(sa + AB_A_BYTES, &tmap_a, h * K + kc * AB_BK, row0 + AB_BM, &full_bar[s]);
+          if (W_MN) {                                        // boxes of 64 n x 64 k, each a stack of 8-row swizzle atoms
 #pragma unroll
-          for (int j = 0; j < AB_BN / 64; j++)
-            tma_load_2d(sb + j * 8192, &tmap_b, nt * AB_BN + j * 64, h * b_rows_per_head + b_row_off + kc * AB_BK, &full_bar[s]);
-        } else {
-          // [n][k]: one box of 64 k x 256 n rows
-          tma_load_2d(sb, &tmap_b, kc * AB_BK, h * b_rows_per_head + b_row_off + nt * AB_BN, &full_bar[s]);
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      // ---- tensor-core issue ----
-      const uint32_t idesc = tc::make_idesc(AB_BM, AB_BN, tc::FMT_F16, tc::FMT_F16, false, B_MN);
-      for (int kc = 0; kc < nk; kc++) {
-        const int s = kc % AB_STAGES;
-        if (!tc::mbar_wait<32>(&full_bar[s], (kc / AB_STAGES) & 1, &abort_flag, 2)) break;
-        tc::fence_after_sync();
-        const uint32_t a_addr = tc::smem_u32(smem + s * AB_STAGE), b_addr = a_addr + AB_A_BYTES;
-#pragma unroll
-        for (int k16 = 0; k16 < AB_BK / 16; k16++) {
-          const uint64_t ad = tc::make_sdesc_sw128(a_addr + k16 * 32, 16, 1024);
-          const uint64_t bd = B_MN ? tc::make_sdesc_sw128(b_addr + k16 * 2048, 8192, 1024)
-                                   : tc::make_sdesc_sw128(b_addr + k16 * 32, 16, 1024);
-          tc::mma_f16(tmem, ad, bd, idesc, kc > 0 || k16 > 0);
-        }
-        tc::mma_commit(&empty_bar[s]);
-      }
-      tc::mma_commit(&done_bar);
-    }
-  } else {
-    // ---- epilogue: warps 2-5 cover the four TMEM lane quarters (a warp may only touch quarter warp % 4) ----
-    const int q = warp & 3;
-    const int row = row0 + q * 32 + lane;
-    const bool ok = tc::mbar_wait<64>(&done_bar, 0, &abort_flag, 3);
-    tc::fence_after_sync();
-    if (ok && use_tma_out) {
-      // The fp16 tile leaves through the copy engine: every thread lays its row into the (now idle) operand stages as
-      // four 128-row x 64-column boxes in the 128-byte-swizzle pattern (16-byte piece c of row r at c ^ (r % 8):
-      // conflict-free), one thread hands the four boxes over as tiled stores (rows past the end are clipped).  Direct
-      // stores put 32 different rows into every warp instruction.
-      const int r = q * 32 + lane;
-#pragma unroll 1
-      for (int c0 = 0; c0 < AB_BN; c0 += 32) {
-        uint32_t rr[32];
-        tc::tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c0, rr);
-        tc::tmem_ld_wait();
-        uint8_t* box = smem + (c0 >> 6) * 16384 + r * 128;
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          uint4 p;
-          __half2 h0 = __floats2half2_rn(__uint_as_float(rr[8 * u + 0]), __uint_as_float(rr[8 * u + 1]));
-          __half2 h1 = __floats2half2_rn(__uint_as_float(rr[8 * u + 2]), __uint_as_float(rr[8 * u + 3]));
-          __half2 h2 = __floats2half2_rn(__uint_as_float(rr[8 * u + 4]), __uint_as_float(rr[8 * u + 5]));
-          __half2 h3 = __floats2half2_rn(__uint_as_float(rr[8 * u + 6]), __uint_as_float(rr[8 * u + 7]));
-          p.x = *reinterpret_cast<uint32_t*>(&h0); p.y = *reinterpret_cast<uint32_t*>(&h1);
-          p.z = *reinterpret_cast<uint32_t*>(&h2); p.w = *reinterpret_cast<uint32_t*>(&h3);
-          const int cc = ((c0 & 63) >> 3) + u;
-          *reinterpret_cast<uint4*>(box + ((cc ^ (r & 7)) << 4)) = p;
-        }
-      }
-      tc::fence_async_smem();
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (warp == 2 && lane == 0) {
-#pragma unroll
-        for (int j = 0; j < AB_BN / 64; j++)
-          asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(&tmap_o),
-                       "r"(nt * AB_BN + j * 64), "r"(h), "r"(row0), "r"(tc::smem_u32(smem + j * 16384))
-                       : "memory");
-        tc::bulk_commit();
-        tc::bulk_wait_read<0>();                  // the boxes have been read: the CTA may leave
-      }
-    } else if (ok) {
-      __half* orow = out + ((size_t)row * 64 + h) * n_out + nt * AB_BN;
-#pragma unroll 1
-      for (int c0 = 0; c0 < AB_BN; c0 += 32) {
-        uint32_t r[32];
-        tc::tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c0, r);
-        tc::tmem_ld_wait();
-        if (row < n_rows) {
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            uint4 p;
-            __half2 h0 = __floats2half2_rn(__uint_as_float(r[8 * u + 0]), __uint_as_float(r[8 * u + 1]));
-            __half2 h1 = __floats2half2_rn(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3]));
-            __half2 h2 = __floats2half2_rn(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5]));
-            __half2 h3 = __floats2half2_rn(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7]));
-            p.x = *reinterpret_cast<uint32_t*>(&h0); p.y = *reinterpret_cast<uint32_t*>(&h1);
-            p.z = *reinterpret_cast<uint32_t*>(&h2); p.w = *reinterpret_cast<uint32_t*>(&h3);
-            *reinterpret_cast<uint4*>(orow + c0 + 8 * u) = p;
+            for (int j = 0; j < AB_BN / 64; j++) tma_load_2d(sw + j * 8192, &tmap_w, n0 + j * 64, wy + kc * AB_BK, &full_bar[s]);
+          } else {                                           // one box of 64 k x 256 n rows
+            tma_load_2d(sw, &tmap_w, kc * AB_BK, wy + n0, &full_bar[s]);
           }
         }
       }
     }
+  } else if (warp == 1) {
+    const uint32_t leader = tc::elect_one();
+    const uint32_t idesc = tc::make_idesc(AB_BM, AB_BN, tc::FMT_F16, tc::FMT_F16, false, W_MN);
+    bool ok = true;
+    auto wait_u = [&](uint64_t* bar, uint32_t parity, int code) {   // every lane waits (tc05.cuh)
+      const bool done = tc::mbar_wait<32>(bar, parity, &abort_flag, code);
+      ok = __all_sync(0xffffffffu, done) != 0 && ok;
+    };
+    uint32_t n = 0, used[2] = {0, 0};                        // chunks, and tiles of either half, so far
+    for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+      int n0, h, row0;
+      place(t, n0, h, row0);
+      const bool two = row0 + AB_BM < n_rows;
+      for (int kc = 0; kc < NK && ok; kc++, n++) {
+        const int s = n % AB_STAGES;
+        wait_u(&full_bar[s], (n / AB_STAGES) & 1, 2);
+        tc::fence_after_sync();
+        const uint32_t a_addr = tc::smem_u32(smem + s * AB_STAGE), w_addr = a_addr + 2 * AB_A_BYTES;
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+          if (m == 1 && !two) break;
+          if (kc == 0) {
+            if (used[m] > 0) {
+              wait_u(&acc_empty[m], (used[m] - 1) & 1, 3);
+              tc::fence_after_sync();
+            }
+            used[m]++;
+          }
+          if (!ok) break;
+#pragma unroll
+          for (int k16 = 0; k16 < AB_BK / 16; k16++)
+            tc::mma_f16_if(leader, tmem + m * AB_BN, tc::make_sdesc_sw128(a_addr + m * AB_A_BYTES + k16 * 32, 16, 1024),
+                           W_MN ? tc::make_sdesc_sw128(w_addr + k16 * 2048, 8192, 1024) : tc::make_sdesc_sw128(w_addr + k16 * 32, 16, 1024),
+                           idesc, kc > 0 || k16 > 0);
+          if (m == (two ? 1 : 0)) tc::mma_commit_if(leader, &empty_bar[s]);
+          if (kc == NK - 1) tc::mma_commit_if(leader, &acc_full[m]);
+        }
+      }
+    }
+  } else {
+    // ---- epilogue: four warps per half; a warp may only touch the TMEM lane quarter warp % 4 ----
+    const int q = warp & 3, m = (warp - 2) >> 2;
+    uint8_t* box = smem + AB_STAGES * AB_STAGE + (warp - 2) * AB_BOX;
+    uint32_t used = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+      int n0, h, row0;
+      place(t, n0, h, row0);
+      row0 += m * AB_BM;
+      if (row0 >= n_rows) break;                             // only the last row tile is short, and it comes last
+      ok = __all_sync(0xffffffffu, tc::mbar_wait<64>(&acc_full[m], used & 1, &abort_flag, 4)) != 0;
+      used++;
+      if (!ok) break;
+      tc::fence_after_sync();
+      uint32_t pk[AB_BN / 2];                                // this lane's row: the accumulator is free again before the first store
+#pragma unroll
+      for (int c0 = 0; c0 < AB_BN; c0 += 32) {
+        uint32_t v[32];
+        tc::tmem_ld32(tmem + m * AB_BN + c0 + ((uint32_t)(q * 32) << 16), v);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 16; e++) {
+          const __half2 h2 = __floats2half2_rn(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+          pk[c0 / 2 + e] = *reinterpret_cast<const uint32_t*>(&h2);
+        }
+      }
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&acc_empty[m]);
+#pragma unroll
+      for (int c0 = 0; c0 < AB_BN; c0 += 64) {
+        if (lane == 0) tc::bulk_wait_read<0>();              // the box before has left
+        __syncwarp();
+        // a lane lays its row into the box in the 128-byte-swizzle pattern: 16-byte piece u of row r at u ^ (r % 8)
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const uint32_t* w = pk + c0 / 2 + 4 * u;
+          *reinterpret_cast<uint4*>(box + lane * 128 + ((u ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        tc::fence_async_smem();
+        __syncwarp();
+        if (lane == 0 && row0 + q * 32 < n_rows) {           // rows past the end are clipped
+          asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(&tmap_o),
+                       "r"(n0 + c0), "r"(h), "r"(row0 + q * 32), "r"(tc::smem_u32(box))
+                       : "memory");
+          tc::bulk_commit();
+        }
+      }
+    }
+    if (lane == 0) tc::bulk_wait_read<0>();
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 2) tc::tmem_dealloc(tmem, AB_BN);
+  if (warp == 2) tc::tmem_dealloc(tmem, 512);
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
 }
 
 // ------------------------------------------------------------------------------------------------
-// A few rows (decode, at most 32): the 16.8 MB of weights are all there is to move.  The kernel above gives such a call 128
-// (q) or 64 (o) CTAs of 128-row tiles whose two-stage ring has at most 96 KB in flight, on 64 SMs for o: 7.8 and 10.5 us.
-// Here the WEIGHTS are the M operand, 64 output columns per CTA (512 and 256 CTAs, all resident), the rows are N (8 to 32),
-// and a CTA requests its whole K at once (32 / 64 KB, a barrier per 64-channel chunk): no ring, no empty barriers.
+// A few rows (decode, at most 32): the 16.8 MB of weights are all there is to move.  As 128-row tiles such a call has 128
+// tiles, on 128 SMs, of which a row uses 1/128: 7.8 (q) and 10.5 us (o).  Here the WEIGHTS are the M operand, 64 output
+// columns per CTA (512 and 256 CTAs, all resident), the rows are N (8 to 32), and a CTA requests its whole K at once (32 /
+// 64 KB, a barrier per 64-channel chunk): no ring, no empty barriers.
 // ------------------------------------------------------------------------------------------------
 constexpr int AF_BM = 64, AF_BK = 64, AF_MAX_ROWS = 32, AF_THREADS = 128;
 constexpr uint32_t AF_A_CHUNK = AF_BM * AF_BK * 2;            // 8 KB
@@ -324,6 +350,42 @@ static int absorb_few_rows(const void* x, const void* w, void* out, int n_rows, 
              : HK_ERR_CUDA;
 }
 
+template <bool W_MN, int K>
+static int absorb_rows(const void* x, const void* w, void* out, int n_rows, int n_out, uint64_t w_rows, uint64_t w_cols,
+                       int w_rows_per_head, int w_row_off, cudaStream_t s) {
+  alignas(64) CUtensorMap mx, mw, mo;
+  memset(&mx, 0, sizeof(mx));
+  memset(&mw, 0, sizeof(mw));
+  memset(&mo, 0, sizeof(mo));
+  if (!make_map_2d(&mx, x, (uint64_t)n_rows, (uint64_t)64 * K, AB_BM, AB_BK) ||
+      !make_map_2d(&mw, w, w_rows, w_cols, W_MN ? AB_BK : AB_BN, 64))
+    return HK_ERR_UNSUPPORTED;
+  // output as [row][head][n_out]: boxes of 64 columns x 1 head x 32 rows
+  const cuuint64_t dims[3] = {(cuuint64_t)n_out, 64, (cuuint64_t)n_rows};
+  const cuuint64_t strides[2] = {(cuuint64_t)n_out * 2, (cuuint64_t)64 * n_out * 2};
+  const cuuint32_t box[3] = {64, 1, 32};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  if (encode_tiled_fn()(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return HK_ERR_UNSUPPORTED;
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    if (cudaFuncSetAttribute(absorb_gemm_tc_kernel<W_MN, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AB_SMEM) != cudaSuccess)
+      return HK_ERR_CUDA;
+    attr_set[dev] = true;
+  }
+  const int n_tiles = n_out / AB_BN;
+  const int64_t total = (int64_t)64 * n_tiles * ((n_rows + 2 * AB_BM - 1) / (2 * AB_BM));
+  if (total > 1 << 30) return HK_ERR_UNSUPPORTED;
+  const int grid = (int)(total < sm_count() ? total : sm_count());
+  return pdl_launch(absorb_gemm_tc_kernel<W_MN, K>, dim3(grid), dim3(AB_THREADS), AB_SMEM, s, mx, mw, mo, n_rows, n_tiles,
+                    w_rows_per_head, w_row_off, device_status_ptr()) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
+}
+
 // a [n_rows][64*K], weights as described above, out [n_rows][64*n_out]; returns HK_ERR_UNSUPPORTED when the
 // tensor maps cannot be built (the caller then uses the CUDA-core kernels)
 int absorb_gemm_tc(const void* a, const void* b, void* out, int n_rows, int K, int n_out, bool b_mn,
@@ -334,40 +396,10 @@ int absorb_gemm_tc(const void* a, const void* b, void* out, int n_rows, int K, i
     if (K == 512 && !b_mn) return absorb_few_rows<false, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
     if (K == 512 && b_mn) return absorb_few_rows<true, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
   }
-  alignas(64) CUtensorMap ma, mb;
-  memset(&ma, 0, sizeof(ma));
-  memset(&mb, 0, sizeof(mb));
-  if (!make_map_2d(&ma, a, (uint64_t)n_rows, (uint64_t)64 * K, AB_BM, AB_BK)) return HK_ERR_UNSUPPORTED;
-  if (!make_map_2d(&mb, b, b_rows, b_cols, b_mn ? AB_BK : AB_BN, 64)) return HK_ERR_UNSUPPORTED;
-  // output as [row][head][n_out]: boxes of 64 columns x 1 head x 128 rows for the tiled stores of the epilogue
-  alignas(64) CUtensorMap mo;
-  memset(&mo, 0, sizeof(mo));
-  int use_tma_out = 0;
-  {
-    EncodeTiledFn enc = encode_tiled_fn();
-    const cuuint64_t dims[3] = {(cuuint64_t)n_out, 64, (cuuint64_t)n_rows};
-    const cuuint64_t strides[2] = {(cuuint64_t)n_out * 2, (cuuint64_t)64 * n_out * 2};
-    const cuuint32_t box[3] = {64, 1, AB_BM};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    if (enc && enc(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
-      use_tma_out = 1;
-  }
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(absorb_gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AB_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(absorb_gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AB_SMEM) != cudaSuccess)
-      return HK_ERR_CUDA;
-    attr_set[dev] = true;
-  }
-  const dim3 grid(n_out / AB_BN, (n_rows + AB_BM - 1) / AB_BM, 64);
-  if (b_mn)
-    absorb_gemm_tc_kernel<true><<<grid, AB_THREADS, AB_SMEM, s>>>(ma, mb, mo, use_tma_out, (__half*)out, n_rows, K, n_out, b_rows_per_head, b_row_off, device_status_ptr());
-  else
-    absorb_gemm_tc_kernel<false><<<grid, AB_THREADS, AB_SMEM, s>>>(ma, mb, mo, use_tma_out, (__half*)out, n_rows, K, n_out, b_rows_per_head, b_row_off, device_status_ptr());
-  return cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+  if (K == 256 && b_mn) return absorb_rows<true, 256>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
+  if (K == 512 && !b_mn) return absorb_rows<false, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
+  if (K == 512 && b_mn) return absorb_rows<true, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
+  return HK_ERR_UNSUPPORTED;
 }
 
 }  // namespace hk

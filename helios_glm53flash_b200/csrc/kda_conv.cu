@@ -4,9 +4,9 @@
 // bf16 round-to-nearest output, state = last K inputs.
 //
 // Four kernels (the last one is the fused cast + convolution over token-major fp32 input, further below):
-//   conv4_row_kernel   prefill with whole 16-token groups: K = 4, no history, seqlen % 16 == 0.  No
-//                      shared memory: a lane keeps 2 channels x 16 (or 32) tokens in registers (32-byte reads
-//                      per channel row, 128-byte warp stores per output row).
+//   conv4_row_kernel   prefill with whole 8-token pieces: K = 4, no history, seqlen % 8 == 0.  Persistent CTAs over
+//                      [64 channel][64 token] tiles: asynchronous 16-byte copies into a three-stage ring, a lane computes 2
+//                      channels x 16 tokens (128-byte warp stores per output row).
 //   conv4_tile_kernel  other prefill lengths: a CTA transposes a [64 channel][128 token] tile
 //                      through shared memory: 16-byte reads along tokens (the input is channel-major),
 //                      128-byte coalesced writes along channels (the output is token-major).  The rows of a
@@ -118,84 +118,143 @@ __global__ __launch_bounds__(256) void conv4_tile_kernel(
   }
 }
 
-// Prefill with whole 16-token groups (seqlen % 16 == 0): no shared memory at all.  A lane owns 2 adjacent
-// channels and 16 consecutive tokens: it reads 32 contiguous bytes per channel row (full sectors), keeps
-// the 19 inputs per channel in registers and writes 4 bytes per token, so that a warp's store covers 128
-// contiguous bytes of one output row.  Same arithmetic as above, about half the instructions per output.
-template <bool ACT, int NG>   // NG groups of 16 consecutive tokens per lane
-__global__ __launch_bounds__(256) void conv4_row_kernel(
+// Prefill with whole 8-token pieces (seqlen % 8 == 0, so every channel row starts on 16 bytes).  2 B are read and 2 B written
+// per channel-token; what a transposing access pattern reaches depends on the length of its runs, and the SiLU's exponential
+// and reciprocal (230 us at 32,768 tokens x 12,288 channels on the special-function units alone) have to run under the copies.
+// With 32 bytes per channel row and lane, straight into registers, that size took 362 us (4.45 TB/s; runs of 128 bytes copy in
+// 268).  So the tile goes through shared memory, copied in asynchronously two tiles ahead: 324 us, and 16.8 -> 14.1 at 1,008
+// tokens, 613 -> 331 at 32,760.  The 16-byte piece p of row r sits at p ^ (r / 2 % 8), which keeps the copies (8 lanes to a
+// row) and the reads (32 lanes on rows 2 l and 2 l + 1) free of bank conflicts.  Small CTAs because one's barrier then stalls
+// only four warps: 64-token tiles and six CTAs per SM 324 us, 128-token tiles and three or four 339, 353; five 345, eight 434
+// (too many streams for the memory).
+constexpr int CW_TOK = 64, CW_THREADS = CW_TOK * 2, CW_STAGES = 3, CW_CTAS = 6;
+constexpr uint32_t CW_TILE = CT_CH * CW_TOK * 2, CW_STAGE = CW_TILE + CT_CH * 8;   // 8 KB and the 4 tokens before each row
+constexpr uint32_t CW_SMEM = CW_STAGES * CW_STAGE;
+
+template <bool ACT>
+__global__ __launch_bounds__(CW_THREADS, CW_CTAS) void conv4_row_kernel(
     const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ state,
     const int* __restrict__ slots, const __nv_bfloat16* __restrict__ weight,
     const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, int dim, int seqlen,
-    int state_size) {
-  constexpr int NT = 16 * NG;                                // tokens per lane
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int c0 = blockIdx.x * CT_CH + lane * 2;
-  const int t0 = (blockIdx.y * 8 + wid) * NT;
-  const int b = blockIdx.z;
+    int state_size, int tok_tiles, int total) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(smem_raw);
+  // tiles run over channels, tokens, batch: the CTAs at work write whole output rows.  A place in that order is moved on by the
+  // grid without divisions.
+  const int ch_tiles = dim / CT_CH, step_t = gridDim.x / ch_tiles, step_c = gridDim.x - step_t * ch_tiles;
+  struct Place {
+    int t, c, s, b;                                          // tile, channel tile, token tile, batch
+  };
+  auto advance = [&](Place& p) {
+    p.t += gridDim.x;
+    p.c += step_c;
+    p.s += step_t;
+    if (p.c >= ch_tiles) {
+      p.c -= ch_tiles;
+      p.s++;
+    }
+    while (p.s >= tok_tiles) {
+      p.s -= tok_tiles;
+      p.b++;
+    }
+  };
+  const int cr = tid >> 3, cp = tid & 7;                     // copies: rows cr + 16 i, piece cp
+  const uint32_t dst = sm0 + cr * 128 + ((cp ^ ((cr >> 1) & 7)) << 4);
+  const size_t row16 = (size_t)seqlen * 16;
+  auto copy_in = [&](const Place& p, int stage) {
+    const __nv_bfloat16* xb = x + ((size_t)p.b * dim + p.c * CT_CH) * seqlen + p.s * CW_TOK;
+    if (p.s * CW_TOK + 8 * cp < seqlen) {
+      const __nv_bfloat16* src = xb + (size_t)cr * seqlen + 8 * cp;
+#pragma unroll
+      for (int i = 0; i < 4; i++) 
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + stage * CW_STAGE + i * 2048), "l"(src + i * row16) : "memory");
+    }
+    if (tid < CT_CH && p.s > 0)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sm0 + stage * CW_STAGE + CW_TILE + tid * 8),
+                   "l"(xb + (size_t)tid * seqlen - 4)
+                   : "memory");
+  };
+  Place in;
+  in.t = blockIdx.x;
+  in.s = in.t / ch_tiles;
+  in.c = in.t - in.s * ch_tiles;
+  in.b = in.s / tok_tiles;
+  in.s -= in.b * tok_tiles;
+  Place at = in;
   pdl_wait();
-  if (t0 >= seqlen) return;                                  // warp-uniform
-  const __nv_bfloat16* r0 = x + ((size_t)b * dim + c0) * seqlen;
-  const __nv_bfloat16* r1 = r0 + seqlen;
-  uint4 ra[2 * NG], re[2 * NG];                              // all loads of the lane are issued before any use
 #pragma unroll
-  for (int j = 0; j < 2 * NG; j++) {
-    ra[j] = ld_stream16(r0 + t0 + 8 * j);
-    re[j] = ld_stream16(r1 + t0 + 8 * j);
+  for (int i = 0; i < CW_STAGES - 1; i++) {
+    if (in.t < total) copy_in(in, i);
+    advance(in);
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  float xa[NT + 3], xe[NT + 3];                              // inputs t0-3 .. t0+NT-1 of the two channels
-  if (t0 == 0) {
-    // the first group takes its 3 predecessors from the window state and rolls the state forward
-    const int slot = slots ? slots[b] : b;
-    __nv_bfloat16* st0 = state + ((size_t)slot * dim + c0) * state_size;
-    __nv_bfloat16* st1 = st0 + state_size;
+  int stage = 0;
+  for (; at.t < total; advance(at)) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(CW_STAGES - 2) : "memory");
+    __syncthreads();                                         // everyone's pieces are there, and the stage before is done with
+    if (in.t < total) copy_in(in, stage == 0 ? CW_STAGES - 1 : stage - 1);
+    advance(in);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const int c0 = at.c * CT_CH + lane * 2, b = at.b;
+    const uint8_t* rows = smem_raw + stage * CW_STAGE + lane * 256;   // channels c0 and c0 + 1
+    const int t0 = at.s * CW_TOK + wid * 16;
+    stage = stage == CW_STAGES - 1 ? 0 : stage + 1;
+    if (t0 >= seqlen) continue;                              // warp-uniform
+    uint2 pa, pe;                                            // tokens t0-4 .. t0-1 (the first is not used)
+    if (t0 == 0) {
+      // the first group takes its predecessors from the window state and rolls the state forward
+      const int slot = slots ? slots[b] : b;
+      __nv_bfloat16* st0 = state + ((size_t)slot * dim + c0) * state_size;
+      __nv_bfloat16* st1 = st0 + state_size;
+      const uint16_t* u0 = reinterpret_cast<const uint16_t*>(st0);
+      const uint16_t* u1 = reinterpret_cast<const uint16_t*>(st1);
+      pa = make_uint2((uint32_t)u0[1] << 16, (uint32_t)u0[2] | ((uint32_t)u0[3] << 16));
+      pe = make_uint2((uint32_t)u1[1] << 16, (uint32_t)u1[2] | ((uint32_t)u1[3] << 16));
+      const __nv_bfloat16* r0 = x + ((size_t)b * dim + c0) * seqlen;
 #pragma unroll
-    for (int h = 0; h < 3; h++) {
-      xa[h] = __bfloat162float(st0[h + 1]);
-      xe[h] = __bfloat162float(st1[h + 1]);
+      for (int k = 0; k < 4; k++) {                          // seqlen >= 16: the new window is the last 4 inputs
+        st0[k] = r0[seqlen - 4 + k];
+        st1[k] = r0[2 * (size_t)seqlen - 4 + k];
+      }
+    } else if (wid == 0) {
+      const uint4 h = *reinterpret_cast<const uint4*>(rows - lane * 256 + CW_TILE + lane * 16);
+      pa = make_uint2(h.x, h.y);
+      pe = make_uint2(h.z, h.w);
+    } else {
+      const int o = ((2 * wid - 1) ^ (lane & 7)) << 4;
+      pa = *reinterpret_cast<const uint2*>(rows + o + 8);
+      pe = *reinterpret_cast<const uint2*>(rows + 128 + o + 8);
     }
+    const uint4 wv = *reinterpret_cast<const uint4*>(weight + (size_t)c0 * 4);
+    const uint64_t w0 = pack2(bf16lo(wv.x), bf16lo(wv.z)), w1 = pack2(bf16hi(wv.x), bf16hi(wv.z));
+    const uint64_t w2 = pack2(bf16lo(wv.y), bf16lo(wv.w)), w3 = pack2(bf16hi(wv.y), bf16hi(wv.w));
+    const uint64_t bs = bias ? pack2(__bfloat162float(bias[c0]), __bfloat162float(bias[c0 + 1])) : 0;
+    uint64_t a0 = pack2(bf16hi(pa.x), bf16hi(pe.x)), a1 = pack2(bf16lo(pa.y), bf16lo(pe.y)), a2 = pack2(bf16hi(pa.y), bf16hi(pe.y));
+    __nv_bfloat16* ob = out + ((size_t)b * seqlen + t0) * dim + c0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {                            // seqlen >= 16: the new window is the last 4 inputs
-      st0[k] = r0[seqlen - 4 + k];
-      st1[k] = r1[seqlen - 4 + k];
+    for (int j = 0; j < 2; j++) {
+      if (t0 + 8 * j >= seqlen) break;
+      const int o = ((2 * wid + j) ^ (lane & 7)) << 4;
+      const uint4 ra = *reinterpret_cast<const uint4*>(rows + o), re = *reinterpret_cast<const uint4*>(rows + 128 + o);
+      const uint32_t wa[4] = {ra.x, ra.y, ra.z, ra.w}, we[4] = {re.x, re.y, re.z, re.w};
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const uint64_t a3 = i & 1 ? pack2(bf16hi(wa[i >> 1]), bf16hi(we[i >> 1])) : pack2(bf16lo(wa[i >> 1]), bf16lo(we[i >> 1]));
+        float y0, y1;
+        unpack2(fma2(w3, a3, fma2(w2, a2, fma2(w1, a1, fma2(w0, a0, bs)))), y0, y1);
+        if (ACT) {
+          y0 = silu_fast(y0);
+          y1 = silu_fast(y1);
+        }
+        __nv_bfloat162 pk;
+        pk.x = __float2bfloat16_rn(y0);
+        pk.y = __float2bfloat16_rn(y1);
+        *reinterpret_cast<__nv_bfloat162*>(ob) = pk;
+        ob += dim;
+        a0 = a1; a1 = a2; a2 = a3;
+      }
     }
-  } else {
-    const uint2 pa = *reinterpret_cast<const uint2*>(r0 + t0 - 4);   // tokens t0-4 .. t0-1
-    const uint2 pe = *reinterpret_cast<const uint2*>(r1 + t0 - 4);
-    xa[0] = bf16hi(pa.x); xa[1] = bf16lo(pa.y); xa[2] = bf16hi(pa.y);
-    xe[0] = bf16hi(pe.x); xe[1] = bf16lo(pe.y); xe[2] = bf16hi(pe.y);
-  }
-#pragma unroll
-  for (int j = 0; j < 2 * NG; j++) {
-    const uint32_t wa[4] = {ra[j].x, ra[j].y, ra[j].z, ra[j].w};
-    const uint32_t we[4] = {re[j].x, re[j].y, re[j].z, re[j].w};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      xa[3 + 8 * j + 2 * i] = bf16lo(wa[i]); xa[4 + 8 * j + 2 * i] = bf16hi(wa[i]);
-      xe[3 + 8 * j + 2 * i] = bf16lo(we[i]); xe[4 + 8 * j + 2 * i] = bf16hi(we[i]);
-    }
-  }
-  const uint4 wv = *reinterpret_cast<const uint4*>(weight + (size_t)c0 * 4);
-  const float w00 = bf16lo(wv.x), w01 = bf16hi(wv.x), w02 = bf16lo(wv.y), w03 = bf16hi(wv.y);
-  const float w10 = bf16lo(wv.z), w11 = bf16hi(wv.z), w12 = bf16lo(wv.w), w13 = bf16hi(wv.w);
-  float b0 = 0.f, b1 = 0.f;
-  if (bias) {
-    b0 = __bfloat162float(bias[c0]);
-    b1 = __bfloat162float(bias[c0 + 1]);
-  }
-  __nv_bfloat16* ob = out + ((size_t)b * seqlen + t0) * dim + c0;
-#pragma unroll
-  for (int i = 0; i < NT; i++) {
-    float y0 = fmaf(w03, xa[i + 3], fmaf(w02, xa[i + 2], fmaf(w01, xa[i + 1], fmaf(w00, xa[i], b0))));
-    float y1 = fmaf(w13, xe[i + 3], fmaf(w12, xe[i + 2], fmaf(w11, xe[i + 1], fmaf(w10, xe[i], b1))));
-    if (ACT) {
-      y0 = silu_fast(y0);
-      y1 = silu_fast(y1);
-    }
-    __nv_bfloat162 pk;
-    pk.x = __float2bfloat16_rn(y0);
-    pk.y = __float2bfloat16_rn(y1);
-    *reinterpret_cast<__nv_bfloat162*>(ob + (size_t)i * dim) = pk;
   }
 }
 
@@ -391,11 +450,20 @@ HK_API int hk_conv1d_update(const void* x, void* conv_state, const int* slots, c
   const bool tile_ok = (K == 4) && !history && (dim % CT_CH == 0) && seqlen >= 16 &&
                        aligned(weight, 16) && aligned(out, 4);
   cudaError_t e;
-  if (tile_ok && seqlen % 16 == 0 && aligned(x, 16)) {
-    // one 16-token group per lane: two groups (NG = 2) measured slower (419 vs 367 us at 32K tokens), fewer warps per SM
-    const dim3 grid(dim / CT_CH, (seqlen + CT_TOK - 1) / CT_TOK, bsz);
-    e = pdl_launch(activation ? conv4_row_kernel<true, 1> : conv4_row_kernel<false, 1>, grid, dim3(256), 0, s, xs, st, slots, w, bs, o, dim,
-                   seqlen, state_size);
+  const int tok_tiles = (seqlen + CW_TOK - 1) / CW_TOK;
+  const int64_t tiles = (int64_t)(dim / CT_CH) * tok_tiles * bsz;
+  if (tile_ok && seqlen % 8 == 0 && aligned(x, 16) && tiles < (1 << 30)) {
+    auto kern = activation ? conv4_row_kernel<true> : conv4_row_kernel<false>;
+    static bool attr_set[64][2] = {{false}};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[dev][activation ? 1 : 0]) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CW_SMEM) != cudaSuccess) return HK_ERR_CUDA;
+      if (dev >= 0 && dev < 64) attr_set[dev][activation ? 1 : 0] = true;
+    }
+    const int64_t room = (int64_t)sm_count() * CW_CTAS;
+    e = pdl_launch(kern, dim3((unsigned)(tiles < room ? tiles : room)), dim3(CW_THREADS), CW_SMEM, s, xs, st, slots, w, bs, o, dim, seqlen,
+                   state_size, tok_tiles, (int)tiles);
   } else if (tile_ok) {
     const dim3 grid(dim / CT_CH, (seqlen + CT_TOK - 1) / CT_TOK, bsz);
     e = pdl_launch(activation ? conv4_tile_kernel<true> : conv4_tile_kernel<false>, grid, dim3(256), 0, s, xs, st, slots, w, bs, o, dim,

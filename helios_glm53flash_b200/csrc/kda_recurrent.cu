@@ -503,23 +503,6 @@ static int launch_decode(const DecodeArgs& a, cudaStream_t s) {
 // shuffles for 16 values instead of 64).
 // CPL is the one that yields 256 CTAs or more from 64, 32 and 16 chains.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-
 // Sums of N values per lane over the 16 lanes of a half warp, lanes 8 apart first, then 1, 2, 4.  While a lane has more than
 // one value it keeps one half and hands the other to its partner; a lane ends with the sum of value sum_index (the same in
 // all lanes that agree in the bits used; sum_owner picks one of them).

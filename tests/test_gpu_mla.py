@@ -216,6 +216,27 @@ def test_absorbed_projections_vs_oracle(m):
     assert sum_rel(f(bits(o1)), want_o) < 2e-3 and sum_rel(f(bits(o2)), want_o) < 2e-3
 
 
+@pytest.mark.parametrize("m", [128, 129, 256, 257, 700])
+def test_absorbed_projections_in_row_tiles(m):
+    """256-row tiles of two halves on a persistent grid: full and missing second halves, several tiles per CTA (fp32 reference on
+    the device); rows past m stay untouched"""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    qn, lo = (torch.randn(m, 64, k, generator=g, device="cuda").half() for k in (256, 512))
+    kb = (0.1 * torch.randn(32768, 512, generator=g, device="cuda")).half()
+    ql = torch.full((m + 1, 64, 512), 7.0, dtype=torch.float16, device="cuda")
+    o1, o2 = (torch.full((m + 1, 64, 256), 7.0, dtype=torch.float16, device="cuda") for _ in range(2))
+    wt = torch.empty(64, 512, 256, dtype=torch.float16, device="cuda")
+    hk.q_latent(qn, kb, ql, m)
+    hk.o_absorb(lo, kb, o1, m)
+    hk.wuv_transpose(kb, wt)
+    hk.o_absorb_t(lo, wt, o2, m)
+    w = kb.view(64, 512, 512).float()
+    for got, want in ((ql, torch.einsum("rhk,hkn->rhn", qn.float(), w[:, :256])), (o1, torch.einsum("rhk,hnk->rhn", lo.float(), w[:, 256:])),
+                      (o2, torch.einsum("rhk,hnk->rhn", lo.float(), w[:, 256:]))):
+        assert (got[:m].float() - want).abs().max() < 2e-3 * want.abs().max()
+        assert (got[m] == 7.0).all()
+
+
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 17, 32, 33])
 def test_absorbed_projections_of_few_rows(m):
     """weights-as-M form (up to 32 rows, N = rows rounded up to 8) and the first size beyond it; rows past m stay untouched"""
