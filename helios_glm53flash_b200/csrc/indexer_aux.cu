@@ -11,13 +11,15 @@ __global__ __launch_bounds__(128) void kpool_write_kernel(
     const __half* __restrict__ ik, const __half* __restrict__ ig, __half* __restrict__ ring,
     int raw_rows, __half* __restrict__ pk_nt, const float* __restrict__ ape, int pos_start,
     int n_new, int first_pool) {
-  kpool_one(ik, ig, ring, raw_rows, pk_nt, ape, pos_start, n_new, first_pool + blockIdx.x, threadIdx.x);
+  pdl_wait();
+  kpool_one(ik, ig, ring, raw_rows, pk_nt, ape, pos_start, n_new, first_pool + blockIdx.x, threadIdx.x, [] {});
 }
 
 // raw[r][4i+j] = 4*pool_i + j if <= cur else -1; raw[r][4*n_sel + i] = cur-3+i (>= 0) - the tail
 // is appended without de-duplication, exactly as the reference does.
 __global__ void pool_expand_kernel(const int* __restrict__ pidx, const int* __restrict__ q_pos,
                                    int* __restrict__ raw, int cur_pos, int n_sel) {
+  pdl_wait();
   const int r = blockIdx.x;
   const int cur = q_pos ? q_pos[r] : cur_pos;
   int4* row = reinterpret_cast<int4*>(raw + (size_t)r * (n_sel * POOL + POOL));
@@ -83,11 +85,10 @@ HK_API int hk_kpool_write(const void* idx_k, const void* idx_g, void* raw_ring, 
   HK_REQUIRE(raw_rows >= n_new + (POOL - 1) || raw_rows >= pos_start + n_new);
   const int first_pool = pos_start / POOL;
   const int last_pool = (pos_start + n_new - 1) / POOL;
-  kpool_write_kernel<<<last_pool - first_pool + 1, 128, 0, as_stream(stream)>>>(
-      (const __half*)idx_k, (const __half*)idx_g, (__half*)raw_ring, raw_rows, (__half*)pool_k_nt,
-      ape, pos_start, n_new, first_pool);
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  return pdl_launch(kpool_write_kernel, dim3(last_pool - first_pool + 1), dim3(128), 0, as_stream(stream), (const __half*)idx_k,
+                    (const __half*)idx_g, (__half*)raw_ring, raw_rows, (__half*)pool_k_nt, ape, pos_start, n_new, first_pool) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 HK_API int hk_pool_expand(const int* pool_idx, const int* q_pos, int* raw_idx, int m, int cur_pos,
@@ -96,9 +97,9 @@ HK_API int hk_pool_expand(const int* pool_idx, const int* q_pos, int* raw_idx, i
   HK_REQUIRE(pool_idx && raw_idx && m >= 0 && n_sel > 0);
   HK_REQUIRE(aligned(raw_idx, 16));
   if (m == 0) return HK_OK;
-  pool_expand_kernel<<<m, 256, 0, as_stream(stream)>>>(pool_idx, q_pos, raw_idx, cur_pos, n_sel);
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  return pdl_launch(pool_expand_kernel, dim3(m), dim3(256), 0, as_stream(stream), pool_idx, q_pos, raw_idx, cur_pos, n_sel) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 HK_API int hk_indexer_score_legacy(const void* q_idx, const void* pool_k, const void* w,

@@ -33,9 +33,13 @@ __device__ __forceinline__ void append_row(const float* __restrict__ kv_row, con
                                            __half* __restrict__ dst_row, __half* __restrict__ dst2_row, float eps, int lane) {
   const float4* xr = reinterpret_cast<const float4*>(kv_row);
   float4 x[4];
+  uint2 lw[4];
   float s[4];
 #pragma unroll
-  for (int w = 0; w < 4; w++) x[w] = xr[w * 32 + lane];
+  for (int w = 0; w < 4; w++) {
+    x[w] = xr[w * 32 + lane];
+    lw[w] = reinterpret_cast<const uint2*>(ln_w)[w * 32 + lane];
+  }
 #pragma unroll
   for (int w = 0; w < 4; w++) {
     float t = 0.f;
@@ -51,7 +55,7 @@ __device__ __forceinline__ void append_row(const float* __restrict__ kv_row, con
   uint2* dst2 = dst2_row ? reinterpret_cast<uint2*>(dst2_row) : nullptr;
 #pragma unroll
   for (int w = 0; w < 4; w++) {
-    const float4 w4 = half4_to_float4(reinterpret_cast<const uint2*>(ln_w)[w * 32 + lane]);
+    const float4 w4 = half4_to_float4(lw[w]);
     float4 o;
     o.x = x[w].x * w4.x * rmf;
     o.y = x[w].y * w4.y * rmf;
@@ -67,6 +71,7 @@ __global__ void __launch_bounds__(256) mla_cache_append_kernel(const float* __re
                                                                const __half* __restrict__ ln_w,
                                                                __half* __restrict__ ckv, __half* __restrict__ ckv_new,
                                                                long long pos, int n, float eps) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (row >= n) return;
@@ -74,16 +79,32 @@ __global__ void __launch_bounds__(256) mla_cache_append_kernel(const float* __re
              ckv_new ? ckv_new + (size_t)row * LATENT : nullptr, eps, lane);
 }
 
-// one warp; xr and yr may alias; y2 (optional) receives the same row (any address space)
+// one warp; xr and yr may alias; y2 (optional) receives the same row (any address space).  DIM 128: one value of each of the
+// reference's four warps per lane, all loads at once (4.7 us for a handful of rows with a loop around every load); 0: any dim.
+template <int DIM>
 __device__ __forceinline__ void layernorm_row(const __half* xr, const __half* __restrict__ w, const __half* __restrict__ b,
                                               __half* yr, __half* y2, int dim, float eps, int lane) {
   float s1[4], s2[4];
+  __half xv[4], wv[4], bv[4];
+  if (DIM == 128) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      xv[q] = xr[q * 32 + lane];
+      wv[q] = w[q * 32 + lane];
+      bv[q] = b[q * 32 + lane];
+    }
+  }
 #pragma unroll
   for (int q = 0; q < 4; q++) {                            // lane `lane` of the reference's warp q
     float sum = 0, sq = 0;
-    for (int i = q * 32 + lane; i < dim; i += 128) {
-      float v = __half2float(xr[i]);
+    if (DIM == 128) {
+      const float v = __half2float(xv[q]);
       sum += v; sq += v * v;
+    } else {
+      for (int i = q * 32 + lane; i < dim; i += 128) {
+        float v = __half2float(xr[i]);
+        sum += v; sq += v * v;
+      }
     }
     s1[q] = warp_sum(sum);
     s2[q] = warp_sum(sq);
@@ -92,21 +113,28 @@ __device__ __forceinline__ void layernorm_row(const __half* xr, const __half* __
   const float m0 = a / dim, m1 = c / dim;
   float mean = m0, var = m1 - mean * mean;
   float inv = rsqrtf(var + eps);
-  for (int i = lane; i < dim; i += 32) {
-    float v = (__half2float(xr[i]) - mean) * inv * __half2float(w[i]) + __half2float(b[i]);
-    const __half h = __float2half_rn(v);
+  auto put = [&](int i, __half x, __half wi, __half bi) {
+    const __half h = __float2half_rn((__half2float(x) - mean) * inv * __half2float(wi) + __half2float(bi));
     if (yr) yr[i] = h;
     if (y2) y2[i] = h;
+  };
+  if (DIM == 128) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) put(q * 32 + lane, xv[q], wv[q], bv[q]);
+  } else {
+    for (int i = lane; i < dim; i += 32) put(i, xr[i], w[i], b[i]);
   }
 }
 
+template <int DIM>
 __global__ void __launch_bounds__(256) layernorm_f16_kernel(const __half* x, const __half* __restrict__ w,   // x and y may alias
                                                             const __half* __restrict__ b, __half* y,
                                                             int rows, int dim, float eps) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (row >= rows) return;
-  layernorm_row(x + (size_t)row * dim, w, b, y + (size_t)row * dim, nullptr, dim, eps, lane);
+  layernorm_row<DIM>(x + (size_t)row * dim, w, b, y + (size_t)row * dim, nullptr, DIM ? DIM : dim, eps, lane);
 }
 
 // Everything an MLA layer does with ONE new token before its attention, in one launch of one CTA: the latent row is
@@ -122,10 +150,10 @@ __global__ void __launch_bounds__(128) mla_decode_prologue_kernel(
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_wait();
   if (warp == 0) append_row(kv_pre, ln_w, ckv + (size_t)pos * LATENT, nullptr, eps_rms, lane);
-  if (warp == 1) layernorm_row(idx_k, knorm_w, knorm_b, idx_kn, s_kn, 128, eps_ln, lane);
+  if (warp == 1) layernorm_row<128>(idx_k, knorm_w, knorm_b, idx_kn, s_kn, 128, eps_ln, lane);
   if (threadIdx.x == 64 && q_pos_out) *q_pos_out = pos;
-  __syncthreads();
-  kpool_one(s_kn, idx_g, ring, raw_rows, pk_nt, ape, pos, 1, pos / POOL, threadIdx.x);
+  // every thread's gates, earlier members and weights are on their way while warps 0 and 1 still normalise
+  kpool_one(s_kn, idx_g, ring, raw_rows, pk_nt, ape, pos, 1, pos / POOL, threadIdx.x, [] { __syncthreads(); });
 }
 
 }  // namespace
@@ -137,22 +165,22 @@ HK_API int hk_mla_cache_append(const float* kv_pre, const void* ln_w_f16, void* 
   HK_REQUIRE(hk::aligned(kv_pre, 16) && hk::aligned(ln_w_f16, 8) && hk::aligned(ckv, 8) &&
              (!ckv_new || hk::aligned(ckv_new, 8)));
   if (n == 0) return HK_OK;
-  hk::mla_cache_append_kernel<<<(n + 7) / 8, 256, 0, hk::as_stream(stream)>>>(
-      kv_pre, static_cast<const __half*>(ln_w_f16), static_cast<__half*>(ckv), static_cast<__half*>(ckv_new), pos, n,
-      epsilon);
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  return hk::pdl_launch(hk::mla_cache_append_kernel, dim3((n + 7) / 8), dim3(256), 0, hk::as_stream(stream), kv_pre,
+                        static_cast<const __half*>(ln_w_f16), static_cast<__half*>(ckv), static_cast<__half*>(ckv_new), pos, n,
+                        epsilon) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 HK_API int hk_layernorm_f16(const void* x, const void* w, const void* b, void* y, int rows, int dim,
                             float epsilon, void* stream) {
   HK_REQUIRE(x && w && b && y && rows >= 0 && dim > 0);
   if (rows == 0) return HK_OK;
-  hk::layernorm_f16_kernel<<<(rows + 7) / 8, 256, 0, hk::as_stream(stream)>>>(
-      static_cast<const __half*>(x), static_cast<const __half*>(w), static_cast<const __half*>(b),
-      static_cast<__half*>(y), rows, dim, epsilon);
-  HK_LAUNCH_CHECK();
-  return HK_OK;
+  return hk::pdl_launch(dim == 128 ? hk::layernorm_f16_kernel<128> : hk::layernorm_f16_kernel<0>, dim3((rows + 7) / 8), dim3(256), 0,
+                        hk::as_stream(stream), static_cast<const __half*>(x), static_cast<const __half*>(w), static_cast<const __half*>(b),
+                        static_cast<__half*>(y), rows, dim, epsilon) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 HK_API int hk_mla_decode_prologue(const float* kv_pre, const void* ln_w_f16, void* ckv, float eps_rms, const void* idx_k,
