@@ -3,122 +3,22 @@
 // (reference: src/cuda/aux/gdn.cu:880-1023): fp32 fma chain k ascending, SiLU as a * 1/(1+exp(-a)),
 // bf16 round-to-nearest output, state = last K inputs.
 //
-// Four kernels (the last one is the fused cast + convolution over token-major fp32 input, further below):
-//   conv4_row_kernel   prefill with whole 8-token pieces: K = 4, no history, seqlen % 8 == 0.  Persistent CTAs over
-//                      [64 channel][64 token] tiles: asynchronous 16-byte copies into a three-stage ring, a lane computes 2
-//                      channels x 16 tokens (128-byte warp stores per output row).
-//   conv4_tile_kernel  other prefill lengths: a CTA transposes a [64 channel][128 token] tile
-//                      through shared memory: 16-byte reads along tokens (the input is channel-major),
-//                      128-byte coalesced writes along channels (the output is token-major).  The rows of a
-//                      length that is no multiple of 8 start anywhere: they are read as the aligned 16-byte
-//                      pieces that cover them (2-byte loads, 32 per thread, before: 6.5 us for 37 tokens x 24,576
-//                      channels).  HBM-bound: 2 B read + 2 B written per channel-token.
+// Three kernels (the last one is the fused cast + convolution over token-major fp32 input, further below):
+//   conv4_row_kernel    prefill (K = 4, no history, 16 tokens or more): persistent CTAs over [64 channel][64 token] tiles,
+//                       asynchronous 16-byte copies into a three-stage ring, a lane computes 2 channels x 16 tokens
+//                       (128-byte warp stores per output row).
 //   conv_generic_kernel decode and every other case (any K <= 16, history, ragged shapes): one
-//                      thread per channel; with seqlen = 1 its accesses are contiguous in channels.
+//                       thread per channel; with seqlen = 1 its accesses are contiguous in channels.
 #include "hk_common.cuh"
 
 namespace hk {
 
 constexpr int CONV_MAX_K = 16;
 constexpr int CT_CH = 64;       // channels per tile
-constexpr int CT_TOK = 128;     // tokens per tile
-constexpr int CT_STRIDE = 146;  // bf16 elements per shared row: 8 halo slots + 17 pieces of 8 + 2 pad
-                                // (73 words, odd, so channel-strided reads spread over the banks)
 
 __device__ __forceinline__ float silu_fast(float a) { return a * (1.0f / (1.0f + __expf(-a))); }
 
-template <bool ACT>
-__global__ __launch_bounds__(256) void conv4_tile_kernel(
-    const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ state,
-    const int* __restrict__ slots, const __nv_bfloat16* __restrict__ weight,
-    const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, int dim, int seqlen,
-    int state_size) {
-  __shared__ __align__(16) __nv_bfloat16 xs[CT_CH * CT_STRIDE];
-  const int d0 = blockIdx.x * CT_CH;
-  const int s0 = blockIdx.y * CT_TOK;
-  const int b = blockIdx.z;
-  const int tid = threadIdx.x;
-  const __nv_bfloat16* xb = x + ((size_t)b * dim + d0) * seqlen;
-
-  pdl_wait();
-  // ---- stage the tile: rows = channels.  Piece c of row r covers tokens s0 - lead + 8 c ..., lead = elements between the
-  //      16-byte boundary and token s0 of that row; token s sits in column 8 + lead + (s - s0).  Pieces that reach over an
-  //      end of the row or of the tile are copied element by element. ----
-  const int s_end = min(seqlen, s0 + CT_TOK);
-  auto row_lead = [&](int r) { return (int)((reinterpret_cast<uintptr_t>(xb + (size_t)r * seqlen + s0) & 15) >> 1); };
-  for (int idx = tid; idx < CT_CH * 17; idx += 256) {
-    const int r = idx / 17, c = idx - r * 17;
-    const __nv_bfloat16* src = xb + (size_t)r * seqlen;
-    const int s = s0 - row_lead(r) + 8 * c;
-    __nv_bfloat16* dst = xs + r * CT_STRIDE + 8 + c * 8;
-    if (s >= s0 && s + 8 <= s_end) {
-      const uint4 v = ld_stream16(src + s);
-      uint32_t* d4 = reinterpret_cast<uint32_t*>(dst);
-      d4[0] = v.x; d4[1] = v.y; d4[2] = v.z; d4[3] = v.w;
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; e++)
-        if (s + e >= s0 && s + e < s_end) dst[e] = src[s + e];
-    }
-  }
-  // ---- halo (3 tokens before the tile) and, in the first tile, the state update ----
-  if (tid < CT_CH) {
-    const int r = tid;
-    __nv_bfloat16* hrow = xs + r * CT_STRIDE + 5 + row_lead(r);
-    if (s0 == 0) {
-      const int slot = slots ? slots[b] : b;
-      __nv_bfloat16* st = state + ((size_t)slot * dim + d0 + r) * state_size;
-      __nv_bfloat16 old[4] = {st[0], st[1], st[2], st[3]};
-      hrow[0] = old[1]; hrow[1] = old[2]; hrow[2] = old[3];
-      // new window = last 4 entries of [old(4) | x(seqlen)]
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        int src_t = seqlen + k;
-        st[k] = (src_t < 4) ? old[src_t] : xb[(size_t)r * seqlen + (src_t - 4)];
-      }
-    } else {
-#pragma unroll
-      for (int h = 0; h < 3; h++) hrow[h] = xb[(size_t)r * seqlen + (s0 - 3 + h)];
-    }
-  }
-  __syncthreads();
-
-  // ---- compute: lane owns 2 adjacent channels; the warps share the tile's tokens evenly (16 each in a whole tile) ----
-  const int lane = tid & 31, wid = tid >> 5;
-  const int c0 = lane * 2;
-  const uint4 wv = *reinterpret_cast<const uint4*>(weight + (size_t)(d0 + c0) * 4);
-  const float w00 = bf16lo(wv.x), w01 = bf16hi(wv.x), w02 = bf16lo(wv.y), w03 = bf16hi(wv.y);
-  const float w10 = bf16lo(wv.z), w11 = bf16hi(wv.z), w12 = bf16lo(wv.w), w13 = bf16hi(wv.w);
-  float b0 = 0.f, b1 = 0.f;
-  if (bias) {
-    b0 = __bfloat162float(bias[d0 + c0]);
-    b1 = __bfloat162float(bias[d0 + c0 + 1]);
-  }
-  const __nv_bfloat16* r0 = xs + c0 * CT_STRIDE + 8 + row_lead(c0);
-  const __nv_bfloat16* r1 = xs + (c0 + 1) * CT_STRIDE + 8 + row_lead(c0 + 1);
-  const int n_tok = s_end - s0, per = (n_tok + 7) >> 3, t0 = wid * per;
-  float a0 = __bfloat162float(r0[t0 - 3]), a1 = __bfloat162float(r0[t0 - 2]), a2 = __bfloat162float(r0[t0 - 1]);
-  float e0 = __bfloat162float(r1[t0 - 3]), e1 = __bfloat162float(r1[t0 - 2]), e2 = __bfloat162float(r1[t0 - 1]);
-  __nv_bfloat16* ob = out + ((size_t)b * seqlen) * dim + d0 + c0;
-#pragma unroll 4
-  for (int t = t0; t < min(t0 + per, n_tok); t++) {
-    float a3 = __bfloat162float(r0[t]), e3 = __bfloat162float(r1[t]);
-    float y0 = fmaf(w03, a3, fmaf(w02, a2, fmaf(w01, a1, fmaf(w00, a0, b0))));
-    float y1 = fmaf(w13, e3, fmaf(w12, e2, fmaf(w11, e1, fmaf(w10, e0, b1))));
-    if (ACT) {
-      y0 = silu_fast(y0);
-      y1 = silu_fast(y1);
-    }
-    __nv_bfloat162 pk;
-    pk.x = __float2bfloat16_rn(y0);
-    pk.y = __float2bfloat16_rn(y1);
-    *reinterpret_cast<__nv_bfloat162*>(ob + (size_t)(s0 + t) * dim) = pk;
-    a0 = a1; a1 = a2; a2 = a3;
-    e0 = e1; e1 = e2; e2 = e3;
-  }
-}
-
-// Prefill with whole 8-token pieces (seqlen % 8 == 0, so every channel row starts on 16 bytes).  2 B are read and 2 B written
+// Prefill.  2 B are read and 2 B written
 // per channel-token; what a transposing access pattern reaches depends on the length of its runs, and the SiLU's exponential
 // and reciprocal (230 us at 32,768 tokens x 12,288 channels on the special-function units alone) have to run under the copies.
 // With 32 bytes per channel row and lane, straight into registers, that size took 362 us (4.45 TB/s; runs of 128 bytes copy in
@@ -127,16 +27,22 @@ __global__ __launch_bounds__(256) void conv4_tile_kernel(
 // row) and the reads (32 lanes on rows 2 l and 2 l + 1) free of bank conflicts.  Small CTAs because one's barrier then stalls
 // only four warps: 64-token tiles and six CTAs per SM 324 us, 128-token tiles and three or four 339, 353; five 345, eight 434
 // (too many streams for the memory).
+// RAGGED: the rows of a length that is no multiple of 8 start anywhere.  Then a row of the tile is the aligned 16-byte pieces
+// that cover the 4 tokens before it and its own, up to ten, and is read word by word, rows that start on an odd element through
+// a 16-bit funnel shift.  Rows lie 11 pieces apart, even ones first, so that the words of 32 lanes spread over all banks.  One
+// element per load before: 690 -> 407 us at 32,763 tokens, 27.4 -> 17.1 at 1,003.
 constexpr int CW_TOK = 64, CW_THREADS = CW_TOK * 2, CW_STAGES = 3, CW_CTAS = 6;
-constexpr uint32_t CW_TILE = CT_CH * CW_TOK * 2, CW_STAGE = CW_TILE + CT_CH * 8;   // 8 KB and the 4 tokens before each row
-constexpr uint32_t CW_SMEM = CW_STAGES * CW_STAGE;
+constexpr uint32_t CW_TILE = CT_CH * CW_TOK * 2, CW_PITCH = 11 * 16;
+// 8 KB and the 4 tokens before each row, or 64 rows of up to ten pieces
+__host__ __device__ constexpr uint32_t cw_stage(bool ragged) { return ragged ? CT_CH * CW_PITCH : CW_TILE + CT_CH * 8; }
 
-template <bool ACT>
+template <bool ACT, bool RAGGED>
 __global__ __launch_bounds__(CW_THREADS, CW_CTAS) void conv4_row_kernel(
     const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ state,
     const int* __restrict__ slots, const __nv_bfloat16* __restrict__ weight,
     const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, int dim, int seqlen,
-    int state_size, int tok_tiles, int total) {
+    int state_size, int tok_tiles, int total, size_t n_elem) {
+  constexpr uint32_t CW_STAGE = cw_stage(RAGGED);
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(smem_raw);
@@ -164,11 +70,32 @@ __global__ __launch_bounds__(CW_THREADS, CW_CTAS) void conv4_row_kernel(
   const size_t row16 = (size_t)seqlen * 16;
   auto copy_in = [&](const Place& p, int stage) {
     const __nv_bfloat16* xb = x + ((size_t)p.b * dim + p.c * CT_CH) * seqlen + p.s * CW_TOK;
+    if (RAGGED) {
+#pragma unroll
+      for (int i = 0; i < 5; i++) {                          // pieces 0-7 with eight lanes to a row, then 8 and 9
+        const int r = i < 4 ? cr + 16 * i : tid >> 1, pc = i < 4 ? cp : 8 + (tid & 1);
+        const uintptr_t row = reinterpret_cast<uintptr_t>(xb + (size_t)r * seqlen);
+        const uintptr_t src = ((row - 8) & ~(uintptr_t)15) + 16 * pc;
+        if (src >= row + 2 * min(CW_TOK, seqlen - p.s * CW_TOK)) continue;
+        const uint32_t to = stage * CW_STAGE + ((r >> 1) + 32 * (r & 1)) * CW_PITCH + 16 * pc;
+        if (src >= reinterpret_cast<uintptr_t>(x) && src + 16 <= reinterpret_cast<uintptr_t>(x + n_elem)) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sm0 + to), "l"(src) : "memory");
+        } else {                                             // over an end of the whole input: element by element
+#pragma unroll
+          for (int e = 0; e < 8; e++) {
+            const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(src) + e;
+            if (q >= x && q < x + n_elem) reinterpret_cast<__nv_bfloat16*>(smem_raw + to)[e] = *q;
+          }
+        }
+      }
+      return;
+    }
     if (p.s * CW_TOK + 8 * cp < seqlen) {
       const __nv_bfloat16* src = xb + (size_t)cr * seqlen + 8 * cp;
 #pragma unroll
-      for (int i = 0; i < 4; i++) 
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + stage * CW_STAGE + i * 2048), "l"(src + i * row16) : "memory");
+      for (int i = 0; i < 4; i++)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + stage * CW_STAGE + i * 2048), "l"(src + i * row16)
+                     : "memory");
     }
     if (tid < CT_CH && p.s > 0)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sm0 + stage * CW_STAGE + CW_TILE + tid * 8),
@@ -197,7 +124,7 @@ __global__ __launch_bounds__(CW_THREADS, CW_CTAS) void conv4_row_kernel(
     advance(in);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const int c0 = at.c * CT_CH + lane * 2, b = at.b;
-    const uint8_t* rows = smem_raw + stage * CW_STAGE + lane * 256;   // channels c0 and c0 + 1
+    const uint8_t* rows = smem_raw + stage * CW_STAGE + lane * (RAGGED ? CW_PITCH : 256);   // channels c0 and c0 + 1
     const int t0 = at.s * CW_TOK + wid * 16;
     stage = stage == CW_STAGES - 1 ? 0 : stage + 1;
     if (t0 >= seqlen) continue;                              // warp-uniform
@@ -217,14 +144,48 @@ __global__ __launch_bounds__(CW_THREADS, CW_CTAS) void conv4_row_kernel(
         st0[k] = r0[seqlen - 4 + k];
         st1[k] = r0[2 * (size_t)seqlen - 4 + k];
       }
-    } else if (wid == 0) {
-      const uint4 h = *reinterpret_cast<const uint4*>(rows - lane * 256 + CW_TILE + lane * 16);
-      pa = make_uint2(h.x, h.y);
-      pe = make_uint2(h.z, h.w);
+    } else if (!RAGGED) {
+      if (wid == 0) {
+        const uint4 h = *reinterpret_cast<const uint4*>(rows - lane * 256 + CW_TILE + lane * 16);
+        pa = make_uint2(h.x, h.y);
+        pe = make_uint2(h.z, h.w);
+      } else {
+        const int o = ((2 * wid - 1) ^ (lane & 7)) << 4;
+        pa = *reinterpret_cast<const uint2*>(rows + o + 8);
+        pe = *reinterpret_cast<const uint2*>(rows + 128 + o + 8);
+      }
+    }
+    uint32_t wa[8], we[8];                                   // 16 tokens of either channel
+    if (RAGGED) {
+      uint32_t v[2][11];                                     // from token t0 - 4 (or the element before it) on
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const uintptr_t row = reinterpret_cast<uintptr_t>(x + ((size_t)b * dim + c0 + h) * seqlen + at.s * CW_TOK) - 8;
+        const int lead = (int)(row & 15) >> 1;
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(rows + h * 32 * CW_PITCH) + (lead >> 1) + wid * 8;
+#pragma unroll
+        for (int i = 0; i < 11; i++) v[h][i] = src[i];
+        const uint32_t sh = 16 * (lead & 1);
+#pragma unroll
+        for (int i = 0; i < 10; i++) v[h][i] = __funnelshift_r(v[h][i], v[h][i + 1], sh);
+      }
+      if (t0 > 0) {
+        pa = make_uint2(v[0][0], v[0][1]);
+        pe = make_uint2(v[1][0], v[1][1]);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        wa[i] = v[0][2 + i];
+        we[i] = v[1][2 + i];
+      }
     } else {
-      const int o = ((2 * wid - 1) ^ (lane & 7)) << 4;
-      pa = *reinterpret_cast<const uint2*>(rows + o + 8);
-      pe = *reinterpret_cast<const uint2*>(rows + 128 + o + 8);
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const int o = ((2 * wid + j) ^ (lane & 7)) << 4;
+        const uint4 ra = *reinterpret_cast<const uint4*>(rows + o), re = *reinterpret_cast<const uint4*>(rows + 128 + o);
+        wa[4 * j] = ra.x; wa[4 * j + 1] = ra.y; wa[4 * j + 2] = ra.z; wa[4 * j + 3] = ra.w;
+        we[4 * j] = re.x; we[4 * j + 1] = re.y; we[4 * j + 2] = re.z; we[4 * j + 3] = re.w;
+      }
     }
     const uint4 wv = *reinterpret_cast<const uint4*>(weight + (size_t)c0 * 4);
     const uint64_t w0 = pack2(bf16lo(wv.x), bf16lo(wv.z)), w1 = pack2(bf16hi(wv.x), bf16hi(wv.z));
@@ -233,27 +194,22 @@ __global__ __launch_bounds__(CW_THREADS, CW_CTAS) void conv4_row_kernel(
     uint64_t a0 = pack2(bf16hi(pa.x), bf16hi(pe.x)), a1 = pack2(bf16lo(pa.y), bf16lo(pe.y)), a2 = pack2(bf16hi(pa.y), bf16hi(pe.y));
     __nv_bfloat16* ob = out + ((size_t)b * seqlen + t0) * dim + c0;
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-      if (t0 + 8 * j >= seqlen) break;
-      const int o = ((2 * wid + j) ^ (lane & 7)) << 4;
-      const uint4 ra = *reinterpret_cast<const uint4*>(rows + o), re = *reinterpret_cast<const uint4*>(rows + 128 + o);
-      const uint32_t wa[4] = {ra.x, ra.y, ra.z, ra.w}, we[4] = {re.x, re.y, re.z, re.w};
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const uint64_t a3 = i & 1 ? pack2(bf16hi(wa[i >> 1]), bf16hi(we[i >> 1])) : pack2(bf16lo(wa[i >> 1]), bf16lo(we[i >> 1]));
-        float y0, y1;
-        unpack2(fma2(w3, a3, fma2(w2, a2, fma2(w1, a1, fma2(w0, a0, bs)))), y0, y1);
-        if (ACT) {
-          y0 = silu_fast(y0);
-          y1 = silu_fast(y1);
-        }
-        __nv_bfloat162 pk;
-        pk.x = __float2bfloat16_rn(y0);
-        pk.y = __float2bfloat16_rn(y1);
-        *reinterpret_cast<__nv_bfloat162*>(ob) = pk;
-        ob += dim;
-        a0 = a1; a1 = a2; a2 = a3;
+    for (int i = 0; i < 16; i++) {
+      if ((RAGGED || i == 8) && t0 + i >= seqlen) break;
+      const uint32_t a = wa[i >> 1], e = we[i >> 1];
+      const uint64_t a3 = i & 1 ? pack2(bf16hi(a), bf16hi(e)) : pack2(bf16lo(a), bf16lo(e));
+      float y0, y1;
+      unpack2(fma2(w3, a3, fma2(w2, a2, fma2(w1, a1, fma2(w0, a0, bs)))), y0, y1);
+      if (ACT) {
+        y0 = silu_fast(y0);
+        y1 = silu_fast(y1);
       }
+      __nv_bfloat162 pk;
+      pk.x = __float2bfloat16_rn(y0);
+      pk.y = __float2bfloat16_rn(y1);
+      *reinterpret_cast<__nv_bfloat162*>(ob) = pk;
+      ob += dim;
+      a0 = a1; a1 = a2; a2 = a3;
     }
   }
 }
@@ -452,22 +408,22 @@ HK_API int hk_conv1d_update(const void* x, void* conv_state, const int* slots, c
   cudaError_t e;
   const int tok_tiles = (seqlen + CW_TOK - 1) / CW_TOK;
   const int64_t tiles = (int64_t)(dim / CT_CH) * tok_tiles * bsz;
-  if (tile_ok && seqlen % 8 == 0 && aligned(x, 16) && tiles < (1 << 30)) {
-    auto kern = activation ? conv4_row_kernel<true> : conv4_row_kernel<false>;
-    static bool attr_set[64][2] = {{false}};
+  if (tile_ok && tiles < (1 << 30)) {
+    const bool ragged = seqlen % 8 != 0 || !aligned(x, 16);
+    auto kern = activation ? (ragged ? conv4_row_kernel<true, true> : conv4_row_kernel<true, false>)
+                           : (ragged ? conv4_row_kernel<false, true> : conv4_row_kernel<false, false>);
+    const uint32_t smem = CW_STAGES * cw_stage(ragged);
+    static bool attr_set[64][4] = {{false}};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !attr_set[dev][activation ? 1 : 0]) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CW_SMEM) != cudaSuccess) return HK_ERR_CUDA;
-      if (dev >= 0 && dev < 64) attr_set[dev][activation ? 1 : 0] = true;
+    const int form = (activation ? 2 : 0) + ragged;
+    if (dev < 0 || dev >= 64 || !attr_set[dev][form]) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return HK_ERR_CUDA;
+      if (dev >= 0 && dev < 64) attr_set[dev][form] = true;
     }
     const int64_t room = (int64_t)sm_count() * CW_CTAS;
-    e = pdl_launch(kern, dim3((unsigned)(tiles < room ? tiles : room)), dim3(CW_THREADS), CW_SMEM, s, xs, st, slots, w, bs, o, dim, seqlen,
-                   state_size, tok_tiles, (int)tiles);
-  } else if (tile_ok) {
-    const dim3 grid(dim / CT_CH, (seqlen + CT_TOK - 1) / CT_TOK, bsz);
-    e = pdl_launch(activation ? conv4_tile_kernel<true> : conv4_tile_kernel<false>, grid, dim3(256), 0, s, xs, st, slots, w, bs, o, dim,
-                   seqlen, state_size);
+    e = pdl_launch(kern, dim3((unsigned)(tiles < room ? tiles : room)), dim3(CW_THREADS), smem, s, xs, st, slots, w, bs, o, dim, seqlen,
+                   state_size, tok_tiles, (int)tiles, (size_t)bsz * dim * seqlen);
   } else {
     auto kern = activation ? (history ? conv_generic_kernel<true, true> : conv_generic_kernel<true, false>)
                            : (history ? conv_generic_kernel<false, true> : conv_generic_kernel<false, false>);

@@ -37,6 +37,20 @@ def test_conv_vs_oracle_and_reference(dim, T):
         assert np.array_equal(g_out, r_out), "same arithmetic as the reference kernel: bit-exact"
 
 
+@pytest.mark.parametrize("bsz,T", [(1, 16), (2, 17), (1, 24), (1, 63), (3, 65), (2, 68), (1, 72), (2, 129), (1, 190)])
+def test_conv_at_the_edges_of_its_tiles(bsz, T):
+    """64-token tiles of 16-token groups: rows that start on 16 bytes, on an even and on an odd element, and several sequences"""
+    dim = 192
+    x = synth.f32_to_bf16_bits(synth.rng(T).standard_normal((bsz, dim, T), dtype=np.float32))
+    st = synth.f32_to_bf16_bits(synth.rng(T + 1).standard_normal((bsz, dim, 4), dtype=np.float32))
+    w = synth.f32_to_bf16_bits(synth.rng(T + 2).standard_normal((dim, 4), dtype=np.float32))
+    o_out, o_st = orc.conv1d_update(x, st, w, None, bsz, dim, T, 4, 4)
+    g_out, g_st = _run_conv(x, st, w, bsz, dim, T)
+    assert np.array_equal(g_st.reshape(-1), o_st.reshape(-1))
+    ulp = bf16_ulp_diff(g_out.reshape(-1), o_out.reshape(-1))
+    assert ulp.max() <= 1 and (ulp > 0).mean() < 5e-3
+
+
 def test_conv_history_and_generic_k():
     dim, T, K, S = 96, 9, 3, 7
     inp = synth.conv_inputs(T, dim, K=K, seed=5)
