@@ -242,6 +242,8 @@ __global__ __launch_bounds__(TK_THREADS) void dsa_topk_kernel(
 // and small CTAs share an SM and hide one another's.  1,024 rows x 1,250 scores 19.3 -> 8.4 us, 1,024 x 4,096 20.3 -> 11.1,
 // 4,096 x 8,192 102 -> 66, 1,024 x 16,000 43.5 -> 36.4.  (More pieces per thread instead of more threads: 128 registers and
 // spills, 1,024 x 8,191 40.7 us; 1,024 threads for 32,000 scores: 83 us against 74.)
+// Up to a row per SM nothing is shared and the time is one CTA's: 1,024 threads with one or two pieces each, 1 x 5,000 scores
+// 7.3 -> 4.6 us, 1 x 16,000 8.2 -> 6.5, 140 x 8,000 7.3 -> 5.0.
 // ------------------------------------------------------------------------------------------------
 constexpr int TKR_MAX_THREADS = 512, TKR_MAX_PIECES = 4 * TKR_MAX_THREADS;
 
@@ -258,13 +260,13 @@ __device__ __forceinline__ void for_keys(const uint4 (&pc)[NP], F f) {
 }
 
 template <int NP, int FIXED>   // FIXED: threads of the CTA, 0 = as launched
-__global__ __launch_bounds__(FIXED ? FIXED : TKR_MAX_THREADS, FIXED ? 4 : 2) void dsa_topk_rows_kernel(const uint16_t* scores, int* __restrict__ out, int T, int s_stride,
+__global__ __launch_bounds__(FIXED ? FIXED : TKR_MAX_THREADS, FIXED == 1024 ? 1 : FIXED ? 4 : 2) void dsa_topk_rows_kernel(const uint16_t* scores, int* __restrict__ out, int T, int s_stride,
                                                                     int k, int k_pad, int* __restrict__ raw,
                                                                     const int* __restrict__ q_pos) {
   constexpr int NB = 8;                                    // buckets of each of the first 256 threads
   __shared__ __align__(16) int hist[2048];
   __shared__ int low[32];
-  __shared__ int wsum[2][TKR_MAX_THREADS / 32];
+  __shared__ int wsum[2][32];
   __shared__ int sel[2];                                   // crossing bucket, count above it
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, threads = FIXED ? FIXED : blockDim.x, warps = threads >> 5;
   const uint16_t* row = scores + (size_t)blockIdx.x * s_stride;
@@ -289,13 +291,8 @@ __global__ __launch_bounds__(FIXED ? FIXED : TKR_MAX_THREADS, FIXED ? 4 : 2) voi
     }
     if (lane == 31) wsum[slot][warp] = incl;
     __syncthreads();
-    int before = 0, all = 0;
-#pragma unroll 8
-    for (int w = 0; w < warps; w++) {
-      const int x = wsum[slot][w];
-      before += w < warp ? x : 0;
-      all += x;
-    }
+    const int x = lane < warps ? wsum[slot][lane] : 0;
+    const int before = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < warp ? x : 0)), all = (int)__reduce_add_sync(0xffffffffu, (unsigned)x);
     *total = all;
     return before + incl - v;
   };
@@ -559,10 +556,12 @@ static int topk_launch(const void* scores, int s_stride, int* indices, int R, in
                                      : (pieces <= 2 * TKC_PIECES ? dsa_topk_cluster_kernel<2> : dsa_topk_cluster_kernel<4>);
     e = pdl_launch(kern, dim3(R * TKC_CTAS), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
   } else if (pieces <= TKR_MAX_PIECES && !t_ptr) {
+    const bool few = R <= sm_count();
     auto kern = pieces <= 256    ? dsa_topk_rows_kernel<1, 256>
+                : few            ? (pieces <= 1024 ? dsa_topk_rows_kernel<1, 1024> : dsa_topk_rows_kernel<2, 1024>)
                 : pieces <= 512  ? dsa_topk_rows_kernel<2, 256>
                 : pieces <= 1024 ? dsa_topk_rows_kernel<4, 256> : dsa_topk_rows_kernel<4, 0>;
-    const int threads = pieces <= 1024 ? 256 : (int)((pieces + 127) / 128) * 32;
+    const int threads = pieces <= 256 ? 256 : few ? 1024 : pieces <= 1024 ? 256 : (int)((pieces + 127) / 128) * 32;
     e = pdl_launch(kern, dim3(R), dim3(threads), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
   } else {
     e = pdl_launch(dsa_topk_kernel, dim3(R), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, t_ptr, t_seq, raw, q_pos);

@@ -145,7 +145,8 @@ def test_topk_bit_exact_vs_oracle_and_reference(R, T, k, k_pad, stride_pad, offs
 
 @pytest.mark.parametrize("R,T,stride_pad,offset", [(1, 65529, 0, 7), (1, 65537, 0, 0), (3, 65552, 1, 5), (1, 131065, 0, 7), (2, 131080, 3, 0),
                                                     (1, 262137, 0, 7), (1, 262145, 0, 0), (18, 16390, 1, 1), (20, 9, 0, 3),
-                                                    (5, 2041, 3, 1), (3, 2048, 8, 0), (3, 4089, 3, 1), (3, 8185, 3, 5), (2, 8192, 8, 1), (2, 16371, 5, 1)])
+                                                    (5, 2041, 3, 1), (3, 2048, 8, 0), (3, 4089, 3, 1), (3, 8185, 3, 5), (2, 8192, 8, 1), (2, 16371, 5, 1),
+                                                    (149, 2041, 3, 1), (149, 4089, 3, 5), (149, 8185, 3, 1), (149, 16371, 5, 1)])
 def test_topk_at_the_edges_of_its_row_forms(R, T, stride_pad, offset):
     """rows off the 16-byte boundary, and the longest row of every pieces-per-thread count of the cluster form"""
     r = synth.rng(R + T)
