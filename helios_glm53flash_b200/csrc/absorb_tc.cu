@@ -237,7 +237,14 @@ __global__ __launch_bounds__(AF_THREADS) void absorb_few_rows_kernel(const __gri
   const uint32_t x_chunk = (uint32_t)nb * AF_BK * 2;
   const int wy = h * w_rows_per_head + w_row_off + (W_MN ? 0 : n0);
   if (tid == 0) {
-    for (int kc = 0; kc < NK; kc++) tc::mbar_init(&full_bar[kc], 1);
+    // the weights on their way into L2 while the kernel before this one may still run (34.2 -> 33.4 us for the MLA layer of one
+    // token; 0.1 us lost where they are in L2 already)
+    for (int kc = 0; kc < NK; kc++) {
+      asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(&tmap_w)),
+                   "r"(W_MN ? n0 : kc * AF_BK), "r"(wy + (W_MN ? kc * AF_BK : 0))
+                   : "memory");
+      tc::mbar_init(&full_bar[kc], 1);
+    }
     tc::mbar_init(&done_bar, 1);
     tc::mbar_fence_init();
     abort_flag = 0;

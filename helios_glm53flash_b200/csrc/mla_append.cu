@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(256) mla_cache_append_kernel(const float* __re
                                                                const __half* __restrict__ ln_w,
                                                                __half* __restrict__ ckv, __half* __restrict__ ckv_new,
                                                                long long pos, int n, float eps) {
+  pdl_release(gridDim.x <= 32);
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -130,6 +131,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256) layernorm_f16_kernel(const __half* x, const __half* __restrict__ w,   // x and y may alias
                                                             const __half* __restrict__ b, __half* y,
                                                             int rows, int dim, float eps) {
+  pdl_release(gridDim.x <= 32);
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -148,6 +150,7 @@ __global__ void __launch_bounds__(128) mla_decode_prologue_kernel(
     __half* __restrict__ pk_nt, const float* __restrict__ ape, int pos, int* __restrict__ q_pos_out) {
   __shared__ __half s_kn[128];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_release();
   pdl_wait();
   if (warp == 0) append_row(kv_pre, ln_w, ckv + (size_t)pos * LATENT, nullptr, eps_rms, lane);
   if (warp == 1) layernorm_row<128>(idx_k, knorm_w, knorm_b, idx_kn, s_kn, 128, eps_ln, lane);
