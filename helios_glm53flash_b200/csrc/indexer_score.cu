@@ -260,6 +260,118 @@ __global__ __launch_bounds__(128) void indexer_tc_decode_kernel(
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
 }
 
+// Up to four rows: the keys are requested before anything else, one shared-memory tile (the registers are the second one) and
+// up to four CTAs per SM, so that the 512 tiles of 65,536 pools are all on their way at once: one row 8.0 -> 6.7 us, 1,250
+// pools 5.3 -> 4.6.  With more rows the queries (8 KB per row) are the longer chain and the CTAs too big for that (8 rows:
+// 25.3 us as above, 26.8 this way).
+template <int FMT>
+__global__ __launch_bounds__(128, 4) void indexer_tc_decode_few_kernel(
+    const uint16_t* __restrict__ q, const uint16_t* __restrict__ pk, const uint16_t* __restrict__ w,
+    const int* __restrict__ q_pos, __half* __restrict__ scores, int m, int npools, int score_stride,
+    int n_tiles, uint32_t tmem_cols, int* __restrict__ status) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + IXD_TILE;                   // (4 m) groups x IXD_SBO
+  const int nb = m * IX_HEADS;                     // N
+  float* w_sm = reinterpret_cast<float*>(sB + (nb / 8) * IXD_SBO);
+  int* pos_sm = reinterpret_cast<int*>(w_sm + IX_RG * IX_HEADS);
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int sub = lane >> 4, chunk = lane & 15;    // a warp instruction covers 2 rows x 16 chunks
+
+  if (tid == 0) {
+    tc::mbar_init(&bar, 1);
+    tc::mbar_fence_init();
+    abort_flag = 0;
+  }
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, tmem_cols);
+  pdl_wait();
+  uint4 stage[16];
+  auto fetch = [&](int tile) {                     // 128 rows x 256 B of one tile into registers
+    const int p0 = tile * IX_TILE_P;
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      const int row = (warp + 4 * j) * 2 + sub;
+      stage[j] = (p0 + row < npools) ? ld_stream16(pk + (size_t)(p0 + row) * IDX_DIM + chunk * 8)
+                                     : make_uint4(0, 0, 0, 0);
+    }
+  };
+  auto stash = [&]() {
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      const int row = (warp + 4 * j) * 2 + sub;
+      *reinterpret_cast<uint4*>(sA + (row >> 3) * IXD_SBO + chunk * IXD_LBO + (row & 7) * 16) = stage[j];
+    }
+  };
+  int tile = blockIdx.x;
+  if (tile < n_tiles) fetch(tile);
+  // query rows -> B operand (as asynchronous copies, which pass L1 by, the CTAs pile up on the same lines of L2: 6.3 -> 12.6 us)
+#pragma unroll 4
+  for (int r2 = warp; r2 < nb / 2; r2 += 4) {
+    const int row = r2 * 2 + sub;
+    const uint4 v = *reinterpret_cast<const uint4*>(q + (size_t)row * IDX_DIM + chunk * 8);
+    *reinterpret_cast<uint4*>(sB + (row >> 3) * IXD_SBO + chunk * IXD_LBO + (row & 7) * 16) = v;
+  }
+  for (int i = tid; i < nb; i += 128) {
+    const uint16_t wb = w[i];
+    w_sm[i] = FMT == tc::FMT_BF16 ? bf16_bits_to_f(wb) : __half2float(__ushort_as_half(wb));
+  }
+  if (tid < m) pos_sm[tid] = q_pos[tid];
+
+  if (tile < n_tiles) stash();
+  tc::fence_async_smem();
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_slot;
+  const uint32_t b_addr = tc::smem_u32(sB);
+  const uint32_t idesc = tc::make_idesc(IX_TILE_P, nb, FMT, FMT, false, false);
+  uint32_t parity = 0;
+  for (; tile < n_tiles; tile += gridDim.x) {
+    const int next = tile + gridDim.x;
+    if (next < n_tiles) fetch(next);               // in flight during the MMA and the epilogue below
+    if (tid == 0) {
+      const uint64_t ad0 = tc::make_sdesc(tc::smem_u32(sA), IXD_LBO, IXD_SBO);
+      const uint64_t bd0 = tc::make_sdesc(b_addr, IXD_LBO, IXD_SBO);
+#pragma unroll
+      for (int kk = 0; kk < IDX_DIM / 16; kk++)
+        tc::mma_f16(tmem, tc::sdesc_advance(ad0, kk * 2 * IXD_LBO), tc::sdesc_advance(bd0, kk * 2 * IXD_LBO), idesc, kk > 0);
+      tc::mma_commit(&bar);
+    }
+    const bool ok = tc::mbar_wait(&bar, parity, &abort_flag, 1);
+    parity ^= 1;
+    tc::fence_after_sync();
+    const int p = tile * IX_TILE_P + tid;          // this thread's pool (TMEM lane tid)
+    if (ok) {
+      for (int rr = 0; rr < m; rr++) {
+        uint32_t c[32];
+        tc::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + rr * IX_HEADS, c);
+        tc::tmem_ld_wait();
+        float tot = 0.f;
+#pragma unroll
+        for (int h = 0; h < IX_HEADS; h++) {
+          const float d = __uint_as_float(c[h]) * 0.08838834764f;
+          tot = fmaf(w_sm[rr * IX_HEADS + h], fmaxf(d, 0.f), tot);
+        }
+        if (p < npools) {
+          const bool vis = p * POOL + POOL - 1 <= pos_sm[rr];
+          scores[(size_t)rr * score_stride + p] =
+              vis ? __float2half_rn(tot * 0.17677669530f) : __ushort_as_half((unsigned short)0xfc00);
+        }
+      }
+    }
+    if (next < n_tiles) stash();                   // the product that read the tile is complete
+    tc::fence_async_smem();
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+  }
+  if (warp == 0) tc::tmem_dealloc(tmem, tmem_cols);
+  if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
+}
+
 }  // namespace hk
 
 // device word that records a bounded wait giving up (read with hk_read_device_status)
@@ -315,23 +427,24 @@ HK_API int hk_indexer_score(const void* q_idx, const void* pool_k_nt, const void
   if (m <= IX_RG) {
     // decode form: persistent CTAs over the pool tiles
     const int nb = m * IX_HEADS;
-    const size_t smem = 2 * IXD_TILE + (size_t)(nb / 8) * IXD_SBO + IX_RG * IX_HEADS * 4 + IX_RG * 4 + 64;
+    const bool few = m <= 4;                       // see indexer_tc_decode_few_kernel
+    const size_t smem = (few ? 1 : 2) * IXD_TILE + (size_t)(nb / 8) * IXD_SBO + IX_RG * IX_HEADS * 4 + IX_RG * 4 + 64;
     uint32_t cols = 32;
     while ((int)cols < nb) cols <<= 1;
     static bool dattr[64] = {false};
     if (dev >= 0 && dev < 64 && !dattr[dev]) {
       const int max_smem = (int)(2 * IXD_TILE + 32 * IXD_SBO + IX_RG * IX_HEADS * 4 + IX_RG * 4 + 64);
-      if (cudaFuncSetAttribute(indexer_tc_decode_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
-          cudaFuncSetAttribute(indexer_tc_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess)
-        return HK_ERR_CUDA;
+      for (auto k : {indexer_tc_decode_kernel<0>, indexer_tc_decode_kernel<1>, indexer_tc_decode_few_kernel<0>, indexer_tc_decode_few_kernel<1>})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess) return HK_ERR_CUDA;
       dattr[dev] = true;
     }
-    const int per_sm = smem <= 100 * 1024 ? 2 : 1;
+    const int fit = (int)(227 * 1024 / (smem + 1024)), per_sm = min(4, min(fit, (int)(512 / cols)));
     int grid_x = per_sm * sm_count();
     if (grid_x > tiles) grid_x = tiles;
     cudaStream_t sd = as_stream(stream);
     int* std_ = device_status_ptr();
-    auto kern = dtype == HK_F16 ? indexer_tc_decode_kernel<0> : indexer_tc_decode_kernel<1>;
+    auto kern = few ? (dtype == HK_F16 ? indexer_tc_decode_few_kernel<0> : indexer_tc_decode_few_kernel<1>)
+                    : (dtype == HK_F16 ? indexer_tc_decode_kernel<0> : indexer_tc_decode_kernel<1>);
     if (pdl_launch(kern, dim3(grid_x), dim3(128), smem, sd, (const uint16_t*)q_idx, (const uint16_t*)pool_k_nt, (const uint16_t*)w,
                    q_pos, (__half*)scores, m, npools, score_stride, tiles, cols, std_) != cudaSuccess)
       return HK_ERR_CUDA;
