@@ -210,6 +210,8 @@ struct DecodeArgs {
   int w_bf16, g_bf16, y_f16, gate_act;
   float eps, cbias, scale;
   int H, n_heads;                       // heads of a sequence; batch * H
+  int Hk;                               // key heads of a sequence (DEC_REC; else H)
+  int* tickets;                         // DEC_STEP: slices of a head that have read its windows
   const int* slots;
 };
 
@@ -218,14 +220,18 @@ struct alignas(16) DecodeToken {                    // one head's token, prepare
   float beta;
 };
 
+enum { DEC_STEP, DEC_LAYER, DEC_REC };   // convolution + recurrence; the whole layer; recurrence of one token alone
+
 constexpr int KD_STATE_WARPS = 8, KD_WARPS = 11, KD_THREADS = KD_WARPS * 32;
 
-// role 0: q, 1: k and decay, 2: v; one warp each
-template <bool LAYER>
-__device__ __forceinline__ void decode_prepare(const DecodeArgs& a, DecodeToken& t, int bh, int role, int lane) {
-  const int b = bh / a.H, head = bh - b * a.H, dim = 3 * a.H * 128;
+// role 0: q, 1: k and decay, 2: v; one warp each.  DEC_STEP leaves the rolled windows in `rolled` (decode_roll stores them)
+template <int MODE>
+__device__ __forceinline__ void decode_prepare(const DecodeArgs& a, DecodeToken& t, int bh, int role, int lane, uint2 (&rolled)[4]) {
+  constexpr bool LAYER = MODE == DEC_LAYER;
+  const int b = bh / a.H, head = bh - b * a.H, dim = (2 * a.Hk + a.H) * 128;
   const int slot = a.slots ? a.slots[b] : b;
-  const int c0 = (role * a.H + head) * 128 + lane;
+  const int kh = MODE == DEC_REC ? head / (a.H / a.Hk) : head;
+  const int c0 = (role * a.Hk + (role == 2 ? head : kh)) * 128 + lane;
   __nv_bfloat16* cs = a.conv_state + ((size_t)slot * dim + c0) * 4;
   __nv_bfloat16 x[4];
   uint2 st[4], w[4];
@@ -235,16 +241,22 @@ __device__ __forceinline__ void decode_prepare(const DecodeArgs& a, DecodeToken&
     const size_t xi = (size_t)b * dim + c0 + 32 * u;
     if (LAYER) x[u] = __float2bfloat16(reinterpret_cast<const float*>(a.x)[xi]);
     else x[u] = reinterpret_cast<const __nv_bfloat16*>(a.x)[xi];
-    st[u] = *reinterpret_cast<const uint2*>(cs + 128 * u);
-    w[u] = *reinterpret_cast<const uint2*>(a.conv_w + (size_t)(c0 + 32 * u) * 4);
-    bias[u] = a.conv_bias ? __bfloat162float(a.conv_bias[c0 + 32 * u]) : 0.f;
+    if (MODE != DEC_REC) {
+      st[u] = *reinterpret_cast<const uint2*>(cs + 128 * u);
+      w[u] = *reinterpret_cast<const uint2*>(a.conv_w + (size_t)(c0 + 32 * u) * 4);
+      bias[u] = a.conv_bias ? __bfloat162float(a.conv_bias[c0 + 32 * u]) : 0.f;
+    }
     if (role == 1) gv[u] = a.g[(size_t)bh * 128 + lane + 32 * u];
   }
   float z[4];
 #pragma unroll
   for (int u = 0; u < 4; u++) {
+    if (MODE == DEC_REC) {
+      z[u] = __bfloat162float(x[u]);
+      continue;
+    }
     z[u] = conv4_silu_bf16(st[u], w[u], bias[u], __bfloat162float(x[u]));
-    *reinterpret_cast<uint2*>(cs + 128 * u) = conv4_rolled(st[u], x[u]);
+    rolled[u] = conv4_rolled(st[u], x[u]);
     if (!LAYER && a.conv_out) a.conv_out[(size_t)b * dim + c0 + 32 * u] = __float2bfloat16_rn(z[u]);
   }
   if (role == 2) {
@@ -270,6 +282,14 @@ __device__ __forceinline__ void decode_prepare(const DecodeArgs& a, DecodeToken&
       t.d[c] = __expf(gl);
     }
   }
+}
+
+__device__ __forceinline__ void decode_roll(const DecodeArgs& a, int bh, int role, int lane, const uint2 (&rolled)[4]) {
+  const int b = bh / a.H, head = bh - b * a.H;
+  const int slot = a.slots ? a.slots[b] : b;
+  __nv_bfloat16* cs = a.conv_state + ((size_t)slot * 3 * a.H * 128 + (role * a.H + head) * 128 + lane) * 4;
+#pragma unroll
+  for (int u = 0; u < 4; u++) *reinterpret_cast<uint2*>(cs + 128 * u) = rolled[u];
 }
 
 // state rows of warp w: groups w (i < 8) and w + 8; columns 4 lane .. 4 lane + 3
@@ -334,8 +354,9 @@ __device__ __forceinline__ void state_update(float4 (&S)[16], const DecodeToken&
 }
 
 // one warp: the head's 128 outputs (lane = 4 columns), and LAYER: their gated RMS norm, as the one-warp-per-row norm kernel
-template <bool LAYER>
+template <int MODE>
 __device__ __forceinline__ void decode_finish(const DecodeArgs& a, const float (*opart)[128], int bh, int lane) {
+  constexpr bool LAYER = MODE == DEC_LAYER;
   const size_t o = (size_t)bh * 128 + 4 * lane;
   float4 ga, w4;
   if (LAYER) {
@@ -372,45 +393,62 @@ __device__ __forceinline__ float* head_state(const DecodeArgs& a, int bh) {
   return a.state + ((size_t)slot * a.H + head) * 128 * 128;
 }
 
-// VEC: the state is 16-byte aligned
-template <bool LAYER, bool VEC>
+// VEC: the state is 16-byte aligned.
+// SLICES = 4: a CTA owns 32 of the head's 128 columns (two state warps, a quarter warp per row group, the same sums in the
+// same order).  One SM moves a head's 64 KB in and out in 0.6 us each, and a few heads leave the other SMs idle: 32 heads 3.25 ->
+// 2.9 us per step, one token's recurrence alone 2.2.  Not for DEC_LAYER, whose norm needs all columns of a head.  The q and k windows are read by every slice
+// and rolled by the one that draws the last ticket; nobody waits for it.
+template <int MODE, bool VEC, int SLICES>
 __global__ __launch_bounds__(KD_THREADS) void kda_decode_kernel(const DecodeArgs a) {
-  const int bh = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int SW = KD_STATE_WARPS / SLICES;                // state warps
+  const int bh = blockIdx.x / SLICES, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rg = SLICES == 1 ? warp : 4 * warp + (lane >> 3);                                   // row group,
+  const int cl = SLICES == 1 ? lane : (int)(blockIdx.x % SLICES) * (32 / SLICES) + (lane & 7);   // four columns
   __shared__ __align__(16) DecodeToken tok;
   __shared__ __align__(16) float part[8][128], opart[8][128];
+  __shared__ int last;
   pdl_wait();
   float4 S[16];
+  uint2 rolled[4];
   float* sp = nullptr;
-  if (warp < KD_STATE_WARPS) {
-    sp = head_state(a, bh) + 4 * lane;
+  if (warp < SW) {
+    sp = head_state(a, bh) + 4 * cl;
 #pragma unroll
     for (int i = 0; i < 16; i++) {
-      const float* p = sp + state_row(warp, i) * 128;
+      const float* p = sp + state_row(rg, i) * 128;
       S[i] = VEC ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
     }
   } else {
-    decode_prepare<LAYER>(a, tok, bh, warp - KD_STATE_WARPS, lane);
+    decode_prepare<MODE>(a, tok, bh, warp - SW, lane, rolled);
+    if (MODE != DEC_REC && SLICES == 1) decode_roll(a, bh, warp - SW, lane, rolled);
   }
   __syncthreads();
-  if (warp < KD_STATE_WARPS) state_kv(S, tok, warp, lane, part);
+  if (MODE == DEC_STEP && SLICES > 1 && threadIdx.x == SW * 32) {
+    __threadfence();
+    last = atomicAdd(&a.tickets[bh], 1) == SLICES - 1;
+  }
+  if (warp < SW) state_kv(S, tok, rg, cl, part);
   __syncthreads();
-  if (warp < KD_STATE_WARPS) {
-    state_update(S, tok, warp, lane, part, opart);
+  if (warp < SW) {
+    state_update(S, tok, rg, cl, part, opart);
 #pragma unroll
     for (int i = 0; i < 16; i++) {
-      float* p = sp + state_row(warp, i) * 128;
+      float* p = sp + state_row(rg, i) * 128;
       if (VEC) *reinterpret_cast<float4*>(p) = S[i];
       else { p[0] = S[i].x; p[1] = S[i].y; p[2] = S[i].z; p[3] = S[i].w; }
     }
+  } else if (MODE == DEC_STEP && SLICES > 1 && last) {
+    decode_roll(a, bh, warp - SW, lane, rolled);
+    if (threadIdx.x == SW * 32) a.tickets[bh] = 0;
   }
   __syncthreads();
-  if (warp == KD_STATE_WARPS) decode_finish<LAYER>(a, opart, bh, lane);
+  if (warp == SW && (SLICES == 1 || lane < 32 / SLICES)) decode_finish<MODE>(a, opart, bh, SLICES == 1 ? lane : cl);
 }
 
 // persistent form: CTA c takes heads c, c + gridDim.x, ...
 constexpr int KD_STAGES = 2;
 constexpr size_t KD_STREAM_SMEM = (size_t)(KD_STAGES + 1) * 65536;
-template <bool LAYER>
+template <int MODE>
 __global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const DecodeArgs a, int* __restrict__ status) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -432,7 +470,12 @@ __global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const Dec
   };
   if (threadIdx.x == 0)
     for (int i = 0; i < KD_STAGES && i < n; i++) fetch(i);
-  if (warp >= KD_STATE_WARPS) decode_prepare<LAYER>(a, tok[0], first, warp - KD_STATE_WARPS, lane);
+  uint2 rolled[4];
+  auto prepare = [&](int i) {
+    decode_prepare<MODE>(a, tok[i & 1], first + i * step, warp - KD_STATE_WARPS, lane, rolled);
+    if (MODE != DEC_REC) decode_roll(a, first + i * step, warp - KD_STATE_WARPS, lane, rolled);
+  };
+  if (warp >= KD_STATE_WARPS) prepare(0);
   __syncthreads();
   bool ok = true;
   for (int i = 0; i < n; i++) {
@@ -454,8 +497,8 @@ __global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const Dec
       for (int r = 0; r < 16; r++) so[state_row(warp, r) * 32] = S[r];
       tc::fence_async_smem();
     } else {
-      if (i > 0 && warp == KD_WARPS - 1) decode_finish<LAYER>(a, opart[(i - 1) & 1], bh - step, lane);
-      if (i + 1 < n) decode_prepare<LAYER>(a, tok[(i + 1) & 1], bh + step, warp - KD_STATE_WARPS, lane);
+      if (i > 0 && warp == KD_WARPS - 1) decode_finish<MODE>(a, opart[(i - 1) & 1], bh - step, lane);
+      if (i + 1 < n) prepare(i + 1);
     }
     __syncthreads();
     if (threadIdx.x == 0 && ok && !abort_flag) {
@@ -463,14 +506,14 @@ __global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const Dec
       tc::bulk_commit();
     }
   }
-  if (warp == KD_WARPS - 1) decode_finish<LAYER>(a, opart[(n - 1) & 1], first + (n - 1) * step, lane);
+  if (warp == KD_WARPS - 1) decode_finish<MODE>(a, opart[(n - 1) & 1], first + (n - 1) * step, lane);
   if (threadIdx.x == 0) {
     tc::bulk_wait_all<0>();
     if (abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
   }
 }
 
-template <bool LAYER>
+template <int MODE>
 static int launch_decode(const DecodeArgs& a, cudaStream_t s) {
   const bool vec = aligned(a.state, 16);
   if (vec && a.n_heads > 2 * sm_count()) {
@@ -478,14 +521,18 @@ static int launch_decode(const DecodeArgs& a, cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-      if (cudaFuncSetAttribute(kda_decode_stream_kernel<LAYER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KD_STREAM_SMEM) != cudaSuccess)
+      if (cudaFuncSetAttribute(kda_decode_stream_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KD_STREAM_SMEM) != cudaSuccess)
         return HK_ERR_CUDA;
       attr_set[dev] = true;
     }
     const int grid = sm_count();
-    return pdl_launch(kda_decode_stream_kernel<LAYER>, dim3(grid), dim3(KD_THREADS), KD_STREAM_SMEM, s, a, device_status_ptr()) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+    return pdl_launch(kda_decode_stream_kernel<MODE>, dim3(grid), dim3(KD_THREADS), KD_STREAM_SMEM, s, a, device_status_ptr()) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
   }
-  auto kern = vec ? kda_decode_kernel<LAYER, true> : kda_decode_kernel<LAYER, false>;
+  if constexpr (MODE != DEC_LAYER) {
+    if (vec && a.n_heads <= sm_count() / 2)
+      return pdl_launch(kda_decode_kernel<MODE, true, 4>, dim3(4 * a.n_heads), dim3(5 * 32), 0, s, a) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+  }
+  auto kern = vec ? kda_decode_kernel<MODE, true, 1> : kda_decode_kernel<MODE, false, 1>;
   return pdl_launch(kern, dim3(a.n_heads), dim3(KD_THREADS), 0, s, a) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 
@@ -788,12 +835,31 @@ HK_API int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* b
   cudaStream_t s = as_stream(stream);
   if (k_head_dim == 128 && channelwise && !history && history_stride == 1) {
     const int64_t chains = (int64_t)bsz * num_v_heads;
-    const int cpl = !aligned(state, 16) || chains < 32 ? 1 : (chains < 64 ? 2 : 4);
-    auto kern = cpl == 4 ? kda_recurrent_cols_kernel<4> : (cpl == 2 ? kda_recurrent_cols_kernel<2> : kda_recurrent_cols_kernel<1>);
-    return pdl_launch(kern, dim3(bsz, num_v_heads, 16 / cpl), dim3(RC_WARPS * 32), 0, s, q, g, bt, state, o, out_f32, seqlen, num_k_heads,
-                      num_v_heads, 1.0f / sqrtf(128.0f), slots) == cudaSuccess
-               ? HK_OK
-               : HK_ERR_CUDA;
+    if (seqlen == 1 && chains <= 1 << 28) {   // one token: the decode step's kernels without the convolution, the same bits
+      DecodeArgs a{};
+      a.x = q;
+      a.g = g;
+      a.beta = bt;
+      a.state = state;
+      a.out = o;
+      a.out_f32 = out_f32;
+      a.scale = 1.0f / sqrtf(128.0f);
+      a.H = num_v_heads;
+      a.Hk = num_k_heads;
+      a.n_heads = (int)chains;
+      a.slots = slots;
+      return launch_decode<DEC_REC>(a, s);
+    }
+    // Two or three tokens of many chains (up to six of a thousand) are mostly the state in and out, which the older kernel moves
+    // in longer runs: 2 tokens of 32 chains 3.5 us against 4.7, of 1,536 chains 44 against 72; 4 of 256 chains 16.1 against 15.7.
+    if (!(chains >= 32 && seqlen <= (chains >= 1024 ? 6 : 3))) {
+      const int cpl = !aligned(state, 16) || chains < 32 ? 1 : (chains < 64 ? 2 : 4);
+      auto kern = cpl == 4 ? kda_recurrent_cols_kernel<4> : (cpl == 2 ? kda_recurrent_cols_kernel<2> : kda_recurrent_cols_kernel<1>);
+      return pdl_launch(kern, dim3(bsz, num_v_heads, 16 / cpl), dim3(RC_WARPS * 32), 0, s, q, g, bt, state, o, out_f32, seqlen, num_k_heads,
+                        num_v_heads, 1.0f / sqrtf(128.0f), slots) == cudaSuccess
+                 ? HK_OK
+                 : HK_ERR_CUDA;
+    }
   }
   // narrower column slices when the (batch x head) count alone cannot cover the SMs
   const bool narrow = (long)bsz * num_v_heads * 4 < sm_count();
@@ -829,10 +895,11 @@ HK_API int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_
   a.out_f32 = out_f32;
   a.conv_out = (__nv_bfloat16*)conv_out;
   a.scale = 1.0f / sqrtf(128.0f);
-  a.H = num_heads;
+  a.H = a.Hk = num_heads;
   a.n_heads = bsz * num_heads;
+  a.tickets = tickets;
   a.slots = slots;
-  return launch_decode<false>(a, as_stream(stream));
+  return launch_decode<DEC_STEP>(a, as_stream(stream));
 }
 
 HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f,
@@ -872,8 +939,8 @@ HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* c
   a.eps = epsilon;
   a.cbias = constant_bias;
   a.scale = 1.0f / sqrtf(128.0f);
-  a.H = num_heads;
+  a.H = a.Hk = num_heads;
   a.n_heads = bsz * num_heads;
   a.slots = slots;
-  return launch_decode<true>(a, as_stream(stream));
+  return launch_decode<DEC_LAYER>(a, as_stream(stream));
 }

@@ -75,7 +75,7 @@ int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* beta, fl
  *   conv_weight [3*H*128][4] bf16   conv_bias [3*H*128] bf16 or NULL   g [bsz][H][128] f32   beta [bsz][H] bf16
  *   rec_state [slots][H][128][128] f32 (in place)   out [bsz][H][128] bf16 (rz)   out_f32 optional
  *   conv_out optional [bsz][3*H*128] bf16: the convolved q|k|v (what the two-kernel sequence leaves in between).
- *   tickets: bsz*H device ints, zero before the first call; left zero (earlier forms counted a head's slices there).   */
+ *   tickets: bsz*H device ints, zero before the first call; left zero (a few heads are split over CTAs, which count here). */
 int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_weight, const void* conv_bias, const float* g,
                        const void* beta, float* rec_state, void* out, float* out_f32, void* conv_out, int bsz,
                        int num_heads, const int* slots, int* tickets, void* stream);

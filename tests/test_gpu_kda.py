@@ -399,9 +399,11 @@ def test_decode_of_many_heads_streams_the_same_bits(H, bsz, slots):
         assert torch.equal(whole, single)
 
 
-@pytest.mark.parametrize("T,Hk,Hv,bsz", [(1, 2, 4, 1), (7, 3, 3, 2), (8, 1, 2, 1), (9, 4, 4, 3), (63, 2, 2, 1)])
+@pytest.mark.parametrize("T,Hk,Hv,bsz", [(1, 2, 4, 1), (7, 3, 3, 2), (8, 1, 2, 1), (9, 4, 4, 3), (63, 2, 2, 1), (1, 37, 74, 1), (1, 25, 75, 1),
+                                            (1, 8, 16, 19), (2, 8, 40, 1), (3, 16, 32, 1), (4, 16, 32, 1)])
 def test_per_token_kernel_around_its_batches_of_eight(T, Hk, Hv, bsz):
-    """token counts either side of the 8 prepared at a time, grouped key heads, against the oracle"""
+    """token counts either side of the 8 prepared at a time, single tokens either side of the head counts that are split over CTAs or
+    streamed, two and three tokens of many chains, grouped key heads, against the oracle"""
     D = 128
     inp = synth.kda_inputs(T, Hv, D, bsz=bsz, seed=T)
     qkv = inp["mixed_qkv"].reshape(bsz, T, 3, Hv, D)
