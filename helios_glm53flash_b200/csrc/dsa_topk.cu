@@ -260,7 +260,7 @@ __device__ __forceinline__ void for_keys(const uint4 (&pc)[NP], F f) {
 }
 
 template <int NP, int FIXED>   // FIXED: threads of the CTA, 0 = as launched
-__global__ __launch_bounds__(FIXED ? FIXED : TKR_MAX_THREADS, FIXED == 1024 ? 1 : FIXED ? 4 : 2) void dsa_topk_rows_kernel(const uint16_t* scores, int* __restrict__ out, int T, int s_stride,
+__global__ __launch_bounds__(FIXED ? FIXED : TKR_MAX_THREADS, FIXED == 256 ? 4 : FIXED ? 1 : 2) void dsa_topk_rows_kernel(const uint16_t* scores, int* __restrict__ out, int T, int s_stride,
                                                                     int k, int k_pad, int* __restrict__ raw,
                                                                     const int* __restrict__ q_pos) {
   constexpr int NB = 8;                                    // buckets of each of the first 256 threads
@@ -560,10 +560,10 @@ static int topk_launch(const void* scores, int s_stride, int* indices, int R, in
   } else if (pieces <= TKR_MAX_PIECES && !t_ptr) {
     const bool few = R <= sm_count();
     auto kern = pieces <= 256    ? dsa_topk_rows_kernel<1, 256>
-                : few            ? (pieces <= 1024 ? dsa_topk_rows_kernel<1, 1024> : dsa_topk_rows_kernel<2, 1024>)
+                : few            ? (pieces <= 512 ? dsa_topk_rows_kernel<1, 512> : pieces <= 1024 ? dsa_topk_rows_kernel<1, 1024> : dsa_topk_rows_kernel<2, 1024>)
                 : pieces <= 512  ? dsa_topk_rows_kernel<2, 256>
                 : pieces <= 1024 ? dsa_topk_rows_kernel<4, 256> : dsa_topk_rows_kernel<4, 0>;
-    const int threads = pieces <= 256 ? 256 : few ? 1024 : pieces <= 1024 ? 256 : (int)((pieces + 127) / 128) * 32;
+    const int threads = pieces <= 256 ? 256 : few ? (pieces <= 512 ? 512 : 1024) : pieces <= 1024 ? 256 : (int)((pieces + 127) / 128) * 32;
     e = pdl_launch(kern, dim3(R), dim3(threads), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
   } else {
     e = pdl_launch(dsa_topk_kernel, dim3(R), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, t_ptr, t_seq, raw, q_pos);

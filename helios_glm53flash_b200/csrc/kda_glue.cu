@@ -15,11 +15,11 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 // src [S][F] fp32 -> dst [F][S] bf16 (round to nearest even).  One CTA moves a tile of 4,096 elements.  HBM-bound (6 B per
 // element): 64 tokens x 64 channels, rows of 256 B in and 128 B out, 6.5 TB/s at 32,768 tokens.
-// LONG: 128 tokens x 32 channels.  The rows of an odd length start inside a sector, so a tile row ends in two partly written
-// ones: twice as long rows halve them (458 -> 426 us at 32,763 tokens; 368 -> 399 at 32,768).  Short calls have more CTAs this
-// way (301 tokens x 3,072 channels 6.6 -> 4.7 us).  4-byte stores from the first even element of a row on.
+// LONG, odd lengths from 32 on: 128 tokens x 32 channels.  The rows start inside a sector, so a tile row ends in two partly written ones:
+// twice as long rows halve them (458 -> 430 us at 32,763 tokens, 6.5 -> 4.4 at 301 x 3,072 channels; 368 -> 399 at 32,768).
+// 4-byte stores from the first even element of a row on.
 // ---------------------------------------------------------------------------------------------
-template <bool LONG>
+template <bool LONG, bool ODD>
 __global__ void __launch_bounds__(256, 8) transpose_cast_kernel(const float* __restrict__ src,
                                                              __nv_bfloat16* __restrict__ dst, int S, int F) {
   constexpr int TS = LONG ? 128 : 64, TF = LONG ? 32 : 64, RS = 256 / TF;
@@ -44,16 +44,16 @@ __global__ void __launch_bounds__(256, 8) transpose_cast_kernel(const float* __r
     const int fl = wid + 8 * j;
     if (f0 + fl >= F) continue;
     __nv_bfloat16* o = dst + (size_t)(f0 + fl) * S + s0;
-    const int odd = LONG ? (int)(reinterpret_cast<uintptr_t>(o) >> 1) & 1 : 0;
+    const int odd = ODD ? (int)(reinterpret_cast<uintptr_t>(o) >> 1) & 1 : 0;
 #pragma unroll
     for (int h = 0; h < TS / 64; h++) {
       const int t = 64 * h + 2 * lane + odd;
       if (t + 1 < n)
         *reinterpret_cast<__nv_bfloat162*>(o + t) = __halves2bfloat162(__float2bfloat16(tile[t][fl]), __float2bfloat16(tile[t + 1][fl]));
-      else if (LONG && t < n)
+      else if (ODD && t < n)
         o[t] = __float2bfloat16(tile[t][fl]);
     }
-    if (LONG && odd && lane == 0) o[0] = __float2bfloat16(tile[0][fl]);
+    if (ODD && odd && lane == 0) o[0] = __float2bfloat16(tile[0][fl]);
   }
 }
 
@@ -275,11 +275,11 @@ int launch_gated_rms_norm(const void* x, const void* w, void* y, const void* g, 
 HK_API int hk_kda_transpose_cast(void* dst_bf16, const float* src, int S, int F, void* stream) {
   HK_REQUIRE(dst_bf16 && src && S >= 0 && F >= 0);
   if (S == 0 || F == 0) return HK_OK;
-  const bool longer = S % 2 != 0 || S < 512;
+  const bool odd = S % 2 != 0, longer = odd && S >= 32;
   const int s_tiles = (S - 1) / (longer ? 128 : 64) + 1;
   HK_REQUIRE(s_tiles <= 65535);
   HK_REQUIRE(hk::aligned(dst_bf16, 4));
-  return hk::pdl_launch(longer ? hk::transpose_cast_kernel<true> : hk::transpose_cast_kernel<false>, dim3((F - 1) / (longer ? 32 : 64) + 1, s_tiles),
+  return hk::pdl_launch(longer ? hk::transpose_cast_kernel<true, true> : odd ? hk::transpose_cast_kernel<false, true> : hk::transpose_cast_kernel<false, false>, dim3((F - 1) / (longer ? 32 : 64) + 1, s_tiles),
                         dim3(256), 0, hk::as_stream(stream), src, static_cast<__nv_bfloat16*>(dst_bf16), S, F) == cudaSuccess
              ? HK_OK
              : HK_ERR_CUDA;
