@@ -17,7 +17,7 @@ namespace {
 // element): 64 tokens x 64 channels, rows of 256 B in and 128 B out, 6.5 TB/s at 32,768 tokens.
 // LONG, odd lengths from 32 on: 128 tokens x 32 channels.  The rows start inside a sector, so a tile row ends in two partly written ones:
 // twice as long rows halve them (458 -> 430 us at 32,763 tokens, 6.5 -> 4.4 at 301 x 3,072 channels; 368 -> 399 at 32,768).
-// 4-byte stores from the first even element of a row on.
+// 4-byte stores from the first even element of a row on.  ODD without LONG: 2-byte stores (3 tokens x 12,288 channels 1.9 us, 2.8 the other way).
 // ---------------------------------------------------------------------------------------------
 template <bool LONG, bool ODD>
 __global__ void __launch_bounds__(256, 8) transpose_cast_kernel(const float* __restrict__ src,
@@ -44,16 +44,19 @@ __global__ void __launch_bounds__(256, 8) transpose_cast_kernel(const float* __r
     const int fl = wid + 8 * j;
     if (f0 + fl >= F) continue;
     __nv_bfloat16* o = dst + (size_t)(f0 + fl) * S + s0;
-    const int odd = ODD ? (int)(reinterpret_cast<uintptr_t>(o) >> 1) & 1 : 0;
+    const int odd = LONG ? (int)(reinterpret_cast<uintptr_t>(o) >> 1) & 1 : 0;
 #pragma unroll
     for (int h = 0; h < TS / 64; h++) {
       const int t = 64 * h + 2 * lane + odd;
-      if (t + 1 < n)
+      if (!LONG && t >= n) continue;
+      if (LONG ? t + 1 < n : !ODD) {
         *reinterpret_cast<__nv_bfloat162*>(o + t) = __halves2bfloat162(__float2bfloat16(tile[t][fl]), __float2bfloat16(tile[t + 1][fl]));
-      else if (ODD && t < n)
+      } else if (t < n) {
         o[t] = __float2bfloat16(tile[t][fl]);
+        if (!LONG && t + 1 < n) o[t + 1] = __float2bfloat16(tile[t + 1][fl]);
+      }
     }
-    if (ODD && odd && lane == 0) o[0] = __float2bfloat16(tile[0][fl]);
+    if (LONG && odd && lane == 0) o[0] = __float2bfloat16(tile[0][fl]);
   }
 }
 
