@@ -448,8 +448,9 @@ __global__ __launch_bounds__(KD_THREADS) void kda_decode_kernel(const DecodeArgs
 // persistent form: CTA c takes heads c, c + gridDim.x, ...
 constexpr int KD_STAGES = 2;
 constexpr size_t KD_STREAM_SMEM = (size_t)(KD_STAGES + 1) * 65536;
+constexpr int KD_STREAM_THREADS = KD_THREADS + 32;               // one more warp, which finishes the head before
 template <int MODE>
-__global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const DecodeArgs a, int* __restrict__ status) {
+__global__ __launch_bounds__(KD_STREAM_THREADS) void kda_decode_stream_kernel(const DecodeArgs a, int* __restrict__ status) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(16) DecodeToken tok[2];
@@ -475,7 +476,7 @@ __global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const Dec
     decode_prepare<MODE>(a, tok[i & 1], first + i * step, warp - KD_STATE_WARPS, lane, rolled);
     if (MODE != DEC_REC) decode_roll(a, first + i * step, warp - KD_STATE_WARPS, lane, rolled);
   };
-  if (warp >= KD_STATE_WARPS) prepare(0);
+  if (warp >= KD_STATE_WARPS && warp < KD_WARPS) prepare(0);
   __syncthreads();
   bool ok = true;
   for (int i = 0; i < n; i++) {
@@ -497,8 +498,8 @@ __global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const Dec
       for (int r = 0; r < 16; r++) so[state_row(warp, r) * 32] = S[r];
       tc::fence_async_smem();
     } else {
-      if (i > 0 && warp == KD_WARPS - 1) decode_finish<MODE>(a, opart[(i - 1) & 1], bh - step, lane);
-      if (i + 1 < n) prepare(i + 1);
+      if (i > 0 && warp == KD_WARPS) decode_finish<MODE>(a, opart[(i - 1) & 1], bh - step, lane);
+      if (i + 1 < n && warp < KD_WARPS) prepare(i + 1);
     }
     __syncthreads();
     if (threadIdx.x == 0 && ok && !abort_flag) {
@@ -506,7 +507,7 @@ __global__ __launch_bounds__(KD_THREADS) void kda_decode_stream_kernel(const Dec
       tc::bulk_commit();
     }
   }
-  if (warp == KD_WARPS - 1) decode_finish<MODE>(a, opart[(n - 1) & 1], first + (n - 1) * step, lane);
+  if (warp == KD_WARPS) decode_finish<MODE>(a, opart[(n - 1) & 1], first + (n - 1) * step, lane);
   if (threadIdx.x == 0) {
     tc::bulk_wait_all<0>();
     if (abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
@@ -526,7 +527,7 @@ static int launch_decode(const DecodeArgs& a, cudaStream_t s) {
       attr_set[dev] = true;
     }
     const int grid = sm_count();
-    return pdl_launch(kda_decode_stream_kernel<MODE>, dim3(grid), dim3(KD_THREADS), KD_STREAM_SMEM, s, a, device_status_ptr()) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+    return pdl_launch(kda_decode_stream_kernel<MODE>, dim3(grid), dim3(KD_STREAM_THREADS), KD_STREAM_SMEM, s, a, device_status_ptr()) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
   }
   if constexpr (MODE != DEC_LAYER) {
     if (vec && a.n_heads <= sm_count() / 2)
