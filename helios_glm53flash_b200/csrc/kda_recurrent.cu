@@ -236,6 +236,8 @@ __device__ __forceinline__ void decode_prepare(const DecodeArgs& a, DecodeToken&
   __nv_bfloat16 x[4];
   uint2 st[4], w[4];
   float bias[4], gv[4];
+  // (asked for up front; the layer's beta, a_log and dt_bias up front as well measured 0.1 us slower)
+  const float beta = !LAYER && role == 2 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.beta)[bh]) : 0.f;
 #pragma unroll
   for (int u = 0; u < 4; u++) {
     const size_t xi = (size_t)b * dim + c0 + 32 * u;
@@ -264,7 +266,7 @@ __device__ __forceinline__ void decode_prepare(const DecodeArgs& a, DecodeToken&
     for (int u = 0; u < 4; u++) t.v[lane + 32 * u] = z[u];
     if (lane == 0)
       t.beta = LAYER ? __bfloat162float(__float2bfloat16(1.0f / (1.0f + __expf(-reinterpret_cast<const float*>(a.beta)[bh]))))
-                     : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.beta)[bh]);
+                     : beta;
     return;
   }
   const float r = inv_norm(z);
