@@ -183,8 +183,8 @@ __device__ __forceinline__ uint2 conv4_rolled(uint2 st, __nv_bfloat16 cur) {
 // operations as in the separate kernels of this library, so results are bit-identical to calling them in turn.
 //
 // A CTA owns a whole head (64 KB of state): 8 warps hold the state (warp = row group, lane = 4 columns), three more prepare
-// the token (q with its norm; k with its norm and the decay; v) and one of them finishes the output.  With the head in one
-// CTA nothing crosses CTAs: the earlier form, 4 or 8 value slices per head, handed the q / k window and the head's outputs
+// the token (q with its norm; k with its norm and the decay; v), and in the layer a twelfth warp asks for the norm's inputs at
+// the start and finishes the output.  With the head in one CTA nothing crosses CTAs: the earlier form, 4 or 8 value slices per head, handed the q / k window and the head's outputs
 // over through two ticket counters, an atomic and an L2 round trip each (5.4 us per layer of 32 heads).
 //
 //   few heads: one head per CTA, state straight between global memory and registers (latency: one memory round trip,
