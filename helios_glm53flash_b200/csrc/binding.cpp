@@ -6,7 +6,8 @@
 // METH_FASTCALL function: tensors are unwrapped to their addresses and the numbers converted straight into the C call.
 //
 // Conversion rules, by the C type of the parameter:
-//   pointer        tensor (or another object with data_ptr()) -> its address, None -> NULL
+//   pointer        tensor (or another object with data_ptr()) -> its address, None -> NULL; a tensor that has no address
+//                  (sparse, wrapped by a transform) raises the RuntimeError of Tensor.data_ptr()
 //   void* stream   (last parameter of a launcher) None -> torch's current stream, torch Stream -> its handle
 //   int            int / bool; a tensor gives the dtype tag HK_F16 / HK_BF16 / HK_F32
 //   int64_t        int; a [rows][512] tensor gives its row count, 0 if it is not laid out that way
@@ -17,6 +18,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/Exception.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
@@ -47,7 +49,10 @@ bool convert(PyObject* o, T& v) {
       return true;
     }
     if (THPVariable_Check(o)) {
-      v = reinterpret_cast<T>(const_cast<void*>(THPVariable_Unpack(o).const_data_ptr()));
+      const at::Tensor& t = THPVariable_Unpack(o);
+      // what the call writes is asked for as such: a lazily cloned tensor gets memory of its own first
+      if constexpr (std::is_const_v<std::remove_pointer_t<T>>) v = reinterpret_cast<T>(t.const_data_ptr());
+      else v = reinterpret_cast<T>(t.mutable_data_ptr());
       return true;
     }
     PyObject* a = PyObject_CallMethod(o, "data_ptr", nullptr);
@@ -119,7 +124,15 @@ bool convert_at(PyObject* o, T& v) {
 template <bool STREAM, class R, class... A, size_t... I>
 PyObject* call(R (*fn)(A...), PyObject* const* args, std::index_sequence<I...>) {
   std::tuple<std::remove_const_t<A>...> v;
-  if (!(convert_at<STREAM, I, sizeof...(A)>(args[I], std::get<I>(v)) && ...)) return nullptr;
+  try {
+    if (!(convert_at<STREAM, I, sizeof...(A)>(args[I], std::get<I>(v)) && ...)) return nullptr;
+  } catch (const c10::Error& e) {          // a tensor without an address: sparse, wrapped by vmap, ...
+    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    return nullptr;
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
   R r;
   if constexpr (STREAM) {
     Py_BEGIN_ALLOW_THREADS;      // a launch may wait for room in the stream's queue
