@@ -335,12 +335,18 @@ def dsa_topk_expand(scores, s_stride, indices, raw_idx, q_pos, R, T, k, after_sc
     _run("hk_dsa_topk_expand", scores, s_stride, indices, raw_idx, q_pos, R, T, k, 1 if after_scorer else 0, stream)
 
 
+def _key_type(t):
+    """bf16 by the tensor's type; fp16 keys may come as any 16-bit type that holds their bit patterns"""
+    import torch
+    return HK_BF16 if t.dtype == torch.bfloat16 else HK_F16
+
+
 def indexer_select(q_idx, pool_k_nt, w, q_pos, scores, indices, raw_idx, m, npools, k=512, stream=None, score_stride=None,
                    n_heads=32):
     """decode-step selection: indexer_score -> top-k with the expansion folded in, two launches (the second a
     programmatic dependent of the first); scores = fp16 workspace [m, score_stride]"""
     _run("hk_indexer_select", q_idx, pool_k_nt, w, q_pos, scores, indices, raw_idx, m, npools, npools if score_stride is None
-         else score_stride, n_heads, q_idx, k, stream)
+         else score_stride, n_heads, _key_type(q_idx), k, stream)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -355,7 +361,7 @@ def indexer_score(q_idx, pool_k_nt, w, q_pos, scores, m, npools, stream=None, sc
                   n_heads=32):
     """helios::attn::indexer_score (src/cuda/attn/attn.cuh:49-55); fp16 or bf16 keys by tensor dtype."""
     _run("hk_indexer_score", q_idx, pool_k_nt, w, q_pos, scores, m, npools, npools if score_stride is None else score_stride,
-         n_heads, q_idx, stream)
+         n_heads, _key_type(q_idx), stream)
 
 
 indexer_score_mma = indexer_score

@@ -99,6 +99,20 @@ def test_indexer_score_vs_oracle_and_reference(m, npools, bf16):
         assert (r != g).mean() < 0.2
 
 
+def test_fp16_keys_may_come_as_bit_patterns():
+    inp = synth.indexer_inputs(200, 2, seed=5)
+    q, k, w, q_pos = dev_f16(inp["q_idx"]), dev_f16(inp["pool_k"]), dev_f16(inp["w"]), dev(np.array([799, 500], dtype=np.int32))
+    res = []
+    for cast in (torch.float16, torch.int16):
+        sc, idx, raw = (torch.zeros(2, n, dtype=d, device="cuda") for n, d in ((200, torch.float16), (512, torch.int32), (2052, torch.int32)))
+        sc2 = torch.zeros_like(sc)
+        hk.indexer_score(q.view(cast), k.view(cast), w.view(cast), q_pos, sc2, 2, 200)
+        hk.indexer_select(q.view(cast), k.view(cast), w.view(cast), q_pos, sc, idx, raw, 2, 200, k=200)
+        res.append((sc, sc2, idx, raw))
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
+
+
 def test_indexer_legacy_matches_tensor_core_kernel():
     m, npools = 5, 300
     q_pos = np.array([1199, 3, 500, 777, 64], dtype=np.int32)
