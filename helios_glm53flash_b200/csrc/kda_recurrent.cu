@@ -2,20 +2,156 @@
 // history (rewindable) mode.  Interface and arithmetic of
 // helios::aux::cuda_recurrent_gated_delta_rule (reference: src/cuda/aux/gdn.cu:555-866).
 //
-// Layout of the work: one CTA per (batch item, head, slice of NV value-columns).  The CTA's
-// [D x NV] slice of the fp32 state lives in REGISTERS for the whole call (the reference re-reads and
-// re-writes it from global memory on every token), so a decode step moves each state byte exactly
-// once in and once out - the HBM floor of 2*H*D*D*4 bytes per layer-step - and a multi-token call
-// costs state traffic only once.  Thread (kg, j) owns column j and the D/KG consecutive k-rows of
-// group kg; the k-reduction is the sum of the KG group sums taken in ascending order, which for
-// D = 128, NV = 32 is exactly the reference's 4 x 32 order (gdn.cu:683-705).
+// Kernels:
+//   kda_decode_kernel, kda_decode_stream_kernel   one token per sequence (the decode step, the decode layer, the recurrence alone)
+//   kda_recurrent_cols_kernel                     several tokens, channelwise decay, no history
+//   kda_recurrent_rows_kernel                     channelwise decay with a history, and two to six tokens of many chains
+//   kda_recurrent_kernel                          one decay per head, 128- and 64-wide heads
+// The state lives in REGISTERS for the whole call (the reference re-reads and re-writes it from global memory on every token),
+// so a call moves each state byte once in and once out, the HBM floor of 2*H*D*D*4 bytes.
+//
+// Channelwise decay: ONE arithmetic for all kernels, so that a token gives the same bits whichever kernel it takes - alone or
+// with others in a call, with or without a history, by launcher, decode step or decode layer:
+//   S_c = S_c d_c;  kv = sum k_c S_c;  u = (v - kv) beta;  S_c = fma(k_c, u, S_c);  o = sum q_c S_c
+// (k_c d_c against the undecayed state, which is then rounded once per token, was no better: errors against 64 bits 2-6 % larger at
+// the model's gates, short prompts 2 % longer).  A sum over the 128 state rows is taken in 16 groups, group rg = the 4-row chunks rg and
+// rg + 16; a group runs over its even and its odd rows separately (the two halves of a packed fp32 pair), ascending; groups rg
+// and rg + 8 are added first, then the 8 sums as a balanced tree.  Norms: inv_norm.
+// One decay per head: 4 or 8 ascending row groups; for 128 x 32 slices that is the reference's 4 x 32 order (gdn.cu:683-705).
 #include "hk_common.cuh"
 #include "kda_norm_common.cuh"
 #include "tc05.cuh"
 
 namespace hk {
 
-template <int D, int NV, bool CW, bool HIST>
+__device__ __forceinline__ float tree8(float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
+  return __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), __fadd_rn(a2, a3)), __fadd_rn(__fadd_rn(a4, a5), __fadd_rn(a6, a7)));
+}
+// 128 channels of one token in one warp, channel lane + 32 u in x[u]: 1 / |x|
+__device__ __forceinline__ float inv_norm(const float (&x)[4]) {
+  float s = 0.f;
+#pragma unroll
+  for (int u = 0; u < 4; u++) s = fmaf(x[u], x[u], s);
+  return rsqrtf(warp_sum(s) + 1e-6f);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Channelwise decay, 128-wide heads: history mode, states with room for one, and two to six tokens of many chains.  One CTA per
+// (batch item, head, slice of NV value-columns); thread (kg, j) owns column j and the 16 / KG row groups of the shared order that
+// make up kg's part of the balanced tree.  Three warps prepare a token (q with its norm; k with its norm; the decay).
+// What bounds it: for few tokens the state in and out, in runs of 128 bytes; for many the three barriers of a token.  With the
+// head-wide kernel's order below, every warp in the norms and four barriers: 3 tokens of 32 chains 5.0 us, now 4.2; 6 of 1,536
+// 91 -> 69; 7 of 64 with history 13.1 -> 10.6; 63 of 8 with history 52 -> 36.
+// ---------------------------------------------------------------------------------------------
+template <int NV, bool HIST>
+__global__ __launch_bounds__(128) void kda_recurrent_rows_kernel(
+    const __nv_bfloat16* __restrict__ mixed_qkv, const float* __restrict__ g, const __nv_bfloat16* __restrict__ beta,
+    float* __restrict__ state, __nv_bfloat16* __restrict__ out, float* __restrict__ out_f32, int seqlen, int Hk, int Hv, float scale,
+    const int* __restrict__ slots, int history_stride) {
+  constexpr int D = 128, KG = 128 / NV, PAIRS = 8 / KG, RPT = D / KG;    // thread groups; pairs of row groups and rows per thread
+  const int b = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * NV;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j = tid % NV, kg = tid / NV;
+  const int k_head = head / (Hv / Hk);
+  const size_t row = (size_t)2 * Hk * D + (size_t)Hv * D, state_size = (size_t)Hv * D * D;
+  float* my_state = state + (size_t)(slots ? slots[b] : b) * history_stride * state_size + (size_t)head * D * D + v0 + j;
+  const __nv_bfloat16* tok = mixed_qkv + (size_t)b * seqlen * row;
+  const float* gp = g + ((size_t)b * seqlen * Hv + head) * D;
+  const __nv_bfloat16* bp = beta + (size_t)b * seqlen * Hv + head;
+  const size_t out_base = ((size_t)b * seqlen * Hv + head) * D + v0 + j;
+  __shared__ __align__(16) float sh_q[D], sh_k[D], sh_d[D];
+  __shared__ float sh_part[2][KG][NV];
+
+  // row e of this thread's group i: groups PAIRS kg ... and the same 8 further on
+  auto row_of = [&](int i, int e) { return 4 * (PAIRS * kg + i % PAIRS + 8 * (i / PAIRS) + 16 * (e >> 2)) + (e & 3); };
+  float S[RPT];
+#pragma unroll
+  for (int r = 0; r < RPT; r++) S[r] = my_state[(size_t)row_of(r >> 3, r & 7) * D];
+  // sums[i]: group i, even and odd rows
+  auto group_sums = [&](float (&s)[2 * PAIRS][2], int r, float c, float x) { s[r >> 3][r & 1] = fmaf(c, x, s[r >> 3][r & 1]); };
+  auto part_of = [&](const float (&s)[2 * PAIRS][2]) {
+    float p[PAIRS];
+#pragma unroll
+    for (int i = 0; i < PAIRS; i++)
+      p[i] = __fadd_rn(__fadd_rn(s[i][0], s[i][1]), __fadd_rn(s[i + PAIRS][0], s[i + PAIRS][1]));
+    return PAIRS == 2 ? __fadd_rn(p[0], p[PAIRS - 1]) : p[0];
+  };
+  auto total_of = [&](const float (&p)[KG][NV]) {
+    if constexpr (KG == 8) return tree8(p[0][j], p[1][j], p[2][j], p[3][j], p[4][j], p[5][j], p[6][j], p[7][j]);
+    else return __fadd_rn(__fadd_rn(p[0][j], p[1][j]), __fadd_rn(p[2][j], p[3][j]));
+  };
+
+  // the next token's operands: channels lane + 32 u of q, k or g by warp 0, 1, 2; this column's v; beta
+  __nv_bfloat16 nx[4], nv, nb;
+  float ng[4];
+  auto fetch = [&](int s) {
+    const __nv_bfloat16* t = tok + (size_t)s * row;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (warp < 2) nx[u] = t[(size_t)(warp * Hk + k_head) * D + lane + 32 * u];
+      if (warp == 2) ng[u] = gp[(size_t)s * Hv * D + lane + 32 * u];
+    }
+    nv = t[(size_t)2 * Hk * D + (size_t)head * D + v0 + j];
+    nb = bp[(size_t)s * Hv];
+  };
+  fetch(0);
+  for (int s = 0; s < seqlen; s++) {
+    const float v = __bfloat162float(nv), be = __bfloat162float(nb);
+    if (warp < 2) {
+      float x[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) x[u] = __bfloat162float(nx[u]);
+      const float r = inv_norm(x);
+#pragma unroll
+      for (int u = 0; u < 4; u++) (warp == 0 ? sh_q : sh_k)[lane + 32 * u] = __fmul_rn(x[u], r);
+    } else if (warp == 2) {
+#pragma unroll
+      for (int u = 0; u < 4; u++) sh_d[lane + 32 * u] = __expf(ng[u]);
+    }
+    if (s + 1 < seqlen) fetch(s + 1);
+    __syncthreads();
+    float a[2 * PAIRS][2] = {};
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+      const int c = row_of(r >> 3, r & 7);
+      S[r] = __fmul_rn(S[r], sh_d[c]);
+      group_sums(a, r, sh_k[c], S[r]);
+    }
+    sh_part[0][kg][j] = part_of(a);
+    __syncthreads();
+    const float un = __fmul_rn(__fsub_rn(v, total_of(sh_part[0])), be);
+    float o[2 * PAIRS][2] = {};
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+      const int c = row_of(r >> 3, r & 7);
+      S[r] = fmaf(sh_k[c], un, S[r]);
+      group_sums(o, r, sh_q[c], S[r]);
+    }
+    sh_part[1][kg][j] = part_of(o);
+    if (HIST) {
+      // step s writes history slot s+1; the last step writes the final slot 0
+      float* dst = s == seqlen - 1 ? my_state : my_state + (size_t)(s + 1) * state_size;
+#pragma unroll
+      for (int r = 0; r < RPT; r++) dst[(size_t)row_of(r >> 3, r & 7) * D] = S[r];
+    }
+    __syncthreads();
+    if (kg == 0) {
+      const float tot = total_of(sh_part[1]) * scale;
+      const size_t oi = out_base + (size_t)s * Hv * D;
+      out[oi] = __float2bfloat16_rz(tot);
+      if (out_f32) out_f32[oi] = tot;
+    }
+  }
+  if (!HIST) {
+#pragma unroll
+    for (int r = 0; r < RPT; r++) my_state[(size_t)row_of(r >> 3, r & 7) * D] = S[r];
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// One decay per head: one CTA per (batch item, head, slice of NV value-columns); thread (kg, j) owns column j and the D/KG
+// consecutive k-rows of group kg.
+// ---------------------------------------------------------------------------------------------
+template <int D, int NV, bool HIST>
 __global__ __launch_bounds__(128) void kda_recurrent_kernel(
     const __nv_bfloat16* __restrict__ mixed_qkv, const float* __restrict__ g,
     const __nv_bfloat16* __restrict__ beta, float* __restrict__ state,
@@ -36,11 +172,11 @@ __global__ __launch_bounds__(128) void kda_recurrent_kernel(
   float* my_state = slot_state + head * head_state + (size_t)(kg * RPT) * D + v0 + j;
 
   const __nv_bfloat16* tok = mixed_qkv + (size_t)b * seqlen * row;
-  const float* gp = g + (size_t)b * seqlen * Hv * (CW ? D : 1) + (size_t)head * (CW ? D : 1);
+  const float* gp = g + (size_t)b * seqlen * Hv + head;
   const __nv_bfloat16* bp = beta + (size_t)b * seqlen * Hv + head;
   const size_t out_base = ((size_t)b * seqlen * Hv + head) * D + v0 + j;
 
-  __shared__ float sh_q[D], sh_k[D], sh_d[D];
+  __shared__ float sh_q[D], sh_k[D];
   __shared__ float sh_red[2][4];
   __shared__ float sh_part[2][KG][NV];
 
@@ -49,13 +185,12 @@ __global__ __launch_bounds__(128) void kda_recurrent_kernel(
   for (int i = 0; i < RPT; i++) S[i] = my_state[(size_t)i * D];
 
   // software prefetch of the next token's operands
-  float nq = 0.f, nk = 0.f, ng = 0.f, nv, nb;
+  float nq = 0.f, nk = 0.f, ng, nv, nb;
   if (tid < D) {
     nq = __bfloat162float(tok[(size_t)k_head * D + tid]);
     nk = __bfloat162float(tok[(size_t)(Hk + k_head) * D + tid]);
-    if (CW) ng = gp[tid];
   }
-  if (!CW) ng = gp[0];
+  ng = gp[0];
   nv = __bfloat162float(tok[(size_t)2 * Hk * D + (size_t)head * D + v0 + j]);
   nb = __bfloat162float(bp[0]);
 
@@ -66,9 +201,8 @@ __global__ __launch_bounds__(128) void kda_recurrent_kernel(
       if (tid < D) {
         nq = __bfloat162float(nt[(size_t)k_head * D + tid]);
         nk = __bfloat162float(nt[(size_t)(Hk + k_head) * D + tid]);
-        if (CW) ng = gp[(size_t)(s + 1) * Hv * D + tid];
       }
-      if (!CW) ng = gp[(size_t)(s + 1) * Hv];
+      ng = gp[(size_t)(s + 1) * Hv];
       nv = __bfloat162float(nt[(size_t)2 * Hk * D + (size_t)head * D + v0 + j]);
       nb = __bfloat162float(bp[(size_t)(s + 1) * Hv]);
     }
@@ -88,17 +222,15 @@ __global__ __launch_bounds__(128) void kda_recurrent_kernel(
       }
       sh_q[tid] = q * rsqrtf(tq + 1e-6f);
       sh_k[tid] = k * rsqrtf(tk + 1e-6f);
-      if (CW) sh_d[tid] = __expf(gv);
     }
     __syncthreads();
-    // ---- kv_j = sum_c k_c d_c S[c][j] (the state is read decayed when channelwise) ----
-    const float g_h = CW ? 1.0f : __expf(gv);
+    // ---- kv_j = sum_c k_c S[c][j] ----
+    const float g_h = __expf(gv);
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < RPT; i++) {
       const int c = kg * RPT + i;
-      if (CW) sum = sum + sh_k[c] * sh_d[c] * S[i];
-      else    sum = sum + sh_k[c] * S[i];
+      sum = sum + sh_k[c] * S[i];
     }
     sh_part[0][kg][j] = sum;
     __syncthreads();
@@ -111,7 +243,7 @@ __global__ __launch_bounds__(128) void kda_recurrent_kernel(
 #pragma unroll
     for (int i = 0; i < RPT; i++) {
       const int c = kg * RPT + i;
-      float st = S[i] * (CW ? sh_d[c] : g_h) + sh_k[c] * vp * beta_h;
+      float st = S[i] * g_h + sh_k[c] * vp * beta_h;
       S[i] = st;
       o = o + sh_q[c] * st;
     }
@@ -137,24 +269,6 @@ __global__ __launch_bounds__(128) void kda_recurrent_kernel(
 #pragma unroll
     for (int i = 0; i < RPT; i++) my_state[(size_t)i * D] = S[i];
   }
-}
-
-// ---------------------------------------------------------------------------------------------
-// Arithmetic shared by the decode kernels and the per-token kernel below (channelwise decay, D = 128): a token run through
-// either gives the same bits.  The 128 state rows of a column form 16 groups, group rg = the 4-row chunks rg and rg + 16; a group
-// sum runs over its even and its odd rows separately (the two halves of a packed fp32 pair), ascending; groups rg and rg + 8 are
-// added first, then the 8 sums as a balanced tree.  S_c = S_c d_c;
-// kv = sum k_c S_c;  u = (v - kv) * beta;  S_c = fma(k_c, u, S_c);  o = sum q_c S_c.
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ float tree8(float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
-  return __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), __fadd_rn(a2, a3)), __fadd_rn(__fadd_rn(a4, a5), __fadd_rn(a6, a7)));
-}
-// 128 channels of one token in one warp, channel lane + 32 u in x[u]: 1 / |x|
-__device__ __forceinline__ float inv_norm(const float (&x)[4]) {
-  float s = 0.f;
-#pragma unroll
-  for (int u = 0; u < 4; u++) s = fmaf(x[u], x[u], s);
-  return rsqrtf(warp_sum(s) + 1e-6f);
 }
 
 // window and taps of one channel arrive as one 8-byte load each
@@ -819,20 +933,27 @@ __global__ __launch_bounds__(RC_WARPS * 32) void kda_recurrent_cols_kernel(
   }
 }
 
+// narrower column slices when the (batch x head) count alone cannot cover the SMs
+static bool narrow_slices(int bsz, int Hv) { return (long)bsz * Hv * 4 < sm_count(); }
+
+static int launch_rows(const __nv_bfloat16* qkv, const float* g, const __nv_bfloat16* beta, float* state, __nv_bfloat16* out,
+                       float* out_f32, int bsz, int seqlen, int Hk, int Hv, int history_stride, const int* slots, bool hist,
+                       cudaStream_t s) {
+  const bool narrow = narrow_slices(bsz, Hv);
+  auto kern = narrow ? (hist ? kda_recurrent_rows_kernel<16, true> : kda_recurrent_rows_kernel<16, false>)
+                     : (hist ? kda_recurrent_rows_kernel<32, true> : kda_recurrent_rows_kernel<32, false>);
+  kern<<<dim3(bsz, Hv, narrow ? 8 : 4), 128, 0, s>>>(qkv, g, beta, state, out, out_f32, seqlen, Hk, Hv, 1.0f / sqrtf(128.0f), slots,
+                                                     history_stride);
+  return cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+}
+
 template <int D, int NV>
 static int launch_recurrent(const __nv_bfloat16* qkv, const float* g, const __nv_bfloat16* beta,
                             float* state, __nv_bfloat16* out, float* out_f32, int bsz, int seqlen,
-                            int Hk, int Hv, int history_stride, const int* slots, bool cw,
-                            bool hist, cudaStream_t s) {
-  dim3 grid(bsz, Hv, D / NV);
-  const float scale = 1.0f / sqrtf((float)D);
-#define HK_RL(CWV, HV)                                                                             \
-  kda_recurrent_kernel<D, NV, CWV, HV><<<grid, 128, 0, s>>>(qkv, g, beta, state, out, out_f32,    \
-                                                            seqlen, Hk, Hv, scale, slots,          \
-                                                            history_stride)
-  if (cw) { if (hist) HK_RL(true, true); else HK_RL(true, false); }
-  else    { if (hist) HK_RL(false, true); else HK_RL(false, false); }
-#undef HK_RL
+                            int Hk, int Hv, int history_stride, const int* slots, bool hist, cudaStream_t s) {
+  auto kern = hist ? kda_recurrent_kernel<D, NV, true> : kda_recurrent_kernel<D, NV, false>;
+  kern<<<dim3(bsz, Hv, D / NV), 128, 0, s>>>(qkv, g, beta, state, out, out_f32, seqlen, Hk, Hv, 1.0f / sqrtf((float)D), slots,
+                                             history_stride);
   return cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 
@@ -881,19 +1002,14 @@ HK_API int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* b
                  : HK_ERR_CUDA;
     }
   }
-  // narrower column slices when the (batch x head) count alone cannot cover the SMs
-  const bool narrow = (long)bsz * num_v_heads * 4 < sm_count();
-  if (k_head_dim == 128) {
-    return narrow ? launch_recurrent<128, 16>(q, g, bt, state, o, out_f32, bsz, seqlen, num_k_heads,
-                                              num_v_heads, history_stride, slots, channelwise,
-                                              history, s)
-                  : launch_recurrent<128, 32>(q, g, bt, state, o, out_f32, bsz, seqlen, num_k_heads,
-                                              num_v_heads, history_stride, slots, channelwise,
-                                              history, s);
-  }
+  if (channelwise)
+    return launch_rows(q, g, bt, state, o, out_f32, bsz, seqlen, num_k_heads, num_v_heads, history_stride, slots, history, s);
+  if (k_head_dim == 128)
+    return narrow_slices(bsz, num_v_heads)
+               ? launch_recurrent<128, 16>(q, g, bt, state, o, out_f32, bsz, seqlen, num_k_heads, num_v_heads, history_stride, slots, history, s)
+               : launch_recurrent<128, 32>(q, g, bt, state, o, out_f32, bsz, seqlen, num_k_heads, num_v_heads, history_stride, slots, history, s);
   if (k_head_dim == 64)
-    return launch_recurrent<64, 32>(q, g, bt, state, o, out_f32, bsz, seqlen, num_k_heads,
-                                    num_v_heads, history_stride, slots, channelwise, history, s);
+    return launch_recurrent<64, 32>(q, g, bt, state, o, out_f32, bsz, seqlen, num_k_heads, num_v_heads, history_stride, slots, history, s);
   return HK_ERR_UNSUPPORTED;
 }
 

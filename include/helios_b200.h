@@ -62,7 +62,11 @@ int hk_conv1d_update(const void* x, void* conv_state, const int* slots, const vo
  *   (channelwise) or [bsz][seqlen][Hv]      beta [bsz][seqlen][Hv] bf16
  *   state [slots][history_stride][Hv][dk][dv] f32 (in place)   out [bsz][seqlen][Hv][dv] bf16 (rz)
  *   out_f32: optional (may be NULL) copy of the output before bf16 rounding, same shape.
- * Supported head dims: (dk,dv) = (128,128) and (64,64).                                          */
+ * Supported head dims: (dk,dv) = (128,128) and (64,64).
+ * With channelwise decay every kernel behind this call, hk_kda_decode_step and hk_kda_decode_layer sums in one order: a token
+ * gives the same bits alone or with others in a call, with or without history, and from any of the three.  It is not the
+ * reference's order (fp32 throughout; errors against 64 bits are no larger).  hk_kda_chunked_prefill is another algorithm and
+ * agrees within its tolerance only.                                                              */
 int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* beta, float* state,
                      void* out, float* out_f32, int bsz, int seqlen, int num_k_heads,
                      int num_v_heads, int k_head_dim, int v_head_dim, int history_stride,

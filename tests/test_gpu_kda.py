@@ -417,3 +417,37 @@ def test_per_token_kernel_around_its_batches_of_eight(T, Hk, Hv, bsz):
     torch.cuda.synchronize()
     assert max_rel(f32.cpu().numpy(), o_32) < 1e-4 and frob_rel(st.cpu().numpy(), o_st) < 1e-5
     assert np.array_equal(bits(out), (f32.cpu().numpy().view(np.uint32) >> 16).astype(np.uint16)), "rounded toward zero"
+
+
+@pytest.mark.parametrize("H,bsz", [(2, 1), (40, 1), (8, 3), (64, 17)])
+def test_token_by_token_routes_agree_bit_for_bit(H, bsz):
+    """tokens one at a time, several in a call, and calls on a state with room for a history, recording it or not: whichever
+    kernel a call takes (2 chains narrow, 40 and 24 the per-token kernel or the older one by length, 1,088 streamed), the same bits"""
+    D, T = 128, 7
+    gen = torch.Generator(device="cuda").manual_seed(H)
+
+    def rnd(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+    qkv, g = rnd(bsz, T, 3 * H * D).to(torch.bfloat16), -5.0 * torch.sigmoid(rnd(bsz, T, H, D))
+    beta, s0 = torch.sigmoid(rnd(bsz, T, H)).to(torch.bfloat16), 0.1 * rnd(bsz, 1, H, D, D)
+
+    def call(t0, n, st, stride=1, history=False):
+        q, gg, b = (x[:, t0:t0 + n].contiguous() for x in (qkv, g, beta))
+        out, f32 = (torch.empty(bsz, n, H, D, dtype=d, device="cuda") for d in (torch.bfloat16, torch.float32))
+        hk.cuda_recurrent_gated_delta_rule(q, gg, b, st, out, bsz, n, H, H, D, D, stride, None, True, history, out_f32=f32)
+        assert torch.equal(out.view(torch.int16), (f32.view(torch.int32) >> 16).to(torch.int16)), "rounded toward zero"
+        return f32
+    st, outs, states = s0.clone(), [], []
+    for t in range(T):
+        outs.append(call(t, 1, st))
+        states.append(st.clone())
+    outs = torch.cat(outs, dim=1)
+    for n in (2, 3, 6, 7):
+        st = s0.clone()
+        assert torch.equal(call(0, n, st), outs[:, :n]) and torch.equal(st, states[n - 1]), n
+    for history in (False, True):
+        st = torch.zeros(bsz, T, H, D, D, device="cuda")
+        st[:, :1] = s0
+        assert torch.equal(call(0, T, st, T, history), outs) and torch.equal(st[:, :1], states[-1])
+        for t in range(T - 1 if history else 0):
+            assert torch.equal(st[:, t + 1:t + 2], states[t])
