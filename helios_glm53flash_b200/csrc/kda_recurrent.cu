@@ -1019,6 +1019,7 @@ HK_API int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_
   using namespace hk;
   HK_REQUIRE(x && conv_state && conv_weight && g && beta && rec_state && out && tickets);
   HK_REQUIRE(bsz > 0 && bsz <= 65535 && num_heads > 0 && num_heads <= 65535);
+  HK_REQUIRE(aligned(conv_state, 8) && aligned(conv_weight, 8));   // a channel's window and taps are one access each
   DecodeArgs a{};
   a.x = x;
   a.conv_state = (__nv_bfloat16*)conv_state;
@@ -1050,6 +1051,7 @@ HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* c
   HK_REQUIRE(y_type == HK_F32 || y_type == HK_F16);
   HK_REQUIRE(g_type == HK_F32 || g_type == HK_BF16);
   HK_REQUIRE(gate_act == 0 || gate_act == 1);
+  HK_REQUIRE(aligned(conv_state, 8) && aligned(conv_weight, 8));
   HK_REQUIRE(aligned(out, 8) && aligned(norm_w, w_type == HK_F32 ? 16 : 8) && aligned(y, y_type == HK_F32 ? 16 : 8) &&
              aligned(gate_out, g_type == HK_F32 ? 16 : 8));
   DecodeArgs a{};

@@ -75,7 +75,8 @@ int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* beta, fl
 /* One KDA decode step with the short convolution inside: what the engine runs per decoded token as
  * cuda_causal_conv1d_update(seqlen 1, K = state_size = 4, SiLU) followed by cuda_recurrent_gated_delta_rule(seqlen 1,
  * channelwise) (src/engine/runner.cpp:443-471), in ONE launch and with the same bits.  Head dim 128, Hk == Hv.
- *   x [bsz][3*H*128] bf16 (the token's pre-conv q|k|v)   conv_state [slots][3*H*128][4] bf16 (in place)
+ *   x [bsz][3*H*128] bf16 (the token's pre-conv q|k|v)   conv_state [slots][3*H*128][4] bf16 (in place); conv_state and
+ *   conv_weight 8-byte aligned
  *   conv_weight [3*H*128][4] bf16   conv_bias [3*H*128] bf16 or NULL   g [bsz][H][128] f32   beta [bsz][H] bf16
  *   rec_state [slots][H][128][128] f32 (in place)   out [bsz][H][128] bf16 (rz)   out_f32 optional
  *   conv_out optional [bsz][3*H*128] bf16: the convolved q|k|v (what the two-kernel sequence leaves in between).

@@ -86,3 +86,12 @@ def test_host_only_answers_of_the_abi(built):
     assert rule(4096, 128, 128, 1, 1) == 0 and rule(4096, 128, 128, 0, 0) == 0 and rule(4096, 64, 64, 1, 0) == 0
     # static no-allocation entry: 64 (split, row) slots
     assert lib.hk_mla_sparse_static_max_slots() == 64
+
+
+def test_decode_refuses_windows_it_cannot_read_in_one_access(built):
+    """conv_state and conv_weight are accessed a channel at a time, 8 bytes: other addresses are an error on the host"""
+    lib, a = hk.load_library(), 1 << 20                      # never dereferenced: refused before any launch
+    for state, weight in ((a + 4, a), (a, a + 2)):
+        assert lib.hk_kda_decode_step(a, state, weight, None, a, a, a, a, None, None, 1, 4, None, a, None) == hk.HK_ERR_INVALID
+        assert lib.hk_kda_decode_layer(a, state, weight, None, a, a, a, a, -5.0, a, a, None, a, hk.HK_F32, a, hk.HK_F32, a, hk.HK_F16,
+                                       1e-6, 0.0, 1, 1, 4, None, a, None) == hk.HK_ERR_INVALID
