@@ -218,20 +218,11 @@ def cuda_recurrent_gated_delta_rule(mixed_qkv, g, beta, recurrent_state, core_at
     return "recurrent"
 
 
-_decode_tickets = {}
-
-
 def kda_decode_step(x, conv_state, conv_weight, conv_bias, g, beta, rec_state, out, bsz, num_heads, slots=None,
                     out_f32=None, conv_out=None, stream=None, tickets=None):
     """cuda_causal_conv1d_update(seqlen 1, K = 4, SiLU) + cuda_recurrent_gated_delta_rule(seqlen 1, channelwise) of one
-    decoded token (src/engine/runner.cpp:443-471) in one launch; head dim 128.  `tickets`: bsz * num_heads zeroed
-    int32 on the device (one buffer per device is kept here when none is given: single-stream use)."""
-    if tickets is None:
-        torch = _require_cuda()
-        key = (x.device.index, bsz * num_heads)
-        tickets = _decode_tickets.get(key)
-        if tickets is None:
-            tickets = _decode_tickets[key] = torch.zeros(bsz * num_heads, dtype=torch.int32, device=x.device)
+    decoded token (src/engine/runner.cpp:443-471) in one launch; head dim 128.  `tickets` is accepted for earlier callers and
+    not used."""
     _run("hk_kda_decode_step", x, conv_state, conv_weight, conv_bias, g, beta, rec_state, out, out_f32, conv_out, bsz,
          num_heads, slots, tickets, stream)
 
@@ -242,13 +233,7 @@ def kda_decode_layer(x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_l
     """The KDA layer of one decoded token in ONE launch (src/engine/runner.cpp:433-489 runs five): x = bf16(x32)
     (glue::kda_transpose_cast of one row), g / beta from f / b (glue::kda_gate), short conv + SiLU, recurrence, gated RMS
     norm of the output (aux::gated_rms_norm with gate `gate_out`, weight `norm_w`) -> y.  `out` receives the recurrence
-    output as the separate calls would leave it.  `tickets`: 2 * bsz * num_heads zeroed int32."""
-    if tickets is None:
-        torch = _require_cuda()
-        key = (x32.device.index, -2 * bsz * num_heads)
-        tickets = _decode_tickets.get(key)
-        if tickets is None:
-            tickets = _decode_tickets[key] = torch.zeros(2 * bsz * num_heads, dtype=torch.int32, device=x32.device)
+    output as the separate calls would leave it.  `tickets` is accepted for earlier callers and not used."""
     _run("hk_kda_decode_layer", x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_log, lower_bound, rec_state, out,
          out_f32, norm_w, norm_w, gate_out, gate_out, y, y, epsilon, constant_bias, int(gate_act), bsz, num_heads, slots,
          tickets, stream)

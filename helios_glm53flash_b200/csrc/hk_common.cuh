@@ -68,19 +68,27 @@ __device__ __forceinline__ void pdl_release(bool small_grid = true) {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// cluster: CTAs of a thread-block cluster along x
 template <class... P, class... A>
-inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
-  cudaLaunchAttribute attr[1];
+inline cudaError_t pdl_launch_cluster(unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = (int64_t)grid.x * grid.y * grid.z <= 8 * sm_count() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = (int64_t)grid.x * grid.y * grid.z <= 8 * sm_count() ? 1 : 0;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  return pdl_launch_cluster(1, kernel, grid, block, smem, s, std::forward<A>(args)...);
 }
 
 // device word (per device) where kernels record that a bounded wait gave up; see hk_read_device_status

@@ -325,7 +325,6 @@ struct DecodeArgs {
   float eps, cbias, scale;
   int H, n_heads;                       // heads of a sequence; batch * H
   int Hk;                               // key heads of a sequence (DEC_REC; else H)
-  int* tickets;                         // DEC_STEP: slices of a head that have read its windows
   const int* slots;
 };
 
@@ -520,9 +519,11 @@ __device__ __forceinline__ float* head_state(const DecodeArgs& a, int bh) {
 
 // VEC: the state is 16-byte aligned.
 // SLICES = 4: a CTA owns 32 of the head's 128 columns (two state warps, a quarter warp per row group, the same sums in the
-// same order).  One SM moves a head's 64 KB in and out in 0.6 us each, and a few heads leave the other SMs idle: 32 heads 3.25 ->
-// 2.9 us per step, one token's recurrence alone 2.2.  Not for DEC_LAYER, whose norm needs all columns of a head.  The q and k windows are read by every slice
-// and rolled by the one that draws the last ticket; nobody waits for it.
+// same order).  One SM moves a head's 64 KB in and out in 0.6 us each, and a few heads leave the other SMs idle: one token's
+// recurrence alone 2.7 us at 32 heads.  Not for DEC_LAYER, whose norm needs all columns of a head.  In DEC_STEP the
+// four are a cluster: the windows are read by every slice and rolled by the first behind a cluster barrier that all have arrived at
+// long before (32 heads 3.0 us per step; counting the slices through a word of global memory per head 3.13, at 8 heads 2.53 and
+// 2.85, and calls on several streams needed counters of their own).
 template <int MODE, bool VEC, int SLICES>
 __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const DecodeArgs a) {
   constexpr int SW = KD_STATE_WARPS / SLICES;                // state warps
@@ -532,7 +533,6 @@ __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const Decod
   const int cl = SLICES == 1 ? lane : (int)(blockIdx.x % SLICES) * (32 / SLICES) + (lane & 7);   // four columns
   __shared__ __align__(16) DecodeToken tok;
   __shared__ __align__(16) float part[8][128], opart[8][128];
-  __shared__ int last;
   pdl_wait();
   float4 S[16];
   uint2 rolled[4];
@@ -552,10 +552,7 @@ __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const Decod
     if (MODE != DEC_REC && SLICES == 1) decode_roll(a, bh, warp - SW, lane, rolled);
   }
   __syncthreads();
-  if (MODE == DEC_STEP && SLICES > 1 && threadIdx.x == SW * 32) {
-    __threadfence();
-    last = atomicAdd(&a.tickets[bh], 1) == SLICES - 1;
-  }
+  if (MODE == DEC_STEP && SLICES > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // windows read
   if (warp < SW) state_kv(S, tok, rg, cl, part);
   __syncthreads();
   if (warp < SW) {
@@ -566,9 +563,10 @@ __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const Decod
       if (VEC) *reinterpret_cast<float4*>(p) = S[i];
       else { p[0] = S[i].x; p[1] = S[i].y; p[2] = S[i].z; p[3] = S[i].w; }
     }
-  } else if (MODE == DEC_STEP && SLICES > 1 && last) {
-    decode_roll(a, bh, warp - SW, lane, rolled);
-    if (threadIdx.x == SW * 32) a.tickets[bh] = 0;
+  }
+  if (MODE == DEC_STEP && SLICES > 1) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp >= SW && blockIdx.x % SLICES == 0) decode_roll(a, bh, warp - SW, lane, rolled);
   }
   __syncthreads();
   if (warp == FW && (SLICES == 1 || lane < 32 / SLICES)) decode_finish<MODE>(a, fin, opart, bh, SLICES == 1 ? lane : cl);
@@ -664,7 +662,9 @@ static int launch_decode(const DecodeArgs& a, cudaStream_t s) {
   }
   if constexpr (MODE != DEC_LAYER) {
     if (vec && a.n_heads <= sm_count() / 2)
-      return pdl_launch(kda_decode_kernel<MODE, true, 4>, dim3(4 * a.n_heads), dim3(5 * 32), 0, s, a) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+      return pdl_launch_cluster(MODE == DEC_STEP ? 4 : 1, kda_decode_kernel<MODE, true, 4>, dim3(4 * a.n_heads), dim3(5 * 32), 0, s, a) == cudaSuccess
+                 ? HK_OK
+                 : HK_ERR_CUDA;
   }
   auto kern = vec ? kda_decode_kernel<MODE, true, 1> : kda_decode_kernel<MODE, false, 1>;
   return pdl_launch(kern, dim3(a.n_heads), dim3(KD_THREADS + (MODE == DEC_LAYER ? 32 : 0)), 0, s, a) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
@@ -1017,7 +1017,8 @@ HK_API int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_
                               const void* beta, float* rec_state, void* out, float* out_f32, void* conv_out, int bsz,
                               int num_heads, const int* slots, int* tickets, void* stream) {
   using namespace hk;
-  HK_REQUIRE(x && conv_state && conv_weight && g && beta && rec_state && out && tickets);
+  HK_REQUIRE(x && conv_state && conv_weight && g && beta && rec_state && out);
+  (void)tickets;
   HK_REQUIRE(bsz > 0 && bsz <= 65535 && num_heads > 0 && num_heads <= 65535);
   HK_REQUIRE(aligned(conv_state, 8) && aligned(conv_weight, 8));   // a channel's window and taps are one access each
   DecodeArgs a{};
@@ -1034,7 +1035,6 @@ HK_API int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_
   a.scale = 1.0f / sqrtf(128.0f);
   a.H = a.Hk = num_heads;
   a.n_heads = bsz * num_heads;
-  a.tickets = tickets;
   a.slots = slots;
   return launch_decode<DEC_STEP>(a, as_stream(stream));
 }
@@ -1045,7 +1045,8 @@ HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* c
                                int y_type, float epsilon, float constant_bias, int gate_act, int bsz, int num_heads,
                                const int* slots, int* tickets, void* stream) {
   using namespace hk;
-  HK_REQUIRE(x32 && conv_state && conv_weight && f && b && dt_bias && a_log && rec_state && out && norm_w && gate_out && y && tickets);
+  HK_REQUIRE(x32 && conv_state && conv_weight && f && b && dt_bias && a_log && rec_state && out && norm_w && gate_out && y);
+  (void)tickets;
   HK_REQUIRE(bsz > 0 && bsz <= 65535 && num_heads > 0 && num_heads <= 65535);
   HK_REQUIRE(w_type == HK_F32 || w_type == HK_BF16);
   HK_REQUIRE(y_type == HK_F32 || y_type == HK_F16);

@@ -80,7 +80,7 @@ int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* beta, fl
  *   conv_weight [3*H*128][4] bf16   conv_bias [3*H*128] bf16 or NULL   g [bsz][H][128] f32   beta [bsz][H] bf16
  *   rec_state [slots][H][128][128] f32 (in place)   out [bsz][H][128] bf16 (rz)   out_f32 optional
  *   conv_out optional [bsz][3*H*128] bf16: the convolved q|k|v (what the two-kernel sequence leaves in between).
- *   tickets: bsz*H device ints, zero before the first call; left zero (a few heads are split over CTAs, which count here). */
+ *   tickets: not used any more, may be NULL (calls on several streams need nothing of their own).                        */
 int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_weight, const void* conv_bias, const float* g,
                        const void* beta, float* rec_state, void* out, float* out_f32, void* conv_out, int bsz,
                        int num_heads, const int* slots, int* tickets, void* stream);
@@ -92,7 +92,7 @@ int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_weight,
  * norm_w [128] of w_type (HK_F32 / HK_BF16), gate_out [bsz*H][128] of g_type (HK_F32 / HK_BF16).  `out` (bf16) and
  * out_f32 (optional) receive the recurrence output.  The reference's decode runs five launches here
  * (src/engine/runner.cpp:433-489); results are bit-identical to calling the five in turn.
- * tickets: 2 * bsz * H zeroed ints of caller memory, left zeroed (not used any more).                               */
+ * tickets: not used any more, may be NULL.                                                                          */
 int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f,
                         const float* b, const float* dt_bias, const float* a_log, float lower_bound, float* rec_state,
                         void* out, float* out_f32, const void* norm_w, int w_type, const void* gate_out, int g_type, void* y,

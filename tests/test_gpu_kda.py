@@ -451,3 +451,31 @@ def test_token_by_token_routes_agree_bit_for_bit(H, bsz):
         assert torch.equal(call(0, T, st, T, history), outs) and torch.equal(st[:, :1], states[-1])
         for t in range(T - 1 if history else 0):
             assert torch.equal(st[:, t + 1:t + 2], states[t])
+
+
+@pytest.mark.parametrize("H", [4, 32])
+def test_decode_steps_share_nothing(H):
+    """heads split over CTAs, on several streams at a time and whatever `tickets` holds: windows, states and outputs of each as
+    when it runs alone"""
+    D, dim, steps = 128, 3 * H * 128, 6
+    gen = torch.Generator(device="cuda").manual_seed(H)
+
+    def rnd(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+    x, w, cs0 = rnd(steps, dim).to(torch.bfloat16), (0.1 * rnd(dim, 4)).to(torch.bfloat16), rnd(1, dim, 4).to(torch.bfloat16)
+    g, beta, s0 = -torch.rand(steps, H, D, generator=gen, device="cuda"), torch.sigmoid(rnd(steps, H)).to(torch.bfloat16), 0.1 * rnd(1, H, D, D)
+
+    def run(stream, tickets, cs, st, out):
+        for t in range(steps):
+            hk.kda_decode_step(x[t], cs, w, None, g[t], beta[t], st, out[t], 1, H, stream=stream, tickets=tickets)
+    junk = torch.full((H,), 3, dtype=torch.int32, device="cuda")
+    jobs = [(torch.cuda.Stream(), junk if i == 3 else None, cs0.clone(), s0.clone(), torch.zeros(steps, H, D, dtype=torch.bfloat16, device="cuda"))
+            for i in range(4)]
+    run(None, torch.zeros(H, dtype=torch.int32, device="cuda"), *jobs[0][2:])
+    torch.cuda.synchronize()
+    for job in jobs[1:]:
+        run(*job)
+    torch.cuda.synchronize()
+    for job in jobs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(job[2:], jobs[0][2:]))
+    assert (junk == 3).all()
