@@ -2,7 +2,8 @@
 // operands staged in the no-swizzle canonical layouts (or, per operand, the 128-byte-swizzle layouts
 // a TMA tensor copy with 128-byte rows produces) and dumps the raw TMEM accumulator
 // (all 128 lanes x N columns), so the host can check both the arithmetic and the row <-> lane
-// mapping of each instruction shape.
+// mapping of each instruction shape.  The weight-stationary form (tc::mma_ws_f16_if) leaves N / 2 columns; its A operand may
+// also sit in tensor memory (tc::mma_ws_f16_tmem_a_if).
 #include "hk_common.cuh"
 #include "tc05.cuh"
 
@@ -20,7 +21,9 @@ __global__ __launch_bounds__(128) void tc05_selftest_kernel(const __half* __rest
   // the offset-swap diagnostics exist for the no-swizzle layouts only: a swapped stride offset of a
   // swizzled tile would point past the operand region
   const bool b_mn = flags & 1, a_mn = flags & 2, swap_a = (flags & 0x100) && !a_sw, swap_b = (flags & 0x200) && !b_sw;
-  const bool converged_issue = flags & 0x400;   // issue from the whole of warp 0 with one elected lane (tc::mma_f16_if)
+  const bool a_tmem = flags & 0x1000;           // A moved to tensor memory, columns 128 on, a copy in either half of the lanes
+  const bool ws = (flags & 0x800) || a_tmem;    // weight-stationary form, converged issue
+  const bool converged_issue = (flags & 0x400) || ws;   // issue from the whole of warp 0 with one elected lane (tc::mma_f16_if)
   const int tid = threadIdx.x, warp = tc::warp_index_uniform();
   uint8_t* sA = smem;
   uint8_t* sB = smem + 128 * 128 * 2;
@@ -89,6 +92,18 @@ __global__ __launch_bounds__(128) void tc05_selftest_kernel(const __half* __rest
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_slot;
+  if (a_tmem) {                                  // A [64][K]: row tid % 64 in lane tid, two elements per column (K % 64 == 0)
+    for (int c0 = 0; c0 < K / 2; c0 += 32) {
+      uint32_t v[32];
+#pragma unroll
+      for (int j = 0; j < 32; j++) v[j] = reinterpret_cast<const uint32_t*>(A + (size_t)(tid & 63) * K)[c0 + j];
+      tc::tmem_st32(tmem + 128 + c0 + ((uint32_t)(warp * 32) << 16), v);
+    }
+    tc::tmem_st_wait();
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+  }
   if (warp == 0) {
     // both issue forms run the same loop: every lane of warp 0 computes the (warp-uniform) descriptors; either
     // lane 0 alone issues from a diverged branch, or an elected lane issues from the converged warp
@@ -109,7 +124,9 @@ __global__ __launch_bounds__(128) void tc05_selftest_kernel(const __half* __rest
         const uint32_t st = tc::smem_u32(sB) + (b_mn ? kk * 2048 : (kk >> 2) * blk_b + (kk & 3) * 32);
         bd = swap_b ? tc::make_sdesc_sw128(st, 1024, blk_b) : tc::make_sdesc_sw128(st, blk_b, 1024);
       }
-      if (converged_issue) tc::mma_f16_if(leader, tmem, ad, bd, idesc, kk > 0);
+      if (a_tmem) tc::mma_ws_f16_tmem_a_if(leader, tmem, tmem + 128 + kk * 8, bd, idesc, kk > 0);
+      else if (ws) tc::mma_ws_f16_if(leader, tmem, ad, bd, idesc, kk > 0);
+      else if (converged_issue) tc::mma_f16_if(leader, tmem, ad, bd, idesc, kk > 0);
       else if (leader) tc::mma_f16(tmem, ad, bd, idesc, kk > 0);
     }
     if (converged_issue) tc::mma_commit_if(leader, &bar);
@@ -119,7 +136,7 @@ __global__ __launch_bounds__(128) void tc05_selftest_kernel(const __half* __rest
   const bool ok = tc::mbar_wait(&bar, 0, &abort_flag, 1);
   tc::fence_after_sync();
   if (ok) {
-    for (int c0 = 0; c0 < N; c0 += 16) {
+    for (int c0 = 0; c0 < (ws ? N / 2 : N); c0 += 16) {
       uint32_t r[16];
       tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0, r);
       tc::tmem_ld_wait();
@@ -209,6 +226,10 @@ HK_API int hk_tc05_selftest(const void* a_f16, const void* b_f16, float* d, int 
   HK_REQUIRE(a_f16 && b_f16 && d && status);
   HK_REQUIRE((M == 64 || M == 128) && N >= 16 && N <= 256 && N % 16 == 0 && K >= 16 && K <= 128 &&
              K % 16 == 0);
+  if (b_layout & 0x1800) {   // weight-stationary: M = 64 only; A in tensor memory is given as [64][K]
+    HK_REQUIRE(M == 64 && (N == 64 || N == 128 || N == 256));
+    HK_REQUIRE(!(b_layout & 0x1000) || (K % 64 == 0 && !(b_layout & 2) && aligned(a_f16, 4)));
+  }
   const size_t smem = 128 * 128 * 2 + 256 * 128 * 2;
   static bool attr_set[64] = {false};
   int dev = 0;

@@ -36,6 +36,22 @@ def test_tc05_gemm_matches_fp32_matmul(M, N, K, b_layout):
     assert torch.allclose(got, want, atol=2e-2, rtol=1e-3), float((got - want).abs().max())
 
 
+@pytest.mark.parametrize("N,K,b_layout", [(64, 128, 0x80c), (64, 64, 0x808), (128, 128, 0x80c), (256, 64, 0x80d), (256, 16, 0x80d),
+                                          (64, 128, 0x1008), (64, 64, 0x1008), (128, 64, 0x1008), (256, 128, 0x1008)])
+def test_weight_stationary_products_match_fp32_matmul(N, K, b_layout):
+    """the forms the attention kernel rests on: scores (A and B K-major, A from shared or from tensor memory) and values (B
+    MN-major, N = 256).  Columns below N / 2 sit in lanes 0-63, the others in lanes 64-127"""
+    g = torch.Generator(device="cpu").manual_seed(N + K + b_layout)
+    a, b = torch.randn(64, K, generator=g).half(), torch.randn(N, K, generator=g).half()
+    b_in = b if (b_layout & 1) == 0 else b.t().contiguous()
+    d, status = hk.tc05_selftest(a.cuda(), b_in.cuda(), 64, N, K, b_layout)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    d = d.cpu()
+    got, want = torch.cat([d[:64, :N // 2], d[64:, :N // 2]], dim=1), a.float() @ b.float().t()
+    assert torch.allclose(got, want, atol=2e-2, rtol=1e-3), float((got - want).abs().max())
+
+
 def test_reference_parity_binary_against_this_library():
     """The reference's own kernel parity test (src/cuda/attn/test/test_attn_parity.cpp), compiled
     from the reference tree and linked against libhelios_b200.so through the helios::attn shim."""
