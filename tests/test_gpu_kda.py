@@ -275,7 +275,7 @@ def test_chunked_fused_launch_equals_two_kernel_form(T, H, bsz):
         assert max_rel(res[1][1], o_32) < 2e-3 and frob_rel(res[1][2], o_st) < 1e-2
 
 
-@pytest.mark.parametrize("H,bsz", [(32, 1), (4, 2), (64, 3)])
+@pytest.mark.parametrize("H,bsz", [(32, 1), (4, 2), (64, 3), (64, 5)])
 def test_decode_step_with_conv_inside_equals_the_two_launch_sequence(H, bsz):
     """hk_kda_decode_step (conv + recurrence of one decoded token in one launch, value slices of a head as a cluster)
     against cuda_causal_conv1d_update followed by cuda_recurrent_gated_delta_rule on the same buffers, 6 tokens in a
@@ -479,3 +479,87 @@ def test_decode_steps_share_nothing(H):
     for job in jobs[1:]:
         assert all(torch.equal(a, b) for a, b in zip(job[2:], jobs[0][2:]))
     assert (junk == 3).all()
+
+
+@pytest.mark.parametrize("H,bsz", [(4, 2), (64, 5)])
+def test_decode_layer_vs_oracle(H, bsz):
+    """one token through the whole layer, a head per CTA (8 heads) and streamed (320, ragged last round), each stage from the
+    stage before it: window and convolution, recurrence and state from the oracle; gates and norm in 64 bits"""
+    D, dim = 128, 3 * H * 128
+    r = synth.rng(40 + H)
+    x32 = r.standard_normal((bsz, dim), dtype=np.float32)
+    raw = synth.kda_raw_gates(bsz, H, D, seed=9)
+    f, b = raw["f"].reshape(bsz, H, D), raw["b"].reshape(bsz, H)
+    w = synth.f32_to_bf16_bits((0.1 * r.standard_normal((dim, 4))).astype(np.float32))
+    cst0 = synth.f32_to_bf16_bits(r.standard_normal((bsz, dim, 4), dtype=np.float32))
+    s0 = (0.1 * r.standard_normal((bsz, 1, H, D, D), dtype=np.float32)).astype(np.float32)
+    nw, go = (1.0 + 0.1 * r.standard_normal(D)).astype(np.float32), r.standard_normal((bsz * H, D), dtype=np.float32)
+    cs, st = dev_bf16(cst0), dev(s0)
+    out, o32 = (torch.empty(bsz, H, D, dtype=d, device="cuda") for d in (torch.bfloat16, torch.float32))
+    y = torch.empty(bsz * H, D, dtype=torch.float32, device="cuda")
+    hk.kda_decode_layer(dev(x32), cs, dev_bf16(w), None, dev(f), dev(b), dev(raw["dt_bias"]), dev(raw["a_log"]), raw["lower_bound"], st, out,
+                        dev(nw), dev(go), y, bsz, H, epsilon=1e-6, gate_act=1, out_f32=o32)
+    torch.cuda.synchronize()
+    assert hk.read_device_status() == 0
+    x16 = synth.f32_to_bf16_bits(x32).reshape(bsz, dim, 1)
+    qkv, o_cs = orc.conv1d_update(x16, cst0, w, None, bsz, dim, 1, 4, 4)
+    assert np.array_equal(bits(cs).reshape(-1), o_cs.reshape(-1)), "rolling window"
+    sig = lambda v: 1.0 / (1.0 + np.exp(-v.astype(np.float64)))
+    g = (raw["lower_bound"] * sig(np.exp(raw["a_log"].astype(np.float64)).reshape(H, 1) * (f + raw["dt_bias"].reshape(H, D)))).astype(np.float32)
+    beta = synth.f32_to_bf16_bits(sig(b).astype(np.float32))
+    _, want, o_st = orc.kda_recurrent(qkv.reshape(bsz, 1, dim), g.reshape(bsz, 1, H, D), beta.reshape(bsz, 1, H), s0, bsz, 1, H, H, D, D)
+    # the fast exponential may flip the last bit (2^-8) of a few of the convolution's and beta's bf16 values: 2e-3 as above
+    assert max_rel(o32.cpu().numpy().reshape(want.shape), want) < 2e-3 and frob_rel(st.cpu().numpy(), o_st) < 2e-3
+    assert np.array_equal(bits(out), (o32.cpu().numpy().view(np.uint32) >> 16).astype(np.uint16)), "rounded toward zero"
+    o = synth.bf16_bits_to_f32(bits(out)).reshape(bsz * H, D).astype(np.float64)
+    y64 = o * nw / np.sqrt((o * o).mean(axis=1, keepdims=True) + 1e-6) * sig(go)
+    assert max_rel(y.cpu().numpy(), y64) < 1e-5
+
+
+@pytest.mark.parametrize("H,bsz", [(4, 1), (40, 2), (64, 5)])
+def test_states_off_the_16_byte_boundary(H, bsz):
+    """a state that starts on any fp32 element: the scalar forms (decode step and layer; 1, 3 and 9 tokens of the recurrence; no
+    streaming) against the same call on an aligned copy, bit for bit"""
+    D, dim, T = 128, 3 * H * 128, 9
+    gen = torch.Generator(device="cuda").manual_seed(H)
+
+    def rnd(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+    n = bsz * H * D * D
+    buf, qkv, g = 0.1 * rnd(n + 1), rnd(bsz, T, dim).to(torch.bfloat16), -torch.rand(bsz, T, H, D, generator=gen, device="cuda")
+    beta, cs0, w = torch.sigmoid(rnd(bsz, T, H)).to(torch.bfloat16), rnd(bsz, dim, 4).to(torch.bfloat16), (0.1 * rnd(dim, 4)).to(torch.bfloat16)
+    x32, nw, go, a_log, dtb = rnd(bsz, dim), 1.0 + 0.1 * rnd(D), rnd(bsz * H, D), rnd(H) * 0.3, rnd(H, D)
+
+    def run(st):
+        res = []
+        for t in (1, 3, 9):
+            out = torch.empty(bsz, t, H, D, dtype=torch.bfloat16, device="cuda")
+            hk.cuda_recurrent_gated_delta_rule(qkv[:, :t].contiguous(), g[:, :t].contiguous(), beta[:, :t].contiguous(), st, out, bsz, t, H, H,
+                                               D, D, 1, None, True, False)
+            res.append(out)
+        cs, out, y = cs0.clone(), torch.empty(2, bsz, H, D, dtype=torch.bfloat16, device="cuda"), torch.empty(bsz * H, D, device="cuda")
+        hk.kda_decode_step(qkv[:, 0].contiguous(), cs, w, None, g[:, 0].contiguous(), beta[:, 0].contiguous(), st, out[0], bsz, H)
+        hk.kda_decode_layer(x32, cs, w, None, g[:, 1].contiguous(), rnd(bsz, H) * 0, dtb, a_log, -5.0, st, out[1], nw, go, y, bsz, H)
+        torch.cuda.synchronize()
+        return res + [cs, out, y, st.clone()]
+    aligned, off = buf[1:].clone(), buf[1:]
+    assert aligned.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 4
+    for a, b in zip(run(aligned), run(off)):
+        assert torch.equal(a, b)
+
+
+def test_an_explicit_stream_is_the_one_that_runs():
+    """the binding's stream argument: a call given a side stream waits for that stream's earlier work, not for the current one's"""
+    S, F = 64, 256
+    src, dst, side = torch.zeros(S, F, device="cuda"), torch.zeros(F, S, dtype=torch.bfloat16, device="cuda"), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)                          # about 10 ms
+        src.fill_(3.0)
+    hk.kda_transpose_cast(dst, src, S, F, stream=side)
+    side.synchronize()
+    assert (dst == 3.0).all()
+    with pytest.raises(AttributeError):
+        hk.kda_transpose_cast(dst, src, S, F, stream=1)
+    with pytest.raises(TypeError):
+        hk.gated_rms_norm(dst, src.int(), src, src, S, F, 1e-6)
