@@ -273,7 +273,7 @@ __global__ __launch_bounds__(FIXED ? FIXED : TKR_MAX_THREADS, FIXED == 256 ? 4 :
   for (int i = t; i < 2048; i += threads) hist[i] = 0;
   if (t < 32) low[t] = 0;
   if (t == 0) sel[0] = -1;
-  pdl_release(gridDim.x <= 16);
+  pdl_release();
   pdl_wait();
   const TopkSink sink{out + (size_t)blockIdx.x * k_pad,
                       raw ? reinterpret_cast<int4*>(raw + (size_t)blockIdx.x * (4 * k_pad + 4)) : nullptr, raw ? q_pos[blockIdx.x] : 0};
@@ -382,7 +382,7 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
     const uint16_t* scores, int* __restrict__ out, int T, int s_stride, int k, int k_pad,
     int* __restrict__ raw, const int* __restrict__ q_pos) {
   namespace cg = cooperative_groups;
-  pdl_release();                                           // at most 16 rows
+  pdl_release();
   pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int c = (int)cluster.block_rank();

@@ -55,17 +55,17 @@ inline int sm_count() {
 // kernel may have written or may still read: the launch itself is over when the kernel before them ends.  EVERY kernel
 // launched this way executes pdl_wait() in every CTA: the wait covers the grid before it only, and the chain of waits is what
 // orders a kernel behind all earlier ones.
-// Small grids (up to a few CTAs per SM: the one-token prologue and its row kernels, top-k of few rows, the merge of few rows'
-// partials) release their dependents at entry (pdl_release): the next kernel's CTAs are placed, set up their barriers and
-// tensor memory and ask for their weights in L2 while the small one runs (MLA layer of one token 34.7 -> 33.4 us, selection +
-// attention 25.0 -> 24.6, 45-layer decode at 262,144 589 -> 574).  Ahead of its wait a kernel may do no more than that: it may
-// not load or store anything.  Other grids do not: CTAs placed beside a running grid land where it left room, not evenly -
-// the per-token KDA kernel behind the convolution took twice as long, scorer and attention releasing theirs cost the decode
-// chains what the others gain, and KDA decode layers behind one another took 4.2 us instead of 3.9.
+// The small kernels of a chain (one-token prologue, cache append, layer norm, pooled keys, top-k, the merge of partials) release
+// their dependents at entry (pdl_release), whatever their grid: the next kernel's CTAs are placed, set up their barriers and tensor
+// memory and ask for their weights in L2 while the small one runs.  Ahead of its wait a kernel may do no more than that: it may
+// not load or store anything.  MLA layer at 5,001 tokens in a graph, nothing released -> released: 1 token 35.0 -> 32.3 us, 8
+// 49.7 -> 44.4, 32 65.0 -> 60.5, 256 129.5 -> 126.7; 45-layer decode at 262,144 618 -> 572 (with limits of 16 to 32 CTAs on some
+// of them, 9 to 256 tokens took 1.1-1.9 us more).
+// The other kernels do not: CTAs placed beside a running grid land where it left room, not evenly - the per-token KDA kernel
+// behind the convolution took twice as long, scorer and attention releasing theirs cost the decode chains what the others gain, and
+// KDA decode layers behind one another took 4.2 us instead of 3.9.
 // Launches of many waves are plain: as programmatic dependents the convolution of 32K tokens took 495 us instead of 362.
-__device__ __forceinline__ void pdl_release(bool small_grid = true) {
-  if (small_grid) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // cluster: CTAs of a thread-block cluster along x

@@ -11,7 +11,7 @@ __global__ __launch_bounds__(128) void kpool_write_kernel(
     const __half* __restrict__ ik, const __half* __restrict__ ig, __half* __restrict__ ring,
     int raw_rows, __half* __restrict__ pk_nt, const float* __restrict__ ape, int pos_start,
     int n_new, int first_pool) {
-  pdl_release(gridDim.x <= 32);
+  pdl_release();
   pdl_wait();
   kpool_one(ik, ig, ring, raw_rows, pk_nt, ape, pos_start, n_new, first_pool + blockIdx.x, threadIdx.x, [] {});
 }

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) mla_cache_append_kernel(const float* __re
                                                                const __half* __restrict__ ln_w,
                                                                __half* __restrict__ ckv, __half* __restrict__ ckv_new,
                                                                long long pos, int n, float eps) {
-  pdl_release(gridDim.x <= 32);
+  pdl_release();
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -131,7 +131,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256) layernorm_f16_kernel(const __half* x, const __half* __restrict__ w,   // x and y may alias
                                                             const __half* __restrict__ b, __half* y,
                                                             int rows, int dim, float eps) {
-  pdl_release(gridDim.x <= 32);
+  pdl_release();
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;

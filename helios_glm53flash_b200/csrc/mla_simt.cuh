@@ -241,7 +241,7 @@ __global__ __launch_bounds__(128 * GROUPS) void lse_combine_kernel(
     const float* __restrict__ part_acc, const float* const* __restrict__ ptrs_m,
     const float* const* __restrict__ ptrs_l, const float* const* __restrict__ ptrs_acc,
     int n_split, int64_t rows, __half* __restrict__ out) {
-  pdl_release(gridDim.x * gridDim.y <= 512);
+  pdl_release();
   pdl_wait();
   const int64_t r = blockIdx.x;
   float gm, gl;
@@ -266,7 +266,7 @@ template <int GROUPS>
 __global__ __launch_bounds__(32 * GROUPS) void lse_combine_cs_kernel(
     const float* __restrict__ part_m, const float* __restrict__ part_l, const float* __restrict__ part_acc,
     int n_split, int64_t rows, __half* __restrict__ out) {
-  pdl_release(gridDim.x * gridDim.y <= 512);
+  pdl_release();
   pdl_wait();
   constexpr int LANES = 128 / LSE_CSPLIT;
   const int64_t r = blockIdx.x;
