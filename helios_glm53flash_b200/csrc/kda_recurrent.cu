@@ -5,7 +5,7 @@
 // Kernels:
 //   kda_decode_kernel, kda_decode_stream_kernel   one token per sequence (the decode step, the decode layer, the recurrence alone)
 //   kda_recurrent_cols_kernel                     several tokens, channelwise decay, no history
-//   kda_recurrent_rows_kernel                     channelwise decay with a history, and two to six tokens of many chains
+//   kda_recurrent_rows_kernel                     channelwise decay with a history, and a few tokens of many chains
 //   kda_recurrent_kernel                          one decay per head, 128- and 64-wide heads
 // The state lives in REGISTERS for the whole call (the reference re-reads and re-writes it from global memory on every token),
 // so a call moves each state byte once in and once out, the HBM floor of 2*H*D*D*4 bytes.
@@ -36,7 +36,7 @@ __device__ __forceinline__ float inv_norm(const float (&x)[4]) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Channelwise decay, 128-wide heads: history mode, states with room for one, and two to six tokens of many chains.  One CTA per
+// Channelwise decay, 128-wide heads: history mode, states with room for one, and a few tokens of many chains.  One CTA per
 // (batch item, head, slice of NV value-columns); thread (kg, j) owns column j and the 16 / KG row groups of the shared order that
 // make up kg's part of the balanced tree.  Three warps prepare a token (q with its norm; k with its norm; the decay).
 // What bounds it: for few tokens the state in and out, in runs of 128 bytes; for many the three barriers of a token.  With the
@@ -305,7 +305,9 @@ __device__ __forceinline__ uint2 conv4_rolled(uint2 st, __nv_bfloat16 cur) {
 //     three barriers);
 //   many heads (more than 2 per SM): persistent, one CTA per SM, heads stream through shared memory as 64 KB bulk copies: two
 //     stages inwards, each asked for again as soon as its head sits in registers, and one outwards (stores straight from
-//     registers held the SM to 26 B per cycle: 49 us for 1,536 heads); the token of the next head is prepared meanwhile.
+//     registers held the SM to 26 B per cycle); the token of the next head is prepared meanwhile.  Layer, a head per CTA / streamed,
+//     us: 144 heads 6.2 / 6.7, 200 9.8 / 9.4, 296 11.1 / 10.9, 320 13.8 / 12.6, 1,536 50.3 / 39.1; recurrence alone 200 heads 8.7 /
+//     9.2, 296 9.9 / 10.0, 320 12.0 / 11.5.
 // ---------------------------------------------------------------------------------------------
 struct DecodeArgs {
   const void* x;                        // LAYER: fp32 projection row [dim], else bf16 [dim]
@@ -518,9 +520,10 @@ __device__ __forceinline__ float* head_state(const DecodeArgs& a, int bh) {
 }
 
 // VEC: the state is 16-byte aligned.
-// SLICES = 4: a CTA owns 32 of the head's 128 columns (two state warps, a quarter warp per row group, the same sums in the
+// SLICES = 4, up to half a head per SM: a CTA owns 32 of the head's 128 columns (two state warps, a quarter warp per row group, the same sums in the
 // same order).  One SM moves a head's 64 KB in and out in 0.6 us each, and a few heads leave the other SMs idle: one token's
-// recurrence alone 2.7 us at 32 heads.  Not for DEC_LAYER, whose norm needs all columns of a head.  In DEC_STEP the
+// recurrence alone, whole / split: 32 heads 3.7 / 2.7 us, 74 4.2 / 3.5, 112 5.1 / 5.2; the step 32 heads 3.9 / 3.2, 64 4.4 / 4.1, 80
+// 4.8 / 4.9.  Not for DEC_LAYER, whose norm needs all columns of a head.  In DEC_STEP the
 // four are a cluster: the windows are read by every slice and rolled by the first behind a cluster barrier that all have arrived at
 // long before (32 heads 3.0 us per step; counting the slices through a word of global memory per head 3.13, at 8 heads 2.53 and
 // 2.85, and calls on several streams needed counters of their own).
@@ -991,9 +994,12 @@ HK_API int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* b
       a.slots = slots;
       return launch_decode<DEC_REC>(a, s);
     }
-    // Two or three tokens of many chains (up to six of a thousand) are mostly the state in and out, which the older kernel moves
-    // in longer runs: 2 tokens of 32 chains 3.5 us against 4.7, of 1,536 chains 44 against 72; 4 of 256 chains 16.1 against 15.7.
-    if (!(chains >= 32 && seqlen <= (chains >= 1024 ? 6 : 3))) {
+    // A few tokens of many chains are mostly the state in and out, which the rows kernel moves in longer runs; more tokens are the
+    // chain from token to token, which is the columns kernel's.  Rows against columns, us: 8 chains 2 tokens 3.1 / 3.1; 16 chains 3
+    // tokens 3.4 / 4.2, 4 tokens 4.2 / 4.1; 64 chains 5.3 / 5.7, 6.1 / 5.9; 256 chains 6 tokens 18.2 / 18.2, 8 tokens 22.0 / 19.8;
+    // 512 chains 12 tokens 46.8 / 46.9, 16 tokens 58.8 / 55.0; 1,536 chains 16 tokens 152 / 158, 24 tokens 220 / 210.
+    const int rows_up_to = chains >= 1024 ? 16 : (chains >= 384 ? 12 : (chains >= 128 ? 6 : (chains >= 16 ? 3 : 1)));
+    if (seqlen > rows_up_to) {
       const int cpl = !aligned(state, 16) || chains < 32 ? 1 : (chains < 64 ? 2 : 4);
       auto kern = cpl == 4 ? kda_recurrent_cols_kernel<4> : (cpl == 2 ? kda_recurrent_cols_kernel<2> : kda_recurrent_cols_kernel<1>);
       return pdl_launch(kern, dim3(bsz, num_v_heads, 16 / cpl), dim3(RC_WARPS * 32), 0, s, q, g, bt, state, o, out_f32, seqlen, num_k_heads,

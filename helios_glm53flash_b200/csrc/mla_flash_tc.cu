@@ -60,10 +60,7 @@ constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_THRESHOLD = 8.0f;         // log2 units: P stays below 2^8, fine for fp16
 // warps 0-3 softmax, Q into tensor memory and epilogue (a TMEM lane quarter each), 4 issues S = Q K^T, 5 issues O += P V, the
 // others load tiles (dense ranges need more than one only for the ragged last tile).
-template <bool G4>
-struct FtRoles {
-  static constexpr int LOAD_WARPS = 4, THREADS = (6 + LOAD_WARPS) * 32, SLOTS = FT_KEYS / LOAD_WARPS;   // key slots per loader warp
-};
+constexpr int FT_LOAD_WARPS = 4, FT_THREADS = (6 + FT_LOAD_WARPS) * 32, FT_SLOTS = FT_KEYS / FT_LOAD_WARPS;   // key slots per loader warp
 
 struct FtMisc {
   uint64_t full[FT_NBUF], free[FT_NBUF];          // ring slot (a key tile or a row's Q): landed, may be overwritten
@@ -136,10 +133,9 @@ __device__ __forceinline__ void tma_gather4_rows(uint32_t leader, uint32_t smem_
 // G4: gathered rows (raw_idx); otherwise dense ranges.  tmap_box: 3-D map of the cache, tmap_rows: 2-D map of the cache for
 // gather4, tmap_q: the queries as tmap_box, tmap_o: 2-D map of the final output.
 template <bool G4>
-__global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(
+__global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
     MlaArgs a, int* __restrict__ status, const __grid_constant__ CUtensorMap tmap_box, const __grid_constant__ CUtensorMap tmap_rows,
     const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_o) {
-  using R = FtRoles<G4>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   FtMisc& ms = *reinterpret_cast<FtMisc*>(smem + FS_MISC);
@@ -155,7 +151,7 @@ __global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(
   if (tid == 0) {
 #pragma unroll
     for (int b = 0; b < FT_NBUF; b++) {
-      tc::mbar_init(&ms.full[b], R::LOAD_WARPS);
+      tc::mbar_init(&ms.full[b], FT_LOAD_WARPS);
       tc::mbar_init(&ms.free[b], 1);
     }
 #pragma unroll
@@ -186,8 +182,8 @@ __global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(
     const uint32_t leader = tc::elect_one();
     // cache row of key slot lw * SLOTS + lane of a tile, -1 = hole; volatile, so that a look-ahead load is issued where it stands
     auto row_of = [&](const FtItem& it, int tile) -> int {
-      const int p = it.k0 + tile * FT_KEYS + lw * R::SLOTS + lane;
-      if (lane >= R::SLOTS || p >= it.k1) return -1;
+      const int p = it.k0 + tile * FT_KEYS + lw * FT_SLOTS + lane;
+      if (lane >= FT_SLOTS || p >= it.k1) return -1;
       if (!G4) return (int)(it.base + p);
       int v;
       asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(a.raw_idx + (size_t)it.r * a.kidx + p));
@@ -244,7 +240,7 @@ __global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(
         }
         const uint32_t valid = __ballot_sync(0xffffffffu, row >= 0);
         const int b = next_slot();
-        if (lane < R::SLOTS / 8) ms.mask[b][lw * (R::SLOTS / 8) + lane] = (uint8_t)(valid >> (8 * lane));
+        if (lane < FT_SLOTS / 8) ms.mask[b][lw * (FT_SLOTS / 8) + lane] = (uint8_t)(valid >> (8 * lane));
         __syncwarp();
         if (!G4 && it.keys(tile) == FT_KEYS) {             // a whole tile of a dense range: one box
           if (lane == 0) {
@@ -256,11 +252,11 @@ __global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(
             }
           }
         } else {
-          if (lane == 0) tc::mbar_arrive_expect_tx(&ms.full[b], R::SLOTS * LATENT * 2);
+          if (lane == 0) tc::mbar_arrive_expect_tx(&ms.full[b], FT_SLOTS * LATENT * 2);
           __syncwarp();
-          const uint32_t dst = tc::smem_u32(smem + FS_K) + b * FT_TILE + lw * R::SLOTS * 128, bar = tc::smem_u32(&ms.full[b]);
+          const uint32_t dst = tc::smem_u32(smem + FS_K) + b * FT_TILE + lw * FT_SLOTS * 128, bar = tc::smem_u32(&ms.full[b]);
 #pragma unroll
-          for (int j = 0; j < R::SLOTS / 4; j++) {
+          for (int j = 0; j < FT_SLOTS / 4; j++) {
             const int r0 = __shfl_sync(0xffffffffu, row, 4 * j), r1 = __shfl_sync(0xffffffffu, row, 4 * j + 1);
             const int r2 = __shfl_sync(0xffffffffu, row, 4 * j + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * j + 3);
 #pragma unroll
@@ -559,7 +555,9 @@ __global__ __launch_bounds__(FtRoles<G4>::THREADS, 1) void mla_flash_tc_kernel(
 }
 
 int mla_flash_tc_auto_splits(int m, int n_keys) {
-  // at most one CTA per SM (a second wave would double the time), at least two tiles per split, splits of equal tile counts
+  // At most one CTA per SM (a second wave would double the time), at least two tiles per split, splits of equal tile counts.  With
+  // the merge, 1 / 2 / 3 tiles per split, us: 2,052 gathered rows of one query 12.1 / 11.3 / 12.7, of four 16.9 / 12.6 / 13.5 (more
+  // partials to write and merge); dense, one row over 2,048 keys 11.8 / 11.2 / 12.7, over 8,192 15.4 / 13.6 / 14.9.
   const int sms = sm_count();
   const int tiles = (n_keys + FT_KEYS - 1) / FT_KEYS;
   int want = sms / (m > 0 ? m : 1);
@@ -640,8 +638,8 @@ int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s) {
   const int64_t items = (int64_t)a.n_split * a.m;
   const dim3 grid((unsigned)(a.raw_idx && a.out && items > sm_count() ? sm_count() : items));
   const cudaError_t e =
-      a.raw_idx ? pdl_launch(mla_flash_tc_kernel<true>, grid, dim3(FtRoles<true>::THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap)
-                : pdl_launch(mla_flash_tc_kernel<false>, grid, dim3(FtRoles<false>::THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap);
+      a.raw_idx ? pdl_launch(mla_flash_tc_kernel<true>, grid, dim3(FT_THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap)
+                : pdl_launch(mla_flash_tc_kernel<false>, grid, dim3(FT_THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap);
   return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 
