@@ -6,10 +6,13 @@
 // row holds fewer than k selectable entries all of them are emitted; the rest of the k_pad-wide
 // output row is -1.  Integer work: results are bit-exact by construction.
 //
-// One CTA of 1024 threads per row, three sweeps of the row (the reference makes four: two
-// histogram sweeps and two compaction sweeps).  Sweep 1 histograms the top 11 key bits, sweep 2 the
-// low 5 bits inside the crossing bucket, sweep 3 is a single ordered compaction that places the
-// "above" entries and the tie entries at once (their final offsets are known after sweep 2).
+// Radix select: a histogram of the top 11 key bits, one of the low 5 bits inside the crossing bucket, then a single ordered
+// compaction that places the "above" entries and the tie entries at once (the reference makes two histogram sweeps and two
+// compaction sweeps of global memory).  Three kernels:
+//   dsa_topk_rows_kernel      rows of up to 16,384 scores, read once into registers, a small CTA each
+//   dsa_topk_cluster_kernel   at most 16 longer rows of up to 262,143 scores, read once into the registers of a cluster of 8 CTAs
+//   dsa_topk_kernel           every other call (many long rows, lengths known on the device only): one CTA of 1,024 threads per
+//                             row, which sweeps the row three times; topk_row also selects among candidates in shared memory
 #include <cooperative_groups.h>
 
 #include "hk_common.cuh"
@@ -224,17 +227,6 @@ __global__ __launch_bounds__(TK_THREADS) void dsa_topk_kernel(
   topk_row(scores + (size_t)blockIdx.x * s_stride, sink, T, k, k_pad);
 }
 
-
-// ------------------------------------------------------------------------------------------------
-// A few long rows (the decode case is ONE row): a thread-block cluster of 8 CTAs works on a row, CTA c on pieces
-// [1024 NP c, 1024 NP (c + 1)), every thread on NP consecutive pieces of 8 elements that stay in registers, so the row is
-// read from global memory once and no sweep is longer than 8 NP keys per thread.  The CTAs meet through distributed shared
-// memory: the bucket histograms are summed slice-wise and the sums stored into every CTA, each CTA then finds the crossing
-// bucket itself; the low-bit count sets are read by every CTA, which finds the threshold and, from the per-CTA counts, the
-// offset of its own ordered output - four cluster barriers in all, no hand-back round trips.
-// NP = 1, 2, 4 cover rows of 65,535, 131,071 and 262,143 scores at any alignment (1M tokens of context).  One row of 65,540
-// scores (262,160 tokens) took 33.9 us in the one-CTA kernel and takes 9.3 us here.
-// ------------------------------------------------------------------------------------------------
 // ------------------------------------------------------------------------------------------------
 // Rows of up to 16,384 scores, a CTA of 256 to 512 threads each: the row is read once, every thread keeps NP <= 4
 // consecutive pieces (8 NP keys) in registers; histogram, threshold and compaction work from there.  What bounds the
@@ -373,6 +365,16 @@ __device__ long long hk_topk_trace[16];
 #else
 #define TK_TRACE(slot) do { } while (0)
 #endif
+// ------------------------------------------------------------------------------------------------
+// A few long rows (the decode case is ONE row): a thread-block cluster of 8 CTAs works on a row, CTA c on pieces
+// [1024 NP c, 1024 NP (c + 1)), every thread on NP consecutive pieces of 8 elements that stay in registers, so the row is
+// read from global memory once and no sweep is longer than 8 NP keys per thread.  The CTAs meet through distributed shared
+// memory: the bucket histograms are summed slice-wise and the sums stored into every CTA, each CTA then finds the crossing
+// bucket itself; the low-bit count sets are read by every CTA, which finds the threshold and, from the per-CTA counts, the
+// offset of its own ordered output - four cluster barriers in all, no hand-back round trips.
+// NP = 1, 2, 4 cover rows of 65,535, 131,071 and 262,143 scores at any alignment (1M tokens of context).  One row of 65,540
+// scores (262,160 tokens) took 33.9 us in the one-CTA kernel and takes 9.3 us here.
+// ------------------------------------------------------------------------------------------------
 constexpr int TKC_CTAS = 8;
 constexpr int TKC_PIECES = TKC_CTAS * TK_THREADS;         // pieces of 8 elements that NP = 1 holds
 constexpr int TKC_MAX_NP = 4;
@@ -546,28 +548,36 @@ namespace hk {
 static int topk_launch(const void* scores, int s_stride, int* indices, int R, int T, int k, int k_pad, const int* t_ptr,
                        int t_seq, int* raw, const int* q_pos, cudaStream_t s) {
   const uint16_t* sc = (const uint16_t*)scores;
-  cudaError_t e;
   // pieces of the longest-reaching row: rows of a stride that is no multiple of 8 start at any offset
   const int lead = R == 1 || s_stride % 8 == 0 ? (int)(((uintptr_t)scores & 15) >> 1) : 7;
   const int64_t pieces = ((int64_t)T + lead + 7) / 8;
-  if (T > 16384 && pieces <= (int64_t)TKC_PIECES * TKC_MAX_NP && R <= 16 && !t_ptr) {
-    // a few long rows (decode): one 8-CTA cluster per row.  With many rows (prefill) the clusters queue for
-    // eight free SMs of one GPC each and the one-CTA kernel below is 3 to 20 times faster (measured at
-    // 64 to 4,096 rows); up to 16,384 scores one CTA is as fast as the cluster even for a single row.
-    auto kern = pieces <= TKC_PIECES ? dsa_topk_cluster_kernel<1>
-                                     : (pieces <= 2 * TKC_PIECES ? dsa_topk_cluster_kernel<2> : dsa_topk_cluster_kernel<4>);
-    e = pdl_launch(kern, dim3(R * TKC_CTAS), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
-  } else if (pieces <= TKR_MAX_PIECES && !t_ptr) {
-    const bool few = R <= sm_count();
-    auto kern = pieces <= 256    ? dsa_topk_rows_kernel<1, 256>
-                : few            ? (pieces <= 512 ? dsa_topk_rows_kernel<1, 512> : pieces <= 1024 ? dsa_topk_rows_kernel<1, 1024> : dsa_topk_rows_kernel<2, 1024>)
-                : pieces <= 512  ? dsa_topk_rows_kernel<2, 256>
-                : pieces <= 1024 ? dsa_topk_rows_kernel<4, 256> : dsa_topk_rows_kernel<4, 0>;
-    const int threads = pieces <= 256 ? 256 : few ? (pieces <= 512 ? 512 : 1024) : pieces <= 1024 ? 256 : (int)((pieces + 127) / 128) * 32;
-    e = pdl_launch(kern, dim3(R), dim3(threads), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
-  } else {
-    e = pdl_launch(dsa_topk_kernel, dim3(R), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, t_ptr, t_seq, raw, q_pos);
-  }
+  auto rows = [&](auto kern, int threads) {
+    return pdl_launch(kern, dim3(R), dim3(threads), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
+  };
+  auto cluster = [&](auto kern) {
+    return pdl_launch(kern, dim3(R * TKC_CTAS), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
+  };
+  auto sweeps = [&]() {
+    return pdl_launch(dsa_topk_kernel, dim3(R), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, t_ptr, t_seq, raw, q_pos);
+  };
+  // (figures at the kernels.  With many rows the clusters queue for eight free SMs of one GPC each and the one-CTA kernel is 3 to 20
+  // times faster, measured at 64 to 4,096 rows; up to 16,384 scores one CTA is as fast as the cluster even for a single row)
+  cudaError_t e;
+  if (t_ptr) e = sweeps();
+  else if (pieces <= 256) e = rows(dsa_topk_rows_kernel<1, 256>, 256);
+  else if (pieces <= TKR_MAX_PIECES && R <= sm_count())      // a row per SM: as many threads as there are pieces, up to 1,024
+    e = pieces <= 512    ? rows(dsa_topk_rows_kernel<1, 512>, 512)
+        : pieces <= 1024 ? rows(dsa_topk_rows_kernel<1, 1024>, 1024)
+                         : rows(dsa_topk_rows_kernel<2, 1024>, 1024);
+  else if (pieces <= TKR_MAX_PIECES)                         // rows share SMs: small CTAs of up to four pieces per thread
+    e = pieces <= 512    ? rows(dsa_topk_rows_kernel<2, 256>, 256)
+        : pieces <= 1024 ? rows(dsa_topk_rows_kernel<4, 256>, 256)
+                         : rows(dsa_topk_rows_kernel<4, 0>, (int)((pieces + 127) / 128) * 32);
+  else if (R <= 16 && T > 16384 && pieces <= (int64_t)TKC_PIECES * TKC_MAX_NP)
+    e = pieces <= TKC_PIECES       ? cluster(dsa_topk_cluster_kernel<1>)
+        : pieces <= 2 * TKC_PIECES ? cluster(dsa_topk_cluster_kernel<2>)
+                                   : cluster(dsa_topk_cluster_kernel<4>);
+  else e = sweeps();
   return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 }  // namespace hk
@@ -586,7 +596,7 @@ HK_API int hk_dsa_topk_expand(const void* scores, int s_stride, int* indices, in
   using namespace hk;
   HK_REQUIRE(scores && indices && raw_idx && q_pos && R >= 0 && T >= 0 && k >= 0 && k <= 512 && s_stride >= 0);
   HK_REQUIRE(aligned(raw_idx, 16));
-  (void)after_scorer;   // every selection kernel is launched as a programmatic dependent now
+  (void)after_scorer;   // every selection kernel is launched as a programmatic dependent
   if (R == 0) return HK_OK;
   return topk_launch(scores, s_stride, indices, R, T, k, 512, nullptr, 0, raw_idx, q_pos, as_stream(stream));
 }

@@ -282,8 +282,9 @@ HK_API int hk_kda_transpose_cast(void* dst_bf16, const float* src, int S, int F,
   const int s_tiles = (S - 1) / (longer ? 128 : 64) + 1;
   HK_REQUIRE(s_tiles <= 65535);
   HK_REQUIRE(hk::aligned(dst_bf16, 4));
-  return hk::pdl_launch(longer ? hk::transpose_cast_kernel<true, true> : odd ? hk::transpose_cast_kernel<false, true> : hk::transpose_cast_kernel<false, false>, dim3((F - 1) / (longer ? 32 : 64) + 1, s_tiles),
-                        dim3(256), 0, hk::as_stream(stream), src, static_cast<__nv_bfloat16*>(dst_bf16), S, F) == cudaSuccess
+  auto kern = longer ? hk::transpose_cast_kernel<true, true> : odd ? hk::transpose_cast_kernel<false, true> : hk::transpose_cast_kernel<false, false>;
+  return hk::pdl_launch(kern, dim3((F - 1) / (longer ? 32 : 64) + 1, s_tiles), dim3(256), 0, hk::as_stream(stream), src,
+                        static_cast<__nv_bfloat16*>(dst_bf16), S, F) == cudaSuccess
              ? HK_OK
              : HK_ERR_CUDA;
 }
