@@ -13,13 +13,15 @@ Call order per chunk of n rows at position pos:
   KDA layer   cast + short conv (fp32 projection rows -> bf16 q|k|v)     hk_kda_cast_conv
               gated chunked prefill (gate preparation inside)            hk_kda_chunked_prefill_gated
               gated RMS norm                                              hk_gated_rms_norm
-  (n == 1)    conv + recurrence in one launch, then the norm             hk_kda_decode_step
+  (n == 1)    the whole KDA layer in one launch                          hk_kda_decode_layer
   MLA layer   RMS norm + append to the latent cache                      hk_mla_cache_append
               indexer key layer norm, ring write + pooling               hk_layernorm_f16, hk_kpool_write
               absorbed query projection                                  hk_q_latent
               per block of 1,024 rows: scores, top-512, expansion        hk_indexer_score, hk_dsa_topk, hk_pool_expand
               sparse attention over the selected latents                 hk_mla_sparse
               absorbed output projection                                 hk_o_absorb
+  (n == 1)    append, key norm, ring write and position in one launch    hk_mla_decode_prologue
+  (n <= 8)    scores, then top-512 with the expansion inside             hk_indexer_select
 `fused=False` runs the KDA layer as the reference's own call sequence instead (transpose+cast, gate, conv,
 recurrence launcher), the form the unchanged engine would call.
 
@@ -95,7 +97,6 @@ class TrunkAttention:
         self.lat_out = t.empty(n, 64, 512, dtype=t.float16, device=dev)
         self.o_abs = t.empty(n, 64, 256, dtype=t.float16, device=dev)
         self.sparse_ws = t.empty(256, dtype=t.uint8, device=dev)          # grown on demand (split partials of few-row calls)
-        self.x16 = t.empty(B, dim, dtype=t.bfloat16, device=dev)          # a decoded token's pre-conv q|k|v
         self.kept = {}
         self.stage_ms = {}
         self._events = []
@@ -163,15 +164,6 @@ class TrunkAttention:
             self._mark("kda_gated_norm")
         if self.keep:
             self.kept.setdefault(("kda", L), []).append((rec.clone(), y.clone()))
-
-    def _decode_gate(self, f, b):
-        """gate preparation of a single decoded token (glue::kda_gate), for the one-launch decode step"""
-        t, ki, B, H, D = self.torch, self.kda_in, self.B, self.H, self.D
-        if not hasattr(self, "_dg"):
-            self._dg = (t.empty(B, H, D, dtype=t.float32, device="cuda"), t.empty(B, H, dtype=t.bfloat16, device="cuda"))
-        g, beta = self._dg
-        self.hk.kda_gate(b.reshape(B, H), f.reshape(B, H, D), ki["dt_bias"], ki["a_log"], ki["lower_bound"], beta, g, B, H, D)
-        return g, beta
 
     def _short(self, qkv, f, b, L, rec, n):
         """rows below one chunk (decode through the unfused call sequence): gate, then the recurrence launcher"""
