@@ -320,10 +320,16 @@ def dsa_topk_expand(scores, s_stride, indices, raw_idx, q_pos, R, T, k, after_sc
     _run("hk_dsa_topk_expand", scores, s_stride, indices, raw_idx, q_pos, R, T, k, 1 if after_scorer else 0, stream)
 
 
+_key_types = {}
+
+
 def _key_type(t):
     """bf16 by the tensor's type; fp16 keys may come as any 16-bit type that holds their bit patterns"""
-    import torch
-    return HK_BF16 if t.dtype == torch.bfloat16 else HK_F16
+    tag = _key_types.get(t.dtype)
+    if tag is None:
+        import torch
+        tag = _key_types[t.dtype] = HK_BF16 if t.dtype == torch.bfloat16 else HK_F16
+    return tag
 
 
 def indexer_select(q_idx, pool_k_nt, w, q_pos, scores, indices, raw_idx, m, npools, k=512, stream=None, score_stride=None,
