@@ -12,16 +12,20 @@
 //   U = Uloc - W S0                                 (delta-rule residuals of the whole chunk)
 //   O = scale (Q+ S0 + (B diag(beta)) U)            S' = diag(e^{G_last}) S0 + Kt^T U
 //
-// Kernel 1 (kda_chunk_prep_kernel) is parallel over every (batch, head, chunk): it builds A and B
-// on the warp-level tensor cores in TF32 with per-16-token re-basing of the exponents (the
-// triangular 16x16 blocks are smaller than a tcgen05 tile and need fp32 exponent range), inverts the
-// unit-triangular system in fp32, and runs the dense W|Uloc = T [K+|V] product as ONE
-// tcgen05 M128 N256 K64 contraction.  It writes, per chunk, operand tiles that are already in the
-// shared-memory layout kernel 2 needs (74,240 bytes).
-// Kernel 2 (kda_chunk_scan_kernel) walks the chunks of one (batch, head, 32-column value slice) in
-// order.  The fp32 state slice stays in registers; per chunk it pulls the 60 KB of operands with TMA
-// bulk copies (three stages in flight) and issues three tcgen05 contractions with TMEM accumulators:
-// [W;Q+] S0 (M128 N32 K128), [0;B beta] U (accumulated onto the Q+ S0 rows) and Kt^T U (M128 N32 K64).
+// The preparation (prep_unit: kernel 1, or the workers of the fused launch) is parallel over every (batch, head, chunk).  It builds A
+// and B on the warp-level tensor cores: 16-token blocks against earlier blocks in fp16 with exponents re-based at block starts (both
+// operands at most 1), a block against itself in TF32 (e^{-x} needs the fp32 exponent range; the triangular tiles are smaller than a
+// tcgen05 tile).  It inverts the unit-triangular system in fp32-class arithmetic and runs the dense W | Uloc = T [K+ | V] product on
+// tcgen05 (M128 N128 K64, twice).  It writes, per chunk, operand tiles that are already in the shared-memory layout the scan
+// needs (74,240 bytes).
+//   What bounds it: latencies.  A unit crosses five barriers of its 256 threads and one product; two units share an SM (128 registers
+//   a thread, 109 KB).  Inputs arrive by tensor copies issued while the unit before is finished.  A worker's unit takes 22-24 thousand
+//   cycles with two workers on the SM, 39 thousand in the form before (k and q rows in separate warps, TF32 for all block pairs,
+//   13 barriers, loads through registers); 32,768 tokens x 32 heads 1.43 -> 1.02 ms, chain-bound, with gates formed inside 1.62 -> 1.09.
+//   Registers decide: everything a thread keeps across stage 2 is the 32 packed left operands; a version that kept the fp32 rows (300
+//   bytes of spills, whose reloads miss the L1 that shared memory leaves) took 30 thousand cycles.
+// The scan walks the chunks of a chain in order; the fp32 state stays in registers.  Per chunk: D1 = [I ; 0] Uloc + [-W ; Q+] S0 (rows
+// 0-63 are U), Kt^T U (state), [. ; B beta] U onto the Q+ S0 rows (outputs), all tcgen05 with TMEM accumulators.
 #include <cuda.h>   // CUtensorMap (types only; the encoder is fetched through the runtime at first use)
 #include <cuda_pipeline_primitives.h>
 
@@ -36,12 +40,18 @@ constexpr int KC = 64;                    // chunk length
 constexpr int KD = 128;                   // head dim (k and v)
 constexpr int KNV = 32;                   // value columns per scan CTA
 constexpr int KVS = KD / KNV;             // value slices
+constexpr int KR = 16;                    // fused form: ring slots (chunks) per chain
+// Flags: [0] launch-wide abort word, then a 128-byte line of ready flags and one for the consumed count per chain slot.  With all of
+// them packed into a few lines of one page the polls of 232 workers held up the chains' own flags: 1.05 or 1.3-1.9 ms for 32,768
+// tokens x 32 heads, by the die that the page's address falls to.
+constexpr int F_FLAG_INTS = 32;
+constexpr int F_LINE = 32;
 
 // ---- per-chunk workspace unit (bytes); every tile is in its final shared-memory layout ----
-constexpr uint32_t U_WQ = 0;              // fp16 A operand, K-major, rows 0-63 W, 64-127 Q+ ; K = 128 channels
-constexpr uint32_t U_BB = 32768;          // fp16 A operand rows (t), K = 64 (s): B_ts beta_s
-constexpr uint32_t U_KT = 40960;          // fp16 A operand rows = 128 channels, K = 64 tokens: Kt^T
-constexpr uint32_t U_UL = 57344;          // fp16 Uloc as [4 slices][64 tokens][32]
+constexpr uint32_t U_WQ = 0;              // fp16 A operand, K-major, rows 0-63 -W, 64-127 Q+ ; K = 128 channels
+constexpr uint32_t U_UL = 32768;          // fp16 Uloc as B operand, MN-major [16 pieces of 8 columns][64 tokens], token t at t ^ 8
+constexpr uint32_t U_BB = 49152;          // fp16 A operand rows (t), K = 64 (s): B_ts beta_s
+constexpr uint32_t U_KT = 57344;          // fp16 A operand rows = 128 channels, K = 64 tokens: Kt^T, MN-major (8 channels of a token per piece)
 constexpr uint32_t U_DEC = 73728;         // f32 e^{G_last}[128]
 constexpr uint32_t U_BYTES = 74240;
 
@@ -56,7 +66,7 @@ __device__ __forceinline__ uint32_t f2tf32(float x) {
   return r;
 }
 __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -94,7 +104,7 @@ __device__ __forceinline__ bool poll_flag_ge(const int* flag, int want, volatile
   for (;;) {
     if (*abort_flag) return false;
     if (ld_acquire_gpu(flag) >= want) return true;
-    __nanosleep(64);
+    __nanosleep(200);
     if (ld_relaxed_gpu(g_abort) != 0 || clock64() - t0 > tc::MBAR_WAIT_CYCLES) {
       *abort_flag = code;
       atomicExch(g_abort, code);
@@ -104,616 +114,688 @@ __device__ __forceinline__ bool poll_flag_ge(const int* flag, int want, volatile
 }
 
 // =================================================================================================
-// kernel 1: per-chunk preparation.  256 threads, 104 KB of shared memory: two CTAs per SM, so the
+// kernel 1: per-chunk preparation.  256 threads, 109 KB of shared memory: two CTAs per SM, so the
 // serial stages of one chunk overlap with another chunk's.
 // =================================================================================================
-constexpr int P1_LD = 132;                               // fp32 row pitch (conflict-free fragment loads)
-constexpr int P1_LDH = 136;                              // 16-bit row pitch of raw k
-constexpr int P1_LDA = 68;                               // fp32 row pitch of the 64x64 matrices
-constexpr uint32_t P1_KP = 0;                            // fp16 K+ = first half of the B operand [K+|V] (16 KB)
-constexpr uint32_t P1_G = 16384;                         // f32 [64][132] cumulative log decay, then R  (later: V half of the B operand)
-constexpr uint32_t P1_KR = P1_G + KC * P1_LD * 4;        // X = inverse, f32 [64][68]
-constexpr uint32_t P1_L = P1_KR + KC * P1_LDH * 2;       // raw bf16 v rows as loaded (16 KB), then the T operand (16 KB)
-constexpr uint32_t P1_A = P1_L + 2 * 16 * P1_LD * 4;     // f32 [64][68] N = A beta (strictly lower); upper blocks = scratch
-constexpr uint32_t P1_P = P1_A + KC * P1_LDA * 4;     // f32 [4][128] G_last - (sum before each 16-token block)
-constexpr uint32_t P1_EP = P1_P + 2048;                  // f32 [4][128] e^{sum before the block}
-constexpr uint32_t P1_BETA = P1_EP + 2048;               // f32 [64]
-constexpr uint32_t P1_RK = P1_BETA + 256;                // f32 [64] 1 / |k_t|
-constexpr uint32_t P1_DD = P1_RK + 256;                  // f32 [6][128] decay between the starts of two blocks
-constexpr uint32_t P1_TOT = P1_DD + 3072;                // f32 [4][128] log-decay total of each block
-constexpr uint32_t P1_SMEM = P1_TOT + 2048;
-static_assert(KC * P1_LD * 4 >= 16384 && 2 * 16 * P1_LD * 4 >= 16384 && KC * P1_LDH * 2 == KC * P1_LDA * 4, "aliases");
+// Warp w owns tokens 8 w .. 8 w + 7: lane 4 g8 + tig holds, of token 8 w + g8, the eight channels from 8 tig of every 32, of the
+// k row and of the q row.  That is the fragment layout of the warp-level products in both places: as the left operand (rows
+// 0-7 of a 16-row tile = k tokens, rows 8-15 = the q rows of the same tokens) and as the right operand (columns = tokens), so the
+// product of a warp's tokens with themselves needs no shared memory, and one exponential serves k and q.
+// Every input tile arrives by tiled tensor copies in the 128-byte-swizzle pattern (16-byte piece p of row r at p ^ (r % 8)).
+constexpr uint32_t P1_PIECE = 1056;                      // bytes between the 8-channel pieces of K+ (1024 + 32: the four pieces that a
+                                                         // quarter-warp writes start in different banks)
+constexpr uint32_t P1_X = 0;                             // f32 log decays, then their sums x: four boxes [64 tokens][32 channels]; then the
+                                                         // right operands of the even warps' tokens, then the inverses of the diagonal blocks
+constexpr uint32_t P1_V = 32768;                         // v: two boxes [64 tokens][64 channels], bf16 as loaded, fp16 in place: the B operand
+constexpr uint32_t P1_RI = 49152;                        // fp16 right operands of the block pairs (i, j < i), 16 tokens x 256 B each;
+                                                         // later the T operand (8 KB)
+constexpr uint32_t P1_N = P1_RI + 6 * 4096;              // f32 N = A beta: rows 0-31 at a pitch of 36, rows 32-63 at 68
+constexpr uint32_t P1_QK = P1_RI;                        // the next unit's q and k: two boxes each, over the two regions before
+constexpr uint32_t P1_K = P1_N + 32 * (36 + 68) * 4;     // fp16 K+, B operand, MN-major, 16 pieces
+constexpr uint32_t P1_TAB = P1_K + 16 * P1_PIECE;        // f32 tables [15][128]
+constexpr uint32_t P1_SMEM = P1_TAB + 15 * 512;
+constexpr int TAB_EP = 0, TAB_ETOT = 4, TAB_KE = 8, TAB_F = 12;   // rows: e^{P_J} | e^{tot_J} | e^{G_last - P_{J+1}} | (2,0), (3,1), (3,0)
+static_assert(P1_SMEM % 1024 == 0 && P1_QK % 1024 == 0 && P1_QK + 32768 <= P1_K && P1_TAB % 16 == 0, "layout");
+constexpr uint32_t P1_BOX = 8192;
+constexpr int P1_LDX = 20;                               // pitch of a diagonal block's inverse
 
-// Optional stage timeline (diagnostic build, -DHK_DIAG): one preparation worker and one scan CTA stamp clock64 at
-// their stage boundaries; hk_debug_kda_trace copies the stamps to the host.
+__device__ __forceinline__ int prep_n_row(int t) { return t < 32 ? t * 36 : 32 * 36 + (t - 32) * 68; }
+__device__ __forceinline__ int prep_inv_at(int blk) { return blk * 16 * P1_LDX; }
+
+// Optional stage timeline (diagnostic build, -DHK_DIAG): one scan CTA stamps clock64 at its stage boundaries;
+// hk_debug_kda_trace copies the stamps to the host.
 #ifdef HK_DIAG
 __device__ long long hk_kda_trace[128];
-// stamps go to shared memory and are copied out once per unit.  A stamp placed after a barrier is taken when the
-// stamping warp ARRIVES there (the clock read is not held back by the barrier): the intervals are that warp's own
-// work, not the stage's length - the slowest warp of a stage shows up in the NEXT interval.
-__shared__ long long hk_kda_stamps[16];
-#define KT_TRACE(slot) do { if (ctx.trace && ctx.tid == 0) hk_kda_stamps[slot] = clock64(); } while (0)
-#define KT_FLUSH() do { if (ctx.trace && ctx.tid == 0) { for (int q_ = 0; q_ < 16; q_++) hk_kda_trace[q_] = hk_kda_stamps[q_]; } } while (0)
 #define KS_TRACE(slot, ch) do { if (threadIdx.x == 0 && blockIdx.x == 1 && (ch) == 100) hk_kda_trace[32 + (slot)] = clock64(); } while (0)
 #define KS_TRACE_AT(slot, ch, want) do { if (threadIdx.x == 0 && blockIdx.x == 1 && (ch) == (want)) hk_kda_trace[32 + (slot)] = clock64(); } while (0)
 #else
 #define KS_TRACE_AT(slot, ch, want) do { } while (0)
-#define KT_TRACE(slot) do { } while (0)
-#define KT_FLUSH() do { } while (0)
 #define KS_TRACE(slot, ch) do { } while (0)
 #endif
 
-// 16 x 16 block product on the warp-level tensor cores: acc += L R with L, R fp32 in shared memory (row
-// pitch P1_LDA).  Each operand is split into a TF32 head and a TF32 tail and the three significant
-// partial products are accumulated in fp32, which keeps the result at fp32-class accuracy.
-__device__ __forceinline__ void block16_mma(const float* __restrict__ L, const float* __restrict__ R,
-                                            float (&acc)[2][4], int lane) {
-  const int g8 = lane >> 2, tig = lane & 3;
-#pragma unroll
-  for (int ks = 0; ks < 2; ks++) {
-    const float af[4] = {L[g8 * P1_LDA + 8 * ks + tig], L[(g8 + 8) * P1_LDA + 8 * ks + tig],
-                         L[g8 * P1_LDA + 8 * ks + tig + 4], L[(g8 + 8) * P1_LDA + 8 * ks + tig + 4]};
-    uint32_t ah[4], al[4];
+// 16 x 16 left operand of a block product as TF32 heads and tails.  The contraction index is taken in the order in which an
+// accumulator holds its columns (k slots tig and tig + 4 of step s are columns 8 s + 2 tig and 8 s + 2 tig + 1), so that the
+// accumulator of one product is the left operand of the next without a detour.
+struct Frag16 {
+  uint32_t h[2][4], l[2][4];
+  __device__ __forceinline__ void set(int ks, const float (&f)[4]) {   // f = (row g8: two columns, row g8 + 8: two columns)
+    const float a[4] = {f[0], f[2], f[1], f[3]};
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-      ah[e] = f2tf32(af[e]);
-      al[e] = f2tf32(af[e] - __uint_as_float(ah[e]));
+      h[ks][e] = f2tf32(a[e]);
+      l[ks][e] = f2tf32(a[e] - __uint_as_float(h[ks][e]));
     }
+  }
+  __device__ __forceinline__ void load(const float* __restrict__ p, int ld, int lane) {
+    const int g8 = lane >> 2, tig = lane & 3;
+#pragma unroll
+    for (int ks = 0; ks < 2; ks++) {
+      const float2 u = *reinterpret_cast<const float2*>(p + g8 * ld + 8 * ks + 2 * tig);
+      const float2 d = *reinterpret_cast<const float2*>(p + (g8 + 8) * ld + 8 * ks + 2 * tig);
+      const float f[4] = {u.x, u.y, d.x, d.y};
+      set(ks, f);
+    }
+  }
+};
+// acc += L R, R fp32 in shared memory.  Both operands are split into a TF32 head and tail and the three significant partial
+// products are accumulated in fp32 (in sums of their own: shorter chains), which keeps the result at fp32-class accuracy.
+__device__ __forceinline__ void block16_mma(const Frag16& L, const float* __restrict__ R, int ld, float (&acc)[2][4], int lane) {
+  const int g8 = lane >> 2, tig = lane & 3;
+  float lo[2][2][4];
+#pragma unroll
+  for (int e = 0; e < 16; e++) lo[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 2; ks++)
 #pragma unroll
     for (int nt = 0; nt < 2; nt++) {
-      const float b0 = R[(8 * ks + tig) * P1_LDA + 8 * nt + g8], b1 = R[(8 * ks + tig + 4) * P1_LDA + 8 * nt + g8];
+      const float b0 = R[(8 * ks + 2 * tig) * ld + 8 * nt + g8], b1 = R[(8 * ks + 2 * tig + 1) * ld + 8 * nt + g8];
       const uint32_t b0h = f2tf32(b0), b1h = f2tf32(b1);
       const uint32_t b0l = f2tf32(b0 - __uint_as_float(b0h)), b1l = f2tf32(b1 - __uint_as_float(b1h));
-      mma_tf32(acc[nt], al, b0h, b1h);
-      mma_tf32(acc[nt], ah, b0l, b1l);
-      mma_tf32(acc[nt], ah, b0h, b1h);
+      mma_tf32(lo[0][nt], L.l[ks], b0h, b1h);
+      mma_tf32(lo[1][nt], L.h[ks], b0l, b1l);
+      mma_tf32(acc[nt], L.h[ks], b0h, b1h);
     }
-  }
+#pragma unroll
+  for (int e = 0; e < 8; e++) acc[e >> 2][e & 3] += lo[0][e >> 2][e & 3] + lo[1][e >> 2][e & 3];
 }
 
-// writes sign * acc (fragment rows g8, g8 + 8; columns 8 nt + 2 tig, + 1) to a 16 x 16 block
-__device__ __forceinline__ void block16_store(float* __restrict__ D, const float (&acc)[2][4], float sign, int lane) {
+// two fp32 values of a register pair -> fp16 pair
+__device__ __forceinline__ uint32_t pack_h2(uint64_t v) {
+  float a, b;
+  unpack2(v, a, b);
+  return pack_h2(a, b);
+}
+// 4 register pairs = 8 channels of a token -> one 16-byte fp16 piece
+__device__ __forceinline__ uint4 pack_piece(const uint64_t* v) { return make_uint4(pack_h2(v[0]), pack_h2(v[1]), pack_h2(v[2]), pack_h2(v[3])); }
+// 8 floats of shared memory as 4 register pairs
+__device__ __forceinline__ void load_pairs(const float* __restrict__ p, uint64_t (&v)[4]) {
+  const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(p), b = *reinterpret_cast<const ulonglong2*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void mma_f16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Row block i of the inverse, right to left: X_ij = - sum_{m = j+1}^{i} X_im P_mj, P_mj = N_mj X_jj (in place of N_mj), one warp,
+// all blocks of the row in registers; each leaves as fp16 for the T operand.  Once X_im is known its products with all P_mj are
+// formed together, so that only one product per block of the row stands behind another.
+template <int I>
+__device__ __forceinline__ void prep_inverse_row(const float* __restrict__ sN, const float* __restrict__ sX, uint8_t* __restrict__ sT, int lane) {
   const int g8 = lane >> 2, tig = lane & 3;
+  float acc[I][2][4];
 #pragma unroll
-  for (int nt = 0; nt < 2; nt++) {
-    *reinterpret_cast<float2*>(D + g8 * P1_LDA + 8 * nt + 2 * tig) = make_float2(sign * acc[nt][0], sign * acc[nt][1]);
-    *reinterpret_cast<float2*>(D + (g8 + 8) * P1_LDA + 8 * nt + 2 * tig) = make_float2(sign * acc[nt][2], sign * acc[nt][3]);
-  }
-}
-
-// Stage 4 of the preparation kernel for one warp: rows 16 ib .. 16 ib + 15 of A (k warps) or B (q warps)
-// against the column blocks jb <= ib.  v = this thread's left-operand fragment values (rows g8, g8 + 8;
-// channel 32 m + 8 tig + j at index 8 m + j).  k-step ks of the m16n8k8 product contracts the channel
-// pairs (32 m + 8 tig + j, + 1), j = 2 (ks % 4), m = ks / 4, in MMA k slots tig and tig + 4.
-__device__ __forceinline__ void prep_ab_block(const int ib, const float (&v)[2][32], bool is_q, const float* __restrict__ sR,
-                                              const float* __restrict__ sDD, const float* __restrict__ sBeta,
-                                              float* __restrict__ sA, uint8_t* __restrict__ unit, int g8, int tig) {
-  // one code path for all row blocks (column blocks jb > ib are skipped by warp-uniform branches): four
-  // specialised copies of this fully unrolled body would not fit the instruction cache
-  float acc[4][2][4];
+  for (int j = 0; j < I; j++)
 #pragma unroll
-  for (int jb = 0; jb < 4; jb++)
+    for (int e = 0; e < 8; e++) acc[j][e >> 2][e & 3] = 0.f;
+  Frag16 X;
+  X.load(sX + prep_inv_at(I), P1_LDX, lane);
 #pragma unroll
-    for (int nt = 0; nt < 2; nt++)
+  for (int m = I; m >= 1; m--) {
 #pragma unroll
-      for (int e = 0; e < 4; e++) acc[jb][nt][e] = 0.f;
-  const float* dd_base = sDD + (ib * (ib - 1) / 2) * KD;
-  // two k-steps per pass: the R rows are read 16 bytes at a time (4 channels = both channel pairs of the
-  // two k-steps), which with the 132-float row pitch is free of bank conflicts (a quarter-warp covers
-  // rows g8, g8 + 1 and the four tig: 4 g8 + 8 tig are eight different 4-bank groups)
-#pragma unroll
-  for (int kp = 0; kp < 8; kp++) {
-    const int m = kp >> 1, j = (kp & 1) * 4;
-    const int c0 = 32 * m + 8 * tig + j;
-    uint32_t a0[4], a1[4];
-    a0[0] = f2tf32(v[0][8 * m + j]); a0[1] = f2tf32(v[1][8 * m + j]);
-    a0[2] = f2tf32(v[0][8 * m + j + 1]); a0[3] = f2tf32(v[1][8 * m + j + 1]);
-    a1[0] = f2tf32(v[0][8 * m + j + 2]); a1[1] = f2tf32(v[1][8 * m + j + 2]);
-    a1[2] = f2tf32(v[0][8 * m + j + 3]); a1[3] = f2tf32(v[1][8 * m + j + 3]);
-#pragma unroll
-    for (int jb = 0; jb < 4; jb++) {
-      if (jb <= ib) {
-        float4 dd = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (jb < ib) dd = *reinterpret_cast<const float4*>(dd_base + jb * KD + c0);
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++) {
-          const float4 r4 = *reinterpret_cast<const float4*>(sR + (jb * 16 + nt * 8 + g8) * P1_LD + c0);
-          mma_tf32(acc[jb][nt], a0, f2tf32(r4.x * dd.x), f2tf32(r4.y * dd.y));
-          mma_tf32(acc[jb][nt], a1, f2tf32(r4.z * dd.z), f2tf32(r4.w * dd.w));
-        }
-      }
-    }
-  }
-  // accumulator fragment: rows t = 16 ib + g8 (+8), columns s = 16 jb + 8 nt + 2 tig (+1)
-#pragma unroll
-  for (int jb = 0; jb < 4; jb++) {
-    if (jb > ib) continue;
+    for (int j = m - 1; j >= 0; j--) block16_mma(X, sN + prep_n_row(16 * m) + 16 * j, m < 2 ? 36 : 68, acc[j], lane);
+    const int j = m - 1;                                   // X_ij is complete
 #pragma unroll
     for (int nt = 0; nt < 2; nt++) {
-      const int s0 = jb * 16 + nt * 8 + tig * 2;
-      const float b0 = sBeta[s0], b1 = sBeta[s0 + 1];
-#pragma unroll
-      for (int hrow = 0; hrow < 2; hrow++) {
-        const int t = ib * 16 + g8 + hrow * 8;
-        if (!is_q) {            // N = A beta, strictly lower
-          if (s0 < t) sA[t * P1_LDA + s0] = acc[jb][nt][2 * hrow] * b0;
-          if (s0 + 1 < t) sA[t * P1_LDA + s0 + 1] = acc[jb][nt][2 * hrow + 1] * b1;
-        } else {                // B beta, lower including the diagonal, fp16 operand tile
-          const float v0 = s0 <= t ? acc[jb][nt][2 * hrow] * b0 : 0.f;
-          const float v1 = s0 + 1 <= t ? acc[jb][nt][2 * hrow + 1] * b1 : 0.f;
-          *reinterpret_cast<uint32_t*>(unit + U_BB + (t >> 3) * SBO_K64 + (s0 >> 3) * LBO + (t & 7) * 16 + (s0 & 7) * 2) =
-              pack_h2(v0, v1);
-        }
-      }
+      const float f[4] = {-acc[j][nt][0], -acc[j][nt][1], -acc[j][nt][2], -acc[j][nt][3]};
+      if (j > 0) X.set(nt, f);
+      uint8_t* p = sT + (2 * I) * SBO_K64 + (2 * j + nt) * LBO + g8 * 16 + tig * 4;
+      *reinterpret_cast<uint32_t*>(p) = pack_h2(f[0], f[1]);
+      *reinterpret_cast<uint32_t*>(p + SBO_K64) = pack_h2(f[2], f[3]);
     }
   }
 }
 
-// What one preparation worker (256 threads) needs besides the tensors: its shared memory, its completion barrier
-// for the tensor-core product, its 256 TMEM columns and how it synchronises.  SUB = false: the worker is a whole
-// CTA (__syncthreads); SUB = true: it is one half of a 512-thread CTA and uses the named barrier `bar_id`.
+// What a preparation worker (256 threads) keeps in static shared memory: its barriers and the units it has at hand (unit number `it`
+// at it % 4; thread registers are too few to carry them through a unit).  SUB = false: the worker is a whole CTA with one unit
+// (__syncthreads); SUB = true: it is one of the two workers of a CTA and uses the named barriers `bar_id` (all of it) and `bar_id + 2`
+// (the four warps that write a unit's last part).
+struct PrepDesc {
+  int tok0;                                                // first token: batch * seqlen + 64 * chunk
+  int b, t0;                                               // batch, first token in it
+  int n_valid;                                             // its tokens, 0: no such unit
+  int head;
+  int unit;                                                // index of its place in the workspace or ring
+  int slot, value;                                         // fused form: chain slot; running chunk number + 1 (the ready flag's value)
+};
+struct PrepShared {
+  uint64_t mma_bar;                                        // the unit's tensor-core product is complete
+  uint64_t g_bar;                                          // its gate rows have landed
+  uint64_t qkv_bar;                                        // its q, k and v rows
+  uint64_t pair_bar[4][4];                                 // right operands of the even warp of block I, channels 32 m .. 32 m + 31
+  PrepDesc unit[4];
+};
 struct PrepCtx {
   uint8_t* smem;
-  uint64_t* bar;
-  uint32_t bar_parity;
+  PrepShared* sh;
   volatile int* abort_flag;
-  uint32_t tmem;
   int tid;
   int bar_id;
-  bool trace;
-  // fused form only: the ring slot this unit is written to must have been drained (flag >= want); thread 0 sampled
-  // the flag at the start of the unit (slot_seen) and polls, with a bound, only if that was too early
-  const int* slot_flag;
-  int slot_want, slot_seen;
-  int* g_abort;
 };
 template <bool SUB>
 __device__ __forceinline__ void prep_sync(const PrepCtx& ctx) {
   if (SUB) asm volatile("bar.sync %0, 256;" ::"r"(ctx.bar_id) : "memory");
   else __syncthreads();
 }
+__device__ __forceinline__ void prep_init(PrepShared& sh) {  // one thread
+  tc::mbar_init(&sh.mma_bar, 1);
+  tc::mbar_init(&sh.g_bar, 1);
+  tc::mbar_init(&sh.qkv_bar, 1);
+  for (int i = 0; i < 16; i++) tc::mbar_init(&sh.pair_bar[i >> 2][i & 3], 1);
+}
+// a field of the unit `it`, read anew at every use
+#define PREP_UNIT(field, it) (*const_cast<volatile int*>(&ctx.sh->unit[(it) & 3].field))
 
-// One (batch, head, chunk) unit of the preparation.
+// Fused form: stores the ready flag of unit `it`.  Called by warp 0, which meets the other three warps of the unit's last writers
+// here; the barriers inside prep_unit order everybody else's writes before them, and the release store is cumulative over all of
+// them.  It waits until the CTA's stores are visible, some thousand cycles when they are fresh: it is put off to a place in the next
+// unit where warp 0 has nothing else to do, unless the worker has to wait for its ring slot.
+__device__ __forceinline__ void prep_publish(const PrepCtx& ctx, int it, int* ready, int n_slots) {
+  asm volatile("bar.sync %0, 128;" ::"r"(ctx.bar_id + 2) : "memory");
+  if (ctx.tid == 0) {
+    const int value = PREP_UNIT(value, it);
+    st_release_gpu(ready + (size_t)PREP_UNIT(slot, it) * F_LINE + (value - 1) % KR, value);
+  }
+}
+
+// Tensor maps of the inputs: qkv as [batch][token][3 H 128] bf16, box 64 tokens x 64 channels; g (or f) as [batch][token][H 128] f32,
+// box 64 tokens x 32 channels; 128-byte swizzle, tokens past the end read as zeros.
+__device__ __forceinline__ void prep_tma(uint8_t* dst, const CUtensorMap* map, int c, int t, int b, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(tc::smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(t), "r"(b), "r"(tc::smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void prep_tma_l2(const CUtensorMap* map, int c, int t, int b) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(t), "r"(b)
+               : "memory");
+}
+// the next unit's inputs, each as soon as its place is free (one thread)
+__device__ __forceinline__ void prep_fetch_g(const PrepCtx& ctx, int it, const CUtensorMap* map_g) {
+  if (PREP_UNIT(n_valid, it) == 0) return;
+  const int c = PREP_UNIT(head, it) * KD, t0 = PREP_UNIT(t0, it), b = PREP_UNIT(b, it);
+  tc::mbar_arrive_expect_tx(&ctx.sh->g_bar, 4 * P1_BOX);
+#pragma unroll
+  for (int m = 0; m < 4; m++) prep_tma(ctx.smem + P1_X + m * P1_BOX, map_g, c + 32 * m, t0, b, &ctx.sh->g_bar);
+}
+__device__ __forceinline__ void prep_fetch_qkv(const PrepCtx& ctx, int it, const CUtensorMap* map_qkv, int H) {
+  if (PREP_UNIT(n_valid, it) == 0) return;
+  const int c = PREP_UNIT(head, it) * KD, t0 = PREP_UNIT(t0, it), b = PREP_UNIT(b, it);
+  tc::mbar_arrive_expect_tx(&ctx.sh->qkv_bar, 6 * P1_BOX);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    prep_tma(ctx.smem + P1_QK + (2 + h) * P1_BOX, map_qkv, H * KD + c + 64 * h, t0, b, &ctx.sh->qkv_bar);
+    prep_tma(ctx.smem + P1_QK + h * P1_BOX, map_qkv, c + 64 * h, t0, b, &ctx.sh->qkv_bar);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++) prep_tma(ctx.smem + P1_V + h * P1_BOX, map_qkv, 2 * H * KD + c + 64 * h, t0, b, &ctx.sh->qkv_bar);
+}
+
+// Unit number `it` of a worker: (batch, head, chunk) of the preparation, into its place of `units`.
 // GATED: `g` holds the raw gate projection f and `beta_in` the raw fp32 b; the kernel applies
 //   g = lower_bound * sigmoid(exp(a_log[head]) * (f + dt_bias[head][channel])),  beta = bf16(sigmoid(b))
 // itself (the arithmetic of the reference's separate gate kernel, src/engine/glue2.cu:347-360), so the
 // fp32 gate tensor is never written to or read back from memory.
-// (pf_head, pf_chunk): a unit whose input rows this worker asks the copy engine to pull into L2 (pf_chunk < 0: none).
-template <bool GATED, bool SUB>
+// The unit's inputs are on their way (prep_fetch_*); its end sends for those of the next.  SUB: `ready` and `consumed` are the flags
+// of the ring; on return the unit's last writes are on their way and its flag is still to be stored (prep_publish).
+// `make_unit(it, desc)` works out a later unit (one thread).
+template <bool GATED, bool SUB, class MakeUnit>
 __device__ __forceinline__ void prep_unit(
-    const PrepCtx& ctx, const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ g,
-    const void* __restrict__ beta_in, uint8_t* __restrict__ unit, int seqlen, int H, int head, int chunk, int b,
-    int pf_head, int pf_chunk, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
-    float lower_bound) {
-  uint8_t* smem = ctx.smem;
-  float* sG = reinterpret_cast<float*>(smem + P1_G);
-  float* sA = reinterpret_cast<float*>(smem + P1_A);
-  float* sGLP = reinterpret_cast<float*>(smem + P1_P);
-  float* sTot = reinterpret_cast<float*>(smem + P1_TOT);
-  float* sEP = reinterpret_cast<float*>(smem + P1_EP);
-  float* sBeta = reinterpret_cast<float*>(smem + P1_BETA);
-  float* sDD = reinterpret_cast<float*>(smem + P1_DD);
-  float* sETot = sTot;                                     // e^{block total}: overwrites the totals once the tables are built
-  float* sEGLN = sGLP;                                     // e^{G_last - (sum up to the END of the block)}
-  uint8_t* sKV = smem + P1_KP;                             // [K+ | V] fp16 B operand; the V half aliases sG, valid after the A/B stage
-  float* sX = reinterpret_cast<float*>(smem + P1_KR);      // alias, valid after the A/B stage
-  uint8_t* sT = smem + P1_L;                               // raw v rows, then the T operand (valid after the conversion of v)
+    const PrepCtx& ctx, const int it, const CUtensorMap* map_qkv, const CUtensorMap* map_g, const void* __restrict__ beta_in,
+    uint8_t* __restrict__ units, int H, const float* __restrict__ dt_bias, const float* __restrict__ a_log, float lower_bound,
+    const uint32_t tmem, int* ready, const int* consumed, int* g_abort, int n_slots, MakeUnit&& make_unit) {
+  uint8_t* const smem = ctx.smem;
+  uint8_t* const sK = smem + P1_K;
+  float* const sX = reinterpret_cast<float*>(smem + P1_X);
+  uint8_t* const sRI = smem + P1_RI;
+  uint8_t* const sT = smem + P1_RI;
+  float* const sN = reinterpret_cast<float*>(smem + P1_N);
+  float* const sTab = reinterpret_cast<float*>(smem + P1_TAB);
 
-  const int tid = ctx.tid, lane = tid & 31, warp = tid >> 5;
-  const int t0 = chunk * KC;
-  const int n_valid = min(KC, seqlen - t0);
-  const size_t row = (size_t)3 * H * KD;
-  const __nv_bfloat16* tok0 = qkv + ((size_t)b * seqlen + t0) * row;
-  const float* g0 = g + (((size_t)b * seqlen + t0) * H + head) * KD;
-
-  KT_TRACE(0);
-  // L2 prefetch of the input rows of a later unit (about one wave of workers ahead): its q, k, v rows (256 B each)
-  // and g rows (512 B), one request per thread.  That unit's own loads then mostly hit L2.
-  {
-    const int pt = pf_chunk * KC + (tid & 63);
-    if (pf_chunk >= 0 && pt < seqlen) {
-      const __nv_bfloat16* ptok = qkv + ((size_t)b * seqlen + pt) * row;
-      const int part = tid >> 6;                          // 0: q, 1: k, 2: v, 3: g
-      if (part < 3) tc::prefetch_l2(ptok + (size_t)(part * H + pf_head) * KD, KD * 2);
-      else tc::prefetch_l2(g + (((size_t)b * seqlen + pt) * H + pf_head) * KD, KD * 4);
-    }
-  }
-  // ---- stage 1: loads.  Ownership for stages 1-4 is the TF32 MMA fragment layout, so that the left
-  //      operands of the A/B products never pass through shared memory: warp -> (16-token row block ib,
-  //      k or q), lane = 4*g8 + tig owns rows 16 ib + g8 and + 8 and, of every 32 channels, the 8
-  //      starting at 8 tig (one 16-byte piece).  Block ib has ib+1 column blocks of work and the k warps
-  //      carry the exponentials of stage 3: every scheduler partition gets one k warp and one q warp
-  //      whose row blocks add up to the same work.
+  int tid = ctx.tid;
+  asm volatile("" : "+r"(tid));                            // addresses are formed anew in every unit: hoisted out of the loop they would be spilled
+  const int lane = tid & 31, warp = tid >> 5;
   const int g8 = lane >> 2, tig = lane & 3;
-  const bool is_q = warp >> 2;                              // warps 0-3: k rows, warps 4-7: q rows
-  const int ib = is_q ? 3 - (warp & 3) : (warp & 3);        // partition s hosts k block s and q block 3 - s
-  float v[2][32];                                           // [row half][4 pieces x 8 channels]
+  const int I = warp >> 1;                                 // 16-token block of this warp
+  const bool odd = warp & 1;
+  const int t = 8 * warp + g8;                             // this lane's token
+#define PREP_OUT (units + (size_t)PREP_UNIT(unit, it) * U_BYTES)
+
+  // ---- stage 1: log-decay sums.  x_t = inclusive sum of the log decay (in units of log 2) INSIDE the 16-token block, in place;
+  //      lane 8 J + p of warp w sums channels 16 w + 2 p, + 1 over block J, so the block totals of a channel sit in four lanes
+  //      of one warp, which turn them into the tables ----
+  int seen = 0;                                            // thread 0: chunks of the slot that have been consumed
+  if (SUB && tid == 0) seen = ld_relaxed_gpu(consumed + PREP_UNIT(slot, it) * F_LINE);
+  float beta = 0.f;
+  if (t < PREP_UNIT(n_valid, it)) {
+    const size_t bi = (size_t)(PREP_UNIT(tok0, it) + t) * H + PREP_UNIT(head, it);
+    if (GATED) beta = static_cast<const float*>(beta_in)[bi];
+    else beta = __bfloat162float(static_cast<const __nv_bfloat16*>(beta_in)[bi]);
+  }
+  const int J = lane >> 3, gc = 16 * warp + 2 * (lane & 7);
+  float2 dec;                                              // e^{G_last} of channels gc, gc + 1 (lanes with J = 3)
   {
-    uint4 raw[2][4];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int t = 16 * ib + g8 + 8 * h;
-      const __nv_bfloat16* src = tok0 + (size_t)t * row + (size_t)(is_q ? head : H + head) * KD + 8 * tig;
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-        raw[h][m] = t < n_valid ? *reinterpret_cast<const uint4*>(src + 32 * m) : make_uint4(0, 0, 0, 0);
+    constexpr float LOG2E = 1.4426950408889634f;
+    constexpr float FLOOR = -85.f * LOG2E;                 // keeps e^{x} and e^{-x} inside fp32
+    float decay = 0.f;
+    float2 bias = make_float2(0.f, 0.f);
+    int n_block = 16;                                      // GATED: tokens of this block that exist (the others read as zeros)
+    if (GATED) {
+      const int head = PREP_UNIT(head, it);
+      n_block = PREP_UNIT(n_valid, it) - 16 * J;
+      decay = __expf(__ldg(a_log + head));
+      bias = __ldg(reinterpret_cast<const float2*>(dt_bias + (size_t)head * KD + gc));
     }
-    // g rows straight to shared memory (warp w: tokens w, w+8, ...; lane: 4 channels)
+    float2 tot = make_float2(0.f, 0.f);
+    uint8_t* const xb = smem + P1_X + (gc >> 5) * P1_BOX + 16 * J * 128 + (gc & 3) * 4;
+    const int piece = (gc >> 2) & 7;
+    tc::mbar_wait(&ctx.sh->g_bar, it & 1, ctx.abort_flag, 12);
+    float2 gr[16];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int t = warp + 8 * i;
-      float* gdst = sG + t * P1_LD + lane * 4;
-      if (t < n_valid) __pipeline_memcpy_async(gdst, g0 + (size_t)t * H * KD + lane * 4, 16);
-      else *reinterpret_cast<float4*>(gdst) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __pipeline_commit();
-    // v rows (raw bf16) are parked where the T operand goes later; chunk cc of row t sits at cc ^ (t % 8)
-    // so that the conversion pass (8 rows of one chunk per quarter-warp) is free of bank conflicts.  (The product
-    // T V needs both operands in ONE 16-bit format: a kind::f16 product of an fp16 T with the bf16 rows as they
-    // were loaded is rejected by the hardware as an illegal instruction.)
+    for (int i = 0; i < 16; i++) gr[i] = *reinterpret_cast<const float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4));
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int i = tid + 256 * j, t = i >> 4, cc = i & 15;
-      uint8_t* vdst = sT + t * 256 + ((cc ^ (t & 7)) << 4);
-      if (t < n_valid) __pipeline_memcpy_async(vdst, tok0 + (size_t)t * row + (size_t)(2 * H + head) * KD + cc * 8, 16);
-      else *reinterpret_cast<uint4*>(vdst) = make_uint4(0, 0, 0, 0);
-    }
-    __pipeline_commit();
-    if (tid < KC) {
-      float bv = 0.f;
-      if (tid < n_valid) {
-        const size_t bi = ((size_t)b * seqlen + t0 + tid) * H + head;
-        if (GATED) bv = __bfloat162float(__float2bfloat16(1.0f / (1.0f + __expf(-static_cast<const float*>(beta_in)[bi]))));
-        else bv = __bfloat162float(static_cast<const __nv_bfloat16*>(beta_in)[bi]);
-      }
-      sBeta[tid] = bv;
-    }
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int t = 16 * ib + g8 + 8 * h;
-      float ss = 0.f;
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        const uint32_t w4[4] = {raw[h][m].x, raw[h][m].y, raw[h][m].z, raw[h][m].w};
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float lo = bf16lo(w4[e]), hi = bf16hi(w4[e]);
-          v[h][8 * m + 2 * e] = lo;
-          v[h][8 * m + 2 * e + 1] = hi;
-          ss = fmaf(lo, lo, fmaf(hi, hi, ss));
+    for (int i = 0; i < 16; i++) {
+      if (GATED) {
+        if (i < n_block) {
+          gr[i].x = lower_bound * (1.0f / (1.0f + __expf(-(decay * (gr[i].x + bias.x)))));
+          gr[i].y = lower_bound * (1.0f / (1.0f + __expf(-(decay * (gr[i].y + bias.y)))));
         }
       }
-      ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-      ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-      const float rn = rsqrtf(ss + 1e-6f);                  // L2 normalisation of the q / k row
-#pragma unroll
-      for (int e = 0; e < 32; e++) v[h][e] *= rn;
+      tot.x = fmaf(gr[i].x, LOG2E, tot.x);
+      tot.y = fmaf(gr[i].y, LOG2E, tot.y);
+      *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = make_float2(fmaxf(tot.x, FLOOR), fmaxf(tot.y, FLOOR));
     }
-  }
-  KT_TRACE(1);
-  __pipeline_wait_prior(1);                                 // g has landed; the v rows may still be in flight
-  if (GATED) {
-    // every thread turns the pieces it copied itself (tokens warp, warp + 8, ...; 4 channels) into gates
-    const float decay = __expf(__ldg(a_log + head));
-    const float4 bias = __ldg(reinterpret_cast<const float4*>(dt_bias + (size_t)head * KD) + lane);
+    float2 before = make_float2(0.f, 0.f), after = make_float2(0.f, 0.f), next1 = before, next2 = before;
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int t = warp + 8 * i;
-      if (t < n_valid) {
-        float4* gp = reinterpret_cast<float4*>(sG + t * P1_LD + lane * 4);
-        float4 fv = *gp;
-        fv.x = lower_bound * (1.0f / (1.0f + __expf(-(decay * (fv.x + bias.x)))));
-        fv.y = lower_bound * (1.0f / (1.0f + __expf(-(decay * (fv.y + bias.y)))));
-        fv.z = lower_bound * (1.0f / (1.0f + __expf(-(decay * (fv.z + bias.z)))));
-        fv.w = lower_bound * (1.0f / (1.0f + __expf(-(decay * (fv.w + bias.w)))));
-        *gp = fv;
-      }
+    for (int q = 0; q < 4; q++) {
+      const float qx = __shfl_sync(0xffffffffu, tot.x, 8 * q + (lane & 7)), qy = __shfl_sync(0xffffffffu, tot.y, 8 * q + (lane & 7));
+      if (q < J) { before.x += qx; before.y += qy; }
+      if (q > J) { after.x += qx; after.y += qy; }
+      if (q == J + 1) next1 = make_float2(qx, qy);
+      if (q == J + 2) next2 = make_float2(next1.x + qx, next1.y + qy);
     }
+    auto put = [&](int r, float2 v) { *reinterpret_cast<float2*>(sTab + r * KD + gc) = make_float2(ex2_approx(v.x), ex2_approx(v.y)); };
+    put(TAB_EP + J, before);
+    // decay from a token to the end of ITS block is e^{tot - x} = e^{-x} e^{tot} (each factor within fp32 range for |x| <= 85),
+    // the decay over the LATER blocks is e^{G_last - P_next} (may underflow: then Kt is 0)
+    put(TAB_ETOT + J, tot);
+    put(TAB_KE + J, after);
+    if (J < 2) put(TAB_F + J, next1);                      // block pairs (2, 0), (3, 1)
+    if (J == 0) put(TAB_F + 2, next2);                     // (3, 0)
+    dec = make_float2(ex2_approx(before.x + tot.x), ex2_approx(before.y + tot.y));
   }
-  // fused form: the ring slot must have been drained before the first write to the unit (all of them follow)
-  if (SUB && tid == 0 && ctx.slot_seen < ctx.slot_want)
-    poll_flag_ge(ctx.slot_flag, ctx.slot_want, ctx.abort_flag, ctx.g_abort, 20);
-  prep_sync<SUB>(ctx);
-
-  KT_TRACE(2);
+  if (GATED && t < PREP_UNIT(n_valid, it)) beta = __bfloat162float(__float2bfloat16(1.0f / (1.0f + __expf(-beta))));
+  // q and k rows: piece 4 m + tig of a row is in box m / 2 (expanded when they are used)
+  uint4 kraw[4], qraw[4];
+  tc::mbar_wait(&ctx.sh->qkv_bar, it & 1, ctx.abort_flag, 13);
+  float rk, rq;                                            // L2 normalisation of the rows
   {
-  // blocks of B beta above the diagonal are never computed: they are zeros in the workspace tile
-  if (tid < 192) {
-    const int blk = tid >> 5, e = tid & 31;             // 6 blocks x (16 rows x 2 chunks)
-    const int zi = blk < 3 ? 0 : (blk < 5 ? 1 : 2);
-    const int zj = blk < 3 ? blk + 1 : (blk < 5 ? blk - 1 : 3);
-    const int t = zi * 16 + (e >> 1), sc = zj * 2 + (e & 1);
-    *reinterpret_cast<uint4*>(unit + U_BB + (t >> 3) * SBO_K64 + sc * LBO + (t & 7) * 16) = make_uint4(0, 0, 0, 0);
-  }
-  }
-  // ---- stage 2: log-decay sums per channel.  x_t = inclusive sum INSIDE the 16-token block (in place
-  //      over g), block totals, then the per-block tables: e^{P_blk} (P = sum before the block),
-  //      G_last - P_blk, the decay between two block starts, and the chunk decay e^{G_last}. ----
-  {
-    const int c = tid & 127, b0 = (tid >> 7) * 2;
-    float a0 = 0.f, a1 = 0.f;
-    float* p0 = sG + (16 * b0) * P1_LD + c;
-    float* p1 = p0 + 16 * P1_LD;
-#pragma unroll
-    for (int t = 0; t < 16; t++) {
-      a0 += p0[t * P1_LD]; p0[t * P1_LD] = a0;
-      a1 += p1[t * P1_LD]; p1[t * P1_LD] = a1;
-    }
-    sTot[b0 * KD + c] = a0;
-    sTot[(b0 + 1) * KD + c] = a1;
-  }
-  prep_sync<SUB>(ctx);
-  // The k warps (threads 0-127, one channel each) build the per-block tables while the q warps scale their rows by
-  // e^{x}, which needs x only.
-  if (!is_q) {
-    const float t0s = sTot[tid], t1s = sTot[KD + tid], t2s = sTot[2 * KD + tid], t3s = sTot[3 * KD + tid];
-    const float P1v = t0s, P2v = P1v + t1s, P3v = P2v + t2s, GL = P3v + t3s;
-    // for Kt: decay from a token to the end of ITS block is e^{tot - x} = e^{-x} e^{tot} (each factor within fp32
-    // range for |x| <= 85), the decay over the LATER blocks is e^{G_last - P_next} (may underflow: then Kt is 0)
-    sEGLN[tid] = __expf(GL - P1v); sEGLN[KD + tid] = __expf(GL - P2v); sEGLN[2 * KD + tid] = __expf(GL - P3v); sEGLN[3 * KD + tid] = 1.f;
-    sETot[tid] = __expf(t0s); sETot[KD + tid] = __expf(t1s); sETot[2 * KD + tid] = __expf(t2s); sETot[3 * KD + tid] = __expf(t3s);
-    sEP[tid] = 1.f; sEP[KD + tid] = __expf(P1v); sEP[2 * KD + tid] = __expf(P2v); sEP[3 * KD + tid] = __expf(P3v);
-    // pair (ib, jb < ib) at index ib (ib - 1) / 2 + jb: e^{P_ib - P_jb}
-    sDD[tid] = __expf(t0s);
-    sDD[KD + tid] = __expf(t0s + t1s); sDD[2 * KD + tid] = __expf(t1s);
-    sDD[3 * KD + tid] = __expf(t0s + t1s + t2s); sDD[4 * KD + tid] = __expf(t1s + t2s); sDD[5 * KD + tid] = __expf(t2s);
-    reinterpret_cast<float*>(unit + U_DEC)[tid] = __expf(GL);
-  }
-  else {
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const float* xr = sG + (16 * ib + g8 + 8 * h) * P1_LD + 8 * tig;
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        const float4 x0 = *reinterpret_cast<const float4*>(xr + 32 * m), x1 = *reinterpret_cast<const float4*>(xr + 32 * m + 4);
-        v[h][8 * m + 0] *= __expf(fmaxf(x0.x, -85.f)); v[h][8 * m + 1] *= __expf(fmaxf(x0.y, -85.f));
-        v[h][8 * m + 2] *= __expf(fmaxf(x0.z, -85.f)); v[h][8 * m + 3] *= __expf(fmaxf(x0.w, -85.f));
-        v[h][8 * m + 4] *= __expf(fmaxf(x1.x, -85.f)); v[h][8 * m + 5] *= __expf(fmaxf(x1.y, -85.f));
-        v[h][8 * m + 6] *= __expf(fmaxf(x1.z, -85.f)); v[h][8 * m + 7] *= __expf(fmaxf(x1.w, -85.f));
-      }
-    }
-  }
-  prep_sync<SUB>(ctx);
-
-  KT_TRACE(3);
-  KT_TRACE(4);
-  // ---- stage 3: the q warps have read x; the k warps turn it into the RIGHT operand R[s][c] = k^_s e^{-x_s} (in
-  //      place, fp32: up to e^85) and scale their own rows by e^{x}; the q warps emit Q+ = q^ e^{G_t} (fp16 tile
-  //      rows 64..127) ----
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const int t = 16 * ib + g8 + 8 * h;
-    float* xr = sG + t * P1_LD + 8 * tig;
+    const uint8_t* qrow = smem + P1_QK + t * 128;
 #pragma unroll
     for (int m = 0; m < 4; m++) {
-      if (!is_q) {
-        float4 x0 = *reinterpret_cast<const float4*>(xr + 32 * m), x1 = *reinterpret_cast<const float4*>(xr + 32 * m + 4);
-        float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, r8[8];
+      const int off = (m >> 1) * P1_BOX + (((4 * (m & 1) + tig) ^ g8) << 4);
+      qraw[m] = *reinterpret_cast<const uint4*>(qrow + off);
+      kraw[m] = *reinterpret_cast<const uint4*>(qrow + 2 * P1_BOX + off);
+    }
+    float sk = 0.f, sq = 0.f;
 #pragma unroll
-        for (int e = 0; e < 8; e++) {
-          const float xc = fmaxf(xs[e], -85.f);
-          r8[e] = v[h][8 * m + e] * __expf(-xc);
-          v[h][8 * m + e] *= __expf(xc);
-        }
-        *reinterpret_cast<float4*>(xr + 32 * m) = make_float4(r8[0], r8[1], r8[2], r8[3]);
-        *reinterpret_cast<float4*>(xr + 32 * m + 4) = make_float4(r8[4], r8[5], r8[6], r8[7]);
+    for (int m = 0; m < 4; m++) {
+      const uint32_t kw[4] = {kraw[m].x, kraw[m].y, kraw[m].z, kraw[m].w}, qw[4] = {qraw[m].x, qraw[m].y, qraw[m].z, qraw[m].w};
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        sk = fmaf(bf16lo(kw[e]), bf16lo(kw[e]), fmaf(bf16hi(kw[e]), bf16hi(kw[e]), sk));
+        sq = fmaf(bf16lo(qw[e]), bf16lo(qw[e]), fmaf(bf16hi(qw[e]), bf16hi(qw[e]), sq));
+      }
+    }
+    sk += __shfl_xor_sync(0xffffffffu, sk, 1); sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+    sk += __shfl_xor_sync(0xffffffffu, sk, 2); sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+    rk = rsqrtf(sk + 1e-6f);
+    rq = rsqrtf(sq + 1e-6f);
+  }
+  // fused form: the ring slot must have been drained before the first write to the unit (all of them follow)
+  bool unpublished = SUB && it > 0;                        // warp 0: the flag of the unit before this one
+  if (SUB && warp == 0) {
+    const int want = PREP_UNIT(value, it) - KR;            // the slot held chunk value - 1 - KR
+    if (__shfl_sync(0xffffffffu, seen, 0) < want) {
+      if (unpublished) prep_publish(ctx, it - 1, ready, n_slots);   // before a wait: the chains may need that unit to get on
+      unpublished = false;
+      if (lane == 0) poll_flag_ge(consumed + PREP_UNIT(slot, it) * F_LINE, want, ctx.abort_flag, g_abort, 20);
+    }
+  }
+  prep_sync<SUB>(ctx);                                     // x and the tables are complete, q and k have been read
+
+  // ---- stage 2: every operand that is a row of this warp's tokens times a decay, and the products of the warp's tokens with
+  //      themselves and, odd warps, with the other eight of their block (TF32: e^{-x} needs the fp32 exponent range).  Left operands
+  //      k^ e^{x}, q^ e^{x}; right operand R = beta k^ e^{-x}; R' = R e^{tot} <= 1 is moved on to the start of each later block (fp16,
+  //      for the pairs of blocks) and to the end of the chunk (Kt) ----
+  uint32_t ah[4][8];                                       // the left operands in fp16, both at most 1 in magnitude
+  {
+    uint8_t* const out = PREP_OUT;
+    if (J == 3) *reinterpret_cast<float2*>(out + U_DEC + gc * 4) = dec;
+    // tiles of B beta above the diagonal are never computed: zeros
+    for (int i = lane; i < (7 - warp) * 8; i += 32)
+      *reinterpret_cast<uint4*>(out + U_BB + warp * SBO_K64 + (warp + 1) * LBO + i * 16) = make_uint4(0, 0, 0, 0);
+    float dg[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* tab = sTab + I * KD + 8 * tig;
+    const uint64_t beta2 = pack2(beta, beta), rk2 = pack2(rk, rk), rq2 = pack2(rq, rq);
+    uint8_t* ri = sRI + (t & 15) * 256;
+    const int sw = (t & 1) << 2;                           // 16-byte pieces of odd rows are swapped in halves of 64 bytes: conflict-free reads
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      float4* const xp0 = reinterpret_cast<float4*>(smem + P1_X + m * P1_BOX + t * 128 + (((2 * tig) ^ g8) << 4));
+      float4* const xp1 = reinterpret_cast<float4*>(smem + P1_X + m * P1_BOX + t * 128 + (((2 * tig + 1) ^ g8) << 4));
+      const float4 x0 = *xp0, x1 = *xp1;
+      const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+      const uint32_t kw[4] = {kraw[m].x, kraw[m].y, kraw[m].z, kraw[m].w}, qw[4] = {qraw[m].x, qraw[m].y, qraw[m].z, qraw[m].w};
+      uint64_t kl[4], ql[4], rb[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const uint64_t kn = mul2(pack2(bf16lo(kw[e]), bf16hi(kw[e])), rk2);
+        const uint64_t up = pack2(ex2_approx(xs[2 * e]), ex2_approx(xs[2 * e + 1]));
+        const uint64_t dn = pack2(ex2_approx(-xs[2 * e]), ex2_approx(-xs[2 * e + 1]));
+        rb[e] = mul2(mul2(kn, beta2), dn);
+        kl[e] = mul2(kn, up);
+        ql[e] = mul2(mul2(pack2(bf16lo(qw[e]), bf16hi(qw[e])), rq2), up);
+        ah[m][(e >> 1) * 4 + (e & 1) * 2] = pack_h2(kl[e]);
+        ah[m][(e >> 1) * 4 + (e & 1) * 2 + 1] = pack_h2(ql[e]);
+      }
+      uint32_t rt[8], a[4][4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        float r0, r1, k0, k1, q0, q1;
+        unpack2(rb[e], r0, r1);
+        unpack2(kl[e], k0, k1);
+        unpack2(ql[e], q0, q1);
+        rt[2 * e] = f2tf32(r0);
+        rt[2 * e + 1] = f2tf32(r1);
+        a[e][0] = f2tf32(k0); a[e][1] = f2tf32(q0); a[e][2] = f2tf32(k1); a[e][3] = f2tf32(q1);
+        mma_tf32(dg, a[e], rt[2 * e], rt[2 * e + 1]);
+      }
+      if (!odd) {                                          // for the odd warp of the block, in place of x
+        *reinterpret_cast<uint4*>(xp0) = make_uint4(rt[0], rt[1], rt[2], rt[3]);
+        *reinterpret_cast<uint4*>(xp1) = make_uint4(rt[4], rt[5], rt[6], rt[7]);
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&ctx.sh->pair_bar[I][m]);
       } else {
-        const float* ep = sEP + ib * KD + 32 * m + 8 * tig;
-        const float4 e0 = *reinterpret_cast<const float4*>(ep), e1 = *reinterpret_cast<const float4*>(ep + 4);
-        uint4 p;
-        p.x = pack_h2(v[h][8 * m + 0] * e0.x, v[h][8 * m + 1] * e0.y); p.y = pack_h2(v[h][8 * m + 2] * e0.z, v[h][8 * m + 3] * e0.w);
-        p.z = pack_h2(v[h][8 * m + 4] * e1.x, v[h][8 * m + 5] * e1.y); p.w = pack_h2(v[h][8 * m + 6] * e1.z, v[h][8 * m + 7] * e1.w);
-        *reinterpret_cast<uint4*>(unit + U_WQ + ((64 + t) >> 3) * SBO_K128 + (4 * m + tig) * LBO + (t & 7) * 16) = p;
+        tc::mbar_wait(&ctx.sh->pair_bar[I][m], it & 1, ctx.abort_flag, 14);
+        const uint4 r0 = *reinterpret_cast<const uint4*>(xp0 - 64), r1 = *reinterpret_cast<const uint4*>(xp1 - 64);   // eight rows up
+        mma_tf32(sb, a[0], r0.x, r0.y);
+        mma_tf32(sb, a[1], r0.z, r0.w);
+        mma_tf32(sb, a[2], r1.x, r1.y);
+        mma_tf32(sb, a[3], r1.z, r1.w);
+      }
+      uint64_t f[4], w[4];
+      const int piece = 4 * m + tig;
+      // K+ = k^ e^{G_t}: B operand; Q+ = q^ e^{G_t}: rows 64-127 of the unit's first tile
+      load_pairs(tab + TAB_EP * KD + 32 * m, f);
+#pragma unroll
+      for (int e = 0; e < 4; e++) w[e] = mul2(kl[e], f[e]);
+      *reinterpret_cast<uint4*>(sK + piece * P1_PIECE + warp * 128 + g8 * 16) = pack_piece(w);
+#pragma unroll
+      for (int e = 0; e < 4; e++) w[e] = mul2(ql[e], f[e]);
+      *reinterpret_cast<uint4*>(out + U_WQ + (8 + warp) * SBO_K128 + piece * LBO + g8 * 16) = pack_piece(w);
+      load_pairs(tab + TAB_ETOT * KD + 32 * m, f);
+#pragma unroll
+      for (int e = 0; e < 4; e++) rb[e] = mul2(rb[e], f[e]);
+      load_pairs(tab + TAB_KE * KD + 32 * m, f);
+#pragma unroll
+      for (int e = 0; e < 4; e++) w[e] = mul2(rb[e], f[e]);
+      *reinterpret_cast<uint4*>(out + U_KT + piece * 1024 + warp * 128 + g8 * 16) = pack_piece(w);
+      const int po = (piece ^ sw) << 4;
+      if (I < 3) *reinterpret_cast<uint4*>(ri + ((I + 1) * I / 2 + I) * 4096 + po) = pack_piece(rb);
+      if (I < 2) {
+        load_pairs(sTab + (TAB_F + I) * KD + 8 * tig + 32 * m, f);
+#pragma unroll
+        for (int e = 0; e < 4; e++) w[e] = mul2(rb[e], f[e]);
+        *reinterpret_cast<uint4*>(ri + ((I + 2) * (I + 1) / 2 + I) * 4096 + po) = pack_piece(w);
+      }
+      if (I < 1) {
+        load_pairs(sTab + (TAB_F + 2) * KD + 8 * tig + 32 * m, f);
+#pragma unroll
+        for (int e = 0; e < 4; e++) w[e] = mul2(rb[e], f[e]);
+        *reinterpret_cast<uint4*>(ri + 3 * 4096 + po) = pack_piece(w);
       }
     }
-  }
-  prep_sync<SUB>(ctx);
-
-  KT_TRACE(5);
-  // ---- stage 4: A and B on the warp-level tensor cores (TF32).  Every warp multiplies its own 16
-  //      rows (fragments from registers) with the R rows of the column blocks jb <= ib; R of an earlier
-  //      block is moved from its own reference P_jb to P_ib by the pair decay while it is loaded.  The
-  //      contraction runs over the channels in the order the registers hold them. ----
-  prep_ab_block(ib, v, is_q, sG, sDD, sBeta, sA, unit, g8, tig);
-  // Kt^T tile (rows = channels, K = tokens) from R: Kt[t][c] = beta_t R[t][c] e^{tot_blk} e^{G_last - P_next}, no
-  // exponentials; all eight warps, a thread = 8 tokens of one channel = one 16-byte piece of the tile
-  for (int i = tid; i < KD * (KC / 8); i += 256) {
-    const int c = i & 127, tg = i >> 7;
-    const float et = sETot[(tg >> 1) * KD + c], en = sEGLN[(tg >> 1) * KD + c];
-    float kt[8];
-#pragma unroll
-    for (int u8 = 0; u8 < 8; u8++) {
-      const int t = tg * 8 + u8;
-      kt[u8] = sBeta[t] * (sG[t * P1_LD + c] * et) * en;
-    }
-    uint4 p;
-    p.x = pack_h2(kt[0], kt[1]); p.y = pack_h2(kt[2], kt[3]); p.z = pack_h2(kt[4], kt[5]); p.w = pack_h2(kt[6], kt[7]);
-    *reinterpret_cast<uint4*>(unit + U_KT + (c >> 3) * SBO_K64 + tg * LBO + (c & 7) * 16) = p;
-  }
-  if (!is_q) {
-    // K+ = k^ e^{G_t}: first half of the [K+ | V] operand
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int t = 16 * ib + g8 + 8 * h;
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        const float* ep = sEP + ib * KD + 32 * m + 8 * tig;
-        const float4 e0 = *reinterpret_cast<const float4*>(ep), e1 = *reinterpret_cast<const float4*>(ep + 4);
-        uint4 p;
-        p.x = pack_h2(v[h][8 * m + 0] * e0.x, v[h][8 * m + 1] * e0.y); p.y = pack_h2(v[h][8 * m + 2] * e0.z, v[h][8 * m + 3] * e0.w);
-        p.z = pack_h2(v[h][8 * m + 4] * e1.x, v[h][8 * m + 5] * e1.y); p.w = pack_h2(v[h][8 * m + 6] * e1.z, v[h][8 * m + 7] * e1.w);
-        *reinterpret_cast<uint4*>(sKV + (4 * m + tig) * 1024 + (t >> 3) * 128 + (t & 7) * 16) = p;
-      }
+    // accumulator of a tile: N row t, columns s0, s0 + 1 (s0 = 8 * tile + 2 tig), then the same of B beta
+    float* nrow = sN + prep_n_row(t) + 2 * tig;
+    uint8_t* bbrow = out + U_BB + warp * SBO_K64 + g8 * 16 + tig * 4;
+    const int s = 2 * tig;                                 // N strictly lower, B lower including the diagonal
+    *reinterpret_cast<float2*>(nrow + 8 * warp) = make_float2(s < g8 ? dg[0] : 0.f, s + 1 < g8 ? dg[1] : 0.f);
+    *reinterpret_cast<uint32_t*>(bbrow + warp * LBO) = pack_h2(s <= g8 ? dg[2] : 0.f, s + 1 <= g8 ? dg[3] : 0.f);
+    if (odd) {
+      *reinterpret_cast<float2*>(nrow + 8 * (warp - 1)) = make_float2(sb[0], sb[1]);
+      *reinterpret_cast<uint32_t*>(bbrow + (warp - 1) * LBO) = pack_h2(sb[2], sb[3]);
     }
   }
-  __pipeline_wait_prior(0);                                 // v rows
-  prep_sync<SUB>(ctx);
-  KT_TRACE(6);
+  prep_sync<SUB>(ctx);                                     // right operands and the diagonal blocks of N are complete
 
-  // from here on sG is dead: the V half of sKV, sX and (after the conversion) sT take their place
-
-  // ---- stage 5: V -> B operand columns 128..255 (bf16 -> fp16), then the blocked inverse X = (I + N)^-1 in fp32
-  //      and its fp16 copy T as the A operand.  The conversion needs no barrier of its own: the inverse works on sA
-  //      and sX only, and the T operand is written (5c) after the barriers of the inverse. ----
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const int i = tid + 256 * j;
-    const int t = (i & 7) + ((i >> 7) << 3), cc = (i >> 3) & 15;
-    const uint4 vr = *reinterpret_cast<const uint4*>(sT + t * 256 + ((cc ^ (t & 7)) << 4));   // bf16 -> fp16
-    uint4 p;
-    p.x = pack_h2(bf16lo(vr.x), bf16hi(vr.x)); p.y = pack_h2(bf16lo(vr.y), bf16hi(vr.y));
-    p.z = pack_h2(bf16lo(vr.z), bf16hi(vr.z)); p.w = pack_h2(bf16lo(vr.w), bf16hi(vr.w));
-    *reinterpret_cast<uint4*>(sKV + (16 + cc) * 1024 + (t >> 3) * 128 + (t & 7) * 16) = p;
-  }
-  KT_TRACE(7);
-  // 5a: the four diagonal 16x16 blocks, one warp each, lane = column: x_r = delta - sum_{s<r} N[r][s] x_s
-  if (warp < 4 && lane < 16) {
-    const int ib = warp;
-    float x[16];
-#pragma unroll
-    for (int r = 0; r < 16; r++) {
-      float a0 = (r == lane) ? 1.f : 0.f, a1 = 0.f;
-      const float* nrow = sA + (ib * 16 + r) * P1_LDA + ib * 16;
-#pragma unroll
-      for (int s = 0; s < r; s++) {
-        if (s & 1) a1 = fmaf(-nrow[s], x[s], a1);
-        else a0 = fmaf(-nrow[s], x[s], a0);
-      }
-      x[r] = a0 + a1;
-    }
-#pragma unroll
-    for (int r = 0; r < 16; r++) sX[(ib * 16 + r) * P1_LDA + ib * 16 + lane] = x[r];
-  }
-  prep_sync<SUB>(ctx);
-  KT_TRACE(8);
-  // 5b: off-diagonal blocks.  M_im = X_ii N_im for the six pairs i > m (kept in the unused mirror block
-  //     (m, i) of sA), then by distance d = i - j: X_ij = - sum_{m=j}^{i-1} M_im X_mj.  One warp per
-  //     16x16 block, products on the warp-level tensor cores with split operands (fp32-class accuracy).
-  if (warp < 6) {
-    const int i = warp < 1 ? 1 : (warp < 3 ? 2 : 3), m = warp - (i * (i - 1)) / 2;
-    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    block16_mma(sX + (i * 16) * P1_LDA + i * 16, sA + (i * 16) * P1_LDA + m * 16, acc, lane);
-    block16_store(sA + (m * 16) * P1_LDA + i * 16, acc, 1.f, lane);
-  }
-  prep_sync<SUB>(ctx);
+  // ---- stage 3: the products with earlier blocks (fp16).  Odd warps: the inverse of their block's 16 x 16 diagonal of I + N;
+  //      even warps convert v meanwhile ----
+  if (SUB && warp == 0 && unpublished) prep_publish(ctx, it - 1, ready, n_slots);   // warp 0 has no earlier block
+  {
+    float* nrow = sN + prep_n_row(t) + 2 * tig;
+    uint8_t* bbrow = PREP_OUT + U_BB + warp * SBO_K64 + g8 * 16 + tig * 4;
+    const uint8_t* rbase = sRI + (I * (I - 1) / 2) * 4096 + g8 * 256;
+    const int sw = (g8 & 1) << 2;
 #pragma unroll 1
-  for (int d = 1; d < 4; d++) {
-    if (warp < 4 - d) {
-      const int i = d + warp, j = warp;
+    for (int jb = 0; jb < I; jb++) {
       float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      for (int m = j; m < i; m++)
-        block16_mma(sA + (m * 16) * P1_LDA + i * 16, sX + (m * 16) * P1_LDA + j * 16, acc, lane);
-      block16_store(sX + (i * 16) * P1_LDA + j * 16, acc, -1.f, lane);
+#pragma unroll
+      for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const uint4 r = *reinterpret_cast<const uint4*>(rbase + jb * 4096 + h * 2048 + (((4 * m + tig) ^ sw) << 4));
+          mma_f16_16816(acc[h], ah[m][0], ah[m][1], ah[m][2], ah[m][3], r.x, r.y);
+          mma_f16_16816(acc[h], ah[m][4], ah[m][5], ah[m][6], ah[m][7], r.z, r.w);
+        }
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        *reinterpret_cast<float2*>(nrow + 16 * jb + 8 * h) = make_float2(acc[h][0], acc[h][1]);
+        *reinterpret_cast<uint32_t*>(bbrow + (2 * jb + h) * LBO) = pack_h2(acc[h][2], acc[h][3]);
+      }
     }
-    prep_sync<SUB>(ctx);
   }
-  KT_TRACE(9);
-  // 5c: T = fp16(X) as the K-major A operand (K = 64): lanes = 8 rows x 4 chunks.  Rows 64..127 of the
-  //     operand are never produced: zero, so the unused TMEM lanes stay finite
-  for (int i = tid; i < 8192 / 16; i += 256) reinterpret_cast<uint4*>(sT + 8192)[i] = make_uint4(0, 0, 0, 0);
-  for (int i = tid; i < KC * (KC / 8); i += 256) {
-    const int t = (i & 7) + ((i >> 6) << 3), jc = (i >> 3) & 7;
-    uint4 p = make_uint4(0, 0, 0, 0);                      // blocks above the diagonal are never computed: zeros
-    if ((jc >> 1) <= (t >> 4)) {
-      const float4 v0 = *reinterpret_cast<const float4*>(sX + t * P1_LDA + jc * 8);
-      const float4 v1 = *reinterpret_cast<const float4*>(sX + t * P1_LDA + jc * 8 + 4);
-      p.x = pack_h2(v0.x, v0.y); p.y = pack_h2(v0.z, v0.w); p.z = pack_h2(v1.x, v1.y); p.w = pack_h2(v1.z, v1.w);
+  if (odd) {
+    // inverse of the unit lower triangular 16 x 16 block, lane = column: x_r = delta - sum_{s<r} N[r][s] x_s
+    if (lane < 16) {
+      float x[16];
+      const float* nd = sN + prep_n_row(16 * I) + 16 * I;
+      const int ld = I < 2 ? 36 : 68;
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        float a0 = (r == lane) ? 1.f : 0.f, a1 = 0.f;
+#pragma unroll
+        for (int s = 0; s < r; s += 4) {
+          const float4 n4 = *reinterpret_cast<const float4*>(nd + r * ld + s);
+          const float nn[4] = {n4.x, n4.y, n4.z, n4.w};
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            if (s + u >= r) break;
+            if (u & 1) a1 = fmaf(-nn[u], x[s + u], a1);
+            else a0 = fmaf(-nn[u], x[s + u], a0);
+          }
+        }
+        x[r] = a0 + a1;
+      }
+      float* xi = sX + prep_inv_at(I) + lane;
+#pragma unroll
+      for (int r = 0; r < 16; r++) xi[r * P1_LDX] = x[r];
     }
-    *reinterpret_cast<uint4*>(sT + (t >> 3) * SBO_K64 + jc * LBO + (t & 7) * 16) = p;
+  } else {
+    // bf16 -> fp16 in place.  (The product T V needs both operands in ONE 16-bit format: a kind::f16 product of an fp16 T with bf16
+    // rows is rejected by the hardware as an illegal instruction.)
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      uint4* vp = reinterpret_cast<uint4*>(smem + P1_V) + I * 32 + lane + 128 * j;
+      const uint4 vr = *vp;
+      *vp = make_uint4(pack_h2(bf16lo(vr.x), bf16hi(vr.x)), pack_h2(bf16lo(vr.y), bf16hi(vr.y)), pack_h2(bf16lo(vr.z), bf16hi(vr.z)),
+                       pack_h2(bf16lo(vr.w), bf16hi(vr.w)));
+    }
+  }
+  prep_sync<SUB>(ctx);                                     // N and the diagonal inverses are complete, the right operands have been read
+
+  // ---- stage 4: X = (I + N)^-1 below its diagonal blocks, and its fp16 copy T as the K-major A operand (K = 64).  First
+  //      P_mj = N_mj X_jj in place of N_mj, one warp per block, while two warps write the diagonal of T and the zeros above it;
+  //      then one warp per row of blocks.  Rows 64-127 of the operand are whatever the memory holds: their lanes of the product
+  //      are never read ----
+  if (warp < 6) {
+    const int m = warp < 1 ? 1 : (warp < 3 ? 2 : 3), j = warp - (m * (m - 1)) / 2, ld = m < 2 ? 36 : 68;
+    float* nb = sN + prep_n_row(16 * m) + 16 * j;
+    Frag16 L;
+    L.load(nb, ld, lane);
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    block16_mma(L, sX + prep_inv_at(j), P1_LDX, acc, lane);
+    __syncwarp();
+#pragma unroll
+    for (int nt = 0; nt < 2; nt++) {
+      *reinterpret_cast<float2*>(nb + g8 * ld + 8 * nt + 2 * tig) = make_float2(acc[nt][0], acc[nt][1]);
+      *reinterpret_cast<float2*>(nb + (g8 + 8) * ld + 8 * nt + 2 * tig) = make_float2(acc[nt][2], acc[nt][3]);
+    }
+  } else {
+    const int e = tid - 192;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {                          // 4 blocks x 16 rows x 2 pieces
+      const int i = e + 64 * q, blk = i >> 5, r = (i & 7) + ((i >> 4) & 1) * 8, h = (i >> 3) & 1;
+      const float* xi = sX + prep_inv_at(blk) + r * P1_LDX + 8 * h;
+      const float4 v0 = *reinterpret_cast<const float4*>(xi), v1 = *reinterpret_cast<const float4*>(xi + 4);
+      *reinterpret_cast<uint4*>(sT + (2 * blk + (r >> 3)) * SBO_K64 + (2 * blk + h) * LBO + (r & 7) * 16) =
+          make_uint4(pack_h2(v0.x, v0.y), pack_h2(v0.z, v0.w), pack_h2(v1.x, v1.y), pack_h2(v1.z, v1.w));
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++) {                          // 6 blocks x 16 rows x 2 pieces
+      const int i = e + 64 * q, blk = i >> 5, zi = blk < 3 ? 0 : (blk < 5 ? 1 : 2), zj = blk < 3 ? blk + 1 : (blk < 5 ? blk - 1 : 3);
+      *reinterpret_cast<uint4*>(sT + (2 * zi + ((i >> 4) & 1)) * SBO_K64 + (2 * zj + ((i >> 3) & 1)) * LBO + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+    }
+  }
+  prep_sync<SUB>(ctx);
+  if (warp == 1) prep_inverse_row<1>(sN, sX, sT, lane);
+  else if (warp == 2) prep_inverse_row<2>(sN, sX, sT, lane);
+  else if (warp == 3) prep_inverse_row<3>(sN, sX, sT, lane);
+  else if (tid == 192) {
+    // the inputs of a unit about one wave of workers ahead, pulled into L2
+    PrepDesc u;
+    make_unit(it + 2, u);
+    ctx.sh->unit[(it + 2) & 3] = u;
+    if (u.n_valid > 0) {
+#pragma unroll
+      for (int m = 0; m < 4; m++) prep_tma_l2(map_g, u.head * KD + 32 * m, u.t0, u.b);
+#pragma unroll
+      for (int m = 0; m < 6; m++) prep_tma_l2(map_qkv, ((m >> 1) * H + u.head) * KD + 64 * (m & 1), u.t0, u.b);
+    }
   }
   tc::fence_async_smem();
   tc::fence_before_sync();
   prep_sync<SUB>(ctx);
   tc::fence_after_sync();
 
-  KT_TRACE(10);
-  // ---- stage 6: [W | Uloc] = T [K+ | V] : tcgen05 M128 N256 K64, fp16 in, fp32 TMEM accumulators ----
-  const uint32_t tmem = ctx.tmem;
+  // ---- stage 5: [W | Uloc] = T [K+ | V] : tcgen05 M128 N128 K64 twice, fp16 in, fp32 TMEM accumulators ----
   if (tid == 0) {
-    const uint32_t idesc = tc::make_idesc(128, 256, tc::FMT_F16, tc::FMT_F16, false, true);
-    const uint32_t a_addr = tc::smem_u32(sT), b_addr = tc::smem_u32(sKV);
+    const uint32_t idesc = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, false, true);
+    const uint32_t a_addr = tc::smem_u32(sT), k_addr = tc::smem_u32(sK);
+    const uint64_t vd = tc::make_sdesc_sw128(tc::smem_u32(smem + P1_V), P1_BOX, 1024);
 #pragma unroll
-    for (int kk = 0; kk < KC / 16; kk++) {
-      const uint64_t ad = tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64);
-      const uint64_t bd = tc::make_sdesc(b_addr + kk * 2 * 128, 128, 1024);
-      tc::mma_f16(tmem, ad, bd, idesc, kk > 0);
-    }
-    tc::mma_commit(ctx.bar);
+    for (int kk = 0; kk < KC / 16; kk++)
+      tc::mma_f16(tmem, tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64), tc::make_sdesc(k_addr + kk * 2 * 128, 128, P1_PIECE), idesc, kk > 0);
+#pragma unroll
+    for (int kk = 0; kk < KC / 16; kk++)
+      tc::mma_f16(tmem + KD, tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64), tc::sdesc_advance(vd, kk * 2048), idesc, kk > 0);
+    tc::mma_commit(&ctx.sh->mma_bar);
   }
-  // one warp polls the barrier (with a back-off); the others park at the block barrier instead of spending
-  // issue slots that the other CTA of this SM can use
-  if (warp == 0) tc::mbar_wait<64>(ctx.bar, ctx.bar_parity, ctx.abort_flag, 1);
-  prep_sync<SUB>(ctx);
-  const bool ok = *ctx.abort_flag == 0;
+  if (tid == 96) prep_fetch_g(ctx, it + 1, map_g);         // x is free
+  __syncwarp();
+  const bool ok = tc::mbar_wait(&ctx.sh->mma_bar, it & 1, ctx.abort_flag, 1);
+  if (tid == 96) prep_fetch_qkv(ctx, it + 1, map_qkv, H);  // and so are T, N, K+ and V
   tc::fence_after_sync();
-  KT_TRACE(11);
-  // ---- stage 7: epilogue. Lanes 0-63 are the tokens; warps 0,1 take W, warps 4,5 take Uloc ----
-  if (ok && (warp & 3) < 2) {
-    const int t = (warp & 3) * 32 + lane;
-    const bool second = warp >= 4;
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (second ? 128 : 0);
+  // ---- stage 6: epilogue. Lanes 0-63 are the tokens; warps 0,1 take W, warps 4,5 take Uloc ----
+  if ((warp & 3) < 2) {
+    if (ok) {
+      uint8_t* const unit = PREP_OUT;
+      const int et = (warp & 3) * 32 + lane;
+      const bool second = warp >= 4;
+      const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (second ? 128 : 0);
 #pragma unroll
-    for (int c0 = 0; c0 < KD; c0 += 32) {
-      uint32_t r[32];
-      tc::tmem_ld32(lane_addr + c0, r);
-      tc::tmem_ld_wait();
-      uint4 p[4];
+      for (int c0 = 0; c0 < KD; c0 += 32) {
+        uint32_t r[32];
+        tc::tmem_ld32(lane_addr + c0, r);
+        tc::tmem_ld_wait();
+        uint4 p[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        p[u].x = pack_h2(__uint_as_float(r[8 * u + 0]), __uint_as_float(r[8 * u + 1]));
-        p[u].y = pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3]));
-        p[u].z = pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5]));
-        p[u].w = pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7]));
-      }
-      if (!second) {
+        for (int u = 0; u < 4; u++) {
+          p[u].x = pack_h2(__uint_as_float(r[8 * u + 0]), __uint_as_float(r[8 * u + 1]));
+          p[u].y = pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3]));
+          p[u].z = pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5]));
+          p[u].w = pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7]));
+        }
+        if (!second) {                                     // -W
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-          *reinterpret_cast<uint4*>(unit + U_WQ + (t >> 3) * SBO_K128 + (c0 / 8 + u) * LBO + (t & 7) * 16) = p[u];
-      } else {
-        uint4* dst = reinterpret_cast<uint4*>(unit + U_UL + (c0 / KNV) * (KC * KNV * 2) + t * (KNV * 2));
+          for (int u = 0; u < 4; u++)
+            *reinterpret_cast<uint4*>(unit + U_WQ + (et >> 3) * SBO_K128 + (c0 / 8 + u) * LBO + (et & 7) * 16) =
+                make_uint4(p[u].x ^ 0x80008000u, p[u].y ^ 0x80008000u, p[u].z ^ 0x80008000u, p[u].w ^ 0x80008000u);
+        } else {
 #pragma unroll
-        for (int u = 0; u < 4; u++) dst[u] = p[u];
+          for (int u = 0; u < 4; u++) *reinterpret_cast<uint4*>(unit + U_UL + (c0 / 8 + u) * 1024 + (et ^ 8) * 16) = p[u];
+        }
       }
     }
+    tc::fence_before_sync();
+    if (SUB && warp != 0) asm volatile("bar.arrive %0, 128;" ::"r"(ctx.bar_id + 2) : "memory");
   }
-  tc::fence_before_sync();
-  prep_sync<SUB>(ctx);
-  KT_TRACE(12);
 }
 
 template <bool GATED>
 __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
-    const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ g,
-    const void* __restrict__ beta_in, uint8_t* __restrict__ ws, int seqlen, int H,
-    int n_chunks, int prefetch_dist, int* __restrict__ status, const float* __restrict__ dt_bias,
-    const float* __restrict__ a_log, float lower_bound) {
+    const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
+    uint8_t* __restrict__ ws, int seqlen, int H, int n_chunks, int prefetch_dist, int* __restrict__ status,
+    const float* __restrict__ dt_bias, const float* __restrict__ a_log, float lower_bound) {
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ uint64_t bar;
+  __shared__ PrepShared sh;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   const int tid = threadIdx.x;
-  // heads are the fastest grid dimension: CTAs that run together read the same tokens, i.e. whole
-  // contiguous rows of the activations
-  const int head = blockIdx.x, chunk = blockIdx.y, b = blockIdx.z;
-  // units are chunk-major: the CTAs that run together (same chunks, all heads) touch adjacent units, in
-  // this kernel and in the scan, so their traffic spreads over all memory channels
-  uint8_t* unit = ws + (((size_t)b * n_chunks + chunk) * H + head) * U_BYTES;
+  // heads are the fastest grid dimension: CTAs that run together read the same tokens, i.e. whole contiguous rows of the
+  // activations.  Units are chunk-major: the CTAs that run together (same chunks, all heads) touch adjacent units, in
+  // this kernel and in the scan, so their traffic spreads over all memory channels.
+  auto describe = [&](int head, int chunk, PrepDesc& u) {
+    u.b = blockIdx.z;
+    u.t0 = chunk * KC;
+    u.tok0 = u.b * seqlen + u.t0;
+    u.n_valid = chunk < n_chunks ? min(KC, seqlen - u.t0) : 0;
+    u.head = head;
+    u.unit = (u.b * n_chunks + chunk) * H + head;
+  };
+  PrepCtx ctx;
+  ctx.smem = smem + ((1024u - (tc::smem_u32(smem) & 1023u)) & 1023u);
+  ctx.sh = &sh; ctx.abort_flag = &abort_flag; ctx.tid = tid; ctx.bar_id = 0;
   if (tid == 0) {
-    tc::mbar_init(&bar, 1);
+    prep_init(sh);
     tc::mbar_fence_init();
     abort_flag = 0;
+    describe(blockIdx.x, blockIdx.y, sh.unit[0]);
+    sh.unit[1].n_valid = 0;                                // a CTA has one unit
+    pdl_wait();
+    prep_fetch_g(ctx, 0, &map_g);
+    prep_fetch_qkv(ctx, 0, &map_qkv, H);
   }
   if (tid < 32) tc::tmem_alloc(&tmem_slot, 256);
   pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  // the CTA that runs `prefetch_dist` blocks later (blocks are scheduled in linear order, heads fastest)
-  const long long lin = (long long)blockIdx.y * H + blockIdx.x + prefetch_dist;
-  const int pchunk = (int)(lin / H);
-  PrepCtx ctx{smem, &bar, 0u, &abort_flag, tmem_slot, tid, 0, false, nullptr, 0, 0, nullptr};
-  prep_unit<GATED, false>(ctx, qkv, g, beta_in, unit, seqlen, H, head, chunk, b, (int)(lin % H),
-                          (prefetch_dist > 0 && pchunk < n_chunks) ? pchunk : -1, dt_bias, a_log, lower_bound);
+  prep_unit<GATED, false>(ctx, 0, &map_qkv, &map_g, beta_in, ws, H, dt_bias, a_log, lower_bound, tmem_slot, nullptr, nullptr, nullptr, 0,
+                          [&](int, PrepDesc& u) {
+    // the unit whose inputs it pulls into L2 is the one of the CTA that runs `prefetch_dist` blocks later (blocks are
+    // scheduled in linear order, heads fastest)
+    const long long lin = (long long)blockIdx.y * H + blockIdx.x + prefetch_dist;
+    describe((int)(lin % H), (int)min(lin / H, (long long)n_chunks), u);
+  });
+  __syncthreads();
   if (tid < 32) tc::tmem_dealloc(tmem_slot, 256);
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
 }
@@ -721,17 +803,29 @@ __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
 // =================================================================================================
 // kernel 2: sequential scan over the chunks of one (batch, head, value slice)
 // =================================================================================================
+// fp16 A operand [I ; 0] (128 rows, K = 64) without storing it: its core matrix (i, j) depends on i - j only, so 23 core
+// matrices, one of them the identity, serve all of them with 128 bytes as both strides.  The two core matrices of a K16 step then
+// come in falling j, which is why Uloc keeps its 8-token blocks in swapped pairs.
+constexpr uint32_t ID_BYTES = 23 * 128;
+__device__ __forceinline__ void write_identity(uint8_t* dst, int tid, int nthreads) {
+  for (int i = tid; i < (int)ID_BYTES / 16; i += nthreads) {
+    const int r = i & 7;                                    // core matrix 7 is the identity, the others are zeros
+    const uint32_t one = (i >> 3) == 7 ? 0x3C00u << (16 * (r & 1)) : 0u;
+    reinterpret_cast<uint4*>(dst)[i] = make_uint4(r >> 1 == 0 ? one : 0u, r >> 1 == 1 ? one : 0u, r >> 1 == 2 ? one : 0u, r >> 1 == 3 ? one : 0u);
+  }
+}
+
 constexpr uint32_t S_WQ = 0;              // 32768
-constexpr uint32_t S_BB = 32768;          // 16384: rows 0-63 zero (never overwritten), rows 64-127 = B beta
-constexpr uint32_t S_KT = 49152;          // 16384
-constexpr uint32_t S_UL = 65536;          // 4096
-constexpr uint32_t S_DEC = 69632;         // 512
-constexpr uint32_t S_STAGE = 70144;
-constexpr uint32_t S_TX = 32768 + 8192 + 16384 + 4096 + 512;  // bytes landing per stage
+constexpr uint32_t S_BB = 32768;          // 8192
+constexpr uint32_t S_KT = 40960;          // 16384
+constexpr uint32_t S_UL = 57344;          // 4096
+constexpr uint32_t S_DEC = 61440;         // 512
+constexpr uint32_t S_STAGE = 61952;
 constexpr int S_NSTAGE = 3;               // operand stages in flight: two chunks of lead time for the bulk copies
 constexpr uint32_t P2_S = S_NSTAGE * S_STAGE;  // fp16 B operand: state slice [128 k][32], MN-major, 8 KB
 constexpr uint32_t P2_U = P2_S + 8192;    // fp16 B operand: U [64 tokens][32], MN-major, 4 KB
-constexpr uint32_t P2_SMEM = P2_U + 4096;
+constexpr uint32_t P2_ID = P2_U + 4096;   // [I ; 0]
+constexpr uint32_t P2_SMEM = P2_ID + ID_BYTES;
 
 __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
     const uint8_t* __restrict__ ws, float* __restrict__ state, __nv_bfloat16* __restrict__ out,
@@ -744,7 +838,7 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5;
   const int vs = blockIdx.x, head = blockIdx.y, b = blockIdx.z;
   const int v0 = vs * KNV;
   const uint8_t* unit0 = ws + ((size_t)b * n_chunks * H + head) * U_BYTES;   // unit of chunk c: + c * H * U_BYTES
@@ -756,10 +850,7 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
     abort_flag = 0;
   }
   if (warp == 0) tc::tmem_alloc(&tmem_slot, 128);
-  // zero halves of the [0 ; B beta] operands
-  for (int i = tid; i < 8192 / 16; i += 128) {
-    for (int st_i = 0; st_i < S_NSTAGE; st_i++) reinterpret_cast<uint4*>(smem + st_i * S_STAGE + S_BB)[i] = make_uint4(0, 0, 0, 0);
-  }
+  write_identity(smem + P2_ID, tid, 128);
   pdl_wait();
   // state slice: thread = k row, 32 fp32 values in registers; fp16 copy as the B operand
   const int slot = slots ? slots[b] : b;
@@ -792,9 +883,9 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
     uint8_t* stg = smem + (chunk % S_NSTAGE) * S_STAGE;
     const uint8_t* u = unit0 + (size_t)chunk * H * U_BYTES;
     uint64_t* bar = &full_bar[chunk % S_NSTAGE];
-    tc::mbar_arrive_expect_tx(bar, S_TX);
+    tc::mbar_arrive_expect_tx(bar, S_STAGE);
     tc::bulk_g2s(stg + S_WQ, u + U_WQ, 32768, bar);
-    tc::bulk_g2s(stg + S_BB + 8192, u + U_BB, 8192, bar);
+    tc::bulk_g2s(stg + S_BB, u + U_BB, 8192, bar);
     tc::bulk_g2s(stg + S_KT, u + U_KT, 16384, bar);
     tc::bulk_g2s(stg + S_UL, u + U_UL + vs * (KC * KNV * 2), 4096, bar);
     tc::bulk_g2s(stg + S_DEC, u + U_DEC, 512, bar);
@@ -804,7 +895,8 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
   }
 
   const uint32_t idesc = tc::make_idesc(128, KNV, tc::FMT_F16, tc::FMT_F16, false, true);
-  const uint32_t s_addr = tc::smem_u32(smem + P2_S), u_addr = tc::smem_u32(smem + P2_U);
+  const uint32_t idesc_kt = tc::make_idesc(128, KNV, tc::FMT_F16, tc::FMT_F16, true, true);   // Kt^T: channels contiguous
+  const uint32_t s_addr = tc::smem_u32(smem + P2_S), u_addr = tc::smem_u32(smem + P2_U), id_addr = tc::smem_u32(smem + P2_ID);
   // The contractions are issued by the whole of warp 0 with one elected lane (descriptors stay warp-uniform for the
   // compiler: ~41 instead of ~47 cycles per M128 N32 product, see tc05.cuh).  Every wait of this kernel is executed
   // by all lanes, so warp 0 stays converged from one contraction to the next.
@@ -852,13 +944,19 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
     KS_TRACE(0, chunk);
     bool ok = tc::mbar_wait(&full_bar[sidx], (chunk / S_NSTAGE) & 1, &abort_flag, 2);
     KS_TRACE(1, chunk);
-    // ---- [W ; Q+] S0 -> D1 (128 x 32) ----
+    // ---- D1 (128 x 32) = [I ; 0] Uloc (exact) + [-W ; Q+] S0: rows 0-63 are U ----
     if (issue_warp) {
+#pragma unroll
+      for (int kk = 0; kk < KC / 16; kk++) {
+        const uint64_t ad = tc::make_sdesc(id_addr + (6 - 2 * kk) * 128, 128, 128);
+        const uint64_t bd = tc::make_sdesc(stg_addr + S_UL + kk * 2 * 128, 128, 1024);
+        tc::mma_f16_if(leader, d1, ad, bd, idesc, kk > 0);
+      }
 #pragma unroll
       for (int kk = 0; kk < KD / 16; kk++) {
         const uint64_t ad = tc::make_sdesc(stg_addr + S_WQ + kk * 2 * LBO, LBO, SBO_K128);
         const uint64_t bd = tc::make_sdesc(s_addr + kk * 2 * 128, 128, 2048);
-        tc::mma_f16_if(leader, d1, ad, bd, idesc, kk > 0);
+        tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
       }
       tc::mma_commit_if(leader, &mma_bar);
     }
@@ -868,29 +966,17 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
     mma_parity ^= 1;
     tc::fence_after_sync();
     KS_TRACE(2, chunk);
-    // ---- U = Uloc - W S0 (token rows = TMEM lanes 0-63) ----
+    // ---- U (token rows = TMEM lanes 0-63) as the next operand ----
     if (warp < 2) {
-      const int t = tid;
       uint32_t r[32];
       tc::tmem_ld32(d1 + ((uint32_t)(warp * 32) << 16), r);
       tc::tmem_ld_wait();
-      const uint4* ul = reinterpret_cast<const uint4*>(stg + S_UL + t * (KNV * 2));
-      uint8_t* urow = smem + P2_U + (t >> 3) * 128 + (t & 7) * 16;  // off(k=t, n) = (n/8)*1024 + ...
+      uint8_t* urow = smem + P2_U + tid * 16;               // off(k=t, n) = (n/8)*1024 + t*16 + (n%8)*2
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const uint4 lv = ul[u];
-        const __half2* lh = reinterpret_cast<const __half2*>(&lv);
-        float uu[8];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float2 f = __half22float2(lh[e]);
-          uu[2 * e] = f.x - __uint_as_float(r[8 * u + 2 * e]);
-          uu[2 * e + 1] = f.y - __uint_as_float(r[8 * u + 2 * e + 1]);
-        }
-        uint4 p;
-        p.x = pack_h2(uu[0], uu[1]); p.y = pack_h2(uu[2], uu[3]); p.z = pack_h2(uu[4], uu[5]); p.w = pack_h2(uu[6], uu[7]);
-        *reinterpret_cast<uint4*>(urow + u * 1024) = p;
-      }
+      for (int u = 0; u < 4; u++)
+        *reinterpret_cast<uint4*>(urow + u * 1024) =
+            make_uint4(pack_h2(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])), pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])),
+                       pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])), pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])));
     }
     tc::fence_async_smem();
     tc::fence_before_sync();
@@ -901,14 +987,14 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
     if (issue_warp) {
 #pragma unroll
       for (int kk = 0; kk < KC / 16; kk++) {
-        const uint64_t ad = tc::make_sdesc(stg_addr + S_KT + kk * 2 * LBO, LBO, SBO_K64);
+        const uint64_t ad = tc::make_sdesc(stg_addr + S_KT + kk * 2 * 128, 128, 1024);
         const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
-        tc::mma_f16_if(leader, d2, ad, bd, idesc, kk > 0);
+        tc::mma_f16_if(leader, d2, ad, bd, idesc_kt, kk > 0);
       }
       tc::mma_commit_if(leader, &mma_bar);
 #pragma unroll
       for (int kk = 0; kk < KC / 16; kk++) {
-        const uint64_t ad = tc::make_sdesc(stg_addr + S_BB + kk * 2 * LBO, LBO, SBO_K64);
+        const uint64_t ad = tc::make_sdesc(stg_addr + S_BB - 8192 + kk * 2 * LBO, LBO, SBO_K64);   // rows 0-63: whatever precedes the tile
         const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
         tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
       }
@@ -983,41 +1069,36 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
 // bound (about a second); on expiry they record HK_ERR_TIMEOUT, raise the launch-wide abort word and finish without
 // waiting again.  All CTAs must be resident at once: the launch is cooperative and sized to the SM count.
 // =================================================================================================
-constexpr int KR = 16;                                    // ring slots (chunks) per chain
-constexpr int F_NSTAGE = 2;                               // the ring protocol of the chain CTA is written for two stages
-constexpr uint32_t F_WQ = 0;                              // 32768
-constexpr uint32_t F_BB = 32768;                          // 16384: rows 0-63 zero (never overwritten), rows 64-127 = B beta
-constexpr uint32_t F_KT = 49152;                          // 16384
-constexpr uint32_t F_UL = 65536;                          // 16384: Uloc as [4 column blocks][64 tokens][32]
-constexpr uint32_t F_DEC = 81920;                         // 512
-constexpr uint32_t F_STAGE = 82432;
+constexpr int F_NSTAGE = 2;                               // operand stages of the chain CTA: a unit each, laid out as in the ring
+constexpr uint32_t F_STAGE = U_BYTES;
 constexpr uint32_t F_S = F_NSTAGE * F_STAGE;              // fp16 B operand: state [128 k][128 v], MN-major, 32 KB
 constexpr uint32_t F_U = F_S + 32768;                     // fp16 B operand: U [64 tokens][128 v], MN-major, 16 KB
 constexpr uint32_t F_O = F_U + 16384;                     // bf16 output rows of one chunk: two swizzled 8 KB boxes for the tiled
                                                           // stores, or plain [64 tokens][256 B] rows when the kernel stores itself
 constexpr uint32_t F_OPITCH = 256;
-constexpr uint32_t F_SMEM_SCAN = F_O + KC * F_OPITCH + 1024;   // + slack to start the tiles at a 1 KB boundary
+constexpr uint32_t F_ID = F_O + KC * F_OPITCH;           // [I ; 0]
+constexpr uint32_t F_SMEM_SCAN = F_ID + ID_BYTES + 1024;     // + slack to start the tiles at a 1 KB boundary
 static_assert(F_O % 1024 == 0 && KC * F_OPITCH >= 16384, "the output tile holds two 8 KB swizzled boxes");
-constexpr uint32_t F_SMEM = F_SMEM_SCAN > 2 * P1_SMEM ? F_SMEM_SCAN : 2 * P1_SMEM;
-static_assert(U_KT + 16384 == U_UL && U_UL + 16384 == U_DEC && F_KT + 16384 == F_UL && F_UL + 16384 == F_DEC,
-              "Kt^T, Uloc and the decay row travel as one copy");
-constexpr int F_FLAG_INTS = 16;                           // [0] launch-wide abort word; the flag arrays follow
+constexpr uint32_t F_SMEM = F_SMEM_SCAN > 2 * P1_SMEM + 1024 ? F_SMEM_SCAN : 2 * P1_SMEM + 1024;
 
 template <bool GATED>
 __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
-    const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ g, const void* __restrict__ beta_in,
+    const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
     uint8_t* __restrict__ ring, int* __restrict__ flags, float* __restrict__ state, __nv_bfloat16* __restrict__ out,
     float* __restrict__ out_f32, int seqlen, int H, int n_chunks, int n_jobs, int n_slots, const int* __restrict__ slots,
     float scale, int* __restrict__ status, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
     float lower_bound, const __grid_constant__ CUtensorMap tmap_out, int use_tma_out) {
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ uint64_t full_bar[F_NSTAGE];
-  // chain: one barrier per contraction group, each completing once per chunk (parity = chunk & 1); the output warps
-  // never wait for the first one, which a barrier shared by both groups would not allow (a skipped phase aliases)
-  __shared__ uint64_t mma_bar;       // chain: [W;Q+] S0;       preparation worker 0: its product
-  __shared__ uint64_t mma2_bar;      // chain: Kt^T U (state path)
-  __shared__ uint64_t out_bar;       // chain: (B beta) U;      preparation worker 1: its product
-  __shared__ uint64_t u_bar;         // chain: the 256 token-row threads have written U (count 256)
+  __shared__ uint64_t wu_bar[F_NSTAGE];    // -W, Q+ and Uloc of a stage have landed
+  __shared__ uint64_t kb_bar[F_NSTAGE];    // B beta, Kt^T and the decays
+  // chain: barriers of a chunk, two of most kinds by chunk parity, so that a warp that is held up may be a chunk behind
+  __shared__ uint64_t mma_bar[2];    // U and Q+ S0 are complete
+  __shared__ uint64_t mma2_bar;      // Kt^T U (state path) is complete
+  __shared__ uint64_t out_bar[2];    // (B beta) U is complete, and with it every product of the chunk (by chunk parity)
+  __shared__ uint64_t u_bar;         // the 256 token-row threads have written U
+  __shared__ uint64_t s_bar[2];      // the 256 state threads have written the state operand
+  __shared__ uint64_t d1_bar[2];     // the two output warps have read this half of D1
+  __shared__ PrepShared prep[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -1028,16 +1109,23 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
   int* g_abort = flags;
   // A chain CTA ("slot") walks n_jobs / n_slots chains one after the other: its running chunk number v counts through
   // all of them (chain v / n_chunks of the slot, chunk v % n_chunks), and ring, flags and barrier parities go by v.
-  int* ready = flags + F_FLAG_INTS;                        // [n_slots][KR]
-  int* consumed = ready + (size_t)n_slots * KR;            // [n_slots]
+  int* ready = flags + F_FLAG_INTS;                        // [n_slots][KR], a line per slot
+  int* consumed = ready + (size_t)n_slots * F_LINE;        // [n_slots], a line each
   const int n_virtual = (n_jobs / n_slots) * n_chunks;     // chunks a slot walks
 
   if (tid == 0) {
-    for (int i = 0; i < F_NSTAGE; i++) tc::mbar_init(&full_bar[i], 1);
-    tc::mbar_init(&mma_bar, 1);
+    for (int i = 0; i < 2; i++) {
+      tc::mbar_init(&wu_bar[i], 1);
+      tc::mbar_init(&kb_bar[i], 1);
+      tc::mbar_init(&mma_bar[i], 1);
+      tc::mbar_init(&out_bar[i], 1);
+      tc::mbar_init(&s_bar[i], 256);
+      tc::mbar_init(&d1_bar[i], 2);
+    }
     tc::mbar_init(&mma2_bar, 1);
-    tc::mbar_init(&out_bar, 1);
     tc::mbar_init(&u_bar, 256);
+    prep_init(prep[0]);
+    prep_init(prep[1]);
     tc::mbar_fence_init();
     abort_flag = 0;
   }
@@ -1046,367 +1134,334 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  uint8_t* const smem_base = smem;
+  // tiles start at a 1 KB boundary: the 128-byte-swizzle pattern is a function of the shared-memory address
+  uint8_t* const smem_base = smem + ((1024u - (tc::smem_u32(smem) & 1023u)) & 1023u);
 
   if ((int)blockIdx.x >= n_slots) {
     // =========================== two preparation workers ===========================
     const int sub = warp >> 3;
-#ifdef HK_DIAG_ONE_WORKER
-    const int worker = (int)blockIdx.x - n_slots, n_workers = (int)gridDim.x - n_slots;
-#else
-    const int worker = ((int)blockIdx.x - n_slots) * 2 + sub, n_workers = ((int)gridDim.x - n_slots) * 2;
-#endif
-    const long long n_units = (long long)n_chunks * n_jobs;
-    PrepCtx ctx{smem + sub * P1_SMEM, sub ? &out_bar : &mma_bar, 0u, &abort_flag, tmem + sub * 256, tid & 255, 1 + sub, false,
-                nullptr, 0, 0, g_abort};
-#ifdef HK_DIAG
-    ctx.trace = false;
-#endif
-    int it = 0;
-#ifdef HK_DIAG_ONE_WORKER
-    if (sub == 1) goto prep_done;                          // diagnostic: stage times of a worker that has its SM alone
-#endif
-    for (long long u = worker; u < n_units; u += n_workers, it++) {
-      // units in the order the slots need them: running chunk v of every slot, then v + 1, ...
-      const int v = (int)(u / n_slots), slot = (int)(u % n_slots);
+    // unit `it` of a worker, in the order the slots need them: running chunk v of every slot, then v + 1, ...
+    auto make_unit = [&](int it, PrepDesc& u) {
+      const long long n = ((int)blockIdx.x - n_slots) * 2 + sub + (long long)it * ((int)gridDim.x - n_slots) * 2;
+      const int v = (int)min(n / n_slots, (long long)n_virtual), slot = (int)(n % n_slots);
       const int chunk = v % n_chunks, job = slot + n_slots * (v / n_chunks);
-      const int b = job / H, head = job % H;
-#ifdef HK_DIAG
-      ctx.trace = (worker == 7 && it == 20);
-#endif
-      // the slot of this chunk must have been drained by the chain CTA (it held chunk - KR): thread 0 asks now and
-      // looks at the answer just before the worker's first write to the unit (prep_unit calls slot_wait there)
-      ctx.slot_flag = consumed + slot;
-      ctx.slot_want = v >= KR ? v - KR + 1 : 0;
-      ctx.slot_seen = (ctx.tid == 0 && ctx.slot_want > 0) ? ld_relaxed_gpu(ctx.slot_flag) : 0;
-      uint8_t* unit = ring + ((size_t)(v % KR) * n_slots + slot) * U_BYTES;
-      const long long pu = u + n_workers;
-      int pf_head = 0, pf_chunk = -1;
-      if (pu < n_units) {
-        const int pv = (int)(pu / n_slots), pjob = (int)(pu % n_slots) + n_slots * (pv / n_chunks);
-        if (pjob / H == b) { pf_chunk = pv % n_chunks; pf_head = pjob % H; }
-      }
-      ctx.bar_parity = it & 1;
-      KT_TRACE(14);
-      prep_unit<GATED, true>(ctx, qkv, g, beta_in, unit, seqlen, H, head, chunk, b, pf_head, pf_chunk, dt_bias, a_log, lower_bound);
-      // publish: prep_unit ends with the worker's barrier, so every thread's writes of this unit precede this
-      // release store (which is cumulative over them)
-      if (ctx.tid == 0) st_release_gpu(ready + (size_t)slot * KR + (v % KR), v + 1);
-      KT_TRACE(15);
-      KT_FLUSH();
+      u.b = job / H;
+      u.t0 = chunk * KC;
+      u.tok0 = u.b * seqlen + u.t0;
+      u.n_valid = v < n_virtual ? min(KC, seqlen - chunk * KC) : 0;
+      u.head = job % H;
+      u.unit = (v % KR) * n_slots + slot;
+      u.slot = slot;
+      u.value = v + 1;
+    };
+    PrepCtx ctx;
+    ctx.smem = smem_base + sub * P1_SMEM; ctx.sh = &prep[sub]; ctx.abort_flag = &abort_flag; ctx.tid = tid & 255; ctx.bar_id = 1 + sub;
+    if (ctx.tid < 2) make_unit(ctx.tid, prep[sub].unit[ctx.tid]);
+    prep_sync<true>(ctx);
+    if (ctx.tid == 0) {
+      prep_fetch_g(ctx, 0, &map_g);
+      prep_fetch_qkv(ctx, 0, &map_qkv, H);
     }
-#ifdef HK_DIAG_ONE_WORKER
-  prep_done:;
-#endif
+    int it = 0;
+    for (; PREP_UNIT(n_valid, it) > 0; it++) {
+      prep_unit<GATED, true>(ctx, it, &map_qkv, &map_g, beta_in, ring, H, dt_bias, a_log, lower_bound, tmem + sub * 256, ready, consumed,
+                             g_abort, n_slots, make_unit);
+    }
+    if (it > 0 && ctx.tid < 32) prep_publish(ctx, it - 1, ready, n_slots);
   } else {
     // =========================== one (batch, head) chain ===========================
-    // the chain CTA's tiles start at a 1 KB boundary (the output tile is written in the 128-byte-swizzle pattern,
-    // which is a function of the shared-memory address)
-    uint8_t* const smem = smem_base + ((1024u - (tc::smem_u32(smem_base) & 1023u)) & 1023u);
+    // Sixteen warps = four TMEM lane quarters (lq) x four groups, joined by mbarriers that complete once per chunk, never by the
+    // whole CTA; what is on the chunk-to-chunk chain is spread over many warps, the rest has warps of its own:
+    //   U         lq 0, 1 of all groups (token rows of D1), 32 columns each
+    //   state     groups 0, 1: a k row and 64 of its columns per thread, fp32 in registers
+    //   outputs   warps 10, 11: a token row each thread
+    //   issuer    warp 14: every product; it waits for operands only
+    //   producer  warp 15: ring protocol and operand copies
+    // A barrier's next phase cannot complete before its waiters have seen this one: U needs every U warp, the state operand every
+    // state warp; out_bar and d1_bar alternate by chunk, since the output warps may be a chunk behind or done with the one before.
+    uint8_t* const smem = smem_base;
     const int cslot = blockIdx.x;                           // this CTA's chain slot
-    const int lq = warp & 3, cb = warp >> 2;               // TMEM lane quarter, 32-column block
-    const int rowi = lq * 32 + (tid & 31);                       // k row of the state / token row of W S0 / output row - 64
-    const int v0 = cb * KNV;
-    // chain number `ci` of this slot: (batch, head) = job cslot + n_slots * ci; its state rows for this thread
-    auto chain_state = [&](int ci) -> float* {
-      const int job = cslot + n_slots * ci, jb = job / H, jh = job % H;
-      const int sl = slots ? slots[jb] : jb;
-      return state + ((size_t)sl * H + jh) * KD * KD + (size_t)rowi * KD + v0;
-    };
-    float* st = chain_state(0);
-    const int* my_ready = ready + (size_t)cslot * KR;
-
-    for (int i = tid; i < 8192 / 16; i += 512)
-      for (int s_i = 0; s_i < F_NSTAGE; s_i++) reinterpret_cast<uint4*>(smem + s_i * F_STAGE + F_BB)[i] = make_uint4(0, 0, 0, 0);
-    float S[KNV];
-#pragma unroll
-    for (int u = 0; u < KNV / 4; u++) {
-      const float4 v = *reinterpret_cast<const float4*>(st + u * 4);
-      S[4 * u] = v.x; S[4 * u + 1] = v.y; S[4 * u + 2] = v.z; S[4 * u + 3] = v.w;
-    }
-    // B operand, MN-major, N = 128: off(k, n) = (n/8)*2048 + (k/8)*128 + (k%8)*16 + (n%8)*2
-    uint8_t* sS_row = smem + F_S + (4 * cb) * 2048 + (rowi >> 3) * 128 + (rowi & 7) * 16;
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      uint4 p;
-      p.x = pack_h2(S[8 * u], S[8 * u + 1]); p.y = pack_h2(S[8 * u + 2], S[8 * u + 3]);
-      p.z = pack_h2(S[8 * u + 4], S[8 * u + 5]); p.w = pack_h2(S[8 * u + 6], S[8 * u + 7]);
-      *reinterpret_cast<uint4*>(sS_row + u * 2048) = p;
-    }
+    const int lane = tid & 31, lq = warp & 3, grp = warp >> 2;
+    const int rowi = lq * 32 + lane;                        // k row of the state / token row of U / output row + 64
+    const int role = tc::warp_index_uniform();
+    // D1 alternates between columns 0-127 and 128-255 by chunk parity, D2 = columns 256-383
+    write_identity(smem + F_ID, tid, 512);
     tc::fence_async_smem();
-    tc::fence_before_sync();
     __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t d2 = tmem + 256;                        // D1 alternates between columns 0-127 and 128-255
 
-    // the producer thread (a lane of the last warp, which is never on the token-row path) owns the ring protocol
-    const bool producer = tid == 480;
-    int issued = 0;                                        // producer only: chunks whose copies have been issued
-    auto issue_loads = [&](int chunk) {
-      uint8_t* stg = smem + (chunk % F_NSTAGE) * F_STAGE;
-      const uint8_t* u = ring + ((size_t)(chunk % KR) * n_slots + cslot) * U_BYTES;
-      uint64_t* bar = &full_bar[chunk % F_NSTAGE];
-      fence_proxy_async_all();
-      tc::mbar_arrive_expect_tx(bar, U_BYTES);
-      tc::bulk_g2s(stg + F_WQ, u + U_WQ, 32768, bar);
-      tc::bulk_g2s(stg + F_BB + 8192, u + U_BB, 8192, bar);
-      tc::bulk_g2s(stg + F_KT, u + U_KT, 16384 + 16384 + 512, bar);
-    };
-    if (producer) {
-      for (; issued < F_NSTAGE && issued < n_virtual; issued++) {
-        poll_flag_ge(my_ready + (issued % KR), issued + 1, &abort_flag, g_abort, 21);
-        issue_loads(issued);
-      }
-    }
-
-    const uint32_t idesc = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, false, true);
-    const uint32_t s_addr = tc::smem_u32(smem + F_S), u_addr = tc::smem_u32(smem + F_U);
-    // two issuing warps: warp 0 the contractions on the chain ([W;Q+] S0 and Kt^T U), warp 2 (an output warp) the
-    // output contraction (B beta) U, so that warp 0 does not spend its issue time before its share of the state update
-    const int warp_u = tc::warp_index_uniform();
-    const bool issue_warp = warp_u == 0, out_issue_warp = warp_u == 2;
-    const uint32_t leader = (issue_warp || out_issue_warp) ? tc::elect_one() : 0u;
-
-    // Output rows of chunk c: TMEM lanes 64-127 of that chunk's D1 range = tokens, lane quarters 2 and 3 (eight warps =
-    // two token halves x four column blocks).  A thread holds 32 columns of one token; stored directly, a warp-wide
-    // 16-byte store would touch 32 different rows (32 L1 requests per instruction, over a thousand per chunk on this
-    // one SM).  The bf16 rows are therefore assembled in shared memory (272-byte pitch: conflict-free both ways) and
-    // written out with every warp instruction covering two whole 256-byte rows.  The eight warps meet at a named
-    // barrier of their own; the block barriers of the chain separate one chunk's reads from the next chunk's writes.
-    // With a tensor map over the output the rows leave as TWO tiled TMA stores per chunk (64 tokens x 64 channels each,
-    // 128-byte-swizzle boxes; rows past the end of the sequence are clipped by the copy engine): the tile is written
-    // conflict-free (16-byte piece p of row r at p ^ (r % 8)) and one thread hands it over.
-    auto emit_outputs = [&](int vc, bool valid) {          // vc: running chunk number of the slot
-      const int c = vc % n_chunks, ejob = cslot + n_slots * (vc / n_chunks), b = ejob / H, head = ejob % H;
-      const int trow = rowi - 64;
-      uint32_t r[32];
-      tc::tmem_ld32(tmem + ((vc & 1) ? 128u : 0u) + (uint32_t)v0 + ((uint32_t)(lq * 32) << 16), r);
-      tc::tmem_ld_wait();
-      const bool issuer = warp == 2 && (tid & 31) == 0;
-      if (use_tma_out) {
-        if (issuer) tc::bulk_wait_read<0>();               // the previous chunk's tile has been read by the copy engine
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-      }
-      uint8_t* orow = use_tma_out ? smem + F_O + (cb >> 1) * 8192 + trow * 128 : smem + F_O + trow * F_OPITCH + cb * (KNV * 2);
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float a = __uint_as_float(r[8 * u + 2 * e]) * scale, c2 = __uint_as_float(r[8 * u + 2 * e + 1]) * scale;
-          const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rz(a));
-          const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16_rz(c2));
-          w[e] = lo | (hi << 16);
-        }
-        const int off = use_tma_out ? ((((cb & 1) * 4 + u) ^ (trow & 7)) << 4) : u * 16;
-        *reinterpret_cast<uint4*>(orow + off) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-      if (use_tma_out) {
-        tc::fence_async_smem();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (issuer && valid) {
-#pragma unroll
-          for (int hb = 0; hb < 2; hb++)
-            asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(&tmap_out),
-                         "r"(hb * 64), "r"(head), "r"(c * KC), "r"(b), "r"(tc::smem_u32(smem + F_O + hb * 8192))
-                         : "memory");
-          tc::bulk_commit();
-        }
-      } else {
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        const int ot = (lq - 2) * 128 + cb * 32 + (tid & 31);   // 0..255 over the eight output warps
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const int piece = ot + 256 * i, prow = piece >> 4, pc = piece & 15;
-          const int ptok = c * KC + prow;
-          if (ptok < seqlen && valid) {
-            const uint4 v = *reinterpret_cast<const uint4*>(smem + F_O + prow * F_OPITCH + pc * 16);
-            *reinterpret_cast<uint4*>(out + (((size_t)b * seqlen + ptok) * H + head) * KD + pc * 8) = v;
-          }
-        }
-      }
-      const int tok = c * KC + trow;
-      if (out_f32 && tok < seqlen && valid) {
-        float4* of = reinterpret_cast<float4*>(out_f32 + (((size_t)b * seqlen + tok) * H + head) * KD + v0);
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-          of[u] = make_float4(__uint_as_float(r[4 * u]) * scale, __uint_as_float(r[4 * u + 1]) * scale,
-                              __uint_as_float(r[4 * u + 2]) * scale, __uint_as_float(r[4 * u + 3]) * scale);
-      }
-    };
-    bool prev_ok = true;
-
-    // `chunk` is the slot's RUNNING chunk number over all of its chains
-    for (int chunk = 0; chunk < n_virtual; chunk++) {
-      if (chunk > 0 && chunk % n_chunks == 0) {
-        // the next chain of this slot: its state replaces the previous one (stored at the end of the last iteration)
-        st = chain_state(chunk / n_chunks);
-#pragma unroll
-        for (int u = 0; u < KNV / 4; u++) {
-          const float4 v = *reinterpret_cast<const float4*>(st + u * 4);
-          S[4 * u] = v.x; S[4 * u + 1] = v.y; S[4 * u + 2] = v.z; S[4 * u + 3] = v.w;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          uint4 p;
-          p.x = pack_h2(S[8 * u], S[8 * u + 1]); p.y = pack_h2(S[8 * u + 2], S[8 * u + 3]);
-          p.z = pack_h2(S[8 * u + 4], S[8 * u + 5]); p.w = pack_h2(S[8 * u + 6], S[8 * u + 7]);
-          *reinterpret_cast<uint4*>(sS_row + u * 2048) = p;
-        }
-        tc::fence_async_smem();
-        tc::fence_before_sync();
-        __syncthreads();
+    // `v` is the slot's RUNNING chunk number over all of its chains
+    if (role == 14) {
+      const uint32_t leader = tc::elect_one();
+      const uint32_t idesc = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, false, true);
+      const uint32_t idesc_kt = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, true, true);   // Kt^T: channels contiguous
+      const uint32_t s_addr = tc::smem_u32(smem + F_S), u_addr = tc::smem_u32(smem + F_U), id_addr = tc::smem_u32(smem + F_ID);
+      for (int v = 0; v < n_virtual; v++) {
+        const uint32_t par = v & 1, ph = (v >> 1) & 1, stg_addr = tc::smem_u32(smem + par * F_STAGE);
+        const uint32_t d1 = tmem + par * 128, d2 = tmem + 256;
+        tc::mbar_wait(&wu_bar[par], ph, &abort_flag, 2);
+        if (v >= 2) tc::mbar_wait(&d1_bar[par], ph ^ 1, &abort_flag, 8);   // the output rows of chunk v - 2 have left this half of D1
         tc::fence_after_sync();
-      }
-      const int sidx = chunk % F_NSTAGE;
-      uint8_t* stg = smem + sidx * F_STAGE;
-      const uint32_t stg_addr = tc::smem_u32(stg);
-      const uint32_t d1 = tmem + ((chunk & 1) ? 128u : 0u);
-      int next_flag = 0;
-      if (producer && issued <= chunk) {                   // the earlier attempts found the unit not written yet
-        poll_flag_ge(my_ready + (chunk % KR), chunk + 1, &abort_flag, g_abort, 22);
-        issue_loads(chunk);
-        issued = chunk + 1;
-      }
-      KS_TRACE(0, chunk);
-      KS_TRACE_AT(8, chunk, 0);
-      KS_TRACE_AT(9, chunk, 50);
-      KS_TRACE_AT(10, chunk, 450);
-      bool ok = tc::mbar_wait(&full_bar[sidx], (chunk / F_NSTAGE) & 1, &abort_flag, 2);
-      KS_TRACE(1, chunk);
-      // ---- [W ; Q+] S0 -> D1 (128 x 128) ----
-      if (issue_warp) {
+        // ---- D1 = [I ; 0] Uloc, ahead of the state: the product with the identity is exact ----
 #pragma unroll
-        for (int kk = 0; kk < KD / 16; kk++) {
-          const uint64_t ad = tc::make_sdesc(stg_addr + F_WQ + kk * 2 * LBO, LBO, SBO_K128);
-          const uint64_t bd = tc::make_sdesc(s_addr + kk * 2 * 128, 128, 2048);
+        for (int kk = 0; kk < KC / 16; kk++) {
+          const uint64_t ad = tc::make_sdesc(id_addr + (6 - 2 * kk) * 128, 128, 128);
+          const uint64_t bd = tc::make_sdesc(stg_addr + U_UL + kk * 2 * 128, 128, 1024);
           tc::mma_f16_if(leader, d1, ad, bd, idesc, kk > 0);
         }
-        tc::mma_commit_if(leader, &mma_bar);
-      }
-      // the previous chunk's output rows leave while this chunk's first contraction runs (off the chain)
-      const uint32_t cpar = chunk & 1;
-      if (lq >= 2 && chunk > 0) emit_outputs(chunk - 1, prev_ok);
-      if (lq < 2) {
-        ok = tc::mbar_wait(&mma_bar, cpar, &abort_flag, 3) && ok;
+        // ---- D1 += [-W ; Q+] S0 ----
+        tc::mbar_wait(&s_bar[par], ph, &abort_flag, 6);
         tc::fence_after_sync();
-      }
-      KS_TRACE(2, chunk);
-      // ---- U = Uloc - W S0 (token rows = TMEM lanes 0-63) ----
-      if (lq < 2) {
-        const int t = rowi;
-        uint32_t r[32];
-        tc::tmem_ld32(d1 + (uint32_t)v0 + ((uint32_t)(lq * 32) << 16), r);
-        tc::tmem_ld_wait();
-        const uint4* ul = reinterpret_cast<const uint4*>(stg + F_UL + cb * (KC * KNV * 2) + t * (KNV * 2));
-        uint8_t* urow = smem + F_U + (4 * cb) * 1024 + (t >> 3) * 128 + (t & 7) * 16;   // off(k=t, n) = (n/8)*1024 + ...
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const uint4 lv = ul[u];
-          const __half2* lh = reinterpret_cast<const __half2*>(&lv);
-          float uu[8];
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const float2 f = __half22float2(lh[e]);
-            uu[2 * e] = f.x - __uint_as_float(r[8 * u + 2 * e]);
-            uu[2 * e + 1] = f.y - __uint_as_float(r[8 * u + 2 * e + 1]);
-          }
-          uint4 p;
-          p.x = pack_h2(uu[0], uu[1]); p.y = pack_h2(uu[2], uu[3]); p.z = pack_h2(uu[4], uu[5]); p.w = pack_h2(uu[6], uu[7]);
-          *reinterpret_cast<uint4*>(urow + u * 1024) = p;
+        for (int kk = 0; kk < KD / 16; kk++) {
+          const uint64_t ad = tc::make_sdesc(stg_addr + U_WQ + kk * 2 * LBO, LBO, SBO_K128);
+          const uint64_t bd = tc::make_sdesc(s_addr + kk * 2 * 128, 128, 2048);
+          tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
         }
-      }
-      // U is complete when all 256 token-row threads have arrived (after their proxy fence); the two issuing warps
-      // wait for that, nobody else does
-      if (lq < 2) {
-        tc::fence_async_smem();
-        tc::mbar_arrive(&u_bar);
-      }
-      KS_TRACE(3, chunk);
-      // The ring protocol runs here, while the producer's warp has nothing to do until the state contraction is
-      // complete.  None of it waits for this thread's earlier global stores (a release store or a fence would, and
-      // the block barriers of the chain would then wait for the output rows to reach memory).
-      if (producer) {
-        // the unit of this chunk has landed in shared memory: its slot may be rewritten.  A relaxed store is enough:
-        // the copy engine's reads are complete, nothing this thread wrote is handed over with the flag.
-        st_relaxed_gpu(consumed + cslot, chunk + 1);
-        // catch-up: the other stage is free while the next chunk's copies have not been issued
-        if (issued == chunk + 1 && chunk + 1 < n_virtual && ld_acquire_gpu(my_ready + ((chunk + 1) % KR)) >= chunk + 2) {
-          issue_loads(chunk + 1);
-          issued = chunk + 2;
-        }
-        // sampled now, used when this chunk's stage is released at the end of the iteration
-        if (issued == chunk + 2 && chunk + 2 < n_virtual) next_flag = ld_acquire_gpu(my_ready + ((chunk + 2) % KR));
-      }
-      // ---- D2 = Kt^T U (state path, warp 0) ;  D1 rows 64-127 += (B beta) U (outputs, warp 2, own barrier) ----
-      if (issue_warp) {
-        ok = tc::mbar_wait(&u_bar, cpar, &abort_flag, 6) && ok;
+        tc::mma_commit_if(leader, &mma_bar[par]);
+        // ---- D2 = Kt^T U (state path), then D1 rows 64-127 += (B beta) U (outputs) ----
+        tc::mbar_wait(&kb_bar[par], ph, &abort_flag, 11);
+        tc::mbar_wait(&u_bar, par, &abort_flag, 7);
         tc::fence_after_sync();
 #pragma unroll
         for (int kk = 0; kk < KC / 16; kk++) {
-          const uint64_t ad = tc::make_sdesc(stg_addr + F_KT + kk * 2 * LBO, LBO, SBO_K64);
+          const uint64_t ad = tc::make_sdesc(stg_addr + U_KT + kk * 2 * 128, 128, 1024);
           const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
-          tc::mma_f16_if(leader, d2, ad, bd, idesc, kk > 0);
+          tc::mma_f16_if(leader, d2, ad, bd, idesc_kt, kk > 0);
         }
         tc::mma_commit_if(leader, &mma2_bar);
-      }
-      if (out_issue_warp) {
-        ok = tc::mbar_wait(&u_bar, cpar, &abort_flag, 7) && ok;
-        tc::fence_after_sync();
+        // rows 0-63 of this operand are the tile below B beta in the unit: they add to U's rows, which have been read
 #pragma unroll
         for (int kk = 0; kk < KC / 16; kk++) {
-          const uint64_t ad = tc::make_sdesc(stg_addr + F_BB + kk * 2 * LBO, LBO, SBO_K64);
+          const uint64_t ad = tc::make_sdesc(stg_addr + U_BB - 8192 + kk * 2 * LBO, LBO, SBO_K64);
           const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
           tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
         }
-        tc::mma_commit_if(leader, &out_bar);
+        tc::mma_commit_if(leader, &out_bar[par]);
       }
-      ok = tc::mbar_wait(&mma2_bar, cpar, &abort_flag, 4) && ok;
-      tc::fence_after_sync();
-      KS_TRACE(4, chunk);
-      // ---- state: S <- S e^{G_last} + Kt^T U (lane = k row), refresh the fp16 operand copy ----
-      {
-        uint32_t r[32];
-        tc::tmem_ld32(d2 + (uint32_t)v0 + ((uint32_t)(lq * 32) << 16), r);
-        tc::tmem_ld_wait();
-        const float dec = reinterpret_cast<const float*>(stg + F_DEC)[rowi];
-#pragma unroll
-        for (int j = 0; j < KNV; j++) S[j] = fmaf(S[j], dec, __uint_as_float(r[j]));
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          uint4 p;
-          p.x = pack_h2(S[8 * u], S[8 * u + 1]); p.y = pack_h2(S[8 * u + 2], S[8 * u + 3]);
-          p.z = pack_h2(S[8 * u + 4], S[8 * u + 5]); p.w = pack_h2(S[8 * u + 6], S[8 * u + 7]);
-          *reinterpret_cast<uint4*>(sS_row + u * 2048) = p;
+    } else if (role == 15) {
+      const int* my_ready = ready + (size_t)cslot * F_LINE;
+      // a unit in two copies: a stage's first part is free as soon as the chunk's first product is complete, most of a chunk before
+      // the rest.  74 KB take about as long as a chunk to arrive.
+      auto load = [&](int v, uint32_t at, uint32_t bytes, uint64_t* bar) {
+        if (lane == 0) {
+          tc::mbar_arrive_expect_tx(bar, bytes);
+          tc::bulk_g2s(smem + (v & 1) * F_STAGE + at, ring + ((size_t)(v % KR) * n_slots + cslot) * U_BYTES + at, bytes, bar);
         }
+        __syncwarp();
+      };
+      // Units are asked for a ring at a time: a flag takes a microsecond or more to read while the workers poll theirs, too long for
+      // every chunk.
+      int known = 0;                                       // units before this one are complete
+      auto await_unit = [&](int v) {
+        const long long t0 = clock64();
+        while (known <= v) {
+          const bool here = lane < KR && ld_acquire_gpu(my_ready + (known + lane) % KR) > known + lane;
+          const uint32_t missing = ~__ballot_sync(0xffffffffu, here);
+          known += __ffs(missing) - 1;                     // lanes from KR on are never here
+          if (known > v) break;
+          const bool give_up = abort_flag || ld_relaxed_gpu(g_abort) != 0 || clock64() - t0 > tc::MBAR_WAIT_CYCLES;
+          if (__any_sync(0xffffffffu, give_up)) {
+            if (lane == 0) {
+              abort_flag = 21;
+              atomicExch(g_abort, 21);
+            }
+            break;
+          }
+          __nanosleep(64);
+        }
+        __syncwarp();
+        if (lane == 0) fence_proxy_async_all();
+      };
+      for (int v = 0; v < F_NSTAGE && v < n_virtual; v++) {
+        await_unit(v);
+        load(v, 0, U_BB, &wu_bar[v]);
+        load(v, U_BB, U_BYTES - U_BB, &kb_bar[v]);
       }
-      if (chunk % n_chunks == n_chunks - 1 && !abort_flag) {
-        // last chunk of a chain: its final state goes back to memory
+      for (int v = 0; v < n_virtual; v++) {
+        const uint32_t par = v & 1, ph = (v >> 1) & 1;
+        const bool more = v + F_NSTAGE < n_virtual;
+        // the unit of this chunk has landed in shared memory: its slot may be rewritten.  A relaxed store is enough:
+        // the copy engine's reads are complete, nothing this thread wrote is handed over with the flag.
+        tc::mbar_wait(&wu_bar[par], ph, &abort_flag, 2);
+        tc::mbar_wait(&kb_bar[par], ph, &abort_flag, 2);
+        if (lane == 0) st_relaxed_gpu(consumed + cslot * F_LINE, v + 1);
+        if (!more) continue;
+        await_unit(v + F_NSTAGE);
+        tc::mbar_wait(&mma_bar[par], ph, &abort_flag, 3);
+        load(v + F_NSTAGE, 0, U_BB, &wu_bar[par]);
+        // all products of the chunk are complete and the state warps have read its decays
+        tc::mbar_wait(&out_bar[par], ph, &abort_flag, 5);
+        tc::mbar_wait(&s_bar[par ^ 1], ((v + 1) >> 1) & 1, &abort_flag, 9);
+        load(v + F_NSTAGE, U_BB, U_BYTES - U_BB, &kb_bar[par]);
+      }
+    } else if (role == 10 || role == 11) {
+      // Output rows: TMEM lanes 64-127 of a chunk's D1 half = tokens; a thread holds the columns of one token.  Stored directly,
+      // a warp-wide 16-byte store would touch 32 different rows (32 L1 requests per instruction, over a thousand per chunk
+      // on this one SM).  The bf16 rows are therefore assembled in shared memory.  With a tensor map over the output they leave
+      // as TWO tiled TMA stores per chunk (64 tokens x 64 channels each, 128-byte-swizzle boxes; rows past the end of the sequence
+      // are clipped by the copy engine): the tile is written conflict-free (16-byte piece p of row r at p ^ (r % 8)) and one
+      // thread hands it over.  Without a map every warp instruction covers two whole 256-byte rows.
+      const int trow = rowi - 64;
+      const bool issuer = role == 10 && lane == 0;
+      bool valid = true;
+      int c = 0, job = cslot;                              // chunk of the chain, chain
+      for (int v = 0; v < n_virtual; v++) {
+        const int b = job / H, head = job % H;
+        const bool ok = tc::mbar_wait(&out_bar[v & 1], (v >> 1) & 1, &abort_flag, 10);
+        valid = valid && ok;
+        tc::fence_after_sync();
+        if (use_tma_out && issuer) tc::bulk_wait_read<0>();   // the previous chunk's tile has been read by the copy engine
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        const int tok = c * KC + trow;
 #pragma unroll
-        for (int u = 0; u < KNV / 4; u++)
-          *reinterpret_cast<float4*>(st + u * 4) = make_float4(S[4 * u], S[4 * u + 1], S[4 * u + 2], S[4 * u + 3]);
+        for (int q = 0; q < 4; q++) {
+          uint32_t r[32];
+          tc::tmem_ld32(tmem + (v & 1) * 128 + (uint32_t)(q * 32) + ((uint32_t)(lq * 32) << 16), r);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const float a = __uint_as_float(r[8 * u + 2 * e]) * scale, c2 = __uint_as_float(r[8 * u + 2 * e + 1]) * scale;
+              const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rz(a));
+              const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16_rz(c2));
+              w[e] = lo | (hi << 16);
+            }
+            const int p = q * 4 + u;
+            uint8_t* o = use_tma_out ? smem + F_O + (p >> 3) * 8192 + trow * 128 + (((p & 7) ^ (trow & 7)) << 4) : smem + F_O + trow * F_OPITCH + p * 16;
+            *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+          if (out_f32 && tok < seqlen && valid) {
+            float4* of = reinterpret_cast<float4*>(out_f32 + (((size_t)b * seqlen + tok) * H + head) * KD + q * 32);
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+              of[u] = make_float4(__uint_as_float(r[4 * u]) * scale, __uint_as_float(r[4 * u + 1]) * scale,
+                                  __uint_as_float(r[4 * u + 2]) * scale, __uint_as_float(r[4 * u + 3]) * scale);
+          }
+        }
+        tc::fence_before_sync();
+        if (lane == 0) tc::mbar_arrive(&d1_bar[v & 1]);           // chunk v + 2 may have this half of D1
+        tc::fence_async_smem();
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        if (use_tma_out) {
+          if (issuer && valid) {
+#pragma unroll
+            for (int hb = 0; hb < 2; hb++)
+              asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(&tmap_out),
+                           "r"(hb * 64), "r"(head), "r"(c * KC), "r"(b), "r"(tc::smem_u32(smem + F_O + hb * 8192))
+                           : "memory");
+            tc::bulk_commit();
+          }
+        } else {
+          const int ot = (lq - 2) * 32 + lane;             // 0..63 over the two output warps
+#pragma unroll 4
+          for (int i = 0; i < 16; i++) {
+            const int piece = ot + 64 * i, prow = piece >> 4, pc = piece & 15;
+            const int ptok = c * KC + prow;
+            if (ptok < seqlen && valid) {
+              const uint4 o4 = *reinterpret_cast<const uint4*>(smem + F_O + prow * F_OPITCH + pc * 16);
+              *reinterpret_cast<uint4*>(out + (((size_t)b * seqlen + ptok) * H + head) * KD + pc * 8) = o4;
+            }
+          }
+        }
+        if (++c == n_chunks) { c = 0; job += n_slots; }
       }
-      KS_TRACE(5, chunk);
-      // the output contraction must be complete before the block barrier: the stage and the U tile it reads are
-      // rewritten after it; the rows themselves are read in the next iteration
-      if (lq >= 2) {
-        ok = tc::mbar_wait(&out_bar, cpar, &abort_flag, 5) && ok;
-        prev_ok = ok;
+      if (use_tma_out && issuer) tc::bulk_wait_all<0>();
+    } else {
+      const bool state_warp = grp < 2, u_warp = lq < 2;
+      // chain number `ci` of this slot: (batch, head) = job cslot + n_slots * ci; its state row for this thread
+      auto chain_state = [&](int ci) -> float* {
+        const int job = cslot + n_slots * ci, jb = job / H, jh = job % H;
+        const int sl = slots ? slots[jb] : jb;
+        return state + ((size_t)sl * H + jh) * KD * KD + (size_t)rowi * KD + grp * 64;
+      };
+      // B operand of the state, MN-major, N = 128: off(k, n) = (n/8)*2048 + (k/8)*128 + (k%8)*16 + (n%8)*2
+      uint8_t* sS_row = smem + F_S + (8 * grp) * 2048 + rowi * 16;
+      float S[64];
+      auto load_state = [&](const float* st) {
+#pragma unroll
+        for (int u = 0; u < 16; u++) {
+          const float4 x = *reinterpret_cast<const float4*>(st + u * 4);
+          S[4 * u] = x.x; S[4 * u + 1] = x.y; S[4 * u + 2] = x.z; S[4 * u + 3] = x.w;
+        }
+      };
+      auto put_operand = [&](int u0, int n) {              // pieces u0 .. u0 + n - 1 of this row's 64 columns as fp16
+#pragma unroll
+        for (int u = u0; u < u0 + n; u++)
+          *reinterpret_cast<uint4*>(sS_row + u * 2048) = make_uint4(pack_h2(S[8 * u], S[8 * u + 1]), pack_h2(S[8 * u + 2], S[8 * u + 3]),
+                                                                    pack_h2(S[8 * u + 4], S[8 * u + 5]), pack_h2(S[8 * u + 6], S[8 * u + 7]));
+      };
+      if (state_warp) {
+        load_state(chain_state(0));
+        put_operand(0, 8);
+        tc::fence_async_smem();
+        tc::mbar_arrive(&s_bar[0]);
       }
-      tc::fence_async_smem();
-      tc::fence_before_sync();
-      __syncthreads();
-      tc::fence_after_sync();
-      KS_TRACE(6, chunk);
-      // refill of this stage, if the unit two chunks ahead was already complete when its flag was sampled
-      if (producer && issued == chunk + 2 && chunk + 2 < n_virtual && next_flag >= chunk + 3) {
-        issue_loads(chunk + 2);
-        issued = chunk + 3;
+      int in_chain = 0, chain = 0;                         // chunk of the chain, chain of the slot
+      for (int v = 0; v < n_virtual; v++) {
+        const uint32_t par = v & 1;
+        const uint32_t d1 = tmem + par * 128, d2 = tmem + 256;
+        KS_TRACE(0, v);
+        KS_TRACE_AT(8, v, 0);
+        KS_TRACE_AT(9, v, 50);
+        KS_TRACE_AT(10, v, 450);
+        // ---- U (token rows = TMEM lanes 0-63 of D1) as the next operand: off(t, n) = (n/8)*1024 + t*16 + (n%8)*2 ----
+        if (u_warp) {
+          tc::mbar_wait(&mma_bar[par], (v >> 1) & 1, &abort_flag, 3);
+          tc::fence_after_sync();
+          KS_TRACE(1, v);
+          uint32_t r[32];
+          tc::tmem_ld32(d1 + (uint32_t)(grp * KNV) + ((uint32_t)(lq * 32) << 16), r);
+          tc::tmem_ld_wait();
+          uint8_t* urow = smem + F_U + (4 * grp) * 1024 + rowi * 16;
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            *reinterpret_cast<uint4*>(urow + u * 1024) =
+                make_uint4(pack_h2(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])), pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])),
+                           pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])), pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])));
+          tc::fence_async_smem();
+          tc::fence_before_sync();
+          tc::mbar_arrive(&u_bar);
+          KS_TRACE(2, v);
+        }
+        // ---- state: S <- S e^{G_last} + Kt^T U (lane = k row), refresh the fp16 operand copy ----
+        if (state_warp) {
+          tc::mbar_wait(&kb_bar[par], (v >> 1) & 1, &abort_flag, 2);
+          const float dec = reinterpret_cast<const float*>(smem + par * F_STAGE + U_DEC)[rowi];
+          tc::mbar_wait(&mma2_bar, par, &abort_flag, 4);
+          tc::fence_after_sync();
+          KS_TRACE(3, v);
+          const bool last = in_chain == n_chunks - 1;
+#pragma unroll
+          for (int hf = 0; hf < 2; hf++) {
+            uint32_t r[32];
+            tc::tmem_ld32(d2 + (uint32_t)(grp * 64 + hf * 32) + ((uint32_t)(lq * 32) << 16), r);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; j++) S[hf * 32 + j] = fmaf(S[hf * 32 + j], dec, __uint_as_float(r[j]));
+            if (!last) put_operand(4 * hf, 4);
+          }
+          if (last) {
+            // last chunk of a chain: its final state goes back to memory and the slot's next chain begins
+            float* st = chain_state(chain);
+            if (!abort_flag) {
+#pragma unroll
+              for (int u = 0; u < 16; u++)
+                *reinterpret_cast<float4*>(st + u * 4) = make_float4(S[4 * u], S[4 * u + 1], S[4 * u + 2], S[4 * u + 3]);
+            }
+            if (v + 1 < n_virtual) {
+              load_state(chain_state(chain + 1));
+              put_operand(0, 8);
+            }
+          }
+          tc::fence_async_smem();
+          tc::fence_before_sync();
+          tc::mbar_arrive(&s_bar[par ^ 1]);
+          KS_TRACE(4, v);
+        }
+        if (++in_chain == n_chunks) { in_chain = 0; chain++; }
       }
-    }
-    if (lq >= 2 && n_virtual > 0) {
-      emit_outputs(n_virtual - 1, prev_ok);
-      if (use_tma_out && warp == 2 && (tid & 31) == 0) tc::bulk_wait_all<0>();
     }
   }
   tc::fence_before_sync();
@@ -1450,8 +1505,29 @@ int fused_slots(long long n_jobs) {
 bool short_call(long long n_jobs, int n_chunks, int n_slots) {
   return n_jobs * n_chunks <= (long long)KR * n_slots && (KVS * n_jobs <= sm_count() || n_chunks <= 12);
 }
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                             const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeFn tensor_map_encoder() {
+  static const EncodeFn fn = []() -> EncodeFn {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess
+               ? (EncodeFn)p
+               : nullptr;
+  }();
+  return fn;
+}
+bool encode_rows(CUtensorMap* map, const void* base, CUtensorMapDataType type, int elem, int channels, int seqlen, int bsz, int box_channels) {
+  const EncodeFn encode = tensor_map_encoder();
+  if (!encode) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)channels, (cuuint64_t)seqlen, (cuuint64_t)bsz};
+  const cuuint64_t strides[2] = {(cuuint64_t)channels * elem, (cuuint64_t)seqlen * channels * elem};
+  const cuuint32_t box[3] = {(cuuint32_t)box_channels, (cuuint32_t)KC, 1}, estr[3] = {1, 1, 1};
+  return encode(map, type, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 size_t fused_flag_bytes(int n_slots) {
-  return (((size_t)F_FLAG_INTS + (size_t)n_slots * (KR + 1)) * sizeof(int) + 255) / 256 * 256;
+  return (((size_t)F_FLAG_INTS + (size_t)n_slots * 2 * F_LINE) * sizeof(int) + 255) / 256 * 256;
 }
 }  // namespace
 }  // namespace hk
@@ -1497,14 +1573,19 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(kda_chunk_prep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P1_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(kda_chunk_prep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P1_SMEM) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kda_chunk_prep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(P1_SMEM + 1024)) != cudaSuccess ||
+        cudaFuncSetAttribute(kda_chunk_prep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(P1_SMEM + 1024)) != cudaSuccess ||
         cudaFuncSetAttribute(kda_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(kda_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(kda_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_SMEM) != cudaSuccess)
       return HK_ERR_CUDA;
     attr_set[dev] = true;
   }
+  // tensor maps of the inputs, [batch][token][channels]: boxes of 64 tokens x 128 bytes, 128-byte swizzle, zeros past the last token
+  alignas(64) CUtensorMap map_qkv, map_g;
+  if (!encode_rows(&map_qkv, mixed_qkv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 3 * num_heads * KD, seqlen, bsz, 64) ||
+      !encode_rows(&map_g, g_or_f, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, num_heads * KD, seqlen, bsz, 32))
+    return HK_ERR_CUDA;
   cudaStream_t s = as_stream(stream);
   int* st = device_status_ptr();
   const int n_slots = fused_slots((long long)bsz * num_heads);
@@ -1523,7 +1604,6 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const __nv_bfloat16* a_qkv = (const __nv_bfloat16*)mixed_qkv;
     uint8_t* a_ring = (uint8_t*)workspace + flag_bytes;
     int* a_flags = (int*)workspace;
     __nv_bfloat16* a_out = (__nv_bfloat16*)out;
@@ -1534,19 +1614,7 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
     memset(&tmap, 0, sizeof(tmap));
     int use_tma_out = 0;
     {
-      typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-      static EncodeFn encode = nullptr;
-      static bool looked_up = false;
-      if (!looked_up) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-          encode = (EncodeFn)fn;
-        looked_up = true;
-      }
+      const EncodeFn encode = tensor_map_encoder();
       if (encode) {
         const cuuint64_t dims[4] = {(cuuint64_t)KD, (cuuint64_t)num_heads, (cuuint64_t)seqlen, (cuuint64_t)bsz};
         const cuuint64_t strides[3] = {(cuuint64_t)KD * 2, (cuuint64_t)num_heads * KD * 2, (cuuint64_t)seqlen * num_heads * KD * 2};
@@ -1561,15 +1629,15 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
     const float* a_al = gated ? a_log : nullptr;
     const float a_lb = gated ? lower_bound : 0.f;
     cudaError_t e = gated
-        ? cudaLaunchKernelEx(&cfg, kda_fused_kernel<true>, a_qkv, g_or_f, beta_or_b, a_ring, a_flags, state, a_out, out_f32,
+        ? cudaLaunchKernelEx(&cfg, kda_fused_kernel<true>, map_qkv, map_g, beta_or_b, a_ring, a_flags, state, a_out, out_f32,
                              seqlen, num_heads, n_chunks, n_jobs, n_slots, slots, a_scale, st, a_dt, a_al, a_lb, tmap, use_tma_out)
-        : cudaLaunchKernelEx(&cfg, kda_fused_kernel<false>, a_qkv, g_or_f, beta_or_b, a_ring, a_flags, state, a_out, out_f32,
+        : cudaLaunchKernelEx(&cfg, kda_fused_kernel<false>, map_qkv, map_g, beta_or_b, a_ring, a_flags, state, a_out, out_f32,
                              seqlen, num_heads, n_chunks, n_jobs, n_slots, slots, a_scale, st, a_dt, a_al, a_lb, tmap, use_tma_out);
     return e == cudaSuccess ? HK_OK : HK_ERR_CUDA;
   }
   const dim3 grid(num_heads, n_chunks, bsz);
   auto prep = gated ? kda_chunk_prep_kernel<true> : kda_chunk_prep_kernel<false>;
-  if (pdl_launch(prep, grid, dim3(256), P1_SMEM, s, (const __nv_bfloat16*)mixed_qkv, g_or_f, beta_or_b, (uint8_t*)workspace, seqlen,
+  if (pdl_launch(prep, grid, dim3(256), P1_SMEM + 1024, s, map_qkv, map_g, beta_or_b, (uint8_t*)workspace, seqlen,
                  num_heads, n_chunks, 2 * sm_count(), st, gated ? dt_bias : nullptr, gated ? a_log : nullptr,
                  gated ? lower_bound : 0.f) != cudaSuccess)
     return HK_ERR_CUDA;
