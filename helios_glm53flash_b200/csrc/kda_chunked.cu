@@ -71,6 +71,12 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// two values rounded toward zero to bf16
+__device__ __forceinline__ uint32_t pack_bf2_rz(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
@@ -917,12 +923,7 @@ __global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
       for (int u = 0; u < 4; u++) {
         uint32_t w[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float a = __uint_as_float(r[8 * u + 2 * e]) * scale, c2 = __uint_as_float(r[8 * u + 2 * e + 1]) * scale;
-          const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rz(a));
-          const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16_rz(c2));
-          w[e] = lo | (hi << 16);
-        }
+        for (int e = 0; e < 4; e++) w[e] = pack_bf2_rz(__uint_as_float(r[8 * u + 2 * e]) * scale, __uint_as_float(r[8 * u + 2 * e + 1]) * scale);
         o[u] = make_uint4(w[0], w[1], w[2], w[3]);
       }
       if (out_f32) {
@@ -1195,18 +1196,25 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
       const uint32_t idesc = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, false, true);
       const uint32_t idesc_kt = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, true, true);   // Kt^T: channels contiguous
       const uint32_t s_addr = tc::smem_u32(smem + F_S), u_addr = tc::smem_u32(smem + F_U), id_addr = tc::smem_u32(smem + F_ID);
-      for (int v = 0; v < n_virtual; v++) {
-        const uint32_t par = v & 1, ph = (v >> 1) & 1, stg_addr = tc::smem_u32(smem + par * F_STAGE);
-        const uint32_t d1 = tmem + par * 128, d2 = tmem + 256;
-        tc::mbar_wait(&wu_bar[par], ph, &abort_flag, 2);
-        if (v >= 2) tc::mbar_wait(&d1_bar[par], ph ^ 1, &abort_flag, 8);   // the output rows of chunk v - 2 have left this half of D1
+      // D1 of chunk w = [I ; 0] Uloc, ahead of the state: the product with the identity is exact
+      auto issue_uloc = [&](int w) {
         tc::fence_after_sync();
-        // ---- D1 = [I ; 0] Uloc, ahead of the state: the product with the identity is exact ----
 #pragma unroll
         for (int kk = 0; kk < KC / 16; kk++) {
           const uint64_t ad = tc::make_sdesc(id_addr + (6 - 2 * kk) * 128, 128, 128);
-          const uint64_t bd = tc::make_sdesc(stg_addr + U_UL + kk * 2 * 128, 128, 1024);
-          tc::mma_f16_if(leader, d1, ad, bd, idesc, kk > 0);
+          const uint64_t bd = tc::make_sdesc(tc::smem_u32(smem + (w & 1) * F_STAGE) + U_UL + kk * 2 * 128, 128, 1024);
+          tc::mma_f16_if(leader, tmem + (w & 1) * 128, ad, bd, idesc, kk > 0);
+        }
+      };
+      int uloc = 0;                                        // chunks whose Uloc has been issued
+      for (int v = 0; v < n_virtual; v++) {
+        const uint32_t par = v & 1, ph = (v >> 1) & 1, stg_addr = tc::smem_u32(smem + par * F_STAGE);
+        const uint32_t d1 = tmem + par * 128, d2 = tmem + 256;
+        if (uloc == v) {
+          tc::mbar_wait(&wu_bar[par], ph, &abort_flag, 2);
+          if (v >= 2) tc::mbar_wait(&d1_bar[par], ph ^ 1, &abort_flag, 8);   // the output rows of chunk v - 2 have left this half of D1
+          issue_uloc(v);
+          uloc++;
         }
         // ---- D1 += [-W ; Q+] S0 ----
         tc::mbar_wait(&s_bar[par], ph, &abort_flag, 6);
@@ -1218,6 +1226,16 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
           tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
         }
         tc::mma_commit_if(leader, &mma_bar[par]);
+        // the next chunk's Uloc while U leaves the tensor memory, if its operands and its half of D1 are there already (otherwise at
+        // the chunk's start, where 260 cycles of products stand between the state and U: 3.5 -> 2.7 thousand cycles a chunk)
+        if (v + 1 < n_virtual) {
+          const uint32_t nph = ((v + 1) >> 1) & 1;
+          const bool here = tc::mbar_test_wait(&wu_bar[par ^ 1], nph) && (v == 0 || tc::mbar_test_wait(&d1_bar[par ^ 1], nph ^ 1));
+          if (__all_sync(0xffffffffu, here)) {
+            issue_uloc(v + 1);
+            uloc++;
+          }
+        }
         // ---- D2 = Kt^T U (state path), then D1 rows 64-127 += (B beta) U (outputs) ----
         tc::mbar_wait(&kb_bar[par], ph, &abort_flag, 11);
         tc::mbar_wait(&u_bar, par, &abort_flag, 7);
@@ -1322,12 +1340,7 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
           for (int u = 0; u < 4; u++) {
             uint32_t w[4];
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-              const float a = __uint_as_float(r[8 * u + 2 * e]) * scale, c2 = __uint_as_float(r[8 * u + 2 * e + 1]) * scale;
-              const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rz(a));
-              const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16_rz(c2));
-              w[e] = lo | (hi << 16);
-            }
+            for (int e = 0; e < 4; e++) w[e] = pack_bf2_rz(__uint_as_float(r[8 * u + 2 * e]) * scale, __uint_as_float(r[8 * u + 2 * e + 1]) * scale);
             const int p = q * 4 + u;
             uint8_t* o = use_tma_out ? smem + F_O + (p >> 3) * 8192 + trow * 128 + (((p & 7) ^ (trow & 7)) << 4) : smem + F_O + trow * F_OPITCH + p * 16;
             *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
