@@ -261,8 +261,8 @@ __device__ __forceinline__ void prep_inverse_row(const float* __restrict__ sN, c
 
 // What a preparation worker (256 threads) keeps in static shared memory: its barriers and the units it has at hand (unit number `it`
 // at it % 4; thread registers are too few to carry them through a unit).  SUB = false: the worker is a whole CTA with one unit
-// (__syncthreads); SUB = true: it is one of the two workers of a CTA and uses the named barriers `bar_id` (all of it) and `bar_id + 2`
-// (the four warps that write a unit's last part).
+// (__syncthreads); SUB = true: it is one of the two workers of a CTA and uses the named barriers `bar_id` and `bar_id + 2` (behind a
+// unit's last writes).
 struct PrepDesc {
   int tok0;                                                // first token: batch * seqlen + 64 * chunk
   int b, t0;                                               // batch, first token in it
@@ -299,13 +299,13 @@ __device__ __forceinline__ void prep_init(PrepShared& sh) {  // one thread
 // a field of the unit `it`, read anew at every use
 #define PREP_UNIT(field, it) (*const_cast<volatile int*>(&ctx.sh->unit[(it) & 3].field))
 
-// Fused form: stores the ready flag of unit `it`.  Called by warp 0, which meets the other three warps of the unit's last writers
-// here; the barriers inside prep_unit order everybody else's writes before them, and the release store is cumulative over all of
-// them.  It waits until the CTA's stores are visible, some thousand cycles when they are fresh: it is put off to a place in the next
-// unit where warp 0 has nothing else to do, unless the worker has to wait for its ring slot.
+// Fused form: stores the ready flag of unit `it`.  Called by one warp, which meets the others behind the unit's last writes here; the
+// release store is cumulative over them.  It waits until the CTA's stores are visible, some thousand cycles when they are fresh: it is
+// put off to a place in the next unit where its warp has little else to do, unless the worker has to wait for its ring slot.
+constexpr int PUB_WARP = 2;
 __device__ __forceinline__ void prep_publish(const PrepCtx& ctx, int it, int* ready, int n_slots) {
-  asm volatile("bar.sync %0, 128;" ::"r"(ctx.bar_id + 2) : "memory");
-  if (ctx.tid == 0) {
+  asm volatile("bar.sync %0, 256;" ::"r"(ctx.bar_id + 2) : "memory");
+  if (ctx.tid == PUB_WARP * 32) {
     const int value = PREP_UNIT(value, it);
     st_release_gpu(ready + (size_t)PREP_UNIT(slot, it) * F_LINE + (value - 1) % KR, value);
   }
@@ -318,10 +318,6 @@ __device__ __forceinline__ void prep_tma(uint8_t* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(tc::smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(t), "r"(b), "r"(tc::smem_u32(bar))
       : "memory");
-}
-__device__ __forceinline__ void prep_tma_l2(const CUtensorMap* map, int c, int t, int b) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(t), "r"(b)
-               : "memory");
 }
 // the next unit's inputs, each as soon as its place is free (one thread)
 __device__ __forceinline__ void prep_fetch_g(const PrepCtx& ctx, int it, const CUtensorMap* map_g) {
@@ -351,7 +347,7 @@ __device__ __forceinline__ void prep_fetch_qkv(const PrepCtx& ctx, int it, const
 // fp32 gate tensor is never written to or read back from memory.
 // The unit's inputs are on their way (prep_fetch_*); its end sends for those of the next.  SUB: `ready` and `consumed` are the flags
 // of the ring; on return the unit's last writes are on their way and its flag is still to be stored (prep_publish).
-// `make_unit(it, desc)` works out a later unit (one thread).
+// `make_unit(it, desc)` works out the next unit (one thread).
 template <bool GATED, bool SUB, class MakeUnit>
 __device__ __forceinline__ void prep_unit(
     const PrepCtx& ctx, const int it, const CUtensorMap* map_qkv, const CUtensorMap* map_g, const void* __restrict__ beta_in,
@@ -377,8 +373,8 @@ __device__ __forceinline__ void prep_unit(
   // ---- stage 1: log-decay sums.  x_t = inclusive sum of the log decay (in units of log 2) INSIDE the 16-token block, in place;
   //      lane 8 J + p of warp w sums channels 16 w + 2 p, + 1 over block J, so the block totals of a channel sit in four lanes
   //      of one warp, which turn them into the tables ----
-  int seen = 0;                                            // thread 0: chunks of the slot that have been consumed
-  if (SUB && tid == 0) seen = ld_relaxed_gpu(consumed + PREP_UNIT(slot, it) * F_LINE);
+  int seen = 0;                                            // publishing warp's first lane: chunks of the slot that have been consumed
+  if (SUB && tid == PUB_WARP * 32) seen = ld_relaxed_gpu(consumed + PREP_UNIT(slot, it) * F_LINE);
   float beta = 0.f;
   if (t < PREP_UNIT(n_valid, it)) {
     const size_t bi = (size_t)(PREP_UNIT(tok0, it) + t) * H + PREP_UNIT(head, it);
@@ -466,8 +462,8 @@ __device__ __forceinline__ void prep_unit(
     rq = rsqrtf(sq + 1e-6f);
   }
   // fused form: the ring slot must have been drained before the first write to the unit (all of them follow)
-  bool unpublished = SUB && it > 0;                        // warp 0: the flag of the unit before this one
-  if (SUB && warp == 0) {
+  bool unpublished = SUB && it > 0;                        // the flag of the unit before this one
+  if (SUB && warp == PUB_WARP) {
     const int want = PREP_UNIT(value, it) - KR;            // the slot held chunk value - 1 - KR
     if (__shfl_sync(0xffffffffu, seen, 0) < want) {
       if (unpublished) prep_publish(ctx, it - 1, ready, n_slots);   // before a wait: the chains may need that unit to get on
@@ -582,9 +578,9 @@ __device__ __forceinline__ void prep_unit(
   }
   prep_sync<SUB>(ctx);                                     // right operands and the diagonal blocks of N are complete
 
-  // ---- stage 3: the products with earlier blocks (fp16).  Odd warps: the inverse of their block's 16 x 16 diagonal of I + N;
-  //      even warps convert v meanwhile ----
-  if (SUB && warp == 0 && unpublished) prep_publish(ctx, it - 1, ready, n_slots);   // warp 0 has no earlier block
+  // ---- stage 3: the products with earlier blocks (fp16), 2 I tiles a warp; the warps of the first block, which have none, invert the
+  //      16 x 16 diagonal blocks of I + N, those of the second and third convert v as well ----
+  if (SUB && warp == PUB_WARP && unpublished) prep_publish(ctx, it - 1, ready, n_slots);
   {
     float* nrow = sN + prep_n_row(t) + 2 * tig;
     uint8_t* bbrow = PREP_OUT + U_BB + warp * SBO_K64 + g8 * 16 + tig * 4;
@@ -608,38 +604,37 @@ __device__ __forceinline__ void prep_unit(
       }
     }
   }
-  if (odd) {
-    // inverse of the unit lower triangular 16 x 16 block, lane = column: x_r = delta - sum_{s<r} N[r][s] x_s
-    if (lane < 16) {
-      float x[16];
-      const float* nd = sN + prep_n_row(16 * I) + 16 * I;
-      const int ld = I < 2 ? 36 : 68;
+  if (I == 0) {
+    // inverse of a unit lower triangular 16 x 16 block, lane = column of one of two blocks: x_r = delta - sum_{s<r} N[r][s] x_s
+    const int blk = 2 * warp + (lane >> 4), col = lane & 15;
+    float x[16];
+    const float* nd = sN + prep_n_row(16 * blk) + 16 * blk;
+    const int ld = warp == 0 ? 36 : 68;
 #pragma unroll
-      for (int r = 0; r < 16; r++) {
-        float a0 = (r == lane) ? 1.f : 0.f, a1 = 0.f;
+    for (int r = 0; r < 16; r++) {
+      float a0 = (r == col) ? 1.f : 0.f, a1 = 0.f;
 #pragma unroll
-        for (int s = 0; s < r; s += 4) {
-          const float4 n4 = *reinterpret_cast<const float4*>(nd + r * ld + s);
-          const float nn[4] = {n4.x, n4.y, n4.z, n4.w};
+      for (int s = 0; s < r; s += 4) {
+        const float4 n4 = *reinterpret_cast<const float4*>(nd + r * ld + s);
+        const float nn[4] = {n4.x, n4.y, n4.z, n4.w};
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
-            if (s + u >= r) break;
-            if (u & 1) a1 = fmaf(-nn[u], x[s + u], a1);
-            else a0 = fmaf(-nn[u], x[s + u], a0);
-          }
+        for (int u = 0; u < 4; u++) {
+          if (s + u >= r) break;
+          if (u & 1) a1 = fmaf(-nn[u], x[s + u], a1);
+          else a0 = fmaf(-nn[u], x[s + u], a0);
         }
-        x[r] = a0 + a1;
       }
-      float* xi = sX + prep_inv_at(I) + lane;
-#pragma unroll
-      for (int r = 0; r < 16; r++) xi[r * P1_LDX] = x[r];
+      x[r] = a0 + a1;
     }
-  } else {
+    float* xi = sX + prep_inv_at(blk) + col;
+#pragma unroll
+    for (int r = 0; r < 16; r++) xi[r * P1_LDX] = x[r];
+  } else if (I < 3) {
     // bf16 -> fp16 in place.  (The product T V needs both operands in ONE 16-bit format: a kind::f16 product of an fp16 T with bf16
     // rows is rejected by the hardware as an illegal instruction.)
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      uint4* vp = reinterpret_cast<uint4*>(smem + P1_V) + I * 32 + lane + 128 * j;
+      uint4* vp = reinterpret_cast<uint4*>(smem + P1_V) + tid - 64 + 128 * j;
       const uint4 vr = *vp;
       *vp = make_uint4(pack_h2(bf16lo(vr.x), bf16hi(vr.x)), pack_h2(bf16lo(vr.y), bf16hi(vr.y)), pack_h2(bf16lo(vr.z), bf16hi(vr.z)),
                        pack_h2(bf16lo(vr.w), bf16hi(vr.w)));
@@ -666,6 +661,7 @@ __device__ __forceinline__ void prep_unit(
     }
   } else {
     const int e = tid - 192;
+    if (SUB && e == 0) make_unit(it + 1, ctx.sh->unit[(it + 1) & 3]);
 #pragma unroll
     for (int q = 0; q < 2; q++) {                          // 4 blocks x 16 rows x 2 pieces
       const int i = e + 64 * q, blk = i >> 5, r = (i & 7) + ((i >> 4) & 1) * 8, h = (i >> 3) & 1;
@@ -684,34 +680,23 @@ __device__ __forceinline__ void prep_unit(
   if (warp == 1) prep_inverse_row<1>(sN, sX, sT, lane);
   else if (warp == 2) prep_inverse_row<2>(sN, sX, sT, lane);
   else if (warp == 3) prep_inverse_row<3>(sN, sX, sT, lane);
-  else if (tid == 192) {
-    // the inputs of a unit about one wave of workers ahead, pulled into L2
-    PrepDesc u;
-    make_unit(it + 2, u);
-    ctx.sh->unit[(it + 2) & 3] = u;
-    if (u.n_valid > 0) {
-#pragma unroll
-      for (int m = 0; m < 4; m++) prep_tma_l2(map_g, u.head * KD + 32 * m, u.t0, u.b);
-#pragma unroll
-      for (int m = 0; m < 6; m++) prep_tma_l2(map_qkv, ((m >> 1) * H + u.head) * KD + 64 * (m & 1), u.t0, u.b);
-    }
-  }
   tc::fence_async_smem();
   tc::fence_before_sync();
   prep_sync<SUB>(ctx);
   tc::fence_after_sync();
 
-  // ---- stage 5: [W | Uloc] = T [K+ | V] : tcgen05 M128 N128 K64 twice, fp16 in, fp32 TMEM accumulators ----
+  // ---- stage 5: W = T K+, Uloc = T V: tcgen05 weight-stationary M64 N128 K64, fp16 in, fp32 TMEM accumulators: columns 0-63 of the 64
+  //      tokens in lanes 0-63, columns 64-127 in lanes 64-127, so that all eight warps read them ----
   if (tid == 0) {
-    const uint32_t idesc = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, false, true);
+    const uint32_t idesc = tc::make_idesc(64, KD, tc::FMT_F16, tc::FMT_F16, false, true);
     const uint32_t a_addr = tc::smem_u32(sT), k_addr = tc::smem_u32(sK);
     const uint64_t vd = tc::make_sdesc_sw128(tc::smem_u32(smem + P1_V), P1_BOX, 1024);
 #pragma unroll
     for (int kk = 0; kk < KC / 16; kk++)
-      tc::mma_f16(tmem, tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64), tc::make_sdesc(k_addr + kk * 2 * 128, 128, P1_PIECE), idesc, kk > 0);
+      tc::mma_ws_f16_if(1, tmem, tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64), tc::make_sdesc(k_addr + kk * 2 * 128, 128, P1_PIECE), idesc, kk > 0);
 #pragma unroll
     for (int kk = 0; kk < KC / 16; kk++)
-      tc::mma_f16(tmem + KD, tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64), tc::sdesc_advance(vd, kk * 2048), idesc, kk > 0);
+      tc::mma_ws_f16_if(1, tmem + 64, tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64), tc::sdesc_advance(vd, kk * 2048), idesc, kk > 0);
     tc::mma_commit(&ctx.sh->mma_bar);
   }
   if (tid == 96) prep_fetch_g(ctx, it + 1, map_g);         // x is free
@@ -719,46 +704,33 @@ __device__ __forceinline__ void prep_unit(
   const bool ok = tc::mbar_wait(&ctx.sh->mma_bar, it & 1, ctx.abort_flag, 1);
   if (tid == 96) prep_fetch_qkv(ctx, it + 1, map_qkv, H);  // and so are T, N, K+ and V
   tc::fence_after_sync();
-  // ---- stage 6: epilogue. Lanes 0-63 are the tokens; warps 0,1 take W, warps 4,5 take Uloc ----
-  if ((warp & 3) < 2) {
-    if (ok) {
-      uint8_t* const unit = PREP_OUT;
-      const int et = (warp & 3) * 32 + lane;
-      const bool second = warp >= 4;
-      const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (second ? 128 : 0);
+  // ---- stage 6: the accumulators leave: warps 0-3 take W, warps 4-7 Uloc, a token and 64 columns each thread ----
+  if (ok) {
+    uint8_t* const out = PREP_OUT;
+    const int et = (warp & 1) * 32 + lane, c0 = (warp & 2) * 32;
+    const uint32_t acc = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
+    uint8_t* const dst = warp < 4 ? out + U_WQ + (et >> 3) * SBO_K128 + (et & 7) * 16 + (c0 >> 3) * LBO : out + U_UL + (et ^ 8) * 16 + (c0 >> 3) * 1024;
+    const uint32_t pitch = warp < 4 ? LBO : 1024, sign = warp < 4 ? 0x80008000u : 0u;   // W is stored negated
 #pragma unroll
-      for (int c0 = 0; c0 < KD; c0 += 32) {
-        uint32_t r[32];
-        tc::tmem_ld32(lane_addr + c0, r);
-        tc::tmem_ld_wait();
-        uint4 p[4];
+    for (int h = 0; h < 2; h++) {
+      uint32_t r[32];
+      tc::tmem_ld32(acc + 32 * h, r);
+      tc::tmem_ld_wait();
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          p[u].x = pack_h2(__uint_as_float(r[8 * u + 0]), __uint_as_float(r[8 * u + 1]));
-          p[u].y = pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3]));
-          p[u].z = pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5]));
-          p[u].w = pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7]));
-        }
-        if (!second) {                                     // -W
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            *reinterpret_cast<uint4*>(unit + U_WQ + (et >> 3) * SBO_K128 + (c0 / 8 + u) * LBO + (et & 7) * 16) =
-                make_uint4(p[u].x ^ 0x80008000u, p[u].y ^ 0x80008000u, p[u].z ^ 0x80008000u, p[u].w ^ 0x80008000u);
-        } else {
-#pragma unroll
-          for (int u = 0; u < 4; u++) *reinterpret_cast<uint4*>(unit + U_UL + (c0 / 8 + u) * 1024 + (et ^ 8) * 16) = p[u];
-        }
-      }
+      for (int u = 0; u < 4; u++)
+        *reinterpret_cast<uint4*>(dst + (4 * h + u) * pitch) = make_uint4(
+            pack_h2(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])) ^ sign, pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])) ^ sign,
+            pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])) ^ sign, pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])) ^ sign);
     }
-    tc::fence_before_sync();
-    if (SUB && warp != 0) asm volatile("bar.arrive %0, 128;" ::"r"(ctx.bar_id + 2) : "memory");
   }
+  tc::fence_before_sync();
+  if (SUB && warp != PUB_WARP) asm volatile("bar.arrive %0, 256;" ::"r"(ctx.bar_id + 2) : "memory");
 }
 
 template <bool GATED>
 __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
     const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
-    uint8_t* __restrict__ ws, int seqlen, int H, int n_chunks, int prefetch_dist, int* __restrict__ status,
+    uint8_t* __restrict__ ws, int seqlen, int H, int n_chunks, int* __restrict__ status,
     const float* __restrict__ dt_bias, const float* __restrict__ a_log, float lower_bound) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ PrepShared sh;
@@ -768,14 +740,6 @@ __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
   // heads are the fastest grid dimension: CTAs that run together read the same tokens, i.e. whole contiguous rows of the
   // activations.  Units are chunk-major: the CTAs that run together (same chunks, all heads) touch adjacent units, in
   // this kernel and in the scan, so their traffic spreads over all memory channels.
-  auto describe = [&](int head, int chunk, PrepDesc& u) {
-    u.b = blockIdx.z;
-    u.t0 = chunk * KC;
-    u.tok0 = u.b * seqlen + u.t0;
-    u.n_valid = chunk < n_chunks ? min(KC, seqlen - u.t0) : 0;
-    u.head = head;
-    u.unit = (u.b * n_chunks + chunk) * H + head;
-  };
   PrepCtx ctx;
   ctx.smem = smem + ((1024u - (tc::smem_u32(smem) & 1023u)) & 1023u);
   ctx.sh = &sh; ctx.abort_flag = &abort_flag; ctx.tid = tid; ctx.bar_id = 0;
@@ -783,26 +747,27 @@ __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
     prep_init(sh);
     tc::mbar_fence_init();
     abort_flag = 0;
-    describe(blockIdx.x, blockIdx.y, sh.unit[0]);
+    PrepDesc& u = sh.unit[0];
+    u.b = blockIdx.z;
+    u.t0 = blockIdx.y * KC;
+    u.tok0 = u.b * seqlen + u.t0;
+    u.n_valid = min(KC, seqlen - u.t0);
+    u.head = blockIdx.x;
+    u.unit = (u.b * n_chunks + (int)blockIdx.y) * H + u.head;
     sh.unit[1].n_valid = 0;                                // a CTA has one unit
     pdl_wait();
     prep_fetch_g(ctx, 0, &map_g);
     prep_fetch_qkv(ctx, 0, &map_qkv, H);
   }
-  if (tid < 32) tc::tmem_alloc(&tmem_slot, 256);
+  if (tid < 32) tc::tmem_alloc(&tmem_slot, 128);
   pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   prep_unit<GATED, false>(ctx, 0, &map_qkv, &map_g, beta_in, ws, H, dt_bias, a_log, lower_bound, tmem_slot, nullptr, nullptr, nullptr, 0,
-                          [&](int, PrepDesc& u) {
-    // the unit whose inputs it pulls into L2 is the one of the CTA that runs `prefetch_dist` blocks later (blocks are
-    // scheduled in linear order, heads fastest)
-    const long long lin = (long long)blockIdx.y * H + blockIdx.x + prefetch_dist;
-    describe((int)(lin % H), (int)min(lin / H, (long long)n_chunks), u);
-  });
+                          [](int, PrepDesc&) {});
   __syncthreads();
-  if (tid < 32) tc::tmem_dealloc(tmem_slot, 256);
+  if (tid < 32) tc::tmem_dealloc(tmem_slot, 128);
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
 }
 
@@ -1157,7 +1122,7 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
     };
     PrepCtx ctx;
     ctx.smem = smem_base + sub * P1_SMEM; ctx.sh = &prep[sub]; ctx.abort_flag = &abort_flag; ctx.tid = tid & 255; ctx.bar_id = 1 + sub;
-    if (ctx.tid < 2) make_unit(ctx.tid, prep[sub].unit[ctx.tid]);
+    if (ctx.tid == 0) make_unit(0, prep[sub].unit[0]);
     prep_sync<true>(ctx);
     if (ctx.tid == 0) {
       prep_fetch_g(ctx, 0, &map_g);
@@ -1168,7 +1133,7 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
       prep_unit<GATED, true>(ctx, it, &map_qkv, &map_g, beta_in, ring, H, dt_bias, a_log, lower_bound, tmem + sub * 256, ready, consumed,
                              g_abort, n_slots, make_unit);
     }
-    if (it > 0 && ctx.tid < 32) prep_publish(ctx, it - 1, ready, n_slots);
+    if (it > 0 && (ctx.tid >> 5) == PUB_WARP) prep_publish(ctx, it - 1, ready, n_slots);
   } else {
     // =========================== one (batch, head) chain ===========================
     // Sixteen warps = four TMEM lane quarters (lq) x four groups, joined by mbarriers that complete once per chunk, never by the
@@ -1651,7 +1616,7 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
   const dim3 grid(num_heads, n_chunks, bsz);
   auto prep = gated ? kda_chunk_prep_kernel<true> : kda_chunk_prep_kernel<false>;
   if (pdl_launch(prep, grid, dim3(256), P1_SMEM + 1024, s, map_qkv, map_g, beta_or_b, (uint8_t*)workspace, seqlen,
-                 num_heads, n_chunks, 2 * sm_count(), st, gated ? dt_bias : nullptr, gated ? a_log : nullptr,
+                 num_heads, n_chunks, st, gated ? dt_bias : nullptr, gated ? a_log : nullptr,
                  gated ? lower_bound : 0.f) != cudaSuccess)
     return HK_ERR_CUDA;
   return pdl_launch(kda_chunk_scan_kernel, dim3(KVS, num_heads, bsz), dim3(128), P2_SMEM, s, (const uint8_t*)workspace, state,
