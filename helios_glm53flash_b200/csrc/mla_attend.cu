@@ -14,6 +14,7 @@ namespace hk {
 // implemented in mla_flash_tc.cu; returns HK_ERR_UNSUPPORTED when the shape is not covered
 int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s);
 int mla_flash_tc_auto_splits(int m, int n_keys);
+bool mla_flash_cluster_shape(int m, int tiles, int* n_split, int* n_cs);
 
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -107,6 +108,14 @@ static int attend(MlaArgs a, int n_keys_hint, int n_split, void* workspace, size
     PartialLayout pl = partial_layout(n_split, rows);
     if (!workspace || workspace_bytes < pl.total) return HK_ERR_WORKSPACE;
     if (!aligned(workspace, 256)) return HK_ERR_INVALID;
+    // Few rows of few tiles: one kernel whose clusters merge the splits.  The rows' tiles are known for gathered rows and causal
+    // ranges; where each row has a length of its own on the device, fewer splits than the GPU has room for mean two tiles each.
+    const int tiles = a.raw_idx || !a.kv_len ? (n_keys_hint + 63) / 64 : (int64_t)a.m * (n_split + 1) <= sm_count() ? 2 * n_split : 1 << 20;
+    MlaArgs c = a;
+    if (tc && mla_flash_cluster_shape(a.m, tiles, &c.n_split, &c.n_cs)) {
+      const int st = mla_flash_tc_launch(c, s);
+      if (st != HK_ERR_UNSUPPORTED) return st;
+    }
     char* ws = (char*)workspace;
     a.part_m = (float*)ws;
     a.part_l = (float*)(ws + pl.off_l);

@@ -62,11 +62,26 @@ constexpr float RESCALE_THRESHOLD = 8.0f;         // log2 units: P stays below 2
 // others load tiles (dense ranges need more than one only for the ragged last tile).
 constexpr int FT_LOAD_WARPS = 4, FT_THREADS = (6 + FT_LOAD_WARPS) * 32, FT_SLOTS = FT_KEYS / FT_LOAD_WARPS;   // key slots per loader warp
 
+constexpr int FT_MINI = 16;                       // keys of a tile in Q's place
+constexpr int FT_MAX_CL = 16;                     // CTAs of a cluster
+constexpr uint32_t FT_CL_STAGE = FT_HEADS * (256 * 4 + 8);  // outgoing shares behind the incoming ones (256 channels or 128)
+// all threads of all CTAs of the cluster.  Relaxed: the barriers only tell that memory is no longer in use, the data that crosses CTAs is
+// announced by mbarriers (.release: 1,000 cycles more each)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// the address of a shared-memory word in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
 struct FtMisc {
   uint64_t full[FT_NBUF], free[FT_NBUF];          // ring slot (a key tile or a row's Q): landed, may be overwritten
   uint64_t s_full[2], s_free[2], p_full[2], pv_done[2];   // per tile parity
   uint64_t q_ready, o_free;                       // per row
-  uint8_t mask[FT_NBUF][FT_KEYS / 8];             // valid key slots of the tile in the ring slot
+  uint64_t full_mini;
+  uint8_t mask[FT_NBUF + 1][FT_KEYS / 8];         // valid key slots of the tile in the ring slot; [FT_NBUF]: the ragged tile in Q's place
   float mx[2][128];                               // tile maxima, by softmax thread and tile parity
   float l[128];
   uint32_t tmem;
@@ -74,17 +89,24 @@ struct FtMisc {
 };
 static_assert(sizeof(FtMisc) <= 2048, "misc area");
 
-// One work item: a row and a key split.
+// One work item: a row and a key split (cluster form: and a part of the output channels).
 struct FtItem {
-  int r, sp, k0, k1, n_tiles;
+  int r, sp, cs, k0, k1, n_tiles;                 // cs: part of the output channels (cluster form)
+  bool mini;                                      // cluster form: the ragged last tile comes first, from memory of its own
   int64_t base;
   __device__ __forceinline__ int keys(int t) const { return min(FT_KEYS, k1 - k0 - t * FT_KEYS); }
+  __device__ __forceinline__ int nth(int i) const { return mini ? (i ? i - 1 : n_tiles - 1) : i; }   // the tile that is i-th in turn
 };
-template <bool G4>
+template <bool G4, bool CL>
 __device__ __forceinline__ FtItem ft_item(const MlaArgs& a, int idx) {
   FtItem it;
   it.sp = idx % a.n_split;
   it.r = idx / a.n_split;
+  it.cs = 0;
+  if (CL) {
+    it.cs = it.r % a.n_cs;
+    it.r /= a.n_cs;
+  }
   // rows of a causal chunk grow with their number: the longest first, so that the CTAs end together
   if (!G4 && !a.kv_len) it.r = a.m - 1 - it.r;
   int n;
@@ -98,9 +120,13 @@ __device__ __forceinline__ FtItem ft_item(const MlaArgs& a, int idx) {
   }
   // split boundaries on tile granularity
   const int tiles = (n + FT_KEYS - 1) / FT_KEYS, per = (tiles + a.n_split - 1) / a.n_split;
-  it.k0 = min(n, it.sp * per * FT_KEYS);
-  it.k1 = min(n, (it.sp + 1) * per * FT_KEYS);
+  // (cluster form: a fixed number of splits, so the tiles are shared out evenly)
+  it.k0 = min(n, (CL ? tiles * it.sp / a.n_split : it.sp * per) * FT_KEYS);
+  it.k1 = min(n, (CL ? tiles * (it.sp + 1) / a.n_split : (it.sp + 1) * per) * FT_KEYS);
   it.n_tiles = (it.k1 - it.k0 + FT_KEYS - 1) / FT_KEYS;
+  // 2,052 keys are 32 tiles and 4 keys more.  A split with a third tile of up to 16 keys would have to wait for a ring slot: that
+  // tile lies where Q's 128 channels are otherwise (16 key rows a block) and is attended to while the whole ones arrive.
+  it.mini = CL && it.n_tiles > 2 && it.keys(it.n_tiles - 1) <= FT_MINI;
   return it;
 }
 
@@ -132,7 +158,13 @@ __device__ __forceinline__ void tma_gather4_rows(uint32_t leader, uint32_t smem_
 
 // G4: gathered rows (raw_idx); otherwise dense ranges.  tmap_box: 3-D map of the cache, tmap_rows: 2-D map of the cache for
 // gather4, tmap_q: the queries as tmap_box, tmap_o: 2-D map of the final output.
-template <bool G4>
+// CL: cluster form for few rows of few keys (a decode step's gathered rows).  The splits of a row are the CTAs of a cluster, which merge
+// their partials through distributed shared memory and write the final output: no partials in memory, no second kernel.  The row's
+// output channels are shared out over n_cs such clusters, each of which computes the scores for itself.
+// What bounds it is latency, one thing after another on 64 SMs: row numbers 1,200 cycles, gathered keys 2,800, two tiles of S, softmax and
+// P V 3,800, laying out and the barrier of the cluster 1,700, the shares 2,200, the merge 1,600.  2,052 gathered rows of one query 10.8 ->
+// 9.2 us; MLA layer of one token at 5,001 32.1 -> 28.9, selection and attention at 262,144 23.8 -> 21.8.
+template <bool G4, bool CL>
 __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
     MlaArgs a, int* __restrict__ status, const __grid_constant__ CUtensorMap tmap_box, const __grid_constant__ CUtensorMap tmap_rows,
     const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_o) {
@@ -144,10 +176,10 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
   const int tid = threadIdx.x, lane = tid & 31;
   // provably warp-uniform role index: the issuing warps' branches stay converged for the compiler
   const int warp = tc::warp_index_uniform();
-  const int n_items = a.n_split * a.m, step = gridDim.x;
+  const int n_items = CL ? gridDim.x : a.n_split * a.m, step = gridDim.x;
   // A CTA with one item of at most two tiles (a decode split) never needs Q's ring slot back: S reads Q from there, and the
-  // 0.6 us of moving it are saved.
-  bool direct_q = false;
+  // 0.6 us of moving it are saved.  In the cluster form Q always stays and the other two slots serve all tiles.
+  bool direct_q = CL;
   if (tid == 0) {
 #pragma unroll
     for (int b = 0; b < FT_NBUF; b++) {
@@ -161,14 +193,16 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
       tc::mbar_init(&ms.p_full[b], 128);
       tc::mbar_init(&ms.pv_done[b], 1);
     }
-    tc::mbar_init(&ms.q_ready, 128);
+    if (CL) tc::mbar_init(&ms.full_mini, FT_LOAD_WARPS);
+    tc::mbar_init(&ms.q_ready, CL ? 1 : 128);              // (cluster form: the shares of the other splits)
     tc::mbar_init(&ms.o_free, 128);
     tc::mbar_fence_init();
+    if (CL) tc::mbar_arrive_expect_tx(&ms.q_ready, FT_HEADS * (LATENT / a.n_cs * 4 + 8));
     ms.abort_flag = 0;
   }
   if (warp == 0) tc::tmem_alloc(&ms.tmem, 512);
   pdl_wait();
-  if (step >= n_items) direct_q = ft_item<G4>(a, blockIdx.x).n_tiles < FT_NBUF;
+  if (!CL && step >= n_items) direct_q = ft_item<G4, CL>(a, blockIdx.x).n_tiles < FT_NBUF;
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -176,6 +210,12 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
   bool ok = true;
 
   // Every role walks the same items and counts the same way: u = ring slots used so far, g = key tiles, q = rows with keys.
+  // Ring slot of use u (the i-th tile of the item) and the earlier uses of that slot; cluster form: Q keeps slot 0.
+  auto slot_of = [](const FtItem& it, uint32_t u, int i) -> int { return !CL ? u % FT_NBUF : it.mini && i == 0 ? FT_NBUF : 1 + ((i - it.mini) & 1); };
+  auto turn_of = [](const FtItem& it, uint32_t u, int i) -> uint32_t { return !CL ? u / FT_NBUF : it.mini && i == 0 ? 0 : (i - it.mini) >> 1; };
+  auto full_of = [&](int b) -> uint64_t* { return CL && b == FT_NBUF ? &ms.full_mini : &ms.full[b]; };
+  auto tile_at = [](int b) -> uint32_t { return CL && b == FT_NBUF ? FS_Q : FS_K + b * FT_TILE; };
+  auto blk_of = [](int b) -> uint32_t { return CL && b == FT_NBUF ? FT_MINI * 128 : FT_BLK; };   // bytes of a 64-channel block
   if (warp >= 6) {
     // =========================== loaders: per row its Q, then its key tiles ===========================
     const int lw = warp - 6;
@@ -193,14 +233,14 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
     auto in_cache = [&](int v) -> int { return (v < 0 || (a.ckv_rows > 0 && (int64_t)v >= a.ckv_rows)) ? -1 : v; };
     // Gathered row numbers are fetched two tiles ahead (the row list of a query is read once, from HBM), across rows.
     int cur = -1, nxt = -1, ahead_item = blockIdx.x, ahead_tile = 0;
-    FtItem ahead = ft_item<G4>(a, ahead_item);
+    FtItem ahead = ft_item<G4, CL>(a, ahead_item);
     auto fetch = [&]() -> int {
       if (!G4 || ahead_item >= n_items || ahead.n_tiles == 0) return -1;   // (gathered rows: every item has the same keys)
-      const int v = row_of(ahead, ahead_tile);
+      const int v = row_of(ahead, ahead.nth(ahead_tile));
       if (++ahead_tile == ahead.n_tiles) {
         ahead_tile = 0;
         ahead_item += step;
-        if (ahead_item < n_items) ahead = ft_item<G4>(a, ahead_item);
+        if (ahead_item < n_items) ahead = ft_item<G4, CL>(a, ahead_item);
       }
       return v;
     };
@@ -209,17 +249,18 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
       nxt = fetch();
     }
     uint32_t u = 0;
-    auto next_slot = [&]() -> int {                        // waits until the slot may be overwritten
-      const int b = u % FT_NBUF;
-      if (u >= FT_NBUF) ok = tc::mbar_wait<FT_POLL_NS>(&ms.free[b], (u / FT_NBUF - 1) & 1, abort_flag, 5) && ok;
+    auto next_slot = [&](const FtItem& it, int i) -> int { // waits until the slot may be overwritten (i < 0: for Q)
+      const int b = CL && i < 0 ? 0 : slot_of(it, u, i);
+      const uint32_t turn = CL && i < 0 ? 0 : turn_of(it, u, i);
+      if (turn > 0) ok = tc::mbar_wait<FT_POLL_NS>(&ms.free[b], (turn - 1) & 1, abort_flag, 5) && ok;
       u++;
       return b;
     };
     for (int idx = blockIdx.x; idx < n_items; idx += step) {
-      const FtItem it = ft_item<G4>(a, idx);
+      const FtItem it = ft_item<G4, CL>(a, idx);
       if (it.n_tiles == 0) continue;
       {
-        const int b = next_slot();
+        const int b = next_slot(it, -1);
         if (lane == 0) {
           if (lw == 0) {
             tc::mbar_arrive_expect_tx(&ms.full[b], FT_TILE);
@@ -229,7 +270,8 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
           }
         }
       }
-      for (int tile = 0; tile < it.n_tiles; tile++) {
+      for (int i = 0; i < it.n_tiles; i++) {
+        const int tile = it.nth(i);
         int row;
         if (G4) {
           row = in_cache(cur);
@@ -239,7 +281,7 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
           row = row_of(it, tile);
         }
         const uint32_t valid = __ballot_sync(0xffffffffu, row >= 0);
-        const int b = next_slot();
+        const int b = next_slot(it, i);
         if (lane < FT_SLOTS / 8) ms.mask[b][lw * (FT_SLOTS / 8) + lane] = (uint8_t)(valid >> (8 * lane));
         __syncwarp();
         if (!G4 && it.keys(tile) == FT_KEYS) {             // a whole tile of a dense range: one box
@@ -252,16 +294,21 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
             }
           }
         } else {
-          if (lane == 0) tc::mbar_arrive_expect_tx(&ms.full[b], FT_SLOTS * LATENT * 2);
+          const bool none = CL && b == FT_NBUF && lw > 0;  // a ragged tile in Q's place has the first warp's key slots only
+          if (lane == 0) {
+            if (none) tc::mbar_arrive(full_of(b));
+            else tc::mbar_arrive_expect_tx(full_of(b), FT_SLOTS * LATENT * 2);
+          }
           __syncwarp();
-          const uint32_t dst = tc::smem_u32(smem + FS_K) + b * FT_TILE + lw * FT_SLOTS * 128, bar = tc::smem_u32(&ms.full[b]);
+          if (none) continue;
+          const uint32_t dst = tc::smem_u32(smem) + tile_at(b) + lw * FT_SLOTS * 128, bar = tc::smem_u32(full_of(b)), blk_bytes = blk_of(b);
 #pragma unroll
           for (int j = 0; j < FT_SLOTS / 4; j++) {
             const int r0 = __shfl_sync(0xffffffffu, row, 4 * j), r1 = __shfl_sync(0xffffffffu, row, 4 * j + 1);
             const int r2 = __shfl_sync(0xffffffffu, row, 4 * j + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * j + 3);
 #pragma unroll
             for (int blk = 0; blk < 8; blk++)
-              tma_gather4_rows(leader, dst + blk * FT_BLK + j * 512, &tmap_rows, blk * 64, r0, r1, r2, r3, bar);
+              tma_gather4_rows(leader, dst + blk * blk_bytes + j * 512, &tmap_rows, blk * 64, r0, r1, r2, r3, bar);
           }
         }
       }
@@ -289,24 +336,27 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
         return tc::make_sdesc_sw128(addr, 16, 1024);
       };
       for (int idx = blockIdx.x; idx < n_items; idx += step) {
-        const int n_tiles = ft_item<G4>(a, idx).n_tiles;
+        const FtItem it = ft_item<G4, CL>(a, idx);
+        const int n_tiles = it.n_tiles;
         if (n_tiles == 0) continue;
         if (direct_q) wait_u(&ms.full[0], 0, 15);
         else wait_u(&ms.q_ready, q & 1, 13);
         u++;                                               // the row's Q
         q++;
         for (int tile = 0; tile < n_tiles; tile++, u++, g++) {
-          const int b = g & 1, kb = u % FT_NBUF;
-          wait_u(&ms.full[kb], (u / FT_NBUF) & 1, 1);
+          const int b = g & 1, kb = slot_of(it, u, tile);
+          wait_u(full_of(kb), turn_of(it, u, tile) & 1, 1);
           if (g >= 2) wait_u(&ms.s_free[b], ((g - 2) >> 1) & 1, 2);
           tc::fence_after_sync();
           // keys as N in 1 KB atoms; 16 channels = 32 B inside the 128-byte row, 64 channels per block
-          const uint64_t kd = desc(smem + FS_K + kb * FT_TILE), qd = desc(smem + (direct_q ? FS_K : FS_Q));
+          const uint64_t kd = desc(smem + tile_at(kb)), qd = desc(smem + (direct_q ? FS_K : FS_Q));
+          const uint32_t kblk = blk_of(kb);
           if (direct_q) {
 #pragma unroll
             for (int kk = 0; kk < LATENT / 16; kk++) {
-              const uint32_t off = (kk >> 2) * FT_BLK + (kk & 3) * 32;
-              tc::mma_ws_f16_if(leader, tmem + FT_S + b * 32, tc::sdesc_advance(qd, off), tc::sdesc_advance(kd, off), idesc, kk > 0);
+              // (a ragged tile's columns past its keys are whatever lies there: masked)
+              tc::mma_ws_f16_if(leader, tmem + FT_S + b * 32, tc::sdesc_advance(qd, (kk >> 2) * FT_BLK + (kk & 3) * 32),
+                                tc::sdesc_advance(kd, (kk >> 2) * kblk + (kk & 3) * 32), idesc, kk > 0);
             }
           } else
 #pragma unroll
@@ -323,18 +373,26 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
     } else {
       const uint32_t idesc = tc::make_idesc(64, 256, tc::FMT_F16, tc::FMT_F16, false, true);
       for (int idx = blockIdx.x; idx < n_items; idx += step) {
-        const FtItem it = ft_item<G4>(a, idx);
+        const FtItem it = ft_item<G4, CL>(a, idx);
         if (it.n_tiles == 0) continue;
         u++;
         for (int tile = 0; tile < it.n_tiles; tile++, u++, g++) {
-          const int b = g & 1, kb = u % FT_NBUF;
+          const int b = g & 1, kb = slot_of(it, u, tile);
           wait_u(&ms.p_full[b], (g >> 1) & 1, 3);
           if (tile == 0 && q > 0) wait_u(&ms.o_free, (q - 1) & 1, 14);   // the row before has left the accumulator
           tc::fence_after_sync();
           const uint64_t pd = tc::make_sdesc_sw128(tc::smem_u32(smem + FS_P + b * FP_BYTES), 16, 1024);
           // V: N = 256 channels = four 64-channel blocks (leading offset), K = keys in 8-row atoms of 1 KB
-          const uint64_t vd = tc::make_sdesc_sw128(tc::smem_u32(smem + FS_K + kb * FT_TILE), FT_BLK, 1024);
-          const int steps = (it.keys(tile) + 15) >> 4;     // a ragged tile ends early
+          const uint64_t vd = tc::make_sdesc_sw128(tc::smem_u32(smem + tile_at(kb)), blk_of(kb), 1024);
+          const int steps = (it.keys(it.nth(tile)) + 15) >> 4;   // a ragged tile ends early
+          if (CL && a.n_cs > 1) {                          // one product of 256 or 128 channels
+            const uint32_t id = a.n_cs == 2 ? idesc : tc::make_idesc(64, 128, tc::FMT_F16, tc::FMT_F16, false, true);
+            const uint64_t vc = tc::sdesc_advance(vd, it.cs * (8 / a.n_cs) * blk_of(kb));
+#pragma unroll
+            for (int kk = 0; kk < FT_KEYS / 16; kk++)
+              if (kk < steps)
+                tc::mma_ws_f16_if(leader, tmem + FT_O, tc::sdesc_advance(pd, kk * 32), tc::sdesc_advance(vc, kk * 2048), id, tile > 0 || kk > 0);
+          } else
 #pragma unroll
           for (int nh = 0; nh < 2; nh++)
 #pragma unroll
@@ -343,7 +401,7 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
                 tc::mma_ws_f16_if(leader, tmem + FT_O + nh * 128, tc::sdesc_advance(pd, kk * 32),
                                   tc::sdesc_advance(vd, nh * 4 * FT_BLK + kk * 2048), idesc, tile > 0 || kk > 0);
           tc::mma_commit_if(leader, &ms.pv_done[b]);
-          tc::mma_commit_if(leader, &ms.free[kb]);
+          if (!CL || kb < FT_NBUF) tc::mma_commit_if(leader, &ms.free[kb]);
         }
         q++;
       }
@@ -386,18 +444,18 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
       u++;
     };
     auto next_row = [&](int idx) {                         // the first item from idx on that has keys
-      while (idx < n_items && ft_item<G4>(a, idx).n_tiles == 0) idx += step;
+      while (idx < n_items && ft_item<G4, CL>(a, idx).n_tiles == 0) idx += step;
       return idx;
     };
     int q_item = next_row(blockIdx.x);                     // the row whose Q is moved next
     if (direct_q) u = 1;
     else if (q_item < n_items) move_q();
     for (int idx = blockIdx.x; idx < n_items; idx += step) {
-      const FtItem it = ft_item<G4>(a, idx);
+      const FtItem it = ft_item<G4, CL>(a, idx);
       float m = -INFINITY, l = 0.f;
       for (int tile = 0; tile < it.n_tiles; tile++, u++, g++) {
-        const int b = g & 1, kb = u % FT_NBUF;
-        ok = tc::mbar_wait<FT_POLL_NS>(&ms.full[kb], (u / FT_NBUF) & 1, abort_flag, 6) && ok;   // makes the tile's mask visible
+        const int b = g & 1, kb = slot_of(it, u, tile);
+        ok = tc::mbar_wait<FT_POLL_NS>(full_of(kb), turn_of(it, u, tile) & 1, abort_flag, 6) && ok;   // makes the tile's mask visible
         ok = tc::mbar_wait<FT_POLL_NS>(&ms.s_full[b], (g >> 1) & 1, abort_flag, 7) && ok;
         tc::fence_after_sync();
         uint32_t sv[32];
@@ -430,7 +488,7 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
           wait_pv(g - 1, 8);
           tc::fence_after_sync();
 #pragma unroll 1
-          for (int c0 = 0; c0 < 256; c0 += 32) {
+          for (int c0 = 0; c0 < (CL ? 256 / a.n_cs : 256); c0 += 32) {
             uint32_t o[32];
             tc::tmem_ld32(tmem + FT_O + c0 + lanes, o);
             tc::tmem_ld_wait();
@@ -474,7 +532,8 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
       tc::fence_after_sync();
       asm volatile("bar.sync 3, 128;" ::: "memory");
       l += ms.l[tid ^ 64];
-      const float f = l > 0.f ? (final_out ? 1.f / l : 1.f) : 0.f;
+      const float f = l > 0.f ? (final_out && !CL ? 1.f / l : 1.f) : 0.f;
+      if (CL) cluster_arrive();                            // this CTA's ring is idle
       auto load_o = [&](int c0, uint32_t (&o)[32]) {       // 32 of this thread's 256 channels, weighed
         if (it.n_tiles > 0) {
           tc::tmem_ld32(tmem + FT_O + c0 + lanes, o);
@@ -483,7 +542,33 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
 #pragma unroll
         for (int j = 0; j < 32; j++) o[j] = l > 0.f ? __float_as_uint(__uint_as_float(o[j]) * f) : 0u;
       };
-      if (final_out) {
+      if (CL) {
+        // The accumulator goes to the cluster's CTAs by heads: CTA j merges n_h of them.  It is laid out by destination in the idle
+        // ring - n_h heads of the cluster's channels (16-byte chunk c of head h at c ^ (h % 8)), then their (m, l) - and leaves as one
+        // bulk copy per CTA (16-byte remote stores: 3.6 us for 32 KB).
+        const int n_h = FT_HEADS / a.n_split, row = LATENT / a.n_cs * 4, share = n_h * (row + 8), j = head / n_h;
+        uint8_t* const out = smem + FS_K + FT_CL_STAGE + j * share;
+#pragma unroll 1
+        for (int c0 = 0; c0 < 256 / a.n_cs; c0 += 32) {
+          uint32_t o[32];
+          load_o(c0, o);
+          const int lc = a.n_cs == 4 ? half * 64 + c0 : half * 128 + c0;   // channel within the cluster's part
+#pragma unroll
+          for (int v = 0; v < 8; v++)
+            *reinterpret_cast<uint4*>(out + (head - j * n_h) * row + ((((lc >> 2) + v) ^ (head & 7)) << 4)) =
+                make_uint4(o[4 * v], o[4 * v + 1], o[4 * v + 2], o[4 * v + 3]);
+        }
+        if (half == 0) *reinterpret_cast<float2*>(out + n_h * row + (head - j * n_h) * 8) = make_float2(l > 0.f ? m : -INFINITY, l);
+        tc::fence_before_sync();
+        tc::fence_async_smem();
+        asm volatile("bar.sync 3, 128;" ::: "memory");
+        cluster_wait();                                    // and so are the others'
+        if (tid < a.n_split)
+          asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                           cluster_addr(tc::smem_u32(smem + FS_K) + it.sp * share, tid)),
+                       "r"(tc::smem_u32(smem + FS_K + FT_CL_STAGE) + tid * share), "r"(share), "r"(cluster_addr(tc::smem_u32(&ms.q_ready), tid))
+                       : "memory");
+      } else if (final_out) {
         // Four rounds of 2 x 64 channels through the P buffers: channels 256 (c0 / 128) + 128 half + c0 % 128 ... of all heads
         // as a swizzled box each.
 #pragma unroll 1
@@ -548,6 +633,45 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
       }
     }
   }
+  if (CL) {
+    if (warp >= 4) {
+      cluster_arrive();
+      cluster_wait();
+    }
+    ok = tc::mbar_wait(&ms.q_ready, 0, abort_flag, 16) && ok;   // every split's share of this CTA's heads has arrived
+    cluster_arrive();
+    const FtItem it = ft_item<G4, CL>(a, blockIdx.x);
+    const int n_h = FT_HEADS / a.n_split, row = LATENT / a.n_cs * 4, share = n_h * (row + 8), chunks = row / 16;
+    if (!*abort_flag) {
+      for (int i = tid; i < n_h * chunks; i += FT_THREADS) {
+        const int h = i / chunks, c = i - h * chunks, head = it.sp * n_h + h;
+        const uint8_t* part = smem + FS_K;
+        const uint8_t* ml = part + n_h * row + h * 8;
+        float gm = -INFINITY, gl = 0.f;
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        // short loops: this code runs once, from a cold instruction cache (unrolled sixteen times 3,100 cycles)
+#pragma unroll 4
+        for (int sp = 0; sp < a.n_split; sp++) gm = fmaxf(gm, *reinterpret_cast<const float*>(ml + sp * share));
+        if (gm == -INFINITY) gm = 0.f;
+        const uint8_t* src = part + h * row + ((c ^ (head & 7)) << 4);
+#pragma unroll 4
+        for (int sp = 0; sp < a.n_split; sp++) {
+          const float2 x = *reinterpret_cast<const float2*>(ml + sp * share);
+          const float4 v = *reinterpret_cast<const float4*>(src + sp * share);
+          const float w = exp2f(x.x - gm);                 // no keys: 0
+          gl = fmaf(w, x.y, gl);
+          o.x = fmaf(w, v.x, o.x); o.y = fmaf(w, v.y, o.y); o.z = fmaf(w, v.z, o.z); o.w = fmaf(w, v.w, o.w);
+        }
+        const float inv = gl > 0.f ? 1.f / gl : 0.f;
+        const __half2 h0 = __floats2half2_rn(o.x * inv, o.y * inv), h1 = __floats2half2_rn(o.z * inv, o.w * inv);
+        uint2 w;
+        w.x = *reinterpret_cast<const uint32_t*>(&h0);
+        w.y = *reinterpret_cast<const uint32_t*>(&h1);
+        *reinterpret_cast<uint2*>(a.out + ((size_t)it.r * FT_HEADS + head) * LATENT + it.cs * (LATENT / a.n_cs) + c * 4) = w;
+      }
+    }
+    cluster_wait();                                        // nobody copies from this CTA's memory any more
+  }
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, 512);
@@ -569,6 +693,58 @@ int mla_flash_tc_auto_splits(int m, int n_keys) {
   return n_split < 1 ? 1 : n_split;
 }
 
+static int ft_prepare() {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    if (cudaFuncSetAttribute(mla_flash_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(mla_flash_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(mla_flash_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(mla_flash_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(mla_flash_tc_kernel<false, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(mla_flash_tc_kernel<true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+      return HK_ERR_CUDA;
+    attr_set[dev] = true;
+  }
+  return HK_OK;
+}
+
+// Cluster form: splits of a row and parts of its channels for m rows of about `tiles` tiles, false where it is not the better one.
+// One row, four parts of the channels, two tiles a split.  2,052 gathered rows 9.2 us against 10.8 with partials in memory; two rows
+// find room for two parts each only (16 CTAs with a whole SM's memory in one GPC: seven clusters at once), whose shares of twice the size
+// take longer to cross: 11.7 against 11.6, three 12.2 against 12.5, and from four rows on the partials' own kernel fills the GPU.
+bool mla_flash_cluster_shape(int m, int tiles, int* n_split, int* n_cs) {
+  int c = 2;
+  while (c < FT_MAX_CL && c * 2 < tiles) c *= 2;
+  if (tiles < 2 || tiles > 2 * FT_MAX_CL + 1 || m != 1) return false;
+  static int fit[64][5] = {{0}};                           // clusters of 2^i CTAs that run at once, + 1
+  int dev = 0, lg = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || ft_prepare() != HK_OK) return false;
+  while ((1 << lg) < c) lg++;
+  if (fit[dev][lg] == 0) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = c;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(FT_THREADS);
+    cfg.dynamicSmemBytes = FS_SMEM;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, mla_flash_tc_kernel<true, true>, &cfg) != cudaSuccess) n = 0;
+    fit[dev][lg] = n + 1;
+  }
+  const int room = fit[dev][lg] - 1;
+  if (room < 4) return false;
+  *n_split = c;
+  *n_cs = 4;
+  return true;
+}
+
 typedef CUresult (*FtEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -588,15 +764,7 @@ static FtEncodeFn ft_encode_fn() {
 int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s) {
   FtEncodeFn encode = ft_encode_fn();
   if (a.n_heads != FT_HEADS || !encode) return HK_ERR_UNSUPPORTED;
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(mla_flash_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(mla_flash_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess)
-      return HK_ERR_CUDA;
-    attr_set[dev] = true;
-  }
+  if (ft_prepare() != HK_OK) return HK_ERR_CUDA;
   // Tensor maps over the latent cache.  The row extent is the cache's row count when the caller gave it (the copy engine
   // zero-fills anything past the end), else an upper bound.
   alignas(64) CUtensorMap box, rows, qmap, omap;
@@ -635,11 +803,19 @@ int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s) {
   }
   // Gathered rows: at most a CTA per SM (592 rows of 2,048 keys 180 -> 166 us).  Dense rows, whose loads start faster: a CTA
   // each (600 rows at 32,768 keys 2.72 ms, persistent 2.85).  Partials always: their rows leave through the idle ring.
+  if (a.n_cs > 0) {
+    const dim3 grid((unsigned)(a.m * a.n_cs * a.n_split));
+    const cudaError_t e = a.raw_idx ? pdl_launch_cluster(a.n_split, mla_flash_tc_kernel<true, true>, grid, dim3(FT_THREADS), FS_SMEM, s, a,
+                                                         device_status_ptr(), box, rows, qmap, omap)
+                                    : pdl_launch_cluster(a.n_split, mla_flash_tc_kernel<false, true>, grid, dim3(FT_THREADS), FS_SMEM, s, a,
+                                                         device_status_ptr(), box, rows, qmap, omap);
+    return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+  }
   const int64_t items = (int64_t)a.n_split * a.m;
   const dim3 grid((unsigned)(a.raw_idx && a.out && items > sm_count() ? sm_count() : items));
   const cudaError_t e =
-      a.raw_idx ? pdl_launch(mla_flash_tc_kernel<true>, grid, dim3(FT_THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap)
-                : pdl_launch(mla_flash_tc_kernel<false>, grid, dim3(FT_THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap);
+      a.raw_idx ? pdl_launch(mla_flash_tc_kernel<true, false>, grid, dim3(FT_THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap)
+                : pdl_launch(mla_flash_tc_kernel<false, false>, grid, dim3(FT_THREADS), FS_SMEM, s, a, device_status_ptr(), box, rows, qmap, omap);
   return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
 

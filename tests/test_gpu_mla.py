@@ -45,6 +45,28 @@ def test_sparse_vs_oracle_and_reference(m, kidx, T, scale, n_split):
         assert sum_rel(rr, o32) < 3e-3, "oracle pinned to the reference kernel"
 
 
+@pytest.mark.parametrize("kidx", [65, 128, 129, 144, 145, 520, 1041, 2048, 2064, 2065, 2112, 2113])
+def test_one_row_merged_in_a_cluster(kidx):
+    """one row of up to 33 tiles: clusters of 2 to 16 CTAs, with and without a ragged tile of up to 16 keys as a split's third,
+    gathered (some rows holes, whole splits of them too) and dense"""
+    T = 4096
+    inp, ridx = _sparse_case(1, kidx, T, 0.0625, seed=kidx)
+    ridx[:, 64:200] = -1
+    q, c = dev_f16(inp["q_lat"]), dev_f16(inp["ckv"])
+    out = torch.empty(1, 64, 512, dtype=torch.float16, device="cuda")
+    for lens in (None, np.array([kidx], dtype=np.int32)):
+        kw = dict(raw_idx=ridx, kidx=kidx) if lens is None else dict(kv_base=np.array([7], dtype=np.int64), kv_len=lens)
+        _, o32 = orc.mla_attend(inp["q_lat"], inp["ckv"], 1, 64, 0.0625, **kw)
+        if lens is None:
+            hk.mla_sparse_decode(q, c, dev(ridx), kidx, out, 1)
+        else:
+            hk.mla_dense_prefill(q, c, out, 1, 0, kv_base=dev(kw["kv_base"]), kv_len=dev(lens), n_keys_hint=kidx)
+        torch.cuda.synchronize()
+        assert hk.read_device_status() == 0
+        g = synth.f16_bits_to_f32(bits(out))
+        assert max_rel(g, o32) < TOL and sum_rel(g, o32) < 3e-3
+
+
 def test_sparse_all_skipped_row_gives_zeros_and_duplicates_count_twice():
     m, kidx, T = 2, 16, 64
     inp, ridx = _sparse_case(m, kidx, T, 0.0625, seed=1, holes=False)
