@@ -369,20 +369,32 @@ __device__ long long hk_topk_trace[16];
 // A few long rows (the decode case is ONE row): a thread-block cluster of 8 CTAs works on a row, CTA c on pieces
 // [1024 NP c, 1024 NP (c + 1)), every thread on NP consecutive pieces of 8 elements that stay in registers, so the row is
 // read from global memory once and no sweep is longer than 8 NP keys per thread.  The CTAs meet through distributed shared
-// memory: the bucket histograms are summed slice-wise and the sums stored into every CTA, each CTA then finds the crossing
-// bucket itself; the low-bit count sets are read by every CTA, which finds the threshold and, from the per-CTA counts, the
-// offset of its own ordered output - four cluster barriers in all, no hand-back round trips.
-// NP = 1, 2, 4 cover rows of 65,535, 131,071 and 262,143 scores at any alignment (1M tokens of context).  One row of 65,540
-// scores (262,160 tokens) took 33.9 us in the one-CTA kernel and takes 9.3 us here.
+// memory: every CTA adds up the row's buckets by eights from all eight CTAs, then looks at the eight buckets of the crossing one; the
+// low-bit count sets are read by every CTA, which finds the threshold and, from the per-CTA counts, the offset of its own
+// ordered output - two cluster barriers that hand data over and one that is arrived at long before it is waited for.
+// What bounds it: these steps one after the other (load and count 1.5 us, the crossing bucket 1.0, low bits 0.9, offsets 0.9, output 1.0).
+// One row of 65,536 scores 6.8 -> 5.8 us against sharing out the 2,048 sums by slices (four barriers); 262,000 scores 18.5 -> 11.8, 16 rows of
+// 30,000 13.9 -> 10.9 (the launch bound names the CTA per SM: at the 32 registers taken without it the four-piece form spilled).
+// NP = 1, 2, 4 cover rows of 65,535, 131,071 and 262,143 scores at any alignment (1M tokens of context).
 // ------------------------------------------------------------------------------------------------
 constexpr int TKC_CTAS = 8;
 constexpr int TKC_PIECES = TKC_CTAS * TK_THREADS;         // pieces of 8 elements that NP = 1 holds
 constexpr int TKC_MAX_NP = 4;
 
 template <int NP>
-__global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void dsa_topk_cluster_kernel(
+__global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) void dsa_topk_cluster_kernel(
     const uint16_t* scores, int* __restrict__ out, int T, int s_stride, int k, int k_pad,
     int* __restrict__ raw, const int* __restrict__ q_pos) {
+  __shared__ __align__(16) int hist[2048];   // this CTA's bucket counts
+  __shared__ int coarse[256];      // the same by eight buckets
+  __shared__ int low[33];          // this CTA: counts of the low 5 bits inside the crossing bucket; [32] = keys above it
+  __shared__ int wsum[2][TK_WARPS];
+  __shared__ int sh_sel[3];
+  __shared__ int sh_off[6];        // threshold low bits, count above threshold, this CTA's bases, total ties
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int i = t; i < 2048; i += TK_THREADS) hist[i] = 0;
+  if (t < 33) low[t] = 0;
+  if (t == 0) sh_sel[0] = -1;
   namespace cg = cooperative_groups;
   pdl_release();
   pdl_wait();
@@ -392,48 +404,63 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
   const uint16_t* row = scores + (size_t)row_id * s_stride;
   const TopkSink row_o{out + (size_t)row_id * k_pad,
                        raw ? reinterpret_cast<int4*>(raw + (size_t)row_id * (4 * k_pad + 4)) : nullptr, raw ? q_pos[row_id] : 0};
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-
-  __shared__ int hist[2048];       // this CTA's bucket counts
-  __shared__ int ghist[2048];      // bucket counts of the whole row (every CTA gets a copy)
-  __shared__ int low[33];          // this CTA: counts of the low 5 bits inside the crossing bucket; [32] = keys above it
-  __shared__ int scan_ws[TK_WARPS + 1];
-  __shared__ int sh_sel[3];
-  __shared__ int sh_off[6];        // threshold low bits, count above threshold, this CTA's bases, total ties
 
   TK_TRACE(0);
   const int lead = row_lead(row), i8 = (c * TK_THREADS + t) * NP;
   uint4 pc[NP];
 #pragma unroll
   for (int u = 0; u < NP; u++) pc[u] = load8_raw(row, lead, i8 + u, T);
-  for (int i = t; i < 2048; i += TK_THREADS) hist[i] = 0;
-  if (t < 33) low[t] = 0;
   __syncthreads();
+  // exclusive prefix over the block; one barrier, `slot` alternates between calls
+  auto exscan = [&](int v, int slot, int* total) {
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += n;
+    }
+    if (lane == 31) wsum[slot][warp] = incl;
+    __syncthreads();
+    const int x = wsum[slot][lane];
+    const int before = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < warp ? x : 0));
+    *total = (int)__reduce_add_sync(0xffffffffu, (unsigned)x);
+    return before + incl - v;
+  };
   for_keys<NP>(pc, [&](int, uint32_t key) {
     if (key > KEY_NEG_INF) atomicAdd(&hist[key >> 5], 1);
   });
-  cluster.sync();                  // (1) all local histograms complete
-  TK_TRACE(1);
-  // slice c of the buckets is summed over the eight CTAs by CTA c and stored into EVERY CTA's copy of
-  // the row histogram (reading all eight histograms in all eight CTAs costs far more distributed traffic)
-  if (t < 2048 / TKC_CTAS) {
-    const int bin = c * (2048 / TKC_CTAS) + t;
-    int sum = 0;
-#pragma unroll
-    for (int rk = 0; rk < TKC_CTAS; rk++) sum += cluster.map_shared_rank(hist, rk)[bin];
-#pragma unroll
-    for (int rk = 0; rk < TKC_CTAS; rk++) cluster.map_shared_rank(ghist, rk)[bin] = sum;
-  }
-  cluster.sync();                  // (2) every CTA holds the row histogram
-  // thread t owns buckets 2047-2t and 2046-2t (descending) and finds where the running count crosses k
-  const int h_hi = ghist[2047 - 2 * t], h_lo = ghist[2046 - 2 * t];
-  int total_sel;
-  const int excl = block_exscan(h_hi + h_lo, scan_ws, &total_sel);
-  if (t == 0) { sh_sel[0] = -1; sh_sel[1] = 0; }
   __syncthreads();
-  if (total_sel >= k && k > 0) {
-    if (excl < k && excl + h_hi >= k) { sh_sel[0] = 2047 - 2 * t; sh_sel[1] = excl; }
-    else if (excl + h_hi < k && excl + h_hi + h_lo >= k) { sh_sel[0] = 2046 - 2 * t; sh_sel[1] = excl + h_hi; }
+  if (t < 256) {
+    const int4 x = *reinterpret_cast<const int4*>(hist + 8 * t), y = *reinterpret_cast<const int4*>(hist + 8 * t + 4);
+    coarse[t] = x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w;
+  }
+  cluster.sync();                  // (1) all local histograms are complete
+  TK_TRACE(1);
+  // Thread t < 256 sums eight buckets over the row (descending) and finds where the running count crosses k; a warp then looks at the
+  // eight.  Every CTA does so for itself: 8 KB of remote counts each and one cluster barrier less than sharing out the sums.
+  int sum = 0;
+  if (t < 256) {
+#pragma unroll
+    for (int rk = 0; rk < TKC_CTAS; rk++) sum += cluster.map_shared_rank(coarse, rk)[255 - t];
+  }
+  int total_sel;
+  const int excl = exscan(sum, 0, &total_sel);
+  if (k > 0 && excl < k && excl + sum >= k) { sh_sel[0] = 255 - t; sh_sel[1] = excl; }
+  __syncthreads();
+  if (warp == 0 && sh_sel[0] >= 0) {
+    // lane 8 r + j: bucket j from the top of the eight, CTAs r and r + 4
+    const int bin = 8 * sh_sel[0] + 7 - (lane & 7), above = sh_sel[1];
+    int v = cluster.map_shared_rank(hist, lane >> 3)[bin] + cluster.map_shared_rank(hist, (lane >> 3) + 4)[bin];
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, incl, o, 8);
+      if ((lane & 7) >= o) incl += n;
+    }
+    __syncwarp();
+    if (lane < 8 && above + incl - v < k && above + incl >= k) { sh_sel[0] = bin; sh_sel[1] = above + incl - v; }
   }
   __syncthreads();
   const int b1 = sh_sel[0], above1 = sh_sel[1];
@@ -447,10 +474,9 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
     if (bk == b1) atomicAdd(&low[key & 31u], 1);
     n_above += bk > b_eff;
   });
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) n_above += __shfl_xor_sync(0xffffffffu, n_above, o);
+  n_above = (int)__reduce_add_sync(0xffffffffu, (unsigned)n_above);
   if (lane == 0 && n_above) atomicAdd(&low[32], n_above);
-  cluster.sync();                  // (3) all local low-bit counts complete
+  cluster.sync();                  // (2) all local low-bit counts complete
   TK_TRACE(3);
   if (warp == 0) {
     // lane l owns low value 31-l (descending); per CTA counts first, then the row's
@@ -480,9 +506,7 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
       int base_gt = 0, base_eq = 0, all_eq = 0;
 #pragma unroll
       for (int rk = 0; rk < TKC_CTAS; rk++) {
-        int hi = lane < src ? mine[rk] : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) hi += __shfl_xor_sync(0xffffffffu, hi, o);
+        const int hi = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < src ? mine[rk] : 0));
         const int eq = __shfl_sync(0xffffffffu, mine[rk], src);
         if (rk < c) { base_gt += above_c[rk] + hi; base_eq += eq; }
         all_eq += eq;
@@ -498,6 +522,8 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
     if (lane == 0) { sh_off[0] = lowbits; sh_off[1] = cnt_gt_row; sh_off[5] = need_eq; }
   }
   __syncthreads();
+  // no CTA leaves while a peer may still read its shared memory: this one has read the others'
+  asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
   uint32_t thresh;
   const int cnt_gt = sh_off[1], n_eq_take = sh_off[5];
   if (b1 < 0) thresh = k == 0 ? 0xffffu : KEY_NEG_INF;
@@ -510,7 +536,7 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
     if (key == thresh && n_eq_take > 0) m_eq |= 1u << j;
   });
   int tot;
-  const int ex = block_exscan(__popc(m_gt) | (__popc(m_eq) << 16), scan_ws, &tot);
+  const int ex = exscan(__popc(m_gt) | (__popc(m_eq) << 16), 1, &tot);
   TK_TRACE(5);
   int o_gt = sh_off[2] + (ex & 0xffff);
   int o_eq = sh_off[3] + (ex >> 16);
@@ -532,7 +558,7 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS) void d
     if (t == 0) row_o.put_tail(k_pad);
   }
   TK_TRACE(6);
-  cluster.sync();                  // (4) no CTA leaves while a peer may still read its shared memory
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 }  // namespace hk
