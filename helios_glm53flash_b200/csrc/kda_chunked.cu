@@ -29,7 +29,7 @@
 #include <cuda.h>   // CUtensorMap (types only; the encoder is fetched through the runtime at first use)
 #include <cuda_pipeline_primitives.h>
 
-#include <cstring>
+#include <climits>
 
 #include "hk_common.cuh"
 #include "tc05.cuh"
@@ -38,10 +38,10 @@ namespace hk {
 
 constexpr int KC = 64;                    // chunk length
 constexpr int KD = 128;                   // head dim (k and v)
-constexpr int KNV = 32;                   // value columns per scan CTA
-constexpr int KVS = KD / KNV;             // value slices
-constexpr int KR = 16;                    // fused form: ring slots (chunks) per chain
-// Flags: [0] launch-wide abort word, then a 128-byte line of ready flags and one for the consumed count per chain slot.  With all of
+// Fused form: ring slots (chunks) per chain slot, a power of two up to 32.  A worker's unit takes ten chunks of a chain from the moment
+// its ring slot is free; few long chains are waited for by many workers and get the deeper ring, many chains keep theirs within L2.
+__host__ __device__ constexpr int ring_depth(int n_slots, int n_virtual) { return n_slots <= 16 && n_virtual >= 64 ? 32 : 16; }
+// Flags: [0] launch-wide abort word, then a 128-byte line of ready flags per chain slot and one for the consumed count per chain CTA.  With all of
 // them packed into a few lines of one page the polls of 232 workers held up the chains' own flags: 1.05 or 1.3-1.9 ms for 32,768
 // tokens x 32 heads, by the die that the page's address falls to.
 constexpr int F_FLAG_INTS = 32;
@@ -147,17 +147,6 @@ constexpr int P1_LDX = 20;                               // pitch of a diagonal 
 
 __device__ __forceinline__ int prep_n_row(int t) { return t < 32 ? t * 36 : 32 * 36 + (t - 32) * 68; }
 __device__ __forceinline__ int prep_inv_at(int blk) { return blk * 16 * P1_LDX; }
-
-// Optional stage timeline (diagnostic build, -DHK_DIAG): one scan CTA stamps clock64 at its stage boundaries;
-// hk_debug_kda_trace copies the stamps to the host.
-#ifdef HK_DIAG
-__device__ long long hk_kda_trace[128];
-#define KS_TRACE(slot, ch) do { if (threadIdx.x == 0 && blockIdx.x == 1 && (ch) == 100) hk_kda_trace[32 + (slot)] = clock64(); } while (0)
-#define KS_TRACE_AT(slot, ch, want) do { if (threadIdx.x == 0 && blockIdx.x == 1 && (ch) == (want)) hk_kda_trace[32 + (slot)] = clock64(); } while (0)
-#else
-#define KS_TRACE_AT(slot, ch, want) do { } while (0)
-#define KS_TRACE(slot, ch) do { } while (0)
-#endif
 
 // 16 x 16 left operand of a block product as TF32 heads and tails.  The contraction index is taken in the order in which an
 // accumulator holds its columns (k slots tig and tig + 4 of step s are columns 8 s + 2 tig and 8 s + 2 tig + 1), so that the
@@ -303,11 +292,11 @@ __device__ __forceinline__ void prep_init(PrepShared& sh) {  // one thread
 // release store is cumulative over them.  It waits until the CTA's stores are visible, some thousand cycles when they are fresh: it is
 // put off to a place in the next unit where its warp has little else to do, unless the worker has to wait for its ring slot.
 constexpr int PUB_WARP = 2;
-__device__ __forceinline__ void prep_publish(const PrepCtx& ctx, int it, int* ready, int n_slots) {
+__device__ __forceinline__ void prep_publish(const PrepCtx& ctx, int it, int* ready, int kr) {
   asm volatile("bar.sync %0, 256;" ::"r"(ctx.bar_id + 2) : "memory");
   if (ctx.tid == PUB_WARP * 32) {
     const int value = PREP_UNIT(value, it);
-    st_release_gpu(ready + (size_t)PREP_UNIT(slot, it) * F_LINE + (value - 1) % KR, value);
+    st_release_gpu(ready + (size_t)PREP_UNIT(slot, it) * F_LINE + ((value - 1) & (kr - 1)), value);
   }
 }
 
@@ -345,14 +334,16 @@ __device__ __forceinline__ void prep_fetch_qkv(const PrepCtx& ctx, int it, const
 //   g = lower_bound * sigmoid(exp(a_log[head]) * (f + dt_bias[head][channel])),  beta = bf16(sigmoid(b))
 // itself (the arithmetic of the reference's separate gate kernel, src/engine/glue2.cu:347-360), so the
 // fp32 gate tensor is never written to or read back from memory.
-// The unit's inputs are on their way (prep_fetch_*); its end sends for those of the next.  SUB: `ready` and `consumed` are the flags
+// The unit's inputs are on their way (prep_fetch_*); its end sends for those of the next.
+// SLICES: chain CTAs of a slot in the fused form (SUB), 0 in the two-kernel form.  SUB: `ready` and `consumed` are the flags
 // of the ring; on return the unit's last writes are on their way and its flag is still to be stored (prep_publish).
 // `make_unit(it, desc)` works out the next unit (one thread).
-template <bool GATED, bool SUB, class MakeUnit>
+template <bool GATED, int SLICES, class MakeUnit>
 __device__ __forceinline__ void prep_unit(
     const PrepCtx& ctx, const int it, const CUtensorMap* map_qkv, const CUtensorMap* map_g, const void* __restrict__ beta_in,
     uint8_t* __restrict__ units, int H, const float* __restrict__ dt_bias, const float* __restrict__ a_log, float lower_bound,
-    const uint32_t tmem, int* ready, const int* consumed, int* g_abort, int n_slots, MakeUnit&& make_unit) {
+    const uint32_t tmem, int* ready, const int* consumed, int* g_abort, int kr, MakeUnit&& make_unit) {
+  constexpr bool SUB = SLICES > 0;
   uint8_t* const smem = ctx.smem;
   uint8_t* const sK = smem + P1_K;
   float* const sX = reinterpret_cast<float*>(smem + P1_X);
@@ -373,8 +364,9 @@ __device__ __forceinline__ void prep_unit(
   // ---- stage 1: log-decay sums.  x_t = inclusive sum of the log decay (in units of log 2) INSIDE the 16-token block, in place;
   //      lane 8 J + p of warp w sums channels 16 w + 2 p, + 1 over block J, so the block totals of a channel sit in four lanes
   //      of one warp, which turn them into the tables ----
-  int seen = 0;                                            // publishing warp's first lane: chunks of the slot that have been consumed
-  if (SUB && tid == PUB_WARP * 32) seen = ld_relaxed_gpu(consumed + PREP_UNIT(slot, it) * F_LINE);
+  int seen = INT_MAX;                                      // publishing warp's first lanes: chunks that each CTA of the slot has consumed
+  if (SUB && tid >= PUB_WARP * 32 && tid < PUB_WARP * 32 + SLICES)
+    seen = ld_relaxed_gpu(consumed + (PREP_UNIT(slot, it) * SLICES + tid - PUB_WARP * 32) * F_LINE);
   float beta = 0.f;
   if (t < PREP_UNIT(n_valid, it)) {
     const size_t bi = (size_t)(PREP_UNIT(tok0, it) + t) * H + PREP_UNIT(head, it);
@@ -464,11 +456,12 @@ __device__ __forceinline__ void prep_unit(
   // fused form: the ring slot must have been drained before the first write to the unit (all of them follow)
   bool unpublished = SUB && it > 0;                        // the flag of the unit before this one
   if (SUB && warp == PUB_WARP) {
-    const int want = PREP_UNIT(value, it) - KR;            // the slot held chunk value - 1 - KR
-    if (__shfl_sync(0xffffffffu, seen, 0) < want) {
-      if (unpublished) prep_publish(ctx, it - 1, ready, n_slots);   // before a wait: the chains may need that unit to get on
+    const int want = PREP_UNIT(value, it) - kr;            // the slot held chunk value - 1 - kr
+    if (__any_sync(0xffffffffu, seen < want)) {
+      if (unpublished) prep_publish(ctx, it - 1, ready, kr);   // before a wait: the chains may need that unit to get on
       unpublished = false;
-      if (lane == 0) poll_flag_ge(consumed + PREP_UNIT(slot, it) * F_LINE, want, ctx.abort_flag, g_abort, 20);
+      if (lane < SLICES) poll_flag_ge(consumed + (PREP_UNIT(slot, it) * SLICES + lane) * F_LINE, want, ctx.abort_flag, g_abort, 20);
+      __syncwarp();
     }
   }
   prep_sync<SUB>(ctx);                                     // x and the tables are complete, q and k have been read
@@ -580,7 +573,7 @@ __device__ __forceinline__ void prep_unit(
 
   // ---- stage 3: the products with earlier blocks (fp16), 2 I tiles a warp; the warps of the first block, which have none, invert the
   //      16 x 16 diagonal blocks of I + N, those of the second and third convert v as well ----
-  if (SUB && warp == PUB_WARP && unpublished) prep_publish(ctx, it - 1, ready, n_slots);
+  if (SUB && warp == PUB_WARP && unpublished) prep_publish(ctx, it - 1, ready, kr);
   {
     float* nrow = sN + prep_n_row(t) + 2 * tig;
     uint8_t* bbrow = PREP_OUT + U_BB + warp * SBO_K64 + g8 * 16 + tig * 4;
@@ -764,15 +757,30 @@ __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  prep_unit<GATED, false>(ctx, 0, &map_qkv, &map_g, beta_in, ws, H, dt_bias, a_log, lower_bound, tmem_slot, nullptr, nullptr, nullptr, 0,
-                          [](int, PrepDesc&) {});
+  prep_unit<GATED, 0>(ctx, 0, &map_qkv, &map_g, beta_in, ws, H, dt_bias, a_log, lower_bound, tmem_slot, nullptr, nullptr, nullptr, 0,
+                      [](int, PrepDesc&) {});
   __syncthreads();
   if (tid < 32) tc::tmem_dealloc(tmem_slot, 128);
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
 }
 
 // =================================================================================================
-// kernel 2: sequential scan over the chunks of one (batch, head, value slice)
+// The scan: one CTA of 512 threads walks the chunks of a chain in order, with NV of the head's 128 value columns (whose states, U and
+// outputs do not depend on the other columns').  Shared by kernel 2 (units in a workspace) and the fused launch (units in a ring).
+//
+// Sixteen warps = four TMEM lane quarters (lq) x four groups, joined by mbarriers that complete once per chunk, never by the
+// whole CTA; what is on the chunk-to-chunk chain is spread over many warps, the rest has warps of its own:
+//   U         lq 0, 1 of all groups (token rows of D1), NV / 4 columns each
+//   state     groups 0, 1: a k row and NV / 2 of its columns per thread, fp32 in registers
+//   outputs   warps 10, 11: a token row each thread
+//   issuer    warp 14: every product; it waits for operands only
+//   producer  warp 15: ring protocol and operand copies
+// A barrier's next phase cannot complete before its waiters have seen this one: U needs every U warp, the state operand every
+// state warp; out_bar and d1_bar alternate by chunk, since the output warps may be a chunk behind or done with the one before.
+//
+// What bounds it: the products and hand-overs of a chunk in turn.  In cycles, NV = 128: state -> U 900 (eight products of 65, 350 until
+// they are seen), U 500, Kt^T U 540, state 650, operand -> issuer 100: 2.7 thousand (2.1 with NV = 64, products of 49).  The form before, whose
+// warps met at block barriers and emitted outputs in between, took 4.1 to 5.4.
 // =================================================================================================
 // fp16 A operand [I ; 0] (128 rows, K = 64) without storing it: its core matrix (i, j) depends on i - j only, so 23 core
 // matrices, one of them the identity, serve all of them with 128 bytes as both strides.  The two core matrices of a K16 step then
@@ -786,310 +794,408 @@ __device__ __forceinline__ void write_identity(uint8_t* dst, int tid, int nthrea
   }
 }
 
-constexpr uint32_t S_WQ = 0;              // 32768
-constexpr uint32_t S_BB = 32768;          // 8192
-constexpr uint32_t S_KT = 40960;          // 16384
-constexpr uint32_t S_UL = 57344;          // 4096
-constexpr uint32_t S_DEC = 61440;         // 512
-constexpr uint32_t S_STAGE = 61952;
-constexpr int S_NSTAGE = 3;               // operand stages in flight: two chunks of lead time for the bulk copies
-constexpr uint32_t P2_S = S_NSTAGE * S_STAGE;  // fp16 B operand: state slice [128 k][32], MN-major, 8 KB
-constexpr uint32_t P2_U = P2_S + 8192;    // fp16 B operand: U [64 tokens][32], MN-major, 4 KB
-constexpr uint32_t P2_ID = P2_U + 4096;   // [I ; 0]
-constexpr uint32_t P2_SMEM = P2_ID + ID_BYTES;
+// shared memory of a chain CTA: two operand stages (a unit with NV columns of Uloc), then the operands it makes itself
+template <int NV>
+struct Chain {
+  static constexpr int SLICES = KD / NV;
+  static constexpr uint32_t UL = U_UL, BB = UL + NV * 128, KT = BB + 8192, DEC = KT + 16384, STAGE = DEC + 512;
+  static constexpr uint32_t S = 2 * STAGE;                  // fp16 B operand: state [128 k][NV], MN-major
+  static constexpr uint32_t U = S + NV * 256;               // fp16 B operand: U [64 tokens][NV], MN-major
+  static constexpr uint32_t O = U + NV * 128;               // bf16 output rows of one chunk: swizzled boxes of 64 tokens x 64 channels
+  static constexpr uint32_t ID = O + NV * 128;              // [I ; 0]
+  static constexpr uint32_t SMEM = ID + ID_BYTES + 1024;    // + slack to start the tiles at a 1 KB boundary
+  static_assert(O % 1024 == 0 && STAGE % 128 == 0 && BB >= 8192, "layout");
+};
+struct ChainBars {                  // two of most kinds by chunk parity, so that a warp that is held up may be a chunk behind
+  uint64_t wu[2];                   // -W, Q+ and Uloc of a stage have landed
+  uint64_t kb[2];                   // B beta, Kt^T and the decays
+  uint64_t mma[2];                  // U and Q+ S0 are complete
+  uint64_t mma2;                    // Kt^T U (state path) is complete
+  uint64_t out[2];                  // (B beta) U is complete, and with it every product of the chunk
+  uint64_t u;                       // the 256 token-row threads have written U
+  uint64_t s[2];                    // the 256 state threads have written the state operand
+  uint64_t d1[2];                   // the two output warps have read this half of D1
+};
+__device__ __forceinline__ void chain_init(ChainBars& bars) {   // one thread
+  for (int i = 0; i < 2; i++) {
+    tc::mbar_init(&bars.wu[i], 1);
+    tc::mbar_init(&bars.kb[i], 1);
+    tc::mbar_init(&bars.mma[i], 1);
+    tc::mbar_init(&bars.out[i], 1);
+    tc::mbar_init(&bars.s[i], 256);
+    tc::mbar_init(&bars.d1[i], 2);
+  }
+  tc::mbar_init(&bars.mma2, 1);
+  tc::mbar_init(&bars.u, 256);
+}
+// Chains job0, job0 + job_step, ... of n_chunks chunks each, n_virtual chunks in all; a job is (batch, head).  Chunk numbers run through
+// all of them (`v`), and ring, flags and barrier parities go by v.  RING: `my_ready` and `my_consumed` are the slot's flags.
+// `unit_of(v)`: the unit of a chunk.
+template <int NV, bool RING, class UnitOf>
+__device__ __forceinline__ void chain_cta(uint8_t* smem, ChainBars& bars, const uint32_t tmem, int* abort_flag, UnitOf&& unit_of, const int* my_ready,
+                                          int* my_consumed, int* g_abort, int kr, int job0, int job_step, int n_chunks, int n_virtual, int slice, int H,
+                                          int seqlen, float* __restrict__ state, float* __restrict__ out_f32, const int* __restrict__ slots,
+                                          float scale, const CUtensorMap* map_out) {
+  using C = Chain<NV>;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lq = warp & 3, grp = warp >> 2;
+  const int rowi = lq * 32 + lane;                        // k row of the state / token row of U / output row + 64
+  const int role = tc::warp_index_uniform();
+  // D1 alternates between columns 0 .. NV - 1 and NV .. 2 NV - 1 by chunk parity, D2 follows
+  write_identity(smem + C::ID, tid, 512);
+  tc::fence_async_smem();
+  __syncthreads();
 
-__global__ __launch_bounds__(128, 1) void kda_chunk_scan_kernel(
-    const uint8_t* __restrict__ ws, float* __restrict__ state, __nv_bfloat16* __restrict__ out,
-    float* __restrict__ out_f32, int seqlen, int H, int n_chunks, const int* __restrict__ slots,
-    float scale, int* __restrict__ status) {
+  if (role == 14) {
+    const uint32_t leader = tc::elect_one();
+    const uint32_t idesc = tc::make_idesc(128, NV, tc::FMT_F16, tc::FMT_F16, false, true);
+    const uint32_t idesc_kt = tc::make_idesc(128, NV, tc::FMT_F16, tc::FMT_F16, true, true);   // Kt^T: channels contiguous
+    const uint32_t s_addr = tc::smem_u32(smem + C::S), u_addr = tc::smem_u32(smem + C::U), id_addr = tc::smem_u32(smem + C::ID);
+    // D1 of chunk w = [I ; 0] Uloc, ahead of the state: the product with the identity is exact
+    auto issue_uloc = [&](int w) {
+      tc::fence_after_sync();
+#pragma unroll
+      for (int kk = 0; kk < KC / 16; kk++) {
+        const uint64_t ad = tc::make_sdesc(id_addr + (6 - 2 * kk) * 128, 128, 128);
+        const uint64_t bd = tc::make_sdesc(tc::smem_u32(smem + (w & 1) * C::STAGE) + C::UL + kk * 2 * 128, 128, 1024);
+        tc::mma_f16_if(leader, tmem + (w & 1) * NV, ad, bd, idesc, kk > 0);
+      }
+    };
+    int uloc = 0;                                          // chunks whose Uloc has been issued
+    for (int v = 0; v < n_virtual; v++) {
+      const uint32_t par = v & 1, ph = (v >> 1) & 1, stg_addr = tc::smem_u32(smem + par * C::STAGE);
+      const uint32_t d1 = tmem + par * NV, d2 = tmem + 2 * NV;
+      if (uloc == v) {
+        tc::mbar_wait(&bars.wu[par], ph, abort_flag, 2);
+        if (v >= 2) tc::mbar_wait(&bars.d1[par], ph ^ 1, abort_flag, 8);   // the output rows of chunk v - 2 have left this half of D1
+        issue_uloc(v);
+        uloc++;
+      }
+      // ---- D1 += [-W ; Q+] S0 ----
+      tc::mbar_wait(&bars.s[par], ph, abort_flag, 6);
+      tc::fence_after_sync();
+#pragma unroll
+      for (int kk = 0; kk < KD / 16; kk++) {
+        const uint64_t ad = tc::make_sdesc(stg_addr + U_WQ + kk * 2 * LBO, LBO, SBO_K128);
+        const uint64_t bd = tc::make_sdesc(s_addr + kk * 2 * 128, 128, 2048);
+        tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
+      }
+      tc::mma_commit_if(leader, &bars.mma[par]);
+      // the next chunk's Uloc while U leaves the tensor memory, if its operands and its half of D1 are there already (otherwise at
+      // the chunk's start, where 260 cycles of products stand between the state and U)
+      if (v + 1 < n_virtual) {
+        const uint32_t nph = ((v + 1) >> 1) & 1;
+        const bool here = tc::mbar_test_wait(&bars.wu[par ^ 1], nph) && (v == 0 || tc::mbar_test_wait(&bars.d1[par ^ 1], nph ^ 1));
+        if (__all_sync(0xffffffffu, here)) {
+          issue_uloc(v + 1);
+          uloc++;
+        }
+      }
+      // ---- D2 = Kt^T U (state path), then D1 rows 64-127 += (B beta) U (outputs) ----
+      tc::mbar_wait(&bars.kb[par], ph, abort_flag, 11);
+      tc::mbar_wait(&bars.u, par, abort_flag, 7);
+      tc::fence_after_sync();
+#pragma unroll
+      for (int kk = 0; kk < KC / 16; kk++) {
+        const uint64_t ad = tc::make_sdesc(stg_addr + C::KT + kk * 2 * 128, 128, 1024);
+        const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
+        tc::mma_f16_if(leader, d2, ad, bd, idesc_kt, kk > 0);
+      }
+      tc::mma_commit_if(leader, &bars.mma2);
+      // rows 0-63 of this operand are whatever lies below B beta in the stage: they add to U's rows, which have been read
+#pragma unroll
+      for (int kk = 0; kk < KC / 16; kk++) {
+        const uint64_t ad = tc::make_sdesc(stg_addr + C::BB - 8192 + kk * 2 * LBO, LBO, SBO_K64);
+        const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
+        tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
+      }
+      tc::mma_commit_if(leader, &bars.out[par]);
+    }
+  } else if (role == 15) {
+    // a unit in two parts: a stage's first part is free as soon as the chunk's first product is complete, most of a chunk before
+    // the rest.  74 KB take about as long as a chunk to arrive.
+    auto load_wu = [&](int v) {
+      if (lane == 0) {
+        uint8_t* stg = smem + (v & 1) * C::STAGE;
+        const uint8_t* u = unit_of(v);
+        tc::mbar_arrive_expect_tx(&bars.wu[v & 1], C::BB);
+        tc::bulk_g2s(stg, u, NV == KD ? C::BB : C::UL, &bars.wu[v & 1]);
+        if (NV < KD) tc::bulk_g2s(stg + C::UL, u + U_UL + slice * (NV * 128), NV * 128, &bars.wu[v & 1]);
+      }
+      __syncwarp();
+    };
+    auto load_kb = [&](int v) {
+      if (lane == 0) {
+        tc::mbar_arrive_expect_tx(&bars.kb[v & 1], C::STAGE - C::BB);
+        tc::bulk_g2s(smem + (v & 1) * C::STAGE + C::BB, unit_of(v) + U_BB, C::STAGE - C::BB, &bars.kb[v & 1]);
+      }
+      __syncwarp();
+    };
+    // Units are asked for a ring at a time: a flag takes a microsecond or more to read while the workers poll theirs, too long for
+    // every chunk.
+    int known = 0;                                         // units before this one are complete
+    auto await_unit = [&](int v) {
+      if (!RING) return;
+      const long long t0 = clock64();
+      while (known <= v) {
+        const bool here = lane < kr && ld_acquire_gpu(my_ready + ((known + lane) & (kr - 1))) > known + lane;
+        const uint32_t missing = ~__ballot_sync(0xffffffffu, here);
+        known += missing ? __ffs(missing) - 1 : 32;
+        if (known > v) break;
+        const bool give_up = *(volatile int*)abort_flag || ld_relaxed_gpu(g_abort) != 0 || clock64() - t0 > tc::MBAR_WAIT_CYCLES;
+        if (__any_sync(0xffffffffu, give_up)) {
+          if (lane == 0) {
+            *(volatile int*)abort_flag = 21;
+            atomicExch(g_abort, 21);
+          }
+          break;
+        }
+        __nanosleep(64);
+      }
+      __syncwarp();
+      if (lane == 0) fence_proxy_async_all();
+    };
+    for (int v = 0; v < 2 && v < n_virtual; v++) {
+      await_unit(v);
+      load_wu(v);
+      load_kb(v);
+    }
+    for (int v = 0; v < n_virtual; v++) {
+      const uint32_t par = v & 1, ph = (v >> 1) & 1;
+      // the unit of this chunk has landed in shared memory: its slot may be rewritten.  A relaxed store is enough:
+      // the copy engine's reads are complete, nothing this thread wrote is handed over with the flag.
+      tc::mbar_wait(&bars.wu[par], ph, abort_flag, 2);
+      tc::mbar_wait(&bars.kb[par], ph, abort_flag, 2);
+      if (RING && lane == 0) st_relaxed_gpu(my_consumed, v + 1);
+      if (v + 2 >= n_virtual) continue;
+      await_unit(v + 2);
+      tc::mbar_wait(&bars.mma[par], ph, abort_flag, 3);
+      load_wu(v + 2);
+      // all products of the chunk are complete and the state warps have read its decays
+      tc::mbar_wait(&bars.out[par], ph, abort_flag, 5);
+      tc::mbar_wait(&bars.s[par ^ 1], ((v + 1) >> 1) & 1, abort_flag, 9);
+      load_kb(v + 2);
+    }
+  } else if (role == 10 || role == 11) {
+    // Output rows: TMEM lanes 64-127 of a chunk's D1 half = tokens; a thread holds the columns of one token.  Stored directly,
+    // a warp-wide 16-byte store would touch 32 different rows (32 L1 requests per instruction, over a thousand per chunk
+    // on this one SM).  The bf16 rows are therefore assembled in shared memory and leave as tiled TMA stores (64 tokens x 64 channels
+    // each, 128-byte-swizzle boxes; rows past the end of the sequence are clipped by the copy engine): the tile is written
+    // conflict-free (16-byte piece p of row r at p ^ (r % 8)) and one thread hands it over.
+    const int trow = rowi - 64;
+    const bool issuer = role == 10 && lane == 0;
+    bool valid = true;
+    int c = 0, job = job0;                                 // chunk of the chain, chain
+    for (int v = 0; v < n_virtual; v++) {
+      const int b = job / H, head = job % H;
+      const bool ok = tc::mbar_wait(&bars.out[v & 1], (v >> 1) & 1, abort_flag, 10);
+      valid = valid && ok;
+      tc::fence_after_sync();
+      if (issuer) tc::bulk_wait_read<0>();                 // the previous chunk's tile has been read by the copy engine
+      asm volatile("bar.sync 1, 64;" ::: "memory");
+      const int tok = c * KC + trow;
+#pragma unroll
+      for (int q = 0; q < NV / 32; q++) {
+        uint32_t r[32];
+        tc::tmem_ld32(tmem + (v & 1) * NV + (uint32_t)(q * 32) + ((uint32_t)(lq * 32) << 16), r);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; e++) w[e] = pack_bf2_rz(__uint_as_float(r[8 * u + 2 * e]) * scale, __uint_as_float(r[8 * u + 2 * e + 1]) * scale);
+          const int p = q * 4 + u;
+          *reinterpret_cast<uint4*>(smem + C::O + (p >> 3) * 8192 + trow * 128 + (((p & 7) ^ (trow & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        if (out_f32 && tok < seqlen && valid) {
+          float4* of = reinterpret_cast<float4*>(out_f32 + (((size_t)b * seqlen + tok) * H + head) * KD + slice * NV + q * 32);
+#pragma unroll
+          for (int u = 0; u < 8; u++)
+            of[u] = make_float4(__uint_as_float(r[4 * u]) * scale, __uint_as_float(r[4 * u + 1]) * scale,
+                                __uint_as_float(r[4 * u + 2]) * scale, __uint_as_float(r[4 * u + 3]) * scale);
+        }
+      }
+      tc::fence_before_sync();
+      if (lane == 0) tc::mbar_arrive(&bars.d1[v & 1]);     // chunk v + 2 may have this half of D1
+      tc::fence_async_smem();
+      asm volatile("bar.sync 1, 64;" ::: "memory");
+      if (issuer && valid) {
+#pragma unroll
+        for (int hb = 0; hb < NV / 64; hb++)
+          asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(map_out),
+                       "r"(slice * NV + hb * 64), "r"(head), "r"(c * KC), "r"(b), "r"(tc::smem_u32(smem + C::O + hb * 8192))
+                       : "memory");
+        tc::bulk_commit();
+      }
+      if (++c == n_chunks) { c = 0; job += job_step; }
+    }
+    if (issuer) tc::bulk_wait_all<0>();
+  } else {
+    constexpr int SC = NV / 2, UC = NV / 4;                // columns of a state thread, of a U thread
+    const bool state_warp = grp < 2, u_warp = lq < 2;
+    // chain number `ci`: its state row for this thread
+    auto chain_state = [&](int ci) -> float* {
+      const int job = job0 + job_step * ci, jb = job / H, jh = job % H;
+      const int sl = slots ? slots[jb] : jb;
+      return state + ((size_t)sl * H + jh) * KD * KD + (size_t)rowi * KD + slice * NV + grp * SC;
+    };
+    // B operand of the state, MN-major: off(k, n) = (n/8)*2048 + (k/8)*128 + (k%8)*16 + (n%8)*2
+    uint8_t* sS_row = smem + C::S + (SC / 8 * grp) * 2048 + rowi * 16;
+    float S[SC];
+    auto load_state = [&](const float* st) {
+#pragma unroll
+      for (int u = 0; u < SC / 4; u++) {
+        const float4 x = *reinterpret_cast<const float4*>(st + u * 4);
+        S[4 * u] = x.x; S[4 * u + 1] = x.y; S[4 * u + 2] = x.z; S[4 * u + 3] = x.w;
+      }
+    };
+    auto put_operand = [&](int u0, int n) {                // pieces u0 .. u0 + n - 1 of this row's columns as fp16
+#pragma unroll
+      for (int u = u0; u < u0 + n; u++)
+        *reinterpret_cast<uint4*>(sS_row + u * 2048) = make_uint4(pack_h2(S[8 * u], S[8 * u + 1]), pack_h2(S[8 * u + 2], S[8 * u + 3]),
+                                                                  pack_h2(S[8 * u + 4], S[8 * u + 5]), pack_h2(S[8 * u + 6], S[8 * u + 7]));
+    };
+    if (state_warp) {
+      load_state(chain_state(0));
+      put_operand(0, SC / 8);
+      tc::fence_async_smem();
+      tc::mbar_arrive(&bars.s[0]);
+    }
+    int in_chain = 0, chain = 0;                           // chunk of the chain, chain of the slot
+    for (int v = 0; v < n_virtual; v++) {
+      const uint32_t par = v & 1;
+      const uint32_t d1 = tmem + par * NV, d2 = tmem + 2 * NV;
+      // ---- U (token rows = TMEM lanes 0-63 of D1) as the next operand: off(t, n) = (n/8)*1024 + t*16 + (n%8)*2 ----
+      if (u_warp) {
+        tc::mbar_wait(&bars.mma[par], (v >> 1) & 1, abort_flag, 3);
+        tc::fence_after_sync();
+        uint32_t r[UC];
+        if constexpr (UC == 32) tc::tmem_ld32(d1 + (uint32_t)(grp * UC) + ((uint32_t)(lq * 32) << 16), r);
+        else tc::tmem_ld16(d1 + (uint32_t)(grp * UC) + ((uint32_t)(lq * 32) << 16), r);
+        tc::tmem_ld_wait();
+        uint8_t* urow = smem + C::U + (UC / 8 * grp) * 1024 + rowi * 16;
+#pragma unroll
+        for (int u = 0; u < UC / 8; u++)
+          *reinterpret_cast<uint4*>(urow + u * 1024) =
+              make_uint4(pack_h2(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])), pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])),
+                         pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])), pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])));
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        tc::mbar_arrive(&bars.u);
+      }
+      // ---- state: S <- S e^{G_last} + Kt^T U (lane = k row), refresh the fp16 operand copy ----
+      if (state_warp) {
+        tc::mbar_wait(&bars.kb[par], (v >> 1) & 1, abort_flag, 2);
+        const float dec = reinterpret_cast<const float*>(smem + par * C::STAGE + C::DEC)[rowi];
+        tc::mbar_wait(&bars.mma2, par, abort_flag, 4);
+        tc::fence_after_sync();
+        const bool last = in_chain == n_chunks - 1;
+#pragma unroll
+        for (int hf = 0; hf < SC / 32; hf++) {
+          uint32_t r[32];
+          tc::tmem_ld32(d2 + (uint32_t)(grp * SC + hf * 32) + ((uint32_t)(lq * 32) << 16), r);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; j++) S[hf * 32 + j] = fmaf(S[hf * 32 + j], dec, __uint_as_float(r[j]));
+          if (!last) put_operand(4 * hf, 4);
+        }
+        if (last) {
+          // last chunk of a chain: its final state goes back to memory and the slot's next chain begins
+          float* st = chain_state(chain);
+          if (!*(volatile int*)abort_flag) {
+#pragma unroll
+            for (int u = 0; u < SC / 4; u++)
+              *reinterpret_cast<float4*>(st + u * 4) = make_float4(S[4 * u], S[4 * u + 1], S[4 * u + 2], S[4 * u + 3]);
+          }
+          if (v + 1 < n_virtual) {
+            load_state(chain_state(chain + 1));
+            put_operand(0, SC / 8);
+          }
+        }
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        tc::mbar_arrive(&bars.s[par ^ 1]);
+      }
+      if (++in_chain == n_chunks) { in_chain = 0; chain++; }
+    }
+  }
+}
+
+// kernel 2: one chain's NV columns per CTA, units in the workspace
+template <int NV>
+__global__ __launch_bounds__(512, 1) void kda_chunk_scan_kernel(
+    const uint8_t* __restrict__ ws, float* __restrict__ state, float* __restrict__ out_f32, int seqlen, int H, int n_chunks,
+    const int* __restrict__ slots, float scale, int* __restrict__ status, const __grid_constant__ CUtensorMap map_out) {
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ uint64_t full_bar[S_NSTAGE];
-  __shared__ uint64_t mma_bar;
-  __shared__ uint64_t out_bar;    // completion of the output contraction (B beta) U, waited on by warps 2, 3 only
+  __shared__ ChainBars bars;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int vs = blockIdx.x, head = blockIdx.y, b = blockIdx.z;
-  const int v0 = vs * KNV;
-  const uint8_t* unit0 = ws + ((size_t)b * n_chunks * H + head) * U_BYTES;   // unit of chunk c: + c * H * U_BYTES
+  const int tid = threadIdx.x;
+  const int slice = blockIdx.x, job = blockIdx.z * H + blockIdx.y;
   if (tid == 0) {
-    for (int i = 0; i < S_NSTAGE; i++) tc::mbar_init(&full_bar[i], 1);
-    tc::mbar_init(&mma_bar, 1);
-    tc::mbar_init(&out_bar, 1);
+    chain_init(bars);
     tc::mbar_fence_init();
     abort_flag = 0;
   }
-  if (warp == 0) tc::tmem_alloc(&tmem_slot, 128);
-  write_identity(smem + P2_ID, tid, 128);
+  if (tid < 32) tc::tmem_alloc(&tmem_slot, 4 * NV);
   pdl_wait();
-  // state slice: thread = k row, 32 fp32 values in registers; fp16 copy as the B operand
-  const int slot = slots ? slots[b] : b;
-  float* st = state + ((size_t)slot * H + head) * KD * KD + (size_t)tid * KD + v0;  // row k = tid
-  float S[KNV];
-#pragma unroll
-  for (int u = 0; u < KNV / 4; u++) {
-    const float4 v = *reinterpret_cast<const float4*>(st + u * 4);
-    S[4 * u] = v.x; S[4 * u + 1] = v.y; S[4 * u + 2] = v.z; S[4 * u + 3] = v.w;
-  }
-  // B operand, MN-major: off(k, n) = (n/8)*2048 + (k/8)*128 + (k%8)*16 + (n%8)*2
-  uint8_t* sS_row = smem + P2_S + (tid >> 3) * 128 + (tid & 7) * 16;
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    uint4 p;
-    p.x = pack_h2(S[8 * u], S[8 * u + 1]); p.y = pack_h2(S[8 * u + 2], S[8 * u + 3]);
-    p.z = pack_h2(S[8 * u + 4], S[8 * u + 5]); p.w = pack_h2(S[8 * u + 6], S[8 * u + 7]);
-    *reinterpret_cast<uint4*>(sS_row + u * 2048) = p;
-  }
-  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  // D1 alternates between two column ranges by chunk parity: the output rows of chunk c are read while the first
-  // contraction of chunk c + 1 fills the other range
-  const uint32_t d2 = tmem + 32;
-
-  auto issue_loads = [&](int chunk) {
-    uint8_t* stg = smem + (chunk % S_NSTAGE) * S_STAGE;
-    const uint8_t* u = unit0 + (size_t)chunk * H * U_BYTES;
-    uint64_t* bar = &full_bar[chunk % S_NSTAGE];
-    tc::mbar_arrive_expect_tx(bar, S_STAGE);
-    tc::bulk_g2s(stg + S_WQ, u + U_WQ, 32768, bar);
-    tc::bulk_g2s(stg + S_BB, u + U_BB, 8192, bar);
-    tc::bulk_g2s(stg + S_KT, u + U_KT, 16384, bar);
-    tc::bulk_g2s(stg + S_UL, u + U_UL + vs * (KC * KNV * 2), 4096, bar);
-    tc::bulk_g2s(stg + S_DEC, u + U_DEC, 512, bar);
-  };
-  if (tid == 0) {
-    for (int c = 0; c < S_NSTAGE && c < n_chunks; c++) issue_loads(c);
-  }
-
-  const uint32_t idesc = tc::make_idesc(128, KNV, tc::FMT_F16, tc::FMT_F16, false, true);
-  const uint32_t idesc_kt = tc::make_idesc(128, KNV, tc::FMT_F16, tc::FMT_F16, true, true);   // Kt^T: channels contiguous
-  const uint32_t s_addr = tc::smem_u32(smem + P2_S), u_addr = tc::smem_u32(smem + P2_U), id_addr = tc::smem_u32(smem + P2_ID);
-  // The contractions are issued by the whole of warp 0 with one elected lane (descriptors stay warp-uniform for the
-  // compiler: ~41 instead of ~47 cycles per M128 N32 product, see tc05.cuh).  Every wait of this kernel is executed
-  // by all lanes, so warp 0 stays converged from one contraction to the next.
-  const bool issue_warp = tc::warp_index_uniform() == 0;
-  const uint32_t leader = issue_warp ? tc::elect_one() : 0u;
-  uint32_t mma_parity = 0, out_parity = 0;
-
-  // output rows of chunk c (TMEM lanes 64-127 of that chunk's D1 range = tokens), warps 2 and 3
-  auto emit_outputs = [&](int c, bool valid) {
-    const int tok = c * KC + (tid - 64);
-    uint32_t r[32];
-    tc::tmem_ld32(tmem + ((c & 1) ? 64u : 0u) + ((uint32_t)(warp * 32) << 16), r);
-    tc::tmem_ld_wait();
-    if (tok < seqlen && valid) {
-      const size_t oi = (((size_t)b * seqlen + tok) * H + head) * KD + v0;
-      uint4* o = reinterpret_cast<uint4*>(out + oi);
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) w[e] = pack_bf2_rz(__uint_as_float(r[8 * u + 2 * e]) * scale, __uint_as_float(r[8 * u + 2 * e + 1]) * scale);
-        o[u] = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-      if (out_f32) {
-        float4* of = reinterpret_cast<float4*>(out_f32 + oi);
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-          of[u] = make_float4(__uint_as_float(r[4 * u]) * scale, __uint_as_float(r[4 * u + 1]) * scale,
-                              __uint_as_float(r[4 * u + 2]) * scale, __uint_as_float(r[4 * u + 3]) * scale);
-      }
-    }
-  };
-  bool prev_ok = true;                                      // warps 2, 3: the previous chunk's waits all succeeded
-
-  for (int chunk = 0; chunk < n_chunks; chunk++) {
-    const int sidx = chunk % S_NSTAGE;
-    uint8_t* stg = smem + sidx * S_STAGE;
-    const uint32_t stg_addr = tc::smem_u32(stg);
-    const uint32_t d1 = tmem + ((chunk & 1) ? 64u : 0u);
-    KS_TRACE(0, chunk);
-    bool ok = tc::mbar_wait(&full_bar[sidx], (chunk / S_NSTAGE) & 1, &abort_flag, 2);
-    KS_TRACE(1, chunk);
-    // ---- D1 (128 x 32) = [I ; 0] Uloc (exact) + [-W ; Q+] S0: rows 0-63 are U ----
-    if (issue_warp) {
-#pragma unroll
-      for (int kk = 0; kk < KC / 16; kk++) {
-        const uint64_t ad = tc::make_sdesc(id_addr + (6 - 2 * kk) * 128, 128, 128);
-        const uint64_t bd = tc::make_sdesc(stg_addr + S_UL + kk * 2 * 128, 128, 1024);
-        tc::mma_f16_if(leader, d1, ad, bd, idesc, kk > 0);
-      }
-#pragma unroll
-      for (int kk = 0; kk < KD / 16; kk++) {
-        const uint64_t ad = tc::make_sdesc(stg_addr + S_WQ + kk * 2 * LBO, LBO, SBO_K128);
-        const uint64_t bd = tc::make_sdesc(s_addr + kk * 2 * 128, 128, 2048);
-        tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
-      }
-      tc::mma_commit_if(leader, &mma_bar);
-    }
-    // the previous chunk's output rows leave while this chunk's first contraction runs (off the chain)
-    if (warp >= 2 && chunk > 0) emit_outputs(chunk - 1, prev_ok);
-    ok = tc::mbar_wait(&mma_bar, mma_parity, &abort_flag, 3) && ok;
-    mma_parity ^= 1;
-    tc::fence_after_sync();
-    KS_TRACE(2, chunk);
-    // ---- U (token rows = TMEM lanes 0-63) as the next operand ----
-    if (warp < 2) {
-      uint32_t r[32];
-      tc::tmem_ld32(d1 + ((uint32_t)(warp * 32) << 16), r);
-      tc::tmem_ld_wait();
-      uint8_t* urow = smem + P2_U + tid * 16;               // off(k=t, n) = (n/8)*1024 + t*16 + (n%8)*2
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        *reinterpret_cast<uint4*>(urow + u * 1024) =
-            make_uint4(pack_h2(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])), pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])),
-                       pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])), pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])));
-    }
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    KS_TRACE(3, chunk);
-    // ---- D2 = Kt^T U (state path, committed first) ;  D1 rows 64-127 += (B beta) U (outputs, own barrier) ----
-    if (issue_warp) {
-#pragma unroll
-      for (int kk = 0; kk < KC / 16; kk++) {
-        const uint64_t ad = tc::make_sdesc(stg_addr + S_KT + kk * 2 * 128, 128, 1024);
-        const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
-        tc::mma_f16_if(leader, d2, ad, bd, idesc_kt, kk > 0);
-      }
-      tc::mma_commit_if(leader, &mma_bar);
-#pragma unroll
-      for (int kk = 0; kk < KC / 16; kk++) {
-        const uint64_t ad = tc::make_sdesc(stg_addr + S_BB - 8192 + kk * 2 * LBO, LBO, SBO_K64);   // rows 0-63: whatever precedes the tile
-        const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
-        tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
-      }
-      tc::mma_commit_if(leader, &out_bar);
-    }
-    ok = tc::mbar_wait(&mma_bar, mma_parity, &abort_flag, 4) && ok;
-    mma_parity ^= 1;
-    tc::fence_after_sync();
-    KS_TRACE(4, chunk);
-    // ---- state: S <- S e^{G_last} + Kt^T U (lane = k row), refresh the fp16 operand copy.  The output
-    //      contraction is still running: only the state is on the chunk-to-chunk chain. ----
-    {
-      uint32_t r[32];
-      tc::tmem_ld32(d2 + ((uint32_t)(warp * 32) << 16), r);
-      tc::tmem_ld_wait();
-      const float dec = reinterpret_cast<const float*>(stg + S_DEC)[tid];
-#pragma unroll
-      for (int j = 0; j < KNV; j++) S[j] = fmaf(S[j], dec, __uint_as_float(r[j]));
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        uint4 p;
-        p.x = pack_h2(S[8 * u], S[8 * u + 1]); p.y = pack_h2(S[8 * u + 2], S[8 * u + 3]);
-        p.z = pack_h2(S[8 * u + 4], S[8 * u + 5]); p.w = pack_h2(S[8 * u + 6], S[8 * u + 7]);
-        *reinterpret_cast<uint4*>(sS_row + u * 2048) = p;
-      }
-    }
-    KS_TRACE(5, chunk);
-    // ---- warps 2, 3 make sure the output contraction is complete before the block barrier (the stage and the U
-    //      tile it reads are rewritten after it); the rows themselves are read in the next iteration ----
-    if (warp >= 2) {
-      ok = tc::mbar_wait(&out_bar, out_parity, &abort_flag, 5) && ok;
-      prev_ok = ok;
-    }
-    out_parity ^= 1;
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    KS_TRACE(6, chunk);
-    // The refill is issued by a thread of warp 3, not by thread 0: the five copy instructions take about 400 cycles
-    // to issue, which the MMA-issuing thread would add to the per-chunk chain (measured: 1.95 -> 1.87 ms at 32K
-    // tokens).  Issuing them while the next contraction runs instead was slower (the barrier polls queue behind them).
-    if (tid == 96 && chunk + S_NSTAGE < n_chunks) issue_loads(chunk + S_NSTAGE);
-  }
-  if (warp >= 2 && n_chunks > 0) emit_outputs(n_chunks - 1, prev_ok);
-  if (!abort_flag) {
-#pragma unroll
-    for (int u = 0; u < KNV / 4; u++)
-      *reinterpret_cast<float4*>(st + u * 4) = make_float4(S[4 * u], S[4 * u + 1], S[4 * u + 2], S[4 * u + 3]);
-  }
+  // the unit of chunk v: heads are the fastest index (see kernel 1)
+  const uint8_t* unit0 = ws + ((size_t)blockIdx.z * n_chunks * H + blockIdx.y) * U_BYTES;
+  chain_cta<NV, false>(smem + ((1024u - (tc::smem_u32(smem) & 1023u)) & 1023u), bars, tmem, &abort_flag,
+                       [&](int v) { return unit0 + (size_t)v * H * U_BYTES; }, nullptr, nullptr, nullptr, 0, job, 1, n_chunks, n_chunks, slice, H, seqlen,
+                       state, out_f32, slots, scale, &map_out);
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem, 128);
+  if (tid < 32) tc::tmem_dealloc(tmem, 4 * NV);
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
 }
-
 
 // =================================================================================================
 // fused form: preparation and scan in ONE persistent launch
 //
-// One CTA of 512 threads per SM.  The first n_slots CTAs are chain slots: each walks the chunks of one (batch, head)
-// chain - or, when the call has more than 48 chains, of n_jobs / n_slots chains one after the other (the state is
-// swapped at the chain boundary; ring, flags and barrier parities go by the slot's running chunk number) - with the
-// whole 128-column state of the head, sixteen warps = four TMEM lane quarters x four 32-column blocks.  Every other CTA
+// One CTA of 512 threads per SM.  The first n_slots x (128 / NV) CTAs are chain CTAs: a slot is one (batch, head)
+// chain - or, when the call has more than 48 chains, n_jobs / n_slots chains one after the other (the state is
+// swapped at the chain boundary) - and has a CTA for every NV value columns.  Every other CTA
 // hosts two preparation workers of 256 threads (its two halves, each with its own shared memory, TMEM columns and
 // named barrier), which take the units round robin in the order the slots need them.  A unit travels through a ring
-// of KR chunk slots per chain slot in global memory - a few tens of MB that stay in L2 - instead of a per-chunk workspace in HBM:
-//   ready[slot][v % KR] = v + 1 once the unit of that chunk is complete (release store after the worker's writes),
-//   consumed[job]     = number of chunks whose unit has landed in the chain CTA's shared memory (the slot of chunk c
-//                       may be rewritten once consumed > c).
+// of 16 or 32 chunk slots per chain slot in global memory - a few tens of MB that stay in L2 - instead of a per-chunk workspace in HBM:
+//   ready[slot][v % depth] = v + 1 once the unit of that chunk is complete (release store after the worker's writes),
+//   consumed[chain CTA]  = number of chunks whose unit has landed in the chain CTA's shared memory (the slot of chunk c
+//                          may be rewritten once consumed > c for all CTAs of the slot).
 // A worker that finds its slot still occupied, and a chain CTA that finds its unit not yet written, poll with a
 // bound (about a second); on expiry they record HK_ERR_TIMEOUT, raise the launch-wide abort word and finish without
 // waiting again.  All CTAs must be resident at once: the launch is cooperative and sized to the SM count.
 // =================================================================================================
-constexpr int F_NSTAGE = 2;                               // operand stages of the chain CTA: a unit each, laid out as in the ring
-constexpr uint32_t F_STAGE = U_BYTES;
-constexpr uint32_t F_S = F_NSTAGE * F_STAGE;              // fp16 B operand: state [128 k][128 v], MN-major, 32 KB
-constexpr uint32_t F_U = F_S + 32768;                     // fp16 B operand: U [64 tokens][128 v], MN-major, 16 KB
-constexpr uint32_t F_O = F_U + 16384;                     // bf16 output rows of one chunk: two swizzled 8 KB boxes for the tiled
-                                                          // stores, or plain [64 tokens][256 B] rows when the kernel stores itself
-constexpr uint32_t F_OPITCH = 256;
-constexpr uint32_t F_ID = F_O + KC * F_OPITCH;           // [I ; 0]
-constexpr uint32_t F_SMEM_SCAN = F_ID + ID_BYTES + 1024;     // + slack to start the tiles at a 1 KB boundary
-static_assert(F_O % 1024 == 0 && KC * F_OPITCH >= 16384, "the output tile holds two 8 KB swizzled boxes");
-constexpr uint32_t F_SMEM = F_SMEM_SCAN > 2 * P1_SMEM + 1024 ? F_SMEM_SCAN : 2 * P1_SMEM + 1024;
+template <int NV>
+constexpr uint32_t fused_smem() { return Chain<NV>::SMEM > 2 * P1_SMEM + 1024 ? Chain<NV>::SMEM : 2 * P1_SMEM + 1024; }
 
-template <bool GATED>
+template <bool GATED, int NV>
 __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
     const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
-    uint8_t* __restrict__ ring, int* __restrict__ flags, float* __restrict__ state, __nv_bfloat16* __restrict__ out,
+    uint8_t* __restrict__ ring, int* __restrict__ flags, float* __restrict__ state,
     float* __restrict__ out_f32, int seqlen, int H, int n_chunks, int n_jobs, int n_slots, const int* __restrict__ slots,
     float scale, int* __restrict__ status, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
-    float lower_bound, const __grid_constant__ CUtensorMap tmap_out, int use_tma_out) {
-  extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ uint64_t wu_bar[F_NSTAGE];    // -W, Q+ and Uloc of a stage have landed
-  __shared__ uint64_t kb_bar[F_NSTAGE];    // B beta, Kt^T and the decays
-  // chain: barriers of a chunk, two of most kinds by chunk parity, so that a warp that is held up may be a chunk behind
-  __shared__ uint64_t mma_bar[2];    // U and Q+ S0 are complete
-  __shared__ uint64_t mma2_bar;      // Kt^T U (state path) is complete
-  __shared__ uint64_t out_bar[2];    // (B beta) U is complete, and with it every product of the chunk (by chunk parity)
-  __shared__ uint64_t u_bar;         // the 256 token-row threads have written U
-  __shared__ uint64_t s_bar[2];      // the 256 state threads have written the state operand
-  __shared__ uint64_t d1_bar[2];     // the two output warps have read this half of D1
+    float lower_bound, const __grid_constant__ CUtensorMap map_out) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  __shared__ ChainBars bars;
   __shared__ PrepShared prep[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5;
-#ifdef HK_DIAG
-  if (tid == 0 && blockIdx.x == 1) hk_kda_trace[32 + 11] = clock64();
-#endif
+  constexpr int SLICES = Chain<NV>::SLICES;
+  const int n_chain_ctas = n_slots * SLICES;
   int* g_abort = flags;
-  // A chain CTA ("slot") walks n_jobs / n_slots chains one after the other: its running chunk number v counts through
-  // all of them (chain v / n_chunks of the slot, chunk v % n_chunks), and ring, flags and barrier parities go by v.
-  int* ready = flags + F_FLAG_INTS;                        // [n_slots][KR], a line per slot
-  int* consumed = ready + (size_t)n_slots * F_LINE;        // [n_slots], a line each
+  int* ready = flags + F_FLAG_INTS;                        // [n_slots][ring depth], a line per slot
+  int* consumed = ready + (size_t)n_slots * F_LINE;        // [n_chain_ctas], a line each
   const int n_virtual = (n_jobs / n_slots) * n_chunks;     // chunks a slot walks
+  const int kr = ring_depth(n_slots, n_virtual);
 
   if (tid == 0) {
-    for (int i = 0; i < 2; i++) {
-      tc::mbar_init(&wu_bar[i], 1);
-      tc::mbar_init(&kb_bar[i], 1);
-      tc::mbar_init(&mma_bar[i], 1);
-      tc::mbar_init(&out_bar[i], 1);
-      tc::mbar_init(&s_bar[i], 256);
-      tc::mbar_init(&d1_bar[i], 2);
-    }
-    tc::mbar_init(&mma2_bar, 1);
-    tc::mbar_init(&u_bar, 256);
+    chain_init(bars);
     prep_init(prep[0]);
     prep_init(prep[1]);
     tc::mbar_fence_init();
@@ -1101,14 +1207,14 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
   tc::fence_after_sync();
   const uint32_t tmem = tmem_slot;
   // tiles start at a 1 KB boundary: the 128-byte-swizzle pattern is a function of the shared-memory address
-  uint8_t* const smem_base = smem + ((1024u - (tc::smem_u32(smem) & 1023u)) & 1023u);
+  uint8_t* const smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
 
-  if ((int)blockIdx.x >= n_slots) {
+  if ((int)blockIdx.x >= n_chain_ctas) {
     // =========================== two preparation workers ===========================
     const int sub = warp >> 3;
     // unit `it` of a worker, in the order the slots need them: running chunk v of every slot, then v + 1, ...
     auto make_unit = [&](int it, PrepDesc& u) {
-      const long long n = ((int)blockIdx.x - n_slots) * 2 + sub + (long long)it * ((int)gridDim.x - n_slots) * 2;
+      const long long n = ((int)blockIdx.x - n_chain_ctas) * 2 + sub + (long long)it * ((int)gridDim.x - n_chain_ctas) * 2;
       const int v = (int)min(n / n_slots, (long long)n_virtual), slot = (int)(n % n_slots);
       const int chunk = v % n_chunks, job = slot + n_slots * (v / n_chunks);
       u.b = job / H;
@@ -1116,12 +1222,12 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
       u.tok0 = u.b * seqlen + u.t0;
       u.n_valid = v < n_virtual ? min(KC, seqlen - chunk * KC) : 0;
       u.head = job % H;
-      u.unit = (v % KR) * n_slots + slot;
+      u.unit = (v & (kr - 1)) * n_slots + slot;
       u.slot = slot;
       u.value = v + 1;
     };
     PrepCtx ctx;
-    ctx.smem = smem_base + sub * P1_SMEM; ctx.sh = &prep[sub]; ctx.abort_flag = &abort_flag; ctx.tid = tid & 255; ctx.bar_id = 1 + sub;
+    ctx.smem = smem + sub * P1_SMEM; ctx.sh = &prep[sub]; ctx.abort_flag = &abort_flag; ctx.tid = tid & 255; ctx.bar_id = 1 + sub;
     if (ctx.tid == 0) make_unit(0, prep[sub].unit[0]);
     prep_sync<true>(ctx);
     if (ctx.tid == 0) {
@@ -1129,318 +1235,15 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
       prep_fetch_qkv(ctx, 0, &map_qkv, H);
     }
     int it = 0;
-    for (; PREP_UNIT(n_valid, it) > 0; it++) {
-      prep_unit<GATED, true>(ctx, it, &map_qkv, &map_g, beta_in, ring, H, dt_bias, a_log, lower_bound, tmem + sub * 256, ready, consumed,
-                             g_abort, n_slots, make_unit);
-    }
-    if (it > 0 && (ctx.tid >> 5) == PUB_WARP) prep_publish(ctx, it - 1, ready, n_slots);
+    for (; PREP_UNIT(n_valid, it) > 0; it++)
+      prep_unit<GATED, SLICES>(ctx, it, &map_qkv, &map_g, beta_in, ring, H, dt_bias, a_log, lower_bound, tmem + sub * 256, ready, consumed,
+                               g_abort, kr, make_unit);
+    if (it > 0 && (ctx.tid >> 5) == PUB_WARP) prep_publish(ctx, it - 1, ready, kr);
   } else {
-    // =========================== one (batch, head) chain ===========================
-    // Sixteen warps = four TMEM lane quarters (lq) x four groups, joined by mbarriers that complete once per chunk, never by the
-    // whole CTA; what is on the chunk-to-chunk chain is spread over many warps, the rest has warps of its own:
-    //   U         lq 0, 1 of all groups (token rows of D1), 32 columns each
-    //   state     groups 0, 1: a k row and 64 of its columns per thread, fp32 in registers
-    //   outputs   warps 10, 11: a token row each thread
-    //   issuer    warp 14: every product; it waits for operands only
-    //   producer  warp 15: ring protocol and operand copies
-    // A barrier's next phase cannot complete before its waiters have seen this one: U needs every U warp, the state operand every
-    // state warp; out_bar and d1_bar alternate by chunk, since the output warps may be a chunk behind or done with the one before.
-    uint8_t* const smem = smem_base;
-    const int cslot = blockIdx.x;                           // this CTA's chain slot
-    const int lane = tid & 31, lq = warp & 3, grp = warp >> 2;
-    const int rowi = lq * 32 + lane;                        // k row of the state / token row of U / output row + 64
-    const int role = tc::warp_index_uniform();
-    // D1 alternates between columns 0-127 and 128-255 by chunk parity, D2 = columns 256-383
-    write_identity(smem + F_ID, tid, 512);
-    tc::fence_async_smem();
-    __syncthreads();
-
-    // `v` is the slot's RUNNING chunk number over all of its chains
-    if (role == 14) {
-      const uint32_t leader = tc::elect_one();
-      const uint32_t idesc = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, false, true);
-      const uint32_t idesc_kt = tc::make_idesc(128, KD, tc::FMT_F16, tc::FMT_F16, true, true);   // Kt^T: channels contiguous
-      const uint32_t s_addr = tc::smem_u32(smem + F_S), u_addr = tc::smem_u32(smem + F_U), id_addr = tc::smem_u32(smem + F_ID);
-      // D1 of chunk w = [I ; 0] Uloc, ahead of the state: the product with the identity is exact
-      auto issue_uloc = [&](int w) {
-        tc::fence_after_sync();
-#pragma unroll
-        for (int kk = 0; kk < KC / 16; kk++) {
-          const uint64_t ad = tc::make_sdesc(id_addr + (6 - 2 * kk) * 128, 128, 128);
-          const uint64_t bd = tc::make_sdesc(tc::smem_u32(smem + (w & 1) * F_STAGE) + U_UL + kk * 2 * 128, 128, 1024);
-          tc::mma_f16_if(leader, tmem + (w & 1) * 128, ad, bd, idesc, kk > 0);
-        }
-      };
-      int uloc = 0;                                        // chunks whose Uloc has been issued
-      for (int v = 0; v < n_virtual; v++) {
-        const uint32_t par = v & 1, ph = (v >> 1) & 1, stg_addr = tc::smem_u32(smem + par * F_STAGE);
-        const uint32_t d1 = tmem + par * 128, d2 = tmem + 256;
-        if (uloc == v) {
-          tc::mbar_wait(&wu_bar[par], ph, &abort_flag, 2);
-          if (v >= 2) tc::mbar_wait(&d1_bar[par], ph ^ 1, &abort_flag, 8);   // the output rows of chunk v - 2 have left this half of D1
-          issue_uloc(v);
-          uloc++;
-        }
-        // ---- D1 += [-W ; Q+] S0 ----
-        tc::mbar_wait(&s_bar[par], ph, &abort_flag, 6);
-        tc::fence_after_sync();
-#pragma unroll
-        for (int kk = 0; kk < KD / 16; kk++) {
-          const uint64_t ad = tc::make_sdesc(stg_addr + U_WQ + kk * 2 * LBO, LBO, SBO_K128);
-          const uint64_t bd = tc::make_sdesc(s_addr + kk * 2 * 128, 128, 2048);
-          tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
-        }
-        tc::mma_commit_if(leader, &mma_bar[par]);
-        // the next chunk's Uloc while U leaves the tensor memory, if its operands and its half of D1 are there already (otherwise at
-        // the chunk's start, where 260 cycles of products stand between the state and U: 3.5 -> 2.7 thousand cycles a chunk)
-        if (v + 1 < n_virtual) {
-          const uint32_t nph = ((v + 1) >> 1) & 1;
-          const bool here = tc::mbar_test_wait(&wu_bar[par ^ 1], nph) && (v == 0 || tc::mbar_test_wait(&d1_bar[par ^ 1], nph ^ 1));
-          if (__all_sync(0xffffffffu, here)) {
-            issue_uloc(v + 1);
-            uloc++;
-          }
-        }
-        // ---- D2 = Kt^T U (state path), then D1 rows 64-127 += (B beta) U (outputs) ----
-        tc::mbar_wait(&kb_bar[par], ph, &abort_flag, 11);
-        tc::mbar_wait(&u_bar, par, &abort_flag, 7);
-        tc::fence_after_sync();
-#pragma unroll
-        for (int kk = 0; kk < KC / 16; kk++) {
-          const uint64_t ad = tc::make_sdesc(stg_addr + U_KT + kk * 2 * 128, 128, 1024);
-          const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
-          tc::mma_f16_if(leader, d2, ad, bd, idesc_kt, kk > 0);
-        }
-        tc::mma_commit_if(leader, &mma2_bar);
-        // rows 0-63 of this operand are the tile below B beta in the unit: they add to U's rows, which have been read
-#pragma unroll
-        for (int kk = 0; kk < KC / 16; kk++) {
-          const uint64_t ad = tc::make_sdesc(stg_addr + U_BB - 8192 + kk * 2 * LBO, LBO, SBO_K64);
-          const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
-          tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
-        }
-        tc::mma_commit_if(leader, &out_bar[par]);
-      }
-    } else if (role == 15) {
-      const int* my_ready = ready + (size_t)cslot * F_LINE;
-      // a unit in two copies: a stage's first part is free as soon as the chunk's first product is complete, most of a chunk before
-      // the rest.  74 KB take about as long as a chunk to arrive.
-      auto load = [&](int v, uint32_t at, uint32_t bytes, uint64_t* bar) {
-        if (lane == 0) {
-          tc::mbar_arrive_expect_tx(bar, bytes);
-          tc::bulk_g2s(smem + (v & 1) * F_STAGE + at, ring + ((size_t)(v % KR) * n_slots + cslot) * U_BYTES + at, bytes, bar);
-        }
-        __syncwarp();
-      };
-      // Units are asked for a ring at a time: a flag takes a microsecond or more to read while the workers poll theirs, too long for
-      // every chunk.
-      int known = 0;                                       // units before this one are complete
-      auto await_unit = [&](int v) {
-        const long long t0 = clock64();
-        while (known <= v) {
-          const bool here = lane < KR && ld_acquire_gpu(my_ready + (known + lane) % KR) > known + lane;
-          const uint32_t missing = ~__ballot_sync(0xffffffffu, here);
-          known += __ffs(missing) - 1;                     // lanes from KR on are never here
-          if (known > v) break;
-          const bool give_up = abort_flag || ld_relaxed_gpu(g_abort) != 0 || clock64() - t0 > tc::MBAR_WAIT_CYCLES;
-          if (__any_sync(0xffffffffu, give_up)) {
-            if (lane == 0) {
-              abort_flag = 21;
-              atomicExch(g_abort, 21);
-            }
-            break;
-          }
-          __nanosleep(64);
-        }
-        __syncwarp();
-        if (lane == 0) fence_proxy_async_all();
-      };
-      for (int v = 0; v < F_NSTAGE && v < n_virtual; v++) {
-        await_unit(v);
-        load(v, 0, U_BB, &wu_bar[v]);
-        load(v, U_BB, U_BYTES - U_BB, &kb_bar[v]);
-      }
-      for (int v = 0; v < n_virtual; v++) {
-        const uint32_t par = v & 1, ph = (v >> 1) & 1;
-        const bool more = v + F_NSTAGE < n_virtual;
-        // the unit of this chunk has landed in shared memory: its slot may be rewritten.  A relaxed store is enough:
-        // the copy engine's reads are complete, nothing this thread wrote is handed over with the flag.
-        tc::mbar_wait(&wu_bar[par], ph, &abort_flag, 2);
-        tc::mbar_wait(&kb_bar[par], ph, &abort_flag, 2);
-        if (lane == 0) st_relaxed_gpu(consumed + cslot * F_LINE, v + 1);
-        if (!more) continue;
-        await_unit(v + F_NSTAGE);
-        tc::mbar_wait(&mma_bar[par], ph, &abort_flag, 3);
-        load(v + F_NSTAGE, 0, U_BB, &wu_bar[par]);
-        // all products of the chunk are complete and the state warps have read its decays
-        tc::mbar_wait(&out_bar[par], ph, &abort_flag, 5);
-        tc::mbar_wait(&s_bar[par ^ 1], ((v + 1) >> 1) & 1, &abort_flag, 9);
-        load(v + F_NSTAGE, U_BB, U_BYTES - U_BB, &kb_bar[par]);
-      }
-    } else if (role == 10 || role == 11) {
-      // Output rows: TMEM lanes 64-127 of a chunk's D1 half = tokens; a thread holds the columns of one token.  Stored directly,
-      // a warp-wide 16-byte store would touch 32 different rows (32 L1 requests per instruction, over a thousand per chunk
-      // on this one SM).  The bf16 rows are therefore assembled in shared memory.  With a tensor map over the output they leave
-      // as TWO tiled TMA stores per chunk (64 tokens x 64 channels each, 128-byte-swizzle boxes; rows past the end of the sequence
-      // are clipped by the copy engine): the tile is written conflict-free (16-byte piece p of row r at p ^ (r % 8)) and one
-      // thread hands it over.  Without a map every warp instruction covers two whole 256-byte rows.
-      const int trow = rowi - 64;
-      const bool issuer = role == 10 && lane == 0;
-      bool valid = true;
-      int c = 0, job = cslot;                              // chunk of the chain, chain
-      for (int v = 0; v < n_virtual; v++) {
-        const int b = job / H, head = job % H;
-        const bool ok = tc::mbar_wait(&out_bar[v & 1], (v >> 1) & 1, &abort_flag, 10);
-        valid = valid && ok;
-        tc::fence_after_sync();
-        if (use_tma_out && issuer) tc::bulk_wait_read<0>();   // the previous chunk's tile has been read by the copy engine
-        asm volatile("bar.sync 1, 64;" ::: "memory");
-        const int tok = c * KC + trow;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          uint32_t r[32];
-          tc::tmem_ld32(tmem + (v & 1) * 128 + (uint32_t)(q * 32) + ((uint32_t)(lq * 32) << 16), r);
-          tc::tmem_ld_wait();
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            uint32_t w[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) w[e] = pack_bf2_rz(__uint_as_float(r[8 * u + 2 * e]) * scale, __uint_as_float(r[8 * u + 2 * e + 1]) * scale);
-            const int p = q * 4 + u;
-            uint8_t* o = use_tma_out ? smem + F_O + (p >> 3) * 8192 + trow * 128 + (((p & 7) ^ (trow & 7)) << 4) : smem + F_O + trow * F_OPITCH + p * 16;
-            *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-          if (out_f32 && tok < seqlen && valid) {
-            float4* of = reinterpret_cast<float4*>(out_f32 + (((size_t)b * seqlen + tok) * H + head) * KD + q * 32);
-#pragma unroll
-            for (int u = 0; u < 8; u++)
-              of[u] = make_float4(__uint_as_float(r[4 * u]) * scale, __uint_as_float(r[4 * u + 1]) * scale,
-                                  __uint_as_float(r[4 * u + 2]) * scale, __uint_as_float(r[4 * u + 3]) * scale);
-          }
-        }
-        tc::fence_before_sync();
-        if (lane == 0) tc::mbar_arrive(&d1_bar[v & 1]);           // chunk v + 2 may have this half of D1
-        tc::fence_async_smem();
-        asm volatile("bar.sync 1, 64;" ::: "memory");
-        if (use_tma_out) {
-          if (issuer && valid) {
-#pragma unroll
-            for (int hb = 0; hb < 2; hb++)
-              asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(&tmap_out),
-                           "r"(hb * 64), "r"(head), "r"(c * KC), "r"(b), "r"(tc::smem_u32(smem + F_O + hb * 8192))
-                           : "memory");
-            tc::bulk_commit();
-          }
-        } else {
-          const int ot = (lq - 2) * 32 + lane;             // 0..63 over the two output warps
-#pragma unroll 4
-          for (int i = 0; i < 16; i++) {
-            const int piece = ot + 64 * i, prow = piece >> 4, pc = piece & 15;
-            const int ptok = c * KC + prow;
-            if (ptok < seqlen && valid) {
-              const uint4 o4 = *reinterpret_cast<const uint4*>(smem + F_O + prow * F_OPITCH + pc * 16);
-              *reinterpret_cast<uint4*>(out + (((size_t)b * seqlen + ptok) * H + head) * KD + pc * 8) = o4;
-            }
-          }
-        }
-        if (++c == n_chunks) { c = 0; job += n_slots; }
-      }
-      if (use_tma_out && issuer) tc::bulk_wait_all<0>();
-    } else {
-      const bool state_warp = grp < 2, u_warp = lq < 2;
-      // chain number `ci` of this slot: (batch, head) = job cslot + n_slots * ci; its state row for this thread
-      auto chain_state = [&](int ci) -> float* {
-        const int job = cslot + n_slots * ci, jb = job / H, jh = job % H;
-        const int sl = slots ? slots[jb] : jb;
-        return state + ((size_t)sl * H + jh) * KD * KD + (size_t)rowi * KD + grp * 64;
-      };
-      // B operand of the state, MN-major, N = 128: off(k, n) = (n/8)*2048 + (k/8)*128 + (k%8)*16 + (n%8)*2
-      uint8_t* sS_row = smem + F_S + (8 * grp) * 2048 + rowi * 16;
-      float S[64];
-      auto load_state = [&](const float* st) {
-#pragma unroll
-        for (int u = 0; u < 16; u++) {
-          const float4 x = *reinterpret_cast<const float4*>(st + u * 4);
-          S[4 * u] = x.x; S[4 * u + 1] = x.y; S[4 * u + 2] = x.z; S[4 * u + 3] = x.w;
-        }
-      };
-      auto put_operand = [&](int u0, int n) {              // pieces u0 .. u0 + n - 1 of this row's 64 columns as fp16
-#pragma unroll
-        for (int u = u0; u < u0 + n; u++)
-          *reinterpret_cast<uint4*>(sS_row + u * 2048) = make_uint4(pack_h2(S[8 * u], S[8 * u + 1]), pack_h2(S[8 * u + 2], S[8 * u + 3]),
-                                                                    pack_h2(S[8 * u + 4], S[8 * u + 5]), pack_h2(S[8 * u + 6], S[8 * u + 7]));
-      };
-      if (state_warp) {
-        load_state(chain_state(0));
-        put_operand(0, 8);
-        tc::fence_async_smem();
-        tc::mbar_arrive(&s_bar[0]);
-      }
-      int in_chain = 0, chain = 0;                         // chunk of the chain, chain of the slot
-      for (int v = 0; v < n_virtual; v++) {
-        const uint32_t par = v & 1;
-        const uint32_t d1 = tmem + par * 128, d2 = tmem + 256;
-        KS_TRACE(0, v);
-        KS_TRACE_AT(8, v, 0);
-        KS_TRACE_AT(9, v, 50);
-        KS_TRACE_AT(10, v, 450);
-        // ---- U (token rows = TMEM lanes 0-63 of D1) as the next operand: off(t, n) = (n/8)*1024 + t*16 + (n%8)*2 ----
-        if (u_warp) {
-          tc::mbar_wait(&mma_bar[par], (v >> 1) & 1, &abort_flag, 3);
-          tc::fence_after_sync();
-          KS_TRACE(1, v);
-          uint32_t r[32];
-          tc::tmem_ld32(d1 + (uint32_t)(grp * KNV) + ((uint32_t)(lq * 32) << 16), r);
-          tc::tmem_ld_wait();
-          uint8_t* urow = smem + F_U + (4 * grp) * 1024 + rowi * 16;
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            *reinterpret_cast<uint4*>(urow + u * 1024) =
-                make_uint4(pack_h2(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])), pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])),
-                           pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])), pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])));
-          tc::fence_async_smem();
-          tc::fence_before_sync();
-          tc::mbar_arrive(&u_bar);
-          KS_TRACE(2, v);
-        }
-        // ---- state: S <- S e^{G_last} + Kt^T U (lane = k row), refresh the fp16 operand copy ----
-        if (state_warp) {
-          tc::mbar_wait(&kb_bar[par], (v >> 1) & 1, &abort_flag, 2);
-          const float dec = reinterpret_cast<const float*>(smem + par * F_STAGE + U_DEC)[rowi];
-          tc::mbar_wait(&mma2_bar, par, &abort_flag, 4);
-          tc::fence_after_sync();
-          KS_TRACE(3, v);
-          const bool last = in_chain == n_chunks - 1;
-#pragma unroll
-          for (int hf = 0; hf < 2; hf++) {
-            uint32_t r[32];
-            tc::tmem_ld32(d2 + (uint32_t)(grp * 64 + hf * 32) + ((uint32_t)(lq * 32) << 16), r);
-            tc::tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; j++) S[hf * 32 + j] = fmaf(S[hf * 32 + j], dec, __uint_as_float(r[j]));
-            if (!last) put_operand(4 * hf, 4);
-          }
-          if (last) {
-            // last chunk of a chain: its final state goes back to memory and the slot's next chain begins
-            float* st = chain_state(chain);
-            if (!abort_flag) {
-#pragma unroll
-              for (int u = 0; u < 16; u++)
-                *reinterpret_cast<float4*>(st + u * 4) = make_float4(S[4 * u], S[4 * u + 1], S[4 * u + 2], S[4 * u + 3]);
-            }
-            if (v + 1 < n_virtual) {
-              load_state(chain_state(chain + 1));
-              put_operand(0, 8);
-            }
-          }
-          tc::fence_async_smem();
-          tc::fence_before_sync();
-          tc::mbar_arrive(&s_bar[par ^ 1]);
-          KS_TRACE(4, v);
-        }
-        if (++in_chain == n_chunks) { in_chain = 0; chain++; }
-      }
-    }
+    const int cslot = blockIdx.x / SLICES;                  // this CTA's chain slot
+    chain_cta<NV, true>(smem, bars, tmem, &abort_flag, [&](int v) { return ring + ((size_t)(v & (kr - 1)) * n_slots + cslot) * U_BYTES; },
+                        ready + (size_t)cslot * F_LINE, consumed + (size_t)blockIdx.x * F_LINE, g_abort, kr, cslot, n_slots, n_chunks, n_virtual,
+                        blockIdx.x % SLICES, H, seqlen, state, out_f32, slots, scale, &map_out);
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -1450,38 +1253,43 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
 
 }  // namespace hk
 
-#ifdef HK_DIAG
-extern "C" __attribute__((visibility("default"))) int hk_debug_kda_trace(long long* host_out) {
-  return cudaMemcpyFromSymbol(host_out, hk::hk_kda_trace, sizeof(long long) * 128) == cudaSuccess ? 0 : 3;
-}
-#endif
-
 namespace hk {
 namespace {
-// The fused launch serves calls with few (batch, head) chains: every chain occupies one SM, the rest prepare.
+// The fused launch serves calls with few (batch, head) chains: every chain occupies an SM or two, the rest prepare.
 // hk_kda_chunked_set_form(1) keeps the two-kernel form for every call (cross-check of the two forms in the tests).
 int g_chunked_form = 0;
-// Number of chain CTAs ("slots") of the fused launch for n_jobs (batch, head) chains, 0 = use the two-kernel form.  Up to
-// 48 chains get a slot each; more chains share slots (a slot walks its chains one after the other), which needs a slot
-// count that divides n_jobs: the largest divisor in [16, 48] that leaves at least 64 SMs to the preparation.
-int fused_slots(long long n_jobs) {
-  if (g_chunked_form != 0 || n_jobs <= 0) return 0;
-  const int room = sm_count() - 64;
+// Chain slots of the fused launch and the value columns of a chain CTA for n_jobs (batch, head) chains; no slots = use the two-kernel
+// form.  Chains share slots evenly (a slot walks its chains one after the other), and the preparation keeps 64 SMs or more.  Of the
+// divisors of n_jobs from 16 to 48, or n_jobs itself, the one for which the longer of the two sides takes least per chunk of all
+// chains: a chain CTA needs 1,380 ns a chunk with all 128 columns, 1,100 with 64, an SM of preparation workers 5,800 ns a unit.
+// (32,768 tokens x 8 heads 719 -> 532 us with two CTAs a chain, x 16 725 -> 580; 32 heads have one, at 84 SMs of workers they would
+// take 1,150; 3 sequences x 8,192 x 32 heads 786 with 48 slots of two chains, 685 with 32 of three.)
+struct FusedShape { int slots, nv; };
+FusedShape fused_shape(long long n_jobs) {
+  FusedShape best{0, KD};
+  if (g_chunked_form != 0 || n_jobs <= 0) return best;
+  const int sms = sm_count();
+  long long best_cost = LLONG_MAX;
   for (int d = 48; d >= 1; d--) {
-    if (d > room || n_jobs % d != 0) continue;
-    if (d == n_jobs || d >= 16) return d;
-    break;
+    if (n_jobs % d != 0 || (d != n_jobs && d < 16)) continue;
+    for (int nv = KD; nv >= 64; nv /= 2) {
+      const int workers = sms - d * (KD / nv);
+      if (workers < 64) continue;
+      const long long chain = (nv == KD ? 1380000LL : 1100000LL) / d, prep = 5800000LL / workers, cost = chain > prep ? chain : prep;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = {d, nv};
+      }
+    }
   }
-  return 0;
+  return best;
 }
-// Short calls run as two kernels although a fused form exists, in the ring's memory: the fused launch costs about 33 us before
-// its first chunk is through (flags cleared, cooperative launch, ring start-up) and 2.6 us per chunk of a chain, the two
-// kernels 15 us and 1.4 us per chunk and wave of scan CTAs (four per chain).  Measured at 32 heads: 64 tokens 33 -> 25 us,
-// 512 53 -> 40, 1,024 77 -> 68, equal at 1,536; 8 heads x 1,024 tokens 71 -> 43; 8 sequences x 64 heads x 64 tokens 176 -> 118.
-// The line: all units fit the ring's memory (16 chunks per slot), and either one wave of scan CTAs or at most 12 chunks
-// (48 heads x 1,024 tokens, two waves: 106 fused, 119 as two kernels).
+// Short calls run as two kernels although a fused form exists, in the ring's memory: the fused launch costs about 20 us before its first
+// chunk is through (flags cleared, cooperative launch, ring start-up).  Fused / two kernels, us: 8 heads x 64 tokens 25 / 18, x 512 32 /
+// 24, x 1,024 41 / 31; 32 heads x 256 33 / 21, x 1,024 60 / 49, x 1,536 75 / 72, x 2,048 89 / 92; 64 heads x 512 67 / 42.  The line
+// is the memory: all units have to fit the ring's (16 chunks per slot).
 bool short_call(long long n_jobs, int n_chunks, int n_slots) {
-  return n_jobs * n_chunks <= (long long)KR * n_slots && (KVS * n_jobs <= sm_count() || n_chunks <= 12);
+  return n_jobs * n_chunks <= 16LL * n_slots && (2 * n_jobs <= sm_count() || n_chunks <= 12);
 }
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1505,7 +1313,7 @@ bool encode_rows(CUtensorMap* map, const void* base, CUtensorMapDataType type, i
                 CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 size_t fused_flag_bytes(int n_slots) {
-  return (((size_t)F_FLAG_INTS + (size_t)n_slots * 2 * F_LINE) * sizeof(int) + 255) / 256 * 256;
+  return (((size_t)F_FLAG_INTS + (size_t)n_slots * 3 * F_LINE) * sizeof(int) + 255) / 256 * 256;
 }
 }  // namespace
 }  // namespace hk
@@ -1527,9 +1335,9 @@ HK_API int hk_kda_chunked_set_form(int form) {
 HK_API size_t hk_kda_chunked_workspace_bytes(int bsz, int seqlen, int num_heads) {
   if (bsz <= 0 || seqlen <= 0 || num_heads <= 0) return 0;
   const long long n_jobs = (long long)bsz * num_heads;
-  if (const int n_slots = hk::fused_slots(n_jobs))
-    return hk::fused_flag_bytes(n_slots) + (size_t)hk::KR * n_slots * hk::U_BYTES;
   const size_t n_chunks = ((size_t)seqlen + hk::KC - 1) / hk::KC;
+  if (const int n_slots = hk::fused_shape(n_jobs).slots)
+    return hk::fused_flag_bytes(n_slots) + (size_t)hk::ring_depth(n_slots, (int)(n_jobs / n_slots * n_chunks)) * n_slots * hk::U_BYTES;
   return (size_t)bsz * num_heads * n_chunks * hk::U_BYTES;
 }
 
@@ -1553,74 +1361,71 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     if (cudaFuncSetAttribute(kda_chunk_prep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(P1_SMEM + 1024)) != cudaSuccess ||
         cudaFuncSetAttribute(kda_chunk_prep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(P1_SMEM + 1024)) != cudaSuccess ||
-        cudaFuncSetAttribute(kda_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(kda_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(kda_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_SMEM) != cudaSuccess)
+        cudaFuncSetAttribute(kda_chunk_scan_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Chain<64>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(kda_chunk_scan_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Chain<128>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(kda_fused_kernel<false, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem<64>()) != cudaSuccess ||
+        cudaFuncSetAttribute(kda_fused_kernel<true, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem<64>()) != cudaSuccess ||
+        cudaFuncSetAttribute(kda_fused_kernel<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem<128>()) != cudaSuccess ||
+        cudaFuncSetAttribute(kda_fused_kernel<true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem<128>()) != cudaSuccess)
       return HK_ERR_CUDA;
     attr_set[dev] = true;
   }
-  // tensor maps of the inputs, [batch][token][channels]: boxes of 64 tokens x 128 bytes, 128-byte swizzle, zeros past the last token
-  alignas(64) CUtensorMap map_qkv, map_g;
+  // tensor maps of the inputs, [batch][token][channels]: boxes of 64 tokens x 128 bytes, 128-byte swizzle, zeros past the last token;
+  // and of the output [batch][token][head][128] bf16: 64 channels x 1 head x 64 tokens x 1 sequence
+  alignas(64) CUtensorMap map_qkv, map_g, map_out;
   if (!encode_rows(&map_qkv, mixed_qkv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 3 * num_heads * KD, seqlen, bsz, 64) ||
       !encode_rows(&map_g, g_or_f, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, num_heads * KD, seqlen, bsz, 32))
     return HK_ERR_CUDA;
+  {
+    const cuuint64_t dims[4] = {(cuuint64_t)KD, (cuuint64_t)num_heads, (cuuint64_t)seqlen, (cuuint64_t)bsz};
+    const cuuint64_t strides[3] = {(cuuint64_t)KD * 2, (cuuint64_t)num_heads * KD * 2, (cuuint64_t)seqlen * num_heads * KD * 2};
+    const cuuint32_t box[4] = {64, 1, (cuuint32_t)KC, 1}, estr[4] = {1, 1, 1, 1};
+    if (tensor_map_encoder()(&map_out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return HK_ERR_CUDA;
+  }
   cudaStream_t s = as_stream(stream);
   int* st = device_status_ptr();
-  const int n_slots = fused_slots((long long)bsz * num_heads);
-  if (n_slots && !short_call((long long)bsz * num_heads, n_chunks, n_slots)) {
-    // one cooperative launch: chain slots on the first n_slots CTAs, preparation workers on all others
-    const int n_jobs = bsz * num_heads;
+  const float scale = 1.0f / sqrtf((float)KD);
+  if (!gated) {
+    dt_bias = a_log = nullptr;
+    lower_bound = 0.f;
+  }
+  const int n_jobs = bsz * num_heads;
+  const FusedShape shape = fused_shape(n_jobs);
+  const int n_slots = shape.slots;
+  if (n_slots && !short_call(n_jobs, n_chunks, n_slots)) {
+    // one cooperative launch: chain CTAs first, preparation workers on all others
     const size_t flag_bytes = fused_flag_bytes(n_slots);
     if (cudaMemsetAsync(workspace, 0, flag_bytes, s) != cudaSuccess) return HK_ERR_CUDA;
+    const bool split = shape.nv < KD;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count());
     cfg.blockDim = dim3(512);
-    cfg.dynamicSmemBytes = F_SMEM;
+    cfg.dynamicSmemBytes = split ? fused_smem<64>() : fused_smem<128>();
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    uint8_t* a_ring = (uint8_t*)workspace + flag_bytes;
-    int* a_flags = (int*)workspace;
-    __nv_bfloat16* a_out = (__nv_bfloat16*)out;
-    const float a_scale = 1.0f / sqrtf((float)KD);
-    // tensor map over the output [bsz][seqlen][H][128] bf16 for the chain CTAs' tiled stores: box = 64 channels x 1 head x
-    // 64 tokens x 1 sequence, 128-byte swizzle; without the encoder the kernel stores the rows itself
-    alignas(64) CUtensorMap tmap;
-    memset(&tmap, 0, sizeof(tmap));
-    int use_tma_out = 0;
-    {
-      const EncodeFn encode = tensor_map_encoder();
-      if (encode) {
-        const cuuint64_t dims[4] = {(cuuint64_t)KD, (cuuint64_t)num_heads, (cuuint64_t)seqlen, (cuuint64_t)bsz};
-        const cuuint64_t strides[3] = {(cuuint64_t)KD * 2, (cuuint64_t)num_heads * KD * 2, (cuuint64_t)seqlen * num_heads * KD * 2};
-        const cuuint32_t box[4] = {64, 1, (cuuint32_t)KC, 1};
-        const cuuint32_t estr[4] = {1, 1, 1, 1};
-        if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
-          use_tma_out = 1;
-      }
-    }
-    const float* a_dt = gated ? dt_bias : nullptr;
-    const float* a_al = gated ? a_log : nullptr;
-    const float a_lb = gated ? lower_bound : 0.f;
-    cudaError_t e = gated
-        ? cudaLaunchKernelEx(&cfg, kda_fused_kernel<true>, map_qkv, map_g, beta_or_b, a_ring, a_flags, state, a_out, out_f32,
-                             seqlen, num_heads, n_chunks, n_jobs, n_slots, slots, a_scale, st, a_dt, a_al, a_lb, tmap, use_tma_out)
-        : cudaLaunchKernelEx(&cfg, kda_fused_kernel<false>, map_qkv, map_g, beta_or_b, a_ring, a_flags, state, a_out, out_f32,
-                             seqlen, num_heads, n_chunks, n_jobs, n_slots, slots, a_scale, st, a_dt, a_al, a_lb, tmap, use_tma_out);
-    return e == cudaSuccess ? HK_OK : HK_ERR_CUDA;
+    auto kern = gated ? (split ? kda_fused_kernel<true, 64> : kda_fused_kernel<true, 128>)
+                      : (split ? kda_fused_kernel<false, 64> : kda_fused_kernel<false, 128>);
+    return cudaLaunchKernelEx(&cfg, kern, map_qkv, map_g, beta_or_b, (uint8_t*)workspace + flag_bytes, (int*)workspace, state, out_f32, seqlen,
+                              num_heads, n_chunks, n_jobs, n_slots, slots, scale, st, dt_bias, a_log, lower_bound, map_out) == cudaSuccess
+               ? HK_OK
+               : HK_ERR_CUDA;
   }
   const dim3 grid(num_heads, n_chunks, bsz);
   auto prep = gated ? kda_chunk_prep_kernel<true> : kda_chunk_prep_kernel<false>;
-  if (pdl_launch(prep, grid, dim3(256), P1_SMEM + 1024, s, map_qkv, map_g, beta_or_b, (uint8_t*)workspace, seqlen,
-                 num_heads, n_chunks, st, gated ? dt_bias : nullptr, gated ? a_log : nullptr,
-                 gated ? lower_bound : 0.f) != cudaSuccess)
+  if (pdl_launch(prep, grid, dim3(256), P1_SMEM + 1024, s, map_qkv, map_g, beta_or_b, (uint8_t*)workspace, seqlen, num_heads, n_chunks, st,
+                 dt_bias, a_log, lower_bound) != cudaSuccess)
     return HK_ERR_CUDA;
-  return pdl_launch(kda_chunk_scan_kernel, dim3(KVS, num_heads, bsz), dim3(128), P2_SMEM, s, (const uint8_t*)workspace, state,
-                    (__nv_bfloat16*)out, out_f32, seqlen, num_heads, n_chunks, slots, 1.0f / sqrtf((float)KD), st) == cudaSuccess
+  // half a head per CTA while these are one wave
+  const bool split = 2 * n_jobs <= sm_count();
+  return pdl_launch(split ? kda_chunk_scan_kernel<64> : kda_chunk_scan_kernel<128>, dim3(split ? 2 : 1, num_heads, bsz), dim3(512),
+                    split ? Chain<64>::SMEM : Chain<128>::SMEM, s, (const uint8_t*)workspace, state, out_f32, seqlen, num_heads, n_chunks, slots,
+                    scale, st, map_out) == cudaSuccess
              ? HK_OK
              : HK_ERR_CUDA;
 }
