@@ -27,8 +27,8 @@
 // The scan walks the chunks of a chain in order; the fp32 state stays in registers.  Per chunk: D1 = [I ; 0] Uloc + [-W ; Q+] S0 (rows
 // 0-63 are U), Kt^T U (state), [. ; B beta] U onto the Q+ S0 rows (outputs), all tcgen05 with TMEM accumulators.
 #include <cuda.h>   // CUtensorMap (types only; the encoder is fetched through the runtime at first use)
-#include <cuda_pipeline_primitives.h>
 
+#include <algorithm>
 #include <climits>
 
 #include "hk_common.cuh"
@@ -39,8 +39,10 @@ namespace hk {
 constexpr int KC = 64;                    // chunk length
 constexpr int KD = 128;                   // head dim (k and v)
 // Fused form: ring slots (chunks) per chain slot, a power of two up to 32.  A worker's unit takes ten chunks of a chain from the moment
-// its ring slot is free; few long chains are waited for by many workers and get the deeper ring, many chains keep theirs within L2.
-__host__ __device__ constexpr int ring_depth(int n_slots, int n_virtual) { return n_slots <= 16 && n_virtual >= 64 ? 32 : 16; }
+// its ring slot is free; few long chains are waited for by many workers and get the deeper ring where the workspace has the room (the
+// query asks for it, a call runs without): 32,768 tokens x 8 heads 578 us, 627 with the ring of 16; x 16 heads 582 / 621; x 1 548 / 583.
+// Many chains keep theirs within L2.
+constexpr int RING = 16, DEEP_RING = 32;
 // Flags: [0] launch-wide abort word, then a 128-byte line of ready flags per chain slot and one for the consumed count per chain CTA.  With all of
 // them packed into a few lines of one page the polls of 232 workers held up the chains' own flags: 1.05 or 1.3-1.9 ms for 32,768
 // tokens x 32 heads, by the die that the page's address falls to.
@@ -829,9 +831,9 @@ __device__ __forceinline__ void chain_init(ChainBars& bars) {   // one thread
   tc::mbar_init(&bars.u, 256);
 }
 // Chains job0, job0 + job_step, ... of n_chunks chunks each, n_virtual chunks in all; a job is (batch, head).  Chunk numbers run through
-// all of them (`v`), and ring, flags and barrier parities go by v.  RING: `my_ready` and `my_consumed` are the slot's flags.
+// all of them (`v`), and ring, flags and barrier parities go by v.  FLAGS (fused form, ring of kr units): `my_ready` and `my_consumed` are the slot's flags.
 // `unit_of(v)`: the unit of a chunk.
-template <int NV, bool RING, class UnitOf>
+template <int NV, bool FLAGS, class UnitOf>
 __device__ __forceinline__ void chain_cta(uint8_t* smem, ChainBars& bars, const uint32_t tmem, int* abort_flag, UnitOf&& unit_of, const int* my_ready,
                                           int* my_consumed, int* g_abort, int kr, int job0, int job_step, int n_chunks, int n_virtual, int slice, int H,
                                           int seqlen, float* __restrict__ state, float* __restrict__ out_f32, const int* __restrict__ slots,
@@ -934,7 +936,7 @@ __device__ __forceinline__ void chain_cta(uint8_t* smem, ChainBars& bars, const 
     // every chunk.
     int known = 0;                                         // units before this one are complete
     auto await_unit = [&](int v) {
-      if (!RING) return;
+      if (!FLAGS) return;
       const long long t0 = clock64();
       while (known <= v) {
         const bool here = lane < kr && ld_acquire_gpu(my_ready + ((known + lane) & (kr - 1))) > known + lane;
@@ -965,7 +967,7 @@ __device__ __forceinline__ void chain_cta(uint8_t* smem, ChainBars& bars, const 
       // the copy engine's reads are complete, nothing this thread wrote is handed over with the flag.
       tc::mbar_wait(&bars.wu[par], ph, abort_flag, 2);
       tc::mbar_wait(&bars.kb[par], ph, abort_flag, 2);
-      if (RING && lane == 0) st_relaxed_gpu(my_consumed, v + 1);
+      if (FLAGS && lane == 0) st_relaxed_gpu(my_consumed, v + 1);
       if (v + 2 >= n_virtual) continue;
       await_unit(v + 2);
       tc::mbar_wait(&bars.mma[par], ph, abort_flag, 3);
@@ -1176,7 +1178,7 @@ template <bool GATED, int NV>
 __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
     const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
     uint8_t* __restrict__ ring, int* __restrict__ flags, float* __restrict__ state,
-    float* __restrict__ out_f32, int seqlen, int H, int n_chunks, int n_jobs, int n_slots, const int* __restrict__ slots,
+    float* __restrict__ out_f32, int seqlen, int H, int n_chunks, int n_jobs, int n_slots, int kr, const int* __restrict__ slots,
     float scale, int* __restrict__ status, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
     float lower_bound, const __grid_constant__ CUtensorMap map_out) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -1192,7 +1194,6 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
   int* ready = flags + F_FLAG_INTS;                        // [n_slots][ring depth], a line per slot
   int* consumed = ready + (size_t)n_slots * F_LINE;        // [n_chain_ctas], a line each
   const int n_virtual = (n_jobs / n_slots) * n_chunks;     // chunks a slot walks
-  const int kr = ring_depth(n_slots, n_virtual);
 
   if (tid == 0) {
     chain_init(bars);
@@ -1264,9 +1265,10 @@ int g_chunked_form = 0;
 // chains: a chain CTA needs 1,380 ns a chunk with all 128 columns, 1,100 with 64, an SM of preparation workers 5,800 ns a unit.
 // (32,768 tokens x 8 heads 719 -> 532 us with two CTAs a chain, x 16 725 -> 580; 32 heads have one, at 84 SMs of workers they would
 // take 1,150; 3 sequences x 8,192 x 32 heads 786 with 48 slots of two chains, 685 with 32 of three.)
-struct FusedShape { int slots, nv; };
+// `room`: the slots that the workspace is sized for, the largest number that divides the chains: it covers calls of fewer sequences.
+struct FusedShape { int slots, nv, room; };
 FusedShape fused_shape(long long n_jobs) {
-  FusedShape best{0, KD};
+  FusedShape best{0, KD, 0};
   if (g_chunked_form != 0 || n_jobs <= 0) return best;
   const int sms = sm_count();
   long long best_cost = LLONG_MAX;
@@ -1275,10 +1277,11 @@ FusedShape fused_shape(long long n_jobs) {
     for (int nv = KD; nv >= 64; nv /= 2) {
       const int workers = sms - d * (KD / nv);
       if (workers < 64) continue;
+      if (!best.room) best.room = d;
       const long long chain = (nv == KD ? 1380000LL : 1100000LL) / d, prep = 5800000LL / workers, cost = chain > prep ? chain : prep;
       if (cost < best_cost) {
         best_cost = cost;
-        best = {d, nv};
+        best = {d, nv, best.room};
       }
     }
   }
@@ -1289,7 +1292,7 @@ FusedShape fused_shape(long long n_jobs) {
 // 24, x 1,024 41 / 31; 32 heads x 256 33 / 21, x 1,024 60 / 49, x 1,536 75 / 72, x 2,048 89 / 92; 64 heads x 512 67 / 42.  The line
 // is the memory: all units have to fit the ring's (16 chunks per slot).
 bool short_call(long long n_jobs, int n_chunks, int n_slots) {
-  return n_jobs * n_chunks <= 16LL * n_slots && (2 * n_jobs <= sm_count() || n_chunks <= 12);
+  return n_jobs * n_chunks <= (long long)RING * n_slots && (2 * n_jobs <= sm_count() || n_chunks <= 12);
 }
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1312,9 +1315,11 @@ bool encode_rows(CUtensorMap* map, const void* base, CUtensorMapDataType type, i
   return encode(map, type, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                 CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+bool deep_ring(int n_slots, long long n_virtual) { return n_slots <= 16 && n_virtual >= 64; }
 size_t fused_flag_bytes(int n_slots) {
   return (((size_t)F_FLAG_INTS + (size_t)n_slots * 3 * F_LINE) * sizeof(int) + 255) / 256 * 256;
 }
+size_t ring_bytes(int n_slots, int depth) { return fused_flag_bytes(n_slots) + (size_t)depth * n_slots * U_BYTES; }
 }  // namespace
 }  // namespace hk
 
@@ -1336,8 +1341,11 @@ HK_API size_t hk_kda_chunked_workspace_bytes(int bsz, int seqlen, int num_heads)
   if (bsz <= 0 || seqlen <= 0 || num_heads <= 0) return 0;
   const long long n_jobs = (long long)bsz * num_heads;
   const size_t n_chunks = ((size_t)seqlen + hk::KC - 1) / hk::KC;
-  if (const int n_slots = hk::fused_shape(n_jobs).slots)
-    return hk::fused_flag_bytes(n_slots) + (size_t)hk::ring_depth(n_slots, (int)(n_jobs / n_slots * n_chunks)) * n_slots * hk::U_BYTES;
+  const hk::FusedShape shape = hk::fused_shape(n_jobs);
+  if (shape.slots) {
+    const size_t ring = hk::ring_bytes(shape.room, hk::RING);
+    return hk::deep_ring(shape.slots, n_jobs / shape.slots * n_chunks) ? std::max(ring, hk::ring_bytes(shape.slots, hk::DEEP_RING)) : ring;
+  }
   return (size_t)bsz * num_heads * n_chunks * hk::U_BYTES;
 }
 
@@ -1353,8 +1361,12 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
   HK_REQUIRE(bsz <= 65535 && (seqlen + KC - 1) / KC <= 65535);   // grid limits
   HK_REQUIRE(aligned(mixed_qkv, 16) && aligned(g_or_f, 16) && aligned(state, 16) && aligned(out, 16) &&
              aligned(workspace, 256) && (!out_f32 || aligned(out_f32, 16)));
-  if (workspace_bytes < hk_kda_chunked_workspace_bytes(bsz, seqlen, num_heads)) return HK_ERR_WORKSPACE;
-  const int n_chunks = (seqlen + KC - 1) / KC;
+  const int n_chunks = (seqlen + KC - 1) / KC, n_jobs = bsz * num_heads;
+  const FusedShape shape = fused_shape(n_jobs);
+  const int n_slots = shape.slots;
+  if (workspace_bytes < (n_slots ? ring_bytes(shape.room, RING) : hk_kda_chunked_workspace_bytes(bsz, seqlen, num_heads))) return HK_ERR_WORKSPACE;
+  const bool deep = n_slots && deep_ring(n_slots, (long long)n_jobs / n_slots * n_chunks) && workspace_bytes >= ring_bytes(n_slots, DEEP_RING);
+  const int kr = deep ? DEEP_RING : RING;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1391,9 +1403,6 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
     dt_bias = a_log = nullptr;
     lower_bound = 0.f;
   }
-  const int n_jobs = bsz * num_heads;
-  const FusedShape shape = fused_shape(n_jobs);
-  const int n_slots = shape.slots;
   if (n_slots && !short_call(n_jobs, n_chunks, n_slots)) {
     // one cooperative launch: chain CTAs first, preparation workers on all others
     const size_t flag_bytes = fused_flag_bytes(n_slots);
@@ -1412,7 +1421,7 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
     auto kern = gated ? (split ? kda_fused_kernel<true, 64> : kda_fused_kernel<true, 128>)
                       : (split ? kda_fused_kernel<false, 64> : kda_fused_kernel<false, 128>);
     return cudaLaunchKernelEx(&cfg, kern, map_qkv, map_g, beta_or_b, (uint8_t*)workspace + flag_bytes, (int*)workspace, state, out_f32, seqlen,
-                              num_heads, n_chunks, n_jobs, n_slots, slots, scale, st, dt_bias, a_log, lower_bound, map_out) == cudaSuccess
+                              num_heads, n_chunks, n_jobs, n_slots, kr, slots, scale, st, dt_bias, a_log, lower_bound, map_out) == cudaSuccess
                ? HK_OK
                : HK_ERR_CUDA;
   }

@@ -4,6 +4,7 @@
 #include "../../include/helios_b200_shim.hpp"
 #pragma GCC visibility pop
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 
@@ -58,6 +59,14 @@ void* scratch(size_t bytes) {
     s.bytes = want;
   }
   return s.ptr;
+}
+
+// As scratch(), for a launcher that can do with less: of host-provided memory `bytes` becomes what there is.
+void* scratch_up_to(size_t& bytes) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && g_scratch[dev].injected) bytes = std::min(bytes, g_scratch[dev].bytes);
+  return scratch(bytes);
 }
 
 }  // namespace
@@ -184,8 +193,9 @@ void cuda_recurrent_gated_delta_rule(const bfloat16* mixed_qkv, const float* g,
                                                   channelwise, history) != 0;
   if (chunked) {
     size_t bytes = hk_kda_chunked_workspace_bytes(bsz, seqlen, num_v_heads);
+    void* ws = scratch_up_to(bytes);
     int st = hk_kda_chunked_prefill(mixed_qkv, g, beta, recurrent_state, core_attn_out, nullptr, bsz,
-                                    seqlen, num_v_heads, slots, scratch(bytes), bytes, stream);
+                                    seqlen, num_v_heads, slots, ws, bytes, stream);
     if (st != HK_ERR_UNSUPPORTED) {
       check(st, "cuda_recurrent_gated_delta_rule (chunked)");
       return;

@@ -275,6 +275,53 @@ def test_chunked_fused_launch_equals_two_kernel_form(T, H, bsz):
         assert max_rel(res[1][1], o_32) < 2e-3 and frob_rel(res[1][2], o_st) < 1e-2
 
 
+@pytest.mark.parametrize("T,H,bsz,strong", [(4097, 1, 1, False), (4160, 16, 1, True), (1090, 23, 1, True), (1090, 24, 1, False),
+                                            (600, 51, 1, False), (1040, 16, 3, True), (1030, 63, 1, False)])
+def test_chunked_chain_shapes_and_ring_depths(T, H, bsz, strong):
+    """One or two CTAs a chain, a slot of one to three chains, rings of 16 and 32 units, raw and formed gates, every token at the
+    bound of the decay: the bits of the two-kernel form.  The deep ring (16 slots or fewer, 64 chunks or more) is asked for, not
+    required: half its units are enough, with the same bits, and a workspace below them is refused."""
+    D, unit = 128, 74240
+    inp = synth.kda_inputs(T, H, D, bsz=bsz, seed=300 + T + H)
+    q, b = dev_bf16(inp["mixed_qkv"]), dev_bf16(inp["beta"])
+    g = dev(np.full_like(inp["g"], -5.0) if strong else inp["g"])
+    gen = torch.Generator(device="cuda").manual_seed(T + H)
+    f, bl = torch.randn(bsz, T, H, D, generator=gen, device="cuda"), torch.randn(bsz, T, H, generator=gen, device="cuda")
+    dt, al = torch.randn(H, D, generator=gen, device="cuda"), torch.randn(H, generator=gen, device="cuda")
+    s0 = 0.1 * torch.randn(bsz, 1, H, D, D, generator=gen, device="cuda")
+    full = hk.kda_chunked_workspace_bytes(bsz, T, H)
+    deep = H * bsz <= 16
+    least = full - 16 * H * bsz * unit if deep else full
+
+    def run(nbytes):
+        ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        got = []
+        for gated in (False, True):
+            st, out = s0.clone(), torch.empty(bsz, T, H, D, dtype=torch.bfloat16, device="cuda")
+            o32 = torch.empty(bsz, T, H, D, device="cuda")
+            if gated:
+                hk.kda_chunked_prefill_gated(q, f, bl, dt, al, -5.0, st, out, bsz, T, H, out_f32=o32, workspace=ws)
+            else:
+                hk.cuda_recurrent_gated_delta_rule(q, g, b, st, out, bsz, T, H, H, D, D, 1, None, True, False, out_f32=o32,
+                                                   workspace=ws)
+            got += [st, out, o32]
+        torch.cuda.synchronize()
+        assert hk.read_device_status() == 0
+        return got
+
+    first = run(full)
+    others = [run(least)] if deep else []
+    with pytest.raises(hk.HeliosB200Error):
+        run(least - 1)
+    try:
+        hk.kda_chunked_set_form(1)
+        others.append(run(hk.kda_chunked_workspace_bytes(bsz, T, H)))
+    finally:
+        hk.kda_chunked_set_form(0)
+    for got in others:
+        assert all(torch.equal(x, y) for x, y in zip(first, got))
+
+
 @pytest.mark.parametrize("H,bsz", [(32, 1), (4, 2), (64, 3), (64, 5)])
 def test_decode_step_with_conv_inside_equals_the_two_launch_sequence(H, bsz):
     """hk_kda_decode_step (conv + recurrence of one decoded token in one launch, value slices of a head as a cluster)
