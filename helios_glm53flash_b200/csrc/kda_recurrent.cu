@@ -4,7 +4,7 @@
 //
 // Kernels:
 //   kda_decode_kernel, kda_decode_stream_kernel   one token per sequence (the decode step, the decode layer, the recurrence alone)
-//   kda_recurrent_cols_kernel                     several tokens, channelwise decay, no history
+//   kda_recurrent_few_kernel, kda_recurrent_cols_kernel   several tokens, channelwise decay, no history: few chains; others
 //   kda_recurrent_rows_kernel                     channelwise decay with a history, and a few tokens of many chains
 //   kda_recurrent_kernel                          one decay per head, 128- and 64-wide heads
 // The state lives in REGISTERS for the whole call (the reference re-reads and re-writes it from global memory on every token),
@@ -18,6 +18,8 @@
 // rg + 16; a group runs over its even and its odd rows separately (the two halves of a packed fp32 pair), ascending; groups rg
 // and rg + 8 are added first, then the 8 sums as a balanced tree.  Norms: inv_norm.
 // One decay per head: 4 or 8 ascending row groups; for 128 x 32 slices that is the reference's 4 x 32 order (gdn.cu:683-705).
+#include <algorithm>
+
 #include "hk_common.cuh"
 #include "kda_norm_common.cuh"
 #include "tc05.cuh"
@@ -685,33 +687,39 @@ static int launch_decode(const DecodeArgs& a, cudaStream_t s) {
 // 6 reads of 4 wavefronts.  With 8 groups over 8 lanes (and k * d as a fourth vector) it was 16 reads (64 heads: 0.84 us per token with one column per lane,
 // 0.57 with four).  The output sums of four tokens are taken together and exchange HALF of their values at each step (15
 // shuffles for 16 values instead of 64).
-// CPL is the one that yields 256 CTAs or more from 64, 32 and 16 chains.
+// CPL 4 takes states on a 16-byte boundary, 1 any.
 // ---------------------------------------------------------------------------------------------
-// Sums of N values per lane over the 16 lanes of a half warp, lanes 8 apart first, then 1, 2, 4.  While a lane has more than
-// one value it keeps one half and hands the other to its partner; a lane ends with the sum of value sum_index (the same in
-// all lanes that agree in the bits used; sum_owner picks one of them).
-template <int N>
+// Sums of N values per lane over the L lanes that share their columns: of 16, lanes 8 apart first; then 1, 2, 4.  While a lane has more than one value it keeps one half and hands the
+// other to its partner; a lane ends with the sum of value sum_index (the same in all lanes that agree in the bits used; sum_owner
+// picks one of them).
+template <int L>
+__device__ __forceinline__ constexpr int sum_mask(int st) { return L == 16 ? (st == 0 ? 8 : 1 << (st - 1)) : 1 << st; }
+template <int N, int L>
 __device__ __forceinline__ int sum_index(int lane) {
-  const int b3 = (lane >> 3) & 1, b0 = lane & 1, b1 = (lane >> 1) & 1, b2 = (lane >> 2) & 1;
-  if (N == 16) return 8 * b3 + 4 * b0 + 2 * b1 + b2;
-  if (N == 8) return 4 * b3 + 2 * b0 + b1;
-  if (N == 4) return 2 * b3 + b0;
-  if (N == 2) return b3;
-  return 0;
+  int idx = 0;
+#pragma unroll
+  for (int st = 0, n = N; n > 1; st++) {
+    n >>= 1;
+    if (lane & sum_mask<L>(st)) idx += n;
+  }
+  return idx;
 }
-template <int N>
+template <int N, int L>
 __device__ __forceinline__ bool sum_owner(int lane) {
-  return N == 16 || (lane & (N == 8 ? 4 : (N == 4 ? 6 : (N == 2 ? 7 : 15)))) == 0;
+  int left = L - 1;
+#pragma unroll
+  for (int st = 0, n = N; n > 1; st++, n >>= 1) left &= ~sum_mask<L>(st);
+  return (lane & left) == 0;
 }
-template <int N>
+template <int N, int L>
 __device__ __forceinline__ float lane_sums(const float* v, int lane) {
   float x[N];
 #pragma unroll
   for (int i = 0; i < N; i++) x[i] = v[i];
   int n = N;
 #pragma unroll
-  for (int st = 0; st < 4; st++) {
-    const int m = st == 0 ? 8 : 1 << (st - 1);
+  for (int st = 0; (1 << st) < L; st++) {
+    const int m = sum_mask<L>(st);
     if (n > 1) {
       n >>= 1;
 #pragma unroll
@@ -728,18 +736,90 @@ __device__ __forceinline__ float lane_sums(const float* v, int lane) {
   }
   return x[0];
 }
-constexpr int RC_TB = 8, RC_WARPS = 4;
+constexpr int RC_TB = 8, RC_WARPS = 4;   // tokens of a batch; warps that prepare it, and that walk through it
 template <int COLS>
 struct alignas(16) RecBatch {           // 8 prepared tokens
   float q[RC_TB][128], k[RC_TB][128], d[RC_TB][128], v[RC_TB][COLS], beta[RC_TB];
 };
+// Tokens warp, warp + 4 of a batch on their way: channel lane + 32 u of q, k, g, columns lane, lane + 32 of v.  Kept as loaded: a
+// conversion in fetch would wait for the loads.
+template <int COLS>
+struct RecTokens {
+  static constexpr int TPW = RC_TB / RC_WARPS, NVL = (COLS + 31) / 32;
+  __nv_bfloat16 q[TPW][4], k[TPW][4], v[TPW][NVL], be[TPW];
+  float g[TPW][4];
+  // tok, gp, bp: first token of the sequence; gp and bp of the head, v_at: first of the CTA's columns in a row
+  __device__ __forceinline__ void fetch(int s0, int seqlen, int warp, int lane, const __nv_bfloat16* tok, size_t row, size_t q_at, size_t k_at,
+                                        size_t v_at, const float* gp, const __nv_bfloat16* bp, int Hv) {
+#pragma unroll
+    for (int p = 0; p < TPW; p++) {
+      const int s = s0 + warp + p * RC_WARPS;
+      if (s >= seqlen) break;
+      const __nv_bfloat16* t = tok + (size_t)s * row;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        q[p][u] = t[q_at + lane + 32 * u];
+        k[p][u] = t[k_at + lane + 32 * u];
+        g[p][u] = gp[(size_t)s * Hv * 128 + lane + 32 * u];
+      }
+#pragma unroll
+      for (int u = 0; u < NVL; u++)
+        if (lane + 32 * u < COLS) v[p][u] = t[v_at + lane + 32 * u];
+      be[p] = bp[(size_t)s * Hv];
+    }
+  }
+  __device__ __forceinline__ void prepare(RecBatch<COLS>& r, int s0, int seqlen, int warp, int lane) const {
+#pragma unroll
+    for (int p = 0; p < TPW; p++) {
+      const int t = warp + p * RC_WARPS;
+      if (s0 + t >= seqlen) break;
+      float fq[4], fk[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        fq[u] = __bfloat162float(q[p][u]);
+        fk[u] = __bfloat162float(k[p][u]);
+      }
+      const float iq = inv_norm(fq), ik = inv_norm(fk);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int c = lane + 32 * u;
+        r.q[t][c] = __fmul_rn(fq[u], iq);
+        r.k[t][c] = __fmul_rn(fk[u], ik);
+        r.d[t][c] = __expf(g[p][u]);
+      }
+#pragma unroll
+      for (int u = 0; u < NVL; u++)
+        if (lane + 32 * u < COLS) r.v[t][lane + 32 * u] = __bfloat162float(v[p][u]);
+      if (lane == 0) r.beta[t] = __bfloat162float(be[p]);
+    }
+  }
+};
+// The CPL columns at p, a vector each way.
+template <int CPL>
+__device__ __forceinline__ void ld_cols(const float* p, float (&x)[CPL]) {
+  if constexpr (CPL == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+  } else if constexpr (CPL == 2) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    x[0] = v.x; x[1] = v.y;
+  } else {
+    x[0] = p[0];
+  }
+}
+template <int CPL>
+__device__ __forceinline__ void st_cols(float* p, const float (&x)[CPL]) {
+  if constexpr (CPL == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+  else if constexpr (CPL == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+  else p[0] = x[0];
+}
 
 template <int CPL>
 __global__ __launch_bounds__(RC_WARPS * 32) void kda_recurrent_cols_kernel(
     const __nv_bfloat16* __restrict__ mixed_qkv, const float* __restrict__ g, const __nv_bfloat16* __restrict__ beta,
     float* __restrict__ state, __nv_bfloat16* __restrict__ out, float* __restrict__ out_f32, int seqlen, int Hk, int Hv, float scale,
     const int* __restrict__ slots) {
-  constexpr int COLS = RC_WARPS * 2 * CPL, TPW = RC_TB / RC_WARPS;      // columns of the CTA, tokens a warp prepares
+  constexpr int COLS = RC_WARPS * 2 * CPL;                             // columns of the CTA
   __shared__ RecBatch<COLS> rb[2];
   __shared__ __align__(16) float s_o[2][RC_TB][COLS];
   const int b = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * COLS;
@@ -754,85 +834,24 @@ __global__ __launch_bounds__(RC_WARPS * 32) void kda_recurrent_cols_kernel(
   const __nv_bfloat16* bp = beta + (size_t)b * seqlen * Hv + head;
   float* sp = state + ((size_t)slot * Hv + head) * 128 * 128 + v0 + col;
 
-  // tokens warp, warp + 4 of a batch: channel lane + 32 u of q, k, g, columns lane, lane + 32 of v
-  constexpr int NVL = (COLS + 31) / 32;
-  // (kept as loaded: a conversion here would wait for the load before the tokens in hand)
-  __nv_bfloat16 rq[TPW][4], rk[TPW][4], rv[TPW][NVL], rbeta[TPW];
-  float rgt[TPW][4];
+  RecTokens<COLS> ahead;
   auto fetch = [&](int s0) {
-#pragma unroll
-    for (int p = 0; p < TPW; p++) {
-      const int s = s0 + warp + p * RC_WARPS;
-      if (s >= seqlen) break;
-      const __nv_bfloat16* t = tok + (size_t)s * row;
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        rq[p][u] = t[(size_t)k_head * 128 + lane + 32 * u];
-        rk[p][u] = t[(size_t)(Hk + k_head) * 128 + lane + 32 * u];
-        rgt[p][u] = gp[(size_t)s * Hv * 128 + lane + 32 * u];
-      }
-#pragma unroll
-      for (int u = 0; u < NVL; u++)
-        if (lane + 32 * u < COLS) rv[p][u] = t[(size_t)2 * Hk * 128 + (size_t)head * 128 + v0 + lane + 32 * u];
-      rbeta[p] = bp[(size_t)s * Hv];
-    }
-  };
-  auto prepare = [&](RecBatch<COLS>& r, int s0) {
-#pragma unroll
-    for (int p = 0; p < TPW; p++) {
-      const int t = warp + p * RC_WARPS;
-      if (s0 + t >= seqlen) break;
-      float fq[4], fk[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        fq[u] = __bfloat162float(rq[p][u]);
-        fk[u] = __bfloat162float(rk[p][u]);
-      }
-      const float iq = inv_norm(fq), ik = inv_norm(fk);
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int c = lane + 32 * u;
-        r.q[t][c] = __fmul_rn(fq[u], iq);
-        r.k[t][c] = __fmul_rn(fk[u], ik);
-        r.d[t][c] = __expf(rgt[p][u]);
-      }
-#pragma unroll
-      for (int u = 0; u < NVL; u++)
-        if (lane + 32 * u < COLS) r.v[t][lane + 32 * u] = __bfloat162float(rv[p][u]);
-      if (lane == 0) r.beta[t] = __bfloat162float(rbeta[p]);
-    }
+    ahead.fetch(s0, seqlen, warp, lane, tok, row, (size_t)k_head * 128, (size_t)(Hk + k_head) * 128, (size_t)2 * Hk * 128 + (size_t)head * 128 + v0, gp, bp,
+                Hv);
   };
   fetch(0);
   // rows 4 (rg + 16 j) + e of the lane's columns, packed by row pairs
-  auto ld_cols = [&](int r, float (&x)[CPL]) {
-    const float* p = sp + (size_t)r * 128;
-    if constexpr (CPL == 4) {
-      const float4 v = *reinterpret_cast<const float4*>(p);
-      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-    } else if constexpr (CPL == 2) {
-      const float2 v = *reinterpret_cast<const float2*>(p);
-      x[0] = v.x; x[1] = v.y;
-    } else {
-      x[0] = p[0];
-    }
-  };
-  auto st_cols = [&](int r, const float (&x)[CPL]) {
-    float* p = sp + (size_t)r * 128;
-    if constexpr (CPL == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
-    else if constexpr (CPL == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
-    else p[0] = x[0];
-  };
   uint64_t S[CPL][4];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int r0 = 4 * (rg + 16 * (i >> 1)) + 2 * (i & 1);
     float x0[CPL], x1[CPL];
-    ld_cols(r0, x0);
-    ld_cols(r0 + 1, x1);
+    ld_cols(sp + (size_t)r0 * 128, x0);
+    ld_cols(sp + (size_t)(r0 + 1) * 128, x1);
 #pragma unroll
     for (int c = 0; c < CPL; c++) S[c][i] = pack2(x0[c], x1[c]);
   }
-  prepare(rb[0], 0);
+  ahead.prepare(rb[0], 0, seqlen, warp, lane);
   __syncthreads();
   int buf = 0;
   for (int s0 = 0; s0 < seqlen; s0 += RC_TB, buf ^= 1) {
@@ -905,18 +924,18 @@ __global__ __launch_bounds__(RC_WARPS * 32) void kda_recurrent_cols_kernel(
       float ov[4 * CPL];                                 // group sums of the outputs of four tokens
 #pragma unroll
       for (int tt = 0; tt < 4; tt++) token(t + tt, ops, ov + tt * CPL);
-      const float o = lane_sums<4 * CPL>(ov, lane);
-      const int idx = sum_index<4 * CPL>(lane);          // value (token t + idx / CPL, column col + idx % CPL)
-      if (sum_owner<4 * CPL>(lane)) s_o[buf][t + idx / CPL][col + idx % CPL] = o;
+      const float o = lane_sums<4 * CPL, 16>(ov, lane);
+      const int idx = sum_index<4 * CPL, 16>(lane);          // value (token t + idx / CPL, column col + idx % CPL)
+      if (sum_owner<4 * CPL, 16>(lane)) s_o[buf][t + idx / CPL][col + idx % CPL] = o;
     }
 #pragma unroll 1
     for (; t < n; t++) {
       float ov[CPL];
       token(t, ops, ov);
-      const float o = lane_sums<CPL>(ov, lane);
-      if (sum_owner<CPL>(lane)) s_o[buf][t][col + sum_index<CPL>(lane)] = o;
+      const float o = lane_sums<CPL, 16>(ov, lane);
+      if (sum_owner<CPL, 16>(lane)) s_o[buf][t][col + sum_index<CPL, 16>(lane)] = o;
     }
-    prepare(rb[buf ^ 1], s0 + RC_TB);
+    ahead.prepare(rb[buf ^ 1], s0 + RC_TB, seqlen, warp, lane);
     __syncthreads();
     for (int i = tid; i < n * COLS; i += RC_WARPS * 32) {
       const float tot = s_o[buf][i / COLS][i % COLS] * scale;
@@ -931,8 +950,191 @@ __global__ __launch_bounds__(RC_WARPS * 32) void kda_recurrent_cols_kernel(
     float x0[CPL], x1[CPL];
 #pragma unroll
     for (int c = 0; c < CPL; c++) unpack2(S[c][i], x0[c], x1[c]);
-    st_cols(r0, x0);
-    st_cols(r0 + 1, x1);
+    st_cols(sp + (size_t)r0 * 128, x0);
+    st_cols(sp + (size_t)(r0 + 1) * 128, x1);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same for few chains, a CTA to an SM at most.  What bounds it is a warp's chain from token to token: nothing else is there to fill an SM's
+// slots.  So the CTA has a second half that takes everything off the chain that does not depend on the state (a batch of tokens prepared
+// ahead, the outputs of the batch before written), handed over with named barriers; and a warp walks two halves of its columns, the
+// second half a token behind by half: while the row sums of one are in their shuffles, the other has its products (both in one
+// instruction stream, with two sets of operands that take turns).  L lanes share a column: with 8 a lane has two row groups (rg and
+// rg + 8: the first of the four sums is a local one).  Plain fp32: in one warp the packed form measured 87-107 cycles for 64 products, this one
+// 82.  37 tokens x 64 chains 18.8 -> 16.1 us, x 32 16.5 -> 11.4, x 16 13.9 -> 9.5; without the halves 16.7 / 11.8 / 9.9.
+// ---------------------------------------------------------------------------------------------
+enum { RC_FULL = 1, RC_DONE = 3 };          // named barriers of the two batches: prepared; walked through
+__device__ __forceinline__ void rc_sync(int bar) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(2 * RC_WARPS * 32) : "memory"); }
+__device__ __forceinline__ void rc_arrive(int bar) { asm volatile("bar.arrive %0, %1;" ::"r"(bar), "n"(2 * RC_WARPS * 32) : "memory"); }
+
+template <int CPL, int L>
+__global__ __launch_bounds__(2 * RC_WARPS * 32, 1) void kda_recurrent_few_kernel(
+    const __nv_bfloat16* __restrict__ mixed_qkv, const float* __restrict__ g, const __nv_bfloat16* __restrict__ beta,
+    float* __restrict__ state, __nv_bfloat16* __restrict__ out, float* __restrict__ out_f32, int seqlen, int Hk, int Hv, float scale,
+    const int* __restrict__ slots) {
+  constexpr int COLS = RC_WARPS * (32 / L) * CPL, ROWS = 128 / L;       // columns of the CTA, rows of a lane
+  __shared__ RecBatch<COLS> rb[2];
+  __shared__ __align__(16) float s_o[2][RC_TB][COLS];
+  const int b = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * COLS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & (RC_WARPS - 1);
+  pdl_wait();
+  if (tid >= RC_WARPS * 32) {
+    const int k_head = head / (Hv / Hk), n_batches = (seqlen + RC_TB - 1) / RC_TB;
+    const size_t row = (size_t)2 * Hk * 128 + (size_t)Hv * 128;
+    RecTokens<COLS> ahead;
+    auto fetch = [&](int s0) {
+      ahead.fetch(s0, seqlen, warp, lane, mixed_qkv + (size_t)b * seqlen * row, row, (size_t)k_head * 128, (size_t)(Hk + k_head) * 128,
+                  (size_t)2 * Hk * 128 + (size_t)head * 128 + v0, g + ((size_t)b * seqlen * Hv + head) * 128, beta + (size_t)b * seqlen * Hv + head, Hv);
+    };
+    fetch(0);
+    for (int j = 0; j < n_batches + 2; j++) {             // batch j prepared, batch j - 2 written out
+      const int buf = j & 1;
+      if (j >= 2) {
+        rc_sync(RC_DONE + buf);
+        const int s0 = (j - 2) * RC_TB, n = min(RC_TB, seqlen - s0);
+        for (int i = tid - RC_WARPS * 32; i < n * COLS; i += RC_WARPS * 32) {
+          const float tot = s_o[buf][i / COLS][i % COLS] * scale;
+          const size_t oi = (((size_t)b * seqlen + s0 + i / COLS) * Hv + head) * 128 + v0 + i % COLS;
+          out[oi] = __float2bfloat16_rz(tot);
+          if (out_f32) out_f32[oi] = tot;
+        }
+      }
+      if (j < n_batches) {
+        ahead.prepare(rb[buf], j * RC_TB, seqlen, warp, lane);
+        rc_arrive(RC_FULL + buf);
+        if (j + 1 < n_batches) fetch((j + 1) * RC_TB);
+      }
+    }
+    return;
+  }
+  const int rg = lane & (L - 1), col = (warp * (32 / L) + lane / L) * CPL;   // row groups from rg on; first column of this lane
+  float* sp = state + ((size_t)(slots ? slots[b] : b) * Hv + head) * 128 * 128 + v0 + col;
+  // row i of the lane: of group rg (i < 8) or rg + 8, of its first or second chunk of four
+  auto row_of = [&](int i) { return 4 * (rg + 8 * (i >> 3) + 16 * ((i >> 2) & 1)) + (i & 3); };
+  float S[CPL][ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; i++) {
+    float x[CPL];
+    ld_cols(sp + (size_t)row_of(i) * 128, x);
+#pragma unroll
+    for (int c = 0; c < CPL; c++) S[c][i] = x[c];
+  }
+  struct Operands {
+    float k[ROWS], d[ROWS], q[ROWS], v[CPL], be;
+  };
+  auto operands = [&](int s, Operands& o) {
+    const RecBatch<COLS>& r = rb[(s / RC_TB) & 1];
+    const int t = s % RC_TB;
+    auto pieces = [&](const float (*p)[128], float (&x)[ROWS]) {
+#pragma unroll
+      for (int j = 0; j < ROWS / 4; j++) {
+        const float4 w = *reinterpret_cast<const float4*>(&p[t][row_of(4 * j)]);
+        x[4 * j] = w.x; x[4 * j + 1] = w.y; x[4 * j + 2] = w.z; x[4 * j + 3] = w.w;
+      }
+    };
+    pieces(r.d, o.d);
+    pieces(r.k, o.k);
+    pieces(r.q, o.q);
+    o.be = r.beta[t];
+#pragma unroll
+    for (int c = 0; c < CPL; c++) o.v[c] = r.v[t][col + c];
+  };
+  // sums over the lane's rows of half f of the columns: even and odd rows of a group by themselves
+  constexpr int HC = CPL / 2;
+  auto group_sum = [&](int f, const float (&x)[ROWS], float (&y)[HC]) {
+    constexpr int P = ROWS / 4;
+    float acc[HC][P];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int c = 0; c < HC; c++)
+#pragma unroll
+        for (int h = 0; h < P; h++) {
+          const int r = 8 * (h >> 1) + 2 * i + (h & 1);
+          acc[c][h] = __fmaf_rn(x[r], S[f * HC + c][r], i ? acc[c][h] : 0.f);
+        }
+#pragma unroll
+    for (int c = 0; c < HC; c++) {
+      y[c] = __fadd_rn(acc[c][0], acc[c][1]);
+      if (P == 4) y[c] = __fadd_rn(y[c], __fadd_rn(acc[c][P - 2], acc[c][P - 1]));
+    }
+  };
+  auto decay = [&](int f, const Operands& o, float (&y)[HC]) {           // S <- d S; the lane's part of k S
+#pragma unroll
+    for (int c = 0; c < HC; c++)
+#pragma unroll
+      for (int i = 0; i < ROWS; i++) S[f * HC + c][i] = __fmul_rn(S[f * HC + c][i], o.d[i]);
+    group_sum(f, o.k, y);
+  };
+  auto across = [&](float (&y)[HC]) {                                     // summed over the lanes
+#pragma unroll
+    for (int st = 0; (1 << st) < L; st++)
+#pragma unroll
+      for (int c = 0; c < HC; c++) y[c] = __fadd_rn(y[c], __shfl_xor_sync(0xffffffffu, y[c], sum_mask<L>(st)));
+  };
+  auto update = [&](int f, const Operands& o, const float (&y)[HC], float (&ov)[HC]) {   // S <- S + k u; the lane's part of q S
+#pragma unroll
+    for (int c = 0; c < HC; c++) {
+      const float un = __fmul_rn(__fsub_rn(o.v[f * HC + c], y[c]), o.be);
+#pragma unroll
+      for (int i = 0; i < ROWS; i++) S[f * HC + c][i] = __fmaf_rn(o.k[i], un, S[f * HC + c][i]);
+    }
+    group_sum(f, o.q, ov);
+  };
+  float ya[HC], yb[HC], oa[HC];                            // half 0 runs half a token ahead of half 1
+  auto emit = [&](int s, const float (&ob)[HC]) {          // output sums of token s
+    float ov[CPL];
+#pragma unroll
+    for (int c = 0; c < HC; c++) {
+      ov[c] = oa[c];
+      ov[HC + c] = ob[c];
+    }
+    const float o = lane_sums<CPL, L>(ov, lane);
+    if (sum_owner<CPL, L>(lane)) s_o[(s / RC_TB) & 1][s % RC_TB][col + sum_index<CPL, L>(lane)] = o;
+    if (s % RC_TB == RC_TB - 1 || s == seqlen - 1) rc_arrive(RC_DONE + ((s / RC_TB) & 1));
+  };
+  auto step = [&](int s, Operands& now, Operands& before) {   // on return `before` holds token s + 1
+    decay(0, now, ya);
+    across(ya);
+    float ob[HC];
+    update(1, before, yb, ob);
+    if ((s + 1) % RC_TB == 0 && s + 1 < seqlen) rc_sync(RC_FULL + (((s + 1) / RC_TB) & 1));
+    operands(min(s + 1, seqlen - 1), before);
+    decay(1, now, yb);
+    emit(s - 1, ob);
+    across(yb);
+    update(0, now, ya, oa);
+  };
+  Operands o0, o1;
+  rc_sync(RC_FULL);
+  operands(0, o0);
+  decay(0, o0, ya);
+  across(ya);
+  operands(min(1, seqlen - 1), o1);
+  decay(1, o0, yb);
+  across(yb);
+  update(0, o0, ya, oa);
+  int s = 1;
+#pragma unroll 1
+  for (; s + 2 <= seqlen; s += 2) {
+    step(s, o1, o0);
+    step(s + 1, o0, o1);
+  }
+  float ob[HC];
+  if (s < seqlen) {
+    step(s, o1, o0);
+    update(1, o1, yb, ob);
+  } else {
+    update(1, o0, yb, ob);
+  }
+  emit(seqlen - 1, ob);
+#pragma unroll
+  for (int i = 0; i < ROWS; i++) {
+    float x[CPL];
+#pragma unroll
+    for (int c = 0; c < CPL; c++) x[c] = S[c][i];
+    st_cols(sp + (size_t)row_of(i) * 128, x);
   }
 }
 
@@ -1000,10 +1202,23 @@ HK_API int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* b
     // 512 chains 12 tokens 46.8 / 46.9, 16 tokens 58.8 / 55.0; 1,536 chains 16 tokens 152 / 158, 24 tokens 220 / 210.
     const int rows_up_to = chains >= 1024 ? 16 : (chains >= 384 ? 12 : (chains >= 128 ? 6 : (chains >= 16 ? 3 : 1)));
     if (seqlen > rows_up_to) {
-      const int cpl = !aligned(state, 16) || chains < 32 ? 1 : (chains < 64 ? 2 : 4);
-      auto kern = cpl == 4 ? kda_recurrent_cols_kernel<4> : (cpl == 2 ? kda_recurrent_cols_kernel<2> : kda_recurrent_cols_kernel<1>);
-      return pdl_launch(kern, dim3(bsz, num_v_heads, 16 / cpl), dim3(RC_WARPS * 32), 0, s, q, g, bt, state, o, out_f32, seqlen, num_k_heads,
-                        num_v_heads, 1.0f / sqrtf(128.0f), slots) == cudaSuccess
+      // As many CTAs to a chain as fit with one on an SM, 8 / 4 / 2: 18, 37 or 74 chains on 148 SMs.  The columns kernel / this one, us:
+      // 8 chains 12 tokens 5.2 / 5.1 (8 tokens 4.4 / 4.7), 16 tokens 6.1 / 6.1, 37 tokens 11.5 / 9.4; 16 chains 8 tokens 5.2 / 4.9, 37 tokens
+      // 13.9 / 9.5; 32 chains 4 tokens 5.5 / 4.9, 37 tokens 16.5 / 11.4, 63 tokens 25.0 / 17.3; 64 chains 4 tokens 5.6 / 5.8, 8 tokens 7.1 /
+      // 7.2, 13 tokens 9.3 / 8.4, 37 tokens 18.8 / 16.1, 63 tokens 29.4 / 24.3.  More chains stay with the columns kernel, whose smaller CTAs
+      // share an SM (this one with two CTAs a chain, 96 chains: 24.9 / 30.4, 256: 53.0 / 60.0), and states off the 16-byte boundary too.
+      const int per_chain = (int)std::min<int64_t>(sm_count() / chains, 8);
+      const int more_than = per_chain < 4 ? 8 : (chains <= sm_count() / 16 ? 12 : 0);
+      if (aligned(state, 16) && per_chain >= 2 && seqlen > more_than) {
+        auto kern = per_chain == 8 ? kda_recurrent_few_kernel<2, 16> : (per_chain >= 4 ? kda_recurrent_few_kernel<4, 16> : kda_recurrent_few_kernel<4, 8>);
+        return pdl_launch(kern, dim3(bsz, num_v_heads, per_chain == 8 ? 8 : (per_chain >= 4 ? 4 : 2)), dim3(2 * RC_WARPS * 32), 0, s, q, g, bt, state, o,
+                          out_f32, seqlen, num_k_heads, num_v_heads, 1.0f / sqrtf(128.0f), slots) == cudaSuccess
+                   ? HK_OK
+                   : HK_ERR_CUDA;
+      }
+      const bool one = !aligned(state, 16) || chains < 16;
+      return pdl_launch(one ? kda_recurrent_cols_kernel<1> : kda_recurrent_cols_kernel<4>, dim3(bsz, num_v_heads, one ? 16 : 4), dim3(RC_WARPS * 32), 0, s, q,
+                        g, bt, state, o, out_f32, seqlen, num_k_heads, num_v_heads, 1.0f / sqrtf(128.0f), slots) == cudaSuccess
                  ? HK_OK
                  : HK_ERR_CUDA;
     }

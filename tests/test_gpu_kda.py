@@ -563,6 +563,31 @@ def test_decode_layer_vs_oracle(H, bsz):
     assert max_rel(y.cpu().numpy(), y64) < 1e-5
 
 
+@pytest.mark.parametrize("Hk,Hv,bsz", [(8, 8, 1), (2, 18, 1), (19, 19, 1), (37, 37, 1), (19, 19, 2), (37, 74, 1)])
+@pytest.mark.parametrize("T", [2, 9, 13, 16, 17, 63])
+def test_few_chains_walk_to_the_same_bits(T, Hk, Hv, bsz):
+    """eight, four and two CTAs a chain, either side of the batches of eight tokens and of the head counts where the split changes, a
+    state of zeros among them, against the kernel that states off the 16-byte boundary take: same bits"""
+    D = 128
+    gen = torch.Generator(device="cuda").manual_seed(100 * T + Hv)
+    qkv = torch.randn(bsz, T, (2 * Hk + Hv) * D, generator=gen, device="cuda").to(torch.bfloat16)
+    qkv[:, ::3, :7] = 0
+    g, beta = -5 * torch.rand(bsz, T, Hv, D, generator=gen, device="cuda"), torch.rand(bsz, T, Hv, generator=gen, device="cuda").to(torch.bfloat16)
+    s0 = 0.1 * torch.randn(bsz, 1, Hv, D, D, generator=gen, device="cuda")
+    s0[:, :, 0] = 0
+    slots = torch.arange(bsz - 1, -1, -1, dtype=torch.int32, device="cuda")
+    res = []
+    for off in (0, 1):
+        st = torch.empty(s0.numel() + 4, device="cuda")[off:off + s0.numel()].view(s0.shape)
+        st.copy_(s0)
+        out, o32 = torch.empty(bsz, T, Hv, D, dtype=torch.bfloat16, device="cuda"), torch.empty(bsz, T, Hv, D, device="cuda")
+        hk.cuda_recurrent_gated_delta_rule(qkv, g, beta, st, out, bsz, T, Hk, Hv, D, D, 1, slots, True, False, out_f32=o32, force_recurrent=True)
+        torch.cuda.synchronize()
+        res.append([bits(out), o32.cpu().numpy().view(np.int32), st.cpu().numpy().view(np.int32)])
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("H,bsz", [(4, 1), (40, 2), (64, 5)])
 def test_states_off_the_16_byte_boundary(H, bsz):
     """a state that starts on any fp32 element: the scalar forms (decode step and layer; 1, 3 and 9 tokens of the recurrence; no
