@@ -15,8 +15,9 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 // src [S][F] fp32 -> dst [F][S] bf16 (round to nearest even).  One CTA moves a tile of 4,096 elements.  HBM-bound (6 B per
 // element): 64 tokens x 64 channels, rows of 256 B in and 128 B out, 6.5 TB/s at 32,768 tokens.
-// LONG, odd lengths from 32 on: 128 tokens x 32 channels.  The rows start inside a sector, so a tile row ends in two partly written ones:
-// twice as long rows halve them (458 -> 430 us at 32,763 tokens, 6.5 -> 4.4 at 301 x 3,072 channels; 368 -> 399 at 32,768).
+// LONG, odd lengths above 192: 128 tokens x 32 channels.  The rows start inside a sector, so a tile row ends in two partly written ones:
+// twice as long rows halve them (458 -> 430 us at 32,763 tokens; 368 -> 399 at 32,768).  Below, the tile's idle rows cost more: 64- / 128-token
+// tiles, 24,576 channels, us: 37 tokens 2.5 / 3.9, 63 2.7 / 3.9, 101 4.1 / 4.3, 129 5.4 / 6.7, 191 5.6 / 6.8, 255 7.5 / 7.1, 501 12.3 / 12.0.
 // 4-byte stores from the first even element of a row on.  ODD without LONG: 2-byte stores (3 tokens x 12,288 channels 1.9 us, 2.8 the other way).
 // ---------------------------------------------------------------------------------------------
 template <bool LONG, bool ODD>
@@ -278,7 +279,7 @@ int launch_gated_rms_norm(const void* x, const void* w, void* y, const void* g, 
 HK_API int hk_kda_transpose_cast(void* dst_bf16, const float* src, int S, int F, void* stream) {
   HK_REQUIRE(dst_bf16 && src && S >= 0 && F >= 0);
   if (S == 0 || F == 0) return HK_OK;
-  const bool odd = S % 2 != 0, longer = odd && S >= 32;
+  const bool odd = S % 2 != 0, longer = odd && S > 192;
   const int s_tiles = (S - 1) / (longer ? 128 : 64) + 1;
   HK_REQUIRE(s_tiles <= 65535);
   HK_REQUIRE(hk::aligned(dst_bf16, 4));
