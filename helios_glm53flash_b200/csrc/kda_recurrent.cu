@@ -961,8 +961,9 @@ __global__ __launch_bounds__(RC_WARPS * 32) void kda_recurrent_cols_kernel(
 // ahead, the outputs of the batch before written), handed over with named barriers; and a warp walks two halves of its columns, the
 // second half a token behind by half: while the row sums of one are in their shuffles, the other has its products (both in one
 // instruction stream, with two sets of operands that take turns).  L lanes share a column: with 8 a lane has two row groups (rg and
-// rg + 8: the first of the four sums is a local one).  Plain fp32: in one warp the packed form measured 87-107 cycles for 64 products, this one
-// 82.  37 tokens x 64 chains 18.8 -> 16.1 us, x 32 16.5 -> 11.4, x 16 13.9 -> 9.5; without the halves 16.7 / 11.8 / 9.9.
+// rg + 8: the first of the four sums is a local one).  Sums in plain fp32: with one warp on a scheduler the packed form measured 107 cycles
+// for 64 products of a sum, this one 82; updates packed (96, but half the issue slots), and the decay where a warp has 16 columns or 8 (two
+// columns a lane: 2-4 % slower).  37 tokens x 64 chains 18.8 -> 15.8 us, x 32 16.5 -> 11.1, x 16 13.9 -> 9.5; without the halves 16.7 / 11.8 / 9.9.
 // ---------------------------------------------------------------------------------------------
 enum { RC_FULL = 1, RC_DONE = 3 };          // named barriers of the two batches: prepared; walked through
 __device__ __forceinline__ void rc_sync(int bar) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(2 * RC_WARPS * 32) : "memory"); }
@@ -1064,7 +1065,15 @@ __global__ __launch_bounds__(2 * RC_WARPS * 32, 1) void kda_recurrent_few_kernel
 #pragma unroll
     for (int c = 0; c < HC; c++)
 #pragma unroll
-      for (int i = 0; i < ROWS; i++) S[f * HC + c][i] = __fmul_rn(S[f * HC + c][i], o.d[i]);
+      for (int i = 0; i < ROWS; i += 2) {
+        float &a = S[f * HC + c][i], &b = S[f * HC + c][i + 1];
+        if (CPL == 4) {
+          unpack2(mul2(pack2(a, b), pack2(o.d[i], o.d[i + 1])), a, b);
+        } else {
+          a = __fmul_rn(a, o.d[i]);
+          b = __fmul_rn(b, o.d[i + 1]);
+        }
+      }
     group_sum(f, o.k, y);
   };
   auto across = [&](float (&y)[HC]) {                                     // summed over the lanes
@@ -1078,7 +1087,10 @@ __global__ __launch_bounds__(2 * RC_WARPS * 32, 1) void kda_recurrent_few_kernel
     for (int c = 0; c < HC; c++) {
       const float un = __fmul_rn(__fsub_rn(o.v[f * HC + c], y[c]), o.be);
 #pragma unroll
-      for (int i = 0; i < ROWS; i++) S[f * HC + c][i] = __fmaf_rn(o.k[i], un, S[f * HC + c][i]);
+      for (int i = 0; i < ROWS; i += 2) {
+        float &a = S[f * HC + c][i], &b = S[f * HC + c][i + 1];
+        unpack2(fma2(pack2(o.k[i], o.k[i + 1]), pack2(un, un), pack2(a, b)), a, b);
+      }
     }
     group_sum(f, o.q, ov);
   };
@@ -1204,8 +1216,8 @@ HK_API int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* b
     if (seqlen > rows_up_to) {
       // As many CTAs to a chain as fit with one on an SM, 8 / 4 / 2: 18, 37 or 74 chains on 148 SMs.  The columns kernel / this one, us:
       // 8 chains 12 tokens 5.2 / 5.1 (8 tokens 4.4 / 4.7), 16 tokens 6.1 / 6.1, 37 tokens 11.5 / 9.4; 16 chains 8 tokens 5.2 / 4.9, 37 tokens
-      // 13.9 / 9.5; 32 chains 4 tokens 5.5 / 4.9, 37 tokens 16.5 / 11.4, 63 tokens 25.0 / 17.3; 64 chains 4 tokens 5.6 / 5.8, 8 tokens 7.1 /
-      // 7.2, 13 tokens 9.3 / 8.4, 37 tokens 18.8 / 16.1, 63 tokens 29.4 / 24.3.  More chains stay with the columns kernel, whose smaller CTAs
+      // 13.9 / 9.5; 32 chains 4 tokens 5.5 / 4.9, 37 tokens 16.5 / 11.1, 63 tokens 25.0 / 16.5; 64 chains 4 tokens 5.6 / 5.8, 8 tokens 7.1 /
+      // 7.2, 13 tokens 9.3 / 8.4, 37 tokens 18.8 / 15.8, 63 tokens 29.4 / 23.7.  More chains stay with the columns kernel, whose smaller CTAs
       // share an SM (this one with two CTAs a chain, 96 chains: 24.9 / 30.4, 256: 53.0 / 60.0), and states off the 16-byte boundary too.
       const int per_chain = (int)std::min<int64_t>(sm_count() / chains, 8);
       const int more_than = per_chain < 4 ? 8 : (chains <= sm_count() / 16 ? 12 : 0);
