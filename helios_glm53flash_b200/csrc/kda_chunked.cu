@@ -1,7 +1,7 @@
 // Chunked KDA prefill (gated delta rule with channelwise decay), chunk = 64 tokens, dk = dv = 128.
 // The reference has no chunked kernel: its prefill runs the per-token recurrence with seqlen = n
 // (src/engine/runner.cpp:468-471 -> src/cuda/aux/gdn.cu:555-749).  This file computes the same
-// function in two kernels.
+// function: one persistent launch, or two kernels.
 //
 // Math, per head, for a chunk with incoming state S0 [128 k][128 v] (q^, k^ = L2-normalised rows,
 // G_t = inclusive cumulative log-decay inside the chunk, all exponentials below have arguments <= 0
@@ -21,7 +21,8 @@
 //   What bounds it: latencies.  A unit crosses five barriers of its 256 threads and one product; two units share an SM (128 registers
 //   a thread, 109 KB).  Inputs arrive by tensor copies issued while the unit before is finished.  A worker's unit takes 22-24 thousand
 //   cycles with two workers on the SM, 39 thousand in the form before (k and q rows in separate warps, TF32 for all block pairs,
-//   13 barriers, loads through registers); 32,768 tokens x 32 heads 1.43 -> 1.02 ms, chain-bound, with gates formed inside 1.62 -> 1.09.
+//   13 barriers, loads through registers); 32,768 tokens x 32 heads 1.43 -> 1.02 ms, with gates formed inside 1.62 -> 1.09 (0.90 and 0.98
+//   with the chain of today).
 //   Registers decide: everything a thread keeps across stage 2 is the 32 packed left operands; a version that kept the fp32 rows (300
 //   bytes of spills, whose reloads miss the L1 that shared memory leaves) took 30 thousand cycles.
 // The scan walks the chunks of a chain in order; the fp32 state stays in registers.  Per chunk: D1 = [I ; 0] Uloc + [-W ; Q+] S0 (rows

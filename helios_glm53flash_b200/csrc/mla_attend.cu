@@ -112,7 +112,10 @@ static int attend(MlaArgs a, int n_keys_hint, int n_split, void* workspace, size
     // ranges; where each row has a length of its own on the device, fewer splits than the GPU has room for mean two tiles each.
     const int tiles = a.raw_idx || !a.kv_len ? (n_keys_hint + 63) / 64 : (int64_t)a.m * (n_split + 1) <= sm_count() ? 2 * n_split : 1 << 20;
     MlaArgs c = a;
-    if (tc && mla_flash_cluster_shape(a.m, tiles, &c.n_split, &c.n_cs)) {
+    // Only where the number of splits is the automatic one: with another, the splits stay CTAs of their own, 17 instead of 64 for a
+    // decode step's rows, which is what several such calls side by side want (a step of 11 layers at 5,000 tokens, us, clusters / own:
+    // 1 sequence 285 / 309, 2 on streams 374 / 359, 3 416 / 414, 4 497 / 447, 8 888 / 666).
+    if (tc && n_split == mla_flash_tc_auto_splits(a.m, n_keys_hint) && mla_flash_cluster_shape(a.m, tiles, &c.n_split, &c.n_cs)) {
       const int st = mla_flash_tc_launch(c, s);
       if (st != HK_ERR_UNSUPPORTED) return st;
     }

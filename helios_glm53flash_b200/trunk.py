@@ -179,7 +179,7 @@ class TrunkAttention:
         step can run side by side (their caches are separate; the shared work buffers of a chunk are not)"""
         if self._dec is None:
             t, hk = self.torch, self.hk
-            ns = hk.mla_auto_splits(1, KIDX)
+            ns = hk.mla_auto_splits(1, KIDX) + 1
             self._dec = [SimpleNamespace(
                 idx_kn=t.empty(1, 128, dtype=t.float16, device="cuda"), q_lat=t.empty(1, 64, 512, dtype=t.float16, device="cuda"),
                 qpos=t.empty(1, dtype=t.int32, device="cuda"), scores=t.empty(1, self.scores.shape[1], dtype=t.float16, device="cuda"),
@@ -231,7 +231,8 @@ class TrunkAttention:
             hk.pool_expand_row(wb.topk[off:off + rows], wb.qpos[off:off + rows], wb.raw_idx[off:off + rows], rows)
         if timed:
             self._mark("mla_expand")
-        ns = hk.mla_auto_splits(n, KIDX)
+        # side by side on streams: a number of its own keeps the splits out of the cluster form, which takes 64 SMs a row
+        ns = hk.mla_auto_splits(n, KIDX) + (bufs is not None)
         need = hk.mla_partial_bytes(ns, n * 64) if ns > 1 else 0
         if need > wb.sparse_ws.numel():
             wb.sparse_ws = t.empty(need, dtype=t.uint8, device="cuda")

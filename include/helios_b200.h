@@ -105,10 +105,11 @@ int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_wei
  * Requires dk = dv = 128, Hk == Hv.  seqlen may be any positive length (a ragged tail shorter
  * than a chunk is processed by the same kernels).  `workspace` must hold at least
  * hk_kda_chunked_workspace_bytes(bsz, seqlen, num_heads) bytes, 256-byte aligned.
- * Two forms.  ONE persistent cooperative launch when the chains fit its chain CTAs (at most 48 chains: a chain per SM;
- * more chains when a number of chain CTAs in [16, 48] divides their count, e.g. 64 heads or 8 x 32: a chain CTA then
- * walks several chains one after the other); the other SMs prepare the chunks and hand them over through a ring of 16
- * chunk slots per chain CTA (workspace = chain CTAs * 16 * 74,240 B + flags, independent of seqlen; it stays in L2).
+ * Two forms.  ONE persistent cooperative launch when the chains fit its chain slots (at most 48 chains, or more when a
+ * number of slots in [16, 48] divides their count, e.g. 64 heads or 8 x 32: a slot then walks several chains one after
+ * the other, with one CTA of 128 value columns or two of 64); the other SMs prepare the chunks and hand them over through
+ * a ring of 16 chunk slots per chain slot (workspace = slots * 16 * 74,240 B + flags, independent of seqlen; it stays in
+ * L2).  For few long chains the query asks for a ring of 32; half its units are enough for the call.
  * Other calls run as two kernels with one 74,240-byte workspace unit per (batch, head, chunk); short calls (all units fit the
  * ring's memory, up to 16 chunks per chain) run as two kernels in it.
  * hk_kda_chunked_set_form(1) selects the two-kernel form for every later call and workspace query of this
@@ -243,7 +244,9 @@ int hk_mla_auto_splits(int m, int n_keys);
  *   q_lat [m][n_heads][512] f16, ckv [ckv_rows][512] f16, lat_out [m][n_heads][512] f16.
  * ckv_rows: rows the cache buffer holds; row numbers at or beyond it are treated as holes instead of being read
  * (0 = not told, as in the reference's signature: every non-negative row number is read).
- * n_split = 0 lets the library choose; workspace may be NULL when the choice is 1.             */
+ * n_split = 0 lets the library choose; workspace may be NULL when the choice is 1.  One row of up to 2,112 keys with that
+ * choice runs as clusters on 64 SMs; several such calls side by side on streams are faster with another number (the choice
+ * and one), which leaves the splits single CTAs.                                               */
 int hk_mla_sparse(const void* q_lat, const void* ckv, int64_t ckv_rows, const int* raw_idx, int kidx, void* lat_out,
                   int m, int n_heads, float scale, int n_split, void* workspace,
                   size_t workspace_bytes, void* stream);

@@ -67,6 +67,21 @@ def test_one_row_merged_in_a_cluster(kidx):
         assert max_rel(g, o32) < TOL and sum_rel(g, o32) < 3e-3
 
 
+@pytest.mark.parametrize("kidx", [130, 2052])
+def test_a_split_number_of_its_own_keeps_partials_in_memory(kidx):
+    """one row: one split more than the automatic number (the last one empty), and half of it, against the oracle"""
+    inp, ridx = _sparse_case(1, kidx, 4096, 0.0625, seed=kidx + 1)
+    q, c = dev_f16(inp["q_lat"]), dev_f16(inp["ckv"])
+    _, o32 = orc.mla_attend(inp["q_lat"], inp["ckv"], 1, 64, 0.0625, raw_idx=ridx, kidx=kidx)
+    auto = hk.mla_auto_splits(1, kidx)
+    for ns in (auto + 1, (auto + 1) // 2):
+        out = torch.empty(1, 64, 512, dtype=torch.float16, device="cuda")
+        hk.mla_sparse_decode(q, c, dev(ridx), kidx, out, 1, n_split=ns)
+        torch.cuda.synchronize()
+        g = synth.f16_bits_to_f32(bits(out))
+        assert max_rel(g, o32) < TOL and sum_rel(g, o32) < 3e-3
+
+
 def test_sparse_all_skipped_row_gives_zeros_and_duplicates_count_twice():
     m, kidx, T = 2, 16, 64
     inp, ridx = _sparse_case(m, kidx, T, 0.0625, seed=1, holes=False)
