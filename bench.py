@@ -360,7 +360,7 @@ def build_kernel_case(name):
         wsb = torch.empty(max(256, hk.mla_partial_bytes(ns, 64)), dtype=torch.uint8, device="cuda")
 
         def fn():
-            hk.mla_sparse_decode(ql, ck, raw, 2052, lo, 1, n_split=ns, workspace=wsb)
+            hk.mla_sparse_decode(ql, ck, raw, 2052, lo, 1, workspace=wsb)
         return fn, 2052 * 1024, True, "sparse MLA decode, 2052 gathered latents of 262144, %d splits" % ns
     if name in ("sparse_prefill_4096", "sparse_prefill_1024"):
         # the trunk's largest prefill stage: every row of a chunk attends its own 2,052 gathered rows of a 32,768-row
@@ -375,7 +375,7 @@ def build_kernel_case(name):
         wsb = torch.empty(max(256, hk.mla_partial_bytes(ns, m * 64)), dtype=torch.uint8, device="cuda")
 
         def fn():
-            hk.mla_sparse_decode(ql, ck, raw, 2052, lo, m, n_split=ns, workspace=wsb)
+            hk.mla_sparse_decode(ql, ck, raw, 2052, lo, m, workspace=wsb)
         return fn, m * 2052 * 1024, False, "sparse MLA prefill, %d rows x 2052 gathered latents of 32768, %d split(s), %.1f GFLOP" % (
             m, ns, m * 2052 * 4 * 64 * 512 / 1e9)
     raise SystemExit("unknown case " + name)
@@ -1067,7 +1067,7 @@ def multi_gpu_measurements(hk, synth, torch, dist, np, rank, local_rank, world, 
                 hk.indexer_score(q_idx, pool_f, w_idx, q_pos, sc, 1, P)
                 hk.dsa_topk(sc, P, topk, 1, P, 512, 512)
                 hk.pool_expand_row(topk, q_pos, raw, 1)
-                hk.mla_sparse_decode(q, ckv_f, raw, 2052, ref, 1, scale=scale, n_split=ns, workspace=ws1)
+                hk.mla_sparse_decode(q, ckv_f, raw, 2052, ref, 1, scale=scale, workspace=ws1)
             for _ in range(3):
                 chain()
             torch.cuda.synchronize()
@@ -1313,7 +1313,7 @@ def side_measurements(hk, synth, torch, np, gpu_index=0):
     f_topk = [lambda: hk.dsa_topk(sc, npools, idx, 1, npools, 512, 512)] * n_mla
     res["topk512_262k_us_per_layer"] = 1e3 * _time_loop(torch, f_topk, flush=flush, label="topk512_262k", gpu_index=gpu_index) / n_mla
     hk.pool_expand_row(idx, q_pos, raw, 1)
-    f_sparse = [(lambda ck=ck: hk.mla_sparse_decode(ql, ck, raw, 2052, lo, 1, n_split=ns, workspace=wsb)) for ck in ckvs]
+    f_sparse = [(lambda ck=ck: hk.mla_sparse_decode(ql, ck, raw, 2052, lo, 1, workspace=wsb)) for ck in ckvs]
     ms = _time_loop(torch, f_sparse, flush=flush, label="mla_sparse_decode_262k", gpu_index=gpu_index) / n_mla
     res["mla_sparse_decode_262k_us_per_layer"] = ms * 1e3
     res["mla_sparse_decode_262k_hbm_gbs"] = 2052 * 1024 / (ms * 1e-3) / 1e9
@@ -1322,14 +1322,14 @@ def side_measurements(hk, synth, torch, np, gpu_index=0):
         hk.indexer_score(qi, pk, w, q_pos, sc, 1, npools)
         hk.dsa_topk(sc, npools, idx, 1, npools, 512, 512)
         hk.pool_expand_row(idx, q_pos, raw, 1)
-        hk.mla_sparse_decode(ql, ck, raw, 2052, lo, 1, n_split=ns, workspace=wsb)
+        hk.mla_sparse_decode(ql, ck, raw, 2052, lo, 1, workspace=wsb)
     f_chain = [(lambda pk=pk, ck=ck: chain(pk, ck)) for pk, ck in zip(pks, ckvs)]
     res["dsa_sparse_mla_decode_262k_us_per_layer"] = 1e3 * _time_loop(torch, f_chain, flush=flush, label="dsa_sparse_mla_decode_262k",
                                                                         gpu_index=gpu_index) / n_mla
 
     def chain2(pk, ck):       # the same step with the selection in two launches (scorer, top-k with the expansion inside)
         hk.indexer_select(qi, pk, w, q_pos, sc, idx, raw, 1, npools)
-        hk.mla_sparse_decode(ql, ck, raw, 2052, lo, 1, n_split=ns, workspace=wsb)
+        hk.mla_sparse_decode(ql, ck, raw, 2052, lo, 1, workspace=wsb)
     f_chain2 = [(lambda pk=pk, ck=ck: chain2(pk, ck)) for pk, ck in zip(pks, ckvs)]
     res["dsa_sparse_mla_decode_262k_fused_selection_us_per_layer"] = 1e3 * _time_loop(
         torch, f_chain2, flush=flush, label="dsa_sparse_mla_decode_262k_fused_selection", gpu_index=gpu_index) / n_mla

@@ -381,15 +381,27 @@ def mla_partial_bytes(n_split, rows):
     return load_library().hk_mla_partial_bytes(n_split, rows)
 
 
+def _splits(n_split, m, n_heads, keys, own_keys):
+    """(number of splits for the call, for its workspace).  No number given: the call is left to choose (0) where it comes to the
+    same number by itself - it goes by `own_keys` keys and the tensor-core form of 64 heads - and may then merge one row's splits in
+    clusters."""
+    if n_split > 0:
+        return n_split, n_split
+    splits = _native.hk_mla_auto_splits(m, keys)
+    same = n_heads == 64 and (keys == own_keys or splits == _native.hk_mla_auto_splits(m, own_keys))
+    return (0 if same else splits), splits
+
+
 def mla_sparse_decode(q_lat, ckv, raw_idx, kidx, lat_out, m, stream=None, scale=0.0625, n_heads=64,
                       n_split=0, workspace=None, ckv_rows=None):
     """helios::attn::mla_sparse_decode (src/cuda/attn/attn.cuh:93-99) with explicit scale / heads; the cache's row
-    count is taken from the tensor, so row numbers beyond it are skipped instead of read."""
-    if n_split <= 0:
-        n_split = _native.hk_mla_auto_splits(m, kidx)
+    count is taken from the tensor, so row numbers beyond it are skipped instead of read.
+    n_split <= 0: the library's choice, the fastest form of a call that has the GPU to itself; calls side by side on streams of
+    their own are faster with n_split = mla_auto_splits(m, kidx), which keeps one row's splits single CTAs (hk_mla_sparse)."""
+    n_split, splits = _splits(n_split, m, n_heads, kidx, kidx)
     ws = workspace
-    if n_split > 1 and ws is None:
-        ws = _scratch(mla_partial_bytes(n_split, m * n_heads), q_lat.device, stream)
+    if splits > 1 and ws is None:
+        ws = _scratch(mla_partial_bytes(splits, m * n_heads), q_lat.device, stream)
     _run("hk_mla_sparse", q_lat, ckv, ckv if ckv_rows is None else ckv_rows, raw_idx, kidx, lat_out, m, n_heads, scale, n_split,
          ws, ws, stream)
 
@@ -406,11 +418,11 @@ def mla_dense_prefill(q_lat, ckv, lat_out, qlen, pos_start, stream=None, scale=0
                       kv_base=None, kv_len=None, n_split=0, workspace=None, n_keys_hint=None, ckv_rows=None):
     """helios::attn::mla_dense_prefill (src/cuda/attn/attn.cuh:104-108); qlen = 1 is dense decode.
     kv_base / kv_len (device int64 / int32 per row) select per-row cache ranges (batched decode)."""
-    if n_split <= 0:
-        n_split = _native.hk_mla_auto_splits(qlen, n_keys_hint if n_keys_hint else pos_start + qlen)
+    own = pos_start + qlen if kv_len is None else pos_start or 4096
+    n_split, splits = _splits(n_split, qlen, n_heads, n_keys_hint or pos_start + qlen, own)
     ws = workspace
-    if n_split > 1 and ws is None:
-        ws = _scratch(mla_partial_bytes(n_split, qlen * n_heads), q_lat.device, stream)
+    if splits > 1 and ws is None:
+        ws = _scratch(mla_partial_bytes(splits, qlen * n_heads), q_lat.device, stream)
     _run("hk_mla_dense", q_lat, ckv, ckv if ckv_rows is None else ckv_rows, kv_base, kv_len, pos_start, lat_out, qlen, n_heads,
          scale, n_split, ws, ws, stream)
 

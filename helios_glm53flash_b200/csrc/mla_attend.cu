@@ -94,8 +94,9 @@ static int combine(const float* pm, const float* pl, const float* pa, int n_spli
   return combine_launch<LSE_GROUPS>(pm, pl, pa, n_split, rows, out, s);
 }
 
-// common driver: final output, optionally through split partials in the workspace
-static int attend(MlaArgs a, int n_keys_hint, int n_split, void* workspace, size_t workspace_bytes,
+// common driver: final output, optionally through split partials in the workspace.  `choose`: the caller leaves the form to the library,
+// which may then merge one row's splits in clusters; a number of splits that the caller gives means that many CTAs a row.
+static int attend(MlaArgs a, int n_keys_hint, int n_split, bool choose, void* workspace, size_t workspace_bytes,
                   cudaStream_t s) {
   const bool tc = (a.n_heads == 64) && !force_simt();
   if (n_split <= 0)
@@ -112,10 +113,10 @@ static int attend(MlaArgs a, int n_keys_hint, int n_split, void* workspace, size
     // ranges; where each row has a length of its own on the device, fewer splits than the GPU has room for mean two tiles each.
     const int tiles = a.raw_idx || !a.kv_len ? (n_keys_hint + 63) / 64 : (int64_t)a.m * (n_split + 1) <= sm_count() ? 2 * n_split : 1 << 20;
     MlaArgs c = a;
-    // Only where the number of splits is the automatic one: with another, the splits stay CTAs of their own, 17 instead of 64 for a
-    // decode step's rows, which is what several such calls side by side want (a step of 11 layers at 5,000 tokens, us, clusters / own:
-    // 1 sequence 285 / 309, 2 on streams 374 / 359, 3 416 / 414, 4 497 / 447, 8 888 / 666).
-    if (tc && n_split == mla_flash_tc_auto_splits(a.m, n_keys_hint) && mla_flash_cluster_shape(a.m, tiles, &c.n_split, &c.n_cs)) {
+    // That is the form for a call that has the GPU to itself: its 64 SMs where the splits alone are 17 CTAs cost several calls side by
+    // side more than each gains, which the library cannot see and the caller says with a number of splits (a step of 11 MLA layers at
+    // 5,000 tokens, us, clusters / 17 CTAs: 1 sequence 275 / 296, 2 on streams 362 / 347, 3 404 / 403, 4 477 / 434, 8 866 / 650).
+    if (tc && choose && mla_flash_cluster_shape(a.m, tiles, &c.n_split, &c.n_cs)) {
       const int st = mla_flash_tc_launch(c, s);
       if (st != HK_ERR_UNSUPPORTED) return st;
     }
@@ -158,7 +159,7 @@ HK_API int hk_mla_sparse(const void* q_lat, const void* ckv, int64_t ckv_rows, c
   a.raw_idx = raw_idx; a.kidx = kidx;
   a.m = m; a.n_heads = n_heads; a.scale = scale;
   a.out = (__half*)lat_out;
-  return attend(a, kidx, n_split, workspace, workspace_bytes, as_stream(stream));
+  return attend(a, kidx, n_split, n_split <= 0, workspace, workspace_bytes, as_stream(stream));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -213,7 +214,8 @@ HK_API int hk_mla_sparse_static(const void* q_lat, const void* ckv, const int* r
   HK_REQUIRE(aligned(q_lat, 16) && aligned(ckv, 16) && aligned(lat_out, 16));
   if (m == 0) return HK_OK;
   if ((size_t)m > HK_STATIC_MAX_SLOTS) return HK_ERR_WORKSPACE;  // beyond the built-in scratch: use hk_mla_sparse
-  if (n_split <= 0) {
+  const bool choose = n_split <= 0;
+  if (choose) {
     n_split = force_simt() ? simt_auto_splits(m, 64, kidx) : mla_flash_tc_auto_splits(m, kidx);
     const int cap = (int)(HK_STATIC_MAX_SLOTS / (size_t)m);
     if (n_split > cap) n_split = cap;
@@ -227,7 +229,7 @@ HK_API int hk_mla_sparse_static(const void* q_lat, const void* ckv, const int* r
   a.raw_idx = raw_idx; a.kidx = kidx;
   a.m = m; a.n_heads = 64; a.scale = scale;
   a.out = (__half*)lat_out;
-  return attend(a, kidx, n_split, scratch, HK_STATIC_SCRATCH_BYTES, as_stream(stream));
+  return attend(a, kidx, n_split, choose, scratch, HK_STATIC_SCRATCH_BYTES, as_stream(stream));
 }
 
 HK_API int hk_mla_dense(const void* q_lat, const void* ckv, int64_t ckv_rows, const int64_t* kv_base,
@@ -248,7 +250,7 @@ HK_API int hk_mla_dense(const void* q_lat, const void* ckv, int64_t ckv_rows, co
   a.out = (__half*)lat_out;
   // without host-visible lengths the split heuristic uses the longest causal row
   const int hint = kv_len ? (pos_start > 0 ? pos_start : 4096) : pos_start + m;
-  return attend(a, hint, n_split, workspace, workspace_bytes, as_stream(stream));
+  return attend(a, hint, n_split, n_split <= 0, workspace, workspace_bytes, as_stream(stream));
 }
 
 HK_API int hk_mla_dense_partial(const void* q_lat, const void* ckv, const int64_t* kv_base,

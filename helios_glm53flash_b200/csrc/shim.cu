@@ -165,7 +165,8 @@ void mla_sparse_decode(const half* q_lat, const half* ckv, const int* raw_idx, i
   const int n_split = hk_mla_auto_splits(m, kidx);
   size_t bytes = n_split > 1 ? hk_mla_partial_bytes(n_split, (int64_t)m * N_HEADS) : 0;
   void* ws = bytes ? scratch(bytes) : nullptr;
-  check(hk_mla_sparse(q_lat, ckv, 0, raw_idx, kidx, lat_out, m, N_HEADS, SCALE, n_split, ws, bytes, s),
+  // the launchers of a GPU share one stream, so the library may choose the form of a call that has the GPU to itself
+  check(hk_mla_sparse(q_lat, ckv, 0, raw_idx, kidx, lat_out, m, N_HEADS, SCALE, 0, ws, bytes, s),
         "mla_sparse_decode");
 }
 void mla_dense_prefill(const half* q_lat, const half* ckv, half* lat_out, int qlen, int pos_start,
@@ -174,7 +175,7 @@ void mla_dense_prefill(const half* q_lat, const half* ckv, half* lat_out, int ql
   const int n_split = hk_mla_auto_splits(qlen, pos_start + qlen);
   size_t bytes = n_split > 1 ? hk_mla_partial_bytes(n_split, (int64_t)qlen * N_HEADS) : 0;
   void* ws = bytes ? scratch(bytes) : nullptr;
-  check(hk_mla_dense(q_lat, ckv, 0, nullptr, nullptr, pos_start, lat_out, qlen, N_HEADS, SCALE, n_split,
+  check(hk_mla_dense(q_lat, ckv, 0, nullptr, nullptr, pos_start, lat_out, qlen, N_HEADS, SCALE, 0,
                      ws, bytes, s),
         "mla_dense_prefill");
 }

@@ -179,7 +179,7 @@ class TrunkAttention:
         step can run side by side (their caches are separate; the shared work buffers of a chunk are not)"""
         if self._dec is None:
             t, hk = self.torch, self.hk
-            ns = hk.mla_auto_splits(1, KIDX) + 1
+            ns = hk.mla_auto_splits(1, KIDX)
             self._dec = [SimpleNamespace(
                 idx_kn=t.empty(1, 128, dtype=t.float16, device="cuda"), q_lat=t.empty(1, 64, 512, dtype=t.float16, device="cuda"),
                 qpos=t.empty(1, dtype=t.int32, device="cuda"), scores=t.empty(1, self.scores.shape[1], dtype=t.float16, device="cuda"),
@@ -231,12 +231,12 @@ class TrunkAttention:
             hk.pool_expand_row(wb.topk[off:off + rows], wb.qpos[off:off + rows], wb.raw_idx[off:off + rows], rows)
         if timed:
             self._mark("mla_expand")
-        # side by side on streams: a number of its own keeps the splits out of the cluster form, which takes 64 SMs a row
-        ns = hk.mla_auto_splits(n, KIDX) + (bufs is not None)
+        ns = hk.mla_auto_splits(n, KIDX)
         need = hk.mla_partial_bytes(ns, n * 64) if ns > 1 else 0
         if need > wb.sparse_ws.numel():
             wb.sparse_ws = t.empty(need, dtype=t.uint8, device="cuda")
-        hk.mla_sparse_decode(wb.q_lat, ckv, wb.raw_idx, KIDX, wb.lat_out, n, n_split=ns, workspace=wb.sparse_ws)
+        # side by side on streams: a number given keeps one row's splits single CTAs, clusters of them take 64 SMs a row
+        hk.mla_sparse_decode(wb.q_lat, ckv, wb.raw_idx, KIDX, wb.lat_out, n, n_split=ns if bufs else 0, workspace=wb.sparse_ws)
         if timed:
             self._mark("mla_sparse_attention")
         hk.o_absorb(wb.lat_out, mi["kv_b"], wb.o_abs, n)

@@ -48,17 +48,19 @@ def test_sparse_vs_oracle_and_reference(m, kidx, T, scale, n_split):
 @pytest.mark.parametrize("kidx", [65, 128, 129, 144, 145, 520, 1041, 2048, 2064, 2065, 2112, 2113])
 def test_one_row_merged_in_a_cluster(kidx):
     """one row of up to 33 tiles: clusters of 2 to 16 CTAs, with and without a ragged tile of up to 16 keys as a split's third,
-    gathered (some rows holes, whole splits of them too) and dense"""
+    gathered (some rows holes, whole splits of them too) and dense; and a dense range of a length on the device (partials in memory)"""
     T = 4096
     inp, ridx = _sparse_case(1, kidx, T, 0.0625, seed=kidx)
     ridx[:, 64:200] = -1
     q, c = dev_f16(inp["q_lat"]), dev_f16(inp["ckv"])
     out = torch.empty(1, 64, 512, dtype=torch.float16, device="cuda")
-    for lens in (None, np.array([kidx], dtype=np.int32)):
-        kw = dict(raw_idx=ridx, kidx=kidx) if lens is None else dict(kv_base=np.array([7], dtype=np.int64), kv_len=lens)
+    lens = np.array([kidx], dtype=np.int32)
+    for kw in (dict(raw_idx=ridx, kidx=kidx), dict(pos_start=kidx - 1), dict(kv_base=np.array([7], dtype=np.int64), kv_len=lens)):
         _, o32 = orc.mla_attend(inp["q_lat"], inp["ckv"], 1, 64, 0.0625, **kw)
-        if lens is None:
+        if "raw_idx" in kw:
             hk.mla_sparse_decode(q, c, dev(ridx), kidx, out, 1)
+        elif "pos_start" in kw:
+            hk.mla_dense_prefill(q, c, out, 1, kidx - 1)
         else:
             hk.mla_dense_prefill(q, c, out, 1, 0, kv_base=dev(kw["kv_base"]), kv_len=dev(lens), n_keys_hint=kidx)
         torch.cuda.synchronize()
@@ -80,6 +82,32 @@ def test_a_split_number_of_its_own_keeps_partials_in_memory(kidx):
         torch.cuda.synchronize()
         g = synth.f16_bits_to_f32(bits(out))
         assert max_rel(g, o32) < TOL and sum_rel(g, o32) < 3e-3
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("kidx", [130, 2052])
+def test_the_number_of_splits_says_the_form(kidx, dense):
+    """one row, a number given: that many splits through the workspace, also when it is the automatic one, and no byte behind them; no
+    number: the splits are merged in clusters, which leave the workspace alone"""
+    inp, ridx = _sparse_case(1, kidx, 4096, 0.0625, seed=kidx + 2)
+    q, c = dev_f16(inp["q_lat"]), dev_f16(inp["ckv"])
+    kw = dict(pos_start=kidx - 1) if dense else dict(raw_idx=ridx, kidx=kidx)
+    _, o32 = orc.mla_attend(inp["q_lat"], inp["ckv"], 1, 64, 0.0625, **kw)
+    auto = hk.mla_auto_splits(1, kidx)
+    for ns in (0, auto, auto - 1, 2, -1):
+        ws = torch.full((hk.mla_partial_bytes(auto + 2, 64),), 0xA5, dtype=torch.uint8, device="cuda")
+        out = torch.empty(1, 64, 512, dtype=torch.float16, device="cuda")
+        if dense:
+            hk.mla_dense_prefill(q, c, out, 1, kidx - 1, n_split=ns, workspace=ws)
+        else:
+            hk.mla_sparse_decode(q, c, dev(ridx), kidx, out, 1, n_split=ns, workspace=ws)
+        torch.cuda.synchronize()
+        g = synth.f16_bits_to_f32(bits(out))
+        assert max_rel(g, o32) < TOL and sum_rel(g, o32) < 3e-3
+        used = hk.mla_partial_bytes(ns, 64) if ns > 1 else 0
+        assert (ws[used:] == 0xA5).all(), "splits beyond the number given"
+        slots = ws[:ns * 64 * 4 if used else 0].view(torch.int32)
+        assert (slots != -1515870811).all(), "fewer splits than the number given (0xA5A5A5A5 is what was there)"
 
 
 def test_sparse_all_skipped_row_gives_zeros_and_duplicates_count_twice():
