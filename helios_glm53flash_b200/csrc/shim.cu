@@ -112,6 +112,17 @@ void release_scratch() {
     g_scratch[dev] = Scratch{};
   }
 }
+size_t mla_sparse_workspace_bytes(int m, int kidx) {
+  const int n_split = hk_mla_auto_splits(m, kidx);
+  return n_split > 1 ? hk_mla_partial_bytes(n_split, (int64_t)m * attn::N_HEADS) : 0;
+}
+void mla_sparse_decode(const half* q_lat, const half* ckv, const int* raw_idx, int kidx, half* lat_out, int m, void* workspace,
+                       size_t workspace_bytes, Stream s) {
+  if (m <= 0) return;
+  check(hk_mla_sparse(q_lat, ckv, 0, raw_idx, kidx, lat_out, m, attn::N_HEADS, attn::SCALE, hk_mla_auto_splits(m, kidx), workspace,
+                      workspace_bytes, s),
+        "mla_sparse_decode");
+}
 }  // namespace b200
 
 namespace attn {
@@ -162,8 +173,7 @@ void kpool_write(const half* idx_k, const half* idx_g, half* raw_ring, int raw_r
 void mla_sparse_decode(const half* q_lat, const half* ckv, const int* raw_idx, int kidx,
                        half* lat_out, int m, Stream s) {
   if (m <= 0) return;
-  const int n_split = hk_mla_auto_splits(m, kidx);
-  size_t bytes = n_split > 1 ? hk_mla_partial_bytes(n_split, (int64_t)m * N_HEADS) : 0;
+  const size_t bytes = b200::mla_sparse_workspace_bytes(m, kidx);
   void* ws = bytes ? scratch(bytes) : nullptr;
   // the launchers of a GPU share one stream, so the library may choose the form of a call that has the GPU to itself
   check(hk_mla_sparse(q_lat, ckv, 0, raw_idx, kidx, lat_out, m, N_HEADS, SCALE, 0, ws, bytes, s),

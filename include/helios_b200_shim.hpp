@@ -13,7 +13,8 @@
 //     per GPU, shared by all launchers of that GPU: call them from ONE stream, as the engine's layer
 //     loop does.  By default it is grow-only (cudaMalloc on first use / growth after a device
 //     synchronisation, like the reference's own dsa_topk workspace, src/cuda/aux/dsa_topk.cu:299-306)
-//     and helios::b200::release_scratch() frees it.  An engine that owns all device memory hands over
+//     and helios::b200::release_scratch() frees it.  (Sparse attention of several sequences on streams of their own has
+//     helios::b200::mla_sparse_decode, which takes its memory from the caller.)  An engine that owns all device memory hands over
 //     its own block once with helios::b200::set_scratch(ptr, bytes) (size it with
 //     scratch_bytes_needed): the launchers then never allocate or synchronise, also under stream
 //     capture, and abort with a message if a call needs more.  The hk_* ABI underneath never allocates.
@@ -107,6 +108,13 @@ void set_scratch(void* ptr, size_t bytes);
 // upper bound of what the launchers ask for when no call has more than max_rows rows (chunk length of the prefill;
 // decode calls are covered), for a KDA side of kda_batch sequences x kda_heads heads
 size_t scratch_bytes_needed(int max_rows, int kda_heads, int kda_batch = 1);
+// attn::mla_sparse_decode for a caller that has several such calls on streams of their own: with memory of the call's own
+// (mla_sparse_workspace_bytes, 256-byte aligned) in place of the GPU's one scratch buffer, and with one row's splits as single CTAs.
+// attn::mla_sparse_decode takes the form that is the faster one alone and the slower one in company (clusters on 64 SMs; figures
+// at hk_mla_sparse).
+size_t mla_sparse_workspace_bytes(int m, int kidx);
+void mla_sparse_decode(const half* q_lat, const half* ckv, const int* raw_idx, int kidx, half* lat_out, int m, void* workspace,
+                       size_t workspace_bytes, Stream s);
 }  // namespace b200
 
 }  // namespace helios

@@ -128,6 +128,32 @@ int main(int argc, char** argv) {
     download("prep2_beta", beta2, (size_t)S * H * 2);
     download("prep2_g", g2, (size_t)S * H * Dk * 4);
   }
+  // ---- sparse attention of one row: the launcher, and two calls side by side with memory of their own ----
+  {
+    const int kidx = 2052;
+    const size_t n = (size_t)attn::N_HEADS * attn::KV_LORA;
+    auto* q = (half*)upload("mla_q");
+    auto* ckv = (half*)upload("mla_ckv");
+    auto* idx = (int*)upload("mla_idx");
+    auto* lone = (half*)alloc(n * 2);
+    attn::mla_sparse_decode(q, ckv, idx, kidx, lone, 1);
+    cudaDeviceSynchronize();
+    download("mla_lone", lone, n * 2);
+    const size_t bytes = b200::mla_sparse_workspace_bytes(1, kidx);
+    half* side[2];
+    void* ws[2];
+    cudaStream_t st[2];
+    for (int i = 0; i < 2; i++) {
+      side[i] = (half*)alloc(n * 2);
+      ws[i] = alloc(bytes);
+      cudaStreamCreateWithFlags(&st[i], cudaStreamNonBlocking);
+    }
+    cudaDeviceSynchronize();
+    for (int i = 0; i < 2; i++) b200::mla_sparse_decode(q, ckv, idx, kidx, side[i], 1, ws[i], bytes, st[i]);
+    cudaDeviceSynchronize();
+    download("mla_side0", side[0], n * 2);
+    download("mla_side1", side[1], n * 2);
+  }
   b200::release_scratch();
   if (cudaDeviceSynchronize() != cudaSuccess) return 5;
   std::puts("SHIM HARNESS DONE");

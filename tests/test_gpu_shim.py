@@ -38,7 +38,9 @@ def test_cpp_launchers_equal_the_c_abi_bit_for_bit():
     S, F = 33, 3 * H * D
     pq = r.standard_normal((S, F), dtype=np.float32)
     raw = synth.kda_raw_gates(S, H, D, seed=41)
-    files = {"rec_qkv": inp["mixed_qkv"], "rec_g": inp["g"], "rec_beta": inp["beta"], "rec_state": s0,
+    mla = synth.mla_inputs(4096, 1, seed=41)
+    ridx = np.random.RandomState(41).randint(0, 4096, (1, 2052)).astype(np.int32)
+    files = {"mla_q": mla["q_lat"], "mla_ckv": mla["ckv"], "mla_idx": ridx, "rec_qkv": inp["mixed_qkv"], "rec_g": inp["g"], "rec_beta": inp["beta"], "rec_state": s0,
              "conv_x": cv["x"], "conv_state": cv["state"], "conv_w": cv["weight"], "topk_scores": sc,
              "norm_x": nx, "norm_w": nw, "norm_g": ng, "prep_qkv": pq, "prep_b": raw["b"], "prep_f": raw["f"],
              "prep_dt_bias": raw["dt_bias"], "prep_a_log": raw["a_log"]}
@@ -55,7 +57,8 @@ def test_cpp_launchers_equal_the_c_abi_bit_for_bit():
                "conv_out": out("conv_out", np.uint16, (37, 1536)), "conv_state": out("conv_state", np.uint16, (1536, 4)),
                "topk_idx": out("topk_idx", np.int32, (3, 512)), "norm_y": out("norm_y", np.uint16, (64, 128)),
                "prep_mixed": out("prep_mixed", np.uint16, (F, S)), "prep_beta": out("prep_beta", np.uint16, (S, H)),
-               "prep_g": out("prep_g", np.float32, (S, H, D)), "prep2_mixed": out("prep2_mixed", np.uint16, (F, S)),
+               "mla_lone": out("mla_lone", np.uint16, (1, 64, 512)), "mla_side0": out("mla_side0", np.uint16, (1, 64, 512)),
+               "mla_side1": out("mla_side1", np.uint16, (1, 64, 512)), "prep_g": out("prep_g", np.float32, (S, H, D)), "prep2_mixed": out("prep2_mixed", np.uint16, (F, S)),
                "prep2_beta": out("prep2_beta", np.uint16, (S, H)), "prep2_g": out("prep2_g", np.float32, (S, H, D))}
     # ---- the same calls through the C ABI (Python wrappers): recurrence in three calls with the same dispatch ----
     q, g, b, st = dev_bf16(inp["mixed_qkv"]), dev(inp["g"]), dev_bf16(inp["beta"]), dev(s0)
@@ -88,6 +91,14 @@ def test_cpp_launchers_equal_the_c_abi_bit_for_bit():
     for k, t in (("prep_mixed", mixed), ("prep_beta", beta), ("prep2_mixed", mixed), ("prep2_beta", beta)):
         assert np.array_equal(bits(t), got[k]), k
     assert np.array_equal(gg.cpu().numpy(), got["prep_g"]) and np.array_equal(gg.cpu().numpy(), got["prep2_g"])
+    # sparse attention: the launcher is the library's choice (clusters), the form for several streams the number given (other bits)
+    lat = [torch.empty(1, 64, 512, dtype=torch.float16, device="cuda") for _ in range(2)]
+    for o16, ns in zip(lat, (0, hk.mla_auto_splits(1, 2052))):
+        hk.mla_sparse_decode(dev_f16(mla["q_lat"]), dev_f16(mla["ckv"]), dev(ridx), 2052, o16, 1, n_split=ns)
+    torch.cuda.synchronize()
+    assert not torch.equal(lat[0], lat[1]), "two forms"
+    assert np.array_equal(bits(lat[0]), got["mla_lone"])
+    assert np.array_equal(bits(lat[1]), got["mla_side0"]) and np.array_equal(bits(lat[1]), got["mla_side1"])
     # values, not only agreement: the recurrence against the oracle
     _, o_32, o_st = orc.kda_recurrent(inp["mixed_qkv"], inp["g"], inp["beta"], s0, 1, T, H, H, D, D)
     assert frob_rel(got["rec_state"].reshape(1, 1, H, D, D), o_st) < 1e-2

@@ -183,12 +183,18 @@ def test_decode_step_of_two_sequences_on_their_own_streams_equals_sequence_by_se
         tr = TrunkAttention(n_kda=2, n_mla=2, heads=H, batch=2, max_ctx=n_tok + 64, max_chunk=chunk, seed=9, fused=fused,
                             keep_outputs=True)
         tr.prefill(n_tok, chunk)
+        if fused:
+            for bufs in tr._decode_bufs():
+                bufs.sparse_ws.fill_(0xA5)
         for s in range(steps):
             tr.run_chunk(n_tok + s, 1)
         torch.cuda.synchronize()
         assert hk.read_device_status() == 0
         runs.append(tr)
     a, b = runs
+    # side by side the splits of a row are single CTAs, with their partials in the sequence's own memory
+    slots = hk.mla_auto_splits(1, KIDX) * 64
+    assert all((bufs.sparse_ws[:4 * slots].view(torch.int32) != -1515870811).all() for bufs in a._dec)
     for seq in range(2):
         for L in range(2):
             assert torch.equal(a.ckv[seq][L], b.ckv[seq][L]) and torch.equal(a.pool[seq][L], b.pool[seq][L])
