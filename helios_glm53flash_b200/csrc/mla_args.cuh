@@ -17,7 +17,6 @@ struct MlaArgs {
   int m, n_heads;
   float scale;
   int n_split;
-  int n_cs;                 // cluster form of the flash kernel: parts that the 512 output channels are shared out in (1, 2, 4)
   __half* out;              // final output (n_split == 1) or null
   float* part_m;            // partials: [n_split][rows], [n_split][rows], [n_split][rows][512]
   float* part_l;

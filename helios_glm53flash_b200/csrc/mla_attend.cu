@@ -12,9 +12,9 @@
 namespace hk {
 
 // implemented in mla_flash_tc.cu; returns HK_ERR_UNSUPPORTED when the shape is not covered
-int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s);
+int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s, bool clusters = false);
 int mla_flash_tc_auto_splits(int m, int n_keys);
-bool mla_flash_cluster_shape(int m, int tiles, int* n_split, int* n_cs);
+bool mla_flash_cluster_shape(int m, int tiles, int* n_split);
 
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -116,8 +116,8 @@ static int attend(MlaArgs a, int n_keys_hint, int n_split, bool choose, void* wo
     // That is the form for a call that has the GPU to itself: its 64 SMs where the splits alone are 17 CTAs cost several calls side by
     // side more than each gains, which the library cannot see and the caller says with a number of splits (a step of 11 MLA layers at
     // 5,000 tokens, us, clusters / 17 CTAs: 1 sequence 275 / 296, 2 on streams 362 / 347, 3 404 / 403, 4 477 / 434, 8 866 / 650).
-    if (tc && choose && mla_flash_cluster_shape(a.m, tiles, &c.n_split, &c.n_cs)) {
-      const int st = mla_flash_tc_launch(c, s);
+    if (tc && choose && mla_flash_cluster_shape(a.m, tiles, &c.n_split)) {
+      const int st = mla_flash_tc_launch(c, s, true);
       if (st != HK_ERR_UNSUPPORTED) return st;
     }
     char* ws = (char*)workspace;

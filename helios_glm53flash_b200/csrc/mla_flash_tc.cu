@@ -64,7 +64,13 @@ constexpr int FT_LOAD_WARPS = 4, FT_THREADS = (6 + FT_LOAD_WARPS) * 32, FT_SLOTS
 
 constexpr int FT_MINI = 16;                       // keys of a tile in Q's place
 constexpr int FT_MAX_CL = 16;                     // CTAs of a cluster
-constexpr uint32_t FT_CL_STAGE = FT_HEADS * (256 * 4 + 8);  // outgoing shares behind the incoming ones (256 channels or 128)
+// Parts that a row's output channels are shared out in, a cluster each.  Four: a quarter of the product, of the accumulator and of the
+// shares for each CTA (11 MLA layers of a decode step 285 us, 303 with two).
+constexpr int FT_CS = 4, FT_CS_CH = LATENT / FT_CS;
+constexpr uint32_t FT_CL_ROW = FT_CS_CH * 4;                            // a head's share: its channels, and 8 bytes (m, l) behind all heads
+constexpr uint32_t FT_CL_STAGE = FT_HEADS * (FT_CL_ROW + 8);            // outgoing shares behind the incoming ones, in the idle ring
+static_assert(2 * FT_CL_STAGE <= FT_NBUF * FT_TILE && FT_CL_STAGE % 16 == 0 && (FT_HEADS / FT_MAX_CL) * (FT_CL_ROW + 8) % 16 == 0, "exchange area");
+static_assert(FT_CS_CH == 128, "a part is one N = 128 product of two 64-channel blocks, a half of it 64 columns of the accumulator");
 // all threads of all CTAs of the cluster.  Relaxed: the barriers only tell that memory is no longer in use, the data that crosses CTAs is
 // announced by mbarriers (.release: 1,000 cycles more each)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
@@ -104,8 +110,8 @@ __device__ __forceinline__ FtItem ft_item(const MlaArgs& a, int idx) {
   it.r = idx / a.n_split;
   it.cs = 0;
   if (CL) {
-    it.cs = it.r % a.n_cs;
-    it.r /= a.n_cs;
+    it.cs = it.r % FT_CS;
+    it.r /= FT_CS;
   }
   // rows of a causal chunk grow with their number: the longest first, so that the CTAs end together
   if (!G4 && !a.kv_len) it.r = a.m - 1 - it.r;
@@ -160,7 +166,7 @@ __device__ __forceinline__ void tma_gather4_rows(uint32_t leader, uint32_t smem_
 // gather4, tmap_q: the queries as tmap_box, tmap_o: 2-D map of the final output.
 // CL: cluster form for few rows of few keys (a decode step's gathered rows).  The splits of a row are the CTAs of a cluster, which merge
 // their partials through distributed shared memory and write the final output: no partials in memory, no second kernel.  The row's
-// output channels are shared out over n_cs such clusters, each of which computes the scores for itself.
+// output channels are shared out over FT_CS such clusters, each of which computes the scores for itself.
 // What bounds it is latency, one thing after another on 64 SMs: row numbers 1,200 cycles, gathered keys 2,800, two tiles of S, softmax and
 // P V 3,800, laying out and the barrier of the cluster 1,700, the shares 2,200, the merge 1,600.  2,052 gathered rows of one query 10.8 ->
 // 9.2 us; MLA layer of one token at 5,001 32.1 -> 28.9, selection and attention at 262,144 23.8 -> 21.8.
@@ -197,7 +203,7 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
     tc::mbar_init(&ms.q_ready, CL ? 1 : 128);              // (cluster form: the shares of the other splits)
     tc::mbar_init(&ms.o_free, 128);
     tc::mbar_fence_init();
-    if (CL) tc::mbar_arrive_expect_tx(&ms.q_ready, FT_HEADS * (LATENT / a.n_cs * 4 + 8));
+    if (CL) tc::mbar_arrive_expect_tx(&ms.q_ready, FT_CL_STAGE);
     ms.abort_flag = 0;
   }
   if (warp == 0) tc::tmem_alloc(&ms.tmem, 512);
@@ -385,9 +391,9 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
           // V: N = 256 channels = four 64-channel blocks (leading offset), K = keys in 8-row atoms of 1 KB
           const uint64_t vd = tc::make_sdesc_sw128(tc::smem_u32(smem + tile_at(kb)), blk_of(kb), 1024);
           const int steps = (it.keys(it.nth(tile)) + 15) >> 4;   // a ragged tile ends early
-          if (CL && a.n_cs > 1) {                          // one product of 256 or 128 channels
-            const uint32_t id = a.n_cs == 2 ? idesc : tc::make_idesc(64, 128, tc::FMT_F16, tc::FMT_F16, false, true);
-            const uint64_t vc = tc::sdesc_advance(vd, it.cs * (8 / a.n_cs) * blk_of(kb));
+          if (CL) {                                        // one product of this cluster's channels
+            const uint32_t id = tc::make_idesc(64, FT_CS_CH, tc::FMT_F16, tc::FMT_F16, false, true);
+            const uint64_t vc = tc::sdesc_advance(vd, it.cs * (FT_CS_CH / 64) * blk_of(kb));
 #pragma unroll
             for (int kk = 0; kk < FT_KEYS / 16; kk++)
               if (kk < steps)
@@ -488,7 +494,7 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
           wait_pv(g - 1, 8);
           tc::fence_after_sync();
 #pragma unroll 1
-          for (int c0 = 0; c0 < (CL ? 256 / a.n_cs : 256); c0 += 32) {
+          for (int c0 = 0; c0 < (CL ? FT_CS_CH / 2 : 256); c0 += 32) {
             uint32_t o[32];
             tc::tmem_ld32(tmem + FT_O + c0 + lanes, o);
             tc::tmem_ld_wait();
@@ -546,13 +552,13 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
         // The accumulator goes to the cluster's CTAs by heads: CTA j merges n_h of them.  It is laid out by destination in the idle
         // ring - n_h heads of the cluster's channels (16-byte chunk c of head h at c ^ (h % 8)), then their (m, l) - and leaves as one
         // bulk copy per CTA (16-byte remote stores: 3.6 us for 32 KB).
-        const int n_h = FT_HEADS / a.n_split, row = LATENT / a.n_cs * 4, share = n_h * (row + 8), j = head / n_h;
+        const int n_h = FT_HEADS / a.n_split, row = FT_CL_ROW, share = n_h * (row + 8), j = head / n_h;
         uint8_t* const out = smem + FS_K + FT_CL_STAGE + j * share;
 #pragma unroll 1
-        for (int c0 = 0; c0 < 256 / a.n_cs; c0 += 32) {
+        for (int c0 = 0; c0 < FT_CS_CH / 2; c0 += 32) {
           uint32_t o[32];
           load_o(c0, o);
-          const int lc = a.n_cs == 4 ? half * 64 + c0 : half * 128 + c0;   // channel within the cluster's part
+          const int lc = half * (FT_CS_CH / 2) + c0;       // channel within the cluster's part
 #pragma unroll
           for (int v = 0; v < 8; v++)
             *reinterpret_cast<uint4*>(out + (head - j * n_h) * row + ((((lc >> 2) + v) ^ (head & 7)) << 4)) =
@@ -641,7 +647,7 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
     ok = tc::mbar_wait(&ms.q_ready, 0, abort_flag, 16) && ok;   // every split's share of this CTA's heads has arrived
     cluster_arrive();
     const FtItem it = ft_item<G4, CL>(a, blockIdx.x);
-    const int n_h = FT_HEADS / a.n_split, row = LATENT / a.n_cs * 4, share = n_h * (row + 8), chunks = row / 16;
+    const int n_h = FT_HEADS / a.n_split, row = FT_CL_ROW, share = n_h * (row + 8), chunks = row / 16;
     if (!*abort_flag) {
       for (int i = tid; i < n_h * chunks; i += FT_THREADS) {
         const int h = i / chunks, c = i - h * chunks, head = it.sp * n_h + h;
@@ -667,7 +673,7 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
         uint2 w;
         w.x = *reinterpret_cast<const uint32_t*>(&h0);
         w.y = *reinterpret_cast<const uint32_t*>(&h1);
-        *reinterpret_cast<uint2*>(a.out + ((size_t)it.r * FT_HEADS + head) * LATENT + it.cs * (LATENT / a.n_cs) + c * 4) = w;
+        *reinterpret_cast<uint2*>(a.out + ((size_t)it.r * FT_HEADS + head) * LATENT + it.cs * FT_CS_CH + c * 4) = w;
       }
     }
     cluster_wait();                                        // nobody copies from this CTA's memory any more
@@ -710,11 +716,11 @@ static int ft_prepare() {
   return HK_OK;
 }
 
-// Cluster form: splits of a row and parts of its channels for m rows of about `tiles` tiles, false where it is not the better one.
-// One row, four parts of the channels, two tiles a split.  2,052 gathered rows 9.2 us against 10.8 with partials in memory; two rows
+// Cluster form: splits of a row for m rows of about `tiles` tiles, false where it is not the better one.
+// One row, two tiles a split.  2,052 gathered rows 9.2 us against 10.8 with partials in memory; two rows
 // find room for two parts each only (16 CTAs with a whole SM's memory in one GPC: seven clusters at once), whose shares of twice the size
 // take longer to cross: 11.7 against 11.6, three 12.2 against 12.5, and from four rows on the partials' own kernel fills the GPU.
-bool mla_flash_cluster_shape(int m, int tiles, int* n_split, int* n_cs) {
+bool mla_flash_cluster_shape(int m, int tiles, int* n_split) {
   int c = 2;
   while (c < FT_MAX_CL && c * 2 < tiles) c *= 2;
   if (tiles < 2 || tiles > 2 * FT_MAX_CL + 1 || m != 1) return false;
@@ -739,9 +745,8 @@ bool mla_flash_cluster_shape(int m, int tiles, int* n_split, int* n_cs) {
     fit[dev][lg] = n + 1;
   }
   const int room = fit[dev][lg] - 1;
-  if (room < 4) return false;
+  if (room < FT_CS) return false;
   *n_split = c;
-  *n_cs = 4;
   return true;
 }
 
@@ -761,7 +766,7 @@ static FtEncodeFn ft_encode_fn() {
   return fn;
 }
 
-int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s) {
+int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s, bool clusters) {
   FtEncodeFn encode = ft_encode_fn();
   if (a.n_heads != FT_HEADS || !encode) return HK_ERR_UNSUPPORTED;
   if (ft_prepare() != HK_OK) return HK_ERR_CUDA;
@@ -803,8 +808,8 @@ int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s) {
   }
   // Gathered rows: at most a CTA per SM (592 rows of 2,048 keys 180 -> 166 us).  Dense rows, whose loads start faster: a CTA
   // each (600 rows at 32,768 keys 2.72 ms, persistent 2.85).  Partials always: their rows leave through the idle ring.
-  if (a.n_cs > 0) {
-    const dim3 grid((unsigned)(a.m * a.n_cs * a.n_split));
+  if (clusters) {
+    const dim3 grid((unsigned)(a.m * FT_CS * a.n_split));
     const cudaError_t e = a.raw_idx ? pdl_launch_cluster(a.n_split, mla_flash_tc_kernel<true, true>, grid, dim3(FT_THREADS), FS_SMEM, s, a,
                                                          device_status_ptr(), box, rows, qmap, omap)
                                     : pdl_launch_cluster(a.n_split, mla_flash_tc_kernel<false, true>, grid, dim3(FT_THREADS), FS_SMEM, s, a,
