@@ -17,7 +17,10 @@ namespace {
 // element): 64 tokens x 64 channels, rows of 256 B in and 128 B out, 6.5 TB/s at 32,768 tokens.
 // LONG, odd lengths above 192: 128 tokens x 32 channels.  The rows start inside a sector, so a tile row ends in two partly written ones:
 // twice as long rows halve them (458 -> 430 us at 32,763 tokens; 368 -> 399 at 32,768).  Below, the tile's idle rows cost more: 64- / 128-token
-// tiles, 24,576 channels, us: 37 tokens 2.5 / 3.9, 63 2.7 / 3.9, 101 4.1 / 4.3, 129 5.4 / 6.7, 191 5.6 / 6.8, 255 7.5 / 7.1, 501 12.3 / 12.0.
+// tiles, 24,576 channels, us: 37 tokens 2.5 / 3.9, 63 2.7 / 3.9, 101 4.1 / 4.2, 129 5.1 / 6.5, 191 5.6 / 6.8, 255 7.5 / 7.1, 501 12.3 / 12.0;
+// 3,072 channels (8 heads) 37 1.5 / 1.9, 127 1.7 / 2.0, 191 1.7 / 2.2.  Just under 128 tokens one long tile is almost full: 127 tokens, 12,288
+// channels 2.8 / 2.8, 18,432 3.35 / 3.32, 24,576 4.37 / 4.23, 49,152 7.52 / 7.06, 98,304 12.7 / 12.0; 121 tokens 2.75 / 2.88, 3.32 / 3.41,
+// 4.33 / 4.32, 7.37 / 7.18, 12.4 / 12.1; 117 tokens 24,576 4.21 / 4.31, 98,304 12.17 / 12.16.
 // 4-byte stores from the first even element of a row on.  ODD without LONG: 2-byte stores (3 tokens x 12,288 channels 1.9 us, 2.8 the other way).
 // ---------------------------------------------------------------------------------------------
 template <bool LONG, bool ODD>
@@ -279,7 +282,7 @@ int launch_gated_rms_norm(const void* x, const void* w, void* y, const void* g, 
 HK_API int hk_kda_transpose_cast(void* dst_bf16, const float* src, int S, int F, void* stream) {
   HK_REQUIRE(dst_bf16 && src && S >= 0 && F >= 0);
   if (S == 0 || F == 0) return HK_OK;
-  const bool odd = S % 2 != 0, longer = odd && S > 192;
+  const bool odd = S % 2 != 0, longer = odd && (S > 192 || (S > 118 && S < 128 && F >= 24576));
   const int s_tiles = (S - 1) / (longer ? 128 : 64) + 1;
   HK_REQUIRE(s_tiles <= 65535);
   HK_REQUIRE(hk::aligned(dst_bf16, 4));

@@ -15,7 +15,8 @@ from helios_glm53flash_b200 import synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("S,F", [(64, 128), (37, 200), (1, 24576), (513, 96), (2048, 1536), (3, 7)])
+@pytest.mark.parametrize("S,F", [(64, 128), (37, 200), (1, 24576), (513, 96), (2048, 1536), (3, 7),
+                                 (117, 24577), (119, 24577), (127, 24576), (129, 24576)])
 def test_transpose_cast(S, F):
     x = synth.rng(S + F).standard_normal((S, F), dtype=np.float32)
     dx = dev(x)
