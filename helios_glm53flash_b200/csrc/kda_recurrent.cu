@@ -1219,6 +1219,9 @@ HK_API int hk_kda_recurrent(const void* mixed_qkv, const float* g, const void* b
       // 13.9 / 9.5; 32 chains 4 tokens 5.5 / 4.9, 37 tokens 16.5 / 11.1, 63 tokens 25.0 / 16.5; 64 chains 4 tokens 5.6 / 5.8, 8 tokens 7.1 /
       // 7.2, 13 tokens 9.3 / 8.4, 37 tokens 18.8 / 15.8, 63 tokens 29.4 / 23.7.  More chains stay with the columns kernel, whose smaller CTAs
       // share an SM (this one with two CTAs a chain, 96 chains: 24.9 / 30.4, 256: 53.0 / 60.0), and states off the 16-byte boundary too.
+      // Between those counts: 10, 12 and 15 chains 2 tokens 3.4 / 3.0-3.2, 4 tokens 3.7 / 3.5, 8 tokens 4.7 / 4.3, 12 tokens 5.9 / 5.0; 20, 24, 30
+      // and 36 chains 4 tokens 4.5-5.4 / 3.6, 12 tokens 7.4-8.8 / 5.4; 38 to 63 chains 9 tokens 8.4-10.5 / 6.6, and their 4 to 8 tokens by the
+      // columns kernel with four columns a lane 4.9-6.6, with two 6.2-9.6.
       const int per_chain = (int)std::min<int64_t>(sm_count() / chains, 8);
       const int more_than = per_chain < 4 ? 8 : (chains <= sm_count() / 16 ? 12 : 0);
       if (aligned(state, 16) && per_chain >= 2 && seqlen > more_than) {
