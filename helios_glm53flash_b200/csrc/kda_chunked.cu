@@ -31,6 +31,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstdlib>
 
 #include "hk_common.cuh"
 #include "tc05.cuh"
@@ -1301,7 +1302,8 @@ EncodeFn tensor_map_encoder() {
   static const EncodeFn fn = []() -> EncodeFn {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult qres;
-    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess
+    return getenv("HK_KDA_NO_TMA") == nullptr &&             // debug switch: no copy engine, i.e. the token-by-token kernels
+                   cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess
                ? (EncodeFn)p
                : nullptr;
   }();
@@ -1309,7 +1311,6 @@ EncodeFn tensor_map_encoder() {
 }
 bool encode_rows(CUtensorMap* map, const void* base, CUtensorMapDataType type, int elem, int channels, int seqlen, int bsz, int box_channels) {
   const EncodeFn encode = tensor_map_encoder();
-  if (!encode) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)channels, (cuuint64_t)seqlen, (cuuint64_t)bsz};
   const cuuint64_t strides[2] = {(cuuint64_t)channels * elem, (cuuint64_t)seqlen * channels * elem};
   const cuuint32_t box[3] = {(cuuint32_t)box_channels, (cuuint32_t)KC, 1}, estr[3] = {1, 1, 1};
@@ -1352,6 +1353,31 @@ HK_API size_t hk_kda_chunked_workspace_bytes(int bsz, int seqlen, int num_heads)
 
 namespace hk {
 namespace {
+// Without the tensor-map encoder, which every input and output of the chunked kernels needs: the same recurrence token by token.  Gates
+// that the call leaves to the preparation are formed by their own kernel, as many tokens at a time as the workspace holds.
+int prefill_without_tensor_maps(const void* mixed_qkv, const float* g_or_f, const void* beta_or_b, const float* dt_bias, const float* a_log,
+                                float lower_bound, bool gated, float* state, void* out, float* out_f32, int bsz, int seqlen, int H,
+                                const int* slots, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!gated)
+    return hk_kda_recurrent(mixed_qkv, g_or_f, beta_or_b, state, out, out_f32, bsz, seqlen, H, H, KD, KD, 1, slots, 1, 0, stream);
+  const size_t row = (size_t)H * KD;
+  const int piece = (int)std::min<size_t>(seqlen, workspace_bytes / (row * 4 + H * 2));
+  if (piece < 1) return HK_ERR_WORKSPACE;
+  float* g = (float*)workspace;
+  void* beta = g + piece * row;
+  for (int b = 0; b < bsz; b++)
+    for (int t = 0; t < seqlen; t += piece) {
+      const int n = std::min(piece, seqlen - t);
+      const size_t at = (size_t)b * seqlen + t;
+      int st = hk_kda_gate((const float*)beta_or_b + at * H, g_or_f + at * row, dt_bias, a_log, lower_bound, beta, g, n, H, KD, stream);
+      if (st == HK_OK)
+        st = hk_kda_recurrent((const __nv_bfloat16*)mixed_qkv + at * 3 * row, g, beta, slots ? state : state + (size_t)b * row * KD,
+                              (__nv_bfloat16*)out + at * row, out_f32 ? out_f32 + at * row : nullptr, 1, n, H, H, KD, KD, 1,
+                              slots ? slots + b : nullptr, 1, 0, stream);
+      if (st != HK_OK) return st;
+    }
+  return HK_OK;
+}
 int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const void* beta_or_b, const float* dt_bias,
                            const float* a_log, float lower_bound, bool gated, float* state, void* out,
                            float* out_f32, int bsz, int seqlen, int num_heads, const int* slots,
@@ -1366,6 +1392,9 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
   const FusedShape shape = fused_shape(n_jobs);
   const int n_slots = shape.slots;
   if (workspace_bytes < (n_slots ? ring_bytes(shape.room, RING) : hk_kda_chunked_workspace_bytes(bsz, seqlen, num_heads))) return HK_ERR_WORKSPACE;
+  if (!tensor_map_encoder())
+    return prefill_without_tensor_maps(mixed_qkv, g_or_f, beta_or_b, dt_bias, a_log, lower_bound, gated, state, out, out_f32, bsz, seqlen,
+                                       num_heads, slots, workspace, workspace_bytes, stream);
   const bool deep = n_slots && deep_ring(n_slots, (long long)n_jobs / n_slots * n_chunks) && workspace_bytes >= ring_bytes(n_slots, DEEP_RING);
   const int kr = deep ? DEEP_RING : RING;
   static bool attr_set[64] = {false};

@@ -1,5 +1,10 @@
 """GPU parity of the KDA kernels (short conv, recurrence) through the C ABI, against the CPU oracle
 and, when it was built, against the reference's own kernels compiled for sm_100a."""
+import os
+import subprocess
+import sys
+import tempfile
+
 import numpy as np
 import pytest
 import torch
@@ -635,3 +640,54 @@ def test_an_explicit_stream_is_the_one_that_runs():
         hk.kda_transpose_cast(dst, src, S, F, stream=1)
     with pytest.raises(TypeError):
         hk.gated_rms_norm(dst, src.int(), src, src, S, F, 1e-6)
+
+
+@pytest.mark.parametrize("T,H,bsz", [(130, 4, 3), (3000, 1, 1)])
+def test_chunked_prefill_without_the_tensor_map_encoder(T, H, bsz):
+    """both chunked entry points are served token by token where the encoder is missing (here: switched off in a child process), with the
+    bits of the gate kernel and the token-by-token recurrence; 3,000 tokens of one head are more gates than the workspace holds"""
+    D, r = 128, synth.rng(T)
+    raw = synth.kda_raw_gates(T, H, D, seed=T)
+    case = {"qkv": r.standard_normal((bsz, T, 3 * H * D), dtype=np.float32), "s0": 0.1 * r.standard_normal((bsz, 1, H, D, D), dtype=np.float32),
+            "f": np.broadcast_to(raw["f"], (bsz, T, H, D)).copy(), "b": r.standard_normal((bsz, T, H), dtype=np.float32),
+            "dt": raw["dt_bias"], "al": raw["a_log"]}
+    t = {k: dev(v.astype(np.float32)) for k, v in case.items()}
+    qkv, g = t["qkv"].to(torch.bfloat16), torch.empty(bsz, T, H, D, device="cuda")
+    beta, slots = torch.empty(bsz, T, H, dtype=torch.bfloat16, device="cuda"), torch.arange(bsz - 1, -1, -1, dtype=torch.int32, device="cuda")
+    for i in range(bsz):
+        hk.kda_gate(t["b"][i], t["f"][i], t["dt"], t["al"], -5.0, beta[i], g[i], T, H, D)
+    want = []
+    for sl in (None, slots):
+        st, out, o32 = t["s0"].clone(), torch.empty(bsz, T, H, D, dtype=torch.bfloat16, device="cuda"), torch.empty(bsz, T, H, D, device="cuda")
+        hk.cuda_recurrent_gated_delta_rule(qkv, g, beta, st, out, bsz, T, H, H, D, D, 1, sl, True, False, out_f32=o32, force_recurrent=True)
+        torch.cuda.synchronize()
+        want += [x.cpu() for x in (st, out, o32)]
+    code = """
+import sys, torch
+import helios_glm53flash_b200 as hk
+d = torch.load(sys.argv[1])
+bsz, T, H, D = d["g"].shape
+c = {k: v.cuda() for k, v in d.items()}
+res = []
+for gated in (False, True):
+    for sl in (None, c["slots"]):
+        st, out, o32 = c["s0"].clone(), torch.empty(bsz, T, H, D, dtype=torch.bfloat16, device="cuda"), torch.empty(bsz, T, H, D, device="cuda")
+        if gated:
+            hk.kda_chunked_prefill_gated(c["qkv"], c["f"], c["b"], c["dt"], c["al"], -5.0, st, out, bsz, T, H, slots=sl, out_f32=o32)
+        else:
+            hk.cuda_recurrent_gated_delta_rule(c["qkv"], c["g"], c["beta"], st, out, bsz, T, H, H, D, D, 1, sl, True, False, out_f32=o32)
+        torch.cuda.synchronize()
+        res += [x.cpu() for x in (st, out, o32)]
+torch.save(res, sys.argv[2])
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    with tempfile.TemporaryDirectory() as d:
+        torch.save({"qkv": qkv.cpu(), "g": g.cpu(), "beta": beta.cpu(), "slots": slots.cpu(), **{k: t[k].cpu() for k in ("s0", "f", "b", "dt", "al")}},
+                   os.path.join(d, "in.pt"))
+        res = subprocess.run([sys.executable, "-c", code, os.path.join(d, "in.pt"), os.path.join(d, "out.pt")], cwd=root, capture_output=True,
+                             text=True, timeout=300, env=dict(os.environ, HK_KDA_NO_TMA="1"))
+        assert res.returncode == 0, res.stderr[-2000:]
+        got = torch.load(os.path.join(d, "out.pt"))
+    assert len(got) == 2 * len(want)
+    for a, b in zip(got, want + want):
+        assert torch.equal(a, b)
