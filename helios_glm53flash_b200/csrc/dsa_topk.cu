@@ -10,7 +10,7 @@
 // compaction that places the "above" entries and the tie entries at once (the reference makes two histogram sweeps and two
 // compaction sweeps of global memory).  Three kernels:
 //   dsa_topk_rows_kernel      rows of up to 16,384 scores, read once into registers, a small CTA each
-//   dsa_topk_cluster_kernel   at most 16 longer rows of up to 262,143 scores, read once into the registers of a cluster of 8 CTAs
+//   dsa_topk_cluster_kernel   at most 16 longer rows of up to 262,144 scores, read once into the registers of a cluster of 8 CTAs
 //   dsa_topk_kernel           every other call (many long rows, lengths known on the device only): one CTA of 1,024 threads per
 //                             row, which sweeps the row three times; topk_row also selects among candidates in shared memory
 #include <cooperative_groups.h>
@@ -375,7 +375,8 @@ __device__ long long hk_topk_trace[16];
 // What bounds it: these steps one after the other (load and count 1.5 us, the crossing bucket 1.0, low bits 0.9, offsets 0.9, output 1.0).
 // One row of 65,536 scores 6.8 -> 5.8 us against sharing out the 2,048 sums by slices (four barriers); 262,000 scores 18.5 -> 11.8, 16 rows of
 // 30,000 13.9 -> 10.9 (the launch bound names the CTA per SM: at the 32 registers taken without it the four-piece form spilled).
-// NP = 1, 2, 4 cover rows of 65,535, 131,071 and 262,143 scores at any alignment (1M tokens of context).
+// NP = 1, 2, 4 cover rows of 65,536, 131,072 and 262,144 scores (1M tokens of context), up to seven fewer where a row starts off a 16-byte
+// boundary.
 // ------------------------------------------------------------------------------------------------
 constexpr int TKC_CTAS = 8;
 constexpr int TKC_PIECES = TKC_CTAS * TK_THREADS;         // pieces of 8 elements that NP = 1 holds

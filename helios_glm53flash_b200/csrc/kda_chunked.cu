@@ -16,8 +16,13 @@
 // and B on the warp-level tensor cores: 16-token blocks against earlier blocks in fp16 with exponents re-based at block starts (both
 // operands at most 1), a block against itself in TF32 (e^{-x} needs the fp32 exponent range; the triangular tiles are smaller than a
 // tcgen05 tile).  It inverts the unit-triangular system in fp32-class arithmetic and runs the dense W | Uloc = T [K+ | V] product on
-// tcgen05 (M128 N128 K64, twice).  It writes, per chunk, operand tiles that are already in the shared-memory layout the scan
-// needs (74,240 bytes).
+// tcgen05 (weight-stationary M64 N128 K64, twice).  It writes, per chunk, operand tiles that are already in the shared-memory layout the
+// scan needs (74,240 bytes).
+//   Pairs of blocks were TF32 products of fp32 rows once.  fp16 has the same 11 bits and less range: values below 6e-5 lose bits, below
+// 3e-8 they are 0.  What comes of the products, B beta and the inverse T, is stored as fp16 itself, with the same absolute spacing, so the
+// operands' loss stays below that of the result.  Error against 64 bits, TF32 -> fp16, 16 seeds, outputs / state: the model's gates 4.19e-4
+// -> 4.19e-4 / 2.94e-4 -> 2.94e-4; no decay 5.2 -> 5.1e-4 / 4.6 -> 4.4e-4; e^-8 and e^-12 a block, values in a chunk's first block only, beta
+// 1e-6 behind it, keys nearly alike: every ratio within 0.993 and 1.003, the spread of the seeds.
 //   What bounds it: latencies.  A unit crosses five barriers of its 256 threads and one product; two units share an SM (128 registers
 //   a thread, 109 KB).  Inputs arrive by tensor copies issued while the unit before is finished.  A worker's unit takes 22-24 thousand
 //   cycles with two workers on the SM, 39 thousand in the form before (k and q rows in separate warps, TF32 for all block pairs,
@@ -641,8 +646,7 @@ __device__ __forceinline__ void prep_unit(
 
   // ---- stage 4: X = (I + N)^-1 below its diagonal blocks, and its fp16 copy T as the K-major A operand (K = 64).  First
   //      P_mj = N_mj X_jj in place of N_mj, one warp per block, while two warps write the diagonal of T and the zeros above it;
-  //      then one warp per row of blocks.  Rows 64-127 of the operand are whatever the memory holds: their lanes of the product
-  //      are never read ----
+  //      then one warp per row of blocks ----
   if (warp < 6) {
     const int m = warp < 1 ? 1 : (warp < 3 ? 2 : 3), j = warp - (m * (m - 1)) / 2, ld = m < 2 ? 36 : 68;
     float* nb = sN + prep_n_row(16 * m) + 16 * j;
@@ -1264,7 +1268,9 @@ int g_chunked_form = 0;
 // Chain slots of the fused launch and the value columns of a chain CTA for n_jobs (batch, head) chains; no slots = use the two-kernel
 // form.  Chains share slots evenly (a slot walks its chains one after the other), and the preparation keeps 64 SMs or more.  Of the
 // divisors of n_jobs from 16 to 48, or n_jobs itself, the one for which the longer of the two sides takes least per chunk of all
-// chains: a chain CTA needs 1,380 ns a chunk with all 128 columns, 1,100 with 64, an SM of preparation workers 5,800 ns a unit.
+// chains: a chain CTA needs 1,380 ns a chunk with all 128 columns, 1,100 with 64, an SM of preparation workers 5,800 ns a unit.  Waits counted
+// in a measuring build bear the sides out, 32,768 tokens: with 32 heads the workers are the longer side (a unit 22,770 cycles, of them 400
+// for a ring slot; a chain CTA's chunk 3,200, of them 940 for its unit), with 16 and 8 the chains are (workers 22 and 64 % of their time).
 // (32,768 tokens x 8 heads 719 -> 532 us with two CTAs a chain, x 16 725 -> 580; 32 heads have one, at 84 SMs of workers they would
 // take 1,150; 3 sequences x 8,192 x 32 heads 786 with 48 slots of two chains, 685 with 32 of three.)
 // `room`: the slots that the workspace is sized for, the largest number that divides the chains: it covers calls of fewer sequences.

@@ -103,7 +103,10 @@ int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_wei
  * hk_kda_recurrent(channelwise=1, history=0) on the same arguments (the reference has no chunked
  * kernel: prefill calls the recurrence with seqlen = n, src/engine/runner.cpp:468-471).
  * Requires dk = dv = 128, Hk == Hv.  seqlen may be any positive length (a ragged tail shorter
- * than a chunk is processed by the same kernels).  `workspace` must hold at least
+ * than a chunk is processed by the same kernels).  Log decays: the sum of a channel's over a 16-token block of a chunk (tokens 0-15,
+ * 16-31, ...) is taken as at least -85, which every product of two factors e^x, e^-x needs; the results are those of
+ * hk_kda_recurrent where no such sum is lower, i.e. for every gate of -5.3 or more (the model's are at least -5), and wrong in
+ * the channels where one is.  `workspace` must hold at least
  * hk_kda_chunked_workspace_bytes(bsz, seqlen, num_heads) bytes, 256-byte aligned.
  * Two forms.  ONE persistent cooperative launch when the chains fit its chain slots (at most 48 chains, or more when a
  * number of slots in [16, 48] divides their count, e.g. 64 heads or 8 x 32: a slot then walks several chains one after
@@ -246,7 +249,7 @@ int hk_mla_auto_splits(int m, int n_keys);
  * (0 = not told, as in the reference's signature: every non-negative row number is read).
  * n_split > 0: that many splits, a CTA each, through the workspace.  n_split <= 0 lets the library choose number and form
  * (hk_mla_auto_splits says the number; workspace may be NULL when it is 1): the fastest form of a call that has the GPU to
- * itself.  One row of 65 to 2,112 keys then runs as clusters on 64 SMs.  Calls that run beside others on streams of their own
+ * itself.  One row of 129 to 2,112 keys then runs as clusters on 64 SMs.  Calls that run beside others on streams of their own
  * are faster as single CTAs, n_split = hk_mla_auto_splits(m, kidx): 11 MLA layers of a decode step at 5,000 tokens, clusters /
  * single CTAs, 1 sequence 275 / 296 us, 2 sequences on two streams 362 / 347, 4 477 / 434, 8 866 / 650.                  */
 int hk_mla_sparse(const void* q_lat, const void* ckv, int64_t ckv_rows, const int* raw_idx, int kidx, void* lat_out,
