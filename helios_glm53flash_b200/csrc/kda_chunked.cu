@@ -386,7 +386,7 @@ __device__ __forceinline__ void prep_unit(
   float2 dec;                                              // e^{G_last} of channels gc, gc + 1 (lanes with J = 3)
   {
     constexpr float LOG2E = 1.4426950408889634f;
-    constexpr float FLOOR = -85.f * LOG2E;                 // keeps e^{x} and e^{-x} inside fp32
+    constexpr float FLOOR = -80.5f * LOG2E;                // keeps k^ e^{x} and k^ e^{-x} inside fp32's normal range (gates of -5: -80)
     float decay = 0.f;
     float2 bias = make_float2(0.f, 0.f);
     int n_block = 16;                                      // GATED: tokens of this block that exist (the others read as zeros)
@@ -415,6 +415,31 @@ __device__ __forceinline__ void prep_unit(
       tot.y = fmaf(gr[i].y, LOG2E, tot.y);
       *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = make_float2(fmaxf(tot.x, FLOOR), fmaxf(tot.y, FLOOR));
     }
+    if (__builtin_expect(__any_sync(0xffffffffu, fminf(tot.x, tot.y) < FLOOR), 0)) {
+      // Rare: a channel decays by more than e^-80 inside the block.  Sums that stopped at the floor would take the tokens behind it as
+      // not decaying at all, so the strongest of its gates are weakened instead: to e^-40, or to e^-20, e^-10 or e^-5, whichever is the
+      // first that keeps the block's sum.
+      float lo_x = tot.x < FLOOR ? -40.f : -INFINITY, lo_y = tot.y < FLOOR ? -40.f : -INFINITY;
+      auto at_least = [](float v, float lo) { return v < lo ? lo : v; };   // (a NaN stays one)
+#pragma unroll 1
+      for (int k = 0; k < 3; k++) {
+        float sx = 0.f, sy = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          sx += at_least(gr[i].x, lo_x);
+          sy += at_least(gr[i].y, lo_y);
+        }
+        if (sx < -80.f) lo_x *= 0.5f;
+        if (sy < -80.f) lo_y *= 0.5f;
+      }
+      tot = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        tot.x = fmaf(at_least(gr[i].x, lo_x), LOG2E, tot.x);
+        tot.y = fmaf(at_least(gr[i].y, lo_y), LOG2E, tot.y);
+        *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = make_float2(fmaxf(tot.x, FLOOR), fmaxf(tot.y, FLOOR));
+      }
+    }
     float2 before = make_float2(0.f, 0.f), after = make_float2(0.f, 0.f), next1 = before, next2 = before;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -426,7 +451,7 @@ __device__ __forceinline__ void prep_unit(
     }
     auto put = [&](int r, float2 v) { *reinterpret_cast<float2*>(sTab + r * KD + gc) = make_float2(ex2_approx(v.x), ex2_approx(v.y)); };
     put(TAB_EP + J, before);
-    // decay from a token to the end of ITS block is e^{tot - x} = e^{-x} e^{tot} (each factor within fp32 range for |x| <= 85),
+    // decay from a token to the end of ITS block is e^{tot - x} = e^{-x} e^{tot} (each factor within fp32 range for |x| <= 80.5),
     // the decay over the LATER blocks is e^{G_last - P_next} (may underflow: then Kt is 0)
     put(TAB_ETOT + J, tot);
     put(TAB_KE + J, after);

@@ -103,10 +103,10 @@ int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_wei
  * hk_kda_recurrent(channelwise=1, history=0) on the same arguments (the reference has no chunked
  * kernel: prefill calls the recurrence with seqlen = n, src/engine/runner.cpp:468-471).
  * Requires dk = dv = 128, Hk == Hv.  seqlen may be any positive length (a ragged tail shorter
- * than a chunk is processed by the same kernels).  Log decays: the sum of a channel's over a 16-token block of a chunk (tokens 0-15,
- * 16-31, ...) is taken as at least -85, which every product of two factors e^x, e^-x needs; the results are those of
- * hk_kda_recurrent where no such sum is lower, i.e. for every gate of -5.3 or more (the model's are at least -5), and wrong in
- * the channels where one is.  `workspace` must hold at least
+ * than a chunk is processed by the same kernels).  Log decays: a channel's sum over a 16-token block of a chunk (tokens 0-15, 16-31,
+ * ...) of at least -80, i.e. every gate of -5 or more (the model's), is taken as it is.  Where a block's sum is lower, its strongest
+ * gates are weakened to -40, -20, -10 or -5, the first that keeps the sum: a few hard resets leave nothing to see (e^-40, e^-20),
+ * sixteen gates in a row all below -5 leave e^-5 = 0.7 % of the state (use hk_kda_recurrent where that matters).  `workspace` must hold at least
  * hk_kda_chunked_workspace_bytes(bsz, seqlen, num_heads) bytes, 256-byte aligned.
  * Two forms.  ONE persistent cooperative launch when the chains fit its chain slots (at most 48 chains, or more when a
  * number of slots in [16, 48] divides their count, e.g. 64 heads or 8 x 32: a slot then walks several chains one after

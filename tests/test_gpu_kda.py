@@ -194,6 +194,40 @@ def test_chunked_prefill_vs_oracle(T, H, gate):
     assert np.array_equal(bits(out), want_bits)
 
 
+@pytest.mark.parametrize("gate,tol", [("resets", 2e-3), ("minus_inf", 2e-3), ("some", 2e-3), ("channels", 1.5e-2), ("strong", 1.5e-2)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_chunked_prefill_of_gates_that_decay_a_block_below_fp32(gate, tol, gated):
+    """a channel's decay over a 16-token block below e^-80: hard resets between mild gates (also e^-inf), a few strong gates in a block, every
+    gate of some channels or of all of them stronger than e^-5.  The strongest of a block are weakened, at worst to e^-5 = 6.7e-3 of the
+    state instead of less, which a token's output and update each see once: 1.5e-2; with room for e^-10 (5e-5) the usual bounds"""
+    T, H, D = 200, 4, 128
+    inp, r = synth.kda_inputs(T, H, D, seed=5), np.random.RandomState(5)
+    f = np.abs(r.standard_normal((1, T, H, D))).astype(np.float32)
+    hard = r.random((1, T, H, D)) < 0.08
+    g = {"resets": np.where(hard, -100.0, -0.05 * f), "minus_inf": np.where(hard, -np.inf if not gated else -500.0, -0.05 * f),
+         "some": np.where(r.random((1, T, H, D)) < 0.25, -30.0, -0.3 * f), "channels": np.where(np.arange(D) % 2, -8.0 - f, -0.05 * f),
+         "strong": -5.5 - 5.0 * f}[gate].astype(np.float32)
+    s0 = (0.1 * r.standard_normal((1, 1, H, D, D))).astype(np.float32)
+    beta, st = inp["beta"], dev(s0)
+    out, o32 = torch.empty(1, T, H, D, dtype=torch.bfloat16, device="cuda"), torch.empty(1, T, H, D, device="cuda")
+    if gated:                                                # raw gates whose prepared values are g: a bound of -600, the sigmoid's inverse
+        lb, fr = -600.0, np.log(np.maximum(-g, 1e-6) / (600.0 + g)).astype(np.float32)
+        gd, bd = torch.empty(1, T, H, D, device="cuda"), torch.empty(1, T, H, dtype=torch.bfloat16, device="cuda")
+        raw_b, zero, one = dev(r.standard_normal((1, T, H)).astype(np.float32)), torch.zeros(H, D, device="cuda"), torch.zeros(H, device="cuda")
+        hk.kda_gate(raw_b, dev(fr), zero, one, lb, bd, gd, T, H, D)
+        g, beta = gd.cpu().numpy(), bits(bd)
+        hk.kda_chunked_prefill_gated(dev_bf16(inp["mixed_qkv"]), dev(fr), raw_b, zero, one, lb, st, out, 1, T, H, out_f32=o32)
+    else:
+        hk.cuda_recurrent_gated_delta_rule(dev_bf16(inp["mixed_qkv"]), dev(g), dev_bf16(beta), st, out, 1, T, H, H, D, D, 1, None, True, False,
+                                           out_f32=o32)
+    torch.cuda.synchronize()
+    assert hk.read_device_status() == 0
+    _, o_32, o_st = orc.kda_recurrent(inp["mixed_qkv"], g, beta, s0, 1, T, H, H, D, D)
+    e_out, e_st = frob_rel(o32.cpu().numpy(), o_32), frob_rel(st.cpu().numpy(), o_st)
+    print("gates %s: outputs %.2e, state %.2e" % (gate, e_out, e_st))
+    assert e_out < tol and e_st < tol
+
+
 def test_chunked_prefill_then_decode_continues_the_state():
     T, H, D, extra = 256, 4, 128, 16
     inp = synth.kda_inputs(T + extra, H, D, seed=9)
