@@ -47,7 +47,7 @@ def test_sparse_vs_oracle_and_reference(m, kidx, T, scale, n_split):
 
 @pytest.mark.parametrize("kidx", [65, 128, 129, 144, 145, 520, 1041, 2048, 2064, 2065, 2112, 2113])
 def test_one_row_merged_in_a_cluster(kidx):
-    """one row of up to 33 tiles: clusters of 2 to 16 CTAs, with and without a ragged tile of up to 16 keys as a split's third,
+    """one row of 3 to 33 tiles (and of two, which is one split): clusters of 2 to 16 CTAs, with and without a ragged tile of up to 16 keys as a split's third,
     gathered (some rows holes, whole splits of them too) and dense; and a dense range of a length on the device (partials in memory)"""
     T = 4096
     inp, ridx = _sparse_case(1, kidx, T, 0.0625, seed=kidx)
