@@ -413,10 +413,10 @@ __device__ __forceinline__ void prep_unit(
       }
       tot.x = fmaf(gr[i].x, LOG2E, tot.x);
       tot.y = fmaf(gr[i].y, LOG2E, tot.y);
-      *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = make_float2(fmaxf(tot.x, FLOOR), fmaxf(tot.y, FLOOR));
+      *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = tot;
     }
     if (__builtin_expect(__any_sync(0xffffffffu, fminf(tot.x, tot.y) < FLOOR), 0)) {
-      // Rare: a channel decays by more than e^-80 inside the block.  Sums that stopped at the floor would take the tokens behind it as
+      // Rare: a channel decays by more than e^-80 inside the block.  Sums that stop at a floor would take the tokens behind it as
       // not decaying at all, so the strongest of its gates are weakened instead: to e^-40, or to e^-20, e^-10 or e^-5, whichever is the
       // first that keeps the block's sum.
       float lo_x = tot.x < FLOOR ? -40.f : -INFINITY, lo_y = tot.y < FLOOR ? -40.f : -INFINITY;
@@ -437,7 +437,7 @@ __device__ __forceinline__ void prep_unit(
       for (int i = 0; i < 16; i++) {
         tot.x = fmaf(at_least(gr[i].x, lo_x), LOG2E, tot.x);
         tot.y = fmaf(at_least(gr[i].y, lo_y), LOG2E, tot.y);
-        *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = make_float2(fmaxf(tot.x, FLOOR), fmaxf(tot.y, FLOOR));
+        *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = tot;
       }
     }
     float2 before = make_float2(0.f, 0.f), after = make_float2(0.f, 0.f), next1 = before, next2 = before;
