@@ -4,10 +4,10 @@
 // with kv_b the raw [64*512][512] fp16 tensor (rows h*512 .. +255 = W_uk[h], +256 .. +511 = W_uv[h]);
 // reference: src/cuda/attn/attn.cu:12-130 (one block per (row, head), the head's weights re-read per row).
 //
-// Two kernels: up to 32 rows with the weights as the M operand (below), more rows in 256 x 256 tiles.  Operands arrive as TMA
-// tensor copies in 128-byte-swizzle boxes (A [rows][64 k]; W either [64 k][64 n] with n contiguous - W_uk, transposed W_uv - or
-// [n][64 k] with k contiguous - raw W_uv, so o_absorb needs no transposed copy of the weights).  Rows past the end of the batch
-// are zero-filled by the copy engine and not stored.  All waits are bounded.
+// Three kernels: up to 8 rows with operands in registers (warp-level products), up to 32 with the weights as the M operand, more in
+// 256 x 256 tiles.  In the last two operands arrive as TMA tensor copies in 128-byte-swizzle boxes (A [rows][64 k]; W either
+// [64 k][64 n] with n contiguous - W_uk, transposed W_uv - or [n][64 k] with k contiguous - raw W_uv, so o_absorb needs no transposed
+// copy of the weights).  Rows past the end of the batch are zero-filled by the copy engine and not stored.  All waits are bounded.
 #include <cuda.h>   // CUtensorMap (types only; the encoder is fetched through the runtime at first use)
 
 #include <cstdlib>
@@ -210,7 +210,7 @@ __global__ __launch_bounds__(AB_THREADS, 1) void absorb_gemm_tc_kernel(
 }
 
 // ------------------------------------------------------------------------------------------------
-// A few rows (decode, at most 32): the 16.8 MB of weights are all there is to move.  As 128-row tiles such a call has 128
+// A few rows (at most 32): the 16.8 MB of weights are all there is to move.  As 128-row tiles such a call has 128
 // tiles, on 128 SMs, of which a row uses 1/128: 7.8 (q) and 10.5 us (o).  Here the WEIGHTS are the M operand, 64 output
 // columns per CTA (512 and 256 CTAs, all resident), the rows are N (8 to 32), and a CTA requests its whole K at once (32 /
 // 64 KB, a barrier per 64-channel chunk): no ring, no empty barriers.
@@ -299,6 +299,118 @@ __global__ __launch_bounds__(AF_THREADS) void absorb_few_rows_kernel(const __gri
   __syncthreads();
   if (warp == 1) tc::tmem_dealloc(tmem, 32);
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Up to eight rows (a decode step).  What bounds it is latency: 16.8 MB over 148 SMs are 1 us from L2, and the tensor-map fetch, tensor
+// memory, products behind barriers and the way back of the kernel above are more than that.  Here a lane loads its operand fragments of
+// the warp-level product straight into registers, all of them at once (m16n8k16, the weights as the 16 rows and the batch as the 8
+// columns, fp32 sums), the warps of a CTA share out K, and their sums meet once in shared memory.  The contraction index is taken in
+// whatever order a lane's pieces hold it, the same for both operands.  1,024 CTAs of 16 KB, seven a SM (512 of 32 KB are 4 or 3: q 4.0).
+// In a graph of 20 calls, weights in L2 / from HBM, 1 row: q 4.5 -> 3.7 / 4.8 -> 3.9 us, o 4.1 -> 3.1 / 5.2 -> 3.4; 8 rows: q 4.6 -> 4.5 /
+// 5.0 -> 4.6, o 4.2 -> 3.4 / 5.4 -> 3.8.  MLA layer of one token at 5,001 29.3 -> 24.8 us.  From nine rows on, and for the transposed W_uv, whose
+// CTAs hold twice the K here (8 rows 4.9 for 4.2), the kernel above is the better one.
+// ------------------------------------------------------------------------------------------------
+constexpr int A8_ROWS = 8;
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void prefetch_l2_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// W_MN: weights [k][n] with n contiguous: a CTA has 32 columns, a warp 64 k of them, a lane four columns of 16 k, whose pairs along k it
+// puts together itself.  Else [n][k]: a CTA has 16 columns, a warp 128 k, and a piece along k is what the product takes.
+template <bool W_MN, int K>
+__global__ __launch_bounds__(W_MN ? K / 2 : K / 4, W_MN ? 2048 / K : 8) void absorb_8_rows_kernel(const __half* __restrict__ w, const __half* x, __half* __restrict__ out,
+                                                                        int n_rows, int n_out, int w_rows_per_head, int w_row_off) {
+  constexpr int WARPS = W_MN ? K / 64 : K / 128, BN = W_MN ? 32 : 16;
+  __shared__ __align__(16) float red[WARPS][A8_ROWS][BN];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * BN, h = blockIdx.y;
+  const bool row = g < n_rows;
+  // 16-byte pieces of a row of sums change places by the row, so that a quarter-warp writes to all banks
+  auto swap = [](int r) -> int { return W_MN ? (r >> 1) << 1 : 0; };
+  if constexpr (W_MN) {
+    // k = 64 warp + 16 s + 4 t + e; columns n0 + 4 g ..
+    const __half* wp = w + (size_t)(h * w_rows_per_head + w_row_off + 64 * warp + 4 * t) * n_out + n0 + 4 * g;
+    if (g == 0)
+#pragma unroll
+      for (int i = 0; i < 16; i++) prefetch_l2_line(wp + (size_t)((i >> 2) * 16 + (i & 3)) * n_out);
+    pdl_wait();
+    uint2 wr[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(wr[i].x), "=r"(wr[i].y) : "l"(wp + (size_t)((i >> 2) * 16 + (i & 3)) * n_out));
+    uint2 xr[4];
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+      xr[s] = row ? __ldcg(reinterpret_cast<const uint2*>(x + ((size_t)g * 64 + h) * K + 64 * warp + 16 * s + 4 * t)) : make_uint2(0, 0);
+    float c[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+      const uint32_t* r0 = &wr[4 * s].x;
+      const uint32_t* r1 = &wr[4 * s + 1].x;
+      const uint32_t* r2 = &wr[4 * s + 2].x;
+      const uint32_t* r3 = &wr[4 * s + 3].x;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {                          // column 4 g + i: its four k as two pairs
+        const uint32_t sel = i & 1 ? 0x7632 : 0x5410;
+        mma_16816(c[i], __byte_perm(r0[i >> 1], r1[i >> 1], sel), 0, __byte_perm(r2[i >> 1], r3[i >> 1], sel), 0, xr[s].x, xr[s].y);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+      if (2 * t + r < n_rows) {
+        float4* p = reinterpret_cast<float4*>(red[warp][2 * t + r]);
+        p[g ^ swap(2 * t)] = make_float4(c[0][r], c[1][r], c[2][r], c[3][r]);
+      }
+  } else {
+    // k = 128 warp + 32 s + 8 t + e; columns n0 + g and n0 + g + 8
+    const __half* wp = w + (size_t)(h * w_rows_per_head + w_row_off + n0 + g) * K + 128 * warp + 8 * t;
+    if (t == 0)
+#pragma unroll
+      for (int i = 0; i < 4; i++) prefetch_l2_line(wp + (i >> 1) * 8 * K + (i & 1) * 64);
+    pdl_wait();
+    uint4 wr[4][2], xr[4];
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+#pragma unroll
+      for (int u = 0; u < 2; u++) wr[s][u] = ld_stream16(wp + u * 8 * K + 32 * s);
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+      xr[s] = row ? __ldcg(reinterpret_cast<const uint4*>(x + ((size_t)g * 64 + h) * K + 128 * warp + 32 * s + 8 * t)) : make_uint4(0, 0, 0, 0);
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+      mma_16816(c, wr[s][0].x, wr[s][1].x, wr[s][0].y, wr[s][1].y, xr[s].x, xr[s].y);
+      mma_16816(c, wr[s][0].z, wr[s][1].z, wr[s][0].w, wr[s][1].w, xr[s].z, xr[s].w);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (2 * t + (e & 1) < n_rows) red[warp][2 * t + (e & 1)][g + 8 * (e >> 1)] = c[e];
+  }
+  __syncthreads();
+  const int n = tid % BN;
+  for (int r = tid / BN; r < n_rows; r += WARPS * 32 / BN) {
+    const int at = n ^ (swap(r) << 2);
+    float sum = red[0][r][at];
+#pragma unroll
+    for (int i = 1; i < WARPS; i++) sum += red[i][r][at];
+    out[((size_t)r * 64 + h) * n_out + n0 + n] = __float2half_rn(sum);
+  }
+}
+
+template <bool W_MN, int K>
+static int absorb_8_rows(const void* x, const void* w, void* out, int n_rows, int n_out, int w_rows_per_head, int w_row_off, cudaStream_t s) {
+  return pdl_launch(absorb_8_rows_kernel<W_MN, K>, dim3(n_out / (W_MN ? 32 : 16), 64), dim3(W_MN ? K / 2 : K / 4), 0, s, (const __half*)w,
+                    (const __half*)x, (__half*)out, n_rows, n_out, w_rows_per_head, w_row_off) == cudaSuccess
+             ? HK_OK
+             : HK_ERR_CUDA;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -400,6 +512,10 @@ static int absorb_rows(const void* x, const void* w, void* out, int n_rows, int 
 int absorb_gemm_tc(const void* a, const void* b, void* out, int n_rows, int K, int n_out, bool b_mn,
                    uint64_t b_rows, uint64_t b_cols, int b_rows_per_head, int b_row_off, cudaStream_t s) {
   if (!aligned(a, 16) || !aligned(b, 16) || !aligned(out, 16)) return HK_ERR_UNSUPPORTED;
+  if (n_rows <= A8_ROWS) {
+    if (K == 256 && b_mn) return absorb_8_rows<true, 256>(a, b, out, n_rows, n_out, b_rows_per_head, b_row_off, s);
+    if (K == 512 && !b_mn) return absorb_8_rows<false, 512>(a, b, out, n_rows, n_out, b_rows_per_head, b_row_off, s);
+  }
   if (n_rows <= AF_MAX_ROWS) {   // q_latent (K 256, n contiguous), o_absorb (K 512, k contiguous), o_absorb_t (K 512, n contiguous)
     if (K == 256 && b_mn) return absorb_few_rows<true, 256>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
     if (K == 512 && !b_mn) return absorb_few_rows<false, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
