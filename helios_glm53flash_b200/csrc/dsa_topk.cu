@@ -9,11 +9,13 @@
 // Radix select: a histogram of the top 11 key bits, one of the low 5 bits inside the crossing bucket, then a single ordered
 // compaction that places the "above" entries and the tie entries at once (the reference makes two histogram sweeps and two
 // compaction sweeps of global memory).  Three kernels:
-//   dsa_topk_rows_kernel      rows of up to 16,384 scores, read once into registers, a small CTA each
-//   dsa_topk_cluster_kernel   at most 16 longer rows of up to 262,144 scores, read once into the registers of a cluster of 8 CTAs
+//   dsa_topk_cluster_kernel   at most 16 rows of 4,096 to 262,144 scores, read once into the registers of a cluster of 8 or 16 CTAs
+//   dsa_topk_rows_kernel      other rows of up to 16,384 scores, read once into registers, a small CTA each
 //   dsa_topk_kernel           every other call (many long rows, lengths known on the device only): one CTA of 1,024 threads per
 //                             row, which sweeps the row three times; topk_row also selects among candidates in shared memory
 #include <cooperative_groups.h>
+
+#include <algorithm>
 
 #include "hk_common.cuh"
 
@@ -234,8 +236,8 @@ __global__ __launch_bounds__(TK_THREADS) void dsa_topk_kernel(
 // and small CTAs share an SM and hide one another's.  1,024 rows x 1,250 scores 19.3 -> 8.4 us, 1,024 x 4,096 20.3 -> 11.1,
 // 4,096 x 8,192 102 -> 66, 1,024 x 16,000 43.5 -> 36.4.  (More pieces per thread instead of more threads: 128 registers and
 // spills, 1,024 x 8,191 40.7 us; 1,024 threads for 32,000 scores: 83 us against 74.)
-// Up to a row per SM nothing is shared and the time is one CTA's: 1,024 threads with one or two pieces each, 1 x 5,000 scores
-// 7.3 -> 4.6 us, 1 x 16,000 8.2 -> 6.5, 140 x 8,000 7.3 -> 5.0.
+// Up to a row per SM nothing is shared and the time is one CTA's: 1,024 threads with one or two pieces each, 140 x 8,000 scores
+// 7.3 -> 5.0 us (up to 16 rows of more than 4,096 scores: clusters, below).
 // ------------------------------------------------------------------------------------------------
 constexpr int TKR_MAX_THREADS = 512, TKR_MAX_PIECES = 4 * TKR_MAX_THREADS;
 
@@ -366,24 +368,25 @@ __device__ long long hk_topk_trace[16];
 #define TK_TRACE(slot) do { } while (0)
 #endif
 // ------------------------------------------------------------------------------------------------
-// A few long rows (the decode case is ONE row): a thread-block cluster of 8 CTAs works on a row, CTA c on pieces
-// [1024 NP c, 1024 NP (c + 1)), every thread on NP consecutive pieces of 8 elements that stay in registers, so the row is
-// read from global memory once and no sweep is longer than 8 NP keys per thread.  The CTAs meet through distributed shared
-// memory: every CTA adds up the row's buckets by eights from all eight CTAs, then looks at the eight buckets of the crossing one; the
+// A few long rows (the decode case is ONE row): a thread-block cluster of 8 or 16 CTAs works on a row, every thread on NP consecutive
+// pieces of 8 elements that stay in registers, so the row is read from global memory once and no sweep is longer than 8 NP keys per
+// thread.  A CTA has as many threads as the row's pieces need in equal shares (256 to 1,024).  The CTAs meet through distributed shared
+// memory: every CTA adds up the row's buckets by eights from all CTAs, then looks at the eight buckets of the crossing one; the
 // low-bit count sets are read by every CTA, which finds the threshold and, from the per-CTA counts, the offset of its own
 // ordered output - two cluster barriers that hand data over and one that is arrived at long before it is waited for.
-// What bounds it: these steps one after the other (load and count 1.5 us, the crossing bucket 1.0, low bits 0.9, offsets 0.9, output 1.0).
-// One row of 65,536 scores 6.8 -> 5.8 us against sharing out the 2,048 sums by slices (four barriers); 262,000 scores 18.5 -> 11.8, 16 rows of
-// 30,000 13.9 -> 10.9 (the launch bound names the CTA per SM: at the 32 registers taken without it the four-piece form spilled).
-// NP = 1, 2, 4 cover rows of 65,536, 131,072 and 262,144 scores (1M tokens of context), up to seven fewer where a row starts off a 16-byte
-// boundary.
+// What bounds it: these steps one after the other (65,536 scores in eight CTAs: load and count 1.5 us, the crossing bucket 1.0, low bits 0.9,
+// offsets 0.9, output 1.0).  With 1,024 threads whatever the row's length the first CTAs had all of it, and a row of 65,552 scores two
+// pieces a thread in half of the CTAs.  One row, eight CTAs of 1,024 threads -> now, us: 5,000 scores 5.1 (one CTA) -> 4.5, 16,384 7.2 -> 4.2,
+// 32,768 5.8 -> 4.6, 65,536 5.75 -> 5.1, 65,552 8.0 -> 5.4, 131,072 7.4 -> 6.2, 200,000 11.9 -> 7.5; 16 rows of 20,000 11.1 -> 5.2.
+// (The launch bound names the CTA per SM: at the 32 registers taken without it the four-piece form spilled.)
+// Eight CTAs with NP = 1, 2, 4 cover rows of 65,536, 131,072 and 262,144 scores (1M tokens of context), up to seven fewer where a row starts
+// off a 16-byte boundary; sixteen with NP = 1, 2 the last two.
 // ------------------------------------------------------------------------------------------------
-constexpr int TKC_CTAS = 8;
-constexpr int TKC_PIECES = TKC_CTAS * TK_THREADS;         // pieces of 8 elements that NP = 1 holds
+constexpr int TKC_PIECES = 8 * TK_THREADS;                // pieces of 8 elements that eight CTAs hold with NP = 1
 constexpr int TKC_MAX_NP = 4;
 
-template <int NP>
-__global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) void dsa_topk_cluster_kernel(
+template <int NP, int CTAS>
+__global__ __launch_bounds__(TK_THREADS, 1) void dsa_topk_cluster_kernel(
     const uint16_t* scores, int* __restrict__ out, int T, int s_stride, int k, int k_pad,
     int* __restrict__ raw, const int* __restrict__ q_pos) {
   __shared__ __align__(16) int hist[2048];   // this CTA's bucket counts
@@ -392,8 +395,8 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) voi
   __shared__ int wsum[2][TK_WARPS];
   __shared__ int sh_sel[3];
   __shared__ int sh_off[6];        // threshold low bits, count above threshold, this CTA's bases, total ties
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  for (int i = t; i < 2048; i += TK_THREADS) hist[i] = 0;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, threads = blockDim.x, warps = threads >> 5;
+  for (int i = t; i < 2048; i += threads) hist[i] = 0;
   if (t < 33) low[t] = 0;
   if (t == 0) sh_sel[0] = -1;
   namespace cg = cooperative_groups;
@@ -401,13 +404,13 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) voi
   pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int c = (int)cluster.block_rank();
-  const int row_id = blockIdx.x / TKC_CTAS;
+  const int row_id = blockIdx.x / CTAS;
   const uint16_t* row = scores + (size_t)row_id * s_stride;
   const TopkSink row_o{out + (size_t)row_id * k_pad,
                        raw ? reinterpret_cast<int4*>(raw + (size_t)row_id * (4 * k_pad + 4)) : nullptr, raw ? q_pos[row_id] : 0};
 
   TK_TRACE(0);
-  const int lead = row_lead(row), i8 = (c * TK_THREADS + t) * NP;
+  const int lead = row_lead(row), i8 = (c * threads + t) * NP;
   uint4 pc[NP];
 #pragma unroll
   for (int u = 0; u < NP; u++) pc[u] = load8_raw(row, lead, i8 + u, T);
@@ -422,7 +425,7 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) voi
     }
     if (lane == 31) wsum[slot][warp] = incl;
     __syncthreads();
-    const int x = wsum[slot][lane];
+    const int x = lane < warps ? wsum[slot][lane] : 0;
     const int before = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < warp ? x : 0));
     *total = (int)__reduce_add_sync(0xffffffffu, (unsigned)x);
     return before + incl - v;
@@ -442,16 +445,18 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) voi
   int sum = 0;
   if (t < 256) {
 #pragma unroll
-    for (int rk = 0; rk < TKC_CTAS; rk++) sum += cluster.map_shared_rank(coarse, rk)[255 - t];
+    for (int rk = 0; rk < CTAS; rk++) sum += cluster.map_shared_rank(coarse, rk)[255 - t];
   }
   int total_sel;
   const int excl = exscan(sum, 0, &total_sel);
   if (k > 0 && excl < k && excl + sum >= k) { sh_sel[0] = 255 - t; sh_sel[1] = excl; }
   __syncthreads();
   if (warp == 0 && sh_sel[0] >= 0) {
-    // lane 8 r + j: bucket j from the top of the eight, CTAs r and r + 4
+    // lane 8 r + j: bucket j from the top of the eight, CTAs r, r + 4, ...
     const int bin = 8 * sh_sel[0] + 7 - (lane & 7), above = sh_sel[1];
-    int v = cluster.map_shared_rank(hist, lane >> 3)[bin] + cluster.map_shared_rank(hist, (lane >> 3) + 4)[bin];
+    int v = 0;
+#pragma unroll
+    for (int rk = 0; rk < CTAS; rk += 4) v += cluster.map_shared_rank(hist, (lane >> 3) + rk)[bin];
     v += __shfl_xor_sync(0xffffffffu, v, 8);
     v += __shfl_xor_sync(0xffffffffu, v, 16);
     int incl = v;
@@ -480,15 +485,15 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) voi
   cluster.sync();                  // (2) all local low-bit counts complete
   TK_TRACE(3);
   if (warp == 0) {
-    // lane l owns low value 31-l (descending); per CTA counts first, then the row's
-    int mine[TKC_CTAS], above_c[TKC_CTAS], g = 0;
+    // lane l owns low value 31-l (descending): the row's count and that of the CTAs before this one; lane rk also keys above the bucket
+    int g = 0, before = 0;
 #pragma unroll
-    for (int rk = 0; rk < TKC_CTAS; rk++) {
-      const int* rl = cluster.map_shared_rank(low, rk);
-      mine[rk] = rl[31 - lane];
-      above_c[rk] = rl[32];
-      g += mine[rk];
+    for (int rk = 0; rk < CTAS; rk++) {
+      const int mine = cluster.map_shared_rank(low, rk)[31 - lane];
+      g += mine;
+      if (rk < c) before += mine;
     }
+    const int above_before = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < c ? cluster.map_shared_rank(low, lane)[32] : 0));
     int lowbits = 0, cnt_gt_row = k > 0 ? total_sel : 0, need_eq = 0;
     if (b1 >= 0) {
       int incl = g;
@@ -503,22 +508,12 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) voi
       lowbits = 31 - src;
       cnt_gt_row = above1 + __shfl_sync(0xffffffffu, incl - g, src);
       need_eq = k - cnt_gt_row;
-      // per CTA: keys above the threshold = above the bucket + low values above lowbits (lanes < src); ties = lane src
-      int base_gt = 0, base_eq = 0, all_eq = 0;
-#pragma unroll
-      for (int rk = 0; rk < TKC_CTAS; rk++) {
-        const int hi = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < src ? mine[rk] : 0));
-        const int eq = __shfl_sync(0xffffffffu, mine[rk], src);
-        if (rk < c) { base_gt += above_c[rk] + hi; base_eq += eq; }
-        all_eq += eq;
-      }
+      // keys above the threshold = above the bucket + low values above lowbits (lanes < src); ties = lane src
+      const int base_gt = above_before + (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < src ? before : 0));
+      const int base_eq = __shfl_sync(0xffffffffu, before, src), all_eq = __shfl_sync(0xffffffffu, g, src);
       if (lane == 0) { sh_off[2] = base_gt; sh_off[3] = base_eq; sh_off[4] = all_eq; }
-    } else {
-      int base_gt = 0;
-#pragma unroll
-      for (int rk = 0; rk < TKC_CTAS; rk++)
-        if (rk < c) base_gt += above_c[rk];
-      if (lane == 0) { sh_off[2] = k > 0 ? base_gt : 0; sh_off[3] = 0; sh_off[4] = 0; }
+    } else if (lane == 0) {
+      sh_off[2] = k > 0 ? above_before : 0; sh_off[3] = 0; sh_off[4] = 0;
     }
     if (lane == 0) { sh_off[0] = lowbits; sh_off[1] = cnt_gt_row; sh_off[5] = need_eq; }
   }
@@ -555,7 +550,7 @@ __global__ __cluster_dims__(TKC_CTAS, 1, 1) __launch_bounds__(TK_THREADS, 1) voi
   }
   if (c == 0) {
     const int emitted = cnt_gt + min(sh_off[4], n_eq_take);
-    for (int j = emitted + t; j < k_pad; j += TK_THREADS) row_o.put(j, -1);
+    for (int j = emitted + t; j < k_pad; j += threads) row_o.put(j, -1);
     if (t == 0) row_o.put_tail(k_pad);
   }
   TK_TRACE(6);
@@ -571,6 +566,32 @@ extern "C" __attribute__((visibility("default"))) int hk_debug_topk_trace(long l
 #endif
 
 namespace hk {
+// clusters of sixteen CTAs of 1,024 threads that run at once; 0 where such clusters cannot be had
+static int wide_clusters() {
+  static int room[64] = {0};                                // + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (!room[dev]) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(TK_THREADS);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(dsa_topk_cluster_kernel<1, 16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(dsa_topk_cluster_kernel<2, 16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, dsa_topk_cluster_kernel<2, 16>, &cfg) != cudaSuccess) {
+      cudaGetLastError();                                   // (no such clusters: not an error of the call)
+      n = 0;
+    }
+    room[dev] = n + 1;
+  }
+  return room[dev] - 1;
+}
 // common launcher; raw != nullptr adds the expansion
 static int topk_launch(const void* scores, int s_stride, int* indices, int R, int T, int k, int k_pad, const int* t_ptr,
                        int t_seq, int* raw, const int* q_pos, cudaStream_t s) {
@@ -581,18 +602,29 @@ static int topk_launch(const void* scores, int s_stride, int* indices, int R, in
   auto rows = [&](auto kern, int threads) {
     return pdl_launch(kern, dim3(R), dim3(threads), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
   };
-  auto cluster = [&](auto kern) {
-    return pdl_launch(kern, dim3(R * TKC_CTAS), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, raw, q_pos);
+  auto cluster = [&](auto kern, int np, int ctas) {         // the pieces in equal shares for all threads
+    const int threads = (int)((pieces + ctas * np * 32 - 1) / (ctas * np * 32)) * 32;
+    return pdl_launch_cluster(ctas, kern, dim3(R * ctas), dim3(threads < 256 ? 256 : threads), 0, s, sc, indices, T, s_stride, k, k_pad, raw,
+                              q_pos);
   };
   auto sweeps = [&]() {
     return pdl_launch(dsa_topk_kernel, dim3(R), dim3(TK_THREADS), 0, s, sc, indices, T, s_stride, k, k_pad, t_ptr, t_seq, raw, q_pos);
   };
   // (figures at the kernels.  With many rows the clusters queue for eight free SMs of one GPC each and the one-CTA kernel is 3 to 20
-  // times faster, measured at 64 to 4,096 rows; up to 16,384 scores one CTA is as fast as the cluster even for a single row)
+  // times faster, measured at 64 to 4,096 rows.  Up to 4,096 scores one CTA is faster than the cluster: 1 x 2,500 4.1 / 4.6 us, 1 x 5,000
+  // 5.1 / 4.5.  Sixteen CTAs a row: from 40,000 scores for up to 3 rows (1 x 33,000 4.8 with eight / 5.0, 1 x 50,000 5.3 / 5.1, 4 x 50,000
+  // 5.4 / 5.8), beyond 65,536 scores, where eight take two pieces a thread, for as many rows as there is room for at once: 7 x 65,552
+  // 6.7 / 5.5, 8 x 65,552 6.5 / 10.6)
   cudaError_t e;
   if (t_ptr) e = sweeps();
   else if (pieces <= 256) e = rows(dsa_topk_rows_kernel<1, 256>, 256);
-  else if (pieces <= TKR_MAX_PIECES && R <= sm_count())      // a row per SM: as many threads as there are pieces, up to 1,024
+  else if (pieces > 512 && pieces <= (int64_t)TKC_PIECES * TKC_MAX_NP && R <= 16) {
+    const bool wide = pieces > 5120 && R <= (pieces <= TKC_PIECES ? std::min(3, wide_clusters()) : wide_clusters());
+    e = wide ? (pieces <= 2 * TKC_PIECES ? cluster(dsa_topk_cluster_kernel<1, 16>, 1, 16) : cluster(dsa_topk_cluster_kernel<2, 16>, 2, 16))
+        : pieces <= TKC_PIECES     ? cluster(dsa_topk_cluster_kernel<1, 8>, 1, 8)
+        : pieces <= 2 * TKC_PIECES ? cluster(dsa_topk_cluster_kernel<2, 8>, 2, 8)
+                                   : cluster(dsa_topk_cluster_kernel<4, 8>, 4, 8);
+  } else if (pieces <= TKR_MAX_PIECES && R <= sm_count())    // a row per SM: as many threads as there are pieces, up to 1,024
     e = pieces <= 512    ? rows(dsa_topk_rows_kernel<1, 512>, 512)
         : pieces <= 1024 ? rows(dsa_topk_rows_kernel<1, 1024>, 1024)
                          : rows(dsa_topk_rows_kernel<2, 1024>, 1024);
@@ -600,10 +632,6 @@ static int topk_launch(const void* scores, int s_stride, int* indices, int R, in
     e = pieces <= 512    ? rows(dsa_topk_rows_kernel<2, 256>, 256)
         : pieces <= 1024 ? rows(dsa_topk_rows_kernel<4, 256>, 256)
                          : rows(dsa_topk_rows_kernel<4, 0>, (int)((pieces + 127) / 128) * 32);
-  else if (R <= 16 && T > 16384 && pieces <= (int64_t)TKC_PIECES * TKC_MAX_NP)
-    e = pieces <= TKC_PIECES       ? cluster(dsa_topk_cluster_kernel<1>)
-        : pieces <= 2 * TKC_PIECES ? cluster(dsa_topk_cluster_kernel<2>)
-                                   : cluster(dsa_topk_cluster_kernel<4>);
   else e = sweeps();
   return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }

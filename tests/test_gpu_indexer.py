@@ -171,6 +171,21 @@ def test_topk_at_the_edges_of_its_row_forms(R, T, stride_pad, offset):
     assert np.array_equal(got, orc.dsa_topk(scb, T + stride_pad, R, T, 512, 512))
 
 
+@pytest.mark.parametrize("R,T,stride_pad,offset", [(16, 4097, 7, 0), (17, 4097, 7, 0), (1, 4096, 0, 1), (3, 40961, 7, 0), (4, 40961, 7, 0),
+                                                    (3, 65536, 0, 0), (4, 65536, 0, 0), (7, 65537, 7, 0), (8, 65537, 7, 0), (3, 131080, 0, 0)])
+def test_topk_where_the_number_of_ctas_a_row_changes(R, T, stride_pad, offset):
+    """one CTA, clusters of eight and of sixteen; a row of one repeated score, a row with fewer than k scores, ties across the CTAs' shares"""
+    r = synth.rng(R + T)
+    sc = np.round(r.standard_normal((R, T + stride_pad), dtype=np.float32) * 4) / 4
+    sc[0, :] = 1.5
+    if R > 1:
+        sc[1, :] = -np.inf
+        sc[1, np.linspace(0, T - 1, 300).astype(int)] = 2.0
+    scb = synth.f32_to_f16_bits(sc)
+    got = _topk_gpu(scb, T + stride_pad, R, T, 512, 512, offset=offset)
+    assert np.array_equal(got, orc.dsa_topk(scb, T + stride_pad, R, T, 512, 512))
+
+
 def test_topk_selects_the_true_top_k():
     """independent of the oracle: the selection is a true top-k, above-threshold entries come out in
     ascending index order followed by the threshold ties in ascending index order"""
