@@ -24,10 +24,12 @@
 // -> 4.19e-4 / 2.94e-4 -> 2.94e-4; no decay 5.2 -> 5.1e-4 / 4.6 -> 4.4e-4; e^-8 and e^-12 a block, values in a chunk's first block only, beta
 // 1e-6 behind it, keys nearly alike: every ratio within 0.993 and 1.003, the spread of the seeds.
 //   What bounds it: latencies.  A unit crosses five barriers of its 256 threads and one product; two units share an SM (128 registers
-//   a thread, 109 KB).  Inputs arrive by tensor copies issued while the unit before is finished.  A worker's unit takes 22-24 thousand
-//   cycles with two workers on the SM, 39 thousand in the form before (k and q rows in separate warps, TF32 for all block pairs,
-//   13 barriers, loads through registers); 32,768 tokens x 32 heads 1.43 -> 1.02 ms, with gates formed inside 1.62 -> 1.09 (0.90 and 0.98
-//   with the chain of today).
+//   a thread, 110 KB).  Inputs arrive by tensor copies issued as soon as their place is free (the log decays when half of the unit before
+//   is over).  A worker's unit takes 20 thousand cycles with two workers on the SM.  It took 22.8 thousand while a warp's accesses met in
+//   the same banks (log decays two channels a lane, q and k in 128-byte rows, operand tiles of 8-row pieces: 2,300 of the 7,650 passes of a
+//   unit through shared memory and L1 were conflicts, now 700 of 6,100), W left as 16-byte halves of sectors, the flag was stored between
+//   two barriers that all wait for, and log decays arrived 1,500 cycles into the unit.  32,768 tokens x 32 heads 0.90 -> 0.80 ms, 8 x 4,096 x
+//   32 with gates formed inside 0.95 -> 0.88.
 //   Registers decide: everything a thread keeps across stage 2 is the 32 packed left operands; a version that kept the fp32 rows (300
 //   bytes of spills, whose reloads miss the L1 that shared memory leaves) took 30 thousand cycles.
 // The scan walks the chunks of a chain in order; the fp32 state stays in registers.  Per chunk: D1 = [I ; 0] Uloc + [-W ; Q+] S0 (rows
@@ -57,16 +59,21 @@ constexpr int F_FLAG_INTS = 32;
 constexpr int F_LINE = 32;
 
 // ---- per-chunk workspace unit (bytes); every tile is in its final shared-memory layout ----
-constexpr uint32_t U_WQ = 0;              // fp16 A operand, K-major, rows 0-63 -W, 64-127 Q+ ; K = 128 channels
+// (the two operands that the preparation writes from its token rows are in 64-byte-swizzle atoms of 8 tokens x 32 channels: a warp's
+// store is one atom, every quarter of it 128 contiguous bytes)
+constexpr uint32_t U_WQ = 0;              // fp16 A operand, K-major, rows 0-63 -W, 64-127 Q+ ; K = 128 channels: [16 x 8 rows][4 x 32 channels] atoms
 constexpr uint32_t U_UL = 32768;          // fp16 Uloc as B operand, MN-major [16 pieces of 8 columns][64 tokens], token t at t ^ 8
 constexpr uint32_t U_BB = 49152;          // fp16 A operand rows (t), K = 64 (s): B_ts beta_s
-constexpr uint32_t U_KT = 57344;          // fp16 A operand rows = 128 channels, K = 64 tokens: Kt^T, MN-major (8 channels of a token per piece)
+constexpr uint32_t U_KT = 57344;          // fp16 A operand rows = 128 channels, K = 64 tokens: Kt^T, MN-major: [4 x 32 channels][8 atoms]
 constexpr uint32_t U_DEC = 73728;         // f32 e^{G_last}[128]
 constexpr uint32_t U_BYTES = 74240;
 
-// K-major tile with K = 128 (16 chunks): LBO 128, SBO 2048; with K = 64 (8 chunks): LBO 128, SBO 1024
+constexpr uint32_t ATOM = 512;            // bytes of an atom
+constexpr uint32_t WQ_ROWS = 4 * ATOM, KT_BLK = 8 * ATOM;   // eight rows of WQ; 32 channels of Kt^T
+__device__ __forceinline__ uint32_t atom_off(int r, int c) { return (uint32_t)(r & 7) * 64 + (uint32_t)((c ^ (r >> 1)) & 3) * 16; }   // chunk c of row r
+
+// K-major tile with K = 64 (8 chunks) and no swizzle: LBO 128, SBO 1024
 constexpr uint32_t LBO = 128;
-constexpr uint32_t SBO_K128 = 2048;
 constexpr uint32_t SBO_K64 = 1024;
 
 __device__ __forceinline__ uint32_t f2tf32(float x) {
@@ -129,7 +136,7 @@ __device__ __forceinline__ bool poll_flag_ge(const int* flag, int want, volatile
 }
 
 // =================================================================================================
-// kernel 1: per-chunk preparation.  256 threads, 109 KB of shared memory: two CTAs per SM, so the
+// kernel 1: per-chunk preparation.  256 threads, 110 KB of shared memory: two CTAs per SM, so the
 // serial stages of one chunk overlap with another chunk's.
 // =================================================================================================
 // Warp w owns tokens 8 w .. 8 w + 7: lane 4 g8 + tig holds, of token 8 w + g8, the eight channels from 8 tig of every 32, of the
@@ -140,15 +147,16 @@ __device__ __forceinline__ bool poll_flag_ge(const int* flag, int want, volatile
 constexpr uint32_t P1_PIECE = 1056;                      // bytes between the 8-channel pieces of K+ (1024 + 32: the four pieces that a
                                                          // quarter-warp writes start in different banks)
 constexpr uint32_t P1_X = 0;                             // f32 log decays, then their sums x: four boxes [64 tokens][32 channels]; then the
-                                                         // right operands of the even warps' tokens, then the inverses of the diagonal blocks
+                                                         // right operands of the even warps' tokens, then the next unit's log decays
 constexpr uint32_t P1_V = 32768;                         // v: two boxes [64 tokens][64 channels], bf16 as loaded, fp16 in place: the B operand
 constexpr uint32_t P1_RI = 49152;                        // fp16 right operands of the block pairs (i, j < i), 16 tokens x 256 B each;
                                                          // later the T operand (8 KB)
 constexpr uint32_t P1_N = P1_RI + 6 * 4096;              // f32 N = A beta: rows 0-31 at a pitch of 36, rows 32-63 at 68
-constexpr uint32_t P1_QK = P1_RI;                        // the next unit's q and k: two boxes each, over the two regions before
-constexpr uint32_t P1_K = P1_N + 32 * (36 + 68) * 4;     // fp16 K+, B operand, MN-major, 16 pieces
-constexpr uint32_t P1_TAB = P1_K + 16 * P1_PIECE;        // f32 tables [15][128]
-constexpr uint32_t P1_SMEM = P1_TAB + 15 * 512;
+constexpr uint32_t P1_QK = P1_RI;                        // the next unit's q and k, [4 x 32 channels][64 tokens][64 B] each, over the two regions before
+constexpr uint32_t P1_K = P1_N + 32 * (36 + 68) * 4;     // fp16 K+, B operand, MN-major, 16 pieces; behind its product W, as it leaves
+constexpr uint32_t P1_TAB = P1_K + 16 * P1_PIECE;        // f32 tables [15][128 + 16], then the inverses of the diagonal blocks
+constexpr int TAB_LD = KD + 16;                          // (blocks J and J + 1 start in different halves of the banks)
+constexpr uint32_t P1_SMEM = (P1_TAB + 15 * TAB_LD * 4 + 1023) / 1024 * 1024;
 constexpr int TAB_EP = 0, TAB_ETOT = 4, TAB_KE = 8, TAB_F = 12;   // rows: e^{P_J} | e^{tot_J} | e^{G_last - P_{J+1}} | (2,0), (3,1), (3,0)
 static_assert(P1_SMEM % 1024 == 0 && P1_QK % 1024 == 0 && P1_QK + 32768 <= P1_K && P1_TAB % 16 == 0, "layout");
 constexpr uint32_t P1_BOX = 8192;
@@ -181,28 +189,6 @@ struct Frag16 {
     }
   }
 };
-// acc += L R, R fp32 in shared memory.  Both operands are split into a TF32 head and tail and the three significant partial
-// products are accumulated in fp32 (in sums of their own: shorter chains), which keeps the result at fp32-class accuracy.
-__device__ __forceinline__ void block16_mma(const Frag16& L, const float* __restrict__ R, int ld, float (&acc)[2][4], int lane) {
-  const int g8 = lane >> 2, tig = lane & 3;
-  float lo[2][2][4];
-#pragma unroll
-  for (int e = 0; e < 16; e++) lo[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
-#pragma unroll
-  for (int ks = 0; ks < 2; ks++)
-#pragma unroll
-    for (int nt = 0; nt < 2; nt++) {
-      const float b0 = R[(8 * ks + 2 * tig) * ld + 8 * nt + g8], b1 = R[(8 * ks + 2 * tig + 1) * ld + 8 * nt + g8];
-      const uint32_t b0h = f2tf32(b0), b1h = f2tf32(b1);
-      const uint32_t b0l = f2tf32(b0 - __uint_as_float(b0h)), b1l = f2tf32(b1 - __uint_as_float(b1h));
-      mma_tf32(lo[0][nt], L.l[ks], b0h, b1h);
-      mma_tf32(lo[1][nt], L.h[ks], b0l, b1l);
-      mma_tf32(acc[nt], L.h[ks], b0h, b1h);
-    }
-#pragma unroll
-  for (int e = 0; e < 8; e++) acc[e >> 2][e & 3] += lo[0][e >> 2][e & 3] + lo[1][e >> 2][e & 3];
-}
-
 // two fp32 values of a register pair -> fp16 pair
 __device__ __forceinline__ uint32_t pack_h2(uint64_t v) {
   float a, b;
@@ -226,6 +212,47 @@ __device__ __forceinline__ void mma_f16_16816(float (&c)[4], uint32_t a0, uint32
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Right operand of a block product (16 x 16, fp32 in shared memory) as TF32 heads and tails
+struct Right16 {
+  uint32_t h[2][2][2], l[2][2][2];                         // [k step][column half][k slot]
+  __device__ __forceinline__ void load(const float* __restrict__ R, int ld, int lane) {
+    const int g8 = lane >> 2, tig = lane & 3;
+#pragma unroll
+    for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+      for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const float b = R[(8 * ks + 2 * tig + u) * ld + 8 * nt + g8];
+          h[ks][nt][u] = f2tf32(b);
+          l[ks][nt][u] = f2tf32(b - __uint_as_float(h[ks][nt][u]));
+        }
+  }
+};
+// acc += L R: the three significant partial products, accumulated in fp32 (in sums of their own: shorter chains), which keeps the
+// result at fp32-class accuracy
+__device__ __forceinline__ void block16_mma(const Frag16& L, const Right16& R, float (&acc)[2][4]) {
+  float lo[2][2][4];
+#pragma unroll
+  for (int e = 0; e < 16; e++) lo[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+    for (int nt = 0; nt < 2; nt++) {
+      mma_tf32(lo[0][nt], L.l[ks], R.h[ks][nt][0], R.h[ks][nt][1]);
+      mma_tf32(lo[1][nt], L.h[ks], R.l[ks][nt][0], R.l[ks][nt][1]);
+      mma_tf32(acc[nt], L.h[ks], R.h[ks][nt][0], R.h[ks][nt][1]);
+    }
+#pragma unroll
+  for (int e = 0; e < 8; e++) acc[e >> 2][e & 3] += lo[0][e >> 2][e & 3] + lo[1][e >> 2][e & 3];
+}
+
+__device__ __forceinline__ void block16_mma(const Frag16& L, const float* __restrict__ R, int ld, float (&acc)[2][4], int lane) {
+  Right16 r;
+  r.load(R, ld, lane);
+  block16_mma(L, r, acc);
 }
 
 // Row block i of the inverse, right to left: X_ij = - sum_{m = j+1}^{i} X_im P_mj, P_mj = N_mj X_jj (in place of N_mj), one warp,
@@ -254,6 +281,57 @@ __device__ __forceinline__ void prep_inverse_row(const float* __restrict__ sN, c
       *reinterpret_cast<uint32_t*>(p) = pack_h2(f[0], f[1]);
       *reinterpret_cast<uint32_t*>(p + SBO_K64) = pack_h2(f[2], f[3]);
     }
+  }
+}
+
+// The same with a warp a block: the blocks of the second diagonal need those of the first, X_30 needs X_31 as well.  What a block needs of
+// the diagonal it forms ahead, and its other right operands are in registers before the left ones are there, so that one product stands
+// behind each of the two barriers (six warps).  What a later block needs goes to shared memory as fp32, in place of N's diagonal
+// blocks, which are inverted already; all go to T as fp16.  The shorter way with more instructions: the two-kernel form, whose CTAs are in
+// step with one another, gains (1,003 tokens x 32 heads, all calls of the layer: 81.7 -> 76.9 us); where other units fill the gaps it loses
+// (fused launch, 8 x 4,096 x 32: 1,455 -> 1,487).
+__device__ __forceinline__ void prep_inverse_blocks(float* __restrict__ sN, const float* __restrict__ sX, uint8_t* __restrict__ sT, int warp, int lane, int bar) {
+  const int g8 = lane >> 2, tig = lane & 3;
+  auto P = [&](int m, int j) { return sN + prep_n_row(16 * m) + 16 * j; };
+  auto ldn = [](int m) { return m < 2 ? 36 : 68; };
+  // warp: 0 X_10, 1 X_21, 2 X_32, 3 X_20, 4 X_31, 5 X_30
+  const int i = warp < 3 ? warp + 1 : warp == 3 ? 2 : 3, j = warp < 3 ? warp : warp == 4 ? 1 : 0;
+  float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+  Frag16 L;
+  Right16 R;
+  auto put = [&](int keep) {                               // keep: the diagonal block whose place it takes, 0 = none
+#pragma unroll
+    for (int nt = 0; nt < 2; nt++) {
+      const float f[4] = {-acc[nt][0], -acc[nt][1], -acc[nt][2], -acc[nt][3]};
+      if (keep) {
+        float* x = sN + prep_n_row(16 * keep) + 16 * keep + 8 * nt + 2 * tig;
+        *reinterpret_cast<float2*>(x + g8 * ldn(keep)) = make_float2(f[0], f[1]);
+        *reinterpret_cast<float2*>(x + (g8 + 8) * ldn(keep)) = make_float2(f[2], f[3]);
+      }
+      uint8_t* p = sT + (2 * i) * SBO_K64 + (2 * j + nt) * LBO + g8 * 16 + tig * 4;
+      *reinterpret_cast<uint32_t*>(p) = pack_h2(f[0], f[1]);
+      *reinterpret_cast<uint32_t*>(p + SBO_K64) = pack_h2(f[2], f[3]);
+    }
+  };
+  L.load(sX + prep_inv_at(i), P1_LDX, lane);
+  R.load(P(i, j), ldn(i), lane);
+  block16_mma(L, R, acc);                                  // X_ii P_ij
+  if (warp < 3) put(warp == 0 ? 0 : warp + 1);             // X_21, X_32
+  else if (warp == 4) R.load(P(2, 1), ldn(2), lane);
+  else R.load(warp == 3 ? P(1, 0) : P(2, 0), ldn(warp == 3 ? 1 : 2), lane);
+  asm volatile("bar.sync %0, 192;" ::"r"(bar) : "memory");
+  if (warp >= 3) {
+    L.load(P(warp == 3 ? 2 : 3, warp == 3 ? 2 : 3), 68, lane);   // X_21 P_10, X_32 P_21, X_32 P_20
+    block16_mma(L, R, acc);
+    if (warp == 5) R.load(P(1, 0), ldn(1), lane);
+    else put(warp == 4 ? 1 : 0);                           // X_31
+  }
+  if (warp < 4) return;
+  asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+  if (warp == 5) {
+    L.load(P(1, 1), 36, lane);                             // X_31 P_10
+    block16_mma(L, R, acc);
+    put(0);
   }
 }
 
@@ -298,24 +376,44 @@ __device__ __forceinline__ void prep_init(PrepShared& sh) {  // one thread
 #define PREP_UNIT(field, it) (*const_cast<volatile int*>(&ctx.sh->unit[(it) & 3].field))
 
 // Fused form: stores the ready flag of unit `it`.  Called by one warp, which meets the others behind the unit's last writes here; the
-// release store is cumulative over them.  It waits until the CTA's stores are visible, some thousand cycles when they are fresh: it is
-// put off to a place in the next unit where its warp has little else to do, unless the worker has to wait for its ring slot.
-constexpr int PUB_WARP = 2;
+// release store is cumulative over them.  It waits until the CTA's stores are visible, 1,000 cycles: it is put off to a place in the next
+// unit where its warp has nothing else to do, unless the worker has to wait for its ring slot.
+constexpr int PUB_WARP = 7;
+constexpr int FETCH_TID = 192;                            // works out the units and asks for q, k and v
 __device__ __forceinline__ void prep_publish(const PrepCtx& ctx, int it, int* ready, int kr) {
   asm volatile("bar.sync %0, 256;" ::"r"(ctx.bar_id + 2) : "memory");
   if (ctx.tid == PUB_WARP * 32) {
+    tc::bulk_wait_all<0>();                                // its copy of W, by this thread, is complete
     const int value = PREP_UNIT(value, it);
     st_release_gpu(ready + (size_t)PREP_UNIT(slot, it) * F_LINE + ((value - 1) & (kr - 1)), value);
   }
 }
 
-// Tensor maps of the inputs: qkv as [batch][token][3 H 128] bf16, box 64 tokens x 64 channels; g (or f) as [batch][token][H 128] f32,
-// box 64 tokens x 32 channels; 128-byte swizzle, tokens past the end read as zeros.
+// Tensor maps of the inputs, tokens past the end read as zeros: qkv as [batch][token][3 H 128] bf16, box 64 tokens x 64 channels (v), and
+// as [batch][32 channels of 3 H 128][token] with 64-byte rows, box 4 x 64 tokens (q and k: in 128-byte rows two of the eight tokens that a
+// quarter-warp reads met in the same banks); g (or f) as [batch][token][H 128] f32, box 64 tokens x 32 channels.  128-byte swizzle for v and g.
 __device__ __forceinline__ void prep_tma(uint8_t* dst, const CUtensorMap* map, int c, int t, int b, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(tc::smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(t), "r"(b), "r"(tc::smem_u32(bar))
       : "memory");
+}
+__device__ __forceinline__ void prep_tma_rows(uint8_t* dst, const CUtensorMap* map, int c32, int t, int b, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(tc::smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(t), "r"(c32), "r"(b), "r"(tc::smem_u32(bar))
+      : "memory");
+}
+// asks for the next unit's q, k and v rows in L2 (their place is free when most of this unit is over; from HBM they then took longer than
+// what was left to do)
+__device__ __forceinline__ void prep_prefetch_qkv(const PrepCtx& ctx, int it, const CUtensorMap* map_qkv, int H) {
+  if (PREP_UNIT(n_valid, it) == 0) return;
+  const int c = PREP_UNIT(head, it) * KD, t0 = PREP_UNIT(t0, it), b = PREP_UNIT(b, it);
+#pragma unroll
+  for (int i = 0; i < 6; i++)
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map_qkv)),
+                 "r"((i >> 1) * H * KD + c + 64 * (i & 1)), "r"(t0), "r"(b)
+                 : "memory");
 }
 // the next unit's inputs, each as soon as its place is free (one thread)
 __device__ __forceinline__ void prep_fetch_g(const PrepCtx& ctx, int it, const CUtensorMap* map_g) {
@@ -325,15 +423,12 @@ __device__ __forceinline__ void prep_fetch_g(const PrepCtx& ctx, int it, const C
 #pragma unroll
   for (int m = 0; m < 4; m++) prep_tma(ctx.smem + P1_X + m * P1_BOX, map_g, c + 32 * m, t0, b, &ctx.sh->g_bar);
 }
-__device__ __forceinline__ void prep_fetch_qkv(const PrepCtx& ctx, int it, const CUtensorMap* map_qkv, int H) {
+__device__ __forceinline__ void prep_fetch_qkv(const PrepCtx& ctx, int it, const CUtensorMap* map_qkv, const CUtensorMap* map_qk, int H) {
   if (PREP_UNIT(n_valid, it) == 0) return;
   const int c = PREP_UNIT(head, it) * KD, t0 = PREP_UNIT(t0, it), b = PREP_UNIT(b, it);
   tc::mbar_arrive_expect_tx(&ctx.sh->qkv_bar, 6 * P1_BOX);
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    prep_tma(ctx.smem + P1_QK + (2 + h) * P1_BOX, map_qkv, H * KD + c + 64 * h, t0, b, &ctx.sh->qkv_bar);
-    prep_tma(ctx.smem + P1_QK + h * P1_BOX, map_qkv, c + 64 * h, t0, b, &ctx.sh->qkv_bar);
-  }
+  prep_tma_rows(ctx.smem + P1_QK + 2 * P1_BOX, map_qk, (H * KD + c) / 32, t0, b, &ctx.sh->qkv_bar);
+  prep_tma_rows(ctx.smem + P1_QK, map_qk, c / 32, t0, b, &ctx.sh->qkv_bar);
 #pragma unroll
   for (int h = 0; h < 2; h++) prep_tma(ctx.smem + P1_V + h * P1_BOX, map_qkv, 2 * H * KD + c + 64 * h, t0, b, &ctx.sh->qkv_bar);
 }
@@ -346,16 +441,16 @@ __device__ __forceinline__ void prep_fetch_qkv(const PrepCtx& ctx, int it, const
 // The unit's inputs are on their way (prep_fetch_*); its end sends for those of the next.
 // SLICES: chain CTAs of a slot in the fused form (SUB), 0 in the two-kernel form.  SUB: `ready` and `consumed` are the flags
 // of the ring; on return the unit's last writes are on their way and its flag is still to be stored (prep_publish).
-// `make_unit(it, desc)` works out the next unit (one thread).
+// `make_unit(it, desc)` works out a unit (one thread; two ahead, its divisions beside the inverse).
 template <bool GATED, int SLICES, class MakeUnit>
 __device__ __forceinline__ void prep_unit(
-    const PrepCtx& ctx, const int it, const CUtensorMap* map_qkv, const CUtensorMap* map_g, const void* __restrict__ beta_in,
+    const PrepCtx& ctx, const int it, const CUtensorMap* map_qkv, const CUtensorMap* map_qk, const CUtensorMap* map_g, const void* __restrict__ beta_in,
     uint8_t* __restrict__ units, int H, const float* __restrict__ dt_bias, const float* __restrict__ a_log, float lower_bound,
     const uint32_t tmem, int* ready, const int* consumed, int* g_abort, int kr, MakeUnit&& make_unit) {
   constexpr bool SUB = SLICES > 0;
   uint8_t* const smem = ctx.smem;
   uint8_t* const sK = smem + P1_K;
-  float* const sX = reinterpret_cast<float*>(smem + P1_X);
+  float* const sX = reinterpret_cast<float*>(smem + P1_TAB);
   uint8_t* const sRI = smem + P1_RI;
   uint8_t* const sT = smem + P1_RI;
   float* const sN = reinterpret_cast<float*>(smem + P1_N);
@@ -370,9 +465,10 @@ __device__ __forceinline__ void prep_unit(
   const int t = 8 * warp + g8;                             // this lane's token
 #define PREP_OUT (units + (size_t)PREP_UNIT(unit, it) * U_BYTES)
 
-  // ---- stage 1: log-decay sums.  x_t = inclusive sum of the log decay (in units of log 2) INSIDE the 16-token block, in place;
-  //      lane 8 J + p of warp w sums channels 16 w + 2 p, + 1 over block J, so the block totals of a channel sit in four lanes
-  //      of one warp, which turn them into the tables ----
+  // ---- stage 1: log-decay sums.  x_t = inclusive sum of the log decay (in units of log 2) INSIDE the 16-token block, in place.  Lane
+  //      8 J + 4 b + p of warp w has channels 16 w + 4 p .. + 3 over tokens 8 b .. 8 b + 7 of block J, in the order 0-7 (b = 0) or
+  //      4-7, 0-3: so the eight lanes of a block read and write all banks.  The block totals of a channel sit in eight lanes of one
+  //      warp, which turn them into the tables, two channels each ----
   int seen = INT_MAX;                                      // publishing warp's first lanes: chunks that each CTA of the slot has consumed
   if (SUB && tid >= PUB_WARP * 32 && tid < PUB_WARP * 32 + SLICES)
     seen = ld_relaxed_gpu(consumed + (PREP_UNIT(slot, it) * SLICES + tid - PUB_WARP * 32) * F_LINE);
@@ -382,64 +478,95 @@ __device__ __forceinline__ void prep_unit(
     if (GATED) beta = static_cast<const float*>(beta_in)[bi];
     else beta = __bfloat162float(static_cast<const __nv_bfloat16*>(beta_in)[bi]);
   }
-  const int J = lane >> 3, gc = 16 * warp + 2 * (lane & 7);
+  const int J = lane >> 3, half = (lane >> 2) & 1, g4 = 16 * warp + 4 * (lane & 3), gc = g4 + 2 * half;
   float2 dec;                                              // e^{G_last} of channels gc, gc + 1 (lanes with J = 3)
   {
     constexpr float LOG2E = 1.4426950408889634f;
     constexpr float FLOOR = -80.5f * LOG2E;                // keeps k^ e^{x} and k^ e^{-x} inside fp32's normal range (gates of -5: -80)
     float decay = 0.f;
-    float2 bias = make_float2(0.f, 0.f);
-    int n_block = 16;                                      // GATED: tokens of this block that exist (the others read as zeros)
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    int n_valid = KC;
     if (GATED) {
       const int head = PREP_UNIT(head, it);
-      n_block = PREP_UNIT(n_valid, it) - 16 * J;
+      n_valid = PREP_UNIT(n_valid, it);
       decay = __expf(__ldg(a_log + head));
-      bias = __ldg(reinterpret_cast<const float2*>(dt_bias + (size_t)head * KD + gc));
+      bias = __ldg(reinterpret_cast<const float4*>(dt_bias + (size_t)head * KD + g4));
     }
-    float2 tot = make_float2(0.f, 0.f);
-    uint8_t* const xb = smem + P1_X + (gc >> 5) * P1_BOX + 16 * J * 128 + (gc & 3) * 4;
-    const int piece = (gc >> 2) & 7;
+    uint8_t* const xb = smem + P1_X + (g4 >> 5) * P1_BOX + (16 * J + 8 * half) * 128;
+    const int piece = (g4 >> 2) & 7, turn = 4 * half;      // slot i holds token i ^ turn of the half
+    auto at = [&](int i) { return reinterpret_cast<float4*>(xb + (i ^ turn) * 128 + ((piece ^ i ^ turn) << 4)); };
     tc::mbar_wait(&ctx.sh->g_bar, it & 1, ctx.abort_flag, 12);
-    float2 gr[16];
+    float4 gr[8];
+    auto load_gates = [&]() {
 #pragma unroll
-    for (int i = 0; i < 16; i++) gr[i] = *reinterpret_cast<const float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4));
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
+      for (int i = 0; i < 8; i++) gr[i] = *at(i);
       if (GATED) {
-        if (i < n_block) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
           gr[i].x = lower_bound * (1.0f / (1.0f + __expf(-(decay * (gr[i].x + bias.x)))));
           gr[i].y = lower_bound * (1.0f / (1.0f + __expf(-(decay * (gr[i].y + bias.y)))));
+          gr[i].z = lower_bound * (1.0f / (1.0f + __expf(-(decay * (gr[i].z + bias.z)))));
+          gr[i].w = lower_bound * (1.0f / (1.0f + __expf(-(decay * (gr[i].w + bias.w)))));
         }
+        if (n_valid < KC)                                  // the tokens past the end, whose f reads as zero, do not decay
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            if (16 * J + 8 * half + (i ^ turn) >= n_valid) gr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      tot.x = fmaf(gr[i].x, LOG2E, tot.x);
-      tot.y = fmaf(gr[i].y, LOG2E, tot.y);
-      *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = tot;
-    }
-    if (__builtin_expect(__any_sync(0xffffffffu, fminf(tot.x, tot.y) < FLOOR), 0)) {
+    };
+    auto add4 = [](float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); };
+    auto other = [&](float4 v) {                           // the same of the block's other half
+      return make_float4(__shfl_xor_sync(0xffffffffu, v.x, 4), __shfl_xor_sync(0xffffffffu, v.y, 4), __shfl_xor_sync(0xffffffffu, v.z, 4),
+                         __shfl_xor_sync(0xffffffffu, v.w, 4));
+    };
+    // gates -> sums inside slots 0-3 and inside slots 4-7
+    auto run_sums = [&]() {
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const float4 r = i & 3 ? gr[i - 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+        gr[i] = make_float4(fmaf(gr[i].x, LOG2E, r.x), fmaf(gr[i].y, LOG2E, r.y), fmaf(gr[i].z, LOG2E, r.z), fmaf(gr[i].w, LOG2E, r.w));
+      }
+    };
+    load_gates();
+    run_sums();
+    float4 mine = add4(gr[3], gr[7]), theirs = other(mine), tot4 = add4(mine, theirs);
+    if (__builtin_expect(__any_sync(0xffffffffu, fminf(fminf(tot4.x, tot4.y), fminf(tot4.z, tot4.w)) < FLOOR), 0)) {
       // Rare: a channel decays by more than e^-80 inside the block.  Sums that stop at a floor would take the tokens behind it as
       // not decaying at all, so the strongest of its gates are weakened instead: to e^-40, or to e^-20, e^-10 or e^-5, whichever is the
       // first that keeps the block's sum.
-      float lo_x = tot.x < FLOOR ? -40.f : -INFINITY, lo_y = tot.y < FLOOR ? -40.f : -INFINITY;
-      auto at_least = [](float v, float lo) { return v < lo ? lo : v; };   // (a NaN stays one)
+      load_gates();
+      auto first_lo = [](float v) { return v < FLOOR ? -40.f : -INFINITY; };
+      float4 lo = make_float4(first_lo(tot4.x), first_lo(tot4.y), first_lo(tot4.z), first_lo(tot4.w));
+      auto at_least = [](float v, float l) { return v < l ? l : v; };   // (a NaN stays one)
+      auto gate = [&](int i) {
+        return make_float4(at_least(gr[i].x, lo.x), at_least(gr[i].y, lo.y), at_least(gr[i].z, lo.z), at_least(gr[i].w, lo.w));
+      };
 #pragma unroll 1
       for (int k = 0; k < 3; k++) {
-        float sx = 0.f, sy = 0.f;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-          sx += at_least(gr[i].x, lo_x);
-          sy += at_least(gr[i].y, lo_y);
-        }
-        if (sx < -80.f) lo_x *= 0.5f;
-        if (sy < -80.f) lo_y *= 0.5f;
+        for (int i = 0; i < 8; i++) sum = add4(sum, gate(i));
+        sum = add4(sum, other(sum));
+        if (sum.x < -80.f) lo.x *= 0.5f;
+        if (sum.y < -80.f) lo.y *= 0.5f;
+        if (sum.z < -80.f) lo.z *= 0.5f;
+        if (sum.w < -80.f) lo.w *= 0.5f;
       }
-      tot = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < 16; i++) {
-        tot.x = fmaf(at_least(gr[i].x, lo_x), LOG2E, tot.x);
-        tot.y = fmaf(at_least(gr[i].y, lo_y), LOG2E, tot.y);
-        *reinterpret_cast<float2*>(xb + i * 128 + ((piece ^ (i & 7)) << 4)) = tot;
-      }
+      for (int i = 0; i < 8; i++) gr[i] = gate(i);
+      run_sums();
+      mine = add4(gr[3], gr[7]);
+      theirs = other(mine);
+      tot4 = add4(mine, theirs);
     }
+    // what goes before the slots: the block's first half (b = 1), and this half's first four tokens, which are slots 4-7 where b = 1
+    const float4 g3 = gr[3];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const float4 carry = i < 4 ? (half ? add4(theirs, gr[7]) : make_float4(0.f, 0.f, 0.f, 0.f)) : (half ? theirs : g3);
+      *at(i) = add4(gr[i], carry);
+    }
+    const float2 tot = half ? make_float2(tot4.z, tot4.w) : make_float2(tot4.x, tot4.y);
     float2 before = make_float2(0.f, 0.f), after = make_float2(0.f, 0.f), next1 = before, next2 = before;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -449,7 +576,7 @@ __device__ __forceinline__ void prep_unit(
       if (q == J + 1) next1 = make_float2(qx, qy);
       if (q == J + 2) next2 = make_float2(next1.x + qx, next1.y + qy);
     }
-    auto put = [&](int r, float2 v) { *reinterpret_cast<float2*>(sTab + r * KD + gc) = make_float2(ex2_approx(v.x), ex2_approx(v.y)); };
+    auto put = [&](int r, float2 v) { *reinterpret_cast<float2*>(sTab + r * TAB_LD + gc) = make_float2(ex2_approx(v.x), ex2_approx(v.y)); };
     put(TAB_EP + J, before);
     // decay from a token to the end of ITS block is e^{tot - x} = e^{-x} e^{tot} (each factor within fp32 range for |x| <= 80.5),
     // the decay over the LATER blocks is e^{G_last - P_next} (may underflow: then Kt is 0)
@@ -460,17 +587,16 @@ __device__ __forceinline__ void prep_unit(
     dec = make_float2(ex2_approx(before.x + tot.x), ex2_approx(before.y + tot.y));
   }
   if (GATED && t < PREP_UNIT(n_valid, it)) beta = __bfloat162float(__float2bfloat16(1.0f / (1.0f + __expf(-beta))));
-  // q and k rows: piece 4 m + tig of a row is in box m / 2 (expanded when they are used)
+  // q and k rows: piece 4 m + tig of a row (expanded when they are used)
   uint4 kraw[4], qraw[4];
   tc::mbar_wait(&ctx.sh->qkv_bar, it & 1, ctx.abort_flag, 13);
   float rk, rq;                                            // L2 normalisation of the rows
   {
-    const uint8_t* qrow = smem + P1_QK + t * 128;
+    const uint8_t* qrow = smem + P1_QK + t * 64 + tig * 16;
 #pragma unroll
     for (int m = 0; m < 4; m++) {
-      const int off = (m >> 1) * P1_BOX + (((4 * (m & 1) + tig) ^ g8) << 4);
-      qraw[m] = *reinterpret_cast<const uint4*>(qrow + off);
-      kraw[m] = *reinterpret_cast<const uint4*>(qrow + 2 * P1_BOX + off);
+      qraw[m] = *reinterpret_cast<const uint4*>(qrow + m * 4096);
+      kraw[m] = *reinterpret_cast<const uint4*>(qrow + 2 * P1_BOX + m * 4096);
     }
     float sk = 0.f, sq = 0.f;
 #pragma unroll
@@ -489,6 +615,10 @@ __device__ __forceinline__ void prep_unit(
   }
   // fused form: the ring slot must have been drained before the first write to the unit (all of them follow)
   bool unpublished = SUB && it > 0;                        // the flag of the unit before this one
+  if (SUB && it == 1 && warp == PUB_WARP) {                // the chains wait for a worker's first
+    prep_publish(ctx, 0, ready, kr);
+    unpublished = false;
+  }
   if (SUB && warp == PUB_WARP) {
     const int want = PREP_UNIT(value, it) - kr;            // the slot held chunk value - 1 - kr
     if (__any_sync(0xffffffffu, seen < want)) {
@@ -498,6 +628,7 @@ __device__ __forceinline__ void prep_unit(
       __syncwarp();
     }
   }
+  if (SUB && it > 0 && tid == PUB_WARP * 32) tc::bulk_wait_read<0>();   // the W of the unit before has left K+'s place
   prep_sync<SUB>(ctx);                                     // x and the tables are complete, q and k have been read
 
   // ---- stage 2: every operand that is a row of this warp's tokens times a decay, and the products of the warp's tokens with
@@ -512,7 +643,7 @@ __device__ __forceinline__ void prep_unit(
     for (int i = lane; i < (7 - warp) * 8; i += 32)
       *reinterpret_cast<uint4*>(out + U_BB + warp * SBO_K64 + (warp + 1) * LBO + i * 16) = make_uint4(0, 0, 0, 0);
     float dg[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
-    const float* tab = sTab + I * KD + 8 * tig;
+    const float* tab = sTab + I * TAB_LD + 8 * tig;
     const uint64_t beta2 = pack2(beta, beta), rk2 = pack2(rk, rk), rq2 = pack2(rq, rq);
     uint8_t* ri = sRI + (t & 15) * 256;
     const int sw = (t & 1) << 2;                           // 16-byte pieces of odd rows are swapped in halves of 64 bytes: conflict-free reads
@@ -562,31 +693,41 @@ __device__ __forceinline__ void prep_unit(
       }
       uint64_t f[4], w[4];
       const int piece = 4 * m + tig;
-      // K+ = k^ e^{G_t}: B operand; Q+ = q^ e^{G_t}: rows 64-127 of the unit's first tile
-      load_pairs(tab + TAB_EP * KD + 32 * m, f);
+      // K+ = k^ e^{G_t}: B operand; Q+ = q^ e^{G_t}: rows 64-127 of the unit's first tile (a chunk's first block: e^{x} is all of it)
+      uint4 kp = make_uint4(ah[m][0], ah[m][2], ah[m][4], ah[m][6]), qp = make_uint4(ah[m][1], ah[m][3], ah[m][5], ah[m][7]);
+      if (I > 0) {
+        load_pairs(tab + TAB_EP * TAB_LD + 32 * m, f);
 #pragma unroll
-      for (int e = 0; e < 4; e++) w[e] = mul2(kl[e], f[e]);
-      *reinterpret_cast<uint4*>(sK + piece * P1_PIECE + warp * 128 + g8 * 16) = pack_piece(w);
+        for (int e = 0; e < 4; e++) w[e] = mul2(kl[e], f[e]);
+        kp = pack_piece(w);
 #pragma unroll
-      for (int e = 0; e < 4; e++) w[e] = mul2(ql[e], f[e]);
-      *reinterpret_cast<uint4*>(out + U_WQ + (8 + warp) * SBO_K128 + piece * LBO + g8 * 16) = pack_piece(w);
-      load_pairs(tab + TAB_ETOT * KD + 32 * m, f);
+        for (int e = 0; e < 4; e++) w[e] = mul2(ql[e], f[e]);
+        qp = pack_piece(w);
+      }
+      *reinterpret_cast<uint4*>(sK + piece * P1_PIECE + warp * 128 + g8 * 16) = kp;
+      *reinterpret_cast<uint4*>(out + U_WQ + (8 + warp) * WQ_ROWS + m * ATOM + atom_off(g8, tig)) = qp;
+      load_pairs(tab + TAB_ETOT * TAB_LD + 32 * m, f);
 #pragma unroll
       for (int e = 0; e < 4; e++) rb[e] = mul2(rb[e], f[e]);
-      load_pairs(tab + TAB_KE * KD + 32 * m, f);
+      const uint4 rp = pack_piece(rb);
+      uint4 kt = rp;                                       // (the last block ends with the chunk)
+      if (I < 3) {
+        load_pairs(tab + TAB_KE * TAB_LD + 32 * m, f);
 #pragma unroll
-      for (int e = 0; e < 4; e++) w[e] = mul2(rb[e], f[e]);
-      *reinterpret_cast<uint4*>(out + U_KT + piece * 1024 + warp * 128 + g8 * 16) = pack_piece(w);
+        for (int e = 0; e < 4; e++) w[e] = mul2(rb[e], f[e]);
+        kt = pack_piece(w);
+      }
+      *reinterpret_cast<uint4*>(out + U_KT + m * KT_BLK + warp * ATOM + atom_off(g8, tig)) = kt;
       const int po = (piece ^ sw) << 4;
-      if (I < 3) *reinterpret_cast<uint4*>(ri + ((I + 1) * I / 2 + I) * 4096 + po) = pack_piece(rb);
+      if (I < 3) *reinterpret_cast<uint4*>(ri + ((I + 1) * I / 2 + I) * 4096 + po) = rp;
       if (I < 2) {
-        load_pairs(sTab + (TAB_F + I) * KD + 8 * tig + 32 * m, f);
+        load_pairs(sTab + (TAB_F + I) * TAB_LD + 8 * tig + 32 * m, f);
 #pragma unroll
         for (int e = 0; e < 4; e++) w[e] = mul2(rb[e], f[e]);
         *reinterpret_cast<uint4*>(ri + ((I + 2) * (I + 1) / 2 + I) * 4096 + po) = pack_piece(w);
       }
       if (I < 1) {
-        load_pairs(sTab + (TAB_F + 2) * KD + 8 * tig + 32 * m, f);
+        load_pairs(sTab + (TAB_F + 2) * TAB_LD + 8 * tig + 32 * m, f);
 #pragma unroll
         for (int e = 0; e < 4; e++) w[e] = mul2(rb[e], f[e]);
         *reinterpret_cast<uint4*>(ri + 3 * 4096 + po) = pack_piece(w);
@@ -603,11 +744,15 @@ __device__ __forceinline__ void prep_unit(
       *reinterpret_cast<uint32_t*>(bbrow + (warp - 1) * LBO) = pack_h2(sb[2], sb[3]);
     }
   }
+  tc::fence_async_smem();
   prep_sync<SUB>(ctx);                                     // right operands and the diagonal blocks of N are complete
 
   // ---- stage 3: the products with earlier blocks (fp16), 2 I tiles a warp; the warps of the first block, which have none, invert the
-  //      16 x 16 diagonal blocks of I + N, those of the second and third convert v as well ----
-  if (SUB && warp == PUB_WARP && unpublished) prep_publish(ctx, it - 1, ready, kr);
+  //      16 x 16 diagonal blocks of I + N, those of the second convert v as well ----
+  if (tid == 0) {
+    prep_fetch_g(ctx, it + 1, map_g);                      // x is free
+  }
+  __syncwarp();
   {
     float* nrow = sN + prep_n_row(t) + 2 * tig;
     uint8_t* bbrow = PREP_OUT + U_BB + warp * SBO_K64 + g8 * 16 + tig * 4;
@@ -656,12 +801,12 @@ __device__ __forceinline__ void prep_unit(
     float* xi = sX + prep_inv_at(blk) + col;
 #pragma unroll
     for (int r = 0; r < 16; r++) xi[r * P1_LDX] = x[r];
-  } else if (I < 3) {
+  } else if (I == 1) {
     // bf16 -> fp16 in place.  (The product T V needs both operands in ONE 16-bit format: a kind::f16 product of an fp16 T with bf16
     // rows is rejected by the hardware as an illegal instruction.)
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      uint4* vp = reinterpret_cast<uint4*>(smem + P1_V) + tid - 64 + 128 * j;
+    for (int j = 0; j < 16; j++) {
+      uint4* vp = reinterpret_cast<uint4*>(smem + P1_V) + tid - 64 + 64 * j;
       const uint4 vr = *vp;
       *vp = make_uint4(pack_h2(bf16lo(vr.x), bf16hi(vr.x)), pack_h2(bf16lo(vr.y), bf16hi(vr.y)), pack_h2(bf16lo(vr.z), bf16hi(vr.z)),
                        pack_h2(bf16lo(vr.w), bf16hi(vr.w)));
@@ -671,7 +816,7 @@ __device__ __forceinline__ void prep_unit(
 
   // ---- stage 4: X = (I + N)^-1 below its diagonal blocks, and its fp16 copy T as the K-major A operand (K = 64).  First
   //      P_mj = N_mj X_jj in place of N_mj, one warp per block, while two warps write the diagonal of T and the zeros above it;
-  //      then one warp per row of blocks ----
+  //      then the blocks of X, while a warp publishes the unit before and one works out the unit after the next ----
   if (warp < 6) {
     const int m = warp < 1 ? 1 : (warp < 3 ? 2 : 3), j = warp - (m * (m - 1)) / 2, ld = m < 2 ? 36 : 68;
     float* nb = sN + prep_n_row(16 * m) + 16 * j;
@@ -687,7 +832,6 @@ __device__ __forceinline__ void prep_unit(
     }
   } else {
     const int e = tid - 192;
-    if (SUB && e == 0) make_unit(it + 1, ctx.sh->unit[(it + 1) & 3]);
 #pragma unroll
     for (int q = 0; q < 2; q++) {                          // 4 blocks x 16 rows x 2 pieces
       const int i = e + 64 * q, blk = i >> 5, r = (i & 7) + ((i >> 4) & 1) * 8, h = (i >> 3) & 1;
@@ -703,9 +847,13 @@ __device__ __forceinline__ void prep_unit(
     }
   }
   prep_sync<SUB>(ctx);
-  if (warp == 1) prep_inverse_row<1>(sN, sX, sT, lane);
+  if (!SUB) {
+    if (warp < 6) prep_inverse_blocks(sN, sX, sT, warp, lane, ctx.bar_id + 4);
+  } else if (warp == 1) prep_inverse_row<1>(sN, sX, sT, lane);
   else if (warp == 2) prep_inverse_row<2>(sN, sX, sT, lane);
   else if (warp == 3) prep_inverse_row<3>(sN, sX, sT, lane);
+  else if (SUB && warp == PUB_WARP && unpublished) prep_publish(ctx, it - 1, ready, kr);
+  else if (SUB && tid == FETCH_TID) make_unit(it + 2, ctx.sh->unit[(it + 2) & 3]);
   tc::fence_async_smem();
   tc::fence_before_sync();
   prep_sync<SUB>(ctx);
@@ -725,28 +873,44 @@ __device__ __forceinline__ void prep_unit(
       tc::mma_ws_f16_if(1, tmem + 64, tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64), tc::sdesc_advance(vd, kk * 2048), idesc, kk > 0);
     tc::mma_commit(&ctx.sh->mma_bar);
   }
-  if (tid == 96) prep_fetch_g(ctx, it + 1, map_g);         // x is free
-  __syncwarp();
   const bool ok = tc::mbar_wait(&ctx.sh->mma_bar, it & 1, ctx.abort_flag, 1);
-  if (tid == 96) prep_fetch_qkv(ctx, it + 1, map_qkv, H);  // and so are T, N, K+ and V
+  if (tid == FETCH_TID) prep_fetch_qkv(ctx, it + 1, map_qkv, map_qk, H);  // T, N, K+ and V are free
+  __syncwarp();
   tc::fence_after_sync();
-  // ---- stage 6: the accumulators leave: warps 0-3 take W, warps 4-7 Uloc, a token and 64 columns each thread ----
+  // ---- stage 6: the accumulators leave: warps 0-3 take W, warps 4-7 Uloc, a token and 64 columns each thread.  A warp's piece of Uloc
+  //      is 512 contiguous bytes; of W it would be 32 halves of 32-byte sectors, so W is put together where K+ was and copied out ----
   if (ok) {
     uint8_t* const out = PREP_OUT;
     const int et = (warp & 1) * 32 + lane, c0 = (warp & 2) * 32;
     const uint32_t acc = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
-    uint8_t* const dst = warp < 4 ? out + U_WQ + (et >> 3) * SBO_K128 + (et & 7) * 16 + (c0 >> 3) * LBO : out + U_UL + (et ^ 8) * 16 + (c0 >> 3) * 1024;
-    const uint32_t pitch = warp < 4 ? LBO : 1024, sign = warp < 4 ? 0x80008000u : 0u;   // W is stored negated
+    auto piece = [](const uint32_t* r, uint32_t sign) {
+      return make_uint4(pack_h2(__uint_as_float(r[0]), __uint_as_float(r[1])) ^ sign, pack_h2(__uint_as_float(r[2]), __uint_as_float(r[3])) ^ sign,
+                        pack_h2(__uint_as_float(r[4]), __uint_as_float(r[5])) ^ sign, pack_h2(__uint_as_float(r[6]), __uint_as_float(r[7])) ^ sign);
+    };
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       uint32_t r[32];
       tc::tmem_ld32(acc + 32 * h, r);
       tc::tmem_ld_wait();
+      if (warp < 4) {                                      // stored negated
+        uint8_t* const dst = sK + (et >> 3) * WQ_ROWS + ((c0 >> 5) + h) * ATOM;
 #pragma unroll
-      for (int u = 0; u < 4; u++)
-        *reinterpret_cast<uint4*>(dst + (4 * h + u) * pitch) = make_uint4(
-            pack_h2(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])) ^ sign, pack_h2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])) ^ sign,
-            pack_h2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])) ^ sign, pack_h2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])) ^ sign);
+        for (int u = 0; u < 4; u++) *reinterpret_cast<uint4*>(dst + atom_off(et, u)) = piece(r + 8 * u, 0x80008000u);
+      } else {
+        uint8_t* const dst = out + U_UL + (et ^ 8) * 16 + ((c0 >> 3) + 4 * h) * 1024;
+#pragma unroll
+        for (int u = 0; u < 4; u++) *reinterpret_cast<uint4*>(dst + u * 1024) = piece(r + 8 * u, 0u);
+      }
+    }
+    if (warp < 4) {
+      tc::fence_async_smem();
+      asm volatile("bar.arrive %0, 160;" ::"r"(ctx.bar_id + 4) : "memory");
+    } else if (warp == PUB_WARP) {
+      asm volatile("bar.sync %0, 160;" ::"r"(ctx.bar_id + 4) : "memory");
+      if (tid == PUB_WARP * 32) {
+        tc::bulk_s2g(out + U_WQ, sK, 8 * WQ_ROWS);
+        tc::bulk_commit();
+      }
     }
   }
   tc::fence_before_sync();
@@ -755,7 +919,7 @@ __device__ __forceinline__ void prep_unit(
 
 template <bool GATED>
 __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
-    const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
+    const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_qk, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
     uint8_t* __restrict__ ws, int seqlen, int H, int n_chunks, int* __restrict__ status,
     const float* __restrict__ dt_bias, const float* __restrict__ a_log, float lower_bound) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -783,15 +947,16 @@ __global__ __launch_bounds__(256, 2) void kda_chunk_prep_kernel(
     sh.unit[1].n_valid = 0;                                // a CTA has one unit
     pdl_wait();
     prep_fetch_g(ctx, 0, &map_g);
-    prep_fetch_qkv(ctx, 0, &map_qkv, H);
+    prep_fetch_qkv(ctx, 0, &map_qkv, &map_qk, H);
   }
   if (tid < 32) tc::tmem_alloc(&tmem_slot, 128);
   pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  prep_unit<GATED, 0>(ctx, 0, &map_qkv, &map_g, beta_in, ws, H, dt_bias, a_log, lower_bound, tmem_slot, nullptr, nullptr, nullptr, 0,
+  prep_unit<GATED, 0>(ctx, 0, &map_qkv, &map_qk, &map_g, beta_in, ws, H, dt_bias, a_log, lower_bound, tmem_slot, nullptr, nullptr, nullptr, 0,
                       [](int, PrepDesc&) {});
+  if (tid == PUB_WARP * 32) tc::bulk_wait_all<0>();
   __syncthreads();
   if (tid < 32) tc::tmem_dealloc(tmem_slot, 128);
   if (tid == 0 && abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
@@ -837,7 +1002,7 @@ struct Chain {
   static constexpr uint32_t O = U + NV * 128;               // bf16 output rows of one chunk: swizzled boxes of 64 tokens x 64 channels
   static constexpr uint32_t ID = O + NV * 128;              // [I ; 0]
   static constexpr uint32_t SMEM = ID + ID_BYTES + 1024;    // + slack to start the tiles at a 1 KB boundary
-  static_assert(O % 1024 == 0 && STAGE % 128 == 0 && BB >= 8192, "layout");
+  static_assert(O % 1024 == 0 && STAGE % ATOM == 0 && KT % ATOM == 0 && BB >= 8192, "layout");
 };
 struct ChainBars {                  // two of most kinds by chunk parity, so that a warp that is held up may be a chunk behind
   uint64_t wu[2];                   // -W, Q+ and Uloc of a stage have landed
@@ -908,7 +1073,7 @@ __device__ __forceinline__ void chain_cta(uint8_t* smem, ChainBars& bars, const 
       tc::fence_after_sync();
 #pragma unroll
       for (int kk = 0; kk < KD / 16; kk++) {
-        const uint64_t ad = tc::make_sdesc(stg_addr + U_WQ + kk * 2 * LBO, LBO, SBO_K128);
+        const uint64_t ad = tc::make_sdesc_sw64(stg_addr + U_WQ + (kk >> 1) * ATOM + (kk & 1) * 32, 16, WQ_ROWS);
         const uint64_t bd = tc::make_sdesc(s_addr + kk * 2 * 128, 128, 2048);
         tc::mma_f16_if(leader, d1, ad, bd, idesc, true);
       }
@@ -929,7 +1094,7 @@ __device__ __forceinline__ void chain_cta(uint8_t* smem, ChainBars& bars, const 
       tc::fence_after_sync();
 #pragma unroll
       for (int kk = 0; kk < KC / 16; kk++) {
-        const uint64_t ad = tc::make_sdesc(stg_addr + C::KT + kk * 2 * 128, 128, 1024);
+        const uint64_t ad = tc::make_sdesc_sw64(stg_addr + C::KT + kk * 2 * ATOM, KT_BLK, ATOM);
         const uint64_t bd = tc::make_sdesc(u_addr + kk * 2 * 128, 128, 1024);
         tc::mma_f16_if(leader, d2, ad, bd, idesc_kt, kk > 0);
       }
@@ -1207,7 +1372,7 @@ constexpr uint32_t fused_smem() { return Chain<NV>::SMEM > 2 * P1_SMEM + 1024 ? 
 
 template <bool GATED, int NV>
 __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
-    const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
+    const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_qk, const __grid_constant__ CUtensorMap map_g, const void* __restrict__ beta_in,
     uint8_t* __restrict__ ring, int* __restrict__ flags, float* __restrict__ state,
     float* __restrict__ out_f32, int seqlen, int H, int n_chunks, int n_jobs, int n_slots, int kr, const int* __restrict__ slots,
     float scale, int* __restrict__ status, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
@@ -1260,15 +1425,15 @@ __global__ __launch_bounds__(512, 1) void kda_fused_kernel(
     };
     PrepCtx ctx;
     ctx.smem = smem + sub * P1_SMEM; ctx.sh = &prep[sub]; ctx.abort_flag = &abort_flag; ctx.tid = tid & 255; ctx.bar_id = 1 + sub;
-    if (ctx.tid == 0) make_unit(0, prep[sub].unit[0]);
+    if (ctx.tid < 2) make_unit(ctx.tid, prep[sub].unit[ctx.tid]);
     prep_sync<true>(ctx);
     if (ctx.tid == 0) {
       prep_fetch_g(ctx, 0, &map_g);
-      prep_fetch_qkv(ctx, 0, &map_qkv, H);
+      prep_fetch_qkv(ctx, 0, &map_qkv, &map_qk, H);
     }
     int it = 0;
     for (; PREP_UNIT(n_valid, it) > 0; it++)
-      prep_unit<GATED, SLICES>(ctx, it, &map_qkv, &map_g, beta_in, ring, H, dt_bias, a_log, lower_bound, tmem + sub * 256, ready, consumed,
+      prep_unit<GATED, SLICES>(ctx, it, &map_qkv, &map_qk, &map_g, beta_in, ring, H, dt_bias, a_log, lower_bound, tmem + sub * 256, ready, consumed,
                                g_abort, kr, make_unit);
     if (it > 0 && (ctx.tid >> 5) == PUB_WARP) prep_publish(ctx, it - 1, ready, kr);
   } else {
@@ -1293,9 +1458,10 @@ int g_chunked_form = 0;
 // Chain slots of the fused launch and the value columns of a chain CTA for n_jobs (batch, head) chains; no slots = use the two-kernel
 // form.  Chains share slots evenly (a slot walks its chains one after the other), and the preparation keeps 64 SMs or more.  Of the
 // divisors of n_jobs from 16 to 48, or n_jobs itself, the one for which the longer of the two sides takes least per chunk of all
-// chains: a chain CTA needs 1,380 ns a chunk with all 128 columns, 1,100 with 64, an SM of preparation workers 5,800 ns a unit.  Waits counted
-// in a measuring build bear the sides out, 32,768 tokens: with 32 heads the workers are the longer side (a unit 22,770 cycles, of them 400
-// for a ring slot; a chain CTA's chunk 3,200, of them 940 for its unit), with 16 and 8 the chains are (workers 22 and 64 % of their time).
+// chains: a chain CTA is taken to need 1,380 ns a chunk with all 128 columns, 1,100 with 64, an SM of preparation workers 5,800 ns a unit (the
+// line between the shapes; 1,550 : 1,150 : 4,700, nearer to what they need with 32 heads, chose 48 slots for 3 x 8,192 x 32: 1,190 us, 1,096
+// with 32).  Waits counted in a measuring build, 32,768 tokens x 32 heads: neither side is much the longer one, a worker waits 2,060 of a
+// unit's 20,600 cycles for a ring slot, a chain CTA 600 of a chunk's 3,000 for the 48 KB it needs first; with 16 and 8 the chains are.
 // (32,768 tokens x 8 heads 719 -> 532 us with two CTAs a chain, x 16 725 -> 580; 32 heads have one, at 84 SMs of workers they would
 // take 1,150; 3 sequences x 8,192 x 32 heads 786 with 48 slots of two chains, 685 with 32 of three.)
 // `room`: the slots that the workspace is sized for, the largest number that divides the chains: it covers calls of fewer sequences.
@@ -1445,10 +1611,20 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
   }
   // tensor maps of the inputs, [batch][token][channels]: boxes of 64 tokens x 128 bytes, 128-byte swizzle, zeros past the last token;
   // and of the output [batch][token][head][128] bf16: 64 channels x 1 head x 64 tokens x 1 sequence
-  alignas(64) CUtensorMap map_qkv, map_g, map_out;
+  alignas(64) CUtensorMap map_qkv, map_qk, map_g, map_out;
   if (!encode_rows(&map_qkv, mixed_qkv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 3 * num_heads * KD, seqlen, bsz, 64) ||
       !encode_rows(&map_g, g_or_f, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, num_heads * KD, seqlen, bsz, 32))
     return HK_ERR_CUDA;
+  {
+    const size_t row = (size_t)3 * num_heads * KD * 2;
+    const cuuint64_t dims[4] = {32, (cuuint64_t)seqlen, (cuuint64_t)3 * num_heads * 4, (cuuint64_t)bsz};
+    const cuuint64_t strides[3] = {row, 64, (cuuint64_t)seqlen * row};
+    const cuuint32_t box[4] = {32, (cuuint32_t)KC, 4, 1}, estr[4] = {1, 1, 1, 1};
+    if (tensor_map_encoder()(&map_qk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(mixed_qkv), dims, strides, box, estr,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return HK_ERR_CUDA;
+  }
   {
     const cuuint64_t dims[4] = {(cuuint64_t)KD, (cuuint64_t)num_heads, (cuuint64_t)seqlen, (cuuint64_t)bsz};
     const cuuint64_t strides[3] = {(cuuint64_t)KD * 2, (cuuint64_t)num_heads * KD * 2, (cuuint64_t)seqlen * num_heads * KD * 2};
@@ -1481,14 +1657,14 @@ int chunked_prefill_launch(const void* mixed_qkv, const float* g_or_f, const voi
     cfg.numAttrs = 1;
     auto kern = gated ? (split ? kda_fused_kernel<true, 64> : kda_fused_kernel<true, 128>)
                       : (split ? kda_fused_kernel<false, 64> : kda_fused_kernel<false, 128>);
-    return cudaLaunchKernelEx(&cfg, kern, map_qkv, map_g, beta_or_b, (uint8_t*)workspace + flag_bytes, (int*)workspace, state, out_f32, seqlen,
+    return cudaLaunchKernelEx(&cfg, kern, map_qkv, map_qk, map_g, beta_or_b, (uint8_t*)workspace + flag_bytes, (int*)workspace, state, out_f32, seqlen,
                               num_heads, n_chunks, n_jobs, n_slots, kr, slots, scale, st, dt_bias, a_log, lower_bound, map_out) == cudaSuccess
                ? HK_OK
                : HK_ERR_CUDA;
   }
   const dim3 grid(num_heads, n_chunks, bsz);
   auto prep = gated ? kda_chunk_prep_kernel<true> : kda_chunk_prep_kernel<false>;
-  if (pdl_launch(prep, grid, dim3(256), P1_SMEM + 1024, s, map_qkv, map_g, beta_or_b, (uint8_t*)workspace, seqlen, num_heads, n_chunks, st,
+  if (pdl_launch(prep, grid, dim3(256), P1_SMEM + 1024, s, map_qkv, map_qk, map_g, beta_or_b, (uint8_t*)workspace, seqlen, num_heads, n_chunks, st,
                  dt_bias, a_log, lower_bound) != cudaSuccess)
     return HK_ERR_CUDA;
   // half a head per CTA while these are one wave

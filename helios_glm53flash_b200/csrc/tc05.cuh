@@ -278,6 +278,13 @@ __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t smem_addr, uint32_
   return make_sdesc(smem_addr, lbo_bytes, sbo_bytes) | ((uint64_t)2 << 61);
 }
 
+// 64-byte-swizzle descriptor (layout type 4): rows of 64 bytes, atoms of 8 rows (512 bytes, the stride offset), 16-byte chunk c of row r
+// at c ^ (r / 2 % 4); the tile base must be 512-byte aligned.  MN-major operands use the leading offset as the distance between blocks
+// of 32 M/N elements.
+__device__ __forceinline__ uint64_t make_sdesc_sw64(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return make_sdesc(smem_addr, lbo_bytes, sbo_bytes) | ((uint64_t)4 << 61);
+}
+
 // byte offset of 16-byte chunk `c` of 128-byte row `r` in a 128-byte-swizzled tile whose blocks of
 // 8 chunks (64 elements of the contiguous dimension) are `block_bytes` apart
 __device__ __forceinline__ uint32_t sw128_off(int r, int c, uint32_t block_bytes) {
