@@ -2,7 +2,7 @@
 // cores: dense causal ranges and gathered (sparse) rows, decode and prefill rows, final output or
 // split-KV partials.  One kernel serves helios::attn::mla_sparse_decode and
 // helios::attn::mla_dense_prefill (reference: src/cuda/attn/attn.cu:394-699, scalar kernels, one
-// block per (row, head) or head pair).
+// block per (row, head) or head pair).  Causal chunks of some length go to mla_pair_tc_kernel (mla_pair_tc.cuh), two rows at a time.
 //
 // Work item = (query row, key split) -> one CTA; all 64 heads of the row share every latent row that
 // is staged, so the cache is read once per row (the reference re-reads it per head pair).
@@ -62,6 +62,7 @@ constexpr float RESCALE_THRESHOLD = 8.0f;         // log2 units: P stays below 2
 // others load tiles (dense ranges need more than one only for the ragged last tile).
 constexpr int FT_LOAD_WARPS = 4, FT_THREADS = (6 + FT_LOAD_WARPS) * 32, FT_SLOTS = FT_KEYS / FT_LOAD_WARPS;   // key slots per loader warp
 
+constexpr int FT_PAIR_KEYS = 700;                 // keys of a row, on average, from which on two rows of a chunk go to a pair of CTAs
 constexpr int FT_MINI = 16;                       // keys of a tile in Q's place
 constexpr int FT_MAX_CL = 16;                     // CTAs of a cluster
 // Parts that a row's output channels are shared out in, a cluster each.  Four: a quarter of the product, of the accumulator and of the
@@ -684,6 +685,10 @@ __global__ __launch_bounds__(FT_THREADS, 1) void mla_flash_tc_kernel(
   if (tid == 0 && ms.abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
 }
 
+}  // namespace hk
+#include "mla_pair_tc.cuh"
+namespace hk {
+
 int mla_flash_tc_auto_splits(int m, int n_keys) {
   // At most one CTA per SM (a second wave would double the time), at least two tiles per split, splits of equal tile counts.  With
   // the merge, 1 / 2 / 3 tiles per split, us: 2,052 gathered rows of one query 12.1 / 11.3 / 12.7, of four 16.9 / 12.6 / 13.5 (more
@@ -708,6 +713,7 @@ static int ft_prepare() {
         cudaFuncSetAttribute(mla_flash_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(mla_flash_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(mla_flash_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(mla_pair_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FS_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(mla_flash_tc_kernel<false, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaFuncSetAttribute(mla_flash_tc_kernel<true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
       return HK_ERR_CUDA;
@@ -788,16 +794,20 @@ int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s, bool clusters) {
       return HK_ERR_UNSUPPORTED;
   }
   // 64 rows x 512 channels as one box: whole key tiles of a dense range, and a row's 64 heads of Q
-  auto box_map = [&](CUtensorMap* m, const void* p, cuuint64_t n) {
+  auto box_map = [&](CUtensorMap* m, const void* p, cuuint64_t n, cuuint32_t keys = 64, cuuint32_t blocks = 8) {
     const cuuint64_t dims[3] = {64, n, 8};
     const cuuint64_t strides[2] = {LATENT * 2, 128};
-    const cuuint32_t b[3] = {64, 64, 8};
+    const cuuint32_t b[3] = {64, keys, blocks};
     return encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(p), dims, strides, b, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   static_assert(FT_KEYS == 64 && FT_HEADS == 64, "one box shape for keys and queries");
   const cuuint64_t q_rows = (cuuint64_t)a.m * FT_HEADS;
-  if (!box_map(&qmap, a.q_lat, q_rows) || (!a.raw_idx && !box_map(&box, a.ckv, extent))) return HK_ERR_UNSUPPORTED;
+  // Two rows of a causal chunk share their keys.  Below 700 keys a row on average the pair's own costs (a cluster to start, the later row's own
+  // key as a tile) are more than it gains: us, a CTA a row / pairs, 148 rows at 300 15.3 / 15.4, at 600 19.7 / 19.5, at 1,000 25.5 / 24.2;
+  // 500 at 300 65.7 / 67.8, at 700 89.7 / 86.5; 1,200 at 0 151 / 154, 1,500 209 / 208, 2,500 470 / 431.
+  const bool pairs = !clusters && !a.raw_idx && !a.kv_len && !a.kv_base && a.out && a.n_split == 1 && a.m >= 2 && a.pos_start + a.m / 2 >= FT_PAIR_KEYS;
+  if (!box_map(&qmap, a.q_lat, q_rows) || (!a.raw_idx && !pairs && !box_map(&box, a.ckv, extent))) return HK_ERR_UNSUPPORTED;
   if (a.out) {
     const cuuint64_t dims[2] = {LATENT, q_rows};
     const cuuint64_t strides[1] = {LATENT * 2};
@@ -805,6 +815,13 @@ int mla_flash_tc_launch(const MlaArgs& a, cudaStream_t s, bool clusters) {
     if (encode(&omap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.out, dims, strides, b, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return HK_ERR_UNSUPPORTED;
+  }
+  if (pairs) {
+    alignas(64) CUtensorMap vbox;
+    if (!box_map(&box, a.ckv, extent, 32, 8) || !box_map(&vbox, a.ckv, extent, 32, 4)) return HK_ERR_UNSUPPORTED;
+    const cudaError_t e = pdl_launch_cluster(2, mla_pair_tc_kernel, dim3((unsigned)((a.m + 1) / 2 * 2)), dim3(PT_THREADS), FS_SMEM, s, a,
+                                             device_status_ptr(), box, vbox, rows, qmap, omap);
+    return e == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? HK_OK : HK_ERR_CUDA;
   }
   // Gathered rows: at most a CTA per SM (592 rows of 2,048 keys 180 -> 166 us).  Dense rows, whose loads start faster: a CTA
   // each (600 rows at 32,768 keys 2.72 ms, persistent 2.85).  Partials always: their rows leave through the idle ring.

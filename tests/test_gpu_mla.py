@@ -146,6 +146,28 @@ def test_dense_vs_oracle_and_reference(qlen, pos_start, scale, n_split):
         assert sum_rel(rr, o32) < 3e-3
 
 
+@pytest.mark.parametrize("m,pos", [(2, 700), (2, 698), (3, 1022), (5, 1023), (4, 1086), (2, 1087), (7, 1280)])
+def test_two_rows_of_a_chunk_by_a_pair_of_ctas(m, pos):
+    """even and odd numbers of rows, common keys that end anywhere in a tile, either side of the length from which on pairs are used; late keys
+    move the maximum.  A cache row of infinities or NaN reaches the row whose own key it is and none before it"""
+    inp = synth.mla_inputs(pos + m, m, seed=m + pos, cache_std=0.5)
+    ckv = synth.f16_bits_to_f32(inp["ckv"]).copy()
+    ckv[pos // 2:] *= 4.0
+    _, o32 = orc.mla_attend(inp["q_lat"], synth.f32_to_f16_bits(ckv), m, 64, 0.0625, pos_start=pos)
+    for bad in (None, np.nan, np.inf):
+        c = ckv.copy()
+        if bad is not None:
+            c[pos + m - 1] = bad
+        out = torch.full((m + 1, 64, 512), 7.0, dtype=torch.float16, device="cuda")
+        hk.mla_dense_prefill(dev_f16(inp["q_lat"]), dev_f16(synth.f32_to_f16_bits(c)), out, m, pos, n_split=1)
+        torch.cuda.synchronize()
+        assert hk.read_device_status() == 0
+        g = synth.f16_bits_to_f32(bits(out))
+        assert (g[m] == 7).all()
+        for i in range(m if bad is None else m - 1):
+            assert max_rel(g[i], o32[i]) < TOL, (i, bad)
+
+
 def test_dense_batched_decode_over_concatenated_caches():
     B, L = 4, 777
     inp = synth.mla_inputs(B * L, B, seed=8, cache_std=0.5)
