@@ -61,6 +61,7 @@ inline int sm_count() {
 // not load or store anything.  MLA layer at 5,001 tokens in a graph, nothing released -> released: 1 token 35.0 -> 32.3 us, 8
 // 49.7 -> 44.4, 32 65.0 -> 60.5, 256 129.5 -> 126.7; 45-layer decode at 262,144 618 -> 572 (with limits of 16 to 32 CTAs on some
 // of them, 9 to 256 tokens took 1.1-1.9 us more).
+// The absorbed projections of ONE row do so too (absorb_tc.cu).
 // The other kernels do not: CTAs placed beside a running grid land where it left room, not evenly - the per-token KDA kernel
 // behind the convolution took twice as long, scorer and attention releasing theirs cost the decode chains what the others gain, and
 // KDA decode layers behind one another took 4.2 us instead of 3.9.
