@@ -241,15 +241,25 @@ __global__ __launch_bounds__(TK_THREADS) void dsa_topk_kernel(
 // ------------------------------------------------------------------------------------------------
 constexpr int TKR_MAX_THREADS = 512, TKR_MAX_PIECES = 4 * TKR_MAX_THREADS;
 
+// scores of a thread's pieces -> their keys, two a word
+template <int NP>
+__device__ __forceinline__ void to_keys(uint4 (&pc)[NP]) {
+#pragma unroll
+  for (int u = 0; u < NP; u++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      uint32_t& w = (&pc[u].x)[i];
+      w ^= ((w >> 15) & 0x00010001u) * 0x7fffu + 0x80008000u;   // sign: all bits, else the top one
+    }
+}
 // f(j, key) over the 8 NP keys of a thread's pieces, j ascending with the element index
 template <int NP, class F>
 __device__ __forceinline__ void for_keys(const uint4 (&pc)[NP], F f) {
 #pragma unroll
   for (int u = 0; u < NP; u++) {
-    uint32_t key[8];
-    keys8(pc[u], key);
+    const uint32_t w[4] = {pc[u].x, pc[u].y, pc[u].z, pc[u].w};
 #pragma unroll
-    for (int j = 0; j < 8; j++) f(8 * u + j, key[j]);
+    for (int j = 0; j < 8; j++) f(8 * u + j, j & 1 ? w[j >> 1] >> 16 : w[j >> 1] & 0xffffu);
   }
 }
 
@@ -275,6 +285,7 @@ __global__ __launch_bounds__(FIXED ? FIXED : TKR_MAX_THREADS, FIXED == 256 ? 4 :
   uint4 pc[NP];
 #pragma unroll
   for (int u = 0; u < NP; u++) pc[u] = load8_raw(row, lead, i8 + u, T);
+  to_keys<NP>(pc);
   __syncthreads();
   // exclusive prefix over the block; one barrier, `slot` alternates between calls
   auto exscan = [&](int v, int slot, int* total) {
@@ -414,6 +425,7 @@ __global__ __launch_bounds__(TK_THREADS, 1) void dsa_topk_cluster_kernel(
   uint4 pc[NP];
 #pragma unroll
   for (int u = 0; u < NP; u++) pc[u] = load8_raw(row, lead, i8 + u, T);
+  to_keys<NP>(pc);
   __syncthreads();
   // exclusive prefix over the block; one barrier, `slot` alternates between calls
   auto exscan = [&](int v, int slot, int* total) {
