@@ -56,6 +56,24 @@ def test_conv_at_the_edges_of_its_tiles(bsz, T):
     assert ulp.max() <= 1 and (ulp > 0).mean() < 5e-3
 
 
+@pytest.mark.parametrize("T", [16, 37, 40, 63, 64])
+def test_conv_of_a_short_call_in_one_wave_and_in_several(T):
+    """a tile per CTA (taps and window asked for ahead) against more tiles than CTAs: the same bits, with permuted slots, a wider window and a
+    bias"""
+    bsz, dim, S, piece = 2, 64 * 450, 6, 64 * 150
+    g = torch.Generator(device="cuda").manual_seed(T)
+    r = lambda *n: torch.randn(*n, generator=g, device="cuda").bfloat16()
+    x, st, w, bias = r(bsz, dim, T), r(3, dim, S), r(dim, 4), r(dim)
+    slots = torch.tensor([2, 0], dtype=torch.int32, device="cuda")
+    whole, out = st.clone(), torch.empty(bsz, T, dim, dtype=torch.bfloat16, device="cuda")
+    hk.cuda_causal_conv1d_update(x, whole, slots, w, bias, out, bsz, dim, T, S, 4, True, False)
+    for c in range(0, dim, piece):
+        part, o = st[:, c:c + piece].contiguous(), torch.empty(bsz, T, piece, dtype=torch.bfloat16, device="cuda")
+        hk.cuda_causal_conv1d_update(x[:, c:c + piece].contiguous(), part, slots, w[c:c + piece].contiguous(), bias[c:c + piece].contiguous(), o, bsz,
+                                     piece, T, S, 4, True, False)
+        assert torch.equal(o, out[:, :, c:c + piece]) and torch.equal(part, whole[:, c:c + piece])
+
+
 def test_conv_history_and_generic_k():
     dim, T, K, S = 96, 9, 3, 7
     inp = synth.conv_inputs(T, dim, K=K, seed=5)
