@@ -300,11 +300,11 @@ __device__ __forceinline__ uint2 conv4_rolled(uint2 st, __nv_bfloat16 cur) {
 //
 // A CTA owns a whole head (64 KB of state): 8 warps hold the state (warp = row group, lane = 4 columns), three more prepare
 // the token (q with its norm; k with its norm and the decay; v), and in the layer a twelfth warp asks for the norm's inputs at
-// the start and finishes the output.  With the head in one CTA nothing crosses CTAs: the earlier form, 4 or 8 value slices per head, handed the q / k window and the head's outputs
+// the start and finishes the output.  With the head in one CTA nothing crosses CTAs: a form of 4 or 8 value slices per head that handed the q / k window and the head's outputs
 // over through two ticket counters, an atomic and an L2 round trip each (5.4 us per layer of 32 heads).
 //
-//   few heads: one head per CTA, state straight between global memory and registers (latency: one memory round trip,
-//     three barriers);
+//   few heads: one head per CTA, or four CTAs a head where that leaves one on an SM (below), state straight between global memory and
+//     registers (latency: one memory round trip, three barriers);
 //   many heads (more than 2 per SM): persistent, one CTA per SM, heads stream through shared memory as 64 KB bulk copies: two
 //     stages inwards, each asked for again as soon as its head sits in registers, and one outwards (stores straight from
 //     registers held the SM to 26 B per cycle); the token of the next head is prepared meanwhile.  Layer, a head per CTA / streamed,
@@ -330,6 +330,7 @@ struct DecodeArgs {
   int H, n_heads;                       // heads of a sequence; batch * H
   int Hk;                               // key heads of a sequence (DEC_REC; else H)
   const int* slots;
+  int* status;
 };
 
 struct alignas(16) DecodeToken {                    // one head's token, prepared
@@ -488,10 +489,9 @@ __device__ __forceinline__ FinishIn load_finish(const DecodeArgs& a, int bh, int
   return f;
 }
 template <int MODE>
-__device__ __forceinline__ void decode_finish(const DecodeArgs& a, const FinishIn& f, const float (*opart)[128], int bh, int lane) {
+__device__ __forceinline__ void decode_finish(const DecodeArgs& a, const FinishIn& f, float4 tot, int bh, int lane) {
   constexpr bool LAYER = MODE == DEC_LAYER;
   const size_t o = (size_t)bh * 128 + 4 * lane;
-  float4 tot = part_tree(opart, lane);
   tot.x *= a.scale; tot.y *= a.scale; tot.z *= a.scale; tot.w *= a.scale;
   __nv_bfloat16 h[4] = {__float2bfloat16_rz(tot.x), __float2bfloat16_rz(tot.y), __float2bfloat16_rz(tot.z), __float2bfloat16_rz(tot.w)};
   if (LAYER) {
@@ -525,10 +525,13 @@ __device__ __forceinline__ float* head_state(const DecodeArgs& a, int bh) {
 // SLICES = 4, up to half a head per SM: a CTA owns 32 of the head's 128 columns (two state warps, a quarter warp per row group, the same sums in the
 // same order).  One SM moves a head's 64 KB in and out in 0.6 us each, and a few heads leave the other SMs idle: one token's
 // recurrence alone, whole / split: 32 heads 3.7 / 2.7 us, 74 4.2 / 3.5, 112 5.1 / 5.2; the step 32 heads 3.9 / 3.2, 64 4.4 / 4.1, 80
-// 4.8 / 4.9.  Not for DEC_LAYER, whose norm needs all columns of a head.  In DEC_STEP the
+// 4.8 / 4.9.  In DEC_STEP and DEC_LAYER the
 // four are a cluster: the windows are read by every slice and rolled by the first behind a cluster barrier that all have arrived at
 // long before (32 heads 3.0 us per step; counting the slices through a word of global memory per head 3.13, at 8 heads 2.53 and
-// 2.85, and calls on several streams needed counters of their own).
+// 2.85, and calls on several streams needed counters of their own).  The layer's norm needs all columns of a head: the slices' outputs
+// go to the first one's memory, 16 bytes a lane, which waits for all of them: up to a
+// slice per SM, us a layer in a graph, whole / split: 8 heads 3.59 / 3.08, 32 3.59 / 3.25, 48 3.63 / 3.70, 74 3.73 / 6.2; 45-layer decode at
+// 262,144 470 -> 459.
 template <int MODE, bool VEC, int SLICES>
 __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const DecodeArgs a) {
   constexpr int SW = KD_STATE_WARPS / SLICES;                // state warps
@@ -538,13 +541,24 @@ __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const Decod
   const int cl = SLICES == 1 ? lane : (int)(blockIdx.x % SLICES) * (32 / SLICES) + (lane & 7);   // four columns
   __shared__ __align__(16) DecodeToken tok;
   __shared__ __align__(16) float part[8][128], opart[8][128];
+  constexpr bool GATHER = MODE == DEC_LAYER && SLICES > 1;   // the first slice finishes the head
+  __shared__ __align__(16) float4 outputs[32];
+  __shared__ uint64_t here;
+  __shared__ int abort_flag;
+  const int slice = blockIdx.x % SLICES;
+  if (GATHER && threadIdx.x == 0) {
+    tc::mbar_init(&here, 1);
+    tc::mbar_fence_init();
+    abort_flag = 0;
+    if (slice == 0) tc::mbar_arrive_expect_tx(&here, sizeof(outputs));
+  }
   pdl_wait();
   float4 S[16];
   uint2 rolled[4];
   FinishIn fin;
   float* sp = nullptr;
   if (MODE == DEC_LAYER && warp == FW) {
-    fin = load_finish<MODE>(a, bh, lane);                    // a warp of its own: 3 x 64 heads 7.46 -> 7.17 us, 1 x 32 3.92 -> 3.84
+    if (slice == 0) fin = load_finish<MODE>(a, bh, lane);                    // a warp of its own: 3 x 64 heads 7.46 -> 7.17 us, 1 x 32 3.92 -> 3.84
   } else if (warp < SW) {
     sp = head_state(a, bh) + 4 * cl;
 #pragma unroll
@@ -557,7 +571,7 @@ __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const Decod
     if (MODE != DEC_REC && SLICES == 1) decode_roll(a, bh, warp - SW, lane, rolled);
   }
   __syncthreads();
-  if (MODE == DEC_STEP && SLICES > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // windows read
+  if (MODE != DEC_REC && SLICES > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // windows read
   if (warp < SW) state_kv(S, tok, rg, cl, part);
   __syncthreads();
   if (warp < SW) {
@@ -569,12 +583,29 @@ __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const Decod
       else { p[0] = S[i].x; p[1] = S[i].y; p[2] = S[i].z; p[3] = S[i].w; }
     }
   }
-  if (MODE == DEC_STEP && SLICES > 1) {
+  if (MODE != DEC_REC && SLICES > 1) {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (warp >= SW && blockIdx.x % SLICES == 0) decode_roll(a, bh, warp - SW, lane, rolled);
+    if (warp >= SW && warp < SW + 3 && slice == 0) decode_roll(a, bh, warp - SW, lane, rolled);
   }
   __syncthreads();
-  if (warp == FW && (SLICES == 1 || lane < 32 / SLICES)) decode_finish<MODE>(a, fin, opart, bh, SLICES == 1 ? lane : cl);
+  if (GATHER) {
+    if (warp != FW) return;
+    if (lane < 32 / SLICES) {
+      const float4 tot = part_tree(opart, cl);
+      uint32_t to, bar;
+      asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"(tc::smem_u32(&outputs[cl])));
+      asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(bar) : "r"(tc::smem_u32(&here)));
+      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to), "r"(__float_as_uint(tot.x)),
+                   "r"(__float_as_uint(tot.y)), "r"(__float_as_uint(tot.z)), "r"(__float_as_uint(tot.w)), "r"(bar)
+                   : "memory");
+    }
+    if (slice > 0) return;
+    const bool ok = tc::mbar_wait(&here, 0, &abort_flag, 1);
+    if (ok) decode_finish<MODE>(a, fin, outputs[lane], bh, lane);
+    else if (a.status) atomicExch(a.status, HK_ERR_TIMEOUT);
+    return;
+  }
+  if (warp == FW && (SLICES == 1 || lane < 32 / SLICES)) decode_finish<MODE>(a, fin, part_tree(opart, SLICES == 1 ? lane : cl), bh, SLICES == 1 ? lane : cl);
 }
 
 // persistent form: CTA c takes heads c, c + gridDim.x, ...
@@ -632,7 +663,7 @@ __global__ __launch_bounds__(KD_STREAM_THREADS) void kda_decode_stream_kernel(co
       tc::fence_async_smem();
     } else {
       if (warp == KD_WARPS) {
-        if (i > 0) decode_finish<MODE>(a, fin, opart[(i - 1) & 1], bh - step, lane);
+        if (i > 0) decode_finish<MODE>(a, fin, part_tree(opart[(i - 1) & 1], lane), bh - step, lane);
         fin = load_finish<MODE>(a, bh, lane);
       }
       if (i + 1 < n && warp < KD_WARPS) prepare(i + 1);
@@ -643,7 +674,7 @@ __global__ __launch_bounds__(KD_STREAM_THREADS) void kda_decode_stream_kernel(co
       tc::bulk_commit();
     }
   }
-  if (warp == KD_WARPS) decode_finish<MODE>(a, fin, opart[(n - 1) & 1], first + (n - 1) * step, lane);
+  if (warp == KD_WARPS) decode_finish<MODE>(a, fin, part_tree(opart[(n - 1) & 1], lane), first + (n - 1) * step, lane);
   if (threadIdx.x == 0) {
     tc::bulk_wait_all<0>();
     if (abort_flag && status) atomicExch(status, HK_ERR_TIMEOUT);
@@ -665,12 +696,12 @@ static int launch_decode(const DecodeArgs& a, cudaStream_t s) {
     const int grid = sm_count();
     return pdl_launch(kda_decode_stream_kernel<MODE>, dim3(grid), dim3(KD_STREAM_THREADS), KD_STREAM_SMEM, s, a, device_status_ptr()) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
   }
-  if constexpr (MODE != DEC_LAYER) {
-    if (vec && a.n_heads <= sm_count() / 2)
-      return pdl_launch_cluster(MODE == DEC_STEP ? 4 : 1, kda_decode_kernel<MODE, true, 4>, dim3(4 * a.n_heads), dim3(5 * 32), 0, s, a) == cudaSuccess
-                 ? HK_OK
-                 : HK_ERR_CUDA;
-  }
+  // (the layer: a slice to an SM)
+  if (vec && a.n_heads <= sm_count() / (MODE == DEC_LAYER ? 4 : 2))
+    return pdl_launch_cluster(MODE == DEC_REC ? 1 : 4, kda_decode_kernel<MODE, true, 4>, dim3(4 * a.n_heads), dim3((MODE == DEC_LAYER ? 6 : 5) * 32), 0, s,
+                              a) == cudaSuccess
+               ? HK_OK
+               : HK_ERR_CUDA;
   auto kern = vec ? kda_decode_kernel<MODE, true, 1> : kda_decode_kernel<MODE, false, 1>;
   return pdl_launch(kern, dim3(a.n_heads), dim3(KD_THREADS + (MODE == DEC_LAYER ? 32 : 0)), 0, s, a) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
 }
@@ -1317,5 +1348,6 @@ HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* c
   a.H = a.Hk = num_heads;
   a.n_heads = bsz * num_heads;
   a.slots = slots;
+  a.status = device_status_ptr();
   return launch_decode<DEC_LAYER>(a, as_stream(stream));
 }

@@ -422,7 +422,8 @@ def test_decode_step_with_conv_inside_equals_the_two_launch_sequence(H, bsz):
     assert max_rel(o32_b[0].cpu().numpy().reshape(bsz, 1, H, D), o_32) < 2e-3
 
 
-@pytest.mark.parametrize("H,bsz,w_bf16,g_bf16,y_f16", [(32, 1, True, False, True), (4, 3, False, True, False), (64, 2, True, True, True)])
+@pytest.mark.parametrize("H,bsz,w_bf16,g_bf16,y_f16", [(32, 1, True, False, True), (4, 3, False, True, False), (64, 2, True, True, True),
+                                                        (37, 1, True, False, True), (19, 2, False, False, False)])
 def test_decode_layer_in_one_launch_equals_the_five_call_sequence(H, bsz, w_bf16, g_bf16, y_f16):
     """hk_kda_decode_layer (cast, gate preparation, conv, recurrence, gated RMS norm of one decoded token in ONE launch)
     against kda_transpose_cast -> kda_gate -> cuda_causal_conv1d_update -> cuda_recurrent_gated_delta_rule ->
