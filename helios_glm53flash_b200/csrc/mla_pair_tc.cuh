@@ -7,7 +7,7 @@
 // both places and are copied inside the SM - and what its products read of K and V is 64 KB instead of 128.
 // What bounds it: power.  A tile takes 1,230 cycles at the 1.32 GHz that the power limit leaves (a CTA a row: 1,900 at 1.6), most of it the
 // softmax of 64 heads x 64 keys by one warp a scheduler (1,080).  4,096 rows at 32,768 keys 17.6 -> 14.8 ms (1.27 PFLOP/s; cuBLAS 1.40
-// sustained; on another box 18.6 -> 15.7), 2,500 rows at 0 470 -> 431 us, 151 at 9,000 297 -> 228.  On the way: arrivals at the first CTA with
+// sustained; on another GPU 18.6 -> 15.7), 2,500 rows at 0 470 -> 431 us, 151 at 9,000 297 -> 228.  On the way: arrivals at the first CTA with
 // cluster-scope release cost 700 cycles each (23.1 ms); K's part given back with V's left each load 1.5 tiles of time (16.4 ms; two
 // loaders, each part given back by itself: 14.8); 64 KB from L2 a tile and CTA 16.5.
 // Roles, buffers, softmax and tensor-memory plan are those of mla_flash_tc_kernel (O 256 columns, S 2 x 32, channels 128-511 of Q 192, the
