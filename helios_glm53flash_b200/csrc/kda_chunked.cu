@@ -873,7 +873,7 @@ __device__ __forceinline__ void prep_unit(
       tc::mma_ws_f16_if(1, tmem + 64, tc::make_sdesc(a_addr + kk * 2 * LBO, LBO, SBO_K64), tc::sdesc_advance(vd, kk * 2048), idesc, kk > 0);
     tc::mma_commit(&ctx.sh->mma_bar);
   }
-  const bool ok = tc::mbar_wait(&ctx.sh->mma_bar, it & 1, ctx.abort_flag, 1);
+  const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&ctx.sh->mma_bar, it & 1, ctx.abort_flag, 1)) != 0;
   if (tid == FETCH_TID) prep_fetch_qkv(ctx, it + 1, map_qkv, map_qk, H);  // T, N, K+ and V are free
   __syncwarp();
   tc::fence_after_sync();
@@ -902,15 +902,16 @@ __device__ __forceinline__ void prep_unit(
         for (int u = 0; u < 4; u++) *reinterpret_cast<uint4*>(dst + u * 1024) = piece(r + 8 * u, 0u);
       }
     }
-    if (warp < 4) {
-      tc::fence_async_smem();
-      asm volatile("bar.arrive %0, 160;" ::"r"(ctx.bar_id + 4) : "memory");
-    } else if (warp == PUB_WARP) {
-      asm volatile("bar.sync %0, 160;" ::"r"(ctx.bar_id + 4) : "memory");
-      if (tid == PUB_WARP * 32) {
-        tc::bulk_s2g(out + U_WQ, sK, 8 * WQ_ROWS);
-        tc::bulk_commit();
-      }
+  }
+  // (the warps meet whatever their waits said: behind one that gave up, the warps of this worker need not agree)
+  if (warp < 4) {
+    tc::fence_async_smem();
+    asm volatile("bar.arrive %0, 160;" ::"r"(ctx.bar_id + 4) : "memory");
+  } else if (warp == PUB_WARP) {
+    asm volatile("bar.sync %0, 160;" ::"r"(ctx.bar_id + 4) : "memory");
+    if (ok && tid == PUB_WARP * 32) {
+      tc::bulk_s2g(PREP_OUT + U_WQ, sK, 8 * WQ_ROWS);
+      tc::bulk_commit();
     }
   }
   tc::fence_before_sync();

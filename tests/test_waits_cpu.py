@@ -1,0 +1,87 @@
+"""No-GPU check of the kernels' source: a wait that gives up must not leave others waiting.
+
+Every wait of the kernels is bounded, and its result is each thread's own: when one expires, some threads of a block see what they waited
+for and others do not.  What stands under a condition on such a result must therefore hold no block, named or cluster barrier: the others
+would wait for good, or a half count would be left for the next use."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "helios_glm53flash_b200", "csrc")
+FILES = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
+WAIT = re.compile(r"\b(mbar_wait|pt_wait|wait_u|poll_flag\w*)\b")
+BARRIER = re.compile(r"bar\.sync|bar\.arrive|bar\.red|barrier\.c|__syncthreads|cluster\.sync|\bprep_sync\b|\bprep_publish\b")
+
+
+def _clean(text):
+    """comments out, line numbers kept"""
+    text = re.sub(r"/\*.*?\*/", lambda m: "\n" * m.group().count("\n"), text, flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def _close(text, i, pair):
+    """index behind the bracket that closes text[i]"""
+    depth = 0
+    while i < len(text):
+        if text[i] == '"':
+            i = text.index('"', i + 1)
+        elif text[i] == pair[0]:
+            depth += 1
+        elif text[i] == pair[1]:
+            depth -= 1
+            if depth == 0:
+                return i + 1
+        i += 1
+    raise ValueError("unbalanced")
+
+
+def _guarded(text, i):
+    """the statement that starts at text[i], with its else"""
+    start = i
+    while True:
+        while text[i].isspace():
+            i += 1
+        m = re.compile(r"(?:if(?:\s+constexpr)?|for|while)\s*(?=\()").match(text, i)
+        if m:
+            i = _close(text, m.end(), "()")
+            continue
+        if text[i] == "{":
+            i = _close(text, i, "{}")
+        else:
+            while text[i] != ";":
+                i = _close(text, i, text[i] + {"(": ")", "{": "}"}[text[i]]) if text[i] in "({" else i + 1
+            i += 1
+        m = re.compile(r"\s*else\b").match(text, i)
+        if not m:
+            return text[start:i]
+        i = m.end()
+
+
+def faults(text):
+    """(line, what, condition) of what stands under a condition on a wait's result and must not"""
+    text = _clean(text)
+    results = {m.group(1) for m in re.finditer(r"\b(\w+)\s*=(?!=)\s*([^;{}]*);", text) if WAIT.search(m.group(2))}
+    found = []
+    for m in re.finditer(r"\bif\s*(?=\()", text):
+        end = _close(text, m.end(), "()")
+        cond = text[m.end():end]
+        if not WAIT.search(cond) and not results & set(re.findall(r"\w+", cond)):
+            continue
+        bad = [b.group() for b in BARRIER.finditer(_guarded(text, end))]
+        found += [(text.count("\n", 0, m.start()) + 1, b, cond) for b in bad]
+    return found
+
+
+@pytest.mark.parametrize("path", FILES, ids=[os.path.basename(f) for f in FILES])
+def test_nothing_that_others_wait_for_hangs_on_a_single_threads_wait(path):
+    assert faults(open(path).read()) == []
+
+
+def test_the_reader_sees_the_forms_of_the_fault():
+    wait = "const bool ok = tc::mbar_wait(&b, 0, &f, 1);"
+    assert faults(wait + 'if (ok) { x(); if (w < 4) asm volatile("bar.arrive %0, 160;" ::"r"(1)); }')
+    assert faults(wait + "if (ok) go(); else __syncthreads();")
+    assert faults("const bool ok = __all_sync(~0u, tc::mbar_wait(&b, 0, &f, 1)) != 0; if (ok) { __syncthreads(); }")
+    assert not faults(wait + "if (ok) { x(); } __syncthreads();")
