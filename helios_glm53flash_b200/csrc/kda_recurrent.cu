@@ -600,7 +600,7 @@ __global__ __launch_bounds__(KD_THREADS + 32) void kda_decode_kernel(const Decod
                    : "memory");
     }
     if (slice > 0) return;
-    const bool ok = tc::mbar_wait(&here, 0, &abort_flag, 1);
+    const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&here, 0, &abort_flag, 1)) != 0;   // (the norm is the whole warp's)
     if (ok) decode_finish<MODE>(a, fin, outputs[lane], bh, lane);
     else if (a.status) atomicExch(a.status, HK_ERR_TIMEOUT);
     return;

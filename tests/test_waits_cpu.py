@@ -1,8 +1,9 @@
 """No-GPU check of the kernels' source: a wait that gives up must not leave others waiting.
 
 Every wait of the kernels is bounded, and its result is each thread's own: when one expires, some threads of a block see what they waited
-for and others do not.  What stands under a condition on such a result must therefore hold no block, named or cluster barrier: the others
-would wait for good, or a half count would be left for the next use."""
+for and others do not.  What stands under a condition on such a result must therefore be nothing that other threads have to take part in:
+no block, named or cluster barrier (the others would wait for good, or a half count would be left for the next use), no warp shuffle or
+vote.  A result that a vote made the warp's own may guard the warp's collectives, still no barrier."""
 import glob
 import os
 import re
@@ -13,6 +14,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 FILES = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
 WAIT = re.compile(r"\b(mbar_wait|pt_wait|wait_u|poll_flag\w*)\b")
 BARRIER = re.compile(r"bar\.sync|bar\.arrive|bar\.red|barrier\.c|__syncthreads|cluster\.sync|\bprep_sync\b|\bprep_publish\b")
+COLLECTIVE = re.compile(r"__shfl\w*|__(all|any|ballot)_sync|__reduce_\w+_sync|\bwarp_(sum|max)\b")
 
 
 def _clean(text):
@@ -59,17 +61,41 @@ def _guarded(text, i):
         i = m.end()
 
 
+def _collectives(text):
+    """functions of the file that hold a warp collective, or call one that does"""
+    bodies = {}
+    for m in re.finditer(r"__device__ __forceinline__ [\w:<>]+ (\w+)\(", text):
+        end = _close(text, m.end() - 1, "()")
+        brace = re.compile(r"\s*(?=\{)").match(text, end)
+        if brace:
+            bodies[m.group(1)] = text[brace.end():_close(text, brace.end(), "{}")]
+    held = {n for n, b in bodies.items() if COLLECTIVE.search(b)}
+    while True:
+        more = {n for n, b in bodies.items() if n not in held and any(re.search(r"\b%s\b" % h, b) for h in held)}
+        if not more:
+            return held - {"mbar_wait"}
+        held |= more
+
+
 def faults(text):
     """(line, what, condition) of what stands under a condition on a wait's result and must not"""
     text = _clean(text)
-    results = {m.group(1) for m in re.finditer(r"\b(\w+)\s*=(?!=)\s*([^;{}]*);", text) if WAIT.search(m.group(2))}
+    results = [(m.start(), m.group(1), "__all_sync" in m.group(2))                # (where, name, the warp's own)
+               for m in re.finditer(r"\b(\w+)\s*=(?!=)\s*([^;{}]*);", text) if WAIT.search(m.group(2))]
+    calls = _collectives(text)
     found = []
     for m in re.finditer(r"\bif\s*(?=\()", text):
         end = _close(text, m.end(), "()")
         cond = text[m.end():end]
-        if not WAIT.search(cond) and not results & set(re.findall(r"\w+", cond)):
+        kinds = {n: whole for at, n, whole in results if at < m.start() and re.search(r"\b%s\b" % n, cond)}   # the last before
+        if WAIT.search(cond):
+            kinds[""] = "__all_sync" in cond
+        if not kinds:
             continue
-        bad = [b.group() for b in BARRIER.finditer(_guarded(text, end))]
+        body = _guarded(text, end)
+        bad = [b.group() for b in BARRIER.finditer(body)]
+        if "__all_sync" not in cond and not all(kinds.values()):
+            bad += [c.group() for c in COLLECTIVE.finditer(body)] + [c for c in calls if re.search(r"\b%s(<\w+>)?\(" % c, body)]
         found += [(text.count("\n", 0, m.start()) + 1, b, cond) for b in bad]
     return found
 
@@ -83,5 +109,8 @@ def test_the_reader_sees_the_forms_of_the_fault():
     wait = "const bool ok = tc::mbar_wait(&b, 0, &f, 1);"
     assert faults(wait + 'if (ok) { x(); if (w < 4) asm volatile("bar.arrive %0, 160;" ::"r"(1)); }')
     assert faults(wait + "if (ok) go(); else __syncthreads();")
+    assert faults(wait + "if (a && ok) v = __shfl_xor_sync(~0u, v, 1);")
+    assert faults("__device__ __forceinline__ void fin(int a) { s = warp_sum(a); }" + wait + "if (ok) fin(3);")
+    assert not faults("const bool ok = __all_sync(~0u, tc::mbar_wait(&b, 0, &f, 1)) != 0; if (ok) v = __shfl_xor_sync(~0u, v, 1);")
     assert faults("const bool ok = __all_sync(~0u, tc::mbar_wait(&b, 0, &f, 1)) != 0; if (ok) { __syncthreads(); }")
     assert not faults(wait + "if (ok) { x(); } __syncthreads();")
