@@ -72,7 +72,9 @@ __device__ __forceinline__ void pt_mma_second(uint32_t leader, uint32_t d, uint6
       "l"(ad), "l"(bd), "r"(idesc), "r"((uint32_t)acc), "r"(leader), "r"(0xffffffffu), "r"(0u)
       : "memory");
 }
-__device__ __forceinline__ void pt_commit(uint32_t leader, uint64_t* bar) {   // arrives at this barrier in both CTAs
+// Arrives at this barrier in both CTAs, some time after the products.  Each such arrival is waited for in both CTAs before either may leave (a
+// slot that no tile takes over again is therefore not given back): behind its end a CTA's shared memory is another's.
+__device__ __forceinline__ void pt_commit(uint32_t leader, uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
       "setp.ne.b32 q, %1, 0;\n\t"
@@ -248,7 +250,7 @@ __global__ __launch_bounds__(PT_THREADS, 1) void mla_pair_tc_kernel(
             pt_mma_tmem_a(leader, tmem + FT_S + b * 32, tmem + FT_Q + (kk - FT_QS / 16) * 8, bd, idesc, true);
         }
         pt_commit(leader, &ms.s_full[b]);
-        pt_commit(leader, &ms.k_free[kb]);
+        if (t + FT_NBUF < n_tiles) pt_commit(leader, &ms.k_free[kb]);
       }
     } else if (rank == 0) {
       const uint32_t idesc = tc::make_idesc(128, 256, tc::FMT_F16, tc::FMT_F16, false, true);
@@ -272,7 +274,7 @@ __global__ __launch_bounds__(PT_THREADS, 1) void mla_pair_tc_kernel(
             pt_mma_second(leader, tmem + FT_O + nh * 128, pd, tc::sdesc_advance(vd, nh * 2 * PT_BLK), idesc, true);
         }
         pt_commit(leader, &ms.pv_done[b]);
-        pt_commit(leader, &ms.v_free[kb]);
+        if (t + FT_NBUF < n_tiles) pt_commit(leader, &ms.v_free[kb]);
       }
     }
   } else {
@@ -376,6 +378,7 @@ __global__ __launch_bounds__(PT_THREADS, 1) void mla_pair_tc_kernel(
     }
     // ---- the row's output: 2 x 64 channels at a time through the P buffers, thread half h has channels 256 h .. 256 h + 255 ----
     ms.l[tid] = l;
+    if (n_tiles >= 2) wait_pv(n_tiles - 2, 36);
     wait_pv(n_tiles - 1, 31);
     tc::fence_after_sync();
     asm volatile("bar.sync 3, 128;" ::: "memory");
@@ -417,6 +420,9 @@ __global__ __launch_bounds__(PT_THREADS, 1) void mla_pair_tc_kernel(
     }
     if (tid == 0) tc::bulk_wait_read<0>();
   }
+  // Behind a wait that gave up the loops above ran on: what they asked for ends first (far less than a millisecond).
+  if (*abort_flag)
+    for (const long long t0 = clock64(); clock64() - t0 < 4000000;) __nanosleep(1000);
   tc::fence_before_sync();
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");   // nothing of either CTA is in use any more

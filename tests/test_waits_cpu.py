@@ -114,3 +114,43 @@ def test_the_reader_sees_the_forms_of_the_fault():
     assert not faults("const bool ok = __all_sync(~0u, tc::mbar_wait(&b, 0, &f, 1)) != 0; if (ok) v = __shfl_xor_sync(~0u, v, 1);")
     assert faults("const bool ok = __all_sync(~0u, tc::mbar_wait(&b, 0, &f, 1)) != 0; if (ok) { __syncthreads(); }")
     assert not faults(wait + "if (ok) { x(); } __syncthreads();")
+
+
+def _conditions(text, at, names):
+    """the conditions around text[at] that are formed from `names` alone, as one expression"""
+    found = []
+    for m in re.finditer(r"\bif\s*(?=\()", text):
+        end = _close(text, m.end(), "()")
+        if end <= at < end + len(_guarded(text, end)):
+            cond = text[m.end():end]
+            if set(re.findall(r"[A-Za-z_]\w*", cond)) <= names:
+                found.append(cond.replace("&&", " and "))
+    return " and ".join(found) or "True"
+
+
+@pytest.mark.parametrize("n_tiles", [1, 2, 3, 4, 5, 6, 7, 8, 13])
+def test_every_commit_that_arrives_at_both_ctas_of_a_pair_is_waited_for(n_tiles):
+    """An arrival that nobody waits for may reach a CTA's shared memory after its end.  By the conditions in the source: the tiles whose
+    products are announced on a barrier are the tiles that are waited for on it."""
+    text = _clean(open(os.path.join(CSRC, "mla_pair_tc.cuh")).read())
+    ring = int(re.search(r"\bFT_NBUF = (\d+)", _clean(open(os.path.join(CSRC, "mla_flash_tc.cu")).read())).group(1))
+    names = {"t", "n_tiles", "FT_NBUF"}
+
+    def tiles(at, which="t"):
+        cond, env = _conditions(text, at, names), {"n_tiles": n_tiles, "FT_NBUF": ring}
+        loop = range(n_tiles) if "t" in re.findall(r"\w+", which + " " + cond) else [0]
+        return {eval(which, {}, {**env, "t": t}) for t in loop if eval(cond, {}, {**env, "t": t})}
+
+    announced, seen = {}, {}
+    for m in re.finditer(r"pt_commit\(leader, &ms\.(\w+)\[", text):
+        announced.setdefault(m.group(1), set()).update(tiles(m.start()))
+    assert set(announced) == {"s_full", "k_free", "pv_done", "v_free"}
+    for m in re.finditer(r"(?:mbar_wait<FT_POLL_NS>|pt_wait)\(&ms\.(s_full|k_free|v_free)\[", text):
+        # a slot's release is waited for by the tile that takes it over
+        seen.setdefault(m.group(1), set()).update(tiles(m.start(), "t" if m.group(1) == "s_full" else "t - FT_NBUF"))
+    for m in re.finditer(r"\bwait_pv\(([^,()]+), \d+\)", text):
+        if "__any_sync" not in text[text.rindex("\n", 0, text.rindex("if (", 0, m.start())):m.start()]:
+            seen.setdefault("pv_done", set()).update(tiles(m.start(), m.group(1)))
+    assert seen["k_free"] == announced["k_free"] and seen["v_free"] == announced["v_free"]
+    assert seen["s_full"] == announced["s_full"] == set(range(n_tiles))
+    assert seen["pv_done"] == announced["pv_done"] == set(range(n_tiles))
