@@ -136,7 +136,7 @@ __global__ __launch_bounds__(IP_THREADS, 1) void indexer_tc_prefill_kernel(
     for (int i = 0; i < n_tiles; i++) {
       const int p = (t0 + i) * IX_TILE_P + pl;
       for (int g = 0; g < n_grp; g++) {
-        ok = tc::mbar_wait<20>(&acc_full[g], i & 1, &abort_flag, 15) && ok;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait<20>(&acc_full[g], i & 1, &abort_flag, 15)) != 0 && ok;
         tc::fence_after_sync();
         const int row0 = g * IX_RG + rhalf * 4;                 // first of this warp's four rows (CTA-relative)
         if (ok && row0 < nr_total) {

@@ -108,7 +108,7 @@ __global__ __launch_bounds__(128) void indexer_tc_kernel(
       }
       tc::mma_commit(&bar);
     }
-    const bool ok = tc::mbar_wait(&bar, parity, &abort_flag, 1);
+    const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&bar, parity, &abort_flag, 1)) != 0;
     parity ^= 1;
     tc::fence_after_sync();
     if (ok) {
@@ -228,7 +228,7 @@ __global__ __launch_bounds__(128) void indexer_tc_decode_kernel(
         tc::mma_f16(tmem, tc::sdesc_advance(ad0, kk * 2 * IXD_LBO), tc::sdesc_advance(bd0, kk * 2 * IXD_LBO), idesc, kk > 0);
       tc::mma_commit(&bar);
     }
-    const bool ok = tc::mbar_wait(&bar, parity, &abort_flag, 1);
+    const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&bar, parity, &abort_flag, 1)) != 0;
     parity ^= 1;
     tc::fence_after_sync();
     const int p = tile * IX_TILE_P + tid;          // this thread's pool (TMEM lane tid)
@@ -344,7 +344,7 @@ __global__ __launch_bounds__(128, 4) void indexer_tc_decode_few_kernel(
         tc::mma_f16(tmem, tc::sdesc_advance(ad0, kk * 2 * IXD_LBO), tc::sdesc_advance(bd0, kk * 2 * IXD_LBO), idesc, kk > 0);
       tc::mma_commit(&bar);
     }
-    const bool ok = tc::mbar_wait(&bar, parity, &abort_flag, 1);
+    const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&bar, parity, &abort_flag, 1)) != 0;
     parity ^= 1;
     tc::fence_after_sync();
     const int p = tile * IX_TILE_P + tid;          // this thread's pool (TMEM lane tid)

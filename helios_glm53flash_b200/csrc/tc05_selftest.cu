@@ -133,7 +133,7 @@ __global__ __launch_bounds__(128) void tc05_selftest_kernel(const __half* __rest
     else if (leader) tc::mma_commit(&bar);
     __syncwarp();
   }
-  const bool ok = tc::mbar_wait(&bar, 0, &abort_flag, 1);
+  const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&bar, 0, &abort_flag, 1)) != 0;
   tc::fence_after_sync();
   if (ok) {
     for (int c0 = 0; c0 < (ws ? N / 2 : N); c0 += 16) {

@@ -2,8 +2,8 @@
 
 Every wait of the kernels is bounded, and its result is each thread's own: when one expires, some threads of a block see what they waited
 for and others do not.  What stands under a condition on such a result must therefore be nothing that other threads have to take part in:
-no block, named or cluster barrier (the others would wait for good, or a half count would be left for the next use), no warp shuffle or
-vote.  A result that a vote made the warp's own may guard the warp's collectives, still no barrier."""
+no block, named or cluster barrier (the others would wait for good, or a half count would be left for the next use), no warp shuffle
+or vote, no access to tensor memory (a whole warp's).  A result that a vote made the warp's own may guard the warp's collectives, still no barrier."""
 import glob
 import os
 import re
@@ -14,7 +14,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 FILES = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
 WAIT = re.compile(r"\b(mbar_wait|pt_wait|wait_u|poll_flag\w*)\b")
 BARRIER = re.compile(r"bar\.sync|bar\.arrive|bar\.red|barrier\.c|__syncthreads|cluster\.sync|\bprep_sync\b|\bprep_publish\b")
-COLLECTIVE = re.compile(r"__shfl\w*|__(all|any|ballot)_sync|__reduce_\w+_sync|\bwarp_(sum|max)\b")
+COLLECTIVE = re.compile(r"__shfl\w*|__(all|any|ballot)_sync|__reduce_\w+_sync|\bwarp_(sum|max)\b|tmem_(ld|st)\d+")
 
 
 def _clean(text):
@@ -111,6 +111,7 @@ def test_the_reader_sees_the_forms_of_the_fault():
     assert faults(wait + "if (ok) go(); else __syncthreads();")
     assert faults(wait + "if (a && ok) v = __shfl_xor_sync(~0u, v, 1);")
     assert faults("__device__ __forceinline__ void fin(int a) { s = warp_sum(a); }" + wait + "if (ok) fin(3);")
+    assert faults(wait + "if (ok) tc::tmem_ld32(t, r);")
     assert not faults("const bool ok = __all_sync(~0u, tc::mbar_wait(&b, 0, &f, 1)) != 0; if (ok) v = __shfl_xor_sync(~0u, v, 1);")
     assert faults("const bool ok = __all_sync(~0u, tc::mbar_wait(&b, 0, &f, 1)) != 0; if (ok) { __syncthreads(); }")
     assert not faults(wait + "if (ok) { x(); } __syncthreads();")
