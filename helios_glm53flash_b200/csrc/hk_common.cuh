@@ -36,11 +36,13 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
-inline int sm_count() {
-  static int cached[64] = {0};
+inline int device_index() {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
+  return dev < 0 || dev >= 64 ? 0 : dev;
+}
+inline int sm_count(int dev = device_index()) {
+  static int cached[64] = {0};
   if (!cached[dev]) {
     int n = 0;
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
@@ -74,7 +76,8 @@ template <class... P, class... A>
 inline cudaError_t pdl_launch_cluster(unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = (int64_t)grid.x * grid.y * grid.z <= 8 * sm_count() ? 1 : 0;
+  const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
+  attr[0].val.programmaticStreamSerializationAllowed = ctas <= 128 || ctas <= 8 * sm_count() ? 1 : 0;   // (no part of a B200 has fewer than 16 SMs)
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = cluster;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
@@ -93,7 +96,7 @@ inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_
 }
 
 // device word (per device) where kernels record that a bounded wait gave up; see hk_read_device_status
-int* device_status_ptr();
+int* device_status_ptr(int dev = device_index());
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

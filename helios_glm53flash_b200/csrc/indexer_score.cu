@@ -392,11 +392,8 @@ HK_API int hk_read_device_status(int* host_out, int reset) {
 }
 
 namespace hk {
-int* device_status_ptr() {
+int* device_status_ptr(int dev) {
   static int* ptr[64] = {nullptr};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
   if (!ptr[dev]) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, hk_g_status) != cudaSuccess) return nullptr;
