@@ -9,7 +9,8 @@
 // Radix select: a histogram of the top 11 key bits, one of the low 5 bits inside the crossing bucket, then a single ordered
 // compaction that places the "above" entries and the tie entries at once (the reference makes two histogram sweeps and two
 // compaction sweeps of global memory).  Three kernels:
-//   dsa_topk_cluster_kernel   at most 16 rows of 4,096 to 262,144 scores, read once into the registers of a cluster of 8 or 16 CTAs
+//   dsa_topk_cluster_kernel   at most 10 rows of 4,096 to 8,192 scores or 16 of up to 262,144, read once into the registers of a cluster of 8
+//                             or 16 CTAs
 //   dsa_topk_rows_kernel      other rows of up to 16,384 scores, read once into registers, a small CTA each
 //   dsa_topk_kernel           every other call (many long rows, lengths known on the device only): one CTA of 1,024 threads per
 //                             row, which sweeps the row three times; topk_row also selects among candidates in shared memory
@@ -237,7 +238,7 @@ __global__ __launch_bounds__(TK_THREADS) void dsa_topk_kernel(
 // 4,096 x 8,192 102 -> 66, 1,024 x 16,000 43.5 -> 36.4.  (More pieces per thread instead of more threads: 128 registers and
 // spills, 1,024 x 8,191 40.7 us; 1,024 threads for 32,000 scores: 83 us against 74.)
 // Up to a row per SM nothing is shared and the time is one CTA's: 1,024 threads with one or two pieces each, 140 x 8,000 scores
-// 7.3 -> 5.0 us (up to 16 rows of more than 4,096 scores: clusters, below).
+// 7.3 -> 5.0 us (few rows of more than 4,096 scores: clusters, below).
 // ------------------------------------------------------------------------------------------------
 constexpr int TKR_MAX_THREADS = 512, TKR_MAX_PIECES = 4 * TKR_MAX_THREADS;
 
@@ -624,13 +625,14 @@ static int topk_launch(const void* scores, int s_stride, int* indices, int R, in
   };
   // (figures at the kernels.  With many rows the clusters queue for eight free SMs of one GPC each and the one-CTA kernel is 3 to 20
   // times faster, measured at 64 to 4,096 rows.  Up to 4,096 scores one CTA is faster than the cluster: 1 x 2,500 4.1 / 4.6 us, 1 x 5,000
-  // 5.1 / 4.5.  Sixteen CTAs a row: from 40,000 scores for up to 3 rows (1 x 33,000 4.8 with eight / 5.0, 1 x 50,000 5.3 / 5.1, 4 x 50,000
+  // 5.1 / 4.5; up to 8,192, a piece a thread of one CTA, from eleven rows on: 10 x 5,000 4.62 / 4.54, 11 4.62 / 4.73, 16 4.62 / 4.95, 16 x 8,192
+  // 4.58 / 4.91, 16 x 8,193 6.36 / 4.94.  Sixteen CTAs a row: from 40,000 scores for up to 3 rows (1 x 33,000 4.8 with eight / 5.0, 1 x 50,000 5.3 / 5.1, 4 x 50,000
   // 5.4 / 5.8), beyond 65,536 scores, where eight take two pieces a thread, for as many rows as there is room for at once: 7 x 65,552
   // 6.7 / 5.5, 8 x 65,552 6.5 / 10.6)
   cudaError_t e;
   if (t_ptr) e = sweeps();
   else if (pieces <= 256) e = rows(dsa_topk_rows_kernel<1, 256>, 256);
-  else if (pieces > 512 && pieces <= (int64_t)TKC_PIECES * TKC_MAX_NP && R <= 16) {
+  else if (pieces > 512 && pieces <= (int64_t)TKC_PIECES * TKC_MAX_NP && R <= (pieces <= 1024 ? 10 : 16)) {
     const bool wide = pieces > 5120 && R <= (pieces <= TKC_PIECES ? std::min(3, wide_clusters()) : wide_clusters());
     e = wide ? (pieces <= 2 * TKC_PIECES ? cluster(dsa_topk_cluster_kernel<1, 16>, 1, 16) : cluster(dsa_topk_cluster_kernel<2, 16>, 2, 16))
         : pieces <= TKC_PIECES     ? cluster(dsa_topk_cluster_kernel<1, 8>, 1, 8)

@@ -186,6 +186,17 @@ def test_topk_where_the_number_of_ctas_a_row_changes(R, T, stride_pad, offset):
     assert np.array_equal(got, orc.dsa_topk(scb, T + stride_pad, R, T, 512, 512))
 
 
+@pytest.mark.parametrize("R,T,offset", [(10, 4097, 0), (11, 4097, 0), (10, 8192, 0), (11, 8192, 0), (11, 8185, 1), (11, 8186, 1), (16, 8200, 0)])
+def test_topk_of_ten_and_eleven_rows(R, T, offset):
+    """up to 8,192 scores eleven rows are one CTA each, ten a cluster each; ties, a row of one score, a row with fewer than k"""
+    sc = np.round(synth.rng(R * T).standard_normal((R, T), dtype=np.float32) * 4) / 4
+    sc[0, :] = -2.0
+    sc[R - 1, 400:] = -np.inf
+    scb = synth.f32_to_f16_bits(sc)
+    got = _topk_gpu(scb, T, R, T, 512, 512, offset=offset)
+    assert np.array_equal(got, orc.dsa_topk(scb, T, R, T, 512, 512))
+
+
 def test_topk_selects_the_true_top_k():
     """independent of the oracle: the selection is a true top-k, above-threshold entries come out in
     ascending index order followed by the threshold ties in ascending index order"""
