@@ -79,6 +79,8 @@ SIGNATURES = {
     "hk_lse_combine_peers": (_i, [_vp, _vp, _vp, _i, _i64, _vp, _vp, _i, _i, _vp]),
     "hk_q_latent": (_i, [_vp, _vp, _vp, _i, _vp]),
     "hk_o_absorb": (_i, [_vp, _vp, _vp, _i, _vp]),
+    "hk_q_latent_beside": (_i, [_vp, _vp, _vp, _i, _vp]),
+    "hk_o_absorb_beside": (_i, [_vp, _vp, _vp, _i, _vp]),
     "hk_wuv_transpose": (_i, [_vp, _vp, _vp]),
     "hk_o_absorb_t": (_i, [_vp, _vp, _vp, _i, _vp]),
     "hk_mla_cache_append": (_i, [_vp, _vp, _vp, _vp, _c.c_longlong, _i, _f, _vp]),
@@ -552,15 +554,16 @@ def lse_combine_peers(ptrs_m, ptrs_l, ptrs_acc, n_split, rows, out, local_flags,
           _ptr(local_flags), epoch, max_wait_ms, _stream(stream))
 
 
-def q_latent(q_nope, kv_b, q_lat, m, stream=None):
-    _run("hk_q_latent", q_nope, kv_b, q_lat, m, stream)
+def q_latent(q_nope, kv_b, q_lat, m, stream=None, beside=False):
+    """`beside`, here and in o_absorb: the caller has such calls on several streams at once (hk_q_latent_beside)"""
+    _run("hk_q_latent_beside" if beside else "hk_q_latent", q_nope, kv_b, q_lat, m, stream)
 
 
 q_latent_t = q_latent
 
 
-def o_absorb(lat_out, kv_b, o, m, stream=None):
-    _run("hk_o_absorb", lat_out, kv_b, o, m, stream)
+def o_absorb(lat_out, kv_b, o, m, stream=None, beside=False):
+    _run("hk_o_absorb_beside" if beside else "hk_o_absorb", lat_out, kv_b, o, m, stream)
 
 
 def wuv_transpose(kv_b, wuv_t, stream=None):

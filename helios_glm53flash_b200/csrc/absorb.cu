@@ -11,7 +11,7 @@
 namespace hk {
 
 int absorb_gemm_tc(const void* a, const void* b, void* out, int n_rows, int K, int n_out, bool b_mn,
-                   uint64_t b_rows, uint64_t b_cols, int b_rows_per_head, int b_row_off, cudaStream_t s);
+                   uint64_t b_rows, uint64_t b_cols, int b_rows_per_head, int b_row_off, cudaStream_t s, bool beside = false);
 
 static bool absorb_force_simt() {
   static const bool v = getenv("HK_ABSORB_FORCE_SIMT") != nullptr;
@@ -87,14 +87,11 @@ __global__ __launch_bounds__(256) void o_absorb_kernel(const __half* __restrict_
   }
 }
 
-}  // namespace hk
-
-HK_API int hk_q_latent(const void* q_nope, const void* kv_b, void* q_lat, int m, void* stream) {
-  using namespace hk;
+static int q_latent(const void* q_nope, const void* kv_b, void* q_lat, int m, bool beside, void* stream) {
   HK_REQUIRE(q_nope && kv_b && q_lat && m >= 0);
   if (m == 0) return HK_OK;
   if (!absorb_force_simt()) {   // q_nope [m][64*256] x W_uk[h] = kv_b rows h*512 .. +255, [k][n] with n contiguous
-    const int st = absorb_gemm_tc(q_nope, kv_b, q_lat, m, 256, 512, true, 64 * 512, 512, 512, 0, as_stream(stream));
+    const int st = absorb_gemm_tc(q_nope, kv_b, q_lat, m, 256, 512, true, 64 * 512, 512, 512, 0, as_stream(stream), beside);
     if (st != HK_ERR_UNSUPPORTED) return st;
   }
   q_latent_kernel<<<dim3(m, 64), 256, 0, as_stream(stream)>>>((const __half*)q_nope, (const __half*)kv_b, (__half*)q_lat);
@@ -102,17 +99,31 @@ HK_API int hk_q_latent(const void* q_nope, const void* kv_b, void* q_lat, int m,
   return HK_OK;
 }
 
-HK_API int hk_o_absorb(const void* lat_out, const void* kv_b, void* o, int m, void* stream) {
-  using namespace hk;
+static int o_absorb(const void* lat_out, const void* kv_b, void* o, int m, bool beside, void* stream) {
   HK_REQUIRE(lat_out && kv_b && o && m >= 0);
   if (m == 0) return HK_OK;
   if (!absorb_force_simt()) {   // lat_out [m][64*512] x W_uv[h]^T: kv_b rows h*512+256 .. +511 are [n][k], k contiguous
-    const int st = absorb_gemm_tc(lat_out, kv_b, o, m, 512, 256, false, 64 * 512, 512, 512, 256, as_stream(stream));
+    const int st = absorb_gemm_tc(lat_out, kv_b, o, m, 512, 256, false, 64 * 512, 512, 512, 256, as_stream(stream), beside);
     if (st != HK_ERR_UNSUPPORTED) return st;
   }
   o_absorb_kernel<<<dim3(m, 64), 256, 0, as_stream(stream)>>>((const __half*)lat_out, (const __half*)kv_b, (__half*)o);
   HK_LAUNCH_CHECK();
   return HK_OK;
+}
+
+}  // namespace hk
+
+HK_API int hk_q_latent(const void* q_nope, const void* kv_b, void* q_lat, int m, void* stream) {
+  return hk::q_latent(q_nope, kv_b, q_lat, m, false, stream);
+}
+HK_API int hk_q_latent_beside(const void* q_nope, const void* kv_b, void* q_lat, int m, void* stream) {
+  return hk::q_latent(q_nope, kv_b, q_lat, m, true, stream);
+}
+HK_API int hk_o_absorb(const void* lat_out, const void* kv_b, void* o, int m, void* stream) {
+  return hk::o_absorb(lat_out, kv_b, o, m, false, stream);
+}
+HK_API int hk_o_absorb_beside(const void* lat_out, const void* kv_b, void* o, int m, void* stream) {
+  return hk::o_absorb(lat_out, kv_b, o, m, true, stream);
 }
 
 HK_API int hk_wuv_transpose(const void* kv_b, void* wuv_t, void* stream) {

@@ -223,8 +223,9 @@ template <bool W_MN, int K>
 __global__ __launch_bounds__(AF_THREADS) void absorb_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                                                      const __grid_constant__ CUtensorMap tmap_x,
                                                                      __half* __restrict__ out, int n_rows, int nb, int n_out,
-                                                                     int w_rows_per_head, int w_row_off, int* __restrict__ status) {
+                                                                     int w_rows_per_head, int w_row_off, int* __restrict__ status, bool release) {
   constexpr int NK = K / AF_BK;
+  if (release) pdl_release();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* sW = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sX = sW + NK * AF_A_CHUNK;
@@ -449,7 +450,7 @@ static bool make_map_2d(CUtensorMap* m, const void* base, uint64_t rows, uint64_
 
 template <bool W_MN, int K>
 static int absorb_few_rows(const void* x, const void* w, void* out, int n_rows, int n_out, uint64_t w_rows, uint64_t w_cols,
-                           int w_rows_per_head, int w_row_off, cudaStream_t s) {
+                           int w_rows_per_head, int w_row_off, bool release, cudaStream_t s) {
   const int nb = (n_rows + 7) & ~7;
   alignas(64) CUtensorMap mw, mx;
   memset(&mw, 0, sizeof(mw));
@@ -467,7 +468,7 @@ static int absorb_few_rows(const void* x, const void* w, void* out, int n_rows, 
   }
   const size_t smem = (size_t)(K / AF_BK) * (AF_A_CHUNK + nb * AF_BK * 2) + 1024;
   return pdl_launch(absorb_few_rows_kernel<W_MN, K>, dim3(n_out / AF_BM, 64), dim3(AF_THREADS), smem, s, mw, mx, (__half*)out, n_rows,
-                    nb, n_out, w_rows_per_head, w_row_off, device_status_ptr()) == cudaSuccess
+                    nb, n_out, w_rows_per_head, w_row_off, device_status_ptr(), release) == cudaSuccess
              ? HK_OK
              : HK_ERR_CUDA;
 }
@@ -511,18 +512,24 @@ static int absorb_rows(const void* x, const void* w, void* out, int n_rows, int 
 }
 
 // a [n_rows][64*K], weights as described above, out [n_rows][64*n_out]; returns HK_ERR_UNSUPPORTED when the
-// tensor maps cannot be built (the caller then uses the CUDA-core kernels)
+// tensor maps cannot be built (the caller then uses the CUDA-core kernels).
+// `beside`: the caller has such calls on other streams.  Up to eight rows the kernel with operands in registers is the faster one alone and the
+// slower one in company, whose 1,024 CTAs take every SM's registers while other streams' attention waits for whole SMs.  11 MLA layers of a
+// decode step, one stream a sequence, that kernel / the one of few rows: at 5,000 tokens 2 sequences 363 / 357 us, 4 474 / 440, 8 731 / 689, at
+// 32,768 381 / 372, 492 / 463, 970 / 908; one sequence 263 / 273.  (Without the early release of one row 367, 441, 684 and 382, 472, 932.)
 int absorb_gemm_tc(const void* a, const void* b, void* out, int n_rows, int K, int n_out, bool b_mn,
-                   uint64_t b_rows, uint64_t b_cols, int b_rows_per_head, int b_row_off, cudaStream_t s) {
+                   uint64_t b_rows, uint64_t b_cols, int b_rows_per_head, int b_row_off, cudaStream_t s, bool beside) {
   if (!aligned(a, 16) || !aligned(b, 16) || !aligned(out, 16)) return HK_ERR_UNSUPPORTED;
-  if (n_rows <= A8_ROWS) {
+  if (n_rows <= A8_ROWS && !beside) {
     if (K == 256 && b_mn) return absorb_8_rows<true, 256>(a, b, out, n_rows, n_out, b_rows_per_head, b_row_off, s);
     if (K == 512 && !b_mn) return absorb_8_rows<false, 512>(a, b, out, n_rows, n_out, b_rows_per_head, b_row_off, s);
   }
-  if (n_rows <= AF_MAX_ROWS) {   // q_latent (K 256, n contiguous), o_absorb (K 512, k contiguous), o_absorb_t (K 512, n contiguous)
-    if (K == 256 && b_mn) return absorb_few_rows<true, 256>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
-    if (K == 512 && !b_mn) return absorb_few_rows<false, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
-    if (K == 512 && b_mn) return absorb_few_rows<true, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
+  if (n_rows <= AF_MAX_ROWS) {
+    const bool release = beside && n_rows == 1;
+    // q_latent (K 256, n contiguous), o_absorb (K 512, k contiguous), o_absorb_t (K 512, n contiguous)
+    if (K == 256 && b_mn) return absorb_few_rows<true, 256>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, release, s);
+    if (K == 512 && !b_mn) return absorb_few_rows<false, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, release, s);
+    if (K == 512 && b_mn) return absorb_few_rows<true, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, release, s);
   }
   if (K == 256 && b_mn) return absorb_rows<true, 256>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);
   if (K == 512 && !b_mn) return absorb_rows<false, 512>(a, b, out, n_rows, n_out, b_rows, b_cols, b_rows_per_head, b_row_off, s);

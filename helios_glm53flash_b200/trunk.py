@@ -205,7 +205,7 @@ class TrunkAttention:
             t.arange(pos, pos + n, dtype=t.int32, device="cuda", out=wb.qpos[:n])
         if timed:
             self._mark("mla_append_kpool")
-        hk.q_latent(mi["q_nope"], mi["kv_b"], wb.q_lat, n)
+        hk.q_latent(mi["q_nope"], mi["kv_b"], wb.q_lat, n, beside=bufs is not None)
         if timed:
             self._mark("mla_q_latent")
         npools = (pos + n) // 4
@@ -239,7 +239,7 @@ class TrunkAttention:
         hk.mla_sparse_decode(wb.q_lat, ckv, wb.raw_idx, KIDX, wb.lat_out, n, n_split=ns if bufs else 0, workspace=wb.sparse_ws)
         if timed:
             self._mark("mla_sparse_attention")
-        hk.o_absorb(wb.lat_out, mi["kv_b"], wb.o_abs, n)
+        hk.o_absorb(wb.lat_out, mi["kv_b"], wb.o_abs, n, beside=bufs is not None)
         if timed:
             self._mark("mla_o_absorb")
         if self.keep:

@@ -346,6 +346,36 @@ def test_absorbed_projections_of_few_rows(m):
         assert max_rel(f(bits(got[:m])), want) < 2e-3 and (got[m:] == 7).all()
 
 
+@pytest.mark.parametrize("m", [1, 2, 8, 9])
+def test_absorbed_projections_beside_others_on_streams(m):
+    """two streams at once, weights-as-M form for up to eight rows too (one row releases its dependents); from nine rows on the same form as
+    a call that is alone.  Rows past m stay untouched"""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    kb = (0.1 * torch.randn(32768, 512, generator=g, device="cuda")).half()
+    w = kb.view(64, 512, 512).float()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = []
+    for s in streams:
+        qn, lo = (torch.randn(m, 64, k, generator=g, device="cuda").half() for k in (256, 512))
+        ql, o = (torch.full((m + 1, 64, n), 7.0, dtype=torch.float16, device="cuda") for n in (512, 256))
+        got.append((s, qn, lo, ql, o))
+    torch.cuda.synchronize()
+    for s, qn, lo, ql, o in got:
+        for _ in range(3):
+            hk.q_latent(qn, kb, ql, m, stream=s, beside=True)
+            hk.o_absorb(lo, kb, o, m, stream=s, beside=True)
+    torch.cuda.synchronize()
+    assert hk.read_device_status() == 0
+    for s, qn, lo, ql, o in got:
+        for out, want in ((ql, torch.einsum("rhk,hkn->rhn", qn.float(), w[:, :256])), (o, torch.einsum("rhk,hnk->rhn", lo.float(), w[:, 256:]))):
+            assert (out[:m].float() - want).abs().max() < 2e-3 * want.abs().max()
+            assert (out[m] == 7.0).all()
+        if m > 8:
+            alone = torch.empty_like(ql[:m])
+            hk.q_latent(qn, kb, alone, m)
+            assert torch.equal(alone, ql[:m])
+
+
 def test_peer_combine_on_one_gpu_and_bounded_wait_times_out_cleanly():
     """the cross-GPU combine path with every 'peer' on this GPU: flags set by hk_peer_signal release the
     wait; a slot that nothing sets makes the bounded wait expire - the kernel returns, the status word
