@@ -404,18 +404,7 @@ __device__ __forceinline__ void prep_tma_rows(uint8_t* dst, const CUtensorMap* m
       "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(t), "r"(c32), "r"(b), "r"(tc::smem_u32(bar))
       : "memory");
 }
-// asks for the next unit's q, k and v rows in L2 (their place is free when most of this unit is over; from HBM they then took longer than
-// what was left to do)
-__device__ __forceinline__ void prep_prefetch_qkv(const PrepCtx& ctx, int it, const CUtensorMap* map_qkv, int H) {
-  if (PREP_UNIT(n_valid, it) == 0) return;
-  const int c = PREP_UNIT(head, it) * KD, t0 = PREP_UNIT(t0, it), b = PREP_UNIT(b, it);
-#pragma unroll
-  for (int i = 0; i < 6; i++)
-    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map_qkv)),
-                 "r"((i >> 1) * H * KD + c + 64 * (i & 1)), "r"(t0), "r"(b)
-                 : "memory");
-}
-// the next unit's inputs, each as soon as its place is free (one thread)
+// the next unit's inputs, each as soon as its place is free (one thread).  (q, k and v asked for in L2 earlier: 1,849 -> 1,861 us a layer.)
 __device__ __forceinline__ void prep_fetch_g(const PrepCtx& ctx, int it, const CUtensorMap* map_g) {
   if (PREP_UNIT(n_valid, it) == 0) return;
   const int c = PREP_UNIT(head, it) * KD, t0 = PREP_UNIT(t0, it), b = PREP_UNIT(b, it);
@@ -749,9 +738,7 @@ __device__ __forceinline__ void prep_unit(
 
   // ---- stage 3: the products with earlier blocks (fp16), 2 I tiles a warp; the warps of the first block, which have none, invert the
   //      16 x 16 diagonal blocks of I + N, those of the second convert v as well ----
-  if (tid == 0) {
-    prep_fetch_g(ctx, it + 1, map_g);                      // x is free
-  }
+  if (tid == 0) prep_fetch_g(ctx, it + 1, map_g);          // x is free
   __syncwarp();
   {
     float* nrow = sN + prep_n_row(t) + 2 * tig;
