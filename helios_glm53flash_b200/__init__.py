@@ -90,6 +90,8 @@ SIGNATURES = {
     "hk_tc05_selftest": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp]),
 }
 
+SIGNATURES["hk_kda_decode_layer_beside"] = SIGNATURES["hk_kda_decode_layer"]
+
 _lib = None
 
 
@@ -231,12 +233,13 @@ def kda_decode_step(x, conv_state, conv_weight, conv_bias, g, beta, rec_state, o
 
 def kda_decode_layer(x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_log, lower_bound, rec_state, out, norm_w,
                      gate_out, y, bsz, num_heads, epsilon=1e-6, gate_act=1, constant_bias=0.0, slots=None, out_f32=None,
-                     stream=None, tickets=None):
+                     stream=None, tickets=None, beside=False):
     """The KDA layer of one decoded token in ONE launch (src/engine/runner.cpp:433-489 runs five): x = bf16(x32)
     (glue::kda_transpose_cast of one row), g / beta from f / b (glue::kda_gate), short conv + SiLU, recurrence, gated RMS
     norm of the output (aux::gated_rms_norm with gate `gate_out`, weight `norm_w`) -> y.  `out` receives the recurrence
-    output as the separate calls would leave it.  `tickets` is accepted for earlier callers and not used."""
-    _run("hk_kda_decode_layer", x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_log, lower_bound, rec_state, out,
+    output as the separate calls would leave it.  `tickets` is accepted for earlier callers and not used.  `beside`: the caller
+    has such calls on four or more streams at once (hk_kda_decode_layer_beside; same bits)."""
+    _run("hk_kda_decode_layer_beside" if beside else "hk_kda_decode_layer", x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_log, lower_bound, rec_state, out,
          out_f32, norm_w, norm_w, gate_out, gate_out, y, y, epsilon, constant_bias, int(gate_act), bsz, num_heads, slots,
          tickets, stream)
 

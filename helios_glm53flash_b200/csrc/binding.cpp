@@ -171,7 +171,7 @@ struct Entry<R (*)(A...)> {
   X(hk_pool_expand, true) X(hk_mla_partial_bytes, false) X(hk_mla_auto_splits, false) X(hk_mla_sparse, true)                 \
   X(hk_mla_sparse_static, true) X(hk_mla_dense, true) X(hk_mla_dense_partial, true) X(hk_mla_dense_partial_ws, true)         \
   X(hk_lse_combine, true) X(hk_q_latent, true) X(hk_o_absorb, true) X(hk_wuv_transpose, true) X(hk_o_absorb_t, true)         \
-  X(hk_q_latent_beside, true) X(hk_o_absorb_beside, true)                                                                    \
+  X(hk_q_latent_beside, true) X(hk_o_absorb_beside, true) X(hk_kda_decode_layer_beside, true)                                \
   X(hk_mla_cache_append, true) X(hk_layernorm_f16, true) X(hk_mla_decode_prologue, true)
 
 #define X(name, stream)                                                                      \

@@ -143,7 +143,8 @@ __device__ __forceinline__ bool poll_flag_ge(const int* flag, int want, volatile
 // k row and of the q row.  That is the fragment layout of the warp-level products in both places: as the left operand (rows
 // 0-7 of a 16-row tile = k tokens, rows 8-15 = the q rows of the same tokens) and as the right operand (columns = tokens), so the
 // product of a warp's tokens with themselves needs no shared memory, and one exponential serves k and q.
-// Every input tile arrives by tiled tensor copies in the 128-byte-swizzle pattern (16-byte piece p of row r at p ^ (r % 8)).
+// Inputs arrive by tiled tensor copies: v and the log decays in the 128-byte-swizzle pattern (16-byte piece p of row r at p ^ (r % 8)), q and k
+// in rows of 64 bytes without a swizzle.
 constexpr uint32_t P1_PIECE = 1056;                      // bytes between the 8-channel pieces of K+ (1024 + 32: the four pieces that a
                                                          // quarter-warp writes start in different banks)
 constexpr uint32_t P1_X = 0;                             // f32 log decays, then their sums x: four boxes [64 tokens][32 channels]; then the
@@ -1446,12 +1447,14 @@ int g_chunked_form = 0;
 // Chain slots of the fused launch and the value columns of a chain CTA for n_jobs (batch, head) chains; no slots = use the two-kernel
 // form.  Chains share slots evenly (a slot walks its chains one after the other), and the preparation keeps 64 SMs or more.  Of the
 // divisors of n_jobs from 16 to 48, or n_jobs itself, the one for which the longer of the two sides takes least per chunk of all
-// chains: a chain CTA is taken to need 1,380 ns a chunk with all 128 columns, 1,100 with 64, an SM of preparation workers 5,800 ns a unit (the
-// line between the shapes; 1,550 : 1,150 : 4,700, nearer to what they need with 32 heads, chose 48 slots for 3 x 8,192 x 32: 1,190 us, 1,096
-// with 32).  Waits counted in a measuring build, 32,768 tokens x 32 heads: neither side is much the longer one, a worker waits 2,060 of a
-// unit's 20,600 cycles for a ring slot, a chain CTA 600 of a chunk's 3,000 for the 48 KB it needs first; with 16 and 8 the chains are.
-// (32,768 tokens x 8 heads 719 -> 532 us with two CTAs a chain, x 16 725 -> 580; 32 heads have one, at 84 SMs of workers they would
-// take 1,150; 3 sequences x 8,192 x 32 heads 786 with 48 slots of two chains, 685 with 32 of three.)
+// chains.  The weights are tuned, not what the sides need: a chain CTA counts 1,380 a chunk with all 128 columns, 1,100 with 64, an SM of
+// preparation workers 5,800 a unit (with 32 heads they need about 1,550 ns, 1,150 and 4,700, by which 3 x 8,192 x 32 would get 48 slots: 754 us,
+// 664 with 32; a slot's start and the units' whole rounds are not in the sum).  What they choose was the fastest of all candidates at each of
+// 18 shapes, among them 32,768 tokens x 8, 16, 32 heads, 16,384 x 64, 2 x 12,000 x 64, 4 x 3,000 x 16, 8 x 4,096 x 32, 6 x 4,000 x 24,
+// 12 x 2,048 x 8, 3 x 5,000 x 16; us, chosen / next: 32,768 x 32 870 with a CTA a chain / 1,169 with two, x 16 573 with two / 686, x 8 561 / 686,
+// 3 x 5,000 x 16 250 with 24 slots / 253 with 48, 5 x 4,096 x 32 562 with 32 / 593 with 40.
+// Waits counted in a measuring build, 32,768 tokens x 32 heads: neither side is much the longer one, a worker waits 2,060 of a unit's 20,600
+// cycles for a ring slot, a chain CTA 600 of a chunk's 3,000 for the 48 KB it needs first; with 16 and 8 heads the chains are the longer side.
 // `room`: the slots that the workspace is sized for, the largest number that divides the chains: it covers calls of fewer sequences.
 struct FusedShape { int slots, nv, room; };
 FusedShape fused_shape(long long n_jobs) {
@@ -1475,8 +1478,8 @@ FusedShape fused_shape(long long n_jobs) {
   return best;
 }
 // Short calls run as two kernels although a fused form exists, in the ring's memory: the fused launch costs about 20 us before its first
-// chunk is through (flags cleared, cooperative launch, ring start-up).  Fused / two kernels, us: 8 heads x 64 tokens 25 / 18, x 512 32 /
-// 24, x 1,024 41 / 31; 32 heads x 256 33 / 21, x 1,024 60 / 49, x 1,536 75 / 72, x 2,048 89 / 92; 64 heads x 512 67 / 42.  The line
+// chunk is through (flags cleared, cooperative launch, ring start-up).  Fused / two kernels, us: 8 heads x 64 tokens 22.6 / 15.5, x 512 30.8 /
+// 21.8, x 1,024 39.0 / 29.3; 32 heads x 256 31.7 / 18.8, x 1,003 61.4 / 46.3, x 1,024 60.6 / 46.6; 64 heads x 512 67.8 / 40.1.  The line
 // is the memory: all units have to fit the ring's (16 chunks per slot).
 bool short_call(long long n_jobs, int n_chunks, int n_slots) {
   return n_jobs * n_chunks <= (long long)RING * n_slots && (2 * n_jobs <= sm_count() || n_chunks <= 12);

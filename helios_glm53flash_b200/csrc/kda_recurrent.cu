@@ -682,7 +682,7 @@ __global__ __launch_bounds__(KD_STREAM_THREADS) void kda_decode_stream_kernel(co
 }
 
 template <int MODE>
-static int launch_decode(DecodeArgs& a, cudaStream_t s) {
+static int launch_decode(DecodeArgs& a, cudaStream_t s, bool beside = false) {
   const bool vec = aligned(a.state, 16);
   // (asked for once, not four times: where the host bounds a call, one layer of 32 heads 3.81 -> 3.73 us; 3.72 with a CTA a head, 3.45 where the GPU does)
   const int dev = device_index(), sms = sm_count(dev);
@@ -695,8 +695,10 @@ static int launch_decode(DecodeArgs& a, cudaStream_t s) {
     }
     return pdl_launch(kda_decode_stream_kernel<MODE>, dim3(sms), dim3(KD_STREAM_THREADS), KD_STREAM_SMEM, s, a, device_status_ptr(dev)) == cudaSuccess ? HK_OK : HK_ERR_CUDA;
   }
-  // (the layer: a slice to an SM)
-  if (vec && a.n_heads <= sms / (MODE == DEC_LAYER ? 4 : 2)) {
+  // The layer: a slice to an SM.  Not where the caller has such calls on other streams (`beside`): a slice's CTA prepares the whole token, and
+  // two of them fill an SM.  30 layers of 32 heads on each of S streams, a CTA a head / four: S = 1 111 / 101 us, 2 117 / 117, 4 153 / 173, 6 188 /
+  // 266, 8 221 / 354; of 16 heads 4 119 / 119, 8 160 / 176.
+  if (vec && !beside && a.n_heads <= sms / (MODE == DEC_LAYER ? 4 : 2)) {
     if (MODE == DEC_LAYER) a.status = device_status_ptr(dev);
     return pdl_launch_cluster(MODE == DEC_REC ? 1 : 4, kda_decode_kernel<MODE, true, 4>, dim3(4 * a.n_heads), dim3((MODE == DEC_LAYER ? 6 : 5) * 32), 0, s,
                               a) == cudaSuccess
@@ -1307,14 +1309,12 @@ HK_API int hk_kda_decode_step(const void* x, void* conv_state, const void* conv_
   return launch_decode<DEC_STEP>(a, as_stream(stream));
 }
 
-HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f,
-                               const float* b, const float* dt_bias, const float* a_log, float lower_bound, float* rec_state,
-                               void* out, float* out_f32, const void* norm_w, int w_type, const void* gate_out, int g_type, void* y,
-                               int y_type, float epsilon, float constant_bias, int gate_act, int bsz, int num_heads,
-                               const int* slots, int* tickets, void* stream) {
-  using namespace hk;
+namespace hk {
+static int decode_layer(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f, const float* b,
+                        const float* dt_bias, const float* a_log, float lower_bound, float* rec_state, void* out, float* out_f32,
+                        const void* norm_w, int w_type, const void* gate_out, int g_type, void* y, int y_type, float epsilon, float constant_bias,
+                        int gate_act, int bsz, int num_heads, const int* slots, bool beside, void* stream) {
   HK_REQUIRE(x32 && conv_state && conv_weight && f && b && dt_bias && a_log && rec_state && out && norm_w && gate_out && y);
-  (void)tickets;
   HK_REQUIRE(bsz > 0 && bsz <= 65535 && num_heads > 0 && num_heads <= 65535);
   HK_REQUIRE(w_type == HK_F32 || w_type == HK_BF16);
   HK_REQUIRE(y_type == HK_F32 || y_type == HK_F16);
@@ -1349,5 +1349,22 @@ HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* c
   a.H = a.Hk = num_heads;
   a.n_heads = bsz * num_heads;
   a.slots = slots;
-  return launch_decode<DEC_LAYER>(a, as_stream(stream));
+  return launch_decode<DEC_LAYER>(a, as_stream(stream), beside);
+}
+}  // namespace hk
+
+HK_API int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f, const float* b,
+                               const float* dt_bias, const float* a_log, float lower_bound, float* rec_state, void* out, float* out_f32,
+                               const void* norm_w, int w_type, const void* gate_out, int g_type, void* y, int y_type, float epsilon,
+                               float constant_bias, int gate_act, int bsz, int num_heads, const int* slots, int* /*tickets*/, void* stream) {
+  return hk::decode_layer(x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_log, lower_bound, rec_state, out, out_f32, norm_w, w_type,
+                          gate_out, g_type, y, y_type, epsilon, constant_bias, gate_act, bsz, num_heads, slots, false, stream);
+}
+HK_API int hk_kda_decode_layer_beside(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f,
+                                      const float* b, const float* dt_bias, const float* a_log, float lower_bound, float* rec_state, void* out,
+                                      float* out_f32, const void* norm_w, int w_type, const void* gate_out, int g_type, void* y, int y_type,
+                                      float epsilon, float constant_bias, int gate_act, int bsz, int num_heads, const int* slots, int* /*tickets*/,
+                                      void* stream) {
+  return hk::decode_layer(x32, conv_state, conv_weight, conv_bias, f, b, dt_bias, a_log, lower_bound, rec_state, out, out_f32, norm_w, w_type,
+                          gate_out, g_type, y, y_type, epsilon, constant_bias, gate_act, bsz, num_heads, slots, true, stream);
 }

@@ -98,6 +98,13 @@ int hk_kda_decode_layer(const float* x32, void* conv_state, const void* conv_wei
                         void* out, float* out_f32, const void* norm_w, int w_type, const void* gate_out, int g_type, void* y,
                         int y_type, float epsilon, float constant_bias, int gate_act, int bsz, int num_heads,
                         const int* slots, int* tickets, void* stream);
+/* The same with a CTA a head also for few heads, for a caller that has such calls on four or more streams at once (30 layers of 32
+ * heads on each of 4 / 6 / 8 streams, the call above / this one: 173 / 153, 266 / 188, 354 / 221 us).  Same bits.          */
+int hk_kda_decode_layer_beside(const float* x32, void* conv_state, const void* conv_weight, const void* conv_bias, const float* f,
+                               const float* b, const float* dt_bias, const float* a_log, float lower_bound, float* rec_state,
+                               void* out, float* out_f32, const void* norm_w, int w_type, const void* gate_out, int g_type, void* y,
+                               int y_type, float epsilon, float constant_bias, int gate_act, int bsz, int num_heads,
+                               const int* slots, int* tickets, void* stream);
 
 /* Chunked (64-token) KDA prefill on the tensor cores; numerically equivalent to
  * hk_kda_recurrent(channelwise=1, history=0) on the same arguments (the reference has no chunked

@@ -470,6 +470,32 @@ def test_decode_layer_in_one_launch_equals_the_five_call_sequence(H, bsz, w_bf16
     assert torch.isfinite(y_b.float()).all()
 
 
+@pytest.mark.parametrize("H", [1, 32, 37, 38])
+def test_decode_layer_beside_others_on_streams_gives_the_same_bits(H):
+    """four streams at once, a CTA a head, against the call that is alone (four CTAs a head up to 37): outputs, windows and states, two tokens"""
+    D, dim, n = 128, 3 * H * 128, 4
+    gen = torch.Generator(device="cuda").manual_seed(H)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    w, dtb, alog, nw = (0.1 * r(dim, 4)).bfloat16(), r(H, D), 0.3 * r(H), (1 + 0.1 * r(D)).bfloat16()
+    calls = [dict(x=r(2, dim), f=r(2, H, D), b=r(2, H), go=r(2, H, D), cs=r(1, dim, 4).bfloat16(), rs=0.1 * r(1, 1, H, D, D)) for _ in range(n)]
+
+    def run(beside):
+        streams = [torch.cuda.Stream() for _ in range(n)] if beside else [None] * n
+        got = [(c["cs"].clone(), c["rs"].clone(), torch.empty(2, H, D, dtype=torch.bfloat16, device="cuda"),
+                torch.empty(2, H, D, dtype=torch.float16, device="cuda")) for c in calls]
+        torch.cuda.synchronize()
+        for t in range(2):
+            for c, (cs, rs, out, y), s in zip(calls, got, streams):
+                hk.kda_decode_layer(c["x"][t], cs, w, None, c["f"][t], c["b"][t], dtb, alog, -5.0, rs, out[t], nw, c["go"][t], y[t], 1, H,
+                                    stream=s, beside=beside)
+        torch.cuda.synchronize()
+        return got
+
+    for alone, beside in zip(run(False), run(True)):
+        assert all(torch.equal(a, b) for a, b in zip(alone, beside))
+    assert hk.read_device_status() == 0
+
+
 @pytest.mark.parametrize("H,bsz,slots", [(64, 5, False), (8, 41, True), (33, 9, True)])
 def test_decode_of_many_heads_streams_the_same_bits(H, bsz, slots):
     """more heads than two per SM: the persistent form (heads stream through shared memory, ragged last round) against the
